@@ -108,6 +108,33 @@ int castle_fwd_prefill(const castle_problem_t* p, const castle_tensor_t* qc, con
  */
 int castle_convert_16bit(int32_t src_dtype, const void* src, void* dst, int64_t count, const float* mul, void* stream);
 
+/* ---- element-wise passes around the parallel kernels -------------------------
+ * One pass over `count` (1 to 6) tensors of `p`'s shape, row width p->dim_head and type p->dtype: each row is
+ * rotated (rotary may be NULL; bit i of rotary_mask = tensor i is rotated), stored as it is to copies[i] (NULL
+ * array or null pointers: nowhere), multiplied by *mul (device pointer, may be NULL), converted to dst_dtype
+ * (saturating where that is fp16 and the source is not) and stored to dst[i] (null pointer: nowhere) with rows
+ * of dst_dim_head elements, cut or zero-padded.  Takes the place of the reference's rotary calls
+ * (lookahead_keys_attention/lookahead_keys_attention.py:106-112), its `.half()` casts
+ * (lookahead_keys_attention_triton.py:437-442, :523, :591-602) and the cache hand-off of callers whose type is
+ * not the kernels' operand type.
+ */
+typedef struct {
+  const void* freqs;  /* dim_head / 2 angular frequencies, NULL = no rotation */
+  int32_t dtype;      /* of freqs */
+  int32_t inverse;    /* rotate back */
+  int64_t position0;  /* position of row 0 */
+} castle_rotary_t;
+
+int castle_transform(const castle_problem_t* p, int32_t count, const castle_tensor_t* src, const castle_tensor_t* dst,
+                     int32_t dst_dtype, int32_t dst_dim_head, const castle_tensor_t* copies,
+                     const castle_rotary_t* rotary, uint32_t rotary_mask, const float* mul, void* stream);
+
+/* The power of two that brings the largest |x| of `count` contiguous elements (a multiple of 8) to at most 64:
+ * out[0] = it, out[1] = its reciprocal.  `state` = two words that are zero before the call; they are zero again
+ * when its kernel has run, so calls on one stream can share them.
+ */
+int castle_amax_scale(int32_t dtype, const void* x, int64_t count, uint32_t* state, float* out, void* stream);
+
 /* ---- parallel backward ---------------------------------------------------
  * Replaces CastleAttentionFunction.backward
  * (lookahead_keys_attention_triton.py:509-602) with its two kernels
@@ -144,7 +171,7 @@ int castle_bwd(const castle_problem_t* p, const castle_tensor_t* qc, const castl
  * attention output for the new token (:190-200).  Requires cache_len < capacity.
  * The six `*_new` tensors are the new token's (batch, heads, 1, dim_head) rows,
  * unscaled.  `workspace` holds split partials.  Caches whose position stride equals dim_head (rows adjacent in
- * memory, at least 128 bytes each) take the fastest path.
+ * memory) take the fastest path.
  */
 size_t castle_decode_workspace_bytes(const castle_problem_t* p, int32_t cache_len);
 
@@ -154,6 +181,19 @@ int castle_decode_step(const castle_problem_t* p, int32_t cache_len, int32_t cap
                        const castle_tensor_t* u_cache, const castle_tensor_t* qu_cache,
                        const castle_tensor_t* kc_cache, const castle_tensor_t* vc_cache, const castle_tensor_t* out,
                        void* workspace, size_t workspace_bytes, int32_t* status, void* stream);
+
+/* The same step with two additions.  `rotary` (may be NULL): the new rows (all but vc_new) are rotated to position
+ * rotary->position0 as they are read (lookahead_keys_attention.py:106-112), so that the caches hold rotated rows.
+ * `counters` (may be NULL): batch * heads words that are zero before the call and zero again when its kernel has
+ * run, so calls on one stream can share them; with them the step is one launch instead of two.
+ */
+int castle_decode_step_fused(const castle_problem_t* p, int32_t cache_len, int32_t capacity,
+                             const castle_tensor_t* qc_new, const castle_tensor_t* kc_new, const castle_tensor_t* vc_new,
+                             const castle_tensor_t* qu_new, const castle_tensor_t* ku_new, const castle_tensor_t* vu_new,
+                             const castle_tensor_t* u_cache, const castle_tensor_t* qu_cache,
+                             const castle_tensor_t* kc_cache, const castle_tensor_t* vc_cache, const castle_tensor_t* out,
+                             const castle_rotary_t* rotary, uint32_t* counters, void* workspace, size_t workspace_bytes,
+                             int32_t* status, void* stream);
 
 /* ---- cached single-token step without caller scratch -----------------------
  * (no counterpart in the reference)  Same step and same arguments as

@@ -1,7 +1,7 @@
-"""Build and load the C-ABI CUDA library (`libcastle_b200.so`, built in-tree).
+"""Build and load the two native parts of the package, both built in-tree: the C-ABI CUDA library
+(`libcastle_b200.so`) and the torch-facing host module (`_host.so`), which prepares its calls.
 
-There is no fallback: if the library is missing or fails to load, every
-operator of this package raises.
+There is no fallback: if either is missing or fails to load, every operator of this package raises.
 """
 from __future__ import annotations
 
@@ -14,7 +14,7 @@ from pathlib import Path
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libcastle_b200.so"
-SOURCES = ["api.cu", "decode.cu", "selftest.cu", "convert.cu", "fwd.cu", "bwd.cu", "bwd128.cu"]
+SOURCES = ["api.cu", "decode.cu", "selftest.cu", "convert.cu", "transform.cu", "fwd.cu", "bwd.cu", "bwd128.cu"]
 
 BF16, F16, F32 = 0, 1, 2
 
@@ -27,6 +27,11 @@ class CastleTensor(ctypes.Structure):
 class CastleProblem(ctypes.Structure):
     _fields_ = [("batch", ctypes.c_int32), ("heads", ctypes.c_int32), ("seq_len", ctypes.c_int32),
                 ("dim_head", ctypes.c_int32), ("dtype", ctypes.c_int32), ("scale", ctypes.c_float)]
+
+
+class CastleRotary(ctypes.Structure):
+    _fields_ = [("freqs", ctypes.c_void_p), ("dtype", ctypes.c_int32), ("inverse", ctypes.c_int32),
+                ("position0", ctypes.c_int64)]
 
 
 def _nvcc():
@@ -43,6 +48,9 @@ def _sources():
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-shared",
               "-Xcompiler", "-fPIC"]
 STAMP_PATH = PKG_DIR / "libcastle_b200.so.stamp"
+HOST_PATH = PKG_DIR / "_host.so"
+HOST_STAMP_PATH = PKG_DIR / "_host.so.stamp"
+HOST_SOURCE = CSRC / "host.cpp"
 
 
 def _deps():
@@ -67,6 +75,35 @@ def needs_build():
     return STAMP_PATH.read_text().strip() != _source_hash()
 
 
+def _host_command(out):
+    import sysconfig
+    import torch
+    inc, lib = Path(torch.__file__).parent / "include", Path(torch.__file__).parent / "lib"
+    nvcc = Path(_nvcc()).resolve()
+    cxx = os.environ.get("CXX") or shutil.which("g++") or "g++"
+    return [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f"-I{inc}", f"-I{inc / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{sysconfig.get_paths()['include']}",
+            f"-I{nvcc.parent.parent / 'include'}", str(HOST_SOURCE), "-o", str(out), f"-L{lib}", "-ltorch_python", "-ltorch",
+            "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+
+
+def _host_hash() -> str:
+    import hashlib
+    import sys
+    import torch
+    h = hashlib.sha256(f"{torch.__version__} {sys.version}".encode())
+    for d in (HOST_SOURCE, PKG_DIR.parent / "include" / "castle_b200.h"):
+        h.update(d.read_bytes())
+    return h.hexdigest()
+
+
+def needs_host_build():
+    if not HOST_PATH.exists() or not HOST_STAMP_PATH.exists():
+        return True
+    return HOST_STAMP_PATH.read_text().strip() != _host_hash()
+
+
 def _locked(fn):
     """Run `fn` holding the build lock (one builder per tree; ranks that start together queue here)."""
     import fcntl
@@ -78,32 +115,45 @@ def _locked(fn):
             fcntl.flock(lock, fcntl.LOCK_UN)
 
 
-def _build_unlocked(verbose: bool = False):
-    tmp = LIB_PATH.with_name(f".libcastle_b200.{os.getpid()}.tmp.so")
-    cmd = [_nvcc()] + NVCC_FLAGS + ["-Xptxas", "-v" if verbose else "-warn-spills", "-o", str(tmp)] + \
-          [str(s) for s in _sources()]
-    digest = _source_hash()
-    try:
-        res = subprocess.run(cmd, capture_output=True, text=True)
-        if res.returncode != 0:
-            raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-        os.replace(tmp, LIB_PATH)          # readers see the old library or the complete new one, never half of it
-        STAMP_PATH.write_text(digest + "\n")
-    finally:
-        if tmp.exists():
-            tmp.unlink()
-    if verbose:
-        print(res.stderr)
-    return LIB_PATH
+def _compile(jobs, verbose: bool = False):
+    """Run the compilers of `jobs` (target, stamp, digest, command for an output path) side by side; readers see
+    each old file or the complete new one, never half of it."""
+    running = []
+    for target, stamp, digest, command in jobs:
+        tmp = target.with_name(f".{target.stem}.{os.getpid()}.tmp.so")
+        running.append((target, stamp, digest, tmp, subprocess.Popen(command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    failed = []
+    for target, stamp, digest, tmp, proc in running:
+        text = proc.communicate()[0]
+        if proc.returncode == 0:
+            os.replace(tmp, target)
+            stamp.write_text(digest + "\n")
+        else:
+            failed.append(f"building {target.name} failed:\n{text}")
+            if tmp.exists():
+                tmp.unlink()
+        if verbose:
+            print(text)
+    if failed:
+        raise RuntimeError("\n".join(failed))
+
+
+def _build_unlocked(force: bool = False, verbose: bool = False):
+    def nvcc(out):
+        return [_nvcc()] + NVCC_FLAGS + ["-t", "0", "-Xptxas", "-v" if verbose else "-warn-spills", "-o", str(out)] + \
+               [str(s) for s in _sources()]
+    jobs = []
+    if force or needs_build():
+        jobs.append((LIB_PATH, STAMP_PATH, _source_hash(), nvcc))
+    if force or needs_host_build():
+        jobs.append((HOST_PATH, HOST_STAMP_PATH, _host_hash(), _host_command))
+    _compile(jobs, verbose)
 
 
 def build(force: bool = False, verbose: bool = False):
-    """Compile every kernel for sm_100a into one shared library next to this file."""
-    def go():
-        if not force and not needs_build():
-            return LIB_PATH
-        return _build_unlocked(verbose)
-    return _locked(go)
+    """Compile every kernel for sm_100a into one shared library next to this file, and the host module."""
+    _locked(lambda: _build_unlocked(force, verbose))
+    return LIB_PATH
 
 
 _lib = None
@@ -119,16 +169,31 @@ _SIGNATURES = {
     "castle_fwd": (ctypes.c_int, [_PR] + [_T] * 7 + [_vp, _T, _i32, _vp, _vp, _sz, _vp, _vp]),
     "castle_fwd_prefill": (ctypes.c_int, [_PR] + [_T] * 7 + [_vp] + [_T] * 4 + [_vp, _vp, _sz, _vp, _vp]),
     "castle_convert_16bit": (ctypes.c_int, [_i32, _vp, _vp, ctypes.c_int64, _vp, _vp]),
+    "castle_transform": (ctypes.c_int, [_PR, _i32, _T, _T, _i32, _i32, _T, P(CastleRotary), ctypes.c_uint32, _vp, _vp]),
+    "castle_amax_scale": (ctypes.c_int, [_i32, _vp, ctypes.c_int64, _vp, _vp, _vp]),
     "castle_bwd_workspace_bytes": (_sz, [_PR]),
     "castle_bwd": (ctypes.c_int, [_PR] + [_T] * 8 + [_vp, _vp] + [_T] * 6 + [_vp, _sz, _vp, _vp]),
     "castle_decode_workspace_bytes": (_sz, [_PR, _i32]),
     "castle_decode_step": (ctypes.c_int, [_PR, _i32, _i32] + [_T] * 11 + [_vp, _sz, _vp, _vp]),
+    "castle_decode_step_fused": (ctypes.c_int, [_PR, _i32, _i32] + [_T] * 11 + [P(CastleRotary), _vp, _vp, _sz, _vp, _vp]),
     "castle_decode_step_static": (ctypes.c_int, [_PR, _i32, _i32] + [_T] * 11 + [_vp, _vp]),
     "castle_set_kernel_events": (ctypes.c_int, [_i32, _vp, _vp]),
     "castle_selftest_mma_rate": (ctypes.c_int, [_i32, _i32, _i32, _vp, _vp, _vp]),
     "castle_selftest_mma": (ctypes.c_int, [_i32, _vp, _vp, _vp, _vp, _vp]),
     "castle_selftest_wait_timeout": (ctypes.c_int, [_i32, _vp, _vp, _vp]),
 }
+
+
+def _ensure_built():
+    """Compile on demand what is missing or was built from other sources; there is no other code path to fall back to."""
+    def go():
+        try:
+            _build_unlocked()
+        except Exception as e:
+            raise RuntimeError(f"{LIB_PATH.name} or {HOST_PATH.name} is missing or stale and could not be rebuilt ({e}); run "
+                               "`python -c 'import __graft_entry__ as g; g.build()'` where nvcc is "
+                               "available - this package has no fallback path") from e
+    _locked(go)
 
 
 def load():
@@ -140,17 +205,7 @@ def load():
     if override:
         return _bind(ctypes.CDLL(override))
 
-    def ensure():
-        # compile on demand when the library is missing or was built from other sources; there is
-        # no other code path to fall back to
-        if needs_build():
-            try:
-                _build_unlocked()
-            except Exception as e:
-                raise RuntimeError(f"{LIB_PATH} is missing or stale and could not be rebuilt ({e}); run "
-                                   "`python -c 'import __graft_entry__ as g; g.build()'` where nvcc is "
-                                   "available - this package has no fallback path") from e
-    _locked(ensure)
+    _ensure_built()
     return _bind(ctypes.CDLL(str(LIB_PATH)))
 
 
@@ -172,3 +227,19 @@ def last_error() -> str:
 def check(rc: int, what: str):
     if rc != 0:
         raise RuntimeError(f"{what} failed (rc={rc}): {last_error()}")
+
+
+_host = None
+
+
+def host():
+    """The native host module, bound to the library; raises if either cannot be built or loaded."""
+    global _host
+    if _host is None:
+        lib = load()
+        if os.environ.get("CASTLE_B200_LIB"):
+            _ensure_built()   # load() took the developer's library as it is
+        from . import _host as native
+        native.bind({name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _SIGNATURES})
+        _host = native
+    return _host

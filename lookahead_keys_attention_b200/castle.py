@@ -3,7 +3,8 @@
 arguments, state-dict keys (`to_all_qkv.weight`, `combine_heads.weight`,
 `norm.weight`), `forward(x, cache=None, return_next_cache=None)` conventions
 and `Cache` tuple.  The attention cores run as sm_100a kernels through the
-C-ABI library; the two projections and the optional RMSNorm stay torch ops.
+C-ABI library, rotary embedding included; the two projections and the optional
+RMSNorm stay torch ops, issued natively (csrc/host.cpp) together with the core.
 
 Difference from the reference, by design: the decode step appends to
 pre-allocated cache buffers and rewrites the lookahead keys `U` IN PLACE
@@ -21,8 +22,9 @@ from collections import namedtuple
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _has_any_global_hook
 
-from .ops import castle_attention, castle_attention_packed, castle_decode_step, prefill_writes_caches
+from . import _lib, ops
 
 Cache = namedtuple("Cache", ("U", "qu_cache", "kc_cache", "vc_cache"))
 
@@ -42,7 +44,7 @@ class _CacheBuffers:
         return self.bufs[0].shape[2]
 
     def views(self, n):
-        return [b[:, :, :n] for b in self.bufs]
+        return _lib.host().first_rows(self.bufs, n)
 
 
 class ModuleCache(Cache):
@@ -53,7 +55,7 @@ class ModuleCache(Cache):
     input and copied into fresh buffers first, so the caller's memory is never written."""
 
     def __new__(cls, state: _CacheBuffers, length: int):
-        self = super().__new__(cls, *state.views(length))
+        self = tuple.__new__(cls, state.views(length))
         self._state, self._length = state, int(length)
         return self
 
@@ -76,7 +78,8 @@ def cache_from_buffers(U, qu_cache, kc_cache, vc_cache, length: int) -> ModuleCa
 
 class _Rotary(nn.Module):
     """This package's own rotary embedding (pairs of adjacent channels rotated by
-    position * theta^(-2i/d)).  The reference delegates to the third-party
+    position * theta^(-2i/d)).  The module's passes apply it inside their kernels (csrc/rotary.cuh),
+    with the rounding points of `rotate`, which states it in torch operations.  The reference delegates to the third-party
     `rotary_embedding_torch` package, which is not available to compare against;
     numerical agreement with that package is not claimed."""
 
@@ -119,75 +122,96 @@ class Castle(nn.Module):
         cap = rows + max(self.cache_headroom, rows // 4)
         return _CacheBuffers([torch.empty(b, h, cap, d, dtype=dtype, device=device) for _ in range(4)], 0)
 
+    def _state_in_place(self, cache, t):
+        """The capacity buffers behind `cache` if row t can be appended to them as they are, else None."""
+        state = getattr(cache, "_state", None) if isinstance(cache, ModuleCache) else None
+        if state is None or cache._length != t:
+            return None
+        if not cache.is_current() and self.inplace_cache:
+            raise RuntimeError(
+                "this cache was advanced in place by a later decode step and no longer holds its rows; "
+                "construct Castle(..., inplace_cache=False) to decode from one cache more than once")
+        return state if self.inplace_cache and t < state.capacity else None
+
     def _buffers_for_step(self, cache, t, like) -> _CacheBuffers:
         """Capacity buffers holding rows [0, t) of `cache` with room for row t."""
-        b, h, _, d = like.shape
-        state = getattr(cache, "_state", None) if isinstance(cache, ModuleCache) else None
-        if state is not None and cache._length == t:
-            if not cache.is_current() and self.inplace_cache:
-                raise RuntimeError(
-                    "this cache was advanced in place by a later decode step and no longer holds its rows; "
-                    "construct Castle(..., inplace_cache=False) to decode from one cache more than once")
-            if self.inplace_cache and t < state.capacity:
-                return state
+        state = self._state_in_place(cache, t)
+        if state is not None:
+            return state
         # a foreign cache, a full buffer, or functional semantics asked for: copy into fresh buffers
+        b, h, _, d = like.shape
         fresh = self._new_buffers(b, h, d, t + 1, like.dtype, like.device)
         if t > 0:
-            for buf, src in zip(fresh.bufs, cache):
-                buf[:, :, :t].copy_(src)
+            with torch.no_grad():
+                for buf, src in zip(fresh.bufs, cache):
+                    buf[:, :, :t].copy_(src)
         fresh.length = t
         return fresh
 
+    def _plain_layer(self):
+        """What the native path takes of this layer: norm weight and eps, the two projection weights and the head
+        sizes; or None where a submodule was replaced, has a bias or has hooks, so that it must be called as a module."""
+        mods = self._modules
+        norm, qkv, combine = mods["norm"], mods["to_all_qkv"], mods["combine_heads"]
+        if type(qkv) is not nn.Linear or type(combine) is not nn.Linear or _has_any_global_hook():
+            return None
+        for m in (norm, qkv, combine):
+            if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks:
+                return None
+        wq, wc = qkv._parameters, combine._parameters
+        if wq["bias"] is not None or wc["bias"] is not None:
+            return None
+        if type(norm) is nn.Identity:
+            return None, None, wq["weight"], wc["weight"], self.heads, self.dim_head
+        if type(norm) is nn.RMSNorm and norm._parameters["weight"] is not None and len(norm.normalized_shape) == 1:
+            return norm._parameters["weight"], norm.eps, wq["weight"], wc["weight"], self.heads, self.dim_head
+        return None
+
+    def _project(self, x):
+        """The packed projection (b, n, 6, heads, dim_head) with the submodules called as modules."""
+        return self.to_all_qkv(self.norm(x)).view(x.shape[0], x.shape[1], 6, self.heads, self.dim_head)
+
     def forward(self, x, cache: Cache | None = None, return_next_cache=None):
+        host = _lib.host()
         seq_len = x.shape[1]
         is_inference = seq_len == 1
         if return_next_cache is None:
             return_next_cache = is_inference
-        x = self.norm(x)
-        qkvs = self.to_all_qkv(x)
-        qu, ku, vu, qc, kc, vc = self._split(qkvs)
-        if self.rotary_emb is not None:
-            offset = cache.kc_cache.shape[-2] if cache is not None else 0
-            qc, kc, qu, ku, vu = (self.rotary_emb.rotate(t, offset) for t in (qc, kc, qu, ku, vu))
+        layer = self._plain_layer()
+        rotary = self.rotary_emb
+        freqs = None if rotary is None else rotary._buffers["freqs"]
 
-        if not is_inference:
-            assert cache is None, "must be inferencing single tokens if receiving cache"
-            packed = None
-            if self.rotary_emb is None:  # the kernels read the projection output in place
-                packed = qkvs.view(x.shape[0], seq_len, 6, self.heads, self.dim_head)
-            if return_next_cache:
-                # the cache lives in buffers with spare rows so that decode steps can append in place
-                b, h, _, d = qu.shape
-                state = self._new_buffers(b, h, d, seq_len, qu.dtype, qu.device)
-                # 16-bit modules: the forward kernels write all four caches themselves (U from the final
-                # lookahead state, qu/kc/vc from the tiles they hold in shared memory)
-                fill = prefill_writes_caches(qu.dtype, d, seq_len)
-                cache_out = tuple(state.views(seq_len)) if fill else None
-                if packed is not None:
-                    out, U = castle_attention_packed(packed, self.scale, True, cache_out)
-                else:
-                    out, U = castle_attention(qc, kc, vc, qu, ku, vu, self.scale, True, cache_out)
-                if not fill:   # fp32 modules (the kernels run on fp16 copies) and odd head widths
-                    with torch.no_grad():
-                        for buf, src in zip(state.bufs, (U, qu, kc, vc)):
-                            buf[:, :, :seq_len].copy_(src)
-                state.length = seq_len
-                next_cache = ModuleCache(state, seq_len)
-            elif packed is not None:
-                out = castle_attention_packed(packed, self.scale, False)
+        if is_inference:
+            t = 0 if cache is None else cache._length if isinstance(cache, ModuleCache) else cache[0].shape[-2]
+            state = self._state_in_place(cache, t)
+            if layer is not None and state is not None:
+                out = host.layer_decode(x, *layer, self.scale, freqs, state.bufs, t)
             else:
-                out = castle_attention(qc, kc, vc, qu, ku, vu, self.scale, False)
-        else:
-            t = 0 if cache is None else cache[0].shape[-2]
-            with torch.no_grad():
-                state = self._buffers_for_step(cache, t, qu)
-                out = castle_decode_step(qc, kc, vc, qu, ku, vu, *state.bufs, t, self.scale)
+                packed = self._project(x)
+                if state is None:
+                    state = self._buffers_for_step(cache, t, packed[:, :, 0].transpose(1, 2))
+                out = self.combine_heads(host.decode_packed(packed, self.scale, freqs, state.bufs, t))
             state.length = t + 1
-            next_cache = ModuleCache(state, t + 1)
+            return (out, ModuleCache(state, t + 1)) if return_next_cache else out
 
-        b, h, n, d = out.shape
-        out = out.permute(0, 2, 1, 3).reshape(b, n, h * d)  # 'b h n d -> b n (h d)'
-        out = self.combine_heads(out)
+        assert cache is None, "must be inferencing single tokens if receiving cache"
+        limits = (ops.MAX_WORKSPACE_BYTES, ops.LONG_SEQ_FP16)
+        native = layer is not None and not torch.is_autocast_enabled("cuda")   # under autocast only the projection knows the type
+        packed = None if native else self._project(x)
+        state = views = None
+        if return_next_cache:
+            # The cache lives in buffers with spare rows so that decode steps can append in place.  The forward's
+            # kernels fill it themselves: from their operand tiles where those are the caller's values, otherwise
+            # in the pass that makes the operands.
+            like = x if native else packed
+            state = self._new_buffers(x.shape[0], self.heads, self.dim_head, seq_len, like.dtype, like.device)
+            views = state.views(seq_len)
+        if native:
+            out = host.layer_forward(x, *layer, self.scale, freqs, views, *limits)
+        else:
+            out = host.attention_packed(packed, self.scale, False, views, *limits, freqs, False)
+            out = self.combine_heads(out.permute(0, 2, 1, 3).reshape(*x.shape[:2], -1))   # 'b h n d -> b n (h d)'
         if not return_next_cache:
             return out
-        return out, next_cache
+        state.length = seq_len
+        return out, ModuleCache(state, seq_len)

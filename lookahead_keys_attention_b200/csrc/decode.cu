@@ -11,6 +11,7 @@
 // kernel merges.
 #include <mutex>
 #include "common.cuh"
+#include "rotary.cuh"
 #include "sm100.cuh"
 
 namespace castle {
@@ -23,6 +24,8 @@ struct DecodeParams {
   int H, t, nsplit, rows_per_split;
   float scale;
   int32_t* status;
+  RotaryParams rot;                                // rotation of the new rows (all but vc); freqs null = none
+  uint32_t* counters;                              // [BH] zeroed: CTAs of a pair that are done; null = merge kernel
 };
 
 template <typename T> struct Vec;  // 16 bytes of T <-> floats
@@ -68,6 +71,19 @@ __device__ __forceinline__ float group_sum(float v) {
   return v;
 }
 
+// The new token's rows are rotated as they are loaded: VEC adjacent elements of a row from column `col`.
+template <typename T>
+__device__ __forceinline__ void rotate_new(const RotaryParams& r, int64_t col, float* a, float* b, float* c) {
+  if (r.freqs == nullptr) return;
+#pragma unroll
+  for (int i = 0; i < Vec<T>::N; i += 2) {
+    const float2 cs = rotary_cos_sin(r, 0, (int)(col + i) / 2);
+    rotate_pair<T>(a[i], a[i + 1], cs);
+    rotate_pair<T>(b[i], b[i + 1], cs);
+    if (c) rotate_pair<T>(c[i], c[i + 1], cs);
+  }
+}
+
 #ifndef CASTLE_DECODE_THREADS
 #define CASTLE_DECODE_THREADS 128
 #endif
@@ -79,6 +95,114 @@ __device__ __forceinline__ float group_sum(float v) {
 #endif
 constexpr int kDecodeThreads = CASTLE_DECODE_THREADS;
 constexpr int kDecodeUnroll = CASTLE_DECODE_UNROLL;
+constexpr int kMaxSplits = 64;   // CTAs that share the rows of one (batch, head) pair
+static_assert(kDecodeThreads == 128, "decode_merge maps 128 threads to the columns of a head");
+
+template <typename T, int D>
+__device__ __forceinline__ void decode_store_out(const DecodeParams& p, int bh, int c, float v) {
+  T* o = reinterpret_cast<T*>(p.out.ptr) + (bh / p.H) * p.out.stride_b + (bh % p.H) * p.out.stride_h;
+  if constexpr (sizeof(T) == 4) o[c] = v;
+  else o[c] = Elem<T>::from_f(v);
+}
+
+// Merge the partials of one (batch, head) pair, by a whole CTA of kDecodeThreads: the weights of the parts once
+// per CTA into shared memory, then D columns x (threads / D) groups of parts, eight loads of a thread in flight.
+template <typename T, int D>
+__device__ __forceinline__ void decode_merge(const DecodeParams& p, int bh) {
+  constexpr int G = kDecodeThreads / D;
+  __shared__ float s_w[kMaxSplits], s_sum[G][D];
+  const int nsplit = p.nsplit;
+  const float* src = p.part + (int64_t)bh * nsplit * (2 + D);
+  const int lane = threadIdx.x & 31;
+  // every warp finds the maximum and the sum over the (at most 64) parts by itself
+  const float m0 = lane < nsplit ? __ldcg(src + lane * (2 + D)) : -INFINITY;
+  const float m1 = lane + 32 < nsplit ? __ldcg(src + (lane + 32) * (2 + D)) : -INFINITY;
+  const float l0 = lane < nsplit ? __ldcg(src + lane * (2 + D) + 1) : 0.f;
+  const float l1 = lane + 32 < nsplit ? __ldcg(src + (lane + 32) * (2 + D) + 1) : 0.f;
+  float mm = fmaxf(m0, m1);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+  const float w0 = m0 == -INFINITY ? 0.f : __expf(m0 - mm), w1 = m1 == -INFINITY ? 0.f : __expf(m1 - mm);
+  float ll = l0 * w0 + l1 * w1;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xffffffffu, ll, o);
+  if (threadIdx.x < 32) { s_w[lane] = w0; s_w[lane + 32] = w1; }
+  __syncthreads();
+  const int c = threadIdx.x % D, g = threadIdx.x / D;
+  float a = 0.f;
+#pragma unroll 8
+  for (int s = g; s < nsplit; s += G) a += __ldcg(src + s * (2 + D) + 2 + c) * s_w[s];
+  if constexpr (G > 1) {
+    s_sum[g][c] = a;
+    __syncthreads();
+    if (g == 0) {
+#pragma unroll
+      for (int k = 1; k < G; ++k) a += s_sum[k][c];
+    }
+  }
+  if (g == 0) decode_store_out<T, D>(p, bh, c, a / ll);
+}
+
+// End of both step kernels: merge the lane groups of a warp, then the warps of the CTA.  A pair whose rows were split
+// leaves a partial; the CTA that leaves a pair's last one (p.counters) merges them, which saves the merge kernel's
+// launch and its wait for the whole grid (3 to 8 us a step).
+template <typename T, int D>
+__device__ __forceinline__ void decode_finish(const DecodeParams& p, int bh, int split, float m, float l, float* acc) {
+  constexpr int VEC = Vec<T>::N, LPR = D / VEC, NW = kDecodeThreads / 32;
+  __shared__ float s_m[NW], s_l[NW], s_acc[NW][D];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int sub = lane % LPR, grp = lane / LPR;
+#pragma unroll
+  for (int o = LPR; o < 32; o <<= 1) {
+    const float m2 = __shfl_xor_sync(0xffffffffu, m, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
+    const float mn = fmaxf(m, m2);
+    const float c1 = (m == -INFINITY) ? 0.f : __expf(m - mn), c2 = (m2 == -INFINITY) ? 0.f : __expf(m2 - mn);
+    l = l * c1 + l2 * c2;
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+      const float a2 = __shfl_xor_sync(0xffffffffu, acc[i], o);
+      acc[i] = acc[i] * c1 + a2 * c2;
+    }
+    m = mn;
+  }
+  if (grp == 0) {
+    if (sub == 0) { s_m[warp] = m; s_l[warp] = l; }
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) s_acc[warp][sub * VEC + i] = acc[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < D) {
+    float mm = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) mm = fmaxf(mm, s_m[w]);
+    float ll = 0.f, aa = 0.f;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      const float c = (s_m[w] == -INFINITY) ? 0.f : __expf(s_m[w] - mm);
+      ll += s_l[w] * c;
+      aa += s_acc[w][threadIdx.x] * c;
+    }
+    if (p.nsplit == 1) {
+      decode_store_out<T, D>(p, bh, threadIdx.x, aa / ll);
+    } else {
+      float* dst = p.part + ((int64_t)bh * p.nsplit + split) * (2 + D);
+      if (threadIdx.x == 0) { dst[0] = mm; dst[1] = ll; }
+      dst[2 + threadIdx.x] = aa;
+    }
+  }
+  if (p.nsplit == 1 || p.counters == nullptr) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(p.counters + bh, 1u) == (uint32_t)p.nsplit - 1;
+    if (s_last) p.counters[bh] = 0;   // ready for the next launch
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  decode_merge<T, D>(p, bh);
+}
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kDecodeThreads, CASTLE_DECODE_MIN_CTAS) castle_decode_kernel(const DecodeParams p) {
@@ -100,6 +224,7 @@ __global__ void __launch_bounds__(kDecodeThreads, CASTLE_DECODE_MIN_CTAS) castle
   Vec<T>::load(row_ptr(p.qc, 0), qcv);
   Vec<T>::load(row_ptr(p.ku, 0), kuv);
   Vec<T>::load(row_ptr(p.vu, 0), vuv);
+  rotate_new<T>(p.rot, col, qcv, kuv, vuv);
 #pragma unroll
   for (int i = 0; i < VEC; ++i) { qcv[i] *= p.scale; kuv[i] *= p.scale; }  // scale*(qu.ku) == qu.(scale*ku)
 
@@ -164,6 +289,7 @@ __global__ void __launch_bounds__(kDecodeThreads, CASTLE_DECODE_MIN_CTAS) castle
     Vec<T>::load(row_ptr(p.kc, 0), kn);
     Vec<T>::load(row_ptr(p.vc, 0), vn);
     Vec<T>::load(row_ptr(p.qu, 0), qn);
+    rotate_new<T>(p.rot, col, kn, qn, nullptr);
 #pragma unroll
     for (int i = 0; i < VEC; ++i) zero[i] = 0.f;
     if (grp == 0) {
@@ -186,48 +312,7 @@ __global__ void __launch_bounds__(kDecodeThreads, CASTLE_DECODE_MIN_CTAS) castle
     }
   }
 
-  // merge the RPW lane groups of a warp, then the warps of the CTA
-#pragma unroll
-  for (int o = LPR; o < 32; o <<= 1) {
-    float m2 = __shfl_xor_sync(0xffffffffu, m, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
-    float mn = fmaxf(m, m2);
-    float c1 = (m == -INFINITY) ? 0.f : __expf(m - mn), c2 = (m2 == -INFINITY) ? 0.f : __expf(m2 - mn);
-    l = l * c1 + l2 * c2;
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      float a2 = __shfl_xor_sync(0xffffffffu, acc[i], o);
-      acc[i] = acc[i] * c1 + a2 * c2;
-    }
-    m = mn;
-  }
-  __shared__ float s_m[NW], s_l[NW], s_acc[NW][D];
-  if (grp == 0) {
-    if (sub == 0) { s_m[warp] = m; s_l[warp] = l; }
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) s_acc[warp][sub * VEC + i] = acc[i];
-  }
-  __syncthreads();
-  if (threadIdx.x < D) {
-    float mm = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) mm = fmaxf(mm, s_m[w]);
-    float ll = 0.f, aa = 0.f;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      float c = (s_m[w] == -INFINITY) ? 0.f : __expf(s_m[w] - mm);
-      ll += s_l[w] * c;
-      aa += s_acc[w][threadIdx.x] * c;
-    }
-    if (p.nsplit == 1) {
-      T* o = reinterpret_cast<T*>(p.out.ptr) + b * p.out.stride_b + h * p.out.stride_h;
-      if constexpr (sizeof(T) == 4) o[threadIdx.x] = aa / ll;
-      else o[threadIdx.x] = Elem<T>::from_f(aa / ll);
-    } else {
-      float* dst = p.part + ((int64_t)bh * p.nsplit + split) * (2 + D);
-      if (threadIdx.x == 0) { dst[0] = mm; dst[1] = ll; }
-      dst[2 + threadIdx.x] = aa;
-    }
-  }
+  decode_finish<T, D>(p, bh, split, m, l, acc);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -237,8 +322,9 @@ __global__ void __launch_bounds__(kDecodeThreads, CASTLE_DECODE_MIN_CTAS) castle
 // per stage, four contiguous copies (the rows of a tile are adjacent in each cache, which is why
 // this variant needs position stride == dim_head); the warps consume a stage row group by row
 // group, write U back from registers, and the stage is refilled after a block-wide barrier.
-constexpr int kRingRows = 16;     // rows per stage
 constexpr int kRingStages = 3;
+// Rows per stage: 4 KB of each cache (fewer and larger copies for narrow heads), at least 16.
+template <typename T, int D> struct RingRows { static constexpr int fit = 4096 / (D * (int)sizeof(T)), value = fit > 16 ? fit : 16; };
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
@@ -252,13 +338,13 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) castle_decode_ring_kernel(c
   constexpr int LPR = D / VEC;
   constexpr int RPW = 32 / LPR;
   constexpr int NW = kDecodeThreads / 32;
+  constexpr int kRingRows = RingRows<T, D>::value;
   constexpr int PASSES = (kRingRows + RPW * NW - 1) / (RPW * NW);
   constexpr uint32_t ROWB = D * sizeof(T);
   constexpr uint32_t TENB = kRingRows * ROWB;            // one tensor's tile
   extern __shared__ __align__(128) uint8_t ring[];       // [stage][tensor: qu, U, kc, vc][row][D]
   __shared__ uint64_t full[kRingStages];
   __shared__ int abort_flag;
-  __shared__ float s_m[NW], s_l[NW], s_acc[NW][D];
 
   const int bh = blockIdx.x, split = blockIdx.y;
   const int b = bh / p.H, h = bh % p.H;
@@ -299,6 +385,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) castle_decode_ring_kernel(c
   Vec<T>::load(row_ptr(p.qc, 0), qcv);
   Vec<T>::load(row_ptr(p.ku, 0), kuv);
   Vec<T>::load(row_ptr(p.vu, 0), vuv);
+  rotate_new<T>(p.rot, col, qcv, kuv, vuv);
 #pragma unroll
   for (int i = 0; i < VEC; ++i) { qcv[i] *= p.scale; kuv[i] *= p.scale; }
 
@@ -365,6 +452,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) castle_decode_ring_kernel(c
     Vec<T>::load(row_ptr(p.kc, 0), kn);
     Vec<T>::load(row_ptr(p.vc, 0), vn);
     Vec<T>::load(row_ptr(p.qu, 0), qn);
+    rotate_new<T>(p.rot, col, kn, qn, nullptr);
 #pragma unroll
     for (int i = 0; i < VEC; ++i) zero[i] = 0.f;
     if (grp == 0 && *abortp == 0) {   // a timed-out step leaves the caches as they were
@@ -387,66 +475,13 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) castle_decode_ring_kernel(c
     }
   }
 
-  // merge the lane groups of a warp, then the warps of the CTA
-#pragma unroll
-  for (int o = LPR; o < 32; o <<= 1) {
-    const float m2 = __shfl_xor_sync(0xffffffffu, m, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
-    const float mn = fmaxf(m, m2);
-    const float c1 = (m == -INFINITY) ? 0.f : __expf(m - mn), c2 = (m2 == -INFINITY) ? 0.f : __expf(m2 - mn);
-    l = l * c1 + l2 * c2;
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      const float a2 = __shfl_xor_sync(0xffffffffu, acc[i], o);
-      acc[i] = acc[i] * c1 + a2 * c2;
-    }
-    m = mn;
-  }
-  if (grp == 0) {
-    if (sub == 0) { s_m[warp] = m; s_l[warp] = l; }
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) s_acc[warp][sub * VEC + i] = acc[i];
-  }
-  __syncthreads();
-  if (threadIdx.x < D) {
-    float mm = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) mm = fmaxf(mm, s_m[w]);
-    float ll = 0.f, aa = 0.f;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      const float c = (s_m[w] == -INFINITY) ? 0.f : __expf(s_m[w] - mm);
-      ll += s_l[w] * c;
-      aa += s_acc[w][threadIdx.x] * c;
-    }
-    if (p.nsplit == 1) {
-      T* o = reinterpret_cast<T*>(p.out.ptr) + b * p.out.stride_b + h * p.out.stride_h;
-      if constexpr (sizeof(T) == 4) o[threadIdx.x] = aa / ll;
-      else o[threadIdx.x] = Elem<T>::from_f(aa / ll);
-    } else {
-      float* dst = p.part + ((int64_t)bh * p.nsplit + split) * (2 + D);
-      if (threadIdx.x == 0) { dst[0] = mm; dst[1] = ll; }
-      dst[2 + threadIdx.x] = aa;
-    }
-  }
+  decode_finish<T, D>(p, bh, split, m, l, acc);
   if (threadIdx.x == 0 && abort_flag) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
 }
 
 template <typename T, int D>
-__global__ void castle_decode_merge_kernel(const DecodeParams p) {
-  const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H, c = threadIdx.x;
-  const float* src = p.part + (int64_t)bh * p.nsplit * (2 + D);
-  float mm = -INFINITY;
-  for (int s = 0; s < p.nsplit; ++s) mm = fmaxf(mm, src[s * (2 + D)]);
-  float ll = 0.f, aa = 0.f;
-  for (int s = 0; s < p.nsplit; ++s) {
-    float ms = src[s * (2 + D)];
-    float w = (ms == -INFINITY) ? 0.f : __expf(ms - mm);
-    ll += src[s * (2 + D) + 1] * w;
-    aa += src[s * (2 + D) + 2 + c] * w;
-  }
-  T* o = reinterpret_cast<T*>(p.out.ptr) + b * p.out.stride_b + h * p.out.stride_h;
-  if constexpr (sizeof(T) == 4) o[c] = aa / ll;
-  else o[c] = Elem<T>::from_f(aa / ll);
+__global__ void __launch_bounds__(kDecodeThreads) castle_decode_merge_kernel(const DecodeParams p) {
+  decode_merge<T, D>(p, blockIdx.x);
 }
 
 // How many CTAs share the rows of one (batch, head) pair.  The kernel is bandwidth bound and runs
@@ -480,9 +515,20 @@ static int decode_nsplit(int BH, int t, int ctas_per_sm = CASTLE_DECODE_MIN_CTAS
 
 constexpr int kRingCtasPerSm = 4;
 
-// The bulk-copy variant needs rows that are adjacent in memory and at least 128 bytes long.
-static bool decode_use_ring(int D, int dtype, const castle_tensor_t* const* caches) {
-  if (kDecodeThreads != 128 || D * elem_size(dtype) < 128) return false;
+// The same for steps that leave SMs idle at 128 rows per CTA (few pairs, short caches): there a CTA's serial walk over
+// its rows is the time, so the rows are cut as fine as two ring stages (32 rows) while the grid stays within one wave.
+static int decode_nsplit_fine(int BH, int t, int ctas_per_sm) {
+  const int best = decode_nsplit(BH, t, ctas_per_sm);
+  const int64_t slots = 148 * ctas_per_sm;
+  if ((int64_t)BH * best >= slots) return best;
+  int ns = (t + 31) / 32;
+  if (ns > slots / BH) ns = (int)(slots / BH);
+  if (ns > kMaxSplits) ns = kMaxSplits;
+  return ns > best ? ns : best;
+}
+
+// The bulk-copy variant needs rows that are adjacent in memory.
+static bool decode_use_ring(int D, const castle_tensor_t* const* caches) {
   for (int i = 0; i < 4; ++i)
     if (caches[i]->stride_n != D) return false;
   return true;
@@ -491,23 +537,21 @@ static bool decode_use_ring(int D, int dtype, const castle_tensor_t* const* cach
 template <typename T, int D>
 static int launch_decode(const DecodeParams& p, int BH, bool ring, cudaStream_t st) {
   dim3 grid(BH, p.nsplit);
-  if constexpr (D * sizeof(T) >= 128) {
-    if (ring) {
-      constexpr size_t smem = (size_t)kRingStages * 4 * kRingRows * D * sizeof(T);
-      cudaError_t e = cudaFuncSetAttribute(castle_decode_ring_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return cuda_fail(e, "castle_decode_step attribute");
-      ev_start(CASTLE_KERNEL_DECODE, st);
-      castle_decode_ring_kernel<T, D><<<grid, kDecodeThreads, smem, st>>>(p);
-      ev_stop(CASTLE_KERNEL_DECODE, st);
-      if (p.nsplit > 1) castle_decode_merge_kernel<T, D><<<BH, D, 0, st>>>(p);
-      e = cudaGetLastError();
-      return e == cudaSuccess ? 0 : cuda_fail(e, "castle_decode_step launch");
-    }
+  if (ring) {
+    constexpr size_t smem = (size_t)kRingStages * 4 * RingRows<T, D>::value * D * sizeof(T);
+    cudaError_t e = cudaFuncSetAttribute(castle_decode_ring_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_fail(e, "castle_decode_step attribute");
+    ev_start(CASTLE_KERNEL_DECODE, st);
+    castle_decode_ring_kernel<T, D><<<grid, kDecodeThreads, smem, st>>>(p);
+    ev_stop(CASTLE_KERNEL_DECODE, st);
+    if (p.nsplit > 1 && !p.counters) castle_decode_merge_kernel<T, D><<<BH, kDecodeThreads, 0, st>>>(p);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : cuda_fail(e, "castle_decode_step launch");
   }
   ev_start(CASTLE_KERNEL_DECODE, st);
   castle_decode_kernel<T, D><<<grid, kDecodeThreads, 0, st>>>(p);
   ev_stop(CASTLE_KERNEL_DECODE, st);
-  if (p.nsplit > 1) castle_decode_merge_kernel<T, D><<<BH, D, 0, st>>>(p);
+  if (p.nsplit > 1 && !p.counters) castle_decode_merge_kernel<T, D><<<BH, kDecodeThreads, 0, st>>>(p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_decode_step launch");
 }
@@ -530,7 +574,7 @@ using namespace castle;
 extern "C" size_t castle_decode_workspace_bytes(const castle_problem_t* p, int32_t cache_len) {
   if (!p) return 0;
   int BH = p->batch * p->heads;
-  int ns = decode_nsplit(BH, cache_len), ns_ring = decode_nsplit(BH, cache_len, kRingCtasPerSm);
+  int ns = decode_nsplit_fine(BH, cache_len, CASTLE_DECODE_MIN_CTAS), ns_ring = decode_nsplit_fine(BH, cache_len, kRingCtasPerSm);
   return (size_t)BH * (ns > ns_ring ? ns : ns_ring) * (2 + p->dim_head) * sizeof(float);
 }
 
@@ -542,6 +586,18 @@ extern "C" int castle_decode_step(const castle_problem_t* p, int32_t cache_len, 
                                   const castle_tensor_t* kc_cache, const castle_tensor_t* vc_cache,
                                   const castle_tensor_t* out, void* workspace, size_t workspace_bytes,
                                   int32_t* status, void* stream) {
+  return castle_decode_step_fused(p, cache_len, capacity, qc_new, kc_new, vc_new, qu_new, ku_new, vu_new, u_cache, qu_cache,
+                                  kc_cache, vc_cache, out, nullptr, nullptr, workspace, workspace_bytes, status, stream);
+}
+
+extern "C" int castle_decode_step_fused(const castle_problem_t* p, int32_t cache_len, int32_t capacity,
+                                        const castle_tensor_t* qc_new, const castle_tensor_t* kc_new,
+                                        const castle_tensor_t* vc_new, const castle_tensor_t* qu_new,
+                                        const castle_tensor_t* ku_new, const castle_tensor_t* vu_new,
+                                        const castle_tensor_t* u_cache, const castle_tensor_t* qu_cache,
+                                        const castle_tensor_t* kc_cache, const castle_tensor_t* vc_cache,
+                                        const castle_tensor_t* out, const castle_rotary_t* rotary, uint32_t* counters,
+                                        void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
   if (!p) return reject("castle_decode_step: null problem");
   if (p->batch <= 0 || p->heads <= 0) return reject("castle_decode_step: empty batch/heads");
   if (cache_len < 0 || cache_len >= capacity)
@@ -559,11 +615,21 @@ extern "C" int castle_decode_step(const castle_problem_t* p, int32_t cache_len, 
   int BH = p->batch * p->heads;
   dp.H = p->heads; dp.t = cache_len; dp.scale = p->scale; dp.status = status;
   const castle_tensor_t* caches[4] = {u_cache, qu_cache, kc_cache, vc_cache};
-  const bool ring = status != nullptr && decode_use_ring(p->dim_head, p->dtype, caches);
-  dp.nsplit = decode_nsplit(BH, cache_len, ring ? kRingCtasPerSm : CASTLE_DECODE_MIN_CTAS);
+  const bool ring = status != nullptr && decode_use_ring(p->dim_head, caches);
+  dp.nsplit = decode_nsplit_fine(BH, cache_len, ring ? kRingCtasPerSm : CASTLE_DECODE_MIN_CTAS);
   dp.rows_per_split = (cache_len + dp.nsplit - 1) / dp.nsplit;
   if (dp.rows_per_split < 1) dp.rows_per_split = 1;
   dp.part = (float*)workspace;
+  // Merging in the step kernel costs every CTA a fence that waits for its U rows to land.  Within one wave of CTAs that
+  // is hidden by the launch it saves (8 pairs x 771 rows: 12.5 us -> 11 us, and one launch less on the host); over several
+  // waves it is not (128 pairs x 8191 rows, 8 waves: 231 us against 213 + 8 us with the merge kernel).
+  const int64_t slots = 148 * (ring ? kRingCtasPerSm : CASTLE_DECODE_MIN_CTAS);
+  dp.counters = (int64_t)BH * dp.nsplit <= slots ? counters : nullptr;
+  dp.rot = RotaryParams{nullptr, CASTLE_F32, 0, 0.f};
+  if (rotary && rotary->freqs) {
+    if (rotary->dtype < CASTLE_BF16 || rotary->dtype > CASTLE_F32) return reject("castle_decode_step: unknown rotary dtype");
+    dp.rot = RotaryParams{rotary->freqs, rotary->dtype, rotary->inverse, (float)rotary->position0};
+  }
   if (dp.nsplit > 1) {
     size_t need = (size_t)BH * dp.nsplit * (2 + p->dim_head) * sizeof(float);
     if (!workspace || workspace_bytes < need)
@@ -651,6 +717,8 @@ extern "C" int castle_decode_step_static(const castle_problem_t* p, int32_t cach
   // Every partial slot the merge kernel reads is written by this same call first, so the
   // array needs no clearing between calls even though it keeps the previous call's contents.
   dp.part = scratch;
+  dp.counters = nullptr;
+  dp.rot = RotaryParams{nullptr, CASTLE_F32, 0, 0.f};
   cudaStream_t st = (cudaStream_t)stream;
   switch (p->dtype) {
     case CASTLE_BF16: return launch_decode_d<__nv_bfloat16>(dp, BH, p->dim_head, false, st);

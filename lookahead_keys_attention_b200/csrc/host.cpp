@@ -1,0 +1,802 @@
+// Host side of the operators: everything between a Python call and the C ABI's launches, natively.
+//
+// A small call of this framework (a decode step, a short training step) spends its time on the host: building tensor
+// descriptors through ctypes, Python autograd functions and chains of small torch operations took 60 to 120 us per
+// call on the token path and 800 us for the smallest training step, against 10 to 150 us of kernels.  This module does
+// the same work in C++: descriptors, scratch, the autograd node, the choice of the passes around the kernels, and for
+// the plain `Castle` module the projections around the core as well.  It holds no kernels; the C ABI of
+// libcastle_b200.so is bound by address (`bind`).
+//
+// Operators and their semantics: ops.py and castle.py.
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/grad_mode.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <map>
+#include <memory>
+#include <mutex>
+#include <optional>
+#include <string>
+#include <vector>
+
+#include "../../include/castle_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+struct AssertError : std::runtime_error { using std::runtime_error::runtime_error; };   // raised as AssertionError
+
+// ------------------------------------------------------------------------------------------------ the C ABI, by address
+struct Api {
+  decltype(&castle_last_error) last_error;
+  decltype(&castle_fwd_workspace_bytes) fwd_workspace_bytes;
+  decltype(&castle_fwd) fwd;
+  decltype(&castle_fwd_prefill) fwd_prefill;
+  decltype(&castle_bwd_workspace_bytes) bwd_workspace_bytes;
+  decltype(&castle_bwd) bwd;
+  decltype(&castle_transform) transform;
+  decltype(&castle_amax_scale) amax_scale;
+  decltype(&castle_decode_workspace_bytes) decode_workspace_bytes;
+  decltype(&castle_decode_step_fused) decode_step_fused;
+} api{};
+
+void check(int rc, const char* what) {
+  if (rc != 0)
+    throw std::runtime_error(std::string(what) + " failed (rc=" + std::to_string(rc) + "): " + api.last_error());
+}
+
+void need(bool ok, const char* message) {
+  if (!ok) throw std::runtime_error(message);
+}
+
+// ------------------------------------------------------------------------------------------------ device state kept between calls
+// Scratch per (device, stream): kernels of one stream run in order, so its calls can share a buffer; two streams must
+// not.  Grown on demand, given back by release_workspaces().  `words` are zeroed counters that every kernel using them
+// leaves zeroed.  The containers are never destroyed (the CUDA context may be gone before static destructors run).
+struct StreamState { Tensor scratch, words; };
+std::mutex state_mutex;
+auto& stream_states = *new std::map<std::pair<int, void*>, StreamState>();
+auto& status_words = *new std::map<int, Tensor>();
+
+constexpr int64_t kAmaxWords = 4;   // words [0, 4): castle_amax_scale; then the decode step's counters
+
+Tensor scratch(const c10::cuda::CUDAStream& s, size_t bytes) {
+  std::lock_guard<std::mutex> lock(state_mutex);
+  Tensor& t = stream_states[{(int)s.device_index(), (void*)s.stream()}].scratch;
+  if (!t.defined() || (size_t)t.numel() < bytes) {
+    t = Tensor();   // give the old buffer back before asking for the larger one
+    t = at::empty({(int64_t)std::max<size_t>(bytes, (size_t)1 << 20)},
+                  at::TensorOptions().dtype(at::kByte).device(at::kCUDA, s.device_index()));
+  }
+  return t;
+}
+
+Tensor zero_words(const c10::cuda::CUDAStream& s, int64_t count) {
+  std::lock_guard<std::mutex> lock(state_mutex);
+  Tensor& t = stream_states[{(int)s.device_index(), (void*)s.stream()}].words;
+  if (!t.defined() || t.numel() < kAmaxWords + count)
+    t = at::zeros({kAmaxWords + std::max<int64_t>(count, 1020)}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, s.device_index()));
+  return t;
+}
+
+Tensor status_word(int device) {
+  std::lock_guard<std::mutex> lock(state_mutex);
+  Tensor& t = status_words[device];
+  if (!t.defined()) t = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+  return t;
+}
+
+// ------------------------------------------------------------------------------------------------ descriptors
+int dtype_code(at::ScalarType t) {
+  return t == at::kBFloat16 ? CASTLE_BF16 : t == at::kHalf ? CASTLE_F16 : t == at::kFloat ? CASTLE_F32 : -1;
+}
+
+castle_tensor_t desc(const Tensor& t) {   // (B, H, N, d), last dimension contiguous
+  return {t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)};
+}
+
+// The ABI's alignment rules: 16-byte base and strides.
+bool aligned(const Tensor& t) {
+  const int64_t es = t.element_size();
+  return (t.stride(3) == 1 || t.size(3) == 1) && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && t.stride(0) * es % 16 == 0 &&
+         t.stride(1) * es % 16 == 0 && t.stride(2) * es % 16 == 0;
+}
+Tensor aligned_view(const Tensor& t) { return aligned(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
+
+// Slot i of a packed (B, N, 6, H, d) tensor as a (B, H, N, d) descriptor.
+castle_tensor_t packed_desc(const Tensor& p, int i) {
+  return {static_cast<char*>(p.data_ptr()) + i * p.stride(2) * p.element_size(), p.stride(0), p.stride(3), p.stride(1)};
+}
+
+castle_tensor_t rect(castle_tensor_t t, int64_t es, int64_t b, int64_t h) {
+  t.ptr = static_cast<char*>(t.ptr) + (b * t.stride_b + h * t.stride_h) * es;
+  return t;
+}
+
+Tensor empty_bnhd(int64_t B, int64_t H, int64_t N, int64_t d, const at::TensorOptions& o) {
+  // a (B, H, N, d) tensor laid out (B, N, H, d): merging the heads afterwards is a free reshape
+  return at::empty_strided({B, H, N, d}, {N * H * d, d, H * d, 1}, o);
+}
+
+// ------------------------------------------------------------------------------------------------ parallel pass
+struct Rotary {
+  Tensor freqs;
+  int64_t position0 = 0;
+  bool on() const { return freqs.defined(); }
+  castle_rotary_t desc(bool inverse) const {
+    return {freqs.data_ptr(), dtype_code(freqs.scalar_type()), inverse ? 1 : 0, position0};
+  }
+};
+constexpr uint32_t kRotated = 0x1f;   // of qu, ku, vu, qc, kc, vc all but vc
+
+struct Options {
+  double scale = 1;
+  bool return_U = false, need_grad = false;
+  int64_t limit = 0;           // bytes of scratch per launch
+  int64_t long_seq = 0;        // from this length on bf16 callers are computed with fp16 operands
+  Rotary rotary;
+  std::vector<Tensor> caches;  // four (B, H, N, d) views (U, qu, kc, vc) to fill, or empty
+};
+
+// The kernels' inputs: six (B, H, N, dp) descriptors in the order qu, ku, vu, qc, kc, vc and what keeps them alive.
+struct Inputs {
+  castle_tensor_t t[6];
+  std::vector<Tensor> keep;   // one packed tensor, or six
+};
+
+struct Problem {
+  int64_t B, H, N, d, dp;
+  at::ScalarType dtype, cdtype;   // the caller's and the operands'
+};
+
+castle_problem_t c_problem(const Problem& p, double scale, at::ScalarType t, int64_t d) {
+  return {(int32_t)p.B, (int32_t)p.H, (int32_t)p.N, (int32_t)d, dtype_code(t), (float)scale};
+}
+
+Problem make_problem(at::IntArrayRef bhnd, at::ScalarType dtype, int64_t long_seq) {
+  Problem p{bhnd[0], bhnd[1], bhnd[2], bhnd[3], 0, dtype, dtype};
+  if (p.d > 128 || p.d % 8 || p.d < 1)
+    throw std::runtime_error("castle_attention: dim_head " + std::to_string(p.d) + " not supported (multiples of 8 up to 128)");
+  need(dtype_code(dtype) >= 0, "castle_attention: tensors must be bf16, fp16 or fp32");
+  p.dp = p.d <= 64 ? 64 : 128;
+  if (!(dtype == at::kHalf || (dtype == at::kBFloat16 && p.N < long_seq))) p.cdtype = at::kHalf;
+  return p;
+}
+
+// Rectangles of the (batch, head) grid that each need at most `limit` bytes of scratch: whole batch rows, or head
+// ranges of one row, so that per-pair buffers of a rectangle stay contiguous (ops.forward_chunks).
+template <typename F>
+void for_chunks(int64_t B, int64_t H, int64_t per_pair, int64_t limit, F&& f) {
+  const int64_t pairs = limit / std::max<int64_t>(per_pair, 1);
+  if (pairs < 1)
+    throw std::runtime_error("castle_attention: one (batch, head) pair needs " + std::to_string(per_pair) +
+                             " bytes of forward scratch, more than the " + std::to_string(limit) +
+                             "-byte bound (sequence too long for this build)");
+  auto size = [](int64_t total, int64_t most) { const int64_t n = (total + most - 1) / most; return (total + n - 1) / n; };
+  if (pairs >= H) {
+    const int64_t s = size(B, std::min(B, pairs / H));
+    for (int64_t b = 0; b < B; b += s) f(b, std::min(B, b + s), (int64_t)0, H);
+  } else {
+    const int64_t s = size(H, pairs);
+    for (int64_t b = 0; b < B; ++b)
+      for (int64_t h = 0; h < H; h += s) f(b, b + 1, h, std::min(H, h + s));
+  }
+}
+
+struct Result {
+  Tensor out;             // (B, H, N, d), the caller's type
+  Tensor U;
+  Inputs in;
+  Tensor out16, lse, w_state;
+};
+
+Result run_forward(const Problem& p, Inputs in, const Options& o, const at::Device& dev) {
+  const c10::cuda::CUDAGuard guard(dev);
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  const auto f32 = at::TensorOptions().dtype(at::kFloat).device(dev);
+  const auto ct = f32.dtype(p.cdtype), st = f32.dtype(p.dtype);
+  Result r;
+  // The forward kernels fill the caches from their operand tiles where those are the caller's values.
+  const bool caches = !o.caches.empty();
+  const bool kernel_fill = caches && p.dtype == p.cdtype && p.d == p.dp;
+  if (p.dtype != p.cdtype || p.d != p.dp || o.rotary.on() || (caches && !kernel_fill)) {
+    Tensor packed = at::empty({p.B, p.N, 6, p.H, p.dp}, ct);
+    castle_tensor_t dst[6], copies[6] = {};
+    for (int i = 0; i < 6; ++i) dst[i] = packed_desc(packed, i);
+    if (caches && !kernel_fill) {
+      copies[0] = desc(o.caches[1]); copies[4] = desc(o.caches[2]); copies[5] = desc(o.caches[3]);
+    }
+    const castle_problem_t cp = c_problem(p, o.scale, p.dtype, p.d);
+    castle_rotary_t rot{};
+    if (o.rotary.on()) rot = o.rotary.desc(false);
+    check(api.transform(&cp, 6, in.t, dst, dtype_code(p.cdtype), (int32_t)p.dp, copies, o.rotary.on() ? &rot : nullptr, kRotated,
+                        nullptr, stream.stream()), "castle_transform");
+    for (int i = 0; i < 6; ++i) in.t[i] = dst[i];
+    in.keep = {packed};
+  }
+  r.out16 = empty_bnhd(p.B, p.H, p.N, p.dp, ct);
+  r.lse = at::empty({p.B, p.H, p.N}, f32);
+  Tensor u;   // what the kernel writes U to
+  if (caches && p.d == p.dp) u = o.caches[0];
+  else if (o.return_U || caches) u = at::empty({p.B, p.H, p.N, p.dp}, st);
+  if (o.need_grad) r.w_state = at::empty({p.B, p.H, p.N, p.dp}, f32);
+  const Tensor status = status_word(dev.index());
+  castle_problem_t one = c_problem(p, o.scale, p.cdtype, p.dp);
+  one.batch = one.heads = 1;
+  const int64_t per_pair = std::max<int64_t>((int64_t)api.fwd_workspace_bytes(&one), 1);
+  int64_t most = 0;
+  for_chunks(p.B, p.H, per_pair, o.limit, [&](int64_t b0, int64_t b1, int64_t h0, int64_t h1) { most = std::max(most, (b1 - b0) * (h1 - h0)); });
+  const Tensor ws = scratch(stream, (size_t)(most * per_pair));
+  const castle_tensor_t out_d = desc(r.out16);
+  for_chunks(p.B, p.H, per_pair, o.limit, [&](int64_t b0, int64_t b1, int64_t h0, int64_t h1) {
+    castle_problem_t cp = one;
+    cp.batch = (int32_t)(b1 - b0);
+    cp.heads = (int32_t)(h1 - h0);
+    castle_tensor_t t[6];
+    for (int i = 0; i < 6; ++i) t[i] = rect(in.t[i], 2, b0, h0);
+    const castle_tensor_t od = rect(out_d, 2, b0, h0);
+    const int64_t pair0 = b0 * p.H + h0;
+    float* lse = r.lse.data_ptr<float>() + pair0 * p.N;
+    float* w = o.need_grad ? r.w_state.data_ptr<float>() + pair0 * p.N * p.dp : nullptr;
+    castle_tensor_t ud{};
+    if (u.defined()) ud = rect(desc(u), u.element_size(), b0, h0);
+    if (kernel_fill) {
+      castle_tensor_t c[3];
+      for (int i = 0; i < 3; ++i) c[i] = rect(desc(o.caches[1 + i]), 2, b0, h0);
+      check(api.fwd_prefill(&cp, &t[3], &t[4], &t[5], &t[0], &t[1], &t[2], &od, lse, &ud, &c[0], &c[1], &c[2], w, ws.data_ptr(),
+                            ws.numel(), status.data_ptr<int32_t>(), stream.stream()), "castle_fwd_prefill");
+    } else {
+      check(api.fwd(&cp, &t[3], &t[4], &t[5], &t[0], &t[1], &t[2], &od, lse, u.defined() ? &ud : nullptr, dtype_code(p.dtype), w,
+                    ws.data_ptr(), ws.numel(), status.data_ptr<int32_t>(), stream.stream()), "castle_fwd");
+    }
+  });
+  r.out = r.out16;
+  if (p.dtype != p.cdtype || p.d != p.dp) {
+    r.out = empty_bnhd(p.B, p.H, p.N, p.d, st);
+    const castle_problem_t cp = c_problem(p, o.scale, p.cdtype, p.dp);
+    const castle_tensor_t dst = desc(r.out);
+    check(api.transform(&cp, 1, &out_d, &dst, dtype_code(p.dtype), (int32_t)p.d, nullptr, nullptr, 0, nullptr, stream.stream()),
+          "castle_transform");
+  }
+  if (caches && p.d != p.dp) o.caches[0].copy_(u.narrow(3, 0, p.d));
+  if (o.return_U) r.U = caches ? o.caches[0].narrow(3, 0, p.d) : u.narrow(3, 0, p.d);
+  r.in = std::move(in);
+  return r;
+}
+
+// The six input gradients as one packed (B, N, 6, H, d) tensor in the caller's type.
+Tensor run_backward(const Problem& p, const castle_tensor_t* in, const Tensor& out16, const Tensor& lse, const Tensor& w_state,
+                    Tensor grad, const Options& o) {
+  const at::Device dev = out16.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  const auto ct = at::TensorOptions().dtype(p.cdtype).device(dev);
+  Tensor factor;   // [s, 1 / s]
+  if (p.dtype != p.cdtype) {
+    // fp16 operands for a caller with a wider exponent range: bring the upstream gradient to a fixed magnitude with a
+    // power of two (exact; every gradient is linear in it) and undo it on the results, so that neither small gradients
+    // underflow nor large ones overflow in fp16.  Everything stays on the device.
+    if (!grad.is_non_overlapping_and_dense() || !aligned(grad)) grad = grad.clone(at::MemoryFormat::Contiguous);
+    factor = at::empty({2}, ct.dtype(at::kFloat));
+    const Tensor words = zero_words(stream, 0);
+    check(api.amax_scale(dtype_code(p.dtype), grad.data_ptr(), grad.numel(), reinterpret_cast<uint32_t*>(words.data_ptr()),
+                         factor.data_ptr<float>(), stream.stream()), "castle_amax_scale");
+  }
+  if (p.dtype != p.cdtype || p.d != p.dp) {
+    grad = aligned_view(grad);
+    Tensor g16 = empty_bnhd(p.B, p.H, p.N, p.dp, ct);
+    const castle_problem_t cp = c_problem(p, o.scale, p.dtype, p.d);
+    const castle_tensor_t src = desc(grad), dst = desc(g16);
+    check(api.transform(&cp, 1, &src, &dst, dtype_code(p.cdtype), (int32_t)p.dp, nullptr, nullptr, 0,
+                        factor.defined() ? factor.data_ptr<float>() : nullptr, stream.stream()), "castle_transform");
+    grad = g16;
+  }
+  grad = aligned_view(grad);
+  Tensor packed = at::empty({p.B, p.N, 6, p.H, p.dp}, ct);
+  castle_tensor_t g[6];
+  for (int i = 0; i < 6; ++i) g[i] = packed_desc(packed, i);
+  const castle_problem_t cp = c_problem(p, o.scale, p.cdtype, p.dp);
+  int64_t bytes = (int64_t)api.bwd_workspace_bytes(&cp);
+  if (p.dp == 128 && bytes > o.limit) {
+    // the tile hand-over scratch of the dim_head-128 kernels may be smaller than asked for: the (batch, head) pairs
+    // then run in smaller chunks, down to one pair at a time
+    const int64_t nblk = (p.N + 127) / 128, pair = nblk * (nblk + 1) / 2 * 3 * 32768;
+    const int64_t asked = std::min<int64_t>(p.B * p.H, std::max<int64_t>(1, ((int64_t)8 << 30) / pair));
+    bytes = std::max(bytes - (asked - 1) * pair, o.limit);
+  }
+  const Tensor ws = scratch(stream, (size_t)bytes);
+  const castle_tensor_t od = desc(out16), gd = desc(grad);
+  check(api.bwd(&cp, &in[3], &in[4], &in[5], &in[0], &in[1], &in[2], &od, &gd, lse.data_ptr<float>(), w_state.data_ptr<float>(),
+                &g[3], &g[4], &g[5], &g[0], &g[1], &g[2], ws.data_ptr(), ws.numel(), status_word(dev.index()).data_ptr<int32_t>(),
+                stream.stream()), "castle_bwd");
+  if (p.dtype == p.cdtype && p.d == p.dp && !o.rotary.on()) return packed;
+  Tensor result = at::empty({p.B, p.N, 6, p.H, p.d}, ct.dtype(p.dtype));
+  castle_tensor_t dst[6];
+  for (int i = 0; i < 6; ++i) dst[i] = packed_desc(result, i);
+  castle_rotary_t rot{};
+  if (o.rotary.on()) rot = o.rotary.desc(true);
+  check(api.transform(&cp, 6, g, dst, dtype_code(p.dtype), (int32_t)p.d, nullptr, o.rotary.on() ? &rot : nullptr, kRotated,
+                      factor.defined() ? factor.data_ptr<float>() + 1 : nullptr, stream.stream()), "castle_transform");
+  return result;
+}
+
+// Gradient node of both operators: one packed input, or six in the operator's order qc, kc, vc, qu, ku, vu.
+struct CastleBackward : public Node {
+  Problem p;
+  Options o;
+  bool packed = false;
+  std::vector<SavedVariable> inputs;
+  SavedVariable out16, lse, w_state;
+  bool out_is_output = false;
+
+  std::string name() const override { return "CastleAttentionBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (auto& v : inputs) v.reset_data();
+    out16.reset_data(); lse.reset_data(); w_state.reset_data();
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list result(packed ? 1 : 6);
+    if (grads.empty() || !grads[0].defined()) return result;
+    at::NoGradGuard no_grad;
+    castle_tensor_t in[6];
+    std::vector<Tensor> keep;
+    for (auto& v : inputs) keep.push_back(v.unpack());
+    for (int i = 0; i < 6; ++i) in[i] = keep.size() == 1 ? packed_desc(keep[0], i) : desc(keep[i]);
+    const Tensor out = out_is_output ? out16.unpack(shared_from_this()) : out16.unpack();
+    Tensor g = run_backward(p, in, out, lse.unpack(), w_state.unpack(), grads[0], o);
+    if (packed) {
+      result[0] = std::move(g);
+    } else {
+      static const int slot[6] = {3, 4, 5, 0, 1, 2};
+      for (int i = 0; i < 6; ++i) result[i] = g.select(2, slot[i]).permute({0, 2, 1, 3});
+    }
+    return result;
+  }
+};
+
+// Forward with its gradient node; `vars` are the differentiable inputs (one packed, or six in operator order).
+Result attention(const Problem& p, Inputs in, Options o, const std::vector<Tensor>& vars) {
+  bool any = false;
+  for (const auto& v : vars) any |= v.requires_grad();
+  o.need_grad = any && at::GradMode::is_enabled();
+  const at::Device dev = vars[0].device();
+  Result r;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    r = run_forward(p, std::move(in), o, dev);
+  }
+  if (!o.need_grad) return r;
+  auto node = std::shared_ptr<CastleBackward>(new CastleBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(vars));
+  node->p = p;
+  o.caches.clear();
+  node->o = o;
+  node->packed = vars.size() == 1;
+  torch::autograd::set_history(r.out, node);
+  for (const auto& t : r.in.keep) node->inputs.emplace_back(t, false);
+  node->out_is_output = r.out.is_same(r.out16);
+  node->out16 = SavedVariable(r.out16, node->out_is_output);
+  node->lse = SavedVariable(r.lse, false);
+  node->w_state = SavedVariable(r.w_state, false);
+  return r;
+}
+
+Result attention_six(const Tensor* v /* qc, kc, vc, qu, ku, vu */, const Options& o) {
+  for (int i = 0; i < 6; ++i) {
+    need(v[i].is_cuda(), "castle_attention: expected CUDA tensors; this package has no CPU path");
+    need(v[i].dim() == 4 && v[i].sizes() == v[0].sizes() && v[i].device() == v[0].device(),
+         "castle_attention: six (B, H, N, d) tensors of one shape and device expected");
+  }
+  const Problem p = make_problem(v[0].sizes(), v[0].scalar_type(), o.long_seq);
+  static const int order[6] = {3, 4, 5, 0, 1, 2};   // qu, ku, vu, qc, kc, vc
+  Inputs in;
+  {
+    at::NoGradGuard no_grad;
+    for (int i = 0; i < 6; ++i) {
+      Tensor t = v[order[i]];
+      if (t.scalar_type() != p.dtype) t = t.to(p.dtype);
+      t = aligned_view(t);
+      in.t[i] = desc(t);
+      in.keep.push_back(t);
+    }
+  }
+  return attention(p, std::move(in), o, std::vector<Tensor>(v, v + 6));
+}
+
+Result attention_packed(const Tensor& packed, const Options& o) {   // (B, N, 6, H, d), order qu, ku, vu, qc, kc, vc
+  need(packed.is_cuda(), "castle_attention: expected CUDA tensors; this package has no CPU path");
+  need(packed.dim() == 5 && packed.size(2) == 6, "castle_attention_packed: a (B, N, 6, H, d) tensor expected");
+  const int64_t B = packed.size(0), N = packed.size(1), H = packed.size(3), d = packed.size(4);
+  const Problem p = make_problem({B, H, N, d}, packed.scalar_type(), o.long_seq);
+  Tensor t = packed;
+  const int64_t es = t.element_size();
+  if (!(t.stride(4) == 1 || d == 1) || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 || t.stride(0) * es % 16 ||
+      t.stride(1) * es % 16 || t.stride(2) * es % 16 || t.stride(3) * es % 16) {
+    at::NoGradGuard no_grad;
+    t = t.clone(at::MemoryFormat::Contiguous);
+  }
+  Inputs in;
+  for (int i = 0; i < 6; ++i) in.t[i] = packed_desc(t, i);
+  in.keep = {t};
+  return attention(p, std::move(in), o, {packed});
+}
+
+// ------------------------------------------------------------------------------------------------ decode step
+// `news` in the operator's order qc, kc, vc, qu, ku, vu; `caches` U, qu, kc, vc.
+Tensor decode_core(const castle_tensor_t* news, const Tensor* caches, int64_t B, int64_t H, int64_t d, at::ScalarType dtype,
+                   int64_t t, double scale, const Rotary& rotary, const at::Device& dev) {
+  const c10::cuda::CUDAGuard guard(dev);
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  const int64_t cap = caches[0].size(2);
+  for (int i = 0; i < 4; ++i) {
+    const Tensor& c = caches[i];
+    if (!(c.scalar_type() == dtype && c.dim() == 4 && c.size(0) == B && c.size(1) == H && c.size(2) == cap && c.size(3) == d &&
+          c.stride(3) == 1))
+      throw AssertError("castle_decode_step: the caches must be (B, H, capacity, d) buffers of the token's type");
+  }
+  Tensor out = at::empty({B, H, 1, d}, caches[0].options());
+  castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
+  const size_t bytes = api.decode_workspace_bytes(&cp, (int32_t)t);
+  const Tensor ws = scratch(stream, bytes), words = zero_words(stream, B * H), status = status_word(dev.index());
+  castle_tensor_t c[4];
+  for (int i = 0; i < 4; ++i) c[i] = desc(caches[i]);
+  const castle_tensor_t od = desc(out);
+  castle_rotary_t rot{};
+  if (rotary.on()) rot = rotary.desc(false);
+  check(api.decode_step_fused(&cp, (int32_t)t, (int32_t)cap, &news[0], &news[1], &news[2], &news[3], &news[4], &news[5], &c[0], &c[1],
+                              &c[2], &c[3], &od, rotary.on() ? &rot : nullptr,
+                              reinterpret_cast<uint32_t*>(words.data_ptr()) + kAmaxWords, ws.data_ptr(), ws.numel(),
+                              status.data_ptr<int32_t>(), stream.stream()), "castle_decode_step");
+  return out;
+}
+
+Tensor decode_step(const Tensor* news, const Tensor* caches, int64_t t, double scale) {
+  need(news[0].is_cuda(), "castle_decode_step: expected CUDA tensors; this package has no CPU path");
+  if (news[0].dim() != 4 || news[0].size(2) != 1) throw AssertError("castle_decode_step: (B, H, 1, d) tensors expected");
+  const auto dtype = news[0].scalar_type();
+  if (dtype_code(dtype) < 0) throw std::runtime_error("castle_decode_step: dtype " + std::string(at::toString(dtype)) + " not supported");
+  at::NoGradGuard no_grad;
+  Tensor keep[6];
+  castle_tensor_t nd[6];
+  for (int i = 0; i < 6; ++i) {
+    need(news[i].scalar_type() == dtype && news[i].sizes() == news[0].sizes(),
+         "castle_decode_step: the new rows must have one shape and type");
+    keep[i] = aligned_view(news[i]);
+    nd[i] = desc(keep[i]);
+  }
+  return decode_core(nd, caches, news[0].size(0), news[0].size(1), news[0].size(3), dtype, t, scale, Rotary{}, news[0].device());
+}
+
+// ------------------------------------------------------------------------------------------------ the plain module
+struct Layer {
+  Tensor norm, to_qkv, combine;   // norm may be undefined
+  std::optional<double> eps;
+  int64_t heads = 0, dim_head = 0;
+};
+
+Tensor project(const Tensor& x, const Layer& l) {   // (B, N, 6, H, d)
+  Tensor h = l.norm.defined() ? at::rms_norm(x, {x.size(-1)}, l.norm, l.eps) : x;
+  return at::linear(h, l.to_qkv).view({x.size(0), x.size(1), 6, l.heads, l.dim_head});
+}
+
+Tensor layer_forward(const Tensor& x, const Layer& l, const Options& o) {
+  const Tensor out = attention_packed(project(x, l), o).out;
+  return at::linear(out.permute({0, 2, 1, 3}).reshape({x.size(0), x.size(1), l.heads * l.dim_head}), l.combine);
+}
+
+// One token from its packed projection (B, 1, 6, H, d): the core's output, (B, 1, H * d).
+Tensor decode_packed(const Tensor& packed, const Tensor* caches, int64_t t, double scale, const Rotary& rotary) {
+  need(packed.is_cuda(), "castle_decode_step: expected CUDA tensors; this package has no CPU path");
+  const int64_t B = packed.size(0), H = packed.size(3), d = packed.size(4);
+  need(dtype_code(packed.scalar_type()) >= 0, "castle_decode_step: bf16, fp16 or fp32 expected");
+  at::NoGradGuard no_grad;
+  static const int order[6] = {3, 4, 5, 0, 1, 2};   // the operator's order out of qu, ku, vu, qc, kc, vc
+  castle_tensor_t nd[6];
+  for (int i = 0; i < 6; ++i) nd[i] = packed_desc(packed, order[i]);
+  return decode_core(nd, caches, B, H, d, packed.scalar_type(), t, scale, rotary, packed.device()).view({B, 1, H * d});
+}
+
+Tensor layer_decode(const Tensor& x, const Layer& l, const Tensor* caches, int64_t t, double scale, const Rotary& rotary) {
+  return at::linear(decode_packed(project(x, l), caches, t, scale, rotary), l.combine);
+}
+
+// ------------------------------------------------------------------------------------------------ Python
+template <typename F>
+PyObject* guarded(F&& f) {   // C++ exceptions become Python ones; `f` runs without the interpreter lock where it says so
+  try {
+    return f();
+  } catch (const AssertError& e) {
+    PyErr_SetString(PyExc_AssertionError, e.what());
+  } catch (const c10::Error& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+  }
+  return nullptr;
+}
+struct Unlocked {   // releases the interpreter lock for its lifetime
+  PyThreadState* s = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(s); }
+};
+
+const Tensor& arg_tensor(PyObject* o) {
+  if (!THPVariable_Check(o)) throw std::runtime_error("castle: a tensor expected");
+  return THPVariable_Unpack(o);
+}
+Tensor arg_optional(PyObject* o) { return o == Py_None ? Tensor() : arg_tensor(o); }
+int64_t arg_int(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); throw std::runtime_error("castle: an integer expected"); }
+  return v;
+}
+double arg_float(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) { PyErr_Clear(); throw std::runtime_error("castle: a number expected"); }
+  return v;
+}
+std::vector<Tensor> arg_caches(PyObject* o) {
+  std::vector<Tensor> v;
+  if (o == Py_None) return v;
+  PyObject* fast = PySequence_Fast(o, "castle: four cache tensors expected");
+  if (!fast) { PyErr_Clear(); throw std::runtime_error("castle: four cache tensors expected"); }
+  for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(fast); ++i) {
+    PyObject* item = PySequence_Fast_GET_ITEM(fast, i);
+    if (!THPVariable_Check(item)) { Py_DECREF(fast); throw std::runtime_error("castle: four cache tensors expected"); }
+    v.push_back(THPVariable_Unpack(item));
+  }
+  Py_DECREF(fast);
+  if (v.size() != 4) throw std::runtime_error("castle: four cache tensors expected");
+  return v;
+}
+void arg_count(Py_ssize_t n, Py_ssize_t want) {
+  if (n != want) throw std::runtime_error("castle: wrong number of arguments");
+}
+
+// The operators' rule for caches: the kernels store their 16-bit operand tiles.
+void check_cache_out(const Options& o, at::IntArrayRef bhnd, at::ScalarType dtype) {
+  if (o.caches.empty()) return;
+  const bool fills = (dtype == at::kHalf || (dtype == at::kBFloat16 && bhnd[2] < o.long_seq)) && (bhnd[3] == 64 || bhnd[3] == 128);
+  need(o.return_U && fills, "castle_attention: cache_out needs return_U, a 16-bit dtype and dim_head 64 or 128");
+  for (const auto& c : o.caches)
+    need(c.sizes() == bhnd && c.scalar_type() == dtype && c.stride(3) == 1,
+         "castle_attention: cache_out tensors must be (B, H, N, d) views in the input dtype");
+}
+
+// t[:, :, :rows] without the dispatcher (a token makes four of these; caches are no part of any graph).
+Tensor first_rows(const Tensor& t, int64_t rows) {
+  if (t.dim() != 4 || rows < 0 || rows > t.size(2) || t.requires_grad()) return t.narrow(2, 0, rows);
+  Tensor v = at::detail::make_tensor<c10::TensorImpl>(c10::TensorImpl::VIEW, c10::Storage(t.storage()), t.key_set(), t.dtype());
+  c10::TensorImpl* impl = v.unsafeGetTensorImpl();
+  impl->set_storage_offset(t.storage_offset());
+  impl->set_sizes_and_strides(std::array<int64_t, 4>{t.size(0), t.size(1), rows, t.size(3)}, t.strides());
+  return v;
+}
+
+PyObject* wrap_result(Result r, bool with_U) {
+  PyObject* out = THPVariable_Wrap(r.out);
+  if (!with_U || !out) return out;
+  PyObject* u = THPVariable_Wrap(r.U);
+  if (!u) { Py_DECREF(out); return nullptr; }
+  PyObject* t = PyTuple_Pack(2, out, u);
+  Py_DECREF(out);
+  Py_DECREF(u);
+  return t;
+}
+
+// attention(qc, kc, vc, qu, ku, vu, scale, return_U, cache_out, limit, long_seq)
+PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    arg_count(n, 11);
+    Tensor v[6];
+    for (int i = 0; i < 6; ++i) v[i] = arg_tensor(a[i]);
+    Options o;
+    o.scale = arg_float(a[6]);
+    o.return_U = PyObject_IsTrue(a[7]) == 1;
+    o.caches = arg_caches(a[8]);
+    o.limit = arg_int(a[9]);
+    o.long_seq = arg_int(a[10]);
+    Result r;
+    {
+      Unlocked u;
+      if (v[0].dim() == 4) check_cache_out(o, v[0].sizes(), v[0].scalar_type());
+      r = attention_six(v, o);
+    }
+    return wrap_result(std::move(r), o.return_U);
+  });
+}
+
+// attention_packed(packed, scale, return_U, cache_out, limit, long_seq, rotary freqs or None, strict): `strict` = the
+// operator's rule for cache_out; the module's own caches may have any type and width
+PyObject* py_attention_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    arg_count(n, 8);
+    const Tensor packed = arg_tensor(a[0]);
+    Options o;
+    o.scale = arg_float(a[1]);
+    o.return_U = PyObject_IsTrue(a[2]) == 1;
+    o.caches = arg_caches(a[3]);
+    o.limit = arg_int(a[4]);
+    o.long_seq = arg_int(a[5]);
+    o.rotary.freqs = arg_optional(a[6]);
+    const bool strict = PyObject_IsTrue(a[7]) == 1;
+    Result r;
+    {
+      Unlocked u;
+      if (strict && packed.dim() == 5)
+        check_cache_out(o, {packed.size(0), packed.size(3), packed.size(1), packed.size(4)}, packed.scalar_type());
+      r = attention_packed(packed, o);
+    }
+    return wrap_result(std::move(r), o.return_U);
+  });
+}
+
+// decode_step(qc, kc, vc, qu, ku, vu, U, qu_cache, kc_cache, vc_cache, cache_len, scale)
+PyObject* py_decode_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    arg_count(n, 12);
+    Tensor v[10], out;
+    for (int i = 0; i < 10; ++i) v[i] = arg_tensor(a[i]);
+    const int64_t t = arg_int(a[10]);
+    const double scale = arg_float(a[11]);
+    {
+      Unlocked u;
+      out = decode_step(v, v + 6, t, scale);
+    }
+    return THPVariable_Wrap(out);
+  });
+}
+
+Layer arg_layer(PyObject* const* a) {   // norm weight or None, eps or None, to_all_qkv weight, combine_heads weight, heads, dim_head
+  Layer l;
+  l.norm = arg_optional(a[0]);
+  if (a[1] != Py_None) l.eps = arg_float(a[1]);
+  l.to_qkv = arg_tensor(a[2]);
+  l.combine = arg_tensor(a[3]);
+  l.heads = arg_int(a[4]);
+  l.dim_head = arg_int(a[5]);
+  return l;
+}
+
+// layer_forward(x, <layer: 6>, scale, rotary freqs or None, caches or None, limit, long_seq)
+PyObject* py_layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    arg_count(n, 12);
+    const Tensor x = arg_tensor(a[0]);
+    const Layer l = arg_layer(a + 1);
+    Options o;
+    o.scale = arg_float(a[7]);
+    o.rotary.freqs = arg_optional(a[8]);
+    o.caches = arg_caches(a[9]);
+    o.limit = arg_int(a[10]);
+    o.long_seq = arg_int(a[11]);
+    Tensor out;
+    {
+      Unlocked u;
+      out = layer_forward(x, l, o);
+    }
+    return THPVariable_Wrap(out);
+  });
+}
+
+// layer_decode(x, <layer: 6>, scale, rotary freqs or None, caches, cache_len)
+PyObject* py_layer_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    arg_count(n, 11);
+    const Tensor x = arg_tensor(a[0]);
+    const Layer l = arg_layer(a + 1);
+    const double scale = arg_float(a[7]);
+    Rotary rotary;
+    rotary.freqs = arg_optional(a[8]);
+    const std::vector<Tensor> caches = arg_caches(a[9]);
+    if (caches.size() != 4) throw std::runtime_error("castle: four cache tensors expected");
+    const int64_t t = rotary.position0 = arg_int(a[10]);
+    Tensor out;
+    {
+      Unlocked u;
+      out = layer_decode(x, l, caches.data(), t, scale, rotary);
+    }
+    return THPVariable_Wrap(out);
+  });
+}
+
+// decode_packed(packed, scale, rotary freqs or None, caches, cache_len)
+PyObject* py_decode_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&] {
+    arg_count(n, 5);
+    const Tensor packed = arg_tensor(a[0]);
+    const double scale = arg_float(a[1]);
+    Rotary rotary;
+    rotary.freqs = arg_optional(a[2]);
+    const std::vector<Tensor> caches = arg_caches(a[3]);
+    if (caches.size() != 4) throw std::runtime_error("castle: four cache tensors expected");
+    const int64_t t = rotary.position0 = arg_int(a[4]);
+    Tensor out;
+    {
+      Unlocked u;
+      out = decode_packed(packed, caches.data(), t, scale, rotary);
+    }
+    return THPVariable_Wrap(out);
+  });
+}
+
+// first_rows(buffers, n): the buffers' [:, :, :n] views as a tuple
+PyObject* py_first_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    arg_count(n, 2);
+    const std::vector<Tensor> bufs = arg_caches(a[0]);
+    const int64_t rows = arg_int(a[1]);
+    PyObject* t = PyTuple_New((Py_ssize_t)bufs.size());
+    for (size_t i = 0; i < bufs.size(); ++i) PyTuple_SET_ITEM(t, (Py_ssize_t)i, THPVariable_Wrap(first_rows(bufs[i], rows)));
+    return t;
+  });
+}
+
+PyObject* py_status_word(PyObject*, PyObject* device) {
+  return guarded([&] { return THPVariable_Wrap(status_word((int)arg_int(device))); });
+}
+PyObject* py_status_devices(PyObject*, PyObject*) {
+  std::lock_guard<std::mutex> lock(state_mutex);
+  PyObject* list = PyList_New(0);
+  for (const auto& kv : status_words) {
+    PyObject* i = PyLong_FromLong(kv.first);
+    PyList_Append(list, i);
+    Py_DECREF(i);
+  }
+  return list;
+}
+PyObject* py_release_workspaces(PyObject*, PyObject*) {
+  std::map<std::pair<int, void*>, StreamState> old;
+  {
+    std::lock_guard<std::mutex> lock(state_mutex);
+    old.swap(stream_states);
+  }
+  Py_RETURN_NONE;
+}
+
+// bind({name: address}): the C ABI's entry points
+PyObject* py_bind(PyObject*, PyObject* d) {
+  return guarded([&]() -> PyObject* {
+    auto get = [&](const char* name) {
+      PyObject* v = PyDict_GetItemString(d, name);
+      if (!v) throw std::runtime_error(std::string("castle: no address for ") + name);
+      return PyLong_AsVoidPtr(v);
+    };
+#define CASTLE_BIND(f) api.f = reinterpret_cast<decltype(api.f)>(get("castle_" #f))
+    CASTLE_BIND(last_error); CASTLE_BIND(fwd_workspace_bytes); CASTLE_BIND(fwd); CASTLE_BIND(fwd_prefill);
+    CASTLE_BIND(bwd_workspace_bytes); CASTLE_BIND(bwd); CASTLE_BIND(transform); CASTLE_BIND(amax_scale);
+    CASTLE_BIND(decode_workspace_bytes); CASTLE_BIND(decode_step_fused);
+#undef CASTLE_BIND
+    Py_RETURN_NONE;
+  });
+}
+
+#define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL
+PyMethodDef methods[] = {{"bind", py_bind, METH_O, nullptr},
+                         {"attention", FAST(py_attention), nullptr},
+                         {"attention_packed", FAST(py_attention_packed), nullptr},
+                         {"decode_step", FAST(py_decode_step), nullptr},
+                         {"layer_forward", FAST(py_layer_forward), nullptr},
+                         {"layer_decode", FAST(py_layer_decode), nullptr},
+                         {"decode_packed", FAST(py_decode_packed), nullptr},
+                         {"first_rows", FAST(py_first_rows), nullptr},
+                         {"status_word", py_status_word, METH_O, nullptr},
+                         {"status_devices", py_status_devices, METH_NOARGS, nullptr},
+                         {"release_workspaces", py_release_workspaces, METH_NOARGS, nullptr},
+                         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "Native host path of the operators.", -1, methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module_def); }
