@@ -195,6 +195,17 @@ int castle_decode_step_fused(const castle_problem_t* p, int32_t cache_len, int32
                              const castle_rotary_t* rotary, uint32_t* counters, void* workspace, size_t workspace_bytes,
                              int32_t* status, void* stream);
 
+/* ---- a token's projections ----------------------------------------------------
+ * y = norm(x) @ weight^T for 1 to 8 rows: the projections around the cached step
+ * (lookahead_keys_attention/lookahead_keys_attention.py:67-80, :99-104, :207) as one launch each.  x: rows of
+ * in_features elements, row_stride elements apart; weight: contiguous (out_features, in_features); y: contiguous
+ * (rows, out_features); norm_weight: RMSNorm's, in_features elements, or NULL for none.  All of `dtype`, sums in
+ * fp32.  castle_token_linear_fits says whether a size is supported.
+ */
+int castle_token_linear_fits(int32_t dtype, int32_t rows, int32_t in_features);
+int castle_token_linear(int32_t dtype, int32_t rows, int32_t in_features, int32_t out_features, const void* x,
+                        int64_t row_stride, const void* norm_weight, float eps, const void* weight, void* y, void* stream);
+
 /* ---- cached single-token step without caller scratch -----------------------
  * (no counterpart in the reference)  Same step and same arguments as
  * castle_decode_step(), minus the workspace: the split partials go to a fixed

@@ -34,14 +34,11 @@ class _CacheBuffers:
     NOW.  Decode steps append to them and rewrite U in place, so only the cache returned by the
     latest step still describes their contents."""
 
-    __slots__ = ("bufs", "length")
+    __slots__ = ("bufs", "length", "capacity")
 
     def __init__(self, bufs, length):
         self.bufs, self.length = list(bufs), int(length)
-
-    @property
-    def capacity(self):
-        return self.bufs[0].shape[2]
+        self.capacity = self.bufs[0].shape[2]
 
     def views(self, n):
         return _lib.host().first_rows(self.bufs, n)
@@ -124,10 +121,10 @@ class Castle(nn.Module):
 
     def _state_in_place(self, cache, t):
         """The capacity buffers behind `cache` if row t can be appended to them as they are, else None."""
-        state = getattr(cache, "_state", None) if isinstance(cache, ModuleCache) else None
-        if state is None or cache._length != t:
+        if not isinstance(cache, ModuleCache) or cache._length != t:
             return None
-        if not cache.is_current() and self.inplace_cache:
+        state = cache._state
+        if state.length != t and self.inplace_cache:
             raise RuntimeError(
                 "this cache was advanced in place by a later decode step and no longer holds its rows; "
                 "construct Castle(..., inplace_cache=False) to decode from one cache more than once")

@@ -75,9 +75,12 @@ __device__ __forceinline__ float group_sum(float v) {
 template <typename T>
 __device__ __forceinline__ void rotate_new(const RotaryParams& r, int64_t col, float* a, float* b, float* c) {
   if (r.freqs == nullptr) return;
+  float f[Vec<T>::N / 2];
+#pragma unroll
+  for (int i = 0; i < Vec<T>::N / 2; ++i) f[i] = rotary_freq(r, (int)col / 2 + i);
 #pragma unroll
   for (int i = 0; i < Vec<T>::N; i += 2) {
-    const float2 cs = rotary_cos_sin(r, 0, (int)(col + i) / 2);
+    const float2 cs = rotary_cos_sin(r, 0, f[i / 2]);
     rotate_pair<T>(a[i], a[i + 1], cs);
     rotate_pair<T>(b[i], b[i + 1], cs);
     if (c) rotate_pair<T>(c[i], c[i + 1], cs);

@@ -15,9 +15,13 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
 #include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <array>
+#include <limits>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -48,6 +52,8 @@ struct Api {
   decltype(&castle_amax_scale) amax_scale;
   decltype(&castle_decode_workspace_bytes) decode_workspace_bytes;
   decltype(&castle_decode_step_fused) decode_step_fused;
+  decltype(&castle_token_linear_fits) token_linear_fits;
+  decltype(&castle_token_linear) token_linear;
 } api{};
 
 void check(int rc, const char* what) {
@@ -137,6 +143,7 @@ struct Rotary {
     return {freqs.data_ptr(), dtype_code(freqs.scalar_type()), inverse ? 1 : 0, position0};
   }
 };
+constexpr int kPackedOrder[6] = {3, 4, 5, 0, 1, 2};   // between the operator's order qc, kc, vc, qu, ku, vu and the packed one, both ways
 constexpr uint32_t kRotated = 0x1f;   // of qu, ku, vu, qc, kc, vc all but vc
 
 struct Options {
@@ -359,8 +366,7 @@ struct CastleBackward : public Node {
     if (packed) {
       result[0] = std::move(g);
     } else {
-      static const int slot[6] = {3, 4, 5, 0, 1, 2};
-      for (int i = 0; i < 6; ++i) result[i] = g.select(2, slot[i]).permute({0, 2, 1, 3});
+      for (int i = 0; i < 6; ++i) result[i] = g.select(2, kPackedOrder[i]).permute({0, 2, 1, 3});
     }
     return result;
   }
@@ -400,12 +406,11 @@ Result attention_six(const Tensor* v /* qc, kc, vc, qu, ku, vu */, const Options
          "castle_attention: six (B, H, N, d) tensors of one shape and device expected");
   }
   const Problem p = make_problem(v[0].sizes(), v[0].scalar_type(), o.long_seq);
-  static const int order[6] = {3, 4, 5, 0, 1, 2};   // qu, ku, vu, qc, kc, vc
   Inputs in;
   {
     at::NoGradGuard no_grad;
     for (int i = 0; i < 6; ++i) {
-      Tensor t = v[order[i]];
+      Tensor t = v[kPackedOrder[i]];
       if (t.scalar_type() != p.dtype) t = t.to(p.dtype);
       t = aligned_view(t);
       in.t[i] = desc(t);
@@ -434,11 +439,7 @@ Result attention_packed(const Tensor& packed, const Options& o) {   // (B, N, 6,
 }
 
 // ------------------------------------------------------------------------------------------------ decode step
-// `news` in the operator's order qc, kc, vc, qu, ku, vu; `caches` U, qu, kc, vc.
-Tensor decode_core(const castle_tensor_t* news, const Tensor* caches, int64_t B, int64_t H, int64_t d, at::ScalarType dtype,
-                   int64_t t, double scale, const Rotary& rotary, const at::Device& dev) {
-  const c10::cuda::CUDAGuard guard(dev);
-  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
+void check_caches(const Tensor* caches, int64_t B, int64_t H, int64_t d, at::ScalarType dtype) {
   const int64_t cap = caches[0].size(2);
   for (int i = 0; i < 4; ++i) {
     const Tensor& c = caches[i];
@@ -446,19 +447,32 @@ Tensor decode_core(const castle_tensor_t* news, const Tensor* caches, int64_t B,
           c.stride(3) == 1))
       throw AssertError("castle_decode_step: the caches must be (B, H, capacity, d) buffers of the token's type");
   }
-  Tensor out = at::empty({B, H, 1, d}, caches[0].options());
-  castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
-  const size_t bytes = api.decode_workspace_bytes(&cp, (int32_t)t);
-  const Tensor ws = scratch(stream, bytes), words = zero_words(stream, B * H), status = status_word(dev.index());
+}
+
+// `news` in the operator's order qc, kc, vc, qu, ku, vu; `caches` U, qu, kc, vc; `out` contiguous (B, H, 1, d).
+void launch_decode(const castle_problem_t& cp, const castle_tensor_t* news, const Tensor* caches, void* out, int64_t t, const Rotary& rotary,
+                   void* ws, size_t ws_bytes, const c10::cuda::CUDAStream& stream) {
+  const Tensor words = zero_words(stream, (int64_t)cp.batch * cp.heads), status = status_word(stream.device_index());
   castle_tensor_t c[4];
   for (int i = 0; i < 4; ++i) c[i] = desc(caches[i]);
-  const castle_tensor_t od = desc(out);
+  const castle_tensor_t od{out, (int64_t)cp.heads * cp.dim_head, cp.dim_head, cp.dim_head};
   castle_rotary_t rot{};
   if (rotary.on()) rot = rotary.desc(false);
-  check(api.decode_step_fused(&cp, (int32_t)t, (int32_t)cap, &news[0], &news[1], &news[2], &news[3], &news[4], &news[5], &c[0], &c[1],
-                              &c[2], &c[3], &od, rotary.on() ? &rot : nullptr,
-                              reinterpret_cast<uint32_t*>(words.data_ptr()) + kAmaxWords, ws.data_ptr(), ws.numel(),
-                              status.data_ptr<int32_t>(), stream.stream()), "castle_decode_step");
+  check(api.decode_step_fused(&cp, (int32_t)t, (int32_t)caches[0].size(2), &news[0], &news[1], &news[2], &news[3], &news[4], &news[5],
+                              &c[0], &c[1], &c[2], &c[3], &od, rotary.on() ? &rot : nullptr,
+                              reinterpret_cast<uint32_t*>(words.data_ptr()) + kAmaxWords, ws, ws_bytes, status.data_ptr<int32_t>(),
+                              stream.stream()), "castle_decode_step");
+}
+
+Tensor decode_core(const castle_tensor_t* news, const Tensor* caches, int64_t B, int64_t H, int64_t d, at::ScalarType dtype,
+                   int64_t t, double scale, const Rotary& rotary, const at::Device& dev) {
+  const c10::cuda::CUDAGuard guard(dev);
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  check_caches(caches, B, H, d, dtype);
+  Tensor out = at::empty({B, H, 1, d}, caches[0].options());
+  const castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
+  const Tensor ws = scratch(stream, api.decode_workspace_bytes(&cp, (int32_t)t));
+  launch_decode(cp, news, caches, out.data_ptr(), t, rotary, ws.data_ptr(), ws.numel(), stream);
   return out;
 }
 
@@ -502,13 +516,59 @@ Tensor decode_packed(const Tensor& packed, const Tensor* caches, int64_t t, doub
   const int64_t B = packed.size(0), H = packed.size(3), d = packed.size(4);
   need(dtype_code(packed.scalar_type()) >= 0, "castle_decode_step: bf16, fp16 or fp32 expected");
   at::NoGradGuard no_grad;
-  static const int order[6] = {3, 4, 5, 0, 1, 2};   // the operator's order out of qu, ku, vu, qc, kc, vc
   castle_tensor_t nd[6];
-  for (int i = 0; i < 6; ++i) nd[i] = packed_desc(packed, order[i]);
+  for (int i = 0; i < 6; ++i) nd[i] = packed_desc(packed, kPackedOrder[i]);
   return decode_core(nd, caches, B, H, d, packed.scalar_type(), t, scale, rotary, packed.device()).view({B, 1, H * d});
 }
 
+// Whether a token's projections can be the framework's own launches: a few rows of plain CUDA tensors of one type, and
+// nothing that changes what a linear call means (autocast, a dispatch mode).
+bool plain_token(const Tensor& x, const Layer& l) {
+  auto plain = [&](const Tensor& t) {
+    return t.is_cuda() && t.scalar_type() == x.scalar_type() && t.is_contiguous() && t.layout() == at::kStrided && t.device() == x.device() &&
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !t.unsafeGetTensorImpl()->is_python_dispatch();
+  };
+  const int64_t inner = l.heads * l.dim_head;
+  return x.dim() == 3 && x.size(1) == 1 && x.is_cuda() && x.stride(2) == 1 && !x.unsafeGetTensorImpl()->is_python_dispatch() &&
+         x.size(0) >= 1 && x.size(0) <= 8 && plain(l.to_qkv) && plain(l.combine) && (!l.norm.defined() || plain(l.norm)) &&
+         l.to_qkv.dim() == 2 && l.to_qkv.size(0) == 6 * inner && l.to_qkv.size(1) == x.size(2) && l.combine.dim() == 2 &&
+         l.combine.size(1) == inner && api.token_linear_fits(dtype_code(x.scalar_type()), (int32_t)x.size(0), (int32_t)x.size(2)) &&
+         api.token_linear_fits(dtype_code(x.scalar_type()), (int32_t)x.size(0), (int32_t)inner) &&
+         reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * x.element_size() % 16 == 0 &&
+         !at::autocast::is_autocast_enabled(at::kCUDA) && !c10::impl::dispatch_mode_enabled();
+}
+
+// Norm, projection, step and output projection of one token as three launches, with what passes between them in the
+// stream's scratch: on the host the allocations would cost as much as the launches.
+Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_t t, double scale, const Rotary& rotary) {
+  const at::Device dev = x.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
+  const auto dtype = x.scalar_type();
+  const int64_t B = x.size(0), H = l.heads, d = l.dim_head, es = x.element_size();
+  check_caches(caches, B, H, d, dtype);
+  const castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
+  const int64_t inner = H * d, row = (B * inner * es + 255) / 256 * 256;
+  const size_t part = (api.decode_workspace_bytes(&cp, (int32_t)t) + 255) / 256 * 256;
+  const Tensor ws = scratch(stream, part + 7 * row);
+  char* packed = static_cast<char*>(ws.data_ptr()) + part;
+  char* core = packed + 6 * row;
+  check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)x.size(2), (int32_t)(6 * inner), x.data_ptr(), x.stride(0),
+                         l.norm.defined() ? l.norm.data_ptr() : nullptr,
+                         (float)l.eps.value_or(std::numeric_limits<float>::epsilon()),   // torch's default for every type
+                         l.to_qkv.data_ptr(), packed, stream.stream()), "castle_token_linear");
+  castle_tensor_t news[6];
+  for (int i = 0; i < 6; ++i) news[i] = {packed + kPackedOrder[i] * inner * es, 6 * inner, d, 6 * inner};
+  launch_decode(cp, news, caches, core, t, rotary, ws.data_ptr(), part, stream);
+  Tensor y = at::empty({B, 1, l.combine.size(0)}, x.options().requires_grad(false));
+  check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)inner, (int32_t)l.combine.size(0), core, inner, nullptr, 0.f,
+                         l.combine.data_ptr(), y.data_ptr(), stream.stream()), "castle_token_linear");
+  return y;
+}
+
 Tensor layer_decode(const Tensor& x, const Layer& l, const Tensor* caches, int64_t t, double scale, const Rotary& rotary) {
+  // no gradient flows through the cached step, so only the last projection could need a graph
+  if (plain_token(x, l) && !(at::GradMode::is_enabled() && l.combine.requires_grad())) return token_layer(x, l, caches, t, scale, rotary);
   return at::linear(decode_packed(project(x, l), caches, t, scale, rotary), l.combine);
 }
 
@@ -776,7 +836,7 @@ PyObject* py_bind(PyObject*, PyObject* d) {
 #define CASTLE_BIND(f) api.f = reinterpret_cast<decltype(api.f)>(get("castle_" #f))
     CASTLE_BIND(last_error); CASTLE_BIND(fwd_workspace_bytes); CASTLE_BIND(fwd); CASTLE_BIND(fwd_prefill);
     CASTLE_BIND(bwd_workspace_bytes); CASTLE_BIND(bwd); CASTLE_BIND(transform); CASTLE_BIND(amax_scale);
-    CASTLE_BIND(decode_workspace_bytes); CASTLE_BIND(decode_step_fused);
+    CASTLE_BIND(decode_workspace_bytes); CASTLE_BIND(decode_step_fused); CASTLE_BIND(token_linear_fits); CASTLE_BIND(token_linear);
 #undef CASTLE_BIND
     Py_RETURN_NONE;
   });

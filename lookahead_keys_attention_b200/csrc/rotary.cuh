@@ -18,11 +18,13 @@ struct RotaryParams {
 // Not inlined: the range reduction's slow path would cost the decode kernels registers in their main loop.
 static __device__ __noinline__ float2 cos_sin(float angle) { return make_float2(cosf(angle), sinf(angle)); }
 
-__device__ __forceinline__ float2 rotary_cos_sin(const RotaryParams& r, int n, int pair) {
-  const float f = r.dtype == CASTLE_F32 ? reinterpret_cast<const float*>(r.freqs)[pair]
-                  : r.dtype == CASTLE_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(r.freqs)[pair])
-                                           : __half2float(reinterpret_cast<const __half*>(r.freqs)[pair]);
-  const float2 cs = cos_sin(__fmul_rn(__fadd_rn((float)n, r.position0), f));
+__device__ __forceinline__ float rotary_freq(const RotaryParams& r, int pair) {
+  return r.dtype == CASTLE_F32 ? reinterpret_cast<const float*>(r.freqs)[pair]
+         : r.dtype == CASTLE_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(r.freqs)[pair])
+                                  : __half2float(reinterpret_cast<const __half*>(r.freqs)[pair]);
+}
+__device__ __forceinline__ float2 rotary_cos_sin(const RotaryParams& r, int n, float freq) {
+  const float2 cs = cos_sin(__fmul_rn(__fadd_rn((float)n, r.position0), freq));
   return make_float2(cs.x, r.inverse ? -cs.y : cs.y);
 }
 

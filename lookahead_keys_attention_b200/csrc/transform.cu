@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kTransformThreads) castle_transform_kernel(con
   const int half = (ROT ? (p.src_d < p.dst_d ? p.src_d : p.dst_d) : 2) / 2;   // pairs of the rotated width
   if constexpr (ROT) {
     for (int i = threadIdx.x; i < nrows * half; i += kTransformThreads)
-      table[i] = rotary_cos_sin(p.rot, n0 + i / half, i % half);
+      table[i] = rotary_cos_sin(p.rot, n0 + i / half, rotary_freq(p.rot, i % half));
     __syncthreads();
   }
   const float mul = p.mul ? *p.mul : 1.f;
