@@ -145,7 +145,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   const uint32_t aQu = smem_u32(sQu), aKc = smem_u32(sKc), aQc = smem_u32(sQc), aVu = smem_u32(sVu),
                  aVc = smem_u32(sVc), adO = smem_u32(sdO), aKP = smem_u32(sKP), aVD = smem_u32(sVD),
                  aWb = smem_u32(sWb), aGb = smem_u32(sGb), aA = smem_u32(sA), aT = smem_u32(sT);
-  const float sl2 = p.scale * kLog2e;
+  const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
 
 #define MMA_WAIT()                       \
   mbar_wait(&bar_mma, ph_mma, abortp);   \
@@ -192,7 +192,10 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = sigmoid_t<T>(v[j] * p.scale);
+      for (int j = 0; j < 32; j += 2) {
+        const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), half_scale);
+        v[j] = a.x; v[j + 1] = a.y;
+      }
       if (diag) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
@@ -222,10 +225,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     BPHASE_MARK(4);
     {  // masked T (rows i, columns j <= i), unscaled
       float v[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+      tmem_ld32_lower(trow + C_S + c0, row, c0, v);
       store_row32<T>(sT, kPanelB, row, c0, v);
     }
     if (c0 < D) {  // 16-bit copy of the peeled state
@@ -258,11 +258,13 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
-        float su0 = v[j] * p.scale, su1 = v[j + 1] * p.scale;
-        float g0 = sigmoid_t<T>(su0), g1 = sigmoid_t<T>(su1);
-        v[j] = -v[j] * g0;          // -silu(su) / scale
-        v[j + 1] = -v[j + 1] * g1;
-        dpk[j / 2] = Elem<T>::pack2(g0 * (1.f + su0 * (1.f - g0)), g1 * (1.f + su1 * (1.f - g1)));
+        const float2 u = make_float2(v[j], v[j + 1]);
+        const float2 g = sigmoid2(u, half_scale);
+        // silu'(su) = g + silu(su) (1 - g)
+        const float2 q = mul2(mul2(u, g), splat(-1.f));   // -silu(su) / scale
+        v[j] = q.x; v[j + 1] = q.y;
+        const float2 d = fma2(mul2(q, splat(-p.scale)), fma2(g, splat(-1.f), splat(1.f)), g);
+        dpk[j / 2] = Elem<T>::pack2(d.x, d.y);
       }
       tmem_st32(trow + C_S + c0, v);
       tmem_st_wait();
@@ -284,7 +286,10 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = ex2_approx(fmaf(v[j], sl2, -lse_b));
+      for (int j = 0; j < 32; j += 2) {
+        const float2 x = fma2(make_float2(v[j], v[j + 1]), splat(sl2), splat(-lse_b));
+        v[j] = ex2_approx(x.x); v[j + 1] = ex2_approx(x.y);
+      }
       if (diag) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
@@ -317,11 +322,10 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
-        float2 pp = Elem<T>::unpack2(ppk[j / 2]);
-        float2 dd = Elem<T>::unpack2(dpk[j / 2]);
-        float ds0 = pp.x * (v[j] - delta_i), ds1 = pp.y * (v[j + 1] - delta_i);
-        v[j] = ds0; v[j + 1] = ds1;
-        w[j] = -ds0 * dd.x; w[j + 1] = -ds1 * dd.y;
+        const float2 ds = mul2(Elem<T>::unpack2(ppk[j / 2]), add2(make_float2(v[j], v[j + 1]), splat(-delta_i)));
+        const float2 du = mul2(ds, Elem<T>::unpack2(dpk[j / 2]));
+        v[j] = ds.x; v[j + 1] = ds.y;
+        w[j] = -du.x; w[j + 1] = -du.y;
       }
       store_row32<T>(sVD, kPanelB, row, c0, v);
       store_row32<T>(sKP, kPanelB, row, c0, w);
@@ -349,7 +353,11 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       load_row32<T>(sA, kPanelB, row, c0, a);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = v[j] * p.scale * a[j] * (1.f - a[j]);
+      for (int j = 0; j < 32; j += 2) {
+        const float2 g = make_float2(a[j], a[j + 1]);
+        const float2 x = mul2(mul2(make_float2(v[j], v[j + 1]), splat(p.scale)), fma2(mul2(g, splat(-1.f)), g, g));   // a (1 - a) = a - a a
+        v[j] = x.x; v[j + 1] = x.y;
+      }
       store_row32<T>(sT, kPanelB, row, c0, v);
     }
     SMEM_TO_MMA_SYNC();
@@ -372,10 +380,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     }
     {  // masked dT (rows i, columns j <= i) -> slot 3 (over dS)
       float v[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+      tmem_ld32_lower(trow + C_S + c0, row, c0, v);
       store_row32<T>(sVD, kPanelB, row, c0, v);
     }
     SMEM_TO_MMA_SYNC();

@@ -137,7 +137,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
   uint32_t ph_a = 0, ph_b = 0, ph_vu2 = 0, ph_mma = 0, ph_x = 0;
   const uint32_t a0 = smem_u32(s0), a1 = smem_u32(s1), a2 = smem_u32(s2), a3 = smem_u32(s3), a4 = smem_u32(s4),
                  a5 = smem_u32(s5), a6 = smem_u32(s6);
-  const float sl2 = p.scale * kLog2e;
+  const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
 
   for (int I = p.nblk - 1; I >= K; --I) {
     const int i0 = I * kBlkB, irow = i0 + row;
@@ -163,7 +163,10 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = sigmoid_t<T>(v[j] * p.scale);
+      for (int j = 0; j < 32; j += 2) {
+        const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), half_scale);
+        v[j] = a.x; v[j + 1] = a.y;
+      }
       if (diag) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
@@ -190,10 +193,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     B128_MARK(0, 4);
     {  // masked T -> s2 (over Vu); 16-bit copy of the peeled state -> s0 (over Qu)
       float v[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+      tmem_ld32_lower(trow + C_S + c0, row, c0, v);
       store_row32<T>(s2, kPanelB, row, c0, v);
       tmem_ld32(trow + C_W + c0, v);
       tmem_ld_wait();
@@ -219,11 +219,13 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
-        float su0 = v[j] * p.scale, su1 = v[j + 1] * p.scale;
-        float g0 = sigmoid_t<T>(su0), g1 = sigmoid_t<T>(su1);
-        v[j] = -v[j] * g0;
-        v[j + 1] = -v[j + 1] * g1;
-        dpk[j / 2] = Elem<T>::pack2(g0 * (1.f + su0 * (1.f - g0)), g1 * (1.f + su1 * (1.f - g1)));
+        const float2 u = make_float2(v[j], v[j + 1]);
+        const float2 g = sigmoid2(u, half_scale);
+        // silu'(su) = g + silu(su) (1 - g)
+        const float2 q = mul2(mul2(u, g), splat(-1.f));   // -silu(su) / scale
+        v[j] = q.x; v[j + 1] = q.y;
+        const float2 d = fma2(mul2(q, splat(-p.scale)), fma2(g, splat(-1.f), splat(1.f)), g);
+        dpk[j / 2] = Elem<T>::pack2(d.x, d.y);
       }
       tmem_st32(trow + C_S + c0, v);
       tmem_st_wait();
@@ -246,7 +248,10 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = ex2_approx(fmaf(v[j], sl2, -lse_b));
+      for (int j = 0; j < 32; j += 2) {
+        const float2 x = fma2(make_float2(v[j], v[j + 1]), splat(sl2), splat(-lse_b));
+        v[j] = ex2_approx(x.x); v[j + 1] = ex2_approx(x.y);
+      }
       if (diag) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
@@ -283,11 +288,10 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
-        float2 pp = Elem<T>::unpack2(ppk[j / 2]);
-        float2 dd = Elem<T>::unpack2(dpk[j / 2]);
-        float ds0 = pp.x * (v[j] - delta_i), ds1 = pp.y * (v[j + 1] - delta_i);
-        v[j] = ds0; v[j + 1] = ds1;
-        w[j] = -ds0 * dd.x; w[j + 1] = -ds1 * dd.y;
+        const float2 ds = mul2(Elem<T>::unpack2(ppk[j / 2]), add2(make_float2(v[j], v[j + 1]), splat(-delta_i)));
+        const float2 du = mul2(ds, Elem<T>::unpack2(dpk[j / 2]));
+        v[j] = ds.x; v[j + 1] = ds.y;
+        w[j] = -du.x; w[j + 1] = -du.y;
       }
       store_row32<T>(s5, kPanelB, row, c0, v);
       store_row32<T>(s6, kPanelB, row, c0, w);
@@ -307,10 +311,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     B128_MARK(0, 12);
     {  // masked dT -> s1 (over the gate)
       float v[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+      tmem_ld32_lower(trow + C_S + c0, row, c0, v);
       store_row32<T>(s1, kPanelB, row, c0, v);
     }
     if (storer) bulk_wait_read0();   // the copy of dSu has read its slot (the dqc staging goes there at the end of the step)
@@ -497,12 +498,13 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       load_row32<T>(sA, kPanelB, row, c0, a);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = v[j] * p.scale * a[j] * (1.f - a[j]);
+      for (int j = 0; j < 32; j += 2) {
+        const float2 g = make_float2(a[j], a[j + 1]);
+        const float2 x = mul2(mul2(make_float2(v[j], v[j + 1]), splat(p.scale)), fma2(mul2(g, splat(-1.f)), g, g));   // a (1 - a) = a - a a
+        v[j] = x.x; v[j + 1] = x.y;
+      }
       store_row32<T>(s3, kPanelB, row, c0, v);
-      tmem_ld32(trow + C_X + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+      tmem_ld32_lower(trow + C_X + c0, row, c0, v);
       store_row32<T>(s0, kPanelB, row, c0, v);
     }
     B128_SYNC();

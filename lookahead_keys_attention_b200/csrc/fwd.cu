@@ -160,7 +160,7 @@ castle_fwd_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   const uint32_t aQu = smem_u32(sQu), aKc = smem_u32(sKc), aVc = smem_u32(sVc), aQc = smem_u32(sQc),
                  aWb = smem_u32(sWb), aKuA = smem_u32(sKuA), aVuT = smem_u32(sVuT);
   const int krow = k0 + row;  // global key index of this thread's row when rows are keys
-  const float sl2 = p.scale * kLog2e;
+  const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
 
   for (int I = K; I < p.nblk; ++I) {
     const int i0 = I * kBlk;
@@ -200,7 +200,10 @@ castle_fwd_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       tmem_ld32(trow + COL_S + c0, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = sigmoid_t<T>(v[j] * p.scale);
+      for (int j = 0; j < 32; j += 2) {
+        const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), half_scale);
+        v[j] = a.x; v[j + 1] = a.y;
+      }
       if (diag) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
@@ -232,10 +235,7 @@ castle_fwd_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     PHASE_MARK(4);
     {  // masked T (j <= i), unscaled
       float v[32];
-      tmem_ld32(trow + COL_O + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+      tmem_ld32_lower(trow + COL_O + c0, row, c0, v);
       tmem_st_packed32<T>(trow + COL_T + c0 / 2, v);   // first operand of the Su correction
     }
     tmem_st_wait();
@@ -278,7 +278,11 @@ castle_fwd_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       tmem_ld32(trow + COL_O + c0, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = fmaf(-w[j], sigmoid_t<T>(w[j] * p.scale), v[j]);
+      for (int j = 0; j < 32; j += 2) {
+        const float2 u = make_float2(w[j], w[j + 1]);
+        const float2 x = fma2(u, neg_sigmoid2(u, half_scale), make_float2(v[j], v[j + 1]));
+        v[j] = x.x; v[j + 1] = x.y;
+      }
       if (diag) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : -INFINITY;
@@ -291,14 +295,15 @@ castle_fwd_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       mx = fmaxf(fmaxf(red_max[0][row], red_max[1][row]), fmaxf(red_max[2][row], red_max[3][row]));
       mrow = mx * p.scale;   // column 0 is never masked, so the maximum is finite
       const float mb = mx * sl2;
-      float lsum = 0.f;
+      float2 lsum = splat(0.f);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        float pe = ex2_approx(fmaf(v[j], sl2, -mb));   // exp(scale*v - max); masked entries give 0
-        lsum += pe;
-        v[j] = pe;
+      for (int j = 0; j < 32; j += 2) {
+        const float2 x = fma2(make_float2(v[j], v[j + 1]), splat(sl2), splat(-mb));
+        v[j] = ex2_approx(x.x);   // exp(scale*v - max); masked entries give 0
+        v[j + 1] = ex2_approx(x.y);
+        lsum = add2(lsum, make_float2(v[j], v[j + 1]));
       }
-      red_sum[cc][row] = lsum;
+      red_sum[cc][row] = lsum.x + lsum.y;
       tmem_st_packed32<T>(trow + COL_A + c0 / 2, v);   // P over the gate's packed copy, first operand of P @ Vc
     }
     tmem_st_wait();
@@ -521,7 +526,7 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
   const uint32_t aQu = smem_u32(sQu), aQV = smem_u32(sQV), aWb = smem_u32(sWb), aKuA = smem_u32(sKuA),
                  aVuT = smem_u32(sVuT);
   const int krow = k0 + row;
-  const float sl2 = p.scale * kLog2e;
+  const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
 
 #define F2_MMA_WAIT()                              \
   mbar_wait_lazy_abort(bar_mma, ph_mma, abortp);   \
@@ -569,7 +574,10 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
       tmem_ld32(trow + COL_S + c0, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = sigmoid_t<T>(v[j] * p.scale);
+      for (int j = 0; j < 32; j += 2) {
+        const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), half_scale);
+        v[j] = a.x; v[j + 1] = a.y;
+      }
       if (diag) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
@@ -614,10 +622,7 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
     for (int c = 0; c < NCH; ++c) {  // masked T (j <= i), unscaled; over Vu[I]
       const int c0 = cbase + c * 32;
       float v[32];
-      tmem_ld32(trow + COL_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+      tmem_ld32_lower(trow + COL_S + c0, row, c0, v);
       tmem_st_packed32<T>(trow + COL_O + c0 / 2, v);   // over the gate's packed copy, which the update has consumed
     }
     tmem_st_wait();
@@ -645,7 +650,11 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
       tmem_ld32(trow + COL_S + c0, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = -v[j] * sigmoid_t<T>(v[j] * p.scale);
+      for (int j = 0; j < 32; j += 2) {
+        const float2 u = make_float2(v[j], v[j + 1]);
+        const float2 x = mul2(u, neg_sigmoid2(u, half_scale));
+        v[j] = x.x; v[j + 1] = x.y;
+      }
       tmem_st32(trow + COL_S + c0, v);
     }
     if (grp < 2) {  // refresh the 16-bit copy of W (now including block I)
@@ -673,7 +682,8 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
       tma_load_4d(sQV, &m_vc, bar_vc, 0, k0, h, b);
     }
     const int irow = i0 + row;
-    float mrow, lsum = 0.f;
+    float mrow;
+    float2 lsum = splat(0.f);
     {
       float v[NCH][32];
 #pragma unroll
@@ -699,12 +709,14 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
 #pragma unroll
       for (int c = 0; c < NCH; ++c) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          v[c][j] = ex2_approx(fmaf(v[c][j], sl2, -mb));
-          lsum += v[c][j];
+        for (int j = 0; j < 32; j += 2) {
+          const float2 x = fma2(make_float2(v[c][j], v[c][j + 1]), splat(sl2), splat(-mb));
+          v[c][j] = ex2_approx(x.x);
+          v[c][j + 1] = ex2_approx(x.y);
+          lsum = add2(lsum, make_float2(v[c][j], v[c][j + 1]));
         }
       }
-      red_sum[grp][row] = lsum;
+      red_sum[grp][row] = lsum.x + lsum.y;
       // P as packed pairs over the first 64 columns of S: every thread of the row has its values in
       // registers since the barrier above, so the accumulator may be overwritten
 #pragma unroll

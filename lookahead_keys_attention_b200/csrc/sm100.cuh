@@ -299,12 +299,59 @@ __device__ __forceinline__ float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// sigmoid as one special-function op: 0.5 * tanh.approx(x / 2) + 0.5.  tanh.approx is good to about 2^-11,
-// i.e. the result to ~2.4e-4: below bf16 rounding (2e-3) and at the level of fp16 rounding (2.4e-4) of the
-// operand tiles the result is packed into.  (An exp-and-divide form costs two special-function ops.)
-template <typename T>
-__device__ __forceinline__ float sigmoid_t(float x) {
-  return fmaf(0.5f, tanh_approx(0.5f * x), 0.5f);
+// Packed fp32 arithmetic (two lanes of a register pair per instruction, the rounding of the single form): the passes
+// over score tiles are bound by instruction issue as much as by the special-function unit.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tadd.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\tfma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
+// sigmoid of a pair as one special-function op each: 0.5 * tanh.approx(x / 2) + 0.5, with `half_scale` = scale / 2 for
+// x = scale * v.  tanh.approx is good to about 2^-11, i.e. the result to ~2.4e-4: below bf16 rounding (2e-3) and at the
+// level of fp16 rounding (2.4e-4) of the operand tiles the result is packed into.  (An exp-and-divide form costs two
+// special-function ops.)
+__device__ __forceinline__ float2 sigmoid2(float2 v, float half_scale) {
+  const float2 x = mul2(v, splat(half_scale));
+  return fma2(make_float2(tanh_approx(x.x), tanh_approx(x.y)), splat(0.5f), splat(0.5f));
+}
+// -sigmoid, for products that want the sign
+__device__ __forceinline__ float2 neg_sigmoid2(float2 v, float half_scale) {
+  const float2 x = mul2(v, splat(half_scale));
+  return fma2(make_float2(tanh_approx(x.x), tanh_approx(x.y)), splat(-0.5f), splat(-0.5f));
+}
+
+// A 32-column chunk (from column c0) of a lower-triangular 128x128 tile, as one warp sees it: rows row0..row0+31.
+// Only the chunk on the diagonal needs a comparison per element.
+enum class Tri { kFull, kDiag, kZero };
+__device__ __forceinline__ Tri tri_chunk(int row0, int c0) { return c0 + 31 <= row0 ? Tri::kFull : c0 > row0 + 31 ? Tri::kZero : Tri::kDiag; }
+// tmem_ld32 of such a chunk with everything above the diagonal (column > row) zero
+__device__ __forceinline__ void tmem_ld32_lower(uint32_t taddr, int row, int c0, float* v) {
+  const Tri t = tri_chunk(row & ~31, c0);
+  if (t == Tri::kZero) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = 0.f;
+    return;
+  }
+  tmem_ld32(taddr, v);
+  tmem_ld_wait();
+  if (t == Tri::kDiag) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+  }
 }
 
 // Write 32 consecutive elements (columns c0..c0+31, c0 a multiple of 32) of row `row`
