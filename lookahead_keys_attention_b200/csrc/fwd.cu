@@ -30,7 +30,8 @@ struct FwdParams {
   int B, H, N, nblk;
   float scale;
   float* part_ml;   // [BH][ntiles][128][2]
-  void* part_o;     // [BH][ntiles][128][D] in the operand type (un-normalised P@Vc of one tile)
+  void* part_o;     // [BH][ntiles][D/8][128][8] in the operand type (un-normalised P@Vc of one tile): a thread that owns a
+                    // row stores 16-byte chunks, and a warp's store of one chunk is 512 contiguous bytes
   float* lse;       // [BH][N]
   float* w_state;   // [BH][N][D] or null
   castle_tensor_t u_out;  // ptr may be null
@@ -38,7 +39,7 @@ struct FwdParams {
   castle_tensor_t out;
   int32_t* status;
   int store_caches;   // also copy the Qu[K], Kc[K], Vc[K] tiles into the decode caches (prefill hand-off)
-  int split_q8;       // dim_head 64: walks of 8+ query blocks are cut after split_q8/256 of their length (0 = never)
+  uint4* tm;          // masked T tiles, or null
 #ifdef CASTLE_PHASE_TIMING
   long long* timing;
 #endif
@@ -48,364 +49,514 @@ __host__ __device__ inline int64_t tri(int64_t i) { return i * (i + 1) / 2; }
 
 constexpr int kFwdThreads = 512;
 
+constexpr int kSplitMin = 8;   // shorter walks are not cut
+// First step of part `seg` of a walk of `walk` query blocks cut in `nseg` parts of equal cost: a part pays c = 0.45 of a
+// step for each state-only step before it, so with parts beginning at x_i, c x_i + x_{i+1} - x_i is the same for all i.
+__device__ inline int walk_cut(int walk, int nseg, int seg) {
+  float a = 1.f, n = 1.f;
+  for (int i = 0; i < nseg; ++i) {
+    n *= 0.55f;
+    if (i < seg) a *= 0.55f;
+  }
+  return (int)((float)walk * (1.f - a) / (1.f - n) + 0.5f);
+}
+
 // Optional phase timing (debug builds only): thread 0 of CTA (0,0) stores clock64() at each phase
 // boundary of its first steps into the soft-max partial buffer's tail, which the host dumps.
 #ifdef CASTLE_PHASE_TIMING
 #define PHASE_MARK(i) do { if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && tstep < 8) p.timing[tstep * 16 + (i)] = clock64(); } while (0)
+#define PIPE_MARK(i) do { if ((tid & 31) == 0 && (tid == 0 || tid == 256) && blockIdx.x == 0 && blockIdx.y == 0 && I - I_begin < 16) p.timing[(I - I_begin) * 16 + (i)] = clock64(); } while (0)
 #else
 #define PHASE_MARK(i) do { } while (0)
+#define PIPE_MARK(i) do { } while (0)
 #endif
 
-// 512 threads: warp w works on TMEM lanes 32*(w%4).. (the hardware's rule) and on the
-// 32-column chunk w/4 of a 128-column accumulator, so thread (row, chunk) owns 32 values.
-template <typename T, int D>
+// ---------------------------------------------------------------------------------------------
+// Two-stage pipeline: the step (I,K) is cut into a lookahead stage, run by warps 0-7 (X), and a soft-max stage, run by
+// warps 8-15 (Y), and Y works on block I while X is on block I+1.  The chain between consecutive query blocks is only
+// the state update, so the two overlap: X forms Z and the gate and issues every product up to the scores; Y turns Su
+// and Sc into P, issues P @ Vc and stores the partial.  One CTA per SM; a group has 256 threads, each with 64 values
+// of a 128x128 tile.
+//
+// The masked T[I,I] = tril(Qc[I] @ Vu[I]^T) is the same for every key block, so from four query blocks on a small kernel
+// computes the tiles once (castle_fwd_t_kernel) and X's threads carry theirs from global memory to tensor memory; that
+// takes a product, an elementwise pass and two hand-offs out of X's chain.  Below that (TM = false) X forms T itself.
+//
+// Tensor memory: W | R1 | R2 | R3 (| Tm), D + 3 * 128 (+ 64) columns.
+//   R1  Z; at dim_head 128 then the masked T as packed pairs (first operand of the Su correction)
+//   R2  Su; at dim_head 128 then P @ Vc
+//   R3  Sc (issued by Y, as soon as these columns are free again), then P as packed pairs; at dim_head 64 its upper half
+//       then takes P @ Vc
+//
+// Shared memory: Qu, Kc, Vc of the key block and the 16-bit copy of W stay.  dim_head 64: two buffers each of Ku, Vu, Qc
+// and the gate, filled a step ahead.  dim_head 128: one of Qc and two 32 KB slots whose roles alternate: in step I slot P
+// holds Ku[I] and, once Z is done, the gate over it; slot Q holds Vu[I] and then, after the state update, Ku[I+1];
+// Vu[I+1] goes over the gate when the scores are done.
+template <int D> struct FwdPipe {
+  static constexpr uint32_t OPB = D / 64 * kPanelBytes;
+  static constexpr uint32_t kRed = 224 * 1024;                  // row max and row sum of the two column halves
+  static constexpr uint32_t kBars = kRed + 4 * kBlk * sizeof(float);
+  static constexpr uint32_t kSmem = kBars + 192;
+};
+
+__device__ __forceinline__ void sync_x() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// The two warps of a group that share 32 rows (and their tensor-memory lanes).
+__device__ __forceinline__ void sync_pair(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void sync_y() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
+
+// 32 values of a row as the state or the lookahead keys (fp32, bf16 or fp16)
+__device__ __forceinline__ void store_u32(void* base, int dtype, int64_t off, const float* v) {
+  if (dtype == CASTLE_F32) {
+    float* dst = reinterpret_cast<float*>(base) + off;
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+  } else {
+    uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(base) + off);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        q[i] = dtype == CASTLE_BF16 ? Elem<__nv_bfloat16>::pack2(v[8 * j + 2 * i], v[8 * j + 2 * i + 1])
+                                    : Elem<__half>::pack2(v[8 * j + 2 * i], v[8 * j + 2 * i + 1]);
+      dst[j] = make_uint4(q[0], q[1], q[2], q[3]);
+    }
+  }
+}
+
+// A masked T tile in global memory: [16 chunks of 8 columns][128 rows] x 16 bytes, so that a warp's access is contiguous.
+constexpr int64_t kTmTile = 16 * kBlk;   // in uint4
+constexpr int kTmBlocks = 4;             // from so many query blocks on the tiles are computed once, up front
+
+template <typename T, int D, bool TM>
 __global__ void __launch_bounds__(kFwdThreads, 1)
-castle_fwd_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
-                  const __grid_constant__ CUtensorMap m_vc, const __grid_constant__ CUtensorMap m_qu,
-                  const __grid_constant__ CUtensorMap m_ku, const __grid_constant__ CUtensorMap m_vu,
-                  const __grid_constant__ CUtensorMap m_quc, const __grid_constant__ CUtensorMap m_kcc,
-                  const __grid_constant__ CUtensorMap m_vcc) {
-  constexpr int NP = D / 64;                         // panels per d-wide operand
-  constexpr uint32_t OPB = NP * kPanelBytes;         // bytes of a d-wide operand tile
-  constexpr uint32_t SQB = 2 * kPanelBytes;          // bytes of a 128x128 tile
-  constexpr uint32_t TM_COLS = (D == 64) ? 256 : 512;
-  static_assert(D == 128, "laid out for dim_head 128 (512 tensor-memory columns)");
-  // accumulators W | S | O, then two 64-column areas for tiles the threads hand to the tensor cores as
-  // packed 16-bit pairs (first operands read from tensor memory): the gate, later P; and the masked T
-  constexpr uint32_t COL_W = 0, COL_S = D, COL_O = D + 128, COL_A = D + 256, COL_T = D + 320;
+castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
+                       const __grid_constant__ CUtensorMap m_vc, const __grid_constant__ CUtensorMap m_qu,
+                       const __grid_constant__ CUtensorMap m_ku, const __grid_constant__ CUtensorMap m_vu,
+                       const __grid_constant__ CUtensorMap m_quc, const __grid_constant__ CUtensorMap m_kcc,
+                       const __grid_constant__ CUtensorMap m_vcc) {
+  using L = FwdPipe<D>;
+  constexpr int NP = D / 64;
+  constexpr bool B2 = D == 64;   // two buffers of everything that is streamed
+  constexpr uint32_t OPB = L::OPB;
+  constexpr uint32_t C_W = 0, C_R1 = D, C_R2 = D + 128, C_R3 = D + 256;
+  constexpr uint32_t C_O = B2 ? C_R3 + 64 : C_R2, C_TM = B2 ? C_R3 + 128 : C_R1;
   constexpr int FMT = Elem<T>::fmt;
   constexpr uint32_t ID_SQ = make_idesc(128, 128, FMT, false, false, false);
   constexpr uint32_t ID_D = make_idesc(128, D, FMT, false, true, false);
   constexpr float kLog2e = 1.4426950408889634f;
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sQu = smem;
-  uint8_t* sKc = sQu + OPB;
-  uint8_t* sVc = sKc + OPB;
-  uint8_t* sQc = sVc + OPB;
-  uint8_t* sWb = sQc + OPB;
-  uint8_t* sKuA = sWb + OPB;   // Ku[I], then the gate A[K,I]; Ku[I+1] arrives once Su is done
-  uint8_t* sVuT = sKuA + SQB;  // Vu[I]; Vu[I+1] arrives once Su (whose commit covers the state update) is done
-  // row max / row sum exchange between the four threads of a row: 4 KB over Qc[I], which is dead
-  // once the last product reading it (Sc) has completed and until the next step's TMA load
-  float (*red_max)[kBlk] = reinterpret_cast<float (*)[kBlk]>(sQc);
-  float (*red_sum)[kBlk] = reinterpret_cast<float (*)[kBlk]>(sQc + 4 * kBlk * sizeof(float));
-  __shared__ uint64_t bar_res, bar_ku, bar_vu, bar_qc, bar_mma, bar_z;
-  __shared__ uint32_t tmem_base_s;
-  __shared__ int abort_flag;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t *sQu = smem, *sKc = sQu + OPB, *sVc = sKc + OPB, *sWb = sVc + OPB, *sStream = sWb + OPB;
+  // streamed tiles; n counts steps from K
+  auto sKu = [&](int n) { return B2 ? sStream + 65536 + (n & 1) * OPB : sStream + OPB + (n & 1) * 32768; };
+  auto sVu = [&](int n) { return B2 ? sStream + 65536 + 2 * OPB + (n & 1) * OPB : sStream + OPB + ((n + 1) & 1) * 32768; };
+  auto sQc = [&](int n) { return B2 ? sStream + 65536 + 4 * OPB + (n & 1) * OPB : sStream; };
+  auto sA = [&](int n) { return B2 ? sStream + (n & 1) * 32768 : sStream + OPB + (n & 1) * 32768; };
+  float (*red_max)[kBlk] = reinterpret_cast<float (*)[kBlk]>(smem + L::kRed);
+  float (*red_sum)[kBlk] = red_max + 2;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
+  // loads: the resident tiles and Ku of the first step; Vu[I], Qc[I] (and, with two buffers, Ku[I+1]) of a step; Ku[I+1]
+  uint64_t *bar_res = bars, *bar_in = bars + 1, *bar_ku = bars + 3;
+  uint64_t *bar_z = bars + 7, *bar_t = bars + 8, *bar_w = bars + 9, *bar_s = bars + 10, *bar_o = bars + 11;
+  uint64_t* bar_r = bars + 12;   // Y has read R2: Su or, at dim_head 128, P @ Vc (one arrival per warp)
+  uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + 14);
+  int* abort_flag = reinterpret_cast<int*>(bars + 15);
+  volatile int* abortp = abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, cc = warp >> 2;
-  const int row = quarter * 32 + lane;   // accumulator row (TMEM lane) of this thread
-  const int c0 = cc * 32;                // first of its 32 columns
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: uniform for the compiler, too
+  const int quarter = warp & 3, grp = (warp >> 2) & 1;   // TMEM lanes 32 * quarter.., columns 64 * grp.. of a score tile
+  const int row = quarter * 32 + lane, cbase = grp * 64;
   const int bh = blockIdx.x, K = blockIdx.y;
   const int b = bh / p.H, h = bh % p.H;
   const int k0 = K * kBlk;
+  // Walk segments (gridDim.z parts, later ones first in the grid): the CTA of a later part first rebuilds the state it
+  // would have inherited in state-only steps (Z, gate, W += A @ Vu).
+  const int walk = p.nblk - K, nseg = walk >= kSplitMin ? (int)gridDim.z : 1, seg = (int)gridDim.z - 1 - (int)blockIdx.z;
+  if (seg >= nseg) return;
+  const int I_begin = K + walk_cut(walk, nseg, seg), I_end = K + walk_cut(walk, nseg, seg + 1);
 
+  if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need 1024-byte alignment
+    if (tid == 0) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
+    return;
+  }
   if (tid == 0) {
-    mbar_init(&bar_res, 1);
-    mbar_init(&bar_ku, 1);
-    mbar_init(&bar_vu, 1);
-    mbar_init(&bar_qc, 1);
-    mbar_init(&bar_z, 1);
-    mbar_init(&bar_mma, 1);
+    for (int i = 0; i < 12; ++i) mbar_init(bars + i, bars + i == bar_s ? 2 : 1);   // the scores: Su by X, Sc by Y
+    mbar_init(bar_r, 8);
     mbar_fence_init();
-    abort_flag = 0;
+    *abort_flag = 0;
     tma_prefetch_desc(&m_qc); tma_prefetch_desc(&m_ku); tma_prefetch_desc(&m_vu);
   }
-  if (warp == 0) { tmem_alloc(&tmem_base_s, TM_COLS); tmem_relinquish(); }
+  if (warp == 0) { tmem_alloc(tmem_base_s, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
+  const uint32_t tmem = *tmem_base_s;
   const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-  volatile int* abortp = &abort_flag;
+  const uint32_t aQu = smem_u32(sQu), aKc = smem_u32(sKc), aVc = smem_u32(sVc), aWb = smem_u32(sWb);
+  const float half_scale = 0.5f * p.scale;
 
-  if (tid == 0) {
-    mbar_expect_tx(&bar_res, 3 * OPB);
+  auto load = [&](uint8_t* dst, const CUtensorMap& m, uint64_t* bar, int r0) {   // one d-wide tile
 #pragma unroll
-    for (int pn = 0; pn < NP; ++pn) {
-      tma_load_4d(sQu + pn * kPanelBytes, &m_qu, &bar_res, pn * 64, k0, h, b);
-      tma_load_4d(sKc + pn * kPanelBytes, &m_kc, &bar_res, pn * 64, k0, h, b);
-      tma_load_4d(sVc + pn * kPanelBytes, &m_vc, &bar_res, pn * 64, k0, h, b);
-    }
-    // the first block's tiles; later blocks are fetched inside the step before, each as soon as its
-    // slot dies (a tile takes 2-4 thousand cycles from issue to arrival)
-    mbar_expect_tx(&bar_ku, OPB);
-    mbar_expect_tx(&bar_vu, OPB);
-    mbar_expect_tx(&bar_qc, OPB);
+    for (int pn = 0; pn < NP; ++pn) tma_load_4d(dst + pn * kPanelBytes, &m, bar, pn * 64, r0, h, b);
+  };
+  // what step n reads: one barrier (two buffers: alternating)
+  auto in_bar = [&](int n) { return B2 ? bar_in + (n & 1) : bar_in; };
+  auto in_par = [&](int n) { return (uint32_t)(B2 ? n >> 1 : n) & 1u; };
+  auto load_step = [&](int n) {
+    const int I = K + n;
+    const bool qc = I >= I_begin, ku = B2 && I + 1 < I_end;
+    uint64_t* bar = in_bar(n);
+    mbar_expect_tx(bar, OPB * (1 + qc + ku));
+    if (ku) load(sKu(n + 1), m_ku, bar, (I + 1) * kBlk);
+    load(sVu(n), m_vu, bar, I * kBlk);
+    if (qc) load(sQc(n), m_qc, bar, I * kBlk);
+  };
+  // One polling lane per warp: a barrier over the group behind a single poll holds every warp up for the issuing one, and
+  // 32 polling lanes take issue slots from the group that is working (735 against 820 and 751 us at B=4 N=4096 H=16).
+  auto wait_warp = [&](uint64_t* bar, uint32_t parity) { if (elect_one()) mbar_wait_lazy_abort(bar, parity, abortp); __syncwarp(); tc_fence_after(); };
+
+  if (warp < 8) {
+    // ============================================================ X: lookahead stage
+    if (warp == 0 && elect_one()) {
+      mbar_expect_tx(bar_res, 4 * OPB);
+      load(sQu, m_qu, bar_res, k0);
+      load(sKu(0), m_ku, bar_res, k0);
+      load_step(0);
+      load(sKc, m_kc, bar_res, k0);
+      load(sVc, m_vc, bar_res, k0);
+      mbar_wait(bar_res, 0, abortp);
+      tc_fence_after();
+      gemm_kk_t<NP>(tmem + C_R1, aQu, smem_u32(sKu(0)), ID_SQ, false);
+      mma_commit(bar_z);
+      // Prefill hand-off: the resident tiles are the rows the decode caches hold for this key block.
+      if (p.store_caches && seg == 0 && !*abortp) {
 #pragma unroll
-    for (int pn = 0; pn < NP; ++pn) {
-      tma_load_4d(sKuA + pn * kPanelBytes, &m_ku, &bar_ku, pn * 64, k0, h, b);
-      tma_load_4d(sVuT + pn * kPanelBytes, &m_vu, &bar_vu, pn * 64, k0, h, b);
-      tma_load_4d(sQc + pn * kPanelBytes, &m_qc, &bar_qc, pn * 64, k0, h, b);
+        for (int pn = 0; pn < NP; ++pn) {
+          tma_store_4d(&m_quc, sQu + pn * kPanelBytes, pn * 64, k0, h, b);
+          tma_store_4d(&m_kcc, sKc + pn * kPanelBytes, pn * 64, k0, h, b);
+          tma_store_4d(&m_vcc, sVc + pn * kPanelBytes, pn * 64, k0, h, b);
+        }
+        bulk_commit();
+      }
     }
-  }
-  mbar_wait(&bar_res, 0, abortp);
-  // Prefill hand-off: the resident tiles of this key block are exactly the rows the decode caches hold for
-  // it, so they go there straight from shared memory (the slots are never overwritten; the stores are
-  // awaited before the CTA exits).
-  if (p.store_caches && tid == 0 && !*abortp) {
+    for (int I = K; I < I_end; ++I) {
+      const int n = I - K;
+      const bool diag = I == K, pre = I < I_begin, more = I + 1 < I_end, again = I > I_begin;
+      const uint32_t ph = n & 1, ph_m = (I - I_begin) & 1;   // barriers that complete in every step; in full steps only
+      const uint32_t aA = smem_u32(sA(n)), aVu = smem_u32(sVu(n)), aQc = smem_u32(sQc(n)), aKn = smem_u32(sKu(n + 1));
+
+      uint4 tq[8];   // this thread's 64 values of the masked T, on their way during the gate
+      if (TM && !pre) {
+        const uint4* src = p.tm + ((int64_t)bh * p.nblk + I) * kTmTile + (cbase / 8) * kBlk + row;
 #pragma unroll
-    for (int pn = 0; pn < NP; ++pn) {
-      tma_store_4d(&m_quc, sQu + pn * kPanelBytes, pn * 64, k0, h, b);
-      tma_store_4d(&m_kcc, sKc + pn * kPanelBytes, pn * 64, k0, h, b);
-      tma_store_4d(&m_vcc, sVc + pn * kPanelBytes, pn * 64, k0, h, b);
-    }
-    bulk_commit();
-  }
+        for (int q = 0; q < 8; ++q) tq[q] = __ldg(src + q * kBlk);
+      }
+      // ---- gate A = sigmoid(scale * Z), kept for j > k (rows k, columns j)
+      wait_warp(bar_z, ph);
+      PIPE_MARK(0);
+      {
+        float v[2][32];
+        tmem_ld32(trow + C_R1 + cbase, v[0]);
+        tmem_ld32(trow + C_R1 + cbase + 32, v[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float2 a = sigmoid2(make_float2(v[c][j], v[c][j + 1]), half_scale);
+            v[c][j] = a.x; v[c][j + 1] = a.y;
+          }
+          if (diag) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[c][j] = (cbase + c * 32 + j > row) ? v[c][j] : 0.f;
+          }
+          store_row32<T>(sA(n), kPanelBytes, row, cbase + c * 32, v[c]);
+        }
+      }
+      PIPE_MARK(1);
+      if (B2) {
+        // Y has the scores of the step before, so its products are done: its buffers are filled for the next one
+        if (again) wait_warp(bar_r, ph_m ^ 1);
+        if (more && warp == 1 && elect_one()) load_step(n + 1);
+        __syncwarp();
+      }
+      if (!pre) {   // the 16-bit copy of W (before this step's update)
+#pragma unroll
+        for (int c = 0; c < NP; ++c) {
+          const int c0 = (grp * NP + c) * 32;
+          float v[32];
+          tmem_ld32(trow + C_W + c0, v);
+          tmem_ld_wait();
+          store_row32<T>(sWb, kPanelBytes, row, c0, v);
+        }
+      }
+      if (TM && !pre) {
+        if (!B2) { tc_fence_before(); sync_pair(3 + quarter); tc_fence_after(); }   // the masked T goes over Z
+#pragma unroll
+        for (int c = 0; c < 2; ++c) tmem_st16(trow + C_TM + cbase / 2 + c * 16, reinterpret_cast<const uint32_t*>(tq + 4 * c));
+        tmem_st_wait();
+      }
+      fence_async_smem();
+      tc_fence_before();
+      // what the products below read is waited for here, by another warp than the issuing one
+      if (warp == 1 && elect_one()) mbar_wait_lazy_abort(in_bar(n), in_par(n), abortp);
+      __syncwarp();
+      sync_x();
+      PIPE_MARK(2);
+      if (!TM && !pre) {
+        // ---- T[I,I] = Qc[I] @ Vu[I]^T over Z, masked (j <= i) into packed pairs
+        if (warp == 0 && elect_one()) {
+          tc_fence_after();
+          gemm_kk_t<NP>(tmem + C_R1, aQc, aVu, ID_SQ, false);
+          mma_commit(bar_t);
+        }
+        wait_warp(bar_t, ph_m);
+        float v[2][32];
+        tmem_ld32_lower(trow + C_R1 + cbase, row, cbase, v[0]);
+        tmem_ld32_lower(trow + C_R1 + cbase + 32, row, cbase + 32, v[1]);
+        if (!B2) { tc_fence_before(); sync_pair(3 + quarter); tc_fence_after(); }   // the rows' T is in registers
+        tmem_st_packed32<T>(trow + C_TM + cbase / 2, v[0]);
+        tmem_st_packed32<T>(trow + C_TM + cbase / 2 + 16, v[1]);
+        tmem_st_wait();
+        tc_fence_before();
+        sync_x();
+      }
 
-  uint32_t ph_load = 0, ph_mma = 0, ph_z = 0;
-  const uint32_t aQu = smem_u32(sQu), aKc = smem_u32(sKc), aVc = smem_u32(sVc), aQc = smem_u32(sQc),
-                 aWb = smem_u32(sWb), aKuA = smem_u32(sKuA), aVuT = smem_u32(sVuT);
-  const int krow = k0 + row;  // global key index of this thread's row when rows are keys
-  const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
-
-  for (int I = K; I < p.nblk; ++I) {
-    const int i0 = I * kBlk;
-    const bool diag = (I == K);
-#ifdef CASTLE_PHASE_TIMING
-    const int tstep = I - K;
-#endif
-    PHASE_MARK(0);
-    const bool more = I + 1 < p.nblk;
-    const int in0 = i0 + kBlk;
-    // Qc[I] goes into its slot only now: that slot doubled as the soft-max exchange buffer until the end
-    // of the step before.  It is needed at the second product phase.  One panel per lane of two warps
-    // (a TMA instruction costs its issuing thread ~150 cycles); the barrier was armed in the step before.
-    if (I > K && lane == 0 && warp >= 4 && warp < 4 + NP)
-      tma_load_4d(sQc + (warp - 4) * kPanelBytes, &m_qc, &bar_qc, (warp - 4) * 64, i0, h, b);
-
-    // ---- Z[K,I] = Qu[K] @ Ku[I]^T  (rows = keys k, columns = positions j)
-    // After the first step this product was already issued behind P @ Vc of the step before (see there).
-    if (diag) {
-      if (tid == 0) {
-        mbar_wait(&bar_ku, ph_load, abortp);
-        PHASE_MARK(1);
+      // ---- W_K += A @ Vu[I];  Su/scale = Qc[I] @ Wb^T + Tm @ A^T;  Z of the next step
+      if (warp == 0 && elect_one()) {
         tc_fence_after();
-        gemm_kk_t<NP>(tmem + COL_S, aQu, aKuA, ID_SQ, false);
-        mma_commit(&bar_mma);
+        if (B2 && more && !pre) {   // R1 has been read: Z first, the next gate waits for nothing else
+          gemm_kk_t<NP>(tmem + C_R1, aQu, aKn, ID_SQ, false);
+          mma_commit(bar_z);
+        }
+        PIPE_MARK(7);
+        gemm_km_t<8>(tmem + C_W, aA, aVu, ID_D, !diag);
+        mma_commit(bar_w);
+        PIPE_MARK(14);
+        if (!pre) {
+          if (!B2 && again) { mbar_wait(bar_r, ph_m ^ 1, abortp); tc_fence_after(); }
+          PIPE_MARK(3);
+          if (!diag) gemm_kk_t<NP>(tmem + C_R2, aQc, aWb, ID_SQ, false);
+          gemm_tk_t<2>(tmem + C_R2, tmem + C_TM, aA, ID_SQ, !diag);
+          mma_commit(bar_s);
+          if (!again) {   // the first Sc (later ones are Y's)
+            gemm_kk_t<NP>(tmem + C_R3, aQc, aKc, ID_SQ, false);
+            mma_commit(bar_s);
+          }
+          PIPE_MARK(5);
+        }
+        if (more && (!B2 || pre)) {   // (state-only steps: behind the update, so that it covers the update too)
+          if (!B2) { mbar_wait(bar_ku, ph, abortp); tc_fence_after(); }
+          gemm_kk_t<NP>(tmem + C_R1, aQu, aKn, ID_SQ, false);
+          mma_commit(bar_z);
+        }
       }
-      mbar_wait(&bar_mma, ph_mma, abortp);
-      ph_mma ^= 1;
-    } else {
-      mbar_wait(&bar_z, ph_z, abortp);
-      ph_z ^= 1;
-    }
-    tc_fence_after();
-    PHASE_MARK(2);
-    {  // gate A = sigmoid(scale * Z), kept for j > k; written over Ku[I]
-      float v[32];
-      tmem_ld32(trow + COL_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), half_scale);
-        v[j] = a.x; v[j + 1] = a.y;
+      if (!B2 && more && warp == 1 && elect_one()) {
+        mbar_wait(bar_w, ph, abortp);   // Vu[I] is consumed by the update: Ku[I+1] over it
+        mbar_expect_tx(bar_ku, OPB);
+        load(sKu(n + 1), m_ku, bar_ku, (I + 1) * kBlk);
+        if (!pre) mbar_wait(bar_s, ph_m, abortp);   // the gate and Qc[I] are consumed by the scores
+        load_step(n + 1);
       }
-      if (diag) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
+      if (!B2) __syncwarp();
+    }
+    // ---- W_K is now U[K] (in the CTA that walked to the last query block)
+    if (I_end == p.nblk && (p.u_out.ptr != nullptr || p.w_state != nullptr)) {
+      wait_warp(bar_w, (uint32_t)(I_end - 1 - K) & 1u);
+#pragma unroll 1
+      for (int c = 0; c < NP; ++c) {
+        const int c0 = (grp * NP + c) * 32;
+        float v[32];
+        tmem_ld32(trow + C_W + c0, v);
+        tmem_ld_wait();
+        if (k0 + row < p.N) {   // (the load is the whole warp's)
+          if (p.w_state != nullptr) store_u32(p.w_state, CASTLE_F32, ((int64_t)bh * p.N + k0 + row) * D + c0, v);
+          if (p.u_out.ptr != nullptr)
+            store_u32(p.u_out.ptr, p.u_dtype, b * p.u_out.stride_b + h * p.u_out.stride_h + (int64_t)(k0 + row) * p.u_out.stride_n + c0, v);
+        }
       }
-      store_row32<T>(sKuA, kPanelBytes, row, c0, v);   // operand of the Su correction (read along rows)
-      tmem_st_packed32<T>(trow + COL_A + c0 / 2, v);   // first operand of the state update
     }
-    tmem_st_wait();
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    PHASE_MARK(3);
-
-    // ---- W_K += A @ Vu[I]   and   T[I,I] = Qc[I] @ Vu[I]^T
-    if (tid == 0) {
-      mbar_wait(&bar_vu, ph_load, abortp);
-      mbar_wait(&bar_qc, ph_load, abortp);
-      tc_fence_after();
-      // T goes into O's columns (free until P @ Vc) and is committed alone: masking it overlaps the state
-      // update and the part of Su that does not need the masked T, which the next commit covers
-      gemm_kk_t<NP>(tmem + COL_O, aQc, aVuT, ID_SQ, false);
-      mma_commit(&bar_mma);
-      gemm_tm_t<8>(tmem + COL_W, tmem + COL_A, aVuT, ID_D, !diag);
-      if (!diag) gemm_kk_t<NP>(tmem + COL_S, aQc, aWb, ID_SQ, false);
-    }
-    mbar_wait(&bar_mma, ph_mma, abortp);
-    ph_mma ^= 1;
-    tc_fence_after();
-    PHASE_MARK(4);
-    {  // masked T (j <= i), unscaled
-      float v[32];
-      tmem_ld32_lower(trow + COL_O + c0, row, c0, v);
-      tmem_st_packed32<T>(trow + COL_T + c0 / 2, v);   // first operand of the Su correction
-    }
-    tmem_st_wait();
-    tc_fence_before();
-    __syncthreads();
-    PHASE_MARK(5);
-
-    // ---- Su/scale = Qc[I] @ Wb^T + Tm @ A^T   (Wb = 16-bit copy of W before this step's update)
-    if (tid == 0) {
-      tc_fence_after();
-      if (more) { mbar_expect_tx(&bar_ku, OPB); mbar_expect_tx(&bar_vu, OPB); }   // loads issued below by other lanes
-      gemm_tk_t<2>(tmem + COL_S, tmem + COL_T, aKuA, ID_SQ, !diag);
-      // the causal score Sc/scale = Qc[I] @ Kc[K]^T beside it, in O's columns (the masked T is consumed, P @ Vc
-      // comes later): one pass then forms S = Sc - silu(Su) and the soft-max numerators
-      gemm_kk_t<NP>(tmem + COL_O, aQc, aKc, ID_SQ, false);
-      mma_commit(&bar_mma);
-    }
-    mbar_wait(&bar_mma, ph_mma, abortp);
-    ph_mma ^= 1;
-    tc_fence_after();
-    PHASE_MARK(6);
-    // the gate, and Vu[I] with the state update, are consumed: Ku[I+1] and Vu[I+1] -> their slots
-    if (more && lane == 0 && warp >= 4 && warp < 4 + NP)
-      tma_load_4d(sKuA + (warp - 4) * kPanelBytes, &m_ku, &bar_ku, (warp - 4) * 64, in0, h, b);
-    if (more && lane == 0 && warp >= 8 && warp < 8 + NP)
-      tma_load_4d(sVuT + (warp - 8) * kPanelBytes, &m_vu, &bar_vu, (warp - 8) * 64, in0, h, b);
-    if (c0 < D) {  // refresh the 16-bit copy of W (now including block I) for the next step
-      float v[32];
-      tmem_ld32(trow + COL_W + c0, v);
-      tmem_ld_wait();
-      store_row32<T>(sWb, kPanelBytes, row, c0, v);
-    }
-    // S/scale = Sc/scale - silu(Su)/scale, row max over the four column chunks, then P = exp(S - max)
-    // (rows = queries i, columns = keys k)
-    const int irow = i0 + row;
-    float mrow;
-    {
-      float v[32], w[32];
-      tmem_ld32(trow + COL_S + c0, w);
-      tmem_ld32(trow + COL_O + c0, v);
-      tmem_ld_wait();
+    if (p.store_caches && warp == 0 && elect_one()) bulk_wait0();
+  } else {
+    // ============================================================ Y: soft-max stage
+    const float sl2 = p.scale * kLog2e;
+    auto issue_sc = [&](int I) {   // Sc/scale = Qc[I] @ Kc[K]^T
+      if (I < I_end && warp == 8 && elect_one()) {
+        tc_fence_after();
+        gemm_kk_t<NP>(tmem + C_R3, smem_u32(sQc(I - K)), aKc, ID_SQ, false);
+        mma_commit(bar_s);
+      }
+      __syncwarp();
+    };
+    if (warp == 8 && elect_one()) mbar_wait(bar_res, 0, abortp);   // Kc, Vc
+    __syncwarp();
+    for (int I = I_begin; I < I_end; ++I) {
+      const uint32_t ph_m = (I - I_begin) & 1;
+      const bool diag = I == K;
+      const int irow = I * kBlk + row;
+      wait_warp(bar_s, ph_m);
+      PIPE_MARK(8);
+      // S/scale = Sc/scale - silu(Su)/scale (rows i, columns k); Su comes in pieces of 16 columns, one ahead of the arithmetic
+      float s[2][32];
+      {
+        float w[2][16];
+        tmem_ld16(trow + C_R2 + cbase, w[0]);
+        tmem_ld32(trow + C_R3 + cbase, s[0]);
+        tmem_ld32(trow + C_R3 + cbase + 32, s[1]);
+        tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 u = make_float2(w[j], w[j + 1]);
-        const float2 x = fma2(u, neg_sigmoid2(u, half_scale), make_float2(v[j], v[j + 1]));
-        v[j] = x.x; v[j + 1] = x.y;
+        for (int q = 0; q < 4; ++q) {
+          if (q < 3) tmem_ld16(trow + C_R2 + cbase + 16 * (q + 1), w[(q + 1) & 1]);
+          float* sq = &s[q >> 1][(q & 1) * 16];
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {
+            const float2 u = make_float2(w[q & 1][j], w[q & 1][j + 1]);
+            const float2 x = fma2(u, neg_sigmoid2(u, half_scale), make_float2(sq[j], sq[j + 1]));
+            sq[j] = x.x; sq[j + 1] = x.y;
+          }
+          if (q < 3) tmem_ld_wait();
+        }
+      }
+      tc_fence_before();
+      if (B2) {   // Su is in registers; at dim_head 128 its columns take P @ Vc first
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_r);
       }
       if (diag) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : -INFINITY;
-      }
-      float mx = v[0];
+        for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int j = 1; j < 32; ++j) mx = fmaxf(mx, v[j]);
-      red_max[cc][row] = mx;
-      __syncthreads();
-      mx = fmaxf(fmaxf(red_max[0][row], red_max[1][row]), fmaxf(red_max[2][row], red_max[3][row]));
-      mrow = mx * p.scale;   // column 0 is never masked, so the maximum is finite
+          for (int j = 0; j < 32; ++j) s[c][j] = (cbase + c * 32 + j <= row) ? s[c][j] : -INFINITY;
+      }
+      float mx = s[0][0];
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int j = 0; j < 32; ++j) mx = fmaxf(mx, s[c][j]);
+      red_max[grp][row] = mx;
+      PIPE_MARK(9);
+      sync_pair(7 + quarter);
+      tc_fence_after();
+      mx = fmaxf(mx, red_max[grp ^ 1][row]);   // column 0 is never masked, so the maximum is finite
       const float mb = mx * sl2;
       float2 lsum = splat(0.f);
 #pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 x = fma2(make_float2(v[j], v[j + 1]), splat(sl2), splat(-mb));
-        v[j] = ex2_approx(x.x);   // exp(scale*v - max); masked entries give 0
-        v[j + 1] = ex2_approx(x.y);
-        lsum = add2(lsum, make_float2(v[j], v[j + 1]));
+      for (int c = 0; c < 2; ++c) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 x = fma2(make_float2(s[c][j], s[c][j + 1]), splat(sl2), splat(-mb));
+          s[c][j] = ex2_approx(x.x);   // exp(scale*v - max); masked entries give 0
+          s[c][j + 1] = ex2_approx(x.y);
+          lsum = add2(lsum, make_float2(s[c][j], s[c][j + 1]));
+        }
+        tmem_st_packed32<T>(trow + C_R3 + cbase / 2 + c * 16, s[c]);   // P over Sc, which everybody has read
       }
-      red_sum[cc][row] = lsum.x + lsum.y;
-      tmem_st_packed32<T>(trow + COL_A + c0 / 2, v);   // P over the gate's packed copy, first operand of P @ Vc
-    }
-    tmem_st_wait();
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    PHASE_MARK(9);
-
-    // ---- O_partial = P @ Vc[K]
-    if (tid == 0) {
-      tc_fence_after();
-      if (more) mbar_expect_tx(&bar_qc, OPB);   // the load is issued at the top of the next step
-      gemm_tm_t<8>(tmem + COL_O, tmem + COL_A, aVc, ID_D, false);
-      mma_commit(&bar_mma);
-      if (more) {  // S is consumed and Ku[I+1] was fetched after the Su product: the next step's Z runs under the
-                   // store of this step's partial
-        mbar_wait(&bar_ku, ph_load ^ 1, abortp);
-        gemm_kk_t<NP>(tmem + COL_S, aQu, aKuA, ID_SQ, false);
-        mma_commit(&bar_z);
+      red_sum[grp][row] = lsum.x + lsum.y;
+      tmem_st_wait();
+      tc_fence_before();
+      sync_y();
+      PIPE_MARK(10);
+      // ---- O_partial = P @ Vc[K]
+      if (warp == 8 && elect_one()) {
+        tc_fence_after();
+        gemm_tm_t<8>(tmem + C_O, tmem + C_R3, aVc, ID_D, false);
+        mma_commit(bar_o);
       }
-    }
-    const int64_t tile = (int64_t)bh * tri(p.nblk) + tri(I) + K;
-    if (cc == 0 && irow < p.N) {
-      float lrow = red_sum[0][row] + red_sum[1][row] + red_sum[2][row] + red_sum[3][row];
-      float2* ml = reinterpret_cast<float2*>(p.part_ml) + tile * kBlk + row;
-      *ml = make_float2(mrow, lrow);
-    }
-    mbar_wait(&bar_mma, ph_mma, abortp);
-    ph_mma ^= 1;
-    tc_fence_after();
-    PHASE_MARK(10);
-    if (c0 < D) {
-      uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.part_o) + (tile * kBlk + row) * D + c0);
-      float v[32];
-      tmem_ld32(trow + COL_O + c0, v);
+      const int64_t tile = (int64_t)bh * tri(p.nblk) + tri(I) + K;
+      if (grp == 0 && irow < p.N)
+        reinterpret_cast<float2*>(p.part_ml)[tile * kBlk + row] = make_float2(mx * p.scale, red_sum[0][row] + red_sum[1][row]);
+      if (I + 1 < I_end && (B2 ? warp == 9 : warp == 8) && elect_one()) mbar_wait_lazy_abort(in_bar(I + 1 - K), in_par(I + 1 - K), abortp);   // Qc for the next Sc
+      wait_warp(bar_o, ph_m);
+      if (!B2) issue_sc(I + 1);   // over P
+      PIPE_MARK(11);
+      float o[NP][32];
+#pragma unroll
+      for (int c = 0; c < NP; ++c) tmem_ld32(trow + C_O + (grp * NP + c) * 32, o[c]);
       tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (B2) sync_y();
+      else if (lane == 0) mbar_arrive(bar_r);
+      PIPE_MARK(12);
+      if (B2) issue_sc(I + 1);   // over P and P @ Vc, which everybody has read
       if (irow < p.N) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          dst[j] = make_uint4(Elem<T>::pack2(v[8 * j], v[8 * j + 1]), Elem<T>::pack2(v[8 * j + 2], v[8 * j + 3]),
-                              Elem<T>::pack2(v[8 * j + 4], v[8 * j + 5]), Elem<T>::pack2(v[8 * j + 6], v[8 * j + 7]));
-      }
-    }
-    fence_async_smem();  // the exchange buffer over Qc[I] was read by threads; TMA writes it next
-    tc_fence_before();
-    __syncthreads();
-    ph_load ^= 1;
-    PHASE_MARK(11);
-  }
-
-  // ---- W_K is now U[K]: the cache's lookahead keys and the backward's starting state
-  if ((p.u_out.ptr != nullptr || p.w_state != nullptr) && c0 < D) {
-    tc_fence_after();
-    float v[32];
-    tmem_ld32(trow + COL_W + c0, v);
-    tmem_ld_wait();
-    if (krow < p.N) {
-      if (p.w_state != nullptr) {
-        float* dst = p.w_state + ((int64_t)bh * p.N + krow) * D + c0;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-      }
-      if (p.u_out.ptr != nullptr) {
-        int64_t off = b * p.u_out.stride_b + h * p.u_out.stride_h + (int64_t)krow * p.u_out.stride_n + c0;
-        if (p.u_dtype == CASTLE_F32) {
-          float* dst = reinterpret_cast<float*>(p.u_out.ptr) + off;
-#pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        } else if (p.u_dtype == CASTLE_BF16) {
-          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.u_out.ptr) + off);
+        for (int c = 0; c < NP; ++c) {
+          uint4* dst = reinterpret_cast<uint4*>(p.part_o) + (tile * (D / 8) + (grp * NP + c) * 4) * kBlk + row;
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            dst[j] = make_uint4(Elem<__nv_bfloat16>::pack2(v[8 * j], v[8 * j + 1]),
-                                Elem<__nv_bfloat16>::pack2(v[8 * j + 2], v[8 * j + 3]),
-                                Elem<__nv_bfloat16>::pack2(v[8 * j + 4], v[8 * j + 5]),
-                                Elem<__nv_bfloat16>::pack2(v[8 * j + 6], v[8 * j + 7]));
-        } else {
-          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.u_out.ptr) + off);
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            dst[j] = make_uint4(Elem<__half>::pack2(v[8 * j], v[8 * j + 1]),
-                                Elem<__half>::pack2(v[8 * j + 2], v[8 * j + 3]),
-                                Elem<__half>::pack2(v[8 * j + 4], v[8 * j + 5]),
-                                Elem<__half>::pack2(v[8 * j + 6], v[8 * j + 7]));
+            dst[j * kBlk] = make_uint4(Elem<T>::pack2(o[c][8 * j], o[c][8 * j + 1]), Elem<T>::pack2(o[c][8 * j + 2], o[c][8 * j + 3]),
+                                       Elem<T>::pack2(o[c][8 * j + 4], o[c][8 * j + 5]), Elem<T>::pack2(o[c][8 * j + 6], o[c][8 * j + 7]));
         }
       }
     }
   }
-  if (p.store_caches && tid == 0) bulk_wait0();
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, TM_COLS);
+  if (warp == 0) tmem_dealloc(tmem, 512);
+  if (tid == 0 && *abort_flag) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
+}
+
+// The masked T tiles: one CTA of 128 threads (a row each) per query block.
+template <typename T, int D>
+__global__ void __launch_bounds__(128) castle_fwd_t_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc,
+                                                           const __grid_constant__ CUtensorMap m_vu) {
+  constexpr int NP = D / 64;
+  constexpr uint32_t OPB = NP * kPanelBytes;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ uint64_t bar_in, bar_t;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int bh = blockIdx.x, I = blockIdx.y, b = bh / p.H, h = bh % p.H;
+  if (tid == 0) {
+    mbar_init(&bar_in, 1);
+    mbar_init(&bar_t, 1);
+    mbar_fence_init();
+    abort_flag = 0;
+  }
+  if (warp == 0) { tmem_alloc(&tmem_base_s, 128); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base_s, trow = tmem + ((uint32_t)(warp * 32) << 16);
+  if (tid == 0) {
+    if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
+    mbar_expect_tx(&bar_in, 2 * OPB);
+#pragma unroll
+    for (int pn = 0; pn < NP; ++pn) {
+      tma_load_4d(smem + pn * kPanelBytes, &m_qc, &bar_in, pn * 64, I * kBlk, h, b);
+      tma_load_4d(smem + OPB + pn * kPanelBytes, &m_vu, &bar_in, pn * 64, I * kBlk, h, b);
+    }
+    mbar_wait(&bar_in, 0, &abort_flag);
+    tc_fence_after();
+    gemm_kk_t<NP>(tmem, smem_u32(smem), smem_u32(smem) + OPB, make_idesc(128, 128, Elem<T>::fmt, false, false, false), false);
+    mma_commit(&bar_t);
+  }
+  mbar_wait(&bar_t, 0, &abort_flag);
+  tc_fence_after();
+  uint4* dst = p.tm + ((int64_t)bh * p.nblk + I) * kTmTile + tid;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    float v[32];
+    tmem_ld32_lower(trow + c * 32, tid, c * 32, v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      dst[(c * 4 + j) * kBlk] = make_uint4(Elem<T>::pack2(v[8 * j], v[8 * j + 1]), Elem<T>::pack2(v[8 * j + 2], v[8 * j + 3]),
+                                           Elem<T>::pack2(v[8 * j + 4], v[8 * j + 5]), Elem<T>::pack2(v[8 * j + 6], v[8 * j + 7]));
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 128);
   if (tid == 0 && abort_flag) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
 }
 
 // ---------------------------------------------------------------------------------------------
-// dim_head 64: a leaner CTA (256 threads, 112 KB of shared memory, 256 TMEM columns) so that TWO
-// CTAs share an SM.  Each CTA's step is a serial chain of products and elementwise passes; with two
-// resident chains one CTA's transcendental work fills the time the other spends waiting on the
-// tensor pipe or on a barrier.  To fit, only Qu[K] stays resident: Kc[K] and Vc[K] are re-fetched by
+// dim_head 64, many short walks (see launch_fwd): a leaner CTA (256 threads, 112 KB of shared memory, 256 TMEM columns) so
+// that TWO CTAs share an SM.  Each CTA's step is a serial chain of products and elementwise passes; with two resident
+// chains one CTA's start-up and waits are filled by the other's work.  To fit, only Qu[K] stays resident: Kc[K] and Vc[K]
+// are re-fetched by
 // TMA each step into slots that have just died (Kc over Vu[I] once Su is done, Vc over Qc[I] once Sc
 // is done); both fetches hide behind the elementwise pass that follows their issue.
 // The three products whose first operand is a tile the threads have just computed (gate A for the state
@@ -423,10 +574,8 @@ constexpr uint32_t kFwd2Smem = 7 * kPanelBytes + 256;   // 112 KB of tiles + bar
 #endif
 constexpr int kFwd2Groups = CASTLE_FWD_GROUPS;
 
-// Tensor maps of the three decode caches a prefill launch stores into; the plain launch carries an empty
-// struct instead.  AUX = the kernel with the two rarely needed paths (cache stores, cut walks) compiled in:
-// as run-time branches of the one kernel they cost the plain path 2.3 % (1.001 against 0.979 ms on the bench
-// workload), so the plain instantiation has none of their code or parameters.
+// Tensor maps of the three decode caches a prefill launch stores into; the plain launch carries an empty struct
+// instead.  AUX = the kernel with the cache stores compiled in.
 template <bool AUX> struct CacheMaps {};
 template <> struct CacheMaps<true> { CUtensorMap qu, kc, vc; };
 
@@ -469,22 +618,9 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
   const int bh = blockIdx.x, K = blockIdx.y;
   const int b = bh / p.H, h = bh % p.H;
   const int k0 = K * kBlk;
-  // Walk segments.  With few (batch, head) pairs the grid is a single wave whose makespan is the longest
-  // walk (key block 0: every query block), so long walks are cut in two, one CTA each.  The CTA that takes
-  // the later part first rebuilds the state it would have inherited with a short pre-loop over the earlier
-  // blocks (Z, gate and W += A @ Vu only, no scores).  blockIdx.z = 0 is the LATER part: those CTAs are the heaviest, and the grid is handed
-  // out in blockIdx order, so they start first.
-  const int seg = AUX ? (int)gridDim.z - 1 - (int)blockIdx.z : 0;
-  const int walk = p.nblk - K;
-  const int cut = (AUX && p.split_q8 > 0 && walk >= 8) ? K + (walk * p.split_q8 + 128) / 256 : p.nblk;
   const bool store_caches = AUX && p.store_caches;
   const CUtensorMap *m_cache_qu = nullptr, *m_cache_kc = nullptr, *m_cache_vc = nullptr;
   if constexpr (AUX) { m_cache_qu = &m_cache.qu; m_cache_kc = &m_cache.kc; m_cache_vc = &m_cache.vc; }
-  const int I_begin = seg == 0 ? K : cut;              // first block whose scores this CTA computes
-  const int I_end = seg == 0 ? cut : p.nblk;           // one past its last
-  if (I_begin >= I_end) return;                        // a short walk is not cut: its later part is empty
-  const bool owns_state = (I_end == p.nblk);                                      // the last segment ends with W_K = U[K]
-
   if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need 1024-byte alignment
     if (tid == 0) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
     return;
@@ -507,10 +643,8 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
   if (tid == 0) {
     mbar_expect_tx(bar_qu, OPB);
     tma_load_4d(sQu, &m_qu, bar_qu, 0, k0, h, b);
-    if (I_begin == K) {   // the pre-loop needs no Qc; the last pre-loop step fetches the first real one
-      mbar_expect_tx(bar_qc, OPB);
-      tma_load_4d(sQV, &m_qc, bar_qc, 0, k0, h, b);
-    }
+    mbar_expect_tx(bar_qc, OPB);
+    tma_load_4d(sQV, &m_qc, bar_qc, 0, k0, h, b);
     mbar_expect_tx(bar_ku, OPB);
     tma_load_4d(sKuA, &m_ku, bar_ku, 0, k0, h, b);
     mbar_expect_tx(bar_vu, OPB);
@@ -518,11 +652,10 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
     mbar_wait(bar_qu, 0, abortp);
     // Prefill hand-off: Qu[K] is the block's rows of the decode cache; Kc[K] and Vc[K] follow in the
     // first step, each when its fetch has landed (see there).
-    if (store_caches && seg == 0 && !*abortp) tma_store_4d(m_cache_qu, sQu, 0, k0, h, b);
+    if (store_caches && !*abortp) tma_store_4d(m_cache_qu, sQu, 0, k0, h, b);
   }
 
-  uint32_t ph_ld = 0, ph_mma = 0;   // Ku/Vu barriers flip once per step (pre-loop steps included) ...
-  uint32_t ph_main = 0;             // ... the Qc/Kc/Vc barriers once per step that computes scores
+  uint32_t ph_ld = 0, ph_mma = 0;   // the load barriers flip once per step
   const uint32_t aQu = smem_u32(sQu), aQV = smem_u32(sQV), aWb = smem_u32(sWb), aKuA = smem_u32(sKuA),
                  aVuT = smem_u32(sVuT);
   const int krow = k0 + row;
@@ -537,10 +670,9 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
   tc_fence_before();   \
   __syncthreads();
 
-  for (int I = K; I < I_end; ++I) {
+  for (int I = K; I < p.nblk; ++I) {
     const int i0 = I * kBlk;
-    const bool diag = (I == K), last = (I == I_end - 1);
-    const bool pre = AUX && I < I_begin;   // state-only step of the pre-loop
+    const bool diag = (I == K), last = (I == p.nblk - 1);
 #ifdef CASTLE_PHASE_TIMING
     const int tstep = I - K;
 #endif
@@ -555,18 +687,6 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
     }
     F2_MMA_WAIT();
     PHASE_MARK(1);
-    if (pre && tid == 0) {
-      // Pre-loop steps are short, so their loads are issued as early as the slots allow: Ku[I] is consumed
-      // by Z (and the gate's shared-memory copy is not needed without scores), so the next Ku goes now,
-      // together with Qc when the next step is the first one that computes scores.
-      const int in0 = i0 + kBlk;   // a pre-loop step is never the last step of its CTA
-      if (I + 1 == I_begin) {
-        mbar_expect_tx(bar_qc, OPB);
-        tma_load_4d(sQV, &m_qc, bar_qc, 0, in0, h, b);
-      }
-      mbar_expect_tx(bar_ku, OPB);
-      tma_load_4d(sKuA, &m_ku, bar_ku, 0, in0, h, b);
-    }
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {  // gate A = sigmoid(scale * Z), kept for j > k; over Ku[I]
       const int c0 = cbase + c * 32;
@@ -582,7 +702,7 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
       }
-      if (!pre) store_row32<T>(sKuA, kPanelBytes, row, c0, v);   // operand of the Su correction (read along rows)
+      store_row32<T>(sKuA, kPanelBytes, row, c0, v);   // operand of the Su correction (read along rows)
       tmem_st_packed32<T>(trow + COL_O + c0 / 2, v);             // first operand of the state update
     }
     tmem_st_wait();
@@ -592,32 +712,14 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
     // ---- W_K += A @ Vu[I]   and   T[I,I] = Qc[I] @ Vu[I]^T
     if (tid == 0) {
       mbar_wait(bar_vu, ph_ld, abortp);
-      if (!pre) mbar_wait(bar_qc, ph_main, abortp);
+      mbar_wait(bar_qc, ph_ld, abortp);
       tc_fence_after();
       gemm_tm_t<8>(tmem + COL_W, tmem + COL_O, aVuT, ID_D, !diag);
-      if (!pre) gemm_kk_t<1>(tmem + COL_S, aQV, aVuT, ID_SQ, false);
+      gemm_kk_t<1>(tmem + COL_S, aQV, aVuT, ID_SQ, false);
       mma_commit(bar_mma);
     }
     F2_MMA_WAIT();
     PHASE_MARK(3);
-    if (pre) {
-      // The state now includes block I.  Before the first step that computes scores, make its 16-bit copy
-      // (the later steps refresh it themselves); then fetch the next block's tiles and go on.
-      const bool next_real = (I + 1 == I_begin);
-      if (next_real && grp < 2) {
-        float v[32];
-        tmem_ld32(trow + COL_W + grp * 32, v);
-        tmem_ld_wait();
-        store_row32<T>(sWb, kPanelBytes, row, grp * 32, v);
-      }
-      F2_SYNC();
-      if (tid == 0) {   // Vu[I] is consumed by the state update: the next one goes now
-        mbar_expect_tx(bar_vu, OPB);
-        tma_load_4d(sVuT, &m_vu, bar_vu, 0, i0 + kBlk, h, b);
-      }
-      ph_ld ^= 1;
-      continue;
-    }
 #pragma unroll
     for (int c = 0; c < NCH; ++c) {  // masked T (j <= i), unscaled; over Vu[I]
       const int c0 = cbase + c * 32;
@@ -669,7 +771,7 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
 
     // ---- S/scale = penalty + Qc[I] @ Kc[K]^T
     if (tid == 0) {
-      mbar_wait(bar_kc, ph_main, abortp);
+      mbar_wait(bar_kc, ph_ld, abortp);
       tc_fence_after();
       gemm_kk_t<1>(tmem + COL_S, aQV, aVuT, ID_SQ, true);
       mma_commit(bar_mma);
@@ -729,7 +831,7 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
 
     // ---- O_partial = P @ Vc[K]
     if (tid == 0) {
-      mbar_wait(bar_vc, ph_main, abortp);
+      mbar_wait(bar_vc, ph_ld, abortp);
       tc_fence_after();
       gemm_tm_t<8>(tmem + COL_O, tmem + COL_S, aQV, ID_D, false);
       mma_commit(bar_mma);
@@ -760,19 +862,18 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
       tma_load_4d(sVuT, &m_vu, bar_vu, 0, in0, h, b);
     }
     if (grp < 2) {
-      uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.part_o) + (tile * kBlk + row) * D + grp * 32);
+      uint4* dst = reinterpret_cast<uint4*>(p.part_o) + (tile * (D / 8) + grp * 4) * kBlk + row;
       float v[32];
       tmem_ld32(trow + COL_O + grp * 32, v);
       tmem_ld_wait();
       if (irow < p.N) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          dst[j] = make_uint4(Elem<T>::pack2(v[8 * j], v[8 * j + 1]), Elem<T>::pack2(v[8 * j + 2], v[8 * j + 3]),
+          dst[j * kBlk] = make_uint4(Elem<T>::pack2(v[8 * j], v[8 * j + 1]), Elem<T>::pack2(v[8 * j + 2], v[8 * j + 3]),
                               Elem<T>::pack2(v[8 * j + 4], v[8 * j + 5]), Elem<T>::pack2(v[8 * j + 6], v[8 * j + 7]));
       }
     }
     ph_ld ^= 1;
-    ph_main ^= 1;
     tc_fence_before();
     __syncthreads();
     PHASE_MARK(10);
@@ -780,45 +881,17 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
 #undef F2_MMA_WAIT
 #undef F2_SYNC
 
-  // ---- W_K is now U[K] (in the CTA that walked to the last query block)
-  if (owns_state && grp < 2 && (p.u_out.ptr != nullptr || p.w_state != nullptr)) {
+  // ---- W_K is now U[K]
+  if (grp < 2 && (p.u_out.ptr != nullptr || p.w_state != nullptr)) {
     tc_fence_after();
     const int c0 = grp * 32;
     float v[32];
     tmem_ld32(trow + COL_W + c0, v);
     tmem_ld_wait();
     if (krow < p.N) {
-      if (p.w_state != nullptr) {
-        float* dst = p.w_state + ((int64_t)bh * p.N + krow) * D + c0;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-      }
-      if (p.u_out.ptr != nullptr) {
-        int64_t off = b * p.u_out.stride_b + h * p.u_out.stride_h + (int64_t)krow * p.u_out.stride_n + c0;
-        if (p.u_dtype == CASTLE_F32) {
-          float* dst = reinterpret_cast<float*>(p.u_out.ptr) + off;
-#pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-        } else if (p.u_dtype == CASTLE_BF16) {
-          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.u_out.ptr) + off);
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            dst[j] = make_uint4(Elem<__nv_bfloat16>::pack2(v[8 * j], v[8 * j + 1]),
-                                Elem<__nv_bfloat16>::pack2(v[8 * j + 2], v[8 * j + 3]),
-                                Elem<__nv_bfloat16>::pack2(v[8 * j + 4], v[8 * j + 5]),
-                                Elem<__nv_bfloat16>::pack2(v[8 * j + 6], v[8 * j + 7]));
-        } else {
-          uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__half*>(p.u_out.ptr) + off);
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            dst[j] = make_uint4(Elem<__half>::pack2(v[8 * j], v[8 * j + 1]),
-                                Elem<__half>::pack2(v[8 * j + 2], v[8 * j + 3]),
-                                Elem<__half>::pack2(v[8 * j + 4], v[8 * j + 5]),
-                                Elem<__half>::pack2(v[8 * j + 6], v[8 * j + 7]));
-        }
-      }
+      if (p.w_state != nullptr) store_u32(p.w_state, CASTLE_F32, ((int64_t)bh * p.N + krow) * D + c0, v);
+      if (p.u_out.ptr != nullptr)
+        store_u32(p.u_out.ptr, p.u_dtype, b * p.u_out.stride_b + h * p.u_out.stride_h + (int64_t)krow * p.u_out.stride_n + c0, v);
     }
   }
   if (store_caches && tid == 0) bulk_wait0();
@@ -829,12 +902,11 @@ castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_q
 }
 
 // Merge the per-key-block partials of one query block: out = sum_K e^{m_K - m} O_K / sum_K e^{m_K - m} l_K.
-// D/8 threads per row, each owning eight consecutive elements (one 16-byte load per partial).
+// One CTA per query block and 32 rows; a warp owns a chunk of eight columns of them (a lane a row), so that its loads
+// are contiguous.
 template <typename T, int D>
-__global__ void __launch_bounds__(256) castle_fwd_merge_kernel(const FwdParams p) {
-  constexpr int TPR = D / 8, ROWS = 256 / TPR;
-  const int bh = blockIdx.y, I = blockIdx.x / (kBlk / ROWS), sub = blockIdx.x % (kBlk / ROWS);
-  const int r = sub * ROWS + threadIdx.x / TPR, c8 = threadIdx.x % TPR;
+__global__ void __launch_bounds__(32 * D / 8) castle_fwd_merge_kernel(const FwdParams p) {
+  const int bh = blockIdx.y, I = blockIdx.x / (kBlk / 32), r = (blockIdx.x % (kBlk / 32)) * 32 + (threadIdx.x & 31), c8 = threadIdx.x >> 5;
   const int i = I * kBlk + r;
   if (i >= p.N) return;
   const int64_t tile0 = (int64_t)bh * tri(p.nblk) + tri(I);
@@ -844,12 +916,13 @@ __global__ void __launch_bounds__(256) castle_fwd_merge_kernel(const FwdParams p
   float l = 0.f, acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  const uint4* po = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.part_o) + (tile0 * kBlk + r) * D) + c8;
+  const uint4* po = reinterpret_cast<const uint4*>(p.part_o) + (tile0 * (D / 8) + c8) * kBlk + r;
+#pragma unroll 4
   for (int K = 0; K <= I; ++K) {
-    float2 v = ml[(int64_t)K * kBlk];
-    float w = __expf(v.x - m);
+    const float2 v = ml[(int64_t)K * kBlk];
+    const uint4 o = po[(int64_t)K * kBlk * (D / 8)];
+    const float w = __expf(v.x - m);
     l += v.y * w;
-    uint4 o = po[(int64_t)K * kBlk * D / 8];
     float2 a = Elem<T>::unpack2(o.x), b2 = Elem<T>::unpack2(o.y), c = Elem<T>::unpack2(o.z), d2 = Elem<T>::unpack2(o.w);
     acc[0] += a.x * w; acc[1] += a.y * w; acc[2] += b2.x * w; acc[3] += b2.y * w;
     acc[4] += c.x * w; acc[5] += c.y * w; acc[6] += d2.x * w; acc[7] += d2.y * w;
@@ -867,54 +940,60 @@ __global__ void __launch_bounds__(256) castle_fwd_merge_kernel(const FwdParams p
 }
 
 template <typename T>
-static int launch_fwd_d64(const FwdParams& p, const CUtensorMap* maps, cudaStream_t st) {
+static int launch_fwd_short(const FwdParams& p, const CUtensorMap* maps, cudaStream_t st) {
   constexpr int G = kFwd2Groups;
-  {  // per device, so set on every call (cheap)
-    cudaError_t e = cudaFuncSetAttribute(castle_fwd_kernel_d64<T, G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
-    if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
-  }
-  // Few (batch, head) pairs: cut the long walks so that the grid is several waves of short CTAs instead of
-  // one wave bounded by the walk of key block 0 (296 CTAs are resident at a time: 2 per SM on 148 SMs).
-  FwdParams q = p;
-  q.split_q8 = 0;
-  if ((int64_t)p.B * p.H * p.nblk < 384 && p.nblk >= 8)   // beyond ~1.3 waves the pre-loops cost more than the balance gains
-    q.split_q8 = 128;   // the middle measured best (0.169 ms at 8 pairs x 32 blocks; 0.240 ms uncut; later cuts slower)
-  const bool aux = q.split_q8 > 0 || p.store_caches;
-  dim3 grid(p.B * p.H, p.nblk, q.split_q8 > 0 ? 2 : 1);
-  ev_start(CASTLE_KERNEL_FWD, st);
-  if (aux) {
+  dim3 grid(p.B * p.H, p.nblk);
+  if (p.store_caches) {
     cudaError_t e = cudaFuncSetAttribute(castle_fwd_kernel_d64<T, G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
     if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
     CacheMaps<true> cm;
     cm.qu = maps[6]; cm.kc = maps[7]; cm.vc = maps[8];
-    castle_fwd_kernel_d64<T, G, true><<<grid, G * 128, kFwd2Smem, st>>>(q, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], cm);
+    castle_fwd_kernel_d64<T, G, true><<<grid, G * 128, kFwd2Smem, st>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], cm);
   } else {
-    castle_fwd_kernel_d64<T, G, false><<<grid, G * 128, kFwd2Smem, st>>>(q, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
+    cudaError_t e = cudaFuncSetAttribute(castle_fwd_kernel_d64<T, G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
+    if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
+    castle_fwd_kernel_d64<T, G, false><<<grid, G * 128, kFwd2Smem, st>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
                                                                         CacheMaps<false>{});
   }
-  ev_stop(CASTLE_KERNEL_FWD, st);
-  constexpr int ROWS = 256 / (64 / 8);
-  dim3 g2(p.nblk * (kBlk / ROWS), p.B * p.H);
-  castle_fwd_merge_kernel<T, 64><<<g2, 256, 0, st>>>(p);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : cuda_fail(e, "castle_fwd launch");
+  return 0;
 }
 
 template <typename T, int D>
-static int launch_fwd(const FwdParams& p, const CUtensorMap* maps, cudaStream_t st) {
-  constexpr size_t smem = 5 * (D / 64) * kPanelBytes + 2 * 2 * kPanelBytes + 1024;
-  {  // per device, so set on every call (cheap)
-    cudaError_t e = cudaFuncSetAttribute(castle_fwd_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+static int launch_fwd_pipe(const FwdParams& p, const CUtensorMap* maps, cudaStream_t st) {
+  // Few pairs: the grid is one wave whose length is the walk of key block 0, while the mean walk is half as long or, with
+  // idle SMs, still less.  `load` = steps per SM over the longest walk.  us uncut / 2 / 3 parts: 4 pairs x 16 blocks at
+  // dim_head 128 74 / 60 / 52 (load 0.23), 4 x 12 44 / 37 / 34 (0.18), 8 x 12 44 / 37 / 40 (0.35), 4 x 32 100 / 78 / 88 (0.45), 16 x 11
+  // 43 / 46 / 52 (0.65), 8 x 32 103 / 138 / 166 (0.89).
+  const float load = (float)(p.B * p.H) * (float)(p.nblk + 1) * (0.5f / 148.f);
+  const int nseg = p.nblk < kSplitMin || load >= 0.6f ? 1 : load >= 0.3f ? 2 : 3;
+  auto kernel = p.tm ? castle_fwd_pipe_kernel<T, D, true> : castle_fwd_pipe_kernel<T, D, false>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FwdPipe<D>::kSmem);   // per device, so on every call (cheap)
+  if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
+  kernel<<<dim3(p.B * p.H, p.nblk, nseg), kFwdThreads, FwdPipe<D>::kSmem, st>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
+                                                                               maps[6], maps[7], maps[8]);
+  return 0;
+}
+
+template <typename T, int D>
+static int launch_fwd(FwdParams p, const CUtensorMap* maps, cudaStream_t st) {
+  // One CTA per SM leaves a CTA's start-up (some 10 us: tensor memory, first tiles, the fill of the pipeline) uncovered, so
+  // where the walks are short and the grid is more than a wave, dim_head 64 takes the kernel with two CTAs per SM.  us, short /
+  // pipeline: 512 pairs x 1 block 28 / 38, 256 x 4 92 / 100, 128 x 5 71 / 74, 128 x 8 143 / 139.
+  const bool brief = D == 64 && p.nblk <= 6 && (int64_t)p.B * p.H * p.nblk > 2 * 148;
+  if (brief) p.tm = nullptr;
+  if (p.tm) {
+    constexpr size_t smem = 2 * (D / 64) * kPanelBytes;
+    cudaError_t e = cudaFuncSetAttribute(castle_fwd_t_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
+    castle_fwd_t_kernel<T, D><<<dim3(p.B * p.H, p.nblk), 128, smem, st>>>(p, maps[0], maps[5]);
   }
-  dim3 grid(p.B * p.H, p.nblk);
   ev_start(CASTLE_KERNEL_FWD, st);
-  castle_fwd_kernel<T, D><<<grid, kFwdThreads, smem, st>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
-                                                            maps[6], maps[7], maps[8]);
+  int rc;
+  if constexpr (D == 64) rc = brief ? launch_fwd_short<T>(p, maps, st) : launch_fwd_pipe<T, D>(p, maps, st);
+  else rc = launch_fwd_pipe<T, D>(p, maps, st);
+  if (rc) return rc;
   ev_stop(CASTLE_KERNEL_FWD, st);
-  constexpr int ROWS = 256 / (D / 8);
-  dim3 g2(p.nblk * (kBlk / ROWS), p.B * p.H);
-  castle_fwd_merge_kernel<T, D><<<g2, 256, 0, st>>>(p);
+  castle_fwd_merge_kernel<T, D><<<dim3(p.nblk * (kBlk / 32), p.B * p.H), 32 * D / 8, 0, st>>>(p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_fwd launch");
 }
@@ -937,7 +1016,9 @@ extern "C" size_t castle_fwd_workspace_bytes(const castle_problem_t* p) {
   if (!p || p->seq_len <= 0) return 0;
   int64_t nb = (p->seq_len + kBlk - 1) / kBlk;
   int64_t tiles = (int64_t)p->batch * p->heads * tri(nb);
-  return (size_t)(tiles * kBlk * (2 * sizeof(float) + p->dim_head * 2));  // (max, sum) fp32 + a 16-bit row
+  size_t bytes = (size_t)(tiles * kBlk * (2 * sizeof(float) + p->dim_head * 2));  // (max, sum) fp32 + a 16-bit row
+  if (nb >= kTmBlocks) bytes += (size_t)((int64_t)p->batch * p->heads * nb * kTmTile * sizeof(uint4));
+  return bytes;
 }
 
 static int fwd_impl(const char* who, const castle_problem_t* p, const castle_tensor_t* qc, const castle_tensor_t* kc,
@@ -977,7 +1058,7 @@ static int fwd_impl(const char* who, const castle_problem_t* p, const castle_ten
   fp.u_dtype = u_dtype;
   fp.out = *out; fp.status = status;
   fp.store_caches = caches ? 1 : 0;
-  fp.split_q8 = 0;
+  fp.tm = fp.nblk >= kTmBlocks ? (uint4*)((uint8_t*)workspace + tiles * kBlk * (2 * sizeof(float) + p->dim_head * 2)) : nullptr;
 #ifdef CASTLE_PHASE_TIMING
   fp.timing = (long long*)((char*)workspace + need);  // the caller leaves 1 KB beyond the partials
 #endif
@@ -995,8 +1076,8 @@ static int fwd_impl(const char* who, const castle_problem_t* p, const castle_ten
   }
   cudaStream_t st = (cudaStream_t)stream;
   if (p->dtype == CASTLE_BF16)
-    return p->dim_head == 64 ? launch_fwd_d64<__nv_bfloat16>(fp, maps, st) : launch_fwd<__nv_bfloat16, 128>(fp, maps, st);
-  return p->dim_head == 64 ? launch_fwd_d64<__half>(fp, maps, st) : launch_fwd<__half, 128>(fp, maps, st);
+    return p->dim_head == 64 ? launch_fwd<__nv_bfloat16, 64>(fp, maps, st) : launch_fwd<__nv_bfloat16, 128>(fp, maps, st);
+  return p->dim_head == 64 ? launch_fwd<__half, 64>(fp, maps, st) : launch_fwd<__half, 128>(fp, maps, st);
 }
 
 extern "C" int castle_fwd(const castle_problem_t* p, const castle_tensor_t* qc, const castle_tensor_t* kc,

@@ -73,6 +73,15 @@ __device__ __forceinline__ void mbar_wait_lazy_abort(uint64_t* bar, uint32_t par
 // Barrier over the 128 threads (four warps) of one chunk group; ids 1..15 (0 is __syncthreads).
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
+// One lane of a converged warp, always the same one.  Code under `warp_uniform_condition && elect_one()` is known to be
+// run by one lane of the warp, so its descriptors and addresses stay in uniform registers, where the tensor-core and
+// TMA instructions take them from.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ---------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_async_smem() {  // generic-proxy smem writes -> async proxy (MMA/TMA) reads
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -231,6 +240,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
       : "r"(taddr)
       : "memory");
 }
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+  uint32_t* r = reinterpret_cast<uint32_t*>(v);
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
   const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
@@ -275,17 +294,20 @@ template <> struct Elem<__half> {
 
 // 32 values of a row as 16 packed 16-bit pairs into 16 consecutive columns of the thread's lane: the
 // layout a tensor-memory A operand wants (see mma_ts).
-template <typename T>
-__device__ __forceinline__ void tmem_st_packed32(uint32_t taddr, const float* v) {
-  uint32_t r[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) r[j] = Elem<T>::pack2(v[2 * j], v[2 * j + 1]);
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(r[0]),
       "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
       "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
       : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void tmem_st_packed32(uint32_t taddr, const float* v) {
+  uint32_t r[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) r[j] = Elem<T>::pack2(v[2 * j], v[2 * j + 1]);
+  tmem_st16(taddr, r);
 }
 
 // ---------------------------------------------------------------- fast transcendentals
