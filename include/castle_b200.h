@@ -135,6 +135,17 @@ int castle_transform(const castle_problem_t* p, int32_t count, const castle_tens
  */
 int castle_amax_scale(int32_t dtype, const void* x, int64_t count, uint32_t* state, float* out, void* stream);
 
+/* ---- RMSNorm of the module's input (lookahead_keys_attention/lookahead_keys_attention.py:67, :99) ------------
+ * rows x dim, contiguous, dim a multiple of 8; x, weight, y, dy, dx, dweight of `dtype`, sums in fp32.  Forward:
+ * y = x * rstd * weight with rstd = rsqrt(mean(x^2) + eps), which is stored (fp32, rows) unless NULL.  Backward: dx
+ * and dweight, each NULL if not wanted; dweight needs the workspace.
+ */
+int castle_rmsnorm_fwd(int32_t dtype, int64_t rows, int32_t dim, const void* x, const void* weight, float eps, void* y,
+                       float* rstd, void* stream);
+size_t castle_rmsnorm_bwd_workspace_bytes(int64_t rows, int32_t dim);
+int castle_rmsnorm_bwd(int32_t dtype, int64_t rows, int32_t dim, const void* dy, const void* x, const void* weight,
+                       const float* rstd, void* dx, void* dweight, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---- parallel backward ---------------------------------------------------
  * Replaces CastleAttentionFunction.backward
  * (lookahead_keys_attention_triton.py:509-602) with its two kernels

@@ -14,7 +14,7 @@ from pathlib import Path
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libcastle_b200.so"
-SOURCES = ["api.cu", "decode.cu", "selftest.cu", "convert.cu", "transform.cu", "token_linear.cu", "fwd.cu", "bwd.cu", "bwd128.cu"]
+SOURCES = ["api.cu", "decode.cu", "selftest.cu", "convert.cu", "transform.cu", "token_linear.cu", "norm.cu", "fwd.cu", "bwd.cu", "bwd128.cu"]
 
 BF16, F16, F32 = 0, 1, 2
 
@@ -171,6 +171,9 @@ _SIGNATURES = {
     "castle_convert_16bit": (ctypes.c_int, [_i32, _vp, _vp, ctypes.c_int64, _vp, _vp]),
     "castle_transform": (ctypes.c_int, [_PR, _i32, _T, _T, _i32, _i32, _T, P(CastleRotary), ctypes.c_uint32, _vp, _vp]),
     "castle_amax_scale": (ctypes.c_int, [_i32, _vp, ctypes.c_int64, _vp, _vp, _vp]),
+    "castle_rmsnorm_fwd": (ctypes.c_int, [_i32, ctypes.c_int64, _i32, _vp, _vp, ctypes.c_float, _vp, _vp, _vp]),
+    "castle_rmsnorm_bwd_workspace_bytes": (_sz, [ctypes.c_int64, _i32]),
+    "castle_rmsnorm_bwd": (ctypes.c_int, [_i32, ctypes.c_int64, _i32] + [_vp] * 7 + [_sz, _vp]),
     "castle_bwd_workspace_bytes": (_sz, [_PR]),
     "castle_bwd": (ctypes.c_int, [_PR] + [_T] * 8 + [_vp, _vp] + [_T] * 6 + [_vp, _sz, _vp, _vp]),
     "castle_decode_workspace_bytes": (_sz, [_PR, _i32]),

@@ -46,6 +46,9 @@ struct Api {
   decltype(&castle_fwd_workspace_bytes) fwd_workspace_bytes;
   decltype(&castle_fwd) fwd;
   decltype(&castle_fwd_prefill) fwd_prefill;
+  decltype(&castle_rmsnorm_fwd) rmsnorm_fwd;
+  decltype(&castle_rmsnorm_bwd_workspace_bytes) rmsnorm_bwd_workspace_bytes;
+  decltype(&castle_rmsnorm_bwd) rmsnorm_bwd;
   decltype(&castle_bwd_workspace_bytes) bwd_workspace_bytes;
   decltype(&castle_bwd) bwd;
   decltype(&castle_transform) transform;
@@ -500,12 +503,136 @@ struct Layer {
   int64_t heads = 0, dim_head = 0;
 };
 
+// Whether the layer can run natively around the core, too: plain CUDA tensors of one type, and nothing that changes what a
+// linear call means (autocast, a dispatch mode).
+bool plain_layer(const Tensor& x, const Layer& l) {
+  auto plain = [&](const Tensor& t) {
+    return t.is_cuda() && t.scalar_type() == x.scalar_type() && t.is_contiguous() && t.layout() == at::kStrided && t.device() == x.device() &&
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !t.unsafeGetTensorImpl()->is_python_dispatch();
+  };
+  const int64_t inner = l.heads * l.dim_head;
+  return x.dim() == 3 && x.is_cuda() && x.numel() > 0 && x.layout() == at::kStrided && !x.unsafeGetTensorImpl()->is_python_dispatch() &&
+         dtype_code(x.scalar_type()) >= 0 && x.size(2) % 8 == 0 && plain(l.to_qkv) && plain(l.combine) &&
+         (!l.norm.defined() || (plain(l.norm) && l.norm.dim() == 1 && l.norm.size(0) == x.size(2))) && l.to_qkv.dim() == 2 &&
+         l.to_qkv.size(0) == 6 * inner && l.to_qkv.size(1) == x.size(2) && l.combine.dim() == 2 && l.combine.size(1) == inner &&
+         !at::autocast::is_autocast_enabled(at::kCUDA) && !c10::impl::dispatch_mode_enabled();
+}
+
+float norm_eps(const Layer& l) { return (float)l.eps.value_or(std::numeric_limits<float>::epsilon()); }   // torch's default for every type
+
+// y = x @ w^T on two-dimensional x
+Tensor matmul_t(const Tensor& x, const Tensor& w) { return at::mm(x, w.t()); }
+
+// Gradient node of a whole layer.  Autograd over the single operations (norm, two linear layers, the views between them
+// and the core) cost 250 us of host time per training step where the kernels of a small one take 120.
+struct LayerBackward : public Node {
+  Problem p;
+  Options o;
+  int64_t dim = 0;
+  bool has_norm = false;
+  SavedVariable x, to_qkv, combine, norm;   // inputs, in the order of the node's outputs
+  Tensor h, rstd, out16, lse, w_state, merged;
+  Inputs in;
+
+  std::string name() const override { return "CastleLayerBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    x.reset_data(); to_qkv.reset_data(); combine.reset_data(); norm.reset_data();
+    h = rstd = out16 = lse = w_state = merged = Tensor();
+    in.keep.clear();
+  }
+  variable_list apply(variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    variable_list result(has_norm ? 4 : 3);
+    if (grads.empty() || !grads[0].defined()) return result;
+    const bool need_x = task_should_compute_output(0), need_qkv = task_should_compute_output(1), need_combine = task_should_compute_output(2),
+               need_norm = has_norm && task_should_compute_output(3);
+    const Tensor xs = x.unpack(), wq = to_qkv.unpack(), wc = combine.unpack();   // (raises on a second backward)
+    at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard guard(xs.device());
+    const auto stream = c10::cuda::getCurrentCUDAStream(xs.device().index());
+    const int64_t rows = p.B * p.N, inner = p.H * p.d;
+    const Tensor g = grads[0].reshape({rows, wc.size(0)});
+    if (need_combine) result[2] = at::mm(g.t(), merged);
+    if (!(need_x || need_qkv || need_norm)) return result;
+    const Tensor dcore = at::mm(g, wc).view({p.B, p.N, p.H, p.d}).permute({0, 2, 1, 3});
+    const Tensor dqkv = run_backward(p, in.t, out16, lse, w_state, dcore, o).view({rows, 6 * inner});
+    if (need_qkv) result[1] = at::mm(dqkv.t(), h);
+    if (!(need_x || need_norm)) return result;
+    Tensor dh = at::mm(dqkv, wq);
+    if (!has_norm) {
+      result[0] = dh.view(xs.sizes());
+      return result;
+    }
+    const Tensor xc = xs.contiguous(), wn = norm.unpack();
+    if (need_x) result[0] = at::empty(xs.sizes(), dh.options());
+    if (need_norm) result[3] = at::empty({dim}, dh.options());
+    const size_t bytes = api.rmsnorm_bwd_workspace_bytes(rows, (int32_t)dim);
+    const Tensor ws = scratch(stream, bytes);
+    check(api.rmsnorm_bwd(dtype_code(p.dtype), rows, (int32_t)dim, dh.data_ptr(), xc.data_ptr(), wn.data_ptr(), rstd.data_ptr<float>(),
+                          need_x ? result[0].data_ptr() : nullptr, need_norm ? result[3].data_ptr() : nullptr, ws.data_ptr(), ws.numel(),
+                          stream.stream()), "castle_rmsnorm_bwd");
+    return result;
+  }
+};
+
+// Norm, projection, core and output projection, for plain_layer().
+Tensor layer_native(const Tensor& x, const Layer& l, Options o) {
+  const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || l.to_qkv.requires_grad() || l.combine.requires_grad() ||
+                                                   (l.norm.defined() && l.norm.requires_grad()));
+  o.need_grad = grad && (x.requires_grad() || l.to_qkv.requires_grad() || (l.norm.defined() && l.norm.requires_grad()));
+  const int64_t B = x.size(0), N = x.size(1), dim = x.size(2), rows = B * N, inner = l.heads * l.dim_head;
+  const Problem p = make_problem({B, l.heads, N, l.dim_head}, x.scalar_type(), o.long_seq);
+  Tensor out, h, rstd, merged;
+  Result r;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard guard(x.device());
+    const auto stream = c10::cuda::getCurrentCUDAStream(x.device().index());
+    h = x.contiguous().view({rows, dim});
+    if (l.norm.defined()) {
+      const Tensor src = h;
+      h = at::empty({rows, dim}, x.options().requires_grad(false));
+      if (o.need_grad) rstd = at::empty({rows}, x.options().dtype(at::kFloat).requires_grad(false));
+      check(api.rmsnorm_fwd(dtype_code(p.dtype), rows, (int32_t)dim, src.data_ptr(), l.norm.data_ptr(), norm_eps(l), h.data_ptr(),
+                            o.need_grad ? rstd.data_ptr<float>() : nullptr, stream.stream()), "castle_rmsnorm_fwd");
+    }
+    const Tensor packed = matmul_t(h, l.to_qkv).view({B, N, 6, l.heads, l.dim_head});
+    Inputs in;
+    for (int i = 0; i < 6; ++i) in.t[i] = packed_desc(packed, i);
+    in.keep = {packed};
+    r = run_forward(p, std::move(in), o, x.device());
+    merged = r.out.permute({0, 2, 1, 3}).view({rows, inner});
+    out = matmul_t(merged, l.combine).view({B, N, l.combine.size(0)});
+  }
+  if (!grad) return out;
+  auto node = std::shared_ptr<LayerBackward>(new LayerBackward(), torch::autograd::deleteNode);
+  std::vector<Tensor> vars{x, l.to_qkv, l.combine};
+  if (l.norm.defined()) vars.push_back(l.norm);
+  node->set_next_edges(torch::autograd::collect_next_edges(vars));
+  node->p = p;
+  o.caches.clear();
+  node->o = o;
+  node->dim = dim;
+  node->has_norm = l.norm.defined();
+  torch::autograd::set_history(out, node);
+  node->x = SavedVariable(x, false);
+  node->to_qkv = SavedVariable(l.to_qkv, false);
+  node->combine = SavedVariable(l.combine, false);
+  if (l.norm.defined()) node->norm = SavedVariable(l.norm, false);
+  node->h = h; node->rstd = rstd; node->merged = merged;
+  node->in = std::move(r.in);
+  node->out16 = r.out16; node->lse = r.lse; node->w_state = r.w_state;
+  return out;
+}
+
 Tensor project(const Tensor& x, const Layer& l) {   // (B, N, 6, H, d)
   Tensor h = l.norm.defined() ? at::rms_norm(x, {x.size(-1)}, l.norm, l.eps) : x;
   return at::linear(h, l.to_qkv).view({x.size(0), x.size(1), 6, l.heads, l.dim_head});
 }
 
 Tensor layer_forward(const Tensor& x, const Layer& l, const Options& o) {
+  if (plain_layer(x, l)) return layer_native(x, l, o);
   const Tensor out = attention_packed(project(x, l), o).out;
   return at::linear(out.permute({0, 2, 1, 3}).reshape({x.size(0), x.size(1), l.heads * l.dim_head}), l.combine);
 }
@@ -521,21 +648,12 @@ Tensor decode_packed(const Tensor& packed, const Tensor* caches, int64_t t, doub
   return decode_core(nd, caches, B, H, d, packed.scalar_type(), t, scale, rotary, packed.device()).view({B, 1, H * d});
 }
 
-// Whether a token's projections can be the framework's own launches: a few rows of plain CUDA tensors of one type, and
-// nothing that changes what a linear call means (autocast, a dispatch mode).
+// Whether a token's projections can be the framework's own launches: a few rows of a plain layer.
 bool plain_token(const Tensor& x, const Layer& l) {
-  auto plain = [&](const Tensor& t) {
-    return t.is_cuda() && t.scalar_type() == x.scalar_type() && t.is_contiguous() && t.layout() == at::kStrided && t.device() == x.device() &&
-           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !t.unsafeGetTensorImpl()->is_python_dispatch();
-  };
-  const int64_t inner = l.heads * l.dim_head;
-  return x.dim() == 3 && x.size(1) == 1 && x.is_cuda() && x.stride(2) == 1 && !x.unsafeGetTensorImpl()->is_python_dispatch() &&
-         x.size(0) >= 1 && x.size(0) <= 8 && plain(l.to_qkv) && plain(l.combine) && (!l.norm.defined() || plain(l.norm)) &&
-         l.to_qkv.dim() == 2 && l.to_qkv.size(0) == 6 * inner && l.to_qkv.size(1) == x.size(2) && l.combine.dim() == 2 &&
-         l.combine.size(1) == inner && api.token_linear_fits(dtype_code(x.scalar_type()), (int32_t)x.size(0), (int32_t)x.size(2)) &&
-         api.token_linear_fits(dtype_code(x.scalar_type()), (int32_t)x.size(0), (int32_t)inner) &&
-         reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * x.element_size() % 16 == 0 &&
-         !at::autocast::is_autocast_enabled(at::kCUDA) && !c10::impl::dispatch_mode_enabled();
+  return plain_layer(x, l) && x.size(1) == 1 && x.stride(2) == 1 && x.size(0) <= 8 &&
+         api.token_linear_fits(dtype_code(x.scalar_type()), (int32_t)x.size(0), (int32_t)x.size(2)) &&
+         api.token_linear_fits(dtype_code(x.scalar_type()), (int32_t)x.size(0), (int32_t)(l.heads * l.dim_head)) &&
+         reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * x.element_size() % 16 == 0;
 }
 
 // Norm, projection, step and output projection of one token as three launches, with what passes between them in the
@@ -555,8 +673,7 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   char* core = packed + 6 * row;
   check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)x.size(2), (int32_t)(6 * inner), x.data_ptr(), x.stride(0),
                          l.norm.defined() ? l.norm.data_ptr() : nullptr,
-                         (float)l.eps.value_or(std::numeric_limits<float>::epsilon()),   // torch's default for every type
-                         l.to_qkv.data_ptr(), packed, stream.stream()), "castle_token_linear");
+                         norm_eps(l), l.to_qkv.data_ptr(), packed, stream.stream()), "castle_token_linear");
   castle_tensor_t news[6];
   for (int i = 0; i < 6; ++i) news[i] = {packed + kPackedOrder[i] * inner * es, 6 * inner, d, 6 * inner};
   launch_decode(cp, news, caches, core, t, rotary, ws.data_ptr(), part, stream);
@@ -835,7 +952,7 @@ PyObject* py_bind(PyObject*, PyObject* d) {
     };
 #define CASTLE_BIND(f) api.f = reinterpret_cast<decltype(api.f)>(get("castle_" #f))
     CASTLE_BIND(last_error); CASTLE_BIND(fwd_workspace_bytes); CASTLE_BIND(fwd); CASTLE_BIND(fwd_prefill);
-    CASTLE_BIND(bwd_workspace_bytes); CASTLE_BIND(bwd); CASTLE_BIND(transform); CASTLE_BIND(amax_scale);
+    CASTLE_BIND(rmsnorm_fwd); CASTLE_BIND(rmsnorm_bwd_workspace_bytes); CASTLE_BIND(rmsnorm_bwd); CASTLE_BIND(bwd_workspace_bytes); CASTLE_BIND(bwd); CASTLE_BIND(transform); CASTLE_BIND(amax_scale);
     CASTLE_BIND(decode_workspace_bytes); CASTLE_BIND(decode_step_fused); CASTLE_BIND(token_linear_fits); CASTLE_BIND(token_linear);
 #undef CASTLE_BIND
     Py_RETURN_NONE;
