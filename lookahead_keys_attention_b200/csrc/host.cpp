@@ -648,44 +648,65 @@ Tensor decode_packed(const Tensor& packed, const Tensor* caches, int64_t t, doub
   return decode_core(nd, caches, B, H, d, packed.scalar_type(), t, scale, rotary, packed.device()).view({B, 1, H * d});
 }
 
-// Whether a token's projections can be the framework's own launches: a few rows of a plain layer.
-bool plain_token(const Tensor& x, const Layer& l) {
-  return plain_layer(x, l) && x.size(1) == 1 && x.stride(2) == 1 && x.size(0) <= 8 &&
-         api.token_linear_fits(dtype_code(x.scalar_type()), (int32_t)x.size(0), (int32_t)x.size(2)) &&
-         api.token_linear_fits(dtype_code(x.scalar_type()), (int32_t)x.size(0), (int32_t)(l.heads * l.dim_head)) &&
-         reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * x.element_size() % 16 == 0;
+// Whether one projection of a token is the framework's own launch.  It is the faster one on the host (3 us against 8 for a
+// library call, with the norm in it); on the GPU the library wins where the weights are large for the rows (own / library:
+// 8 x 512 -> 3072 6.2 / 4 us, 8 x 1472 -> 8832 14.5 / 7, 2 x 2176 -> 13056 16.5 / 10, 1 x 2176 -> 13056 10.4 / 10).
+bool own_projection(int dtype, int64_t rows, int64_t k, int64_t n, int64_t es) {
+  return rows <= 8 && k * n * es <= (rows == 1 ? 64 << 20 : rows == 2 ? 16 << 20 : 8 << 20) &&
+         api.token_linear_fits(dtype, (int32_t)rows, (int32_t)k);
 }
 
-// Norm, projection, step and output projection of one token as three launches, with what passes between them in the
-// stream's scratch: on the host the allocations would cost as much as the launches.
+// Norm, projection, step and output projection of one token, with what passes between them in the stream's scratch: on
+// the host the allocations would cost as much as the launches.
 Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_t t, double scale, const Rotary& rotary) {
   const at::Device dev = x.device();
   const c10::cuda::CUDAGuard guard(dev);
+  at::AutoDispatchBelowADInplaceOrView below;
   const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
   const auto dtype = x.scalar_type();
-  const int64_t B = x.size(0), H = l.heads, d = l.dim_head, es = x.element_size();
+  const int64_t B = x.size(0), dim = x.size(2), H = l.heads, d = l.dim_head, inner = H * d, es = x.element_size();
   check_caches(caches, B, H, d, dtype);
   const castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
-  const int64_t inner = H * d, row = (B * inner * es + 255) / 256 * 256;
+  const int64_t row = (B * inner * es + 255) / 256 * 256;
   const size_t part = (api.decode_workspace_bytes(&cp, (int32_t)t) + 255) / 256 * 256;
   const Tensor ws = scratch(stream, part + 7 * row);
   char* packed = static_cast<char*>(ws.data_ptr()) + part;
   char* core = packed + 6 * row;
-  check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)x.size(2), (int32_t)(6 * inner), x.data_ptr(), x.stride(0),
-                         l.norm.defined() ? l.norm.data_ptr() : nullptr,
-                         norm_eps(l), l.to_qkv.data_ptr(), packed, stream.stream()), "castle_token_linear");
+  Tensor keep;
+  const Tensor xs = x.stride(2) == 1 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * es % 16 == 0 ? x : x.contiguous();
+  if (own_projection(cp.dtype, B, dim, 6 * inner, es)) {
+    check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)dim, (int32_t)(6 * inner), xs.data_ptr(), xs.stride(0),
+                           l.norm.defined() ? l.norm.data_ptr() : nullptr, norm_eps(l), l.to_qkv.data_ptr(), packed, stream.stream()),
+          "castle_token_linear");
+  } else {
+    Tensor h = xs.contiguous().view({B, dim});
+    if (l.norm.defined()) {
+      const Tensor src = h;
+      h = at::empty({B, dim}, x.options().requires_grad(false));
+      check(api.rmsnorm_fwd(cp.dtype, B, (int32_t)dim, src.data_ptr(), l.norm.data_ptr(), norm_eps(l), h.data_ptr(), nullptr, stream.stream()),
+            "castle_rmsnorm_fwd");
+    }
+    keep = matmul_t(h, l.to_qkv);
+    packed = static_cast<char*>(keep.data_ptr());
+  }
   castle_tensor_t news[6];
   for (int i = 0; i < 6; ++i) news[i] = {packed + kPackedOrder[i] * inner * es, 6 * inner, d, 6 * inner};
-  launch_decode(cp, news, caches, core, t, rotary, ws.data_ptr(), part, stream);
-  Tensor y = at::empty({B, 1, l.combine.size(0)}, x.options().requires_grad(false));
-  check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)inner, (int32_t)l.combine.size(0), core, inner, nullptr, 0.f,
-                         l.combine.data_ptr(), y.data_ptr(), stream.stream()), "castle_token_linear");
-  return y;
+  if (own_projection(cp.dtype, B, inner, l.combine.size(0), es)) {
+    launch_decode(cp, news, caches, core, t, rotary, ws.data_ptr(), part, stream);
+    Tensor y = at::empty({B, 1, l.combine.size(0)}, x.options().requires_grad(false));
+    check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)inner, (int32_t)l.combine.size(0), core, inner, nullptr, 0.f,
+                           l.combine.data_ptr(), y.data_ptr(), stream.stream()), "castle_token_linear");
+    return y;
+  }
+  const Tensor o = at::empty({B, inner}, x.options().requires_grad(false));
+  launch_decode(cp, news, caches, o.data_ptr(), t, rotary, ws.data_ptr(), part, stream);
+  return matmul_t(o, l.combine).view({B, 1, l.combine.size(0)});
 }
 
 Tensor layer_decode(const Tensor& x, const Layer& l, const Tensor* caches, int64_t t, double scale, const Rotary& rotary) {
   // no gradient flows through the cached step, so only the last projection could need a graph
-  if (plain_token(x, l) && !(at::GradMode::is_enabled() && l.combine.requires_grad())) return token_layer(x, l, caches, t, scale, rotary);
+  if (plain_layer(x, l) && x.size(1) == 1 && !(at::GradMode::is_enabled() && l.combine.requires_grad()))
+    return token_layer(x, l, caches, t, scale, rotary);
   return at::linear(decode_packed(project(x, l), caches, t, scale, rotary), l.combine);
 }
 

@@ -6,7 +6,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
-@pytest.mark.parametrize("rows,k,n", [(1, 8, 1), (1, 512, 3072), (2, 520, 17), (3, 96, 2400), (5, 1000, 64), (8, 3072, 129)])
+@pytest.mark.parametrize("rows,k,n", [(1, 8, 1), (1, 512, 3072), (2, 520, 17), (3, 96, 2400), (5, 1000, 64), (8, 3072, 129), (4, 40, 15), (6, 264, 7000)])
 @pytest.mark.parametrize("norm", [False, True])
 def test_token_linear(dtype, rows, k, n, norm):
     from lookahead_keys_attention_b200 import _lib as L
@@ -28,5 +28,7 @@ def test_token_linear(dtype, rows, k, n, norm):
 def test_token_linear_refuses_what_does_not_fit():
     from lookahead_keys_attention_b200 import _lib as L
     lib = L.load()
-    assert lib.castle_token_linear_fits(L.BF16, 8, 3072) and not lib.castle_token_linear_fits(L.BF16, 9, 64)
-    assert not lib.castle_token_linear_fits(L.BF16, 8, 3080) and not lib.castle_token_linear_fits(L.F32, 1, 12)
+    assert lib.castle_token_linear_fits(L.F32, 8, 3072) and not lib.castle_token_linear_fits(L.F32, 9, 64)
+    assert not lib.castle_token_linear_fits(L.F32, 8, 3080) and not lib.castle_token_linear_fits(L.F32, 1, 12)
+    assert lib.castle_token_linear_fits(L.BF16, 8, 8192) and not lib.castle_token_linear_fits(L.BF16, 9, 64)
+    assert not lib.castle_token_linear_fits(L.BF16, 8, 16384)
