@@ -196,26 +196,30 @@ int castle_decode_step(const castle_problem_t* p, int32_t cache_len, int32_t cap
 /* The same step with two additions.  `rotary` (may be NULL): the new rows (all but vc_new) are rotated to position
  * rotary->position0 as they are read (lookahead_keys_attention.py:106-112), so that the caches hold rotated rows.
  * `counters` (may be NULL): batch * heads words that are zero before the call and zero again when its kernel has
- * run, so calls on one stream can share them; with them the step is one launch instead of two.
+ * run, so calls on one stream can share them; with them the step is one launch instead of two.  `overlap` != 0: the
+ * launch before it on the stream is castle_token_linear() writing the new rows (and nothing the step reads besides), and
+ * the step may become resident and fetch cache rows before that ends.
  */
 int castle_decode_step_fused(const castle_problem_t* p, int32_t cache_len, int32_t capacity,
                              const castle_tensor_t* qc_new, const castle_tensor_t* kc_new, const castle_tensor_t* vc_new,
                              const castle_tensor_t* qu_new, const castle_tensor_t* ku_new, const castle_tensor_t* vu_new,
                              const castle_tensor_t* u_cache, const castle_tensor_t* qu_cache,
                              const castle_tensor_t* kc_cache, const castle_tensor_t* vc_cache, const castle_tensor_t* out,
-                             const castle_rotary_t* rotary, uint32_t* counters, void* workspace, size_t workspace_bytes,
-                             int32_t* status, void* stream);
+                             const castle_rotary_t* rotary, uint32_t* counters, int32_t overlap, void* workspace,
+                             size_t workspace_bytes, int32_t* status, void* stream);
 
 /* ---- a token's projections ----------------------------------------------------
  * y = norm(x) @ weight^T for 1 to 8 rows: the projections around the cached step
  * (lookahead_keys_attention/lookahead_keys_attention.py:67-80, :99-104, :207) as one launch each.  x: rows of
  * in_features elements, row_stride elements apart; weight: contiguous (out_features, in_features); y: contiguous
  * (rows, out_features); norm_weight: RMSNorm's, in_features elements, or NULL for none.  All of `dtype`, sums in
- * fp32.  castle_token_linear_fits says whether a size is supported.
+ * fp32.  castle_token_linear_fits says whether a size is supported.  `overlap` != 0: the launch before it on the
+ * stream writes x (and not the weights), and this one may become resident and fetch weights before that ends.
  */
 int castle_token_linear_fits(int32_t dtype, int32_t rows, int32_t in_features);
 int castle_token_linear(int32_t dtype, int32_t rows, int32_t in_features, int32_t out_features, const void* x,
-                        int64_t row_stride, const void* norm_weight, float eps, const void* weight, void* y, void* stream);
+                        int64_t row_stride, const void* norm_weight, float eps, const void* weight, void* y, int32_t overlap,
+                        void* stream);
 
 /* ---- cached single-token step without caller scratch -----------------------
  * (no counterpart in the reference)  Same step and same arguments as

@@ -178,9 +178,9 @@ _SIGNATURES = {
     "castle_bwd": (ctypes.c_int, [_PR] + [_T] * 8 + [_vp, _vp] + [_T] * 6 + [_vp, _sz, _vp, _vp]),
     "castle_decode_workspace_bytes": (_sz, [_PR, _i32]),
     "castle_decode_step": (ctypes.c_int, [_PR, _i32, _i32] + [_T] * 11 + [_vp, _sz, _vp, _vp]),
-    "castle_decode_step_fused": (ctypes.c_int, [_PR, _i32, _i32] + [_T] * 11 + [P(CastleRotary), _vp, _vp, _sz, _vp, _vp]),
+    "castle_decode_step_fused": (ctypes.c_int, [_PR, _i32, _i32] + [_T] * 11 + [P(CastleRotary), _vp, _i32, _vp, _sz, _vp, _vp]),
     "castle_token_linear_fits": (ctypes.c_int, [_i32] * 3),
-    "castle_token_linear": (ctypes.c_int, [_i32] * 4 + [_vp, ctypes.c_int64, _vp, ctypes.c_float, _vp, _vp, _vp]),
+    "castle_token_linear": (ctypes.c_int, [_i32] * 4 + [_vp, ctypes.c_int64, _vp, ctypes.c_float, _vp, _vp, _i32, _vp]),
     "castle_decode_step_static": (ctypes.c_int, [_PR, _i32, _i32] + [_T] * 11 + [_vp, _vp]),
     "castle_set_kernel_events": (ctypes.c_int, [_i32, _vp, _vp]),
     "castle_selftest_mma_rate": (ctypes.c_int, [_i32, _i32, _i32, _vp, _vp, _vp]),

@@ -33,6 +33,20 @@ inline int cuda_fail(cudaError_t e, const char* what) {
   return (int)e;
 }
 
+// Launch that may start while the kernel before it on the stream is still running (programmatic dependent launch): its CTAs
+// become resident when all CTAs of that kernel have called overlap_next() or ended, and overlap_wait() holds them until
+// that kernel's writes are visible.  Before overlap_wait() a kernel may only touch what older kernels wrote.
+template <typename... P, typename... A>
+inline cudaError_t launch_kernel(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool overlap, A... args) {
+  cudaLaunchConfig_t c = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  c.gridDim = grid; c.blockDim = dim3(threads); c.dynamicSmemBytes = smem; c.stream = st;
+  c.attrs = attr; c.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 inline int elem_size(int dtype) { return dtype == CASTLE_F32 ? 4 : 2; }
 
 inline bool tensor_ok(const castle_tensor_t* t, int dtype, const char* name, int* rc) {

@@ -25,6 +25,7 @@ struct DecodeParams {
   float scale;
   int32_t* status;
   RotaryParams rot;                                // rotation of the new rows (all but vc); freqs null = none
+  bool overlap;                                    // launched before the kernel that writes the new rows has ended
   uint32_t* counters;                              // [BH] zeroed: CTAs of a pair that are done; null = merge kernel
 };
 
@@ -223,6 +224,8 @@ __global__ void __launch_bounds__(kDecodeThreads, CASTLE_DECODE_MIN_CTAS) castle
     return reinterpret_cast<T*>(t.ptr) + b * t.stride_b + h * t.stride_h + r * t.stride_n + col;
   };
 
+  overlap_next();
+  overlap_wait();   // the new rows may come from the launch before (the caches do not)
   float qcv[VEC], kuv[VEC], vuv[VEC];
   Vec<T>::load(row_ptr(p.qc, 0), qcv);
   Vec<T>::load(row_ptr(p.ku, 0), kuv);
@@ -384,6 +387,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 4) castle_decode_ring_kernel(c
   if (threadIdx.x == 0)
     for (int t0 = 0; t0 < kRingStages && t0 < ntiles; ++t0) issue(t0);
 
+  overlap_next();
+  overlap_wait();   // the new rows may come from the launch before (the caches do not)
   float qcv[VEC], kuv[VEC], vuv[VEC];
   Vec<T>::load(row_ptr(p.qc, 0), qcv);
   Vec<T>::load(row_ptr(p.ku, 0), kuv);
@@ -545,17 +550,19 @@ static int launch_decode(const DecodeParams& p, int BH, bool ring, cudaStream_t 
     cudaError_t e = cudaFuncSetAttribute(castle_decode_ring_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "castle_decode_step attribute");
     ev_start(CASTLE_KERNEL_DECODE, st);
-    castle_decode_ring_kernel<T, D><<<grid, kDecodeThreads, smem, st>>>(p);
+    e = launch_kernel(castle_decode_ring_kernel<T, D>, grid, kDecodeThreads, smem, st, p.overlap, p);
+    if (e != cudaSuccess) return cuda_fail(e, "castle_decode_step launch");
     ev_stop(CASTLE_KERNEL_DECODE, st);
     if (p.nsplit > 1 && !p.counters) castle_decode_merge_kernel<T, D><<<BH, kDecodeThreads, 0, st>>>(p);
     e = cudaGetLastError();
     return e == cudaSuccess ? 0 : cuda_fail(e, "castle_decode_step launch");
   }
   ev_start(CASTLE_KERNEL_DECODE, st);
-  castle_decode_kernel<T, D><<<grid, kDecodeThreads, 0, st>>>(p);
+  cudaError_t e = launch_kernel(castle_decode_kernel<T, D>, grid, kDecodeThreads, 0, st, p.overlap, p);
+  if (e != cudaSuccess) return cuda_fail(e, "castle_decode_step launch");
   ev_stop(CASTLE_KERNEL_DECODE, st);
   if (p.nsplit > 1 && !p.counters) castle_decode_merge_kernel<T, D><<<BH, kDecodeThreads, 0, st>>>(p);
-  cudaError_t e = cudaGetLastError();
+  e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_decode_step launch");
 }
 
@@ -590,7 +597,7 @@ extern "C" int castle_decode_step(const castle_problem_t* p, int32_t cache_len, 
                                   const castle_tensor_t* out, void* workspace, size_t workspace_bytes,
                                   int32_t* status, void* stream) {
   return castle_decode_step_fused(p, cache_len, capacity, qc_new, kc_new, vc_new, qu_new, ku_new, vu_new, u_cache, qu_cache,
-                                  kc_cache, vc_cache, out, nullptr, nullptr, workspace, workspace_bytes, status, stream);
+                                  kc_cache, vc_cache, out, nullptr, nullptr, 0, workspace, workspace_bytes, status, stream);
 }
 
 extern "C" int castle_decode_step_fused(const castle_problem_t* p, int32_t cache_len, int32_t capacity,
@@ -600,7 +607,7 @@ extern "C" int castle_decode_step_fused(const castle_problem_t* p, int32_t cache
                                         const castle_tensor_t* u_cache, const castle_tensor_t* qu_cache,
                                         const castle_tensor_t* kc_cache, const castle_tensor_t* vc_cache,
                                         const castle_tensor_t* out, const castle_rotary_t* rotary, uint32_t* counters,
-                                        void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
+                                        int32_t overlap, void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
   if (!p) return reject("castle_decode_step: null problem");
   if (p->batch <= 0 || p->heads <= 0) return reject("castle_decode_step: empty batch/heads");
   if (cache_len < 0 || cache_len >= capacity)
@@ -628,6 +635,7 @@ extern "C" int castle_decode_step_fused(const castle_problem_t* p, int32_t cache
   // waves it is not (128 pairs x 8191 rows, 8 waves: 231 us against 213 + 8 us with the merge kernel).
   const int64_t slots = 148 * (ring ? kRingCtasPerSm : CASTLE_DECODE_MIN_CTAS);
   dp.counters = (int64_t)BH * dp.nsplit <= slots ? counters : nullptr;
+  dp.overlap = overlap != 0;
   dp.rot = RotaryParams{nullptr, CASTLE_F32, 0, 0.f};
   if (rotary && rotary->freqs) {
     if (rotary->dtype < CASTLE_BF16 || rotary->dtype > CASTLE_F32) return reject("castle_decode_step: unknown rotary dtype");
@@ -721,6 +729,7 @@ extern "C" int castle_decode_step_static(const castle_problem_t* p, int32_t cach
   // array needs no clearing between calls even though it keeps the previous call's contents.
   dp.part = scratch;
   dp.counters = nullptr;
+  dp.overlap = false;
   dp.rot = RotaryParams{nullptr, CASTLE_F32, 0, 0.f};
   cudaStream_t st = (cudaStream_t)stream;
   switch (p->dtype) {

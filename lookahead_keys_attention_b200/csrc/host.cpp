@@ -454,7 +454,7 @@ void check_caches(const Tensor* caches, int64_t B, int64_t H, int64_t d, at::Sca
 
 // `news` in the operator's order qc, kc, vc, qu, ku, vu; `caches` U, qu, kc, vc; `out` contiguous (B, H, 1, d).
 void launch_decode(const castle_problem_t& cp, const castle_tensor_t* news, const Tensor* caches, void* out, int64_t t, const Rotary& rotary,
-                   void* ws, size_t ws_bytes, const c10::cuda::CUDAStream& stream) {
+                   bool overlap, void* ws, size_t ws_bytes, const c10::cuda::CUDAStream& stream) {
   const Tensor words = zero_words(stream, (int64_t)cp.batch * cp.heads), status = status_word(stream.device_index());
   castle_tensor_t c[4];
   for (int i = 0; i < 4; ++i) c[i] = desc(caches[i]);
@@ -463,7 +463,7 @@ void launch_decode(const castle_problem_t& cp, const castle_tensor_t* news, cons
   if (rotary.on()) rot = rotary.desc(false);
   check(api.decode_step_fused(&cp, (int32_t)t, (int32_t)caches[0].size(2), &news[0], &news[1], &news[2], &news[3], &news[4], &news[5],
                               &c[0], &c[1], &c[2], &c[3], &od, rotary.on() ? &rot : nullptr,
-                              reinterpret_cast<uint32_t*>(words.data_ptr()) + kAmaxWords, ws, ws_bytes, status.data_ptr<int32_t>(),
+                              reinterpret_cast<uint32_t*>(words.data_ptr()) + kAmaxWords, overlap, ws, ws_bytes, status.data_ptr<int32_t>(),
                               stream.stream()), "castle_decode_step");
 }
 
@@ -475,7 +475,7 @@ Tensor decode_core(const castle_tensor_t* news, const Tensor* caches, int64_t B,
   Tensor out = at::empty({B, H, 1, d}, caches[0].options());
   const castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
   const Tensor ws = scratch(stream, api.decode_workspace_bytes(&cp, (int32_t)t));
-  launch_decode(cp, news, caches, out.data_ptr(), t, rotary, ws.data_ptr(), ws.numel(), stream);
+  launch_decode(cp, news, caches, out.data_ptr(), t, rotary, false, ws.data_ptr(), ws.numel(), stream);
   return out;
 }
 
@@ -674,9 +674,14 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   char* core = packed + 6 * row;
   Tensor keep;
   const Tensor xs = x.stride(2) == 1 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * es % 16 == 0 ? x : x.contiguous();
-  if (own_projection(cp.dtype, B, dim, 6 * inner, es)) {
+  // The step and the last projection are launched ahead (see the C ABI's `overlap`).  The buffers they fetch early must be
+  // in place before the first of the three launches: zero_words() and status_word() may launch a fill on first use.
+  const bool overlap = own_projection(cp.dtype, B, dim, 6 * inner, es);
+  zero_words(stream, B * H);
+  status_word(dev.index());
+  if (overlap) {
     check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)dim, (int32_t)(6 * inner), xs.data_ptr(), xs.stride(0),
-                           l.norm.defined() ? l.norm.data_ptr() : nullptr, norm_eps(l), l.to_qkv.data_ptr(), packed, stream.stream()),
+                           l.norm.defined() ? l.norm.data_ptr() : nullptr, norm_eps(l), l.to_qkv.data_ptr(), packed, 0, stream.stream()),
           "castle_token_linear");
   } else {
     Tensor h = xs.contiguous().view({B, dim});
@@ -692,14 +697,14 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   castle_tensor_t news[6];
   for (int i = 0; i < 6; ++i) news[i] = {packed + kPackedOrder[i] * inner * es, 6 * inner, d, 6 * inner};
   if (own_projection(cp.dtype, B, inner, l.combine.size(0), es)) {
-    launch_decode(cp, news, caches, core, t, rotary, ws.data_ptr(), part, stream);
+    launch_decode(cp, news, caches, core, t, rotary, overlap, ws.data_ptr(), part, stream);
     Tensor y = at::empty({B, 1, l.combine.size(0)}, x.options().requires_grad(false));
     check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)inner, (int32_t)l.combine.size(0), core, inner, nullptr, 0.f,
-                           l.combine.data_ptr(), y.data_ptr(), stream.stream()), "castle_token_linear");
+                           l.combine.data_ptr(), y.data_ptr(), 1, stream.stream()), "castle_token_linear");
     return y;
   }
   const Tensor o = at::empty({B, inner}, x.options().requires_grad(false));
-  launch_decode(cp, news, caches, o.data_ptr(), t, rotary, ws.data_ptr(), part, stream);
+  launch_decode(cp, news, caches, o.data_ptr(), t, rotary, overlap, ws.data_ptr(), part, stream);
   return matmul_t(o, l.combine).view({B, 1, l.combine.size(0)});
 }
 

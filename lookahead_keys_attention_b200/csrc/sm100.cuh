@@ -82,6 +82,10 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
+// ---------------------------------------------------------------- overlap of dependent launches (see launch_kernel)
+__device__ __forceinline__ void overlap_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void overlap_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- fences
 __device__ __forceinline__ void fence_async_smem() {  // generic-proxy smem writes -> async proxy (MMA/TMA) reads
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

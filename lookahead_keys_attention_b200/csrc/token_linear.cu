@@ -38,6 +38,7 @@ struct TokenLinearParams {
   int rows, K, N;
   int64_t ldx;
   float eps;
+  bool overlap;   // launched before the kernel that writes x has ended
 };
 
 // R = rows of x (padded up to 1, 2, 4 or 8), WR = rows of w per warp.
@@ -58,6 +59,8 @@ __global__ void __launch_bounds__(kTokenThreads) castle_token_linear_kernel(cons
 #pragma unroll
     for (int i = 0; i < WR; ++i) q[i] = wrow[i][lane];
   }
+  overlap_next();
+  overlap_wait();   // x may come from the launch before
   float ss[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) ss[r] = 0.f;
@@ -168,6 +171,8 @@ __global__ void __launch_bounds__(kTokenMmaThreads) castle_token_mma_kernel(cons
   T* xs = reinterpret_cast<T*>(raw);                         // [R][ldx]
   float* red = reinterpret_cast<float*>(raw + (size_t)R * ldx * sizeof(T));   // [8 warps][16][R] where K is sliced
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  overlap_next();
+  overlap_wait();   // x may come from the launch before
   // ---- x, normalised, into shared memory: a warp per row
   for (int r = warp; r < R; r += kTokenMmaThreads / 32) {
     const T* src = reinterpret_cast<const T*>(p.x) + (int64_t)min(r, p.rows - 1) * p.ldx;
@@ -280,8 +285,7 @@ static int launch_token_mma(const TokenLinearParams& p, cudaStream_t st) {
   while (q.ks < 8 && q.groups * q.ks * 2 <= 8) q.ks *= 2;
   const int side = 8 / q.ks;
   q.groups = (q.groups + side - 1) / side * side;
-  castle_token_mma_kernel<T><<<(total + q.groups - 1) / q.groups, kTokenMmaThreads, smem, st>>>(q);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_kernel(castle_token_mma_kernel<T>, dim3((total + q.groups - 1) / q.groups), kTokenMmaThreads, smem, st, p.overlap, q);
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_token_linear launch");
 }
 
@@ -293,8 +297,7 @@ static int launch_token(const TokenLinearParams& p, cudaStream_t st) {
     if (e != cudaSuccess) return cuda_fail(e, "castle_token_linear attribute");
   }
   constexpr int per_cta = kTokenThreads / 32 * WR;
-  castle_token_linear_kernel<T, R, WR><<<(p.N + per_cta - 1) / per_cta, kTokenThreads, smem, st>>>(p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_kernel(castle_token_linear_kernel<T, R, WR>, dim3((p.N + per_cta - 1) / per_cta), kTokenThreads, smem, st, p.overlap, p);
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_token_linear launch");
 }
 template <typename T, int R>
@@ -325,13 +328,13 @@ extern "C" int castle_token_linear_fits(int32_t dtype, int32_t rows, int32_t in_
 
 extern "C" int castle_token_linear(int32_t dtype, int32_t rows, int32_t in_features, int32_t out_features, const void* x,
                                    int64_t row_stride, const void* norm_weight, float eps, const void* weight, void* y,
-                                   void* stream) {
+                                   int32_t overlap, void* stream) {
   if (!castle_token_linear_fits(dtype, rows, in_features) || out_features <= 0)
     return reject("castle_token_linear: %d rows of %d -> %d not supported (see castle_token_linear_fits)", rows, in_features, out_features);
   if (!x || !weight || !y) return reject("castle_token_linear: null tensor");
   if (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)norm_weight) % 16 || row_stride * elem_size(dtype) % 16)
     return reject("castle_token_linear: pointers and the row stride must be 16-byte aligned");
-  const TokenLinearParams p{x, norm_weight, weight, y, rows, in_features, out_features, row_stride, eps};
+  const TokenLinearParams p{x, norm_weight, weight, y, rows, in_features, out_features, row_stride, eps, overlap != 0};
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == CASTLE_BF16) return launch_token_t<__nv_bfloat16>(p, st);
   if (dtype == CASTLE_F16) return launch_token_t<__half>(p, st);

@@ -17,7 +17,7 @@ def test_token_linear(dtype, rows, k, n, norm):
     g, eps = torch.rand(k, device="cuda").to(dtype) + 0.5, 1e-3
     y = torch.full((rows + 1, n), 7.0, device="cuda", dtype=dtype)
     L.check(L.load().castle_token_linear(code, rows, k, n, x.data_ptr(), k + 8, g.data_ptr() if norm else None, eps,
-                                         w.data_ptr(), y.data_ptr(), None), "token_linear")
+                                         w.data_ptr(), y.data_ptr(), 0, None), "token_linear")
     h = torch.nn.functional.rms_norm(x, (k,), g, eps) if norm else x
     ref = h.double() @ w.double().T
     tol = {torch.bfloat16: 2e-2, torch.float16: 3e-3, torch.float32: 2e-5}[dtype]
