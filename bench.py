@@ -455,7 +455,7 @@ def run_cfg4(world, dev, peaks):
             "frac_of_tensor_peak": round(tf / (peaks["tflops"] * world), 4),
             "kernels": {"fwd_main_ms": round(fwd_ms, 3), "fwd_main_tflops": round(f_fwd / (fwd_ms * 1e-3) / 1e12, 2),
                         "bwd_main_ms": round(bwd_ms, 3), "bwd_main_tflops": round(f_bwd / (bwd_ms * 1e-3) / 1e12, 2)},
-            "roofline": {"kernel": "castle_bwd128_kv_kernel + castle_bwd128_la_kernel", "bound": "tensor",
+            "roofline": {"kernel": "castle_bwd128 kv + reverse + la + dqu kernels", "bound": "tensor",
                          "achieved": round(f_bwd / (bwd_ms * 1e-3) / 1e12, 2), "peak": peaks["tflops"], "unit": "TFLOP/s",
                          "frac": round(f_bwd / (bwd_ms * 1e-3) / 1e12 / peaks["tflops"], 4),
                          "traffic": captured_traffic("bwd_d128", B * H * nblk * (nblk + 1) // 2),

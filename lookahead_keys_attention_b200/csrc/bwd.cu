@@ -514,16 +514,14 @@ static int launch_bwd(const BwdParams& p, const CUtensorMap* maps, cudaStream_t 
   }
   const int64_t rows = (int64_t)p.B * p.H * p.N;
   constexpr int RPB = 256 / (D / 8);
-  cudaError_t e = cudaMemsetAsync(p.acc_dqc, 0, (size_t)rows * D * 3 * sizeof(float), st);
-  if (e != cudaSuccess) return cuda_fail(e, "castle_bwd memset");
-  castle_bwd_delta_kernel<T, D><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
+  castle_bwd_delta_kernel<T, D, 3><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
   dim3 grid(p.B * p.H, p.nblk);
   ev_start(CASTLE_KERNEL_BWD, st);
   castle_bwd_kernel<T, D><<<grid, kBwdThreads, smem, st>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6],
                                                          maps[7], maps[8], maps[9]);
   ev_stop(CASTLE_KERNEL_BWD, st);
   castle_bwd_finish_kernel<T, D, 3><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_bwd launch");
 }
 

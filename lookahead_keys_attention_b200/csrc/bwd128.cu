@@ -1,131 +1,154 @@
-// CASTLE parallel backward for dim_head 128.
+// CASTLE parallel backward for dim_head 128: four kernels that hand 16-bit tiles on through global memory.
 //
-// At d = 128 the five per-key-block accumulators of the d = 64 kernel (W, G, dkc, dvc, dqu) would
-// need 640 TMEM columns, and seven 32 KB operand tiles already fill shared memory.  The pass is
-// therefore split into two kernels, each walking the query blocks I downwards for one key block K:
+//   kv       per key block K, query blocks I downwards: the scores (gate A, the peeled state W, T, Su, Sc), P, dS, dSu; dkc and
+//            dvc in tensor memory, dqc[I] by TMA reduce.  A and dSu -> tiles.
+//   reverse  per K, I downwards: G += dSu^T Qc[I]; the 16-bit copy of G before each step -> tiles.
+//   la       per query block I, over K: dA = Gb Vu^T + dSu^T T, dZ (-> tiles, over A); dku[I], dvu[I] and dT summed in tensor
+//            memory; at the end the masked dT's share of dvu and dqc, and all three gradients are written.
+//   dqu      per K: dqu = sum over I of dZ Ku[I].
 //
-//   castle_bwd128_kv_kernel   TMEM: W | dkc | dvc | scratch.  Recomputes the scores (Z, gate, peeled
-//                             state W, T, Su, Sc) the way the d = 64 kernel does, accumulates dkc and
-//                             dvc in TMEM, builds dqc[I] = dS@Kc + dSu@Wb + dT@Vu in the scratch and
-//                             adds it to the fp32 workspace with a TMA reduce.  It also stores the gate A,
-//                             dSu and the masked T of every (I, K) step to a global scratch, as the
-//                             16-bit tiles lie in shared memory (3 x 32 KB per step).
-//   castle_bwd128_la_kernel   TMEM: dqu | G | scratch | scratch.  Runs after it on the same stream,
-//                             loads those three tiles and recomputes nothing: carries the reverse
-//                             state G and dqu[K] in TMEM and reduces dvu[I], dku[I] per step.
+// Every gradient but dqc is owned by a CTA that keeps it in tensor memory.  A TMA reduce moves some 18 bytes per cycle and SM,
+// so a lookahead kernel that owned a key block and reduced dku[I] and dvu[I] (128 KB a step, with dT masked and multiplied in
+// every step) took 18.5 k cycles a step, 12.1 k without the reduces; reverse + la + dqu take 3.1 + 8.0 + 1.9 k, and kv, which
+// no longer forms dT, went from 20.8 to 18.9 k.  Measured on B=1 H=8 N=8190 bf16: 2365 -> 1882 us for the kernels, B=2 H=8 N=1333:
+// 249 -> 205 us.  What bounds them: kv its chain of six products with a pass behind each; la and reverse the tiles, which
+// come at 20 to 30 bytes per cycle and SM with one step's worth of shared memory to prefetch into; dqu HBM.  (Handing W on
+// as well, from a kernel of its own, so that kv starts at Su: 4.4 + 17 k cycles instead of 18.9 k.)
 //
-// The scratch is bounded (see kTileScratchLimit): the (batch, head) pairs run in chunks, one launch
-// of each kernel per chunk.
-//
-// Shared memory is seven 32 KB slots that are re-used as tiles die; each comment "-> sN" below
-// says which slot a tile lands in.  512 threads: warp w owns TMEM lanes 32*(w%4).. and columns
-// 32*(w/4).. of every 128-column accumulator.
+// Tiles of a step (I,K): A, then dZ | dSu | Gb; 32 KB each, as they lie in shared memory (128-byte swizzle).  The scratch is
+// bounded (kTileScratchLimit): the (batch, head) pairs run in chunks, one launch of each kernel per chunk.
 #include "bwd_common.cuh"
 
 namespace castle {
 
-constexpr int kB128Threads = 512;
-constexpr uint32_t kSlot = 2 * kPanelB;                      // 32 KB
-constexpr size_t kB128Smem = 7 * kSlot + 1024;
+constexpr uint32_t kSq = 2 * kPanelB;   // a 128x128 tile: 32 KB
+constexpr uint32_t kTileA = 0, kTileDsu = kSq, kTileG = 2 * kSq, kStepTiles = 3 * kSq;
+constexpr int kB128Threads = 512;      // a thread: a row and 32 columns
+constexpr size_t kB128Smem = 7 * kSq + 256;
 
-// Timing experiments only (never in the shipped library): drop the reduces to see what they cost.
-#ifdef CASTLE_TIMING_SKIP_REDUCE
-#define tma_reduce_add_3d(...) do { } while (0)
-#endif
-
-// Optional phase timing (debug builds only): thread 0 of CTA (0,0) stores clock64() at phase boundaries of
-// its first steps behind the fp32 workspace (key/value kernel at slot 0, lookahead kernel at slot 256).
-#ifdef CASTLE_PHASE_TIMING
-#define B128_MARK(base, i) do { if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && p.nblk - 1 - I < 8) p.timing[(base) + (p.nblk - 1 - I) * 32 + (i)] = clock64(); } while (0)
-#else
-#define B128_MARK(base, i) do { } while (0)
-#endif
-
-#define B128_MMA_WAIT()                  \
-  mbar_wait(&bar_mma, ph_mma, abortp);   \
-  ph_mma ^= 1;                           \
-  tc_fence_after();
-#define B128_SYNC()    \
-  fence_async_smem();  \
-  tc_fence_before();   \
-  __syncthreads();
-
-template <int NP>
-__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* m, uint64_t* bar, int r0, int h, int b) {
+// 32 values times `mul` to a row of a 16-bit tensor
+template <typename T>
+__device__ __forceinline__ void store_grad32(T* dst, const float* v, float mul) {
 #pragma unroll
-  for (int pn = 0; pn < NP; ++pn) tma_load_4d(dst + pn * kPanelB, m, bar, pn * 64, r0, h, b);
+  for (int j = 0; j < 4; ++j) {
+    uint4 q;
+    q.x = Elem<T>::pack2(v[8 * j] * mul, v[8 * j + 1] * mul);
+    q.y = Elem<T>::pack2(v[8 * j + 2] * mul, v[8 * j + 3] * mul);
+    q.z = Elem<T>::pack2(v[8 * j + 4] * mul, v[8 * j + 5] * mul);
+    q.w = Elem<T>::pack2(v[8 * j + 6] * mul, v[8 * j + 7] * mul);
+    *reinterpret_cast<uint4*>(dst + j * 8) = q;
+  }
+}
+template <typename T>
+__device__ __forceinline__ T* grad_row(const castle_tensor_t& t, int b, int h, int row, int c0) {
+  return reinterpret_cast<T*>(t.ptr) + b * t.stride_b + h * t.stride_h + (int64_t)row * t.stride_n + c0;
 }
 
-// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void load_op(uint8_t* dst, const CUtensorMap& m, uint64_t* bar, int r0, int h, int b) {
+#pragma unroll
+  for (int pn = 0; pn < 2; ++pn) tma_load_4d(dst + pn * kPanelB, &m, bar, pn * 64, r0, h, b);
+}
+__device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K) {   // of this CTA's pair
+  return p.tiles + ((int64_t)blockIdx.x * p.ntiles + (int64_t)I * (I + 1) / 2 + K) * kStepTiles;
+}
+// What every kernel starts with: shared memory behind the operands, barriers, tensor memory.  NBAR barriers (of one arrival).
+#define B128_BEGIN(OPERANDS, NBAR, COLS)                                                      \
+  extern __shared__ __align__(1024) uint8_t smem[];                                            \
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + (OPERANDS));                       \
+  uint32_t* const tmem_base_s = reinterpret_cast<uint32_t*>(bars + (NBAR));                    \
+  volatile int* const abortp = reinterpret_cast<int*>(bars + (NBAR)) + 1;                      \
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  \
+  const int bh = p.bh0 + blockIdx.x, b = bh / p.H, h = bh % p.H;                               \
+  if (tid == 0) {                                                                              \
+    if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);                  \
+    for (int i = 0; i < (NBAR); ++i) mbar_init(bars + i, 1);                                   \
+    mbar_fence_init();                                                                         \
+    *abortp = 0;                                                                               \
+  }                                                                                            \
+  if (warp == 0) { tmem_alloc(tmem_base_s, COLS); tmem_relinquish(); }                         \
+  overlap_wait();                                                                              \
+  tc_fence_before();                                                                           \
+  __syncthreads();                                                                             \
+  tc_fence_after();                                                                            \
+  const uint32_t tmem = *tmem_base_s, trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+
+#define B128_END(COLS)                                                                        \
+  overlap_next();                                                                              \
+  tc_fence_before();                                                                           \
+  __syncthreads();                                                                             \
+  if (warp == 0) tmem_dealloc(tmem, COLS);                                                     \
+  if (tid == 0 && *abortp) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
+
+// Phase timing (debug builds only): thread 0 of CTA (0,0) stores clock64() at the phase boundaries of its first steps behind
+// the workspace.
+#ifdef CASTLE_PHASE_TIMING
+#define B128_MARK(base, n, i) do { if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && (n) < 8) p.timing[(base) + (n) * 32 + (i)] = clock64(); } while (0)
+#else
+#define B128_MARK(base, n, i) do { } while (0)
+#endif
+
+#define B128_SYNC()    \
+  fence_async_smem();   \
+  tc_fence_before();    \
+  __syncthreads();
+
+// ------------------------------------------------------------------------------------------------ scores, dkc, dvc, dqc
+// One chain per step, six products with a pass behind each:
+//   Z | gate A;  T, W -= A Vu | T masked, Wb;  Su | silu';  Sc (while silu' is formed) | P;  dP, dvc | dS, dSu;  dqc, dkc | staging
+// Tensor memory: W | dkc | dvc | scratch.  Shared memory, seven tiles:
+//   s0 Qu, then Wb | s1 Ku, A, dS | s2 Vu, T, P | s3 Qc | s4 Kc | s5 Vc, staging | s6 dO, dSu, staging
+// TMA works its queue off in order, and a reduce moves some 18 bytes a cycle: a load queued behind the 64 KB of dqc waits
+// 3.6 k cycles.  So the loads that the next step starts with (Qu, Ku, Vu, Qc) are issued before the reduces, and what is
+// staged over are the tiles that it needs last: dO, and Vc, which is loaded again for that (step 21.7 k cycles with the
+// loads behind the reduces, 19.5 k with Qu, Ku and Qc before them).
 template <typename T>
 __global__ void __launch_bounds__(kB128Threads, 1)
 castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
                         const __grid_constant__ CUtensorMap m_vc, const __grid_constant__ CUtensorMap m_qu,
                         const __grid_constant__ CUtensorMap m_ku, const __grid_constant__ CUtensorMap m_vu,
                         const __grid_constant__ CUtensorMap m_do, const __grid_constant__ CUtensorMap m_acc_dqc) {
-  constexpr int D = 128;
   constexpr int FMT = Elem<T>::fmt;
-  constexpr uint32_t ID_KK = make_idesc(128, 128, FMT, false, false, false);
-  constexpr uint32_t ID_KM = make_idesc(128, 128, FMT, false, true, false);
-  constexpr uint32_t ID_KM_NEG = make_idesc(128, 128, FMT, false, true, true);
-  constexpr uint32_t ID_MM = make_idesc(128, 128, FMT, true, true, false);
-  constexpr float kLog2e = 1.4426950408889634f;
   constexpr uint32_t C_W = 0, C_DKC = 128, C_DVC = 256, C_S = 384;
-
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* s0 = smem;              // Qu[K] -> Wb
-  uint8_t* s1 = s0 + kSlot;        // Ku[I] -> gate A -> dT
-  uint8_t* s2 = s1 + kSlot;        // Vu[I] -> masked T -> P -> Vu[I] again
-  uint8_t* s3 = s2 + kSlot;        // Qc[I]
-  uint8_t* s4 = s3 + kSlot;        // Kc[K]
-  uint8_t* s5 = s4 + kSlot;        // Vc[K] -> dS -> dqc staging
-  uint8_t* s6 = s5 + kSlot;        // dO[I] -> dSu -> dqc staging
-  __shared__ uint64_t bar_a, bar_b, bar_vu2, bar_mma, bar_x1, bar_x2;
-  __shared__ uint32_t tmem_base_s;
-  __shared__ int abort_flag;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, cc = warp >> 2;
-  const int row = quarter * 32 + lane, c0 = cc * 32;
-  const int bh = p.bh0 + blockIdx.x, K = blockIdx.y;
-  const int b = bh / p.H, h = bh % p.H;
-  const int k0 = K * kBlkB, krow = k0 + row;
-  const bool issuer = (quarter == 0 && lane == 0);   // threads 0, 128, 256, 384: one reduce each per step
-  // One lane hands three tiles of every step to the lookahead kernel through global memory, bytes as they lie
-  // in shared memory: the gate A, the masked T and dSu.  That kernel then recomputes nothing.
-  const bool storer = (tid == 64);
-  uint8_t* const tile_base = p.tiles + (int64_t)blockIdx.x * p.ntiles * 3 * kSlot;
-
-  if (tid == 0) {
-    mbar_init(&bar_a, 1); mbar_init(&bar_b, 1); mbar_init(&bar_vu2, 1); mbar_init(&bar_mma, 1);
-    mbar_init(&bar_x1, 1); mbar_init(&bar_x2, 1);
-    mbar_fence_init();
-    abort_flag = 0;
-  }
-  if (warp == 0) { tmem_alloc(&tmem_base_s, 512); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
-  const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-  volatile int* abortp = &abort_flag;
-
-  if (tid == 0) {
+  constexpr uint32_t ID_KK = make_idesc(128, 128, FMT, false, false, false), ID_KM = make_idesc(128, 128, FMT, false, true, false),
+                     ID_KM_NEG = make_idesc(128, 128, FMT, false, true, true), ID_MM = make_idesc(128, 128, FMT, true, true, false);
+  constexpr float kLog2e = 1.4426950408889634f;
+  const int K = blockIdx.y, k0 = K * kBlkB, steps = p.nblk - K;
+  B128_BEGIN(7 * kSq, 12, 512)
+  uint8_t *s0 = smem, *s1 = s0 + kSq, *s2 = s1 + kSq, *s3 = s2 + kSq, *s4 = s3 + kSq, *s5 = s4 + kSq, *s6 = s5 + kSq;
+  const uint32_t a0 = smem_u32(s0), a1 = smem_u32(s1), a2 = smem_u32(s2), a3 = smem_u32(s3), a4 = smem_u32(s4), a5 = smem_u32(s5),
+                 a6 = smem_u32(s6);
+  uint64_t *bar_res = bars, *bar_z = bars + 1 /* Qu, Ku */, *bar_qc = bars + 2, *bar_vu = bars + 3, *bar_do = bars + 4,
+           *bar_mma = bars + 5 /* Z, Su, Sc, dP: one after another */, *bar_t = bars + 6, *bar_w = bars + 7, *bar_dv = bars + 8,
+           *bar_x0 = bars + 9, *bar_x = bars + 10, *bar_k = bars + 11;
+  const int row = (warp & 3) * 32 + lane, cc = warp >> 2, c0 = cc * 32, krow = k0 + row;
+  // Lanes with a duty besides the products (warp 0's): the panel of dqc that chunk group cc stages and that panel's
+  // refill with Vc or dO; the copies of A and dSu; the other loads.
+  const bool reducer = (warp & 3) == 1, storer = warp == 8, loader = warp == 2;
+  auto load_panel = [&](int i0) {
+    if (cc < 2) tma_load_4d(s5 + cc * kPanelB, &m_vc, bar_do, cc * 64, k0, h, b);
+    else tma_load_4d(s5 + cc * kPanelB, &m_do, bar_do, (cc - 2) * 64, i0, h, b);
+  };
+  if (loader && elect_one()) {
     const int il = (p.nblk - 1) * kBlkB;
-    mbar_expect_tx(&bar_a, 5 * kSlot);
-    load_tile<2>(s0, &m_qu, &bar_a, k0, h, b);
-    load_tile<2>(s1, &m_ku, &bar_a, il, h, b);
-    load_tile<2>(s2, &m_vu, &bar_a, il, h, b);
-    load_tile<2>(s3, &m_qc, &bar_a, il, h, b);
-    load_tile<2>(s4, &m_kc, &bar_a, k0, h, b);
+    mbar_expect_tx(bar_z, 2 * kSq);
+    load_op(s0, m_qu, bar_z, k0, h, b);
+    load_op(s1, m_ku, bar_z, il, h, b);
+    mbar_expect_tx(bar_qc, kSq);
+    load_op(s3, m_qc, bar_qc, il, h, b);
+    mbar_expect_tx(bar_vu, kSq);
+    load_op(s2, m_vu, bar_vu, il, h, b);
+    mbar_expect_tx(bar_do, 2 * kSq);
+    mbar_expect_tx(bar_res, kSq);
+    load_op(s4, m_kc, bar_res, k0, h, b);
   }
-  {  // W_K starts as the forward's final state
-    const float* src = p.w_state + ((int64_t)bh * p.N + krow) * D + c0;
+  if (reducer && elect_one()) load_panel((p.nblk - 1) * kBlkB);
+  __syncwarp();
+  {  // W starts as the forward's final state
+    const float* src = p.w_state + ((int64_t)bh * p.N + krow) * 128 + c0;
     float v[32];
 #pragma unroll
     for (int j = 0; j < 32; j += 4) {
-      float4 q = (krow < p.N) ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 q = (krow < p.N) ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
       v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w;
     }
     tmem_st32(trow + C_W + c0, v);
@@ -134,31 +157,35 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
   tc_fence_before();
   __syncthreads();
 
-  uint32_t ph_a = 0, ph_b = 0, ph_vu2 = 0, ph_mma = 0, ph_x = 0;
-  const uint32_t a0 = smem_u32(s0), a1 = smem_u32(s1), a2 = smem_u32(s2), a3 = smem_u32(s3), a4 = smem_u32(s4),
-                 a5 = smem_u32(s5), a6 = smem_u32(s6);
+  uint32_t ph_mma = 0;
   const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
-
-  for (int I = p.nblk - 1; I >= K; --I) {
-    const int i0 = I * kBlkB, irow = i0 + row;
-    const bool diag = (I == K), first = (I == p.nblk - 1);
-    const bool rvalid = irow < p.N;
+  for (int n = 0; n < steps; ++n) {
+    const uint32_t ph = n & 1;
+    const int I = p.nblk - 1 - n, i0 = I * kBlkB, irow = i0 + row;
+    const bool diag = I == K, rvalid = irow < p.N, more = n + 1 < steps;
     const float lse_b = rvalid ? p.lse[(int64_t)bh * p.N + irow] * kLog2e : 0.f;
     const float delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
-
-    B128_MARK(0, 0);
-    // ---- M0: Z = Qu[K] @ Ku[I]^T
-    if (tid == 0) {
-      mbar_wait(&bar_a, ph_a, abortp);
-      B128_MARK(0, 1);
+    uint8_t* const tile = step_tiles(p, I, K);
+    B128_MARK(0, n, 0);
+    // ---- Z = Qu Ku^T
+    if (warp == 0 && elect_one()) {
+      mbar_wait(bar_z, ph, abortp);
       tc_fence_after();
       gemm_kk_t<2>(tmem + C_S, a0, a1, ID_KK, false);
-      mma_commit(&bar_mma);
+      mma_commit(bar_mma);
     }
-    ph_a ^= 1;
-    B128_MMA_WAIT();
-    B128_MARK(0, 2);
-    {  // gate A -> s1 (over Ku)
+    __syncwarp();
+    B128_MARK(0, n, 1);
+    mbar_wait(bar_mma, ph_mma, abortp);
+    ph_mma ^= 1;
+    tc_fence_after();
+    B128_MARK(0, n, 2);
+    if (reducer && n > 0 && elect_one()) {   // the reduce of the step before has had time to read its panel
+      bulk_wait_read0();
+      load_panel(i0);
+    }
+    __syncwarp();
+    {
       float v[32];
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
@@ -173,50 +200,62 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       }
       store_row32<T>(s1, kPanelB, row, c0, v);
     }
-    if (issuer) bulk_wait_read0();  // this lane's dqc panel of the step before (in s5|s6) has been read
-    B128_SYNC();
-    B128_MARK(0, 3);
-    uint8_t* const tile = tile_base + ((int64_t)I * (I + 1) / 2 + K) * 3 * kSlot;
-    if (storer) { bulk_s2g(tile, s1, kSlot); bulk_commit(); }   // gate A
-
-    // ---- M1: peel W -= A @ Vu[I];  T = Qc[I] @ Vu[I]^T
-    if (tid == 0) {
+    B128_SYNC()
+    B128_MARK(0, n, 3);
+    // ---- T = Qc Vu^T;  W -= A Vu
+    if (warp == 0 && elect_one()) {
+      mbar_wait(bar_qc, ph, abortp);
+      mbar_wait(bar_vu, ph, abortp);
       tc_fence_after();
-      gemm_km_t<8>(tmem + C_W, a1, a2, ID_KM_NEG, true);
       gemm_kk_t<2>(tmem + C_S, a3, a2, ID_KK, false);
-      mma_commit(&bar_mma);
-      mbar_expect_tx(&bar_b, 2 * kSlot);   // needed at the fifth phase; issued behind the products
-      load_tile<2>(s5, &m_vc, &bar_b, k0, h, b);
-      load_tile<2>(s6, &m_do, &bar_b, i0, h, b);
+      mma_commit(bar_t);
+      gemm_km_t<8>(tmem + C_W, a1, a2, ID_KM_NEG, true);
+      mma_commit(bar_w);
     }
-    B128_MMA_WAIT();
-    B128_MARK(0, 4);
-    {  // masked T -> s2 (over Vu); 16-bit copy of the peeled state -> s0 (over Qu)
-      float v[32];
+    if (storer && elect_one()) { bulk_s2g(tile + kTileA, s1, kSq); bulk_commit(); }
+    __syncwarp();
+    mbar_wait(bar_t, ph, abortp);
+    tc_fence_after();
+    B128_MARK(0, n, 4);
+    {  // T over Vu, Wb over Qu
+      float v[32], w[32];
       tmem_ld32_lower(trow + C_S + c0, row, c0, v);
+      mbar_wait(bar_w, ph, abortp);
+      tc_fence_after();
+      tmem_ld32(trow + C_W + c0, w);
       store_row32<T>(s2, kPanelB, row, c0, v);
-      tmem_ld32(trow + C_W + c0, v);
       tmem_ld_wait();
-      store_row32<T>(s0, kPanelB, row, c0, v);
+      store_row32<T>(s0, kPanelB, row, c0, w);
     }
-    B128_SYNC();
-    B128_MARK(0, 5);
-    if (storer) { bulk_s2g(tile + 2 * kSlot, s2, kSlot); bulk_commit(); }   // masked T
-
-    // ---- M2: Su/scale = Qc[I] @ Wb^T + Tm @ A^T
-    if (tid == 0) {
+    B128_SYNC()
+    B128_MARK(0, n, 5);
+    // ---- Su/scale = Qc Wb^T + T A^T
+    if (warp == 0 && elect_one()) {
       tc_fence_after();
       if (!diag) gemm_kk_t<2>(tmem + C_S, a3, a0, ID_KK, false);
       gemm_kk_t<2>(tmem + C_S, a2, a1, ID_KK, !diag);
-      mma_commit(&bar_mma);
+      mma_commit(bar_mma);
     }
-    B128_MMA_WAIT();
-    B128_MARK(0, 6);
+    __syncwarp();
+    mbar_wait(bar_mma, ph_mma, abortp);
+    ph_mma ^= 1;
+    tc_fence_after();
+    B128_MARK(0, n, 6);
     uint32_t dpk[16], ppk[16];
     {
-      float v[32];
+      float v[32], w[32];
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
+      tc_fence_before();
+      __syncthreads();
+      // ---- Sc/scale = Qc Kc^T, while silu' is formed
+      if (warp == 0 && elect_one()) {
+        if (n == 0) mbar_wait(bar_res, 0, abortp);
+        tc_fence_after();
+        gemm_kk_t<2>(tmem + C_S, a3, a4, ID_KK, false);
+        mma_commit(bar_mma);
+      }
+      __syncwarp();
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
         const float2 u = make_float2(v[j], v[j + 1]);
@@ -227,29 +266,15 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         const float2 d = fma2(mul2(q, splat(-p.scale)), fma2(g, splat(-1.f), splat(1.f)), g);
         dpk[j / 2] = Elem<T>::pack2(d.x, d.y);
       }
-      tmem_st32(trow + C_S + c0, v);
-      tmem_st_wait();
-    }
-    if (storer) bulk_wait_read0();   // the copies of the gate and of the masked T have read their slots (P goes over T next)
-    tc_fence_before();
-    __syncthreads();
-    B128_MARK(0, 7);
-
-    // ---- M3: S/scale = penalty + Qc[I] @ Kc[K]^T
-    if (tid == 0) {
+      B128_MARK(0, n, 7);
+      mbar_wait(bar_mma, ph_mma, abortp);
+      ph_mma ^= 1;
       tc_fence_after();
-      gemm_kk_t<2>(tmem + C_S, a3, a4, ID_KK, true);
-      mma_commit(&bar_mma);
-    }
-    B128_MMA_WAIT();
-    B128_MARK(0, 8);
-    {  // P -> s2 (over the masked T)
-      float v[32];
-      tmem_ld32(trow + C_S + c0, v);
+      tmem_ld32(trow + C_S + c0, w);
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
-        const float2 x = fma2(make_float2(v[j], v[j + 1]), splat(sl2), splat(-lse_b));
+        const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(sl2), splat(-lse_b));
         v[j] = ex2_approx(x.x); v[j + 1] = ex2_approx(x.y);
       }
       if (diag) {
@@ -262,27 +287,27 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       }
 #pragma unroll
       for (int j = 0; j < 32; j += 2) ppk[j / 2] = Elem<T>::pack2(v[j], v[j + 1]);
-      store_row32<T>(s2, kPanelB, row, c0, v);
+      store_row32<T>(s2, kPanelB, row, c0, v);   // P, over T
     }
-    B128_SYNC();
-    B128_MARK(0, 9);
-
-    // ---- M4: dvc += P^T @ dO[I];  dP = dO[I] @ Vc[K]^T
-    if (tid == 0) {
-      mbar_wait(&bar_b, ph_b, abortp);
+    if (storer && elect_one()) bulk_wait_read0();   // A has been read: dS goes there
+    __syncwarp();
+    B128_SYNC()
+    B128_MARK(0, n, 8);
+    // ---- dP = dO Vc^T;  dvc += P^T dO
+    if (warp == 0 && elect_one()) {
+      mbar_wait(bar_do, ph, abortp);
       tc_fence_after();
-      mbar_expect_tx(&bar_vu2, kSlot);   // armed here, the two loads are issued below by other lanes
-      gemm_mm_t<8>(tmem + C_DVC, a2, a6, ID_MM, !first);
       gemm_kk_t<2>(tmem + C_S, a6, a5, ID_KK, false);
-      mma_commit(&bar_mma);
+      mma_commit(bar_mma);
+      gemm_mm_t<8>(tmem + C_DVC, a2, a6, ID_MM, n > 0);
+      mma_commit(bar_dv);
     }
-    ph_b ^= 1;
-    B128_MMA_WAIT();
-    B128_MARK(0, 10);
-    // P is consumed: Vu[I] comes back into s2 for the last product (one panel per lane: a TMA
-    // instruction costs its issuing thread ~150 cycles)
-    if (lane == 0 && (warp == 5 || warp == 9)) tma_load_4d(s2 + (warp == 9) * kPanelB, &m_vu, &bar_vu2, (warp == 9) * 64, i0, h, b);
-    {  // dS -> s5 (over Vc), dSu -> s6 (over dO)
+    __syncwarp();
+    mbar_wait(bar_mma, ph_mma, abortp);
+    ph_mma ^= 1;
+    tc_fence_after();
+    B128_MARK(0, n, 9);
+    {
       float v[32], w[32];
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
@@ -293,208 +318,216 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         v[j] = ds.x; v[j + 1] = ds.y;
         w[j] = -du.x; w[j + 1] = -du.y;
       }
-      store_row32<T>(s5, kPanelB, row, c0, v);
-      store_row32<T>(s6, kPanelB, row, c0, w);
+      store_row32<T>(s1, kPanelB, row, c0, v);   // dS
+      mbar_wait(bar_dv, ph, abortp);
+      store_row32<T>(s6, kPanelB, row, c0, w);   // dSu, over dO
     }
-    B128_SYNC();
-    B128_MARK(0, 11);
-    if (storer) { bulk_s2g(tile + kSlot, s6, kSlot); bulk_commit(); }   // dSu
-
-    // ---- M5: dkc += dS^T @ Qc[I];  dT = dSu @ A
-    if (tid == 0) {
+    B128_SYNC()
+    B128_MARK(0, n, 10);
+    // ---- dqc = dSu Wb + dS Kc;  dkc += dS^T Qc
+    if (warp == 0 && elect_one()) {
       tc_fence_after();
-      gemm_km_t<8>(tmem + C_S, a6, a1, ID_KM, false);
-      mma_commit(&bar_mma);  // dT alone: masking it overlaps the dkc product, which the next commit covers
-      gemm_mm_t<8>(tmem + C_DKC, a5, a3, ID_MM, !first);
+      if (!diag) gemm_km_t<8>(tmem + C_S, a6, a0, ID_KM, false);
+      mma_commit(bar_x0);
+      gemm_km_t<8>(tmem + C_S, a1, a4, ID_KM, !diag);
+      mma_commit(bar_x);
+      gemm_mm_t<8>(tmem + C_DKC, a1, a3, ID_MM, n > 0);
+      mma_commit(bar_k);
     }
-    B128_MMA_WAIT();
-    B128_MARK(0, 12);
-    {  // masked dT -> s1 (over the gate)
-      float v[32];
-      tmem_ld32_lower(trow + C_S + c0, row, c0, v);
-      store_row32<T>(s1, kPanelB, row, c0, v);
+    if (storer && elect_one()) { bulk_s2g(tile + kTileDsu, s6, kSq); bulk_commit(); }
+    if (loader && more && elect_one()) {
+      mbar_expect_tx(bar_z, 2 * kSq);
+      mbar_expect_tx(bar_qc, kSq);
+      mbar_expect_tx(bar_vu, kSq);
+      mbar_expect_tx(bar_do, 2 * kSq);
+      mbar_wait(bar_x0, ph, abortp);
+      load_op(s0, m_qu, bar_z, k0, h, b);
     }
-    if (storer) bulk_wait_read0();   // the copy of dSu has read its slot (the dqc staging goes there at the end of the step)
-    B128_SYNC();
-    B128_MARK(0, 13);
-
-    // ---- M6: dqc[I] (unscaled) = dT @ Vu[I] + dSu @ Wb + dS @ Kc[K]
-    // Three commits, in the order in which the products free the per-step slots, so that the next
-    // block's tiles are fetched as early as possible (a tile takes 2-4 thousand cycles to arrive): behind
-    // the first Ku, Vu and Qc (s1, s2; s3's last reader, the dkc product issued in the phase before, is
-    // covered too), behind the second Qu (s0).  One 16 KB panel per lane of eight warps.
-    if (tid == 0) {
-      mbar_wait(&bar_vu2, ph_vu2, abortp);
-      tc_fence_after();
-      if (I > K) mbar_expect_tx(&bar_a, 4 * kSlot);   // armed here, the eight loads are issued by other lanes
-      gemm_km_t<8>(tmem + C_S, a1, a2, ID_KM, false);
-      mma_commit(&bar_x1);
-      if (!diag) gemm_km_t<8>(tmem + C_S, a6, a0, ID_KM, true);
-      mma_commit(&bar_x2);
-      gemm_km_t<8>(tmem + C_S, a5, a4, ID_KM, true);
-      mma_commit(&bar_mma);
-    }
-    ph_vu2 ^= 1;
-    if (lane == 0 && warp < 8 && I > K) {
-      const int in0 = (I - 1) * kBlkB;
-      const int t = warp >> 1, pn = warp & 1;   // tile 0: Qu -> s0, 1: Ku -> s1, 2: Vu -> s2, 3: Qc -> s3
-      const CUtensorMap* m = t == 0 ? &m_qu : (t == 1 ? &m_ku : (t == 2 ? &m_vu : &m_qc));
-      mbar_wait(t == 0 ? &bar_x2 : &bar_x1, ph_x, abortp);
-      tma_load_4d(smem + t * kSlot + pn * kPanelB, m, &bar_a, pn * 64, t == 0 ? k0 : in0, h, b);
-    }
-    ph_x ^= 1;
-    B128_MMA_WAIT();
-    B128_MARK(0, 14);
-    {  // stage dqc[I] as four fp32 panels over s5|s6 and add it to the workspace by TMA reduce:
-       // chunk group cc stages panel cc and one of its lanes issues that panel's reduce
-      float v[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-      store_row32_f32(s5 + cc * kPanelB, row, v);
-      fence_async_smem();
-      group_sync(1 + cc);
-      if (issuer) {
-        tma_reduce_add_3d(&m_acc_dqc, s5 + cc * kPanelB, cc * 32, i0, bh);
-        bulk_commit();
-      }
-    }
+    __syncwarp();
+    mbar_wait(bar_x, ph, abortp);
+    tc_fence_after();
+    B128_MARK(0, n, 11);
+    float v[32];
+    tmem_ld32(trow + C_S + c0, v);
+    tmem_ld_wait();
+    if (storer && elect_one()) bulk_wait_read0();   // dSu has been read
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
-    B128_MARK(0, 15);
-  }
-  if (issuer || storer) bulk_wait0();
-
-  // ---- dkc (x scale) and dvc of the key block
-  {
-    tc_fence_after();
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const castle_tensor_t& dt = t == 0 ? p.dkc : p.dvc;
-      const float mul = t == 0 ? p.scale : 1.f;
-      T* dst = reinterpret_cast<T*>(dt.ptr) + b * dt.stride_b + h * dt.stride_h + (int64_t)krow * dt.stride_n + c0;
-      float v[32];
-      tmem_ld32(trow + (t == 0 ? C_DKC : C_DVC) + c0, v);
-      tmem_ld_wait();
-      if (krow < p.N) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint4 q;
-          q.x = Elem<T>::pack2(v[8 * j] * mul, v[8 * j + 1] * mul);
-          q.y = Elem<T>::pack2(v[8 * j + 2] * mul, v[8 * j + 3] * mul);
-          q.z = Elem<T>::pack2(v[8 * j + 4] * mul, v[8 * j + 5] * mul);
-          q.w = Elem<T>::pack2(v[8 * j + 6] * mul, v[8 * j + 7] * mul);
-          *reinterpret_cast<uint4*>(dst + j * 8) = q;
-        }
-      }
+    B128_MARK(0, n, 12);
+    // before the reduces, which loads would queue behind
+    if (loader && more && elect_one()) {
+      load_op(s2, m_vu, bar_vu, i0 - kBlkB, h, b);
+      mbar_wait(bar_k, ph, abortp);
+      load_op(s1, m_ku, bar_z, i0 - kBlkB, h, b);
+      load_op(s3, m_qc, bar_qc, i0 - kBlkB, h, b);
+    }
+    __syncwarp();
+    uint8_t* panel = s5 + cc * kPanelB;
+    store_row32_f32(panel, row, v);
+    fence_async_smem();
+    group_sync(1 + cc);
+    B128_MARK(0, n, 13);
+    if (reducer && elect_one()) {
+      mbar_wait(bar_k, ph, abortp);
+      tma_reduce_add_3d(&m_acc_dqc, panel, cc * 32, i0, bh);
+      bulk_commit();
     }
   }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 512);
-  if (tid == 0 && abort_flag) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
+  if ((reducer || storer) && elect_one()) bulk_wait0();
+  __syncwarp();
+  mbar_wait(bar_k, (uint32_t)(steps - 1) & 1u, abortp);
+  tc_fence_after();
+  {
+    float v[32], w[32];
+    tmem_ld32(trow + C_DKC + c0, v);
+    tmem_ld32(trow + C_DVC + c0, w);
+    tmem_ld_wait();
+    if (krow < p.N) {
+      store_grad32<T>(grad_row<T>(p.dkc, b, h, krow, c0), v, p.scale);
+      store_grad32<T>(grad_row<T>(p.dvc, b, h, krow, c0), w, 1.f);
+    }
+  }
+  B128_END(512)
 }
 
-// ------------------------------------------------------------------------------------------------
-// Lookahead-gradient kernel.  It recomputes nothing: the gate A, dSu and the masked T of every (I, K) step come
-// from the key/value kernel through global memory (three 32 KB tiles per step, copied as they lay in shared
-// memory).  TMEM: dqu | G | scratch | scratch: with the forward state gone from this kernel, dqu[K] accumulates
-// in tensor memory over the walk and is written once at the end (no reduce, and deterministic).
+// ------------------------------------------------------------------------------------------------ reverse state
+// Step m adds query block I = nblk-1-m to G and hands the copy to step (I-1, K).  Two buffers of everything.
+template <typename T>
+__global__ void __launch_bounds__(kB128Threads, 1)
+castle_bwd128_reverse_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc) {
+  constexpr uint32_t ID_MM = make_idesc(128, 128, Elem<T>::fmt, true, true, false);
+  const int K = blockIdx.y, steps = p.nblk - 1 - K;
+  B128_BEGIN(6 * kSq, 4, 128)
+  uint64_t *bar_in = bars, *bar_g = bars + 2;   // two each
+  const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;
+  const bool loader = warp == 4, storer = warp == 8;
+  auto load = [&](int m) {
+    uint8_t* dst = smem + (m & 1) * 2 * kSq;
+    const int I = p.nblk - 1 - m;
+    mbar_expect_tx(bar_in + (m & 1), 2 * kSq);
+    bulk_g2s(dst, step_tiles(p, I, K) + kTileDsu, kSq, bar_in + (m & 1));
+    load_op(dst + kSq, m_qc, bar_in + (m & 1), I * kBlkB, h, b);
+  };
+  auto product = [&](int m) {
+    const uint32_t a = smem_u32(smem + (m & 1) * 2 * kSq);
+    mbar_wait(bar_in + (m & 1), (uint32_t)(m >> 1) & 1u, abortp);
+    tc_fence_after();
+    gemm_mm_t<8>(tmem, a, a + kSq, ID_MM, m > 0);
+    mma_commit(bar_g + (m & 1));
+  };
+  if (loader && elect_one())
+    for (int m = 0; m < steps && m < 2; ++m) load(m);
+  if (warp == 0 && steps > 0 && elect_one()) product(0);
+  __syncwarp();
+  for (int m = 0; m < steps; ++m) {
+    uint8_t* gb = smem + (4 + (m & 1)) * kSq;
+    mbar_wait(bar_g + (m & 1), (uint32_t)(m >> 1) & 1u, abortp);
+    tc_fence_after();
+    float v[32];
+    tmem_ld32(trow + c0, v);
+    tmem_ld_wait();
+    if (storer && elect_one()) bulk_wait_read1();   // of the copy made two steps ago
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0 && m + 1 < steps && elect_one()) product(m + 1);
+    if (loader && m + 2 < steps && elect_one()) load(m + 2);
+    __syncwarp();
+    store_row32<T>(gb, kPanelB, row, c0, v);
+    fence_async_smem();
+    __syncthreads();
+    if (storer && elect_one()) {
+      bulk_s2g(step_tiles(p, p.nblk - 2 - m, K) + kTileG, gb, kSq);
+      bulk_commit();
+    }
+    __syncwarp();
+  }
+  if (storer && elect_one()) bulk_wait0();
+  __syncwarp();
+  B128_END(128)
+}
+
+// ------------------------------------------------------------------------------------------------ dku, dvu, dT, dqc
 template <typename T>
 __global__ void __launch_bounds__(kB128Threads, 1)
 castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_qu,
-                        const __grid_constant__ CUtensorMap m_ku, const __grid_constant__ CUtensorMap m_vu,
-                        const __grid_constant__ CUtensorMap m_acc_dvu, const __grid_constant__ CUtensorMap m_acc_dku) {
+                       const __grid_constant__ CUtensorMap m_vu) {
   constexpr int FMT = Elem<T>::fmt;
-  constexpr uint32_t ID_KK = make_idesc(128, 128, FMT, false, false, false);
-  constexpr uint32_t ID_KM = make_idesc(128, 128, FMT, false, true, false);
-  constexpr uint32_t ID_MM = make_idesc(128, 128, FMT, true, true, false);
-  constexpr uint32_t C_DQU = 0, C_G = 128, C_S = 256, C_X = 384;
-
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sG = smem;              // 16-bit copy of G (kept across steps)
-  uint8_t* sA = sG + kSlot;        // gate A (from the key/value kernel) -> Qu[K]
-  uint8_t* s0 = sA + kSlot;        // masked dT
-  uint8_t* s1 = s0 + kSlot;        // Vu[I] -> Ku[I] -> dvu / dku staging
-  uint8_t* s2 = s1 + kSlot;        // Qc[I] -> dvu / dku staging
-  uint8_t* s3 = s2 + kSlot;        // masked T (from the key/value kernel) -> dZ
-  uint8_t* s4 = s3 + kSlot;        // dSu (from the key/value kernel)
-  __shared__ uint64_t bar_a, bar_v, bar_ku2, bar_qu2, bar_mma;
-  __shared__ uint32_t tmem_base_s;
-  __shared__ int abort_flag;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, cc = warp >> 2;
-  const int row = quarter * 32 + lane, c0 = cc * 32;
-  const int bh = p.bh0 + blockIdx.x, K = blockIdx.y;
-  const int b = bh / p.H, h = bh % p.H;
-  const int k0 = K * kBlkB, krow = k0 + row;
-  // one lane per chunk group issues that group's reduces and, once they have read their staging panels,
-  // refills the panels it owns; not thread 0, which must not be held up on its way to the next products
-  const bool issuer = (quarter == 1 && lane == 0);   // threads 32, 160, 288, 416
-  const uint8_t* const tile_base = p.tiles + (int64_t)blockIdx.x * p.ntiles * 3 * kSlot;
-
-  if (tid == 0) {
-    mbar_init(&bar_a, 1); mbar_init(&bar_v, 1); mbar_init(&bar_ku2, 1); mbar_init(&bar_qu2, 1); mbar_init(&bar_mma, 1);
-    mbar_fence_init();
-    abort_flag = 0;
+  constexpr uint32_t C_DKU = 0, C_DVU = 128, C_DT = 256, C_DA = 384;
+  constexpr uint32_t ID_KK = make_idesc(128, 128, FMT, false, false, false), ID_KM = make_idesc(128, 128, FMT, false, true, false),
+                     ID_MM = make_idesc(128, 128, FMT, true, true, false);
+  const int I = p.nblk - 1 - blockIdx.y, i0 = I * kBlkB;   // the longest walks first
+  const bool last = I == p.nblk - 1;                       // no G there yet
+  B128_BEGIN(7 * kSq, 7, 512)
+  uint8_t *sVu = smem, *sT = smem + kSq, *sA = smem + 2 * kSq, *sS = smem + 3 * kSq, *sG = smem + 4 * kSq, *sQu = smem + 5 * kSq,
+          *sZ = smem + 6 * kSq;
+  uint64_t *bar_res = bars, *bar_in = bars + 1, *bar_qu = bars + 2, *bar_da = bars + 3, *bar_v = bars + 4, *bar_k = bars + 5, *bar_t = bars + 6;
+  const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;
+  const bool loader = warp == 4;
+  auto load_tiles = [&](int K) {
+    const uint8_t* t = step_tiles(p, I, K);
+    mbar_expect_tx(bar_in, last ? 2 * kSq : 3 * kSq);
+    if (!last) bulk_g2s(sG, t + kTileG, kSq, bar_in);
+    bulk_g2s(sS, t + kTileDsu, kSq, bar_in);
+    bulk_g2s(sA, t + kTileA, kSq, bar_in);
+  };
+  auto load_qu = [&](int K) {
+    mbar_expect_tx(bar_qu, kSq);
+    load_op(sQu, m_qu, bar_qu, K * kBlkB, h, b);
+  };
+  if (loader && elect_one()) {
+    mbar_expect_tx(bar_res, 2 * kSq);
+    load_op(sVu, m_vu, bar_res, i0, h, b);
+    load_op(sZ, m_qc, bar_res, i0, h, b);
+    load_tiles(0);
+    load_qu(0);
   }
-  if (warp == 0) { tmem_alloc(&tmem_base_s, 512); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  const uint32_t aVu = smem_u32(sVu), aT = smem_u32(sT), aA = smem_u32(sA), aS = smem_u32(sS), aG = smem_u32(sG), aQu = smem_u32(sQu),
+                 aZ = smem_u32(sZ);
+  // ---- the masked T = tril(Qc Vu^T)
+  if (warp == 0 && elect_one()) {
+    mbar_wait(bar_res, 0, abortp);
+    tc_fence_after();
+    gemm_kk_t<2>(tmem + C_DA, aZ, aVu, ID_KK, false);
+    mma_commit(bar_t);
+  }
+  __syncwarp();
+  mbar_wait(bar_t, 0, abortp);
   tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
-  const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-  volatile int* abortp = &abort_flag;
-
-  uint32_t ph_a = 0, ph_ku2 = 0, ph_qu2 = 0, ph_mma = 0;   // ph_a also serves bar_v
-  const uint32_t aG = smem_u32(sG), aA = smem_u32(sA), a0 = smem_u32(s0), a1 = smem_u32(s1), a2 = smem_u32(s2),
-                 a3 = smem_u32(s3), a4 = smem_u32(s4);
-
-  auto tile_of = [&](int I) { return tile_base + ((int64_t)I * (I + 1) / 2 + K) * 3 * kSlot; };
-  if (tid == 0) {  // the first block's tiles; later ones are fetched inside the step before (see the last phase)
-    const int il = (p.nblk - 1) * kBlkB;
-    const uint8_t* t = tile_of(p.nblk - 1);
-    mbar_expect_tx(&bar_a, 3 * kSlot);
-    bulk_g2s(sA, t, kSlot, &bar_a);
-    bulk_g2s(s4, t + kSlot, kSlot, &bar_a);
-    bulk_g2s(s3, t + 2 * kSlot, kSlot, &bar_a);
-    mbar_expect_tx(&bar_v, 2 * kSlot);
-    load_tile<2>(s1, &m_vu, &bar_v, il, h, b);
-    load_tile<2>(s2, &m_qc, &bar_v, il, h, b);
+  {
+    float v[32];
+    tmem_ld32_lower(trow + C_DA + c0, row, c0, v);
+    store_row32<T>(sT, kPanelB, row, c0, v);
   }
-  for (int I = p.nblk - 1; I >= K; --I) {
-    const int i0 = I * kBlkB;
-    const bool first = (I == p.nblk - 1);
-    // Vu[I] and Qc[I] go into the panels that held the dku staging of the step before: each issuing lane
-    // waits until its reduce has read its panel and refills exactly that panel (nobody else touches it),
-    // so no barrier is needed.  The three hand-over tiles were fetched during the step before.
-    if (issuer && I < p.nblk - 1) {
-      bulk_wait_read0();
-      tma_load_4d((cc < 2 ? s1 : s2) + (cc & 1) * kPanelB, cc < 2 ? &m_vu : &m_qc, &bar_v, (cc & 1) * 64, i0, h, b);
-    }
-
-    // ---- dA/scale = Gb @ Vu[I]^T + dSu^T @ Tm;  dT = dSu @ A;  G += dSu^T @ Qc[I]
-    if (tid == 0) {
-      mbar_wait(&bar_a, ph_a, abortp);
-      mbar_wait(&bar_v, ph_a, abortp);
+  B128_SYNC()
+  for (int K = 0; K <= I; ++K) {
+    const uint32_t ph = K & 1;
+    // ---- dA/scale = Gb Vu^T + dSu^T T;  dT += dSu A;  dvu += A^T Gb
+    if (warp == 0 && elect_one()) {
+      B128_MARK(512, K, 0);
+      mbar_wait(bar_in, ph, abortp);
       tc_fence_after();
-      mbar_expect_tx(&bar_ku2, kSlot);   // armed here; the loads are issued below by two other lanes
-      if (!first) gemm_kk_t<2>(tmem + C_S, aG, a1, ID_KK, false);
-      gemm_mm_t<8>(tmem + C_S, a4, a3, ID_MM, !first);
-      gemm_km_t<8>(tmem + C_X, a4, aA, ID_KM, false);
-      mma_commit(&bar_mma);  // dA and dT: the pass below overlaps the G update, which the next commit covers
-      gemm_mm_t<8>(tmem + C_G, a4, a2, ID_MM, !first);
+      B128_MARK(512, K, 1);
+      if (!last) gemm_kk_t<2>(tmem + C_DA, aG, aVu, ID_KK, false);
+      gemm_mm_t<8>(tmem + C_DA, aS, aT, ID_MM, !last);
+      mma_commit(bar_da);
+      gemm_km_t<8>(tmem + C_DT, aS, aA, ID_KM, K > 0);
+      if (!last) gemm_mm_t<8>(tmem + C_DVU, aA, aG, ID_MM, K > 0);
+      mma_commit(bar_v);
     }
-    ph_a ^= 1;
-    B128_MARK(256, 0);
-    B128_MMA_WAIT();
-    B128_MARK(256, 1);
-    // Vu[I] is consumed (dSu is not yet: the G update still reads it): Ku[I] -> s1 for the dqu product
-    if (lane == 0 && (warp == 5 || warp == 9)) tma_load_4d(s1 + (warp == 9) * kPanelB, &m_ku, &bar_ku2, (warp == 9) * 64, i0, h, b);
-    {  // dZ = dA A (1 - A) -> s3 (over the masked T); masked dT -> s0
+    __syncwarp();
+    if (loader && elect_one()) bulk_wait_read0();   // dZ of the step before has been copied
+    __syncwarp();
+    B128_MARK(512, K, 2);
+    mbar_wait(bar_da, ph, abortp);   // (its last reader, the dku product, came before these)
+    __syncthreads();
+    tc_fence_after();
+    B128_MARK(512, K, 3);
+    {
       float v[32], a[32];
-      tmem_ld32(trow + C_S + c0, v);
+      tmem_ld32(trow + C_DA + c0, v);
       load_row32<T>(sA, kPanelB, row, c0, a);
       tmem_ld_wait();
 #pragma unroll
@@ -503,122 +536,130 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         const float2 x = mul2(mul2(make_float2(v[j], v[j + 1]), splat(p.scale)), fma2(mul2(g, splat(-1.f)), g, g));   // a (1 - a) = a - a a
         v[j] = x.x; v[j + 1] = x.y;
       }
-      store_row32<T>(s3, kPanelB, row, c0, v);
-      tmem_ld32_lower(trow + C_X + c0, row, c0, v);
-      store_row32<T>(s0, kPanelB, row, c0, v);
+      store_row32<T>(sZ, kPanelB, row, c0, v);
     }
-    B128_SYNC();
-    B128_MARK(256, 2);
-
-    // ---- dvu[I] (unscaled) = A^T @ Gb + dT^T @ Qc[I];  dqu[K] += dZ @ Ku[I]
-    if (tid == 0) {
+    B128_SYNC()
+    B128_MARK(512, K, 4);
+    // ---- dku += dZ^T Qu
+    if (warp == 0 && elect_one()) {
+      mbar_wait(bar_qu, ph, abortp);
+      B128_MARK(512, K, 5);
       tc_fence_after();
-      mbar_expect_tx(&bar_qu2, kSlot);   // armed here; the loads are issued below by two other lanes
-      if (!first) gemm_mm_t<8>(tmem + C_X, aA, aG, ID_MM, false);
-      gemm_mm_t<8>(tmem + C_X, a0, a2, ID_MM, !first);
-      mbar_wait(&bar_ku2, ph_ku2, abortp);
-      gemm_km_t<8>(tmem + C_DQU, a3, a1, ID_KM, !first);
-      mma_commit(&bar_mma);
+      gemm_mm_t<8>(tmem + C_DKU, aZ, aQu, ID_MM, K > 0);
+      mma_commit(bar_k);
     }
-    ph_ku2 ^= 1;
-    B128_MMA_WAIT();
-    B128_MARK(256, 3);
-    // the gate is consumed: Qu[K] -> sA for the dku product
-    if (lane == 0 && (warp == 5 || warp == 9)) tma_load_4d(sA + (warp == 9) * kPanelB, &m_qu, &bar_qu2, (warp == 9) * 64, k0, h, b);
-    {  // stage dvu[I] over s1|s2 (four fp32 panels, one per chunk group)
-      float v[32];
-      tmem_ld32(trow + C_X + c0, v);
-      tmem_ld_wait();
-      store_row32_f32((cc < 2 ? s1 : s2) + (cc & 1) * kPanelB, row, v);
-    }
-    fence_async_smem();
-    group_sync(1 + cc);
-    if (issuer) {  // chunk group cc staged panel cc; its lane issues that panel's reduce
-      tma_reduce_add_3d(&m_acc_dvu, (cc < 2 ? s1 : s2) + (cc & 1) * kPanelB, cc * 32, i0, bh);
+    if (loader && elect_one()) {   // the copy last: loads would queue behind it
+      if (K < I) {
+        mbar_wait(bar_v, ph, abortp);
+        load_tiles(K + 1);
+      }
+      bulk_s2g(step_tiles(p, I, K) + kTileA, sZ, kSq);
       bulk_commit();
-    }
-    tc_fence_before();
-    __syncthreads();
-    B128_MARK(256, 4);
-
-    // ---- dku[I] (unscaled) = dZ^T @ Qu[K]
-    if (tid == 0) {
-      mbar_wait(&bar_qu2, ph_qu2, abortp);
-      tc_fence_after();
-      gemm_mm_t<8>(tmem + C_X, a3, aA, ID_MM, false);
-      mma_commit(&bar_mma);
-      if (I > K) {  // the next step's tiles: three fetched below, two at the top of the next step
-        mbar_expect_tx(&bar_a, 3 * kSlot);
-        mbar_expect_tx(&bar_v, 2 * kSlot);
+      if (K < I) {
+        mbar_wait(bar_k, ph, abortp);
+        load_qu(K + 1);
       }
     }
-    ph_qu2 ^= 1;
-    if (issuer) bulk_wait_read0();  // this lane's dvu panel has been read: its slot is free again
-    B128_MMA_WAIT();
-    __syncthreads();  // orders the issuing lanes' waits before everybody's staging stores
-    B128_MARK(256, 5);
-    // The dvu reduce has drained and the last product is done, so the slots of the
-    // next step's hand-over tiles are all free: A -> sA, dSu -> s4, masked T -> s3, one 16 KB half per lane
-    // of six warps; they arrive while dku is staged.
-    if (lane == 0 && warp < 6 && I > K) {
-      const int t = warp >> 1, pn = warp & 1;
-      uint8_t* dst = (t == 0 ? sA : t == 1 ? s4 : s3) + pn * kPanelB;
-      bulk_g2s(dst, tile_of(I - 1) + t * kSlot + pn * kPanelB, kPanelB, &bar_a);
-    }
-    {
-      float v[32];
-      tmem_ld32(trow + C_X + c0, v);
-      tmem_ld_wait();
-      store_row32_f32((cc < 2 ? s1 : s2) + (cc & 1) * kPanelB, row, v);
-      // 16-bit copy of G including block I, for the next (lower) block
-      tmem_ld32(trow + C_G + c0, v);
-      tmem_ld_wait();
-      store_row32<T>(sG, kPanelB, row, c0, v);
-    }
-    fence_async_smem();
-    group_sync(1 + cc);
-    if (issuer) {
-      tma_reduce_add_3d(&m_acc_dku, (cc < 2 ? s1 : s2) + (cc & 1) * kPanelB, cc * 32, i0, bh);
-      bulk_commit();
-    }
-    tc_fence_before();
-    __syncthreads();
-    B128_MARK(256, 6);
+    __syncwarp();
   }
-  if (issuer) bulk_wait0();
-
-  // ---- dqu (x scale) of the key block
-  {
-    tc_fence_after();
-    T* dst = reinterpret_cast<T*>(p.dqu.ptr) + b * p.dqu.stride_b + h * p.dqu.stride_h + (int64_t)krow * p.dqu.stride_n + c0;
-    float v[32];
-    tmem_ld32(trow + C_DQU + c0, v);
-    tmem_ld_wait();
-    if (krow < p.N) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        uint4 q;
-        q.x = Elem<T>::pack2(v[8 * j] * p.scale, v[8 * j + 1] * p.scale);
-        q.y = Elem<T>::pack2(v[8 * j + 2] * p.scale, v[8 * j + 3] * p.scale);
-        q.z = Elem<T>::pack2(v[8 * j + 4] * p.scale, v[8 * j + 5] * p.scale);
-        q.w = Elem<T>::pack2(v[8 * j + 6] * p.scale, v[8 * j + 7] * p.scale);
-        *reinterpret_cast<uint4*>(dst + j * 8) = q;
-      }
-    }
-  }
-  tc_fence_before();
+  // ---- the masked dT (over dZ):  dvu += dT^T Qc;  dqc += dT Vu
+  if (loader && elect_one()) bulk_wait_read0();
+  mbar_wait(bar_k, (uint32_t)I & 1u, abortp);
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 512);
-  if (tid == 0 && abort_flag) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
+  tc_fence_after();
+  if (loader && elect_one()) {
+    mbar_expect_tx(bar_res, kSq);
+    load_op(sQu, m_qc, bar_res, i0, h, b);
+  }
+  __syncwarp();
+  {
+    float v[32];
+    tmem_ld32_lower(trow + C_DT + c0, row, c0, v);
+    store_row32<T>(sZ, kPanelB, row, c0, v);
+  }
+  B128_SYNC()
+  if (warp == 0 && elect_one()) {
+    mbar_wait(bar_res, 1, abortp);
+    tc_fence_after();
+    gemm_mm_t<8>(tmem + C_DVU, aZ, aQu, ID_MM, !last);
+    gemm_km_t<8>(tmem + C_DA, aZ, aVu, ID_KM, false);
+    mma_commit(bar_da);
+  }
+  __syncwarp();
+  const int irow = i0 + row;
+  float v[32];
+  tmem_ld32(trow + C_DKU + c0, v);
+  tmem_ld_wait();
+  if (irow < p.N) store_grad32<T>(grad_row<T>(p.dku, b, h, irow, c0), v, p.scale);
+  mbar_wait(bar_da, (uint32_t)(I + 1) & 1u, abortp);
+  tc_fence_after();
+  tmem_ld32(trow + C_DVU + c0, v);
+  tmem_ld_wait();
+  if (irow < p.N) store_grad32<T>(grad_row<T>(p.dvu, b, h, irow, c0), v, p.scale);
+  tmem_ld32(trow + C_DA + c0, v);
+  tmem_ld_wait();
+  if (irow < p.N) {
+    const float4* acc = reinterpret_cast<const float4*>(p.acc_dqc + ((int64_t)bh * p.N + irow) * 128 + c0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float4 q = acc[j];
+      v[4 * j] += q.x; v[4 * j + 1] += q.y; v[4 * j + 2] += q.z; v[4 * j + 3] += q.w;
+    }
+    store_grad32<T>(grad_row<T>(p.dqc, b, h, irow, c0), v, p.scale);
+  }
+  if (loader && elect_one()) bulk_wait0();
+  __syncwarp();
+  B128_END(512)
 }
 
-#undef B128_MMA_WAIT
-#undef B128_SYNC
+// ------------------------------------------------------------------------------------------------ dqu
+// A stream of dZ and Ku tiles through three stages into one accumulator.
+template <typename T>
+__global__ void __launch_bounds__(128)
+castle_bwd128_dqu_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_ku) {
+  constexpr uint32_t ID_KM = make_idesc(128, 128, Elem<T>::fmt, false, true, false);
+  const int K = blockIdx.y, k0 = K * kBlkB, steps = p.nblk - K;
+  B128_BEGIN(6 * kSq, 7, 128)
+  uint64_t *bar_in = bars, *bar_done = bars + 3, *bar_end = bars + 6;   // three, three, one
+  if (warp == 0 && elect_one()) {
+    auto load = [&](int n) {
+      const int s = n % 3;
+      mbar_expect_tx(bar_in + s, 2 * kSq);
+      bulk_g2s(smem + s * 2 * kSq, step_tiles(p, K + n, K) + kTileA, kSq, bar_in + s);
+      load_op(smem + (s * 2 + 1) * kSq, m_ku, bar_in + s, k0 + n * kBlkB, h, b);
+    };
+    for (int n = 0; n < steps && n < 3; ++n) load(n);
+    for (int n = 0; n < steps; ++n) {
+      const int s = n % 3;
+      mbar_wait(bar_in + s, (uint32_t)(n / 3) & 1u, abortp);
+      tc_fence_after();
+      gemm_km_t<8>(tmem, smem_u32(smem + s * 2 * kSq), smem_u32(smem + (s * 2 + 1) * kSq), ID_KM, n > 0);
+      mma_commit(bar_done + s);
+      if (n > 0 && n + 2 < steps) {   // the stage of the step before: its product is done or about to be
+        mbar_wait(bar_done + (n - 1) % 3, (uint32_t)((n - 1) / 3) & 1u, abortp);
+        load(n + 2);
+      }
+    }
+    mma_commit(bar_end);
+  }
+  __syncwarp();
+  mbar_wait(bar_end, 0, abortp);
+  tc_fence_after();
+  const int krow = k0 + tid;
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    float v[32];
+    tmem_ld32(trow + c * 32, v);
+    tmem_ld_wait();
+    if (krow < p.N) store_grad32<T>(grad_row<T>(p.dqu, b, h, krow, c * 32), v, p.scale);
+  }
+  (void)lane;
+  B128_END(128)
+}
 
-// Scratch of the tile hand-over: three 32 KB tiles per (query block, key block) step and (batch, head) pair.
-// The pairs run in chunks so that it stays below 8 GiB per launch pair.
+// ------------------------------------------------------------------------------------------------ launches
 constexpr int64_t kTileScratchLimit = (int64_t)8 << 30;
-size_t bwd128_pair_bytes(int nblk) { return (size_t)nblk * (nblk + 1) / 2 * 3 * kSlot; }
+size_t bwd128_pair_bytes(int nblk) { return (size_t)nblk * (nblk + 1) / 2 * kStepTiles; }
 int bwd128_chunk_pairs(int BH, int nblk) {
   int64_t n = kTileScratchLimit / (int64_t)bwd128_pair_bytes(nblk);
   if (n < 1) n = 1;
@@ -628,35 +669,37 @@ int bwd128_chunk_pairs(int BH, int nblk) {
 template <typename T>
 static int launch_bwd128_t(const BwdParams& p, const CUtensorMap* in, cudaStream_t st) {
   constexpr int D = 128;
-  cudaError_t e = cudaFuncSetAttribute(castle_bwd128_kv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kB128Smem);
-  if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
-  e = cudaFuncSetAttribute(castle_bwd128_la_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kB128Smem);
-  if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
-  CUtensorMap acc[3];
-  float* bases[3] = {p.acc_dqc, p.acc_dvu, p.acc_dku};
-  for (int i = 0; i < 3; ++i) {
-    int rc = make_tmap_f32_rows(&acc[i], bases[i], p.B * p.H, p.N, D, "gradient workspace");
-    if (rc) return rc;
+  const void* kernels[4] = {(const void*)castle_bwd128_kv_kernel<T>,
+                            (const void*)castle_bwd128_reverse_kernel<T>, (const void*)castle_bwd128_la_kernel<T>, (const void*)castle_bwd128_dqu_kernel<T>};
+  const size_t smem[4] = {kB128Smem, 6 * kSq + 256, kB128Smem, 6 * kSq + 256};
+  for (int i = 0; i < 4; ++i) {
+    cudaError_t e = cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[i]);
+    if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
   }
+  CUtensorMap acc;
+  int rc = make_tmap_f32_rows(&acc, p.acc_dqc, p.B * p.H, p.N, D, "gradient workspace");
+  if (rc) return rc;
   const int64_t rows = (int64_t)p.B * p.H * p.N;
   constexpr int RPB = 256 / (D / 8);
-  e = cudaMemsetAsync(p.acc_dqc, 0, (size_t)rows * D * 3 * sizeof(float), st);
-  if (e != cudaSuccess) return cuda_fail(e, "castle_bwd memset");
-  castle_bwd_delta_kernel<T, D><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
+  castle_bwd_delta_kernel<T, D, 1><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
   const int BH = p.B * p.H, chunk = p.chunk_pairs;
   ev_start(CASTLE_KERNEL_BWD, st);
   for (int bh0 = 0; bh0 < BH; bh0 += chunk) {
     BwdParams q = p;
     q.bh0 = bh0;
     q.ntiles = (int64_t)p.nblk * (p.nblk + 1) / 2;
-    dim3 grid(BH - bh0 < chunk ? BH - bh0 : chunk, p.nblk);
+    const int pairs = BH - bh0 < chunk ? BH - bh0 : chunk;
+    const dim3 grid(pairs, p.nblk);
     // in[]: qc, kc, vc, qu, ku, vu, dout
-    castle_bwd128_kv_kernel<T><<<grid, kB128Threads, kB128Smem, st>>>(q, in[0], in[1], in[2], in[3], in[4], in[5], in[6], acc[0]);
-    castle_bwd128_la_kernel<T><<<grid, kB128Threads, kB128Smem, st>>>(q, in[0], in[3], in[4], in[5], acc[1], acc[2]);
+    // each starts while the one before it ends
+    cudaError_t e = launch_kernel(castle_bwd128_kv_kernel<T>, grid, kB128Threads, smem[0], st, true, q, in[0], in[1], in[2], in[3], in[4], in[5], in[6], acc);
+    if (e == cudaSuccess && p.nblk > 1) e = launch_kernel(castle_bwd128_reverse_kernel<T>, dim3(pairs, p.nblk - 1), kB128Threads, smem[1], st, true, q, in[0]);
+    if (e == cudaSuccess) e = launch_kernel(castle_bwd128_la_kernel<T>, grid, kB128Threads, smem[2], st, true, q, in[0], in[3], in[5]);
+    if (e == cudaSuccess) e = launch_kernel(castle_bwd128_dqu_kernel<T>, grid, 128, smem[3], st, true, q, in[4]);
+    if (e != cudaSuccess) return cuda_fail(e, "castle_bwd launch");
   }
   ev_stop(CASTLE_KERNEL_BWD, st);
-  castle_bwd_finish_kernel<T, D, 3><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_bwd launch");
 }
 

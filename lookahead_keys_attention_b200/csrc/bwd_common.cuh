@@ -16,10 +16,9 @@ struct BwdParams {
   const float* w_state;  // [BH][N][D]
   float* delta;          // [BH][N]
   float* acc_dqc;        // [BH][N][D] fp32, zeroed
-  float* acc_dvu;
+  float* acc_dvu;        // these two at dim_head 64
   float* acc_dku;
-  uint8_t* tiles;        // dim_head 128: per (pair, query block, key block) the 32 KB tiles A | dSu | Tm that the
-                         // key/value kernel hands to the lookahead kernel
+  uint8_t* tiles;        // dim_head 128: the tiles that its kernels hand on, per (pair, query block, key block)
   int64_t ntiles;        // query-block x key-block pairs per (batch, head) pair
   int bh0;               // dim_head 128: first (batch, head) pair of this launch (the pairs run in chunks)
   int chunk_pairs;       // dim_head 128: pairs per chunk (what the caller's scratch holds)
@@ -31,8 +30,9 @@ struct BwdParams {
 #endif
 };
 
-// delta[b,h,i] = sum_d out * dout  (lookahead_keys_attention_triton.py:175-214 in the reference)
-template <typename T, int D>
+// delta[b,h,i] = sum_d out * dout  (lookahead_keys_attention_triton.py:175-214 in the reference); clears the first NACC of the
+// fp32 accumulators on the way (a memset of its own is a launch more).
+template <typename T, int D, int NACC>
 __global__ void castle_bwd_delta_kernel(const BwdParams p) {
   constexpr int LPR = D / 8;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x / LPR) + threadIdx.x / LPR;
@@ -54,6 +54,14 @@ __global__ void castle_bwd_delta_kernel(const BwdParams p) {
 #pragma unroll
   for (int o = LPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (row < total && sub == 0) p.delta[row] = s;
+  if (row < total) {
+    float* const accs[3] = {p.acc_dqc, p.acc_dvu, p.acc_dku};
+#pragma unroll
+    for (int t = 0; t < NACC; ++t) {
+      float4* a = reinterpret_cast<float4*>(accs[t] + row * D + sub * 8);
+      a[0] = a[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
 }
 
 // fp32 accumulators -> scaled 16-bit gradients in the caller's (strided) tensors.
