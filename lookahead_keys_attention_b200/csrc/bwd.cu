@@ -88,7 +88,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   uint8_t* sGb = sWb + OPB;
   uint8_t* sA = sGb + OPB;             // slot 1: gate A
   uint8_t* sT = sA + SQB;              // slot 2: masked T, later dZ
-  __shared__ uint64_t bar_res, bar_load, bar_vd, bar_ku, bar_mma, bar_x1, bar_x2, bar_kn;
+  __shared__ uint64_t bar_res, bar_load, bar_vd, bar_ku, bar_mma, bar_x1, bar_x2, bar_kn, bar_w, bar_dv;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
@@ -103,6 +103,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   if (tid == 0) {
     mbar_init(&bar_res, 1); mbar_init(&bar_load, 1); mbar_init(&bar_vd, 1); mbar_init(&bar_ku, 1); mbar_init(&bar_mma, 1);
     mbar_init(&bar_x1, 1); mbar_init(&bar_x2, 1); mbar_init(&bar_kn, 1);
+    mbar_init(&bar_w, 1); mbar_init(&bar_dv, 1);
     mbar_fence_init();
     abort_flag = 0;
   }
@@ -205,14 +206,15 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     SMEM_TO_MMA_SYNC();
     BPHASE_MARK(3);
 
-    // ---- M2: peel W_K -= A @ Vu[I];  T = Qc[I] @ Vu[I]^T
+    // ---- M2: T = Qc[I] @ Vu[I]^T;  peel W_K -= A @ Vu[I], a commit each: T is masked while the state is peeled
     if (tid == 0) {
       mbar_wait(&bar_load, ph_load, abortp);   // Qc[I], Vu[I]
       BPHASE_MARK(21);
       tc_fence_after();
-      gemm_km_t<8>(tmem + C_W, aA, aVu, ID_D_KM_NEG, true);
       gemm_kk_t<1>(tmem + C_S, aQc, aVu, ID_SQ_KK, false);
       mma_commit(&bar_mma);
+      gemm_km_t<8>(tmem + C_W, aA, aVu, ID_D_KM_NEG, true);
+      mma_commit(&bar_w);
     }
     // The reduces of the step before must have finished reading their staging tiles before these are
     // written again.  A reduce takes a few thousand cycles to drain, so each issuing lane waits for its
@@ -228,6 +230,8 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       tmem_ld32_lower(trow + C_S + c0, row, c0, v);
       store_row32<T>(sT, kPanelB, row, c0, v);
     }
+    mbar_wait(&bar_w, ph_x, abortp);
+    tc_fence_after();
     if (c0 < D) {  // 16-bit copy of the peeled state
       float v[32];
       tmem_ld32(trow + C_W + c0, v);
@@ -253,9 +257,18 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     uint32_t dpk[16];  // silu'(Su), later dSu, two 16-bit values per register
     uint32_t ppk[16];  // P
     {
-      float v[32];
+      float v[32], w[32];
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
+      tc_fence_before();
+      __syncthreads();
+      BPHASE_MARK(7);
+      // ---- M4: Sc/scale = Qc[I] @ Kc[K]^T, while silu' is formed
+      if (tid == 0) {
+        tc_fence_after();
+        gemm_kk_t<1>(tmem + C_S, aQc, aKc, ID_SQ_KK, false);
+        mma_commit(&bar_mma);
+      }
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
         const float2 u = make_float2(v[j], v[j + 1]);
@@ -266,28 +279,14 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         const float2 d = fma2(mul2(q, splat(-p.scale)), fma2(g, splat(-1.f), splat(1.f)), g);
         dpk[j / 2] = Elem<T>::pack2(d.x, d.y);
       }
-      tmem_st32(trow + C_S + c0, v);
-      tmem_st_wait();
-    }
-    tc_fence_before();
-    __syncthreads();
-    BPHASE_MARK(7);
-
-    // ---- M4: S/scale = penalty + Qc[I] @ Kc[K]^T
-    if (tid == 0) {
-      tc_fence_after();
-      gemm_kk_t<1>(tmem + C_S, aQc, aKc, ID_SQ_KK, true);
-      mma_commit(&bar_mma);
-    }
-    MMA_WAIT();
-    BPHASE_MARK(8);
-    {  // P = exp(S - lse) (rows i, columns k); into slot 4 over Ku
-      float v[32];
-      tmem_ld32(trow + C_S + c0, v);
+      MMA_WAIT();
+      BPHASE_MARK(8);
+      // P = exp(S - lse) (rows i, columns k); into slot 4 over Ku
+      tmem_ld32(trow + C_S + c0, w);
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
-        const float2 x = fma2(make_float2(v[j], v[j + 1]), splat(sl2), splat(-lse_b));
+        const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(sl2), splat(-lse_b));
         v[j] = ex2_approx(x.x); v[j + 1] = ex2_approx(x.y);
       }
       if (diag) {
@@ -305,13 +304,14 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     SMEM_TO_MMA_SYNC();
     BPHASE_MARK(9);
 
-    // ---- M5: dvc += P^T @ dO[I];  dP = dO[I] @ Vc[K]^T
+    // ---- M5: dP = dO[I] @ Vc[K]^T;  dvc += P^T @ dO[I], which runs while dS is formed
     if (tid == 0) {
       tc_fence_after();
       mbar_wait(&bar_vd, ph_vd, abortp);
-      gemm_mm_t<8>(tmem + C_DVC, aKP, adO, ID_D_MM, !first);
       gemm_kk_t<1>(tmem + C_S, adO, aVc, ID_SQ_KK, false);
       mma_commit(&bar_mma);
+      gemm_mm_t<8>(tmem + C_DVC, aKP, adO, ID_D_MM, !first);
+      mma_commit(&bar_dv);
     }
     MMA_WAIT();
     BPHASE_MARK(10);
@@ -327,6 +327,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         v[j] = ds.x; v[j + 1] = ds.y;
         w[j] = -du.x; w[j + 1] = -du.y;
       }
+      mbar_wait(&bar_dv, ph_x, abortp);   // dO and P have been read
       store_row32<T>(sVD, kPanelB, row, c0, v);
       store_row32<T>(sKP, kPanelB, row, c0, w);
     }
