@@ -108,6 +108,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     abort_flag = 0;
   }
   if (warp == 0) { tmem_alloc(&tmem_base_s, 512); tmem_relinquish(); }
+  overlap_wait();   // launched while delta is being written
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -518,11 +519,11 @@ static int launch_bwd(const BwdParams& p, const CUtensorMap* maps, cudaStream_t 
   castle_bwd_delta_kernel<T, D, 3><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
   dim3 grid(p.B * p.H, p.nblk);
   ev_start(CASTLE_KERNEL_BWD, st);
-  castle_bwd_kernel<T, D><<<grid, kBwdThreads, smem, st>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6],
-                                                         maps[7], maps[8], maps[9]);
+  cudaError_t e = launch_kernel(castle_bwd_kernel<T, D>, grid, kBwdThreads, smem, st, true, p, maps[0], maps[1], maps[2], maps[3], maps[4],
+                                maps[5], maps[6], maps[7], maps[8], maps[9]);
   ev_stop(CASTLE_KERNEL_BWD, st);
-  castle_bwd_finish_kernel<T, D, 3><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
-  const cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = launch_kernel(castle_bwd_finish_kernel<T, D, 3>, dim3((unsigned)((rows + RPB - 1) / RPB)), 256, 0, st, true, p);
+  if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_bwd launch");
 }
 

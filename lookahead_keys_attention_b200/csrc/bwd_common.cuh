@@ -71,6 +71,7 @@ __global__ void castle_bwd_finish_kernel(const BwdParams p) {
   constexpr int LPR = D / 8;
   const int64_t row = (int64_t)blockIdx.x * (blockDim.x / LPR) + threadIdx.x / LPR;
   const int sub = threadIdx.x % LPR;
+  overlap_wait();   // launched while the sums are being written
   if (row >= (int64_t)p.B * p.H * p.N) return;
   int bh = row / p.N, i = row % p.N, b = bh / p.H, h = bh % p.H;
   const float* srcs[3] = {p.acc_dqc, p.acc_dvu, p.acc_dku};

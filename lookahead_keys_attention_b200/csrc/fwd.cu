@@ -188,6 +188,7 @@ castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_
     tma_prefetch_desc(&m_qc); tma_prefetch_desc(&m_ku); tma_prefetch_desc(&m_vu);
   }
   if (warp == 0) { tmem_alloc(tmem_base_s, 512); tmem_relinquish(); }
+  overlap_wait();   // launched while the T tiles are being written
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -908,6 +909,7 @@ template <typename T, int D>
 __global__ void __launch_bounds__(32 * D / 8) castle_fwd_merge_kernel(const FwdParams p) {
   const int bh = blockIdx.y, I = blockIdx.x / (kBlk / 32), r = (blockIdx.x % (kBlk / 32)) * 32 + (threadIdx.x & 31), c8 = threadIdx.x >> 5;
   const int i = I * kBlk + r;
+  overlap_wait();   // launched while the partials are being written
   if (i >= p.N) return;
   const int64_t tile0 = (int64_t)bh * tri(p.nblk) + tri(I);
   const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + tile0 * kBlk + r;
@@ -969,9 +971,9 @@ static int launch_fwd_pipe(const FwdParams& p, const CUtensorMap* maps, cudaStre
   auto kernel = p.tm ? castle_fwd_pipe_kernel<T, D, true> : castle_fwd_pipe_kernel<T, D, false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FwdPipe<D>::kSmem);   // per device, so on every call (cheap)
   if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
-  kernel<<<dim3(p.B * p.H, p.nblk, nseg), kFwdThreads, FwdPipe<D>::kSmem, st>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
-                                                                               maps[6], maps[7], maps[8]);
-  return 0;
+  e = launch_kernel(kernel, dim3(p.B * p.H, p.nblk, nseg), kFwdThreads, FwdPipe<D>::kSmem, st, p.tm != nullptr, p, maps[0], maps[1], maps[2],
+                    maps[3], maps[4], maps[5], maps[6], maps[7], maps[8]);
+  return e == cudaSuccess ? 0 : cuda_fail(e, "castle_fwd launch");
 }
 
 template <typename T, int D>
@@ -993,8 +995,8 @@ static int launch_fwd(FwdParams p, const CUtensorMap* maps, cudaStream_t st) {
   else rc = launch_fwd_pipe<T, D>(p, maps, st);
   if (rc) return rc;
   ev_stop(CASTLE_KERNEL_FWD, st);
-  castle_fwd_merge_kernel<T, D><<<dim3(p.nblk * (kBlk / 32), p.B * p.H), 32 * D / 8, 0, st>>>(p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_kernel(castle_fwd_merge_kernel<T, D>, dim3(p.nblk * (kBlk / 32), p.B * p.H), 32 * D / 8, 0, st, true, p);
+  if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_fwd launch");
 }
 
