@@ -360,7 +360,7 @@ def run_ours(args):
                 "h2d_bytes_per_step": 2 * x_host.numel() * 2 * world,
                 "d2h_bytes_per_step": 2 * out_host.numel() * 2 * world,
                 "exchange": None if group is None else "positions <-> heads all-to-all inside each batch row's group, twice per pass"},
-        "gpu_launches": 5 * args.steps,
+        "gpu_launches": 6 * args.steps,
         "kernels": {"fwd_main_ms": round(fwd_ms, 4), "fwd_main_tflops": round(fwd_tflops, 2),
                     "bwd_main_ms": round(bwd_ms, 4), "bwd_main_tflops": round(bwd_tflops, 2)},
         "roofline": {"kernel": "castle_bwd_kernel", "bound": "tensor", "achieved": round(bwd_tflops, 2),
