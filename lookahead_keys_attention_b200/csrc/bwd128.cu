@@ -10,10 +10,10 @@
 // Every gradient but dqc is owned by a CTA that keeps it in tensor memory.  A TMA reduce moves some 18 bytes per cycle and SM,
 // so a lookahead kernel that owned a key block and reduced dku[I] and dvu[I] (128 KB a step, with dT masked and multiplied in
 // every step) took 18.5 k cycles a step, 12.1 k without the reduces; reverse + la + dqu take 3.1 + 8.0 + 1.9 k, and kv, which
-// no longer forms dT, went from 20.8 to 18.9 k.  Measured on B=1 H=8 N=8190 bf16: 2365 -> 1882 us for the kernels, B=2 H=8 N=1333:
-// 249 -> 205 us.  What bounds them: kv its chain of six products with a pass behind each; la and reverse the tiles, which
+// no longer forms dT, went from 20.8 to 16.2 k.  Measured on B=1 H=8 N=8190 bf16: 2365 -> 1774 us for the kernels, B=2 H=8 N=1333:
+// 249 -> 195 us.  What bounds them: kv its chain of six products with a pass behind each; la and reverse the tiles, which
 // come at 20 to 30 bytes per cycle and SM with one step's worth of shared memory to prefetch into; dqu HBM.  (Handing W on
-// as well, from a kernel of its own, so that kv starts at Su: 4.4 + 17 k cycles instead of 18.9 k.)
+// as well, from a kernel of its own, so that kv starts at Su: 4.4 + 17 k cycles.)
 //
 // Tiles of a step (I,K): A, then dZ | dSu | Gb; 32 KB each, as they lie in shared memory (128-byte swizzle).  The scratch is
 // bounded (kTileScratchLimit): the (batch, head) pairs run in chunks, one launch of each kernel per chunk.
@@ -97,10 +97,12 @@ __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K)
 //   Z | gate A;  T, W -= A Vu | T masked, Wb;  Su | silu';  Sc (while silu' is formed) | P;  dP, dvc | dS, dSu;  dqc, dkc | staging
 // Tensor memory: W | dkc | dvc | scratch.  Shared memory, seven tiles:
 //   s0 Qu, then Wb | s1 Ku, A, dS | s2 Vu, T, P | s3 Qc | s4 Kc | s5 Vc, staging | s6 dO, dSu, staging
+// with the roles of s1 and s2 exchanged in every other step: P dies first, so that the next Ku lands over it and the next Z runs
+// while dqc is staged.
 // TMA works its queue off in order, and a reduce moves some 18 bytes a cycle: a load queued behind the 64 KB of dqc waits
 // 3.6 k cycles.  So the loads that the next step starts with (Qu, Ku, Vu, Qc) are issued before the reduces, and what is
 // staged over are the tiles that it needs last: dO, and Vc, which is loaded again for that (step 21.7 k cycles with the
-// loads behind the reduces, 19.5 k with Qu, Ku and Qc before them).
+// loads behind the reduces, 18.9 k so, 17.1 k with the next Z under the staging and 16.2 k with the copy of dSu behind the next Qu).
 template <typename T>
 __global__ void __launch_bounds__(kB128Threads, 1)
 castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
@@ -113,17 +115,17 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
                      ID_KM_NEG = make_idesc(128, 128, FMT, false, true, true), ID_MM = make_idesc(128, 128, FMT, true, true, false);
   constexpr float kLog2e = 1.4426950408889634f;
   const int K = blockIdx.y, k0 = K * kBlkB, steps = p.nblk - K;
-  B128_BEGIN(7 * kSq, 12, 512)
+  B128_BEGIN(7 * kSq, 11, 512)
   uint8_t *s0 = smem, *s1 = s0 + kSq, *s2 = s1 + kSq, *s3 = s2 + kSq, *s4 = s3 + kSq, *s5 = s4 + kSq, *s6 = s5 + kSq;
   const uint32_t a0 = smem_u32(s0), a1 = smem_u32(s1), a2 = smem_u32(s2), a3 = smem_u32(s3), a4 = smem_u32(s4), a5 = smem_u32(s5),
                  a6 = smem_u32(s6);
-  uint64_t *bar_res = bars, *bar_z = bars + 1 /* Qu, Ku */, *bar_qc = bars + 2, *bar_vu = bars + 3, *bar_do = bars + 4,
-           *bar_mma = bars + 5 /* Z, Su, Sc, dP: one after another */, *bar_t = bars + 6, *bar_w = bars + 7, *bar_dv = bars + 8,
-           *bar_x0 = bars + 9, *bar_x = bars + 10, *bar_k = bars + 11;
+  uint64_t *bar_res = bars, *bar_z = bars + 1 /* Qu, Ku */, *bar_in = bars + 2 /* Qc, Vu */, *bar_do = bars + 3,
+           *bar_mma = bars + 4 /* Z, Su, Sc, dP: one after another */, *bar_t = bars + 5, *bar_w = bars + 6, *bar_dv = bars + 7,
+           *bar_x0 = bars + 8, *bar_x = bars + 9, *bar_k = bars + 10;
   const int row = (warp & 3) * 32 + lane, cc = warp >> 2, c0 = cc * 32, krow = k0 + row;
   // Lanes with a duty besides the products (warp 0's): the panel of dqc that chunk group cc stages and that panel's
   // refill with Vc or dO; the copies of A and dSu; the other loads.
-  const bool reducer = (warp & 3) == 1, storer = warp == 8, loader = warp == 2;
+  const bool reducer = (warp & 3) == 1, storer = warp == 8, loader = warp == 10;
   auto load_panel = [&](int i0) {
     if (cc < 2) tma_load_4d(s5 + cc * kPanelB, &m_vc, bar_do, cc * 64, k0, h, b);
     else tma_load_4d(s5 + cc * kPanelB, &m_do, bar_do, (cc - 2) * 64, i0, h, b);
@@ -133,10 +135,9 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     mbar_expect_tx(bar_z, 2 * kSq);
     load_op(s0, m_qu, bar_z, k0, h, b);
     load_op(s1, m_ku, bar_z, il, h, b);
-    mbar_expect_tx(bar_qc, kSq);
-    load_op(s3, m_qc, bar_qc, il, h, b);
-    mbar_expect_tx(bar_vu, kSq);
-    load_op(s2, m_vu, bar_vu, il, h, b);
+    mbar_expect_tx(bar_in, 2 * kSq);
+    load_op(s3, m_qc, bar_in, il, h, b);
+    load_op(s2, m_vu, bar_in, il, h, b);
     mbar_expect_tx(bar_do, 2 * kSq);
     mbar_expect_tx(bar_res, kSq);
     load_op(s4, m_kc, bar_res, k0, h, b);
@@ -157,6 +158,14 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
   tc_fence_before();
   __syncthreads();
 
+  // Z = Qu Ku^T of the first step; a later one's is issued in the step before
+  if (warp == 0 && elect_one()) {
+    mbar_wait(bar_z, 0, abortp);
+    tc_fence_after();
+    gemm_kk_t<2>(tmem + C_S, a0, a1, ID_KK, false);
+    mma_commit(bar_mma);
+  }
+  __syncwarp();
   uint32_t ph_mma = 0;
   const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
   for (int n = 0; n < steps; ++n) {
@@ -166,25 +175,14 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     const float lse_b = rvalid ? p.lse[(int64_t)bh * p.N + irow] * kLog2e : 0.f;
     const float delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
     uint8_t* const tile = step_tiles(p, I, K);
+    uint8_t *const sK = n & 1 ? s2 : s1, *const sV = n & 1 ? s1 : s2;
+    const uint32_t aK = n & 1 ? a2 : a1, aV = n & 1 ? a1 : a2;
     B128_MARK(0, n, 0);
-    // ---- Z = Qu Ku^T
-    if (warp == 0 && elect_one()) {
-      mbar_wait(bar_z, ph, abortp);
-      tc_fence_after();
-      gemm_kk_t<2>(tmem + C_S, a0, a1, ID_KK, false);
-      mma_commit(bar_mma);
-    }
-    __syncwarp();
     B128_MARK(0, n, 1);
     mbar_wait(bar_mma, ph_mma, abortp);
     ph_mma ^= 1;
     tc_fence_after();
     B128_MARK(0, n, 2);
-    if (reducer && n > 0 && elect_one()) {   // the reduce of the step before has had time to read its panel
-      bulk_wait_read0();
-      load_panel(i0);
-    }
-    __syncwarp();
     {
       float v[32];
       tmem_ld32(trow + C_S + c0, v);
@@ -198,21 +196,20 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
       }
-      store_row32<T>(s1, kPanelB, row, c0, v);
+      store_row32<T>(sK, kPanelB, row, c0, v);
     }
     B128_SYNC()
     B128_MARK(0, n, 3);
     // ---- T = Qc Vu^T;  W -= A Vu
     if (warp == 0 && elect_one()) {
-      mbar_wait(bar_qc, ph, abortp);
-      mbar_wait(bar_vu, ph, abortp);
+      mbar_wait(bar_in, ph, abortp);
       tc_fence_after();
-      gemm_kk_t<2>(tmem + C_S, a3, a2, ID_KK, false);
+      gemm_kk_t<2>(tmem + C_S, a3, aV, ID_KK, false);
       mma_commit(bar_t);
-      gemm_km_t<8>(tmem + C_W, a1, a2, ID_KM_NEG, true);
+      gemm_km_t<8>(tmem + C_W, aK, aV, ID_KM_NEG, true);
       mma_commit(bar_w);
     }
-    if (storer && elect_one()) { bulk_s2g(tile + kTileA, s1, kSq); bulk_commit(); }
+    if (storer && elect_one()) { bulk_s2g(tile + kTileA, sK, kSq); bulk_commit(); }
     __syncwarp();
     mbar_wait(bar_t, ph, abortp);
     tc_fence_after();
@@ -223,7 +220,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       mbar_wait(bar_w, ph, abortp);
       tc_fence_after();
       tmem_ld32(trow + C_W + c0, w);
-      store_row32<T>(s2, kPanelB, row, c0, v);
+      store_row32<T>(sV, kPanelB, row, c0, v);
       tmem_ld_wait();
       store_row32<T>(s0, kPanelB, row, c0, w);
     }
@@ -233,8 +230,13 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     if (warp == 0 && elect_one()) {
       tc_fence_after();
       if (!diag) gemm_kk_t<2>(tmem + C_S, a3, a0, ID_KK, false);
-      gemm_kk_t<2>(tmem + C_S, a2, a1, ID_KK, !diag);
+      gemm_kk_t<2>(tmem + C_S, aV, aK, ID_KK, !diag);
       mma_commit(bar_mma);
+    }
+    __syncwarp();
+    if (reducer && n > 0 && elect_one()) {   // the reduce of the step before has had time to read its panel, and all wait for Su anyway
+      bulk_wait_read0();
+      load_panel(i0);
     }
     __syncwarp();
     mbar_wait(bar_mma, ph_mma, abortp);
@@ -287,7 +289,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       }
 #pragma unroll
       for (int j = 0; j < 32; j += 2) ppk[j / 2] = Elem<T>::pack2(v[j], v[j + 1]);
-      store_row32<T>(s2, kPanelB, row, c0, v);   // P, over T
+      store_row32<T>(sV, kPanelB, row, c0, v);   // P, over T
     }
     if (storer && elect_one()) bulk_wait_read0();   // A has been read: dS goes there
     __syncwarp();
@@ -299,7 +301,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       tc_fence_after();
       gemm_kk_t<2>(tmem + C_S, a6, a5, ID_KK, false);
       mma_commit(bar_mma);
-      gemm_mm_t<8>(tmem + C_DVC, a2, a6, ID_MM, n > 0);
+      gemm_mm_t<8>(tmem + C_DVC, aV, a6, ID_MM, n > 0);
       mma_commit(bar_dv);
     }
     __syncwarp();
@@ -318,7 +320,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         v[j] = ds.x; v[j + 1] = ds.y;
         w[j] = -du.x; w[j + 1] = -du.y;
       }
-      store_row32<T>(s1, kPanelB, row, c0, v);   // dS
+      store_row32<T>(sK, kPanelB, row, c0, v);   // dS
       mbar_wait(bar_dv, ph, abortp);
       store_row32<T>(s6, kPanelB, row, c0, w);   // dSu, over dO
     }
@@ -329,19 +331,22 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       tc_fence_after();
       if (!diag) gemm_km_t<8>(tmem + C_S, a6, a0, ID_KM, false);
       mma_commit(bar_x0);
-      gemm_km_t<8>(tmem + C_S, a1, a4, ID_KM, !diag);
+      gemm_km_t<8>(tmem + C_S, aK, a4, ID_KM, !diag);
       mma_commit(bar_x);
-      gemm_mm_t<8>(tmem + C_DKC, a1, a3, ID_MM, n > 0);
+      gemm_mm_t<8>(tmem + C_DKC, aK, a3, ID_MM, n > 0);
       mma_commit(bar_k);
     }
-    if (storer && elect_one()) { bulk_s2g(tile + kTileDsu, s6, kSq); bulk_commit(); }
-    if (loader && more && elect_one()) {
+    if (loader && elect_one()) {
+      if (more) {
       mbar_expect_tx(bar_z, 2 * kSq);
-      mbar_expect_tx(bar_qc, kSq);
-      mbar_expect_tx(bar_vu, kSq);
+      mbar_expect_tx(bar_in, 2 * kSq);
       mbar_expect_tx(bar_do, 2 * kSq);
+      load_op(sV, m_ku, bar_z, i0 - kBlkB, h, b);   // over P
       mbar_wait(bar_x0, ph, abortp);
       load_op(s0, m_qu, bar_z, k0, h, b);
+      }
+      bulk_s2g(tile + kTileDsu, s6, kSq);   // behind what the next product waits for
+      bulk_commit();
     }
     __syncwarp();
     mbar_wait(bar_x, ph, abortp);
@@ -350,19 +355,27 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     float v[32];
     tmem_ld32(trow + C_S + c0, v);
     tmem_ld_wait();
-    if (storer && elect_one()) bulk_wait_read0();   // dSu has been read
-    __syncwarp();
     tc_fence_before();
     __syncthreads();
     B128_MARK(0, n, 12);
+    // ---- the next step's Z, while dqc is staged
+    if (warp == 0 && more && elect_one()) {
+      mbar_wait(bar_z, ph ^ 1, abortp);
+      tc_fence_after();
+      gemm_kk_t<2>(tmem + C_S, a0, aV, ID_KK, false);
+      mma_commit(bar_mma);
+    }
     // before the reduces, which loads would queue behind
-    if (loader && more && elect_one()) {
-      load_op(s2, m_vu, bar_vu, i0 - kBlkB, h, b);
-      mbar_wait(bar_k, ph, abortp);
-      load_op(s1, m_ku, bar_z, i0 - kBlkB, h, b);
-      load_op(s3, m_qc, bar_qc, i0 - kBlkB, h, b);
+    if (loader && elect_one()) {
+       if (more) {
+        mbar_wait(bar_k, ph, abortp);
+        load_op(s3, m_qc, bar_in, i0 - kBlkB, h, b);
+        load_op(sK, m_vu, bar_in, i0 - kBlkB, h, b);
+      }
+      bulk_wait_read0();   // dSu has been read
     }
     __syncwarp();
+    if (cc >= 2) asm volatile("bar.sync 5, 256;" ::: "memory");   // the two groups that stage over dSu
     uint8_t* panel = s5 + cc * kPanelB;
     store_row32_f32(panel, row, v);
     fence_async_smem();
@@ -374,7 +387,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       bulk_commit();
     }
   }
-  if ((reducer || storer) && elect_one()) bulk_wait0();
+  if ((reducer || storer || loader) && elect_one()) bulk_wait0();
   __syncwarp();
   mbar_wait(bar_k, (uint32_t)(steps - 1) & 1u, abortp);
   tc_fence_after();
