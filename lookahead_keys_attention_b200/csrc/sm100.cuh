@@ -279,7 +279,8 @@ template <> struct Elem<__nv_bfloat16> {
     return *reinterpret_cast<uint32_t*>(&p);
   }
   static __device__ __forceinline__ float2 unpack2(uint32_t u) {
-    return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
+    // as 32-bit words: taken apart into halves the packed pairs cost the score passes registers (spills in the backward)
+    return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
   }
   static __device__ __forceinline__ float to_f(__nv_bfloat16 x) { return __bfloat162float(x); }
   static __device__ __forceinline__ __nv_bfloat16 from_f(float x) { return __float2bfloat16_rn(x); }
