@@ -74,8 +74,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   constexpr uint32_t C_W = 0, C_G = 64, C_DKC = 128, C_DVC = 192, C_DQU = 256, C_S = 320, C_X = 448;
   constexpr uint32_t C_X2 = C_S, C_X3 = C_S + 64;
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQu = smem;                 // resident
   uint8_t* sKc = sQu + OPB;            // resident
   uint8_t* sQc = sKc + OPB;            // per step
@@ -88,7 +87,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   uint8_t* sGb = sWb + OPB;
   uint8_t* sA = sGb + OPB;             // slot 1: gate A
   uint8_t* sT = sA + SQB;              // slot 2: masked T, later dZ
-  __shared__ uint64_t bar_res, bar_load, bar_vd, bar_ku, bar_mma, bar_x1, bar_x2, bar_kn, bar_w, bar_dv;
+  __shared__ uint64_t bar_res, bar_load, bar_vd, bar_ku, bar_mma, bar_x1, bar_x2, bar_kn, bar_w, bar_dv, bar_g;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
@@ -101,9 +100,10 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   const int k0 = K * kBlkB, krow = k0 + row;
 
   if (tid == 0) {
+    if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
     mbar_init(&bar_res, 1); mbar_init(&bar_load, 1); mbar_init(&bar_vd, 1); mbar_init(&bar_ku, 1); mbar_init(&bar_mma, 1);
     mbar_init(&bar_x1, 1); mbar_init(&bar_x2, 1); mbar_init(&bar_kn, 1);
-    mbar_init(&bar_w, 1); mbar_init(&bar_dv, 1);
+    mbar_init(&bar_w, 1); mbar_init(&bar_dv, 1); mbar_init(&bar_g, 1);
     mbar_fence_init();
     abort_flag = 0;
   }
@@ -158,11 +158,13 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   tc_fence_before();       \
   __syncthreads();
 
-  float lse_nx = 0.f, delta_nx = 0.f;
-  if ((p.nblk - 1) * kBlkB + row < p.N) {
-    lse_nx = p.lse[(int64_t)bh * p.N + (p.nblk - 1) * kBlkB + row];
-    delta_nx = p.delta[(int64_t)bh * p.N + (p.nblk - 1) * kBlkB + row];
-  }
+  auto issue_z = [&](uint32_t phase) {
+    mbar_wait(&bar_kn, phase, abortp);
+    tc_fence_after();
+    gemm_kk_t<1>(tmem + C_S, aQu, aKP, ID_SQ_KK, false);
+    mma_commit(&bar_mma);
+  };
+  if (tid == 0) issue_z(0);
   for (int I = p.nblk - 1; I >= K; --I) {
     const int i0 = I * kBlkB, irow = i0 + row;
     const bool diag = (I == K), first = (I == p.nblk - 1);
@@ -172,21 +174,10 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
 #endif
     BPHASE_MARK(0);
 
-    // the row statistics were fetched one step ahead (their latency hides behind the step before)
-    const float lse_b = lse_nx * kLog2e, delta_i = delta_nx;
-    if (I > K) {
-      const int64_t nrow = (int64_t)bh * p.N + irow - kBlkB;   // rows of block I-1 always exist
-      lse_nx = p.lse[nrow];
-      delta_nx = p.delta[nrow];
-    }
-    // ---- M1: Z = Qu[K] @ Ku[I]^T   (Ku[I] was fetched during the last phase of the step before)
-    if (tid == 0) {
-      mbar_wait(&bar_kn, ph_load, abortp);
-      BPHASE_MARK(1);
-      tc_fence_after();
-      gemm_kk_t<1>(tmem + C_S, aQu, aKP, ID_SQ_KK, false);
-      mma_commit(&bar_mma);
-    }
+    // needed some thousand cycles on: their latency hides behind the passes before
+    const float lse_i = rvalid ? p.lse[(int64_t)bh * p.N + irow] : 0.f, delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
+    // ---- M1: Z = Qu[K] @ Ku[I]^T was issued at the end of the step before
+    BPHASE_MARK(1);
     MMA_WAIT();
     BPHASE_MARK(2);
     {  // gate A (rows k, columns j), zero unless j > k
@@ -248,9 +239,12 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       if (!diag) gemm_kk_t<1>(tmem + C_S, aQc, aWb, ID_SQ_KK, false);
       gemm_kk_t<2>(tmem + C_S, aT, aA, ID_SQ_KK, !diag);
       mma_commit(&bar_mma);
-      bulk_wait_read0();   // this thread's dvu reduce of the step before has read Vc|dO's slot
-      mbar_expect_tx(&bar_vd, 2 * OPB);
-      tma_load_4d(sVc, &m_vc, &bar_vd, 0, k0, h, b);   // needed at the fifth phase
+      mbar_expect_tx(&bar_vd, 2 * OPB);   // needed at the fifth phase; each into the panel that its issuer's dvu reduce of the
+      bulk_wait_read0();                  // step before has read
+      tma_load_4d(sVc, &m_vc, &bar_vd, 0, k0, h, b);
+    }
+    if (tid == kPrefetchTid) {
+      bulk_wait_read0();
       tma_load_4d(sdO, &m_do, &bar_vd, 0, i0, h, b);
     }
     MMA_WAIT();
@@ -287,7 +281,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
-        const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(sl2), splat(-lse_b));
+        const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(sl2), splat(-lse_i * kLog2e));
         v[j] = ex2_approx(x.x); v[j + 1] = ex2_approx(x.y);
       }
       if (diag) {
@@ -373,6 +367,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       gemm_km_t<8>(tmem + C_S, aKP, aA, ID_SQ_KM, false);
       mma_commit(&bar_mma);
       gemm_mm_t<8>(tmem + C_G, aKP, aQc, ID_D_MM, !first);
+      mma_commit(&bar_g);
     }
     MMA_WAIT();
     BPHASE_MARK(14);
@@ -394,9 +389,10 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     // takes thousands of cycles to drain and loads issued behind one wait for it).  After each commit the
     // query-block gradient it completes is staged as fp32 panels in an operand slot that is dead by then
     // and handed to a TMA reduce (whole lines at L2 instead of scattered atomics): chunk group 1 takes
-    // dqc (into Wb + the spare half of slot 4), group 2 dku (into slot 2, which held dZ), group 0 - the
-    // issuing thread's, busy until the end - dvu (into Vc|dO, which held dT and is re-loaded last in the
-    // next step); group 3 fetches the next tiles and refreshes the 16-bit copy of G.
+    // dqc (into Wb + the spare half of slot 4), group 2 dku (into slot 2, which held dZ), groups 0 and 3 a panel each of dvu
+    // (into Vc|dO, which held dT and is re-loaded last in the next step); group 3 also fetches the next tiles and refreshes the
+    // 16-bit copy of G.  Z of the next step is issued as soon as dvu has been read from its columns and runs under that
+    // staging; Ku is fetched first, behind the G update (2582 -> 2507 us at B=4 N=4096 H=16 bf16; 2589 -> 2462 at B=1 N=16384 H=4).
     if (tid == 0) {
       tc_fence_after();
       gemm_mm_t<8>(tmem + C_X2, aVD, aQc, ID_D_MM, false);
@@ -410,14 +406,13 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       mma_commit(&bar_mma);
     }
     ph_ku ^= 1;
-    const bool issuer = (quarter == 0 && lane == 0);   // threads 0, 128, 256 issue the reduces
     if (cc == 1) {
       mbar_wait(&bar_x1, ph_x, abortp);
       tc_fence_after();
       stage_f32_tile(trow + C_X, sWb, sKP + kPanelB, row);
       fence_async_smem();
       group_sync(1);
-      if (issuer) {
+      if (quarter == 0 && lane == 0) {
         tma_reduce_add_3d(&m_acc_dqc, sWb, 0, i0, bh);
         tma_reduce_add_3d(&m_acc_dqc, sKP + kPanelB, 32, i0, bh);
         bulk_commit();
@@ -428,17 +423,20 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       stage_f32_tile(trow + C_X3, sT, sT + kPanelB, row);
       fence_async_smem();
       group_sync(2);
-      if (issuer) {
+      if (quarter == 0 && lane == 0) {
         tma_reduce_add_3d(&m_acc_dku, sT, 0, i0, bh);
         tma_reduce_add_3d(&m_acc_dku, sT + kPanelB, 32, i0, bh);
         bulk_commit();
       }
     } else if (cc == 3) {
-      mbar_wait(&bar_x1, ph_x, abortp);   // Qc[I], Vu[I], Ku[I] are consumed
-      if (tid == kPrefetchTid && I > K) {
-        const int in0 = i0 - kBlkB;
+      const int in0 = i0 - kBlkB;
+      if (tid == kPrefetchTid && I > K) {   // Ku first: the next Z waits for it, and its slot (dSu) is free as soon as G is done
+        mbar_wait(&bar_g, ph_x, abortp);
         mbar_expect_tx(&bar_kn, OPB);
         tma_load_4d(sKP, &m_ku, &bar_kn, 0, in0, h, b);
+      }
+      mbar_wait(&bar_x1, ph_x, abortp);   // Qc[I], Vu[I], Ku[I] are consumed
+      if (tid == kPrefetchTid && I > K) {
         mbar_expect_tx(&bar_load, 2 * OPB);
         tma_load_4d(sQc, &m_qc, &bar_load, 0, in0, h, b);
         tma_load_4d(sVu, &m_vu, &bar_load, 0, in0, h, b);
@@ -449,30 +447,38 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     BPHASE_MARK(16);
     MMA_WAIT();
     BPHASE_MARK(17);
-    if (cc == 0) {
-      stage_f32_tile(trow + C_X2, sVD, sVD + kPanelB, row);
+    // The products' last columns are read, then the next step's Z is issued over them and runs while dvu is staged and G copied.
+    float v[32];
+    if (cc == 0 || cc == 3) {   // a panel of dvu each
+      tmem_ld32(trow + C_X2 + (cc == 3 ? 32 : 0), v);
+      tmem_ld_wait();
+    }
+    tc_fence_before();
+    __syncthreads();
+    BPHASE_MARK(18);
+    if (tid == 0 && I > K) issue_z(ph_load);
+    if (cc == 0 || cc == 3) {
+      uint8_t* panel = cc == 3 ? sVD + kPanelB : sVD;
+      store_row32_f32(panel, row, v);
       fence_async_smem();
-      group_sync(3);
-      if (issuer) {
-        tma_reduce_add_3d(&m_acc_dvu, sVD, 0, i0, bh);
-        tma_reduce_add_3d(&m_acc_dvu, sVD + kPanelB, 32, i0, bh);
+      group_sync(cc == 0 ? 3 : 4);
+      if (quarter == 0 && lane == 0) {
+        tma_reduce_add_3d(&m_acc_dvu, panel, cc == 3 ? 32 : 0, i0, bh);
         bulk_commit();
       }
-    } else if (cc == 3) {  // 16-bit copy of G including block I, for the next (lower) block
+    }
+    if (cc == 3) {  // 16-bit copy of G including block I, for the next (lower) block; ordered by the next step's barriers
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
-        float v[32];
         tmem_ld32(trow + C_G + c * 32, v);
         tmem_ld_wait();
         store_row32<T>(sGb, kPanelB, row, c * 32, v);
       }
     }
-    BPHASE_MARK(18);
     BPHASE_MARK(19);
-    SMEM_TO_MMA_SYNC();
     BPHASE_MARK(20);
   }
-  if (cc < 3 && quarter == 0 && lane == 0) bulk_wait0();
+  if (quarter == 0 && lane == 0) bulk_wait0();
 #undef MMA_WAIT
 #undef SMEM_TO_MMA_SYNC
 
