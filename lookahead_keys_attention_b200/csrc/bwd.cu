@@ -91,7 +91,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int quarter = warp & 3, cc = warp >> 2;
   const int row = quarter * 32 + lane;
   const int c0 = cc * 32;
@@ -149,7 +149,9 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
                  aWb = smem_u32(sWb), aGb = smem_u32(sGb), aA = smem_u32(sA), aT = smem_u32(sT);
   const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
 
+// (the issuing thread's warp converges before it polls)
 #define MMA_WAIT()                       \
+  __syncwarp();                          \
   mbar_wait(&bar_mma, ph_mma, abortp);   \
   ph_mma ^= 1;                           \
   tc_fence_after();
@@ -161,7 +163,9 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   auto issue_z = [&](uint32_t phase) {
     mbar_wait(&bar_kn, phase, abortp);
     tc_fence_after();
-    gemm_kk_t<1>(tmem + C_S, aQu, aKP, ID_SQ_KK, false);
+    uint32_t base = smem_u32(smem);
+    asm volatile("" : "+r"(base));   // the descriptors are made here, not kept in registers over the step
+    gemm_kk_t<1>(tmem + C_S, base + (uint32_t)(sQu - smem), base + (uint32_t)(sKP - smem), ID_SQ_KK, false);
     mma_commit(&bar_mma);
   };
   if (tid == 0) issue_z(0);
@@ -174,8 +178,6 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
 #endif
     BPHASE_MARK(0);
 
-    // needed some thousand cycles on: their latency hides behind the passes before
-    const float lse_i = rvalid ? p.lse[(int64_t)bh * p.N + irow] : 0.f, delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
     // ---- M1: Z = Qu[K] @ Ku[I]^T was issued at the end of the step before
     BPHASE_MARK(1);
     MMA_WAIT();
@@ -247,6 +249,8 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       bulk_wait_read0();
       tma_load_4d(sdO, &m_do, &bar_vd, 0, i0, h, b);
     }
+    // loaded here, not at the top of the step, where the wait for Z is short (2552 -> 2467 us)
+    const float lse_i = rvalid ? p.lse[(int64_t)bh * p.N + irow] : 0.f, delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
     MMA_WAIT();
     BPHASE_MARK(6);
     uint32_t dpk[16];  // silu'(Su), later dSu, two 16-bit values per register
@@ -392,7 +396,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     // dqc (into Wb + the spare half of slot 4), group 2 dku (into slot 2, which held dZ), groups 0 and 3 a panel each of dvu
     // (into Vc|dO, which held dT and is re-loaded last in the next step); group 3 also fetches the next tiles and refreshes the
     // 16-bit copy of G.  Z of the next step is issued as soon as dvu has been read from its columns and runs under that
-    // staging; Ku is fetched first, behind the G update (2582 -> 2507 us at B=4 N=4096 H=16 bf16; 2589 -> 2462 at B=1 N=16384 H=4).
+    // staging; Ku is fetched first, behind the G update (2582 -> 2551 us at B=4 N=4096 H=16 bf16; 2589 -> 2485 at B=1 N=16384 H=4).
     if (tid == 0) {
       tc_fence_after();
       gemm_mm_t<8>(tmem + C_X2, aVD, aQc, ID_D_MM, false);
@@ -461,7 +465,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       uint8_t* panel = cc == 3 ? sVD + kPanelB : sVD;
       store_row32_f32(panel, row, v);
       fence_async_smem();
-      group_sync(cc == 0 ? 3 : 4);
+      group_sync(3 + cc);
       if (quarter == 0 && lane == 0) {
         tma_reduce_add_3d(&m_acc_dvu, panel, cc == 3 ? 32 : 0, i0, bh);
         bulk_commit();
