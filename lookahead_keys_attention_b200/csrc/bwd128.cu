@@ -9,9 +9,9 @@
 //
 // Every gradient but dqc is owned by a CTA that keeps it in tensor memory.  A TMA reduce moves some 18 bytes per cycle and SM,
 // so a lookahead kernel that owned a key block and reduced dku[I] and dvu[I] (128 KB a step, with dT masked and multiplied in
-// every step) took 18.5 k cycles a step, 12.1 k without the reduces; reverse + la + dqu take 3.1 + 8.0 + 1.9 k, and kv, which
-// no longer forms dT, went from 20.8 to 16.2 k.  Measured on B=1 H=8 N=8190 bf16: 2365 -> 1774 us for the kernels, B=2 H=8 N=1333:
-// 249 -> 195 us.  What bounds them: kv its chain of six products with a pass behind each; la and reverse the tiles, which
+// every step) took 18.5 k cycles a step, 12.1 k without the reduces; reverse + la + dqu take 3.1 + 7.3 + 1.9 k, and kv, which
+// no longer forms dT, went from 20.8 to 16.2 k.  Measured on B=1 H=8 N=8190 bf16: 2365 -> 1708 us for the kernels, B=2 H=8 N=1333:
+// 249 -> 182 us.  What bounds them: kv its chain of six products with a pass behind each; la and reverse the tiles, which
 // come at 20 to 30 bytes per cycle and SM with one step's worth of shared memory to prefetch into; dqu HBM.  (Handing W on
 // as well, from a kernel of its own, so that kv starts at Su: 4.4 + 17 k cycles.)
 //
@@ -462,8 +462,16 @@ castle_bwd128_reverse_kernel(const BwdParams p, const __grid_constant__ CUtensor
 }
 
 // ------------------------------------------------------------------------------------------------ dku, dvu, dT, dqc
+// 16 warps for the passes and one that moves tiles: a tile's slot is filled again as soon as its last reader is done, so the
+// products are ordered by what they free (Gb first): 1737 -> 1708 us of backward at N=8190 H=8 against loads issued by one of
+// the 16 warps after its pass.
+__device__ __forceinline__ void sync_passes() {
+  fence_async_smem();
+  tc_fence_before();
+  asm volatile("bar.sync 1, 512;" ::: "memory");
+}
 template <typename T>
-__global__ void __launch_bounds__(kB128Threads, 1)
+__global__ void __launch_bounds__(kB128Threads + 32, 1)
 castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_qu,
                        const __grid_constant__ CUtensorMap m_vu) {
   constexpr int FMT = Elem<T>::fmt;
@@ -472,31 +480,55 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
                      ID_MM = make_idesc(128, 128, FMT, true, true, false);
   const int I = p.nblk - 1 - blockIdx.y, i0 = I * kBlkB;   // the longest walks first
   const bool last = I == p.nblk - 1;                       // no G there yet
-  B128_BEGIN(7 * kSq, 7, 512)
+  B128_BEGIN(7 * kSq, 10, 512)
   uint8_t *sVu = smem, *sT = smem + kSq, *sA = smem + 2 * kSq, *sS = smem + 3 * kSq, *sG = smem + 4 * kSq, *sQu = smem + 5 * kSq,
           *sZ = smem + 6 * kSq;
-  uint64_t *bar_res = bars, *bar_in = bars + 1, *bar_qu = bars + 2, *bar_da = bars + 3, *bar_v = bars + 4, *bar_k = bars + 5, *bar_t = bars + 6;
+  uint64_t *bar_res = bars, *bar_in = bars + 1, *bar_qu = bars + 2, *bar_da = bars + 3, *bar_v = bars + 4, *bar_k = bars + 5, *bar_t = bars + 6,
+           *bar_g = bars + 7, *bar_p = bars + 8, *bar_zf = bars + 9;
   const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;
-  const bool loader = warp == 4;
-  auto load_tiles = [&](int K) {
-    const uint8_t* t = step_tiles(p, I, K);
-    mbar_expect_tx(bar_in, last ? 2 * kSq : 3 * kSq);
-    if (!last) bulk_g2s(sG, t + kTileG, kSq, bar_in);
-    bulk_g2s(sS, t + kTileDsu, kSq, bar_in);
-    bulk_g2s(sA, t + kTileA, kSq, bar_in);
-  };
-  auto load_qu = [&](int K) {
-    mbar_expect_tx(bar_qu, kSq);
-    load_op(sQu, m_qu, bar_qu, K * kBlkB, h, b);
-  };
-  if (loader && elect_one()) {
-    mbar_expect_tx(bar_res, 2 * kSq);
-    load_op(sVu, m_vu, bar_res, i0, h, b);
-    load_op(sZ, m_qc, bar_res, i0, h, b);
-    load_tiles(0);
-    load_qu(0);
-  }
-  __syncwarp();
+  if (warp == 16) {
+    if (elect_one()) {
+      auto load_qu = [&](int K) {
+        mbar_expect_tx(bar_qu, kSq);
+        load_op(sQu, m_qu, bar_qu, K * kBlkB, h, b);
+      };
+      mbar_expect_tx(bar_res, 2 * kSq);
+      load_op(sVu, m_vu, bar_res, i0, h, b);
+      load_op(sZ, m_qc, bar_res, i0, h, b);
+      const uint32_t bytes = last ? 2 * kSq : 3 * kSq;
+      mbar_expect_tx(bar_in, bytes);
+      if (!last) bulk_g2s(sG, step_tiles(p, I, 0) + kTileG, kSq, bar_in);
+      bulk_g2s(sS, step_tiles(p, I, 0) + kTileDsu, kSq, bar_in);
+      bulk_g2s(sA, step_tiles(p, I, 0) + kTileA, kSq, bar_in);
+      load_qu(0);
+      for (int K = 0; K <= I; ++K) {
+        const uint32_t ph = K & 1;
+        const bool more = K < I;
+        const uint8_t* next = step_tiles(p, I, K + 1);
+        if (more) {
+          mbar_wait_lazy_abort(last ? bar_v : bar_g, ph, abortp);
+          mbar_expect_tx(bar_in, bytes);
+          if (!last) {
+            bulk_g2s(sG, next + kTileG, kSq, bar_in);
+            mbar_wait_lazy_abort(bar_v, ph, abortp);
+          }
+          bulk_g2s(sS, next + kTileDsu, kSq, bar_in);
+        }
+        mbar_wait_lazy_abort(bar_p, ph, abortp);   // the pass has read A and written dZ
+        if (more) bulk_g2s(sA, next + kTileA, kSq, bar_in);
+        bulk_s2g(step_tiles(p, I, K) + kTileA, sZ, kSq);   // behind the loads, which would queue behind it
+        bulk_commit();
+        if (more) {
+          mbar_wait_lazy_abort(bar_k, ph, abortp);
+          load_qu(K + 1);
+        }
+        bulk_wait_read0();
+        mbar_arrive(bar_zf);
+      }
+      bulk_wait0();
+    }
+    __syncwarp();
+  } else {
   const uint32_t aVu = smem_u32(sVu), aT = smem_u32(sT), aA = smem_u32(sA), aS = smem_u32(sS), aG = smem_u32(sG), aQu = smem_u32(sQu),
                  aZ = smem_u32(sZ);
   // ---- the masked T = tril(Qc Vu^T)
@@ -514,28 +546,29 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     tmem_ld32_lower(trow + C_DA + c0, row, c0, v);
     store_row32<T>(sT, kPanelB, row, c0, v);
   }
-  B128_SYNC()
+  sync_passes();
   for (int K = 0; K <= I; ++K) {
     const uint32_t ph = K & 1;
-    // ---- dA/scale = Gb Vu^T + dSu^T T;  dT += dSu A;  dvu += A^T Gb
+    // ---- dA/scale = Gb Vu^T + dSu^T T;  dvu += A^T Gb;  dT += dSu A
     if (warp == 0 && elect_one()) {
       B128_MARK(512, K, 0);
       mbar_wait(bar_in, ph, abortp);
       tc_fence_after();
       B128_MARK(512, K, 1);
-      if (!last) gemm_kk_t<2>(tmem + C_DA, aG, aVu, ID_KK, false);
+      if (!last) {
+        gemm_kk_t<2>(tmem + C_DA, aG, aVu, ID_KK, false);
+        gemm_mm_t<8>(tmem + C_DVU, aA, aG, ID_MM, K > 0);
+        mma_commit(bar_g);
+      }
       gemm_mm_t<8>(tmem + C_DA, aS, aT, ID_MM, !last);
       mma_commit(bar_da);
       gemm_km_t<8>(tmem + C_DT, aS, aA, ID_KM, K > 0);
-      if (!last) gemm_mm_t<8>(tmem + C_DVU, aA, aG, ID_MM, K > 0);
       mma_commit(bar_v);
     }
     __syncwarp();
-    if (loader && elect_one()) bulk_wait_read0();   // dZ of the step before has been copied
-    __syncwarp();
     B128_MARK(512, K, 2);
-    mbar_wait(bar_da, ph, abortp);   // (its last reader, the dku product, came before these)
-    __syncthreads();
+    mbar_wait(bar_da, ph, abortp);   // (dZ's last reader, the dku product, came before these)
+    if (K > 0) mbar_wait(bar_zf, ph ^ 1, abortp);   // and its copy has been made
     tc_fence_after();
     B128_MARK(512, K, 3);
     {
@@ -551,7 +584,7 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       }
       store_row32<T>(sZ, kPanelB, row, c0, v);
     }
-    B128_SYNC()
+    sync_passes();
     B128_MARK(512, K, 4);
     // ---- dku += dZ^T Qu
     if (warp == 0 && elect_one()) {
@@ -561,26 +594,14 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       gemm_mm_t<8>(tmem + C_DKU, aZ, aQu, ID_MM, K > 0);
       mma_commit(bar_k);
     }
-    if (loader && elect_one()) {   // the copy last: loads would queue behind it
-      if (K < I) {
-        mbar_wait(bar_v, ph, abortp);
-        load_tiles(K + 1);
-      }
-      bulk_s2g(step_tiles(p, I, K) + kTileA, sZ, kSq);
-      bulk_commit();
-      if (K < I) {
-        mbar_wait(bar_k, ph, abortp);
-        load_qu(K + 1);
-      }
-    }
+    if (warp == 1 && elect_one()) mbar_arrive(bar_p);
     __syncwarp();
   }
   // ---- the masked dT (over dZ):  dvu += dT^T Qc;  dqc += dT Vu
-  if (loader && elect_one()) bulk_wait_read0();
+  mbar_wait(bar_zf, (uint32_t)I & 1u, abortp);
   mbar_wait(bar_k, (uint32_t)I & 1u, abortp);
-  __syncthreads();
   tc_fence_after();
-  if (loader && elect_one()) {
+  if (warp == 4 && elect_one()) {
     mbar_expect_tx(bar_res, kSq);
     load_op(sQu, m_qc, bar_res, i0, h, b);
   }
@@ -590,7 +611,7 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     tmem_ld32_lower(trow + C_DT + c0, row, c0, v);
     store_row32<T>(sZ, kPanelB, row, c0, v);
   }
-  B128_SYNC()
+  sync_passes();
   if (warp == 0 && elect_one()) {
     mbar_wait(bar_res, 1, abortp);
     tc_fence_after();
@@ -620,8 +641,7 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     }
     store_grad32<T>(grad_row<T>(p.dqc, b, h, irow, c0), v, p.scale);
   }
-  if (loader && elect_one()) bulk_wait0();
-  __syncwarp();
+  }
   B128_END(512)
 }
 
@@ -707,7 +727,7 @@ static int launch_bwd128_t(const BwdParams& p, const CUtensorMap* in, cudaStream
     // each starts while the one before it ends
     cudaError_t e = launch_kernel(castle_bwd128_kv_kernel<T>, grid, kB128Threads, smem[0], st, true, q, in[0], in[1], in[2], in[3], in[4], in[5], in[6], acc);
     if (e == cudaSuccess && p.nblk > 1) e = launch_kernel(castle_bwd128_reverse_kernel<T>, dim3(pairs, p.nblk - 1), kB128Threads, smem[1], st, true, q, in[0]);
-    if (e == cudaSuccess) e = launch_kernel(castle_bwd128_la_kernel<T>, grid, kB128Threads, smem[2], st, true, q, in[0], in[3], in[5]);
+    if (e == cudaSuccess) e = launch_kernel(castle_bwd128_la_kernel<T>, grid, kB128Threads + 32, smem[2], st, true, q, in[0], in[3], in[5]);
     if (e == cudaSuccess) e = launch_kernel(castle_bwd128_dqu_kernel<T>, grid, 128, smem[3], st, true, q, in[4]);
     if (e != cudaSuccess) return cuda_fail(e, "castle_bwd launch");
   }
