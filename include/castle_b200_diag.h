@@ -52,6 +52,10 @@ int castle_selftest_mma_rate(int32_t form, int32_t n, int32_t reps, long long* c
  * polls[0] receives the number of polls the first wait made, polls[1] the second (device int32[2]). */
 int castle_selftest_wait_timeout(int32_t poll_limit, int32_t* polls, int32_t* status, void* stream);
 
+/* y[i] = 2^x[i] for `count` (even, at most 2^26) values as the score passes at dim_head 64 compute a part of their
+ * exponentials, without the special-function unit (no counterpart in the reference). */
+int castle_selftest_exp2(const float* x, float* y, int32_t count, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -286,7 +286,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
         const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(sl2), splat(-lse_i * kLog2e));
-        const float2 e = j % 16 == 0 ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));   // an eighth off the busiest unit: 2409 -> 2388 us
+        const float2 e = j % 16 == 0 ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));   // an eighth off the busiest unit: 2421 -> 2410 us
         v[j] = e.x; v[j + 1] = e.y;
       }
       if (diag) {

@@ -448,7 +448,7 @@ castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_
         for (int j = 0; j < 32; j += 2) {
           const float2 x = fma2(make_float2(s[c][j], s[c][j + 1]), splat(sl2), splat(-mb));
           // exp(scale*v - max); masked entries give 0.  An eighth of them at dim_head 64, where the special-function unit is
-          // the busiest (53 %), is computed on the FMA pipe: 745 -> 728 us at B=4 N=4096 H=16 (a quarter: 742); no gain at 128.
+          // the busiest (53 %), is computed on the FMA pipe: 752 -> 746 us at B=4 N=4096 H=16; no gain at 128.
           const float2 e = D == 64 && j % 16 == 0 ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));
           s[c][j] = e.x;
           s[c][j + 1] = e.y;

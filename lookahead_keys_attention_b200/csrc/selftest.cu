@@ -226,3 +226,18 @@ extern "C" int castle_selftest_wait_timeout(int32_t poll_limit, int32_t* polls, 
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_selftest_wait_timeout launch");
 }
+
+// ---------------------------------------------------------------------------------------------
+namespace castle {
+__global__ void __launch_bounds__(256) castle_exp2_kernel(const float2* x, float2* y, int32_t pairs) {
+  for (int32_t i = blockIdx.x * 256 + threadIdx.x; i < pairs; i += gridDim.x * 256) y[i] = exp2_fma2(x[i]);
+}
+}  // namespace castle
+
+extern "C" int castle_selftest_exp2(const float* x, float* y, int32_t count, void* stream) {
+  if (!x || !y || count < 2 || count % 2 || count > 1 << 26) return reject("castle_selftest_exp2: bad arguments");
+  if (((uintptr_t)x) % 8 || ((uintptr_t)y) % 8) return reject("castle_selftest_exp2: pointers must be 8-byte aligned");
+  castle_exp2_kernel<<<148, 256, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float2*>(x), reinterpret_cast<float2*>(y), count / 2);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : cuda_fail(e, "castle_selftest_exp2 launch");
+}

@@ -348,21 +348,30 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return d;
 }
 __device__ __forceinline__ float2 splat(float x) { return make_float2(x, x); }
-// 2^x of a pair without the special-function unit, for part of a pass that saturates it: x = n + f with n = floor(x) (the low
-// bits of x + 1.5 * 2^23, rounded down), 2^f as 1 + f q(f), q of degree 4 fitted for the least relative error on [0, 1), and n
-// added to the exponent.  Error at most 1.5e-7 (ex2.approx: 2^-22.5 = 1.7e-7); exact at integers; 0 at and below -127.
+__device__ __forceinline__ float clamp_nan(float x, float lo, float hi) {   // NaN stays NaN (fminf and fmaxf drop it)
+  float y;
+  asm("{\n\t.reg .f32 a;\n\tmax.NaN.f32 a, %1, %2;\n\tmin.NaN.f32 %0, a, %3;\n\t}" : "=f"(y) : "f"(x), "f"(lo), "f"(hi));
+  return y;
+}
+// 2^x of a pair without the special-function unit, for part of a pass that saturates it (range reduction and a polynomial, as
+// in Cody and Waite, Software Manual for the Elementary Functions): x = n + f with n = floor(x), 2^f as 1 + f q(f), q of
+// degree 4 fitted for the least relative error on [0, 1), times 2^n.  The low bits of x + (1.5 * 2^23 + 127), rounded down,
+// are n + 127, which shifted to the exponent's place is the float 2^n.  Error at most 1.7e-7 (ex2.approx: 2^-22.5 = 1.7e-7);
+// exact at integers; 0 below -126, infinity from 128 on and NaN for NaN like ex2.approx.ftz: the product carries a NaN, which an
+// addition to the exponent bits would turn into a number.
 __device__ __forceinline__ float2 exp2_fma2(float2 x) {
-  x = make_float2(fmaxf(x.x, -127.f), fmaxf(x.y, -127.f));
+  x = make_float2(clamp_nan(x.x, -127.f, 128.f), clamp_nan(x.y, -127.f, 128.f));
+  constexpr float kBias = 12582912.f + 127.f;
   float2 t;
   asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tadd.rm.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
-      : "=f"(t.x), "=f"(t.y) : "f"(x.x), "f"(x.y), "f"(12582912.f));
-  const float2 f = fma2(add2(t, splat(-12582912.f)), splat(-1.f), x);
+      : "=f"(t.x), "=f"(t.y) : "f"(x.x), "f"(x.y), "f"(kBias));
+  const float2 f = fma2(add2(t, splat(-kBias)), splat(-1.f), x);
   float2 p = fma2(splat(0.0018689563730731606f), f, splat(0.009014884941279888f));
   p = fma2(p, f, splat(0.05579930171370506f));
   p = fma2(p, f, splat(0.24016565084457397f));
   p = fma2(p, f, splat(0.69315105676651f));
   p = fma2(p, f, splat(1.f));
-  return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)), __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
+  return mul2(p, make_float2(__int_as_float(__float_as_int(t.x) << 23), __int_as_float(__float_as_int(t.y) << 23)));
 }
 // sigmoid of a pair as one special-function op each: 0.5 * tanh.approx(x / 2) + 0.5, with `half_scale` = scale / 2 for
 // x = scale * v.  tanh.approx is good to about 2^-11, i.e. the result to ~2.4e-4: below bf16 rounding (2e-3) and at the
