@@ -8,6 +8,7 @@
 // libcastle_b200.so is bound by address (`bind`).
 //
 // Operators and their semantics: ops.py and castle.py.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/grad_mode.h>
@@ -722,10 +723,8 @@ PyObject* guarded(F&& f) {   // C++ exceptions become Python ones; `f` runs with
     return f();
   } catch (const AssertError& e) {
     PyErr_SetString(PyExc_AssertionError, e.what());
-  } catch (const c10::Error& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (const std::exception&) {   // as torch's own bindings do: a Python exception of a hook, OutOfMemoryError and so on
+    torch::translate_exception_to_python(std::current_exception());
   }
   return nullptr;
 }

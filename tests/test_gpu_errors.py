@@ -1,0 +1,56 @@
+"""GPU: exceptions keep their types on the way through the native host path (csrc/host.cpp)."""
+import pytest
+import torch
+from torch.utils.checkpoint import checkpoint
+
+pytestmark = pytest.mark.gpu
+
+
+class Refused(Exception):
+    pass
+
+
+def _refuse(t):
+    raise Refused("no")
+
+
+@pytest.mark.parametrize("layer", [False, True])
+def test_an_exception_of_a_hook_keeps_its_type(layer):
+    from lookahead_keys_attention_b200 import Castle, castle_attention_packed
+    if layer:
+        f = Castle(96, heads=2, prenorm=True).cuda().bfloat16()
+        x = torch.randn(1, 130, 96, device="cuda").bfloat16().requires_grad_()
+    else:
+        f = lambda t: castle_attention_packed(t, 0.125)   # noqa: E731
+        x = torch.randn(1, 130, 6, 2, 64, device="cuda").bfloat16().requires_grad_()
+    with pytest.raises(Refused), torch.autograd.graph.saved_tensors_hooks(_refuse, lambda t: t):
+        f(x)
+
+
+def test_checkpoint_may_stop_the_second_forward_early():
+    """Non-reentrant checkpointing ends its recomputation with an exception out of the last hook it needs."""
+    from lookahead_keys_attention_b200 import castle_attention_packed
+    x = torch.randn(1, 130, 6, 2, 64, device="cuda").bfloat16().requires_grad_()
+    g = torch.randn(1, 2, 130, 64, device="cuda").bfloat16()
+    plain = torch.autograd.grad(castle_attention_packed(x, 0.125), x, g)[0]
+    again = torch.autograd.grad(checkpoint(castle_attention_packed, x, 0.125, use_reentrant=False), x, g)[0]
+    assert (again.float() - plain.float()).norm().item() <= 4e-3 * plain.float().norm().item()   # dqc is summed in arrival order
+
+
+def test_out_of_memory_keeps_its_type():
+    from lookahead_keys_attention_b200 import castle_attention_packed, check_status, release_workspaces
+    x = torch.randn(1, 1024, 6, 8, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        out = castle_attention_packed(x, 0.125)
+        release_workspaces()
+        del out
+        torch.cuda.empty_cache()
+        total = torch.cuda.get_device_properties(0).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (4 << 20)) / total)
+        try:
+            with pytest.raises(torch.OutOfMemoryError):
+                castle_attention_packed(x, 0.125)
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        castle_attention_packed(x, 0.125)   # nothing is left half made
+    check_status()
