@@ -128,6 +128,14 @@ castle_tensor_t packed_desc(const Tensor& p, int i) {
   return {static_cast<char*>(p.data_ptr()) + i * p.stride(2) * p.element_size(), p.stride(0), p.stride(3), p.stride(1)};
 }
 
+// A packed (B, N, 6, H, d) tensor as the kernels take it: itself, or a copy.
+Tensor aligned_packed(const Tensor& t) {
+  const int64_t es = t.element_size();
+  const bool ok = (t.stride(4) == 1 || t.size(4) == 1) && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && t.stride(0) * es % 16 == 0 &&
+                  t.stride(1) * es % 16 == 0 && t.stride(2) * es % 16 == 0 && t.stride(3) * es % 16 == 0;
+  return ok ? t : t.clone(at::MemoryFormat::Contiguous);
+}
+
 castle_tensor_t rect(castle_tensor_t t, int64_t es, int64_t b, int64_t h) {
   t.ptr = static_cast<char*>(t.ptr) + (b * t.stride_b + h * t.stride_h) * es;
   return t;
@@ -341,32 +349,86 @@ Tensor run_backward(const Problem& p, const castle_tensor_t* in, const Tensor& o
   return result;
 }
 
-// Gradient node of both operators: one packed input, or six in the operator's order qc, kc, vc, qu, ku, vu.
-struct CastleBackward : public Node {
+// A tensor that went through saved-tensor hooks: whatever they gave back must be the tensor that was saved, since the
+// kernels get its address.  Its strides may be others (save_on_cpu gives contiguous ones).
+Tensor restored(const Tensor& t, at::IntArrayRef sizes, at::ScalarType dtype, const at::Device& dev) {
+  if (!t.defined() || t.sizes() != sizes || t.scalar_type() != dtype || t.device() != dev || t.layout() != at::kStrided)
+    throw std::runtime_error("castle_attention: a saved tensor came back from its hooks with another shape, type or device");
+  return t;
+}
+Tensor restored_contiguous(const Tensor& t, at::IntArrayRef sizes, at::ScalarType dtype, const at::Device& dev) {
+  restored(t, sizes, dtype, dev);
+  return t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
+}
+
+// What the core's backward needs of its forward.  Unpacking may run a user's hooks (checkpointing runs the whole forward
+// again there), so it comes before anything that changes the thread's dispatch or gradient mode.
+struct SavedCore {
   Problem p;
   Options o;
-  bool packed = false;
-  std::vector<SavedVariable> inputs;
-  SavedVariable out16, lse, w_state;
+  std::vector<SavedVariable> inputs;   // one packed tensor, or six
+  SavedVariable out16, lse, w_state, freqs;
   bool out_is_output = false;
+
+  struct Unpacked { std::vector<Tensor> inputs; Tensor out16, lse, w_state, freqs; };
+
+  // After set_history() of the node's output; `output`: out16 is that output.
+  void save(const Problem& problem, const Options& options, const Result& r, bool output) {
+    p = problem;
+    o = options;
+    o.caches.clear();
+    freqs = SavedVariable(o.rotary.freqs, false);
+    for (const auto& t : r.in.keep) inputs.emplace_back(t, false);
+    out_is_output = output;
+    out16 = SavedVariable(r.out16, output);
+    lse = SavedVariable(r.lse, false);
+    w_state = SavedVariable(r.w_state, false);
+  }
+  void reset() {
+    for (auto& v : inputs) v.reset_data();
+    out16.reset_data(); lse.reset_data(); w_state.reset_data(); freqs.reset_data();
+  }
+  Unpacked unpack(const std::shared_ptr<Node>& self) const {
+    Unpacked u;
+    for (const auto& v : inputs) u.inputs.push_back(v.unpack());
+    u.out16 = out_is_output ? out16.unpack(self) : out16.unpack();
+    u.lse = lse.unpack(); u.w_state = w_state.unpack(); u.freqs = freqs.unpack();
+    return u;
+  }
+  Tensor backward(const Unpacked& u, const Tensor& grad) const {
+    const at::Device dev = grad.device();
+    const std::vector<int64_t> bhnd{p.B, p.H, p.N, p.dp};
+    Options now = o;
+    if (o.rotary.on()) now.rotary.freqs = restored_contiguous(u.freqs, o.rotary.freqs.sizes(), o.rotary.freqs.scalar_type(), dev);
+    castle_tensor_t in[6];
+    std::vector<Tensor> keep;
+    for (const auto& t : u.inputs) {
+      if (u.inputs.size() == 1) keep.push_back(aligned_packed(restored(t, {p.B, p.N, 6, p.H, p.dp}, p.cdtype, dev)));
+      else keep.push_back(aligned_view(restored(t, bhnd, p.cdtype, dev)));
+    }
+    for (int i = 0; i < 6; ++i) in[i] = keep.size() == 1 ? packed_desc(keep[0], i) : desc(keep[i]);
+    return run_backward(p, in, aligned_view(restored(u.out16, bhnd, p.cdtype, dev)), restored_contiguous(u.lse, {p.B, p.H, p.N}, at::kFloat, dev),
+                        restored_contiguous(u.w_state, bhnd, at::kFloat, dev), grad, now);
+  }
+};
+
+// Gradient node of both operators: one packed input, or six in the operator's order qc, kc, vc, qu, ku, vu.
+struct CastleBackward : public Node {
+  SavedCore core;
+  bool packed = false;
 
   std::string name() const override { return "CastleAttentionBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    for (auto& v : inputs) v.reset_data();
-    out16.reset_data(); lse.reset_data(); w_state.reset_data();
+    core.reset();
   }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
     variable_list result(packed ? 1 : 6);
     if (grads.empty() || !grads[0].defined()) return result;
+    const SavedCore::Unpacked saved = core.unpack(shared_from_this());
     at::NoGradGuard no_grad;
-    castle_tensor_t in[6];
-    std::vector<Tensor> keep;
-    for (auto& v : inputs) keep.push_back(v.unpack());
-    for (int i = 0; i < 6; ++i) in[i] = keep.size() == 1 ? packed_desc(keep[0], i) : desc(keep[i]);
-    const Tensor out = out_is_output ? out16.unpack(shared_from_this()) : out16.unpack();
-    Tensor g = run_backward(p, in, out, lse.unpack(), w_state.unpack(), grads[0], o);
+    Tensor g = core.backward(saved, grads[0]);
     if (packed) {
       result[0] = std::move(g);
     } else {
@@ -390,16 +452,9 @@ Result attention(const Problem& p, Inputs in, Options o, const std::vector<Tenso
   if (!o.need_grad) return r;
   auto node = std::shared_ptr<CastleBackward>(new CastleBackward(), torch::autograd::deleteNode);
   node->set_next_edges(torch::autograd::collect_next_edges(vars));
-  node->p = p;
-  o.caches.clear();
-  node->o = o;
   node->packed = vars.size() == 1;
   torch::autograd::set_history(r.out, node);
-  for (const auto& t : r.in.keep) node->inputs.emplace_back(t, false);
-  node->out_is_output = r.out.is_same(r.out16);
-  node->out16 = SavedVariable(r.out16, node->out_is_output);
-  node->lse = SavedVariable(r.lse, false);
-  node->w_state = SavedVariable(r.w_state, false);
+  node->core.save(p, o, r, r.out.is_same(r.out16));
   return r;
 }
 
@@ -429,12 +484,10 @@ Result attention_packed(const Tensor& packed, const Options& o) {   // (B, N, 6,
   need(packed.dim() == 5 && packed.size(2) == 6, "castle_attention_packed: a (B, N, 6, H, d) tensor expected");
   const int64_t B = packed.size(0), N = packed.size(1), H = packed.size(3), d = packed.size(4);
   const Problem p = make_problem({B, H, N, d}, packed.scalar_type(), o.long_seq);
-  Tensor t = packed;
-  const int64_t es = t.element_size();
-  if (!(t.stride(4) == 1 || d == 1) || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 || t.stride(0) * es % 16 ||
-      t.stride(1) * es % 16 || t.stride(2) * es % 16 || t.stride(3) * es % 16) {
+  Tensor t;
+  {
     at::NoGradGuard no_grad;
-    t = t.clone(at::MemoryFormat::Contiguous);
+    t = aligned_packed(packed);
   }
   Inputs in;
   for (int i = 0; i < 6; ++i) in.t[i] = packed_desc(t, i);
@@ -527,20 +580,22 @@ Tensor matmul_t(const Tensor& x, const Tensor& w) { return at::mm(x, w.t()); }
 // Gradient node of a whole layer.  Autograd over the single operations (norm, two linear layers, the views between them
 // and the core) cost 250 us of host time per training step where the kernels of a small one take 120.
 struct LayerBackward : public Node {
-  Problem p;
-  Options o;
   int64_t dim = 0;
-  bool has_norm = false;
-  SavedVariable x, to_qkv, combine, norm;   // inputs, in the order of the node's outputs
-  Tensor h, rstd, out16, lse, w_state, merged;
-  Inputs in;
+  bool has_norm = false, separate_h = false, separate_merged = false;
+  at::ScalarType dtype = at::kFloat;
+  std::vector<int64_t> x_sizes;
+  // Like autograd over the single operations would, each kept only where a gradient that was asked for needs it, and
+  // nothing is kept beside them: a hook (checkpointing, save_on_cpu) sees all of it.
+  SavedCore core;
+  SavedVariable x, to_qkv, combine, norm, rstd;
+  SavedVariable h;        // the projection's input, unless that is x
+  SavedVariable merged;   // the output projection's input, unless that is the core's output
 
   std::string name() const override { return "CastleLayerBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    x.reset_data(); to_qkv.reset_data(); combine.reset_data(); norm.reset_data();
-    h = rstd = out16 = lse = w_state = merged = Tensor();
-    in.keep.clear();
+    core.reset();
+    for (SavedVariable* v : {&x, &to_qkv, &combine, &norm, &rstd, &h, &merged}) v->reset_data();
   }
   variable_list apply(variable_list&& grads) override {
     std::lock_guard<std::mutex> lock(mutex_);
@@ -548,29 +603,41 @@ struct LayerBackward : public Node {
     if (grads.empty() || !grads[0].defined()) return result;
     const bool need_x = task_should_compute_output(0), need_qkv = task_should_compute_output(1), need_combine = task_should_compute_output(2),
                need_norm = has_norm && task_should_compute_output(3);
-    const Tensor xs = x.unpack(), wq = to_qkv.unpack(), wc = combine.unpack();   // (raises on a second backward)
-    at::AutoDispatchBelowADInplaceOrView below;
-    const c10::cuda::CUDAGuard guard(xs.device());
-    const auto stream = c10::cuda::getCurrentCUDAStream(xs.device().index());
+    const bool need_core = need_x || need_qkv || need_norm, need_out = need_combine && !separate_merged;
+    const Problem& p = core.p;
     const int64_t rows = p.B * p.N, inner = p.H * p.d;
-    const Tensor g = grads[0].reshape({rows, wc.size(0)});
-    if (need_combine) result[2] = at::mm(g.t(), merged);
-    if (!(need_x || need_qkv || need_norm)) return result;
+    const at::Device dev = grads[0].device();
+    SavedCore::Unpacked saved;   // (unpacking raises on a second backward)
+    if (need_core) saved = core.unpack(shared_from_this());
+    else if (need_out) saved.out16 = core.out16.unpack();
+    const Tensor wc = need_core ? combine.unpack() : Tensor(), wq = need_x || need_norm ? to_qkv.unpack() : Tensor(),
+                 xs = (need_qkv && !separate_h) || (has_norm && (need_x || need_norm)) ? x.unpack() : Tensor(),
+                 hs = need_qkv && separate_h ? h.unpack() : Tensor(), ms = need_combine && separate_merged ? merged.unpack() : Tensor(),
+                 ws_norm = has_norm && (need_x || need_norm) ? norm.unpack() : Tensor(),
+                 rs_norm = has_norm && (need_x || need_norm) ? rstd.unpack() : Tensor();
+    at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard guard(dev);
+    const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
+    const Tensor g = grads[0].reshape({rows, grads[0].size(-1)});
+    if (need_combine)
+      result[2] = at::mm(g.t(), separate_merged ? ms : restored(saved.out16, {p.B, p.H, p.N, p.dp}, p.cdtype, dev).permute({0, 2, 1, 3}).reshape({rows, inner}));
+    if (!need_core) return result;
     const Tensor dcore = at::mm(g, wc).view({p.B, p.N, p.H, p.d}).permute({0, 2, 1, 3});
-    const Tensor dqkv = run_backward(p, in.t, out16, lse, w_state, dcore, o).view({rows, 6 * inner});
-    if (need_qkv) result[1] = at::mm(dqkv.t(), h);
+    const Tensor dqkv = core.backward(saved, dcore).view({rows, 6 * inner});
+    if (need_qkv) result[1] = at::mm(dqkv.t(), separate_h ? hs : xs.reshape({rows, dim}));
     if (!(need_x || need_norm)) return result;
     Tensor dh = at::mm(dqkv, wq);
     if (!has_norm) {
-      result[0] = dh.view(xs.sizes());
+      result[0] = dh.view(x_sizes);
       return result;
     }
-    const Tensor xc = xs.contiguous(), wn = norm.unpack();
-    if (need_x) result[0] = at::empty(xs.sizes(), dh.options());
+    const Tensor xc = restored_contiguous(xs, x_sizes, dtype, dev), wn = restored_contiguous(ws_norm, {dim}, dtype, dev),
+                 rs = restored_contiguous(rs_norm, {rows}, at::kFloat, dev);
+    if (need_x) result[0] = at::empty(x_sizes, dh.options());
     if (need_norm) result[3] = at::empty({dim}, dh.options());
     const size_t bytes = api.rmsnorm_bwd_workspace_bytes(rows, (int32_t)dim);
     const Tensor ws = scratch(stream, bytes);
-    check(api.rmsnorm_bwd(dtype_code(p.dtype), rows, (int32_t)dim, dh.data_ptr(), xc.data_ptr(), wn.data_ptr(), rstd.data_ptr<float>(),
+    check(api.rmsnorm_bwd(dtype_code(dtype), rows, (int32_t)dim, dh.data_ptr(), xc.data_ptr(), wn.data_ptr(), rs.data_ptr<float>(),
                           need_x ? result[0].data_ptr() : nullptr, need_norm ? result[3].data_ptr() : nullptr, ws.data_ptr(), ws.numel(),
                           stream.stream()), "castle_rmsnorm_bwd");
     return result;
@@ -579,9 +646,10 @@ struct LayerBackward : public Node {
 
 // Norm, projection, core and output projection, for plain_layer().
 Tensor layer_native(const Tensor& x, const Layer& l, Options o) {
-  const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || l.to_qkv.requires_grad() || l.combine.requires_grad() ||
-                                                   (l.norm.defined() && l.norm.requires_grad()));
-  o.need_grad = grad && (x.requires_grad() || l.to_qkv.requires_grad() || (l.norm.defined() && l.norm.requires_grad()));
+  const bool grad = at::GradMode::is_enabled(), has_norm = l.norm.defined();
+  const bool need_x = grad && x.requires_grad(), need_qkv = grad && l.to_qkv.requires_grad(), need_combine = grad && l.combine.requires_grad(),
+             need_norm = grad && has_norm && l.norm.requires_grad();
+  o.need_grad = need_x || need_qkv || need_norm;
   const int64_t B = x.size(0), N = x.size(1), dim = x.size(2), rows = B * N, inner = l.heads * l.dim_head;
   const Problem p = make_problem({B, l.heads, N, l.dim_head}, x.scalar_type(), o.long_seq);
   Tensor out, h, rstd, merged;
@@ -591,7 +659,7 @@ Tensor layer_native(const Tensor& x, const Layer& l, Options o) {
     const c10::cuda::CUDAGuard guard(x.device());
     const auto stream = c10::cuda::getCurrentCUDAStream(x.device().index());
     h = x.contiguous().view({rows, dim});
-    if (l.norm.defined()) {
+    if (has_norm) {
       const Tensor src = h;
       h = at::empty({rows, dim}, x.options().requires_grad(false));
       if (o.need_grad) rstd = at::empty({rows}, x.options().dtype(at::kFloat).requires_grad(false));
@@ -606,24 +674,33 @@ Tensor layer_native(const Tensor& x, const Layer& l, Options o) {
     merged = r.out.permute({0, 2, 1, 3}).view({rows, inner});
     out = matmul_t(merged, l.combine).view({B, N, l.combine.size(0)});
   }
-  if (!grad) return out;
+  if (!(o.need_grad || need_combine)) return out;
   auto node = std::shared_ptr<LayerBackward>(new LayerBackward(), torch::autograd::deleteNode);
   std::vector<Tensor> vars{x, l.to_qkv, l.combine};
-  if (l.norm.defined()) vars.push_back(l.norm);
+  if (has_norm) vars.push_back(l.norm);
   node->set_next_edges(torch::autograd::collect_next_edges(vars));
-  node->p = p;
-  o.caches.clear();
-  node->o = o;
   node->dim = dim;
-  node->has_norm = l.norm.defined();
+  node->has_norm = has_norm;
+  node->dtype = p.dtype;
+  node->x_sizes = x.sizes().vec();
   torch::autograd::set_history(out, node);
-  node->x = SavedVariable(x, false);
-  node->to_qkv = SavedVariable(l.to_qkv, false);
-  node->combine = SavedVariable(l.combine, false);
-  if (l.norm.defined()) node->norm = SavedVariable(l.norm, false);
-  node->h = h; node->rstd = rstd; node->merged = merged;
-  node->in = std::move(r.in);
-  node->out16 = r.out16; node->lse = r.lse; node->w_state = r.w_state;
+  auto keep = [](const Tensor& t) { return SavedVariable(t, false); };
+  if (o.need_grad) {
+    node->core.save(p, o, r, false);
+    node->combine = keep(l.combine);
+  } else {
+    node->core.p = p;
+  }
+  node->separate_merged = need_combine && !(o.need_grad && r.out.is_same(r.out16));
+  if (node->separate_merged) node->merged = keep(merged);
+  node->separate_h = need_qkv && (has_norm || !x.is_contiguous());
+  if (node->separate_h) node->h = keep(h);
+  if ((need_qkv && !node->separate_h) || (has_norm && (need_x || need_norm))) node->x = keep(x);
+  if (need_x || need_norm) node->to_qkv = keep(l.to_qkv);
+  if (has_norm && (need_x || need_norm)) {
+    node->norm = keep(l.norm);
+    node->rstd = keep(rstd);
+  }
   return out;
 }
 

@@ -84,14 +84,36 @@ def test_operator_under_checkpoint_and_on_cpu(dtype, d, packed):
     _same([out.detach(), *torch.autograd.grad(out, [x], g)], plain)
 
 
-def test_an_exception_of_a_hook_keeps_its_type():
-    m, wanted, _ = _layer(torch.bfloat16, True, False, 64)
+def test_checkpoint_around_more_than_the_layer():
+    """The second forward runs inside the unpacking of the layer's tensors and has to record its own graph there."""
+    m, wanted, g = _layer(torch.bfloat16, True, False, 64)
+    first, last = (torch.nn.Linear(DIM, DIM, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    wanted = [*wanted, *first.parameters(), *last.parameters()]
 
-    class Refused(Exception):
-        pass
+    def f(x):
+        return last(torch.nn.functional.gelu(m(first(x))))
 
-    def pack(t):
-        raise Refused("no")
+    plain = _grads(f, wanted, g)
+    _same(_grads(lambda t: checkpoint(f, t, use_reentrant=False), wanted, g), plain)
 
-    with pytest.raises(Refused), torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
-        m(wanted[0])
+
+def test_hooks_that_change_a_tensor_are_refused():
+    m, wanted, g = _layer(torch.bfloat16, False, False, 64)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.half() if t.dtype == torch.bfloat16 else t):
+        out = m(wanted[0])
+    with pytest.raises(RuntimeError, match="saved tensor came back"):
+        torch.autograd.grad(out, wanted, g)
+
+
+def test_only_what_a_gradient_needs_is_guarded_against_changes():
+    """As with the single operations: a frozen projection's input may change after the forward."""
+    m, wanted, g = _layer(torch.bfloat16, False, False, 64)
+    x = wanted[0].detach().clone()
+    m.to_all_qkv.weight.requires_grad_(False)
+    h = x.clone().requires_grad_()
+    y = h * 1
+    out = m(y)
+    plain = torch.autograd.grad(m(h), [h, m.combine_heads.weight], g)
+    with torch.no_grad():
+        y.zero_()
+    _same(torch.autograd.grad(out, [h, m.combine_heads.weight], g), plain)
