@@ -73,31 +73,52 @@ void need(bool ok, const char* message) {
 // Scratch per (device, stream): kernels of one stream run in order, so its calls can share a buffer; two streams must
 // not.  Grown on demand, given back by release_workspaces().  `words` are zeroed counters that every kernel using them
 // leaves zeroed.  The containers are never destroyed (the CUDA context may be gone before static destructors run).
-struct StreamState { Tensor scratch, words; };
-std::mutex state_mutex;
-auto& stream_states = *new std::map<std::pair<int, void*>, StreamState>();
+//
+// Calls of several host threads on one stream (the autograd engine's among them) must not mix: what a call's launches
+// hand on through the scratch would be overwritten by a launch of another call in between.  A StreamUse is the stream's
+// turn: it holds the stream's lock from before the first launch that touches the scratch until after the last.  Nobody
+// waits for it (or for state_mutex) holding the interpreter lock, which a holder may need.
+struct StreamState {
+  std::recursive_mutex mutex;
+  Tensor scratch, words;
+};
+std::mutex state_mutex;   // of the maps alone
+auto& stream_states = *new std::map<std::pair<int, void*>, std::shared_ptr<StreamState>>();
 auto& status_words = *new std::map<int, Tensor>();
 
 constexpr int64_t kAmaxWords = 4;   // words [0, 4): castle_amax_scale; then the decode step's counters
 
-Tensor scratch(const c10::cuda::CUDAStream& s, size_t bytes) {
-  std::lock_guard<std::mutex> lock(state_mutex);
-  Tensor& t = stream_states[{(int)s.device_index(), (void*)s.stream()}].scratch;
-  if (!t.defined() || (size_t)t.numel() < bytes) {
-    t = Tensor();   // give the old buffer back before asking for the larger one
-    t = at::empty({(int64_t)std::max<size_t>(bytes, (size_t)1 << 20)},
-                  at::TensorOptions().dtype(at::kByte).device(at::kCUDA, s.device_index()));
+class StreamUse {
+ public:
+  explicit StreamUse(const c10::cuda::CUDAStream& s) : device(s.device_index()) {
+    {
+      std::lock_guard<std::mutex> lock(state_mutex);
+      auto& e = stream_states[{(int)device, (void*)s.stream()}];
+      if (!e) e = std::make_shared<StreamState>();
+      state = e;
+    }
+    turn = std::unique_lock<std::recursive_mutex>(state->mutex);
   }
-  return t;
-}
+  Tensor scratch(size_t bytes) {
+    Tensor& t = state->scratch;
+    if (!t.defined() || (size_t)t.numel() < bytes) {
+      t = Tensor();   // give the old buffer back before asking for the larger one
+      t = at::empty({(int64_t)std::max<size_t>(bytes, (size_t)1 << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, device));
+    }
+    return t;
+  }
+  Tensor zero_words(int64_t count) {
+    Tensor& t = state->words;
+    if (!t.defined() || t.numel() < kAmaxWords + count)
+      t = at::zeros({kAmaxWords + std::max<int64_t>(count, 1020)}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+    return t;
+  }
 
-Tensor zero_words(const c10::cuda::CUDAStream& s, int64_t count) {
-  std::lock_guard<std::mutex> lock(state_mutex);
-  Tensor& t = stream_states[{(int)s.device_index(), (void*)s.stream()}].words;
-  if (!t.defined() || t.numel() < kAmaxWords + count)
-    t = at::zeros({kAmaxWords + std::max<int64_t>(count, 1020)}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, s.device_index()));
-  return t;
-}
+ private:
+  c10::DeviceIndex device;
+  std::shared_ptr<StreamState> state;   // (release_workspaces() may drop it from the map meanwhile)
+  std::unique_lock<std::recursive_mutex> turn;
+};
 
 Tensor status_word(int device) {
   std::lock_guard<std::mutex> lock(state_mutex);
@@ -255,7 +276,8 @@ Result run_forward(const Problem& p, Inputs in, const Options& o, const at::Devi
   const int64_t per_pair = std::max<int64_t>((int64_t)api.fwd_workspace_bytes(&one), 1);
   int64_t most = 0;
   for_chunks(p.B, p.H, per_pair, o.limit, [&](int64_t b0, int64_t b1, int64_t h0, int64_t h1) { most = std::max(most, (b1 - b0) * (h1 - h0)); });
-  const Tensor ws = scratch(stream, (size_t)(most * per_pair));
+  StreamUse use(stream);
+  const Tensor ws = use.scratch((size_t)(most * per_pair));
   const castle_tensor_t out_d = desc(r.out16);
   for_chunks(p.B, p.H, per_pair, o.limit, [&](int64_t b0, int64_t b1, int64_t h0, int64_t h1) {
     castle_problem_t cp = one;
@@ -300,6 +322,7 @@ Tensor run_backward(const Problem& p, const castle_tensor_t* in, const Tensor& o
   const c10::cuda::CUDAGuard guard(dev);
   const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
   const auto ct = at::TensorOptions().dtype(p.cdtype).device(dev);
+  StreamUse use(stream);
   Tensor factor;   // [s, 1 / s]
   if (p.dtype != p.cdtype) {
     // fp16 operands for a caller with a wider exponent range: bring the upstream gradient to a fixed magnitude with a
@@ -307,7 +330,7 @@ Tensor run_backward(const Problem& p, const castle_tensor_t* in, const Tensor& o
     // underflow nor large ones overflow in fp16.  Everything stays on the device.
     if (!grad.is_non_overlapping_and_dense() || !aligned(grad)) grad = grad.clone(at::MemoryFormat::Contiguous);
     factor = at::empty({2}, ct.dtype(at::kFloat));
-    const Tensor words = zero_words(stream, 0);
+    const Tensor words = use.zero_words(0);
     check(api.amax_scale(dtype_code(p.dtype), grad.data_ptr(), grad.numel(), reinterpret_cast<uint32_t*>(words.data_ptr()),
                          factor.data_ptr<float>(), stream.stream()), "castle_amax_scale");
   }
@@ -333,7 +356,7 @@ Tensor run_backward(const Problem& p, const castle_tensor_t* in, const Tensor& o
     const int64_t asked = std::min<int64_t>(p.B * p.H, std::max<int64_t>(1, ((int64_t)8 << 30) / pair));
     bytes = std::max(bytes - (asked - 1) * pair, o.limit);
   }
-  const Tensor ws = scratch(stream, (size_t)bytes);
+  const Tensor ws = use.scratch((size_t)bytes);
   const castle_tensor_t od = desc(out16), gd = desc(grad);
   check(api.bwd(&cp, &in[3], &in[4], &in[5], &in[0], &in[1], &in[2], &od, &gd, lse.data_ptr<float>(), w_state.data_ptr<float>(),
                 &g[3], &g[4], &g[5], &g[0], &g[1], &g[2], ws.data_ptr(), ws.numel(), status_word(dev.index()).data_ptr<int32_t>(),
@@ -508,8 +531,8 @@ void check_caches(const Tensor* caches, int64_t B, int64_t H, int64_t d, at::Sca
 
 // `news` in the operator's order qc, kc, vc, qu, ku, vu; `caches` U, qu, kc, vc; `out` contiguous (B, H, 1, d).
 void launch_decode(const castle_problem_t& cp, const castle_tensor_t* news, const Tensor* caches, void* out, int64_t t, const Rotary& rotary,
-                   bool overlap, void* ws, size_t ws_bytes, const c10::cuda::CUDAStream& stream) {
-  const Tensor words = zero_words(stream, (int64_t)cp.batch * cp.heads), status = status_word(stream.device_index());
+                   bool overlap, void* ws, size_t ws_bytes, const c10::cuda::CUDAStream& stream, StreamUse& use) {
+  const Tensor words = use.zero_words((int64_t)cp.batch * cp.heads), status = status_word(stream.device_index());
   castle_tensor_t c[4];
   for (int i = 0; i < 4; ++i) c[i] = desc(caches[i]);
   const castle_tensor_t od{out, (int64_t)cp.heads * cp.dim_head, cp.dim_head, cp.dim_head};
@@ -528,8 +551,9 @@ Tensor decode_core(const castle_tensor_t* news, const Tensor* caches, int64_t B,
   check_caches(caches, B, H, d, dtype);
   Tensor out = at::empty({B, H, 1, d}, caches[0].options());
   const castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
-  const Tensor ws = scratch(stream, api.decode_workspace_bytes(&cp, (int32_t)t));
-  launch_decode(cp, news, caches, out.data_ptr(), t, rotary, false, ws.data_ptr(), ws.numel(), stream);
+  StreamUse use(stream);
+  const Tensor ws = use.scratch(api.decode_workspace_bytes(&cp, (int32_t)t));
+  launch_decode(cp, news, caches, out.data_ptr(), t, rotary, false, ws.data_ptr(), ws.numel(), stream, use);
   return out;
 }
 
@@ -636,7 +660,8 @@ struct LayerBackward : public Node {
     if (need_x) result[0] = at::empty(x_sizes, dh.options());
     if (need_norm) result[3] = at::empty({dim}, dh.options());
     const size_t bytes = api.rmsnorm_bwd_workspace_bytes(rows, (int32_t)dim);
-    const Tensor ws = scratch(stream, bytes);
+    StreamUse use(stream);
+    const Tensor ws = use.scratch(bytes);
     check(api.rmsnorm_bwd(dtype_code(dtype), rows, (int32_t)dim, dh.data_ptr(), xc.data_ptr(), wn.data_ptr(), rs.data_ptr<float>(),
                           need_x ? result[0].data_ptr() : nullptr, need_norm ? result[3].data_ptr() : nullptr, ws.data_ptr(), ws.numel(),
                           stream.stream()), "castle_rmsnorm_bwd");
@@ -747,15 +772,16 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   const castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
   const int64_t row = (B * inner * es + 255) / 256 * 256;
   const size_t part = (api.decode_workspace_bytes(&cp, (int32_t)t) + 255) / 256 * 256;
-  const Tensor ws = scratch(stream, part + 7 * row);
+  StreamUse use(stream);
+  const Tensor ws = use.scratch(part + 7 * row);
   char* packed = static_cast<char*>(ws.data_ptr()) + part;
   char* core = packed + 6 * row;
   Tensor keep;
   const Tensor xs = x.stride(2) == 1 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * es % 16 == 0 ? x : x.contiguous();
   // The step and the last projection are launched ahead (see the C ABI's `overlap`).  The buffers they fetch early must be
-  // in place before the first of the three launches: zero_words() and status_word() may launch a fill on first use.
+  // in place before the first of the three launches: the words and the status word may launch a fill on first use.
   const bool overlap = own_projection(cp.dtype, B, dim, 6 * inner, es);
-  zero_words(stream, B * H);
+  use.zero_words(B * H);
   status_word(dev.index());
   if (overlap) {
     check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)dim, (int32_t)(6 * inner), xs.data_ptr(), xs.stride(0),
@@ -775,14 +801,14 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   castle_tensor_t news[6];
   for (int i = 0; i < 6; ++i) news[i] = {packed + kPackedOrder[i] * inner * es, 6 * inner, d, 6 * inner};
   if (own_projection(cp.dtype, B, inner, l.combine.size(0), es)) {
-    launch_decode(cp, news, caches, core, t, rotary, overlap, ws.data_ptr(), part, stream);
+    launch_decode(cp, news, caches, core, t, rotary, overlap, ws.data_ptr(), part, stream, use);
     Tensor y = at::empty({B, 1, l.combine.size(0)}, x.options().requires_grad(false));
     check(api.token_linear(cp.dtype, (int32_t)B, (int32_t)inner, (int32_t)l.combine.size(0), core, inner, nullptr, 0.f,
                            l.combine.data_ptr(), y.data_ptr(), 1, stream.stream()), "castle_token_linear");
     return y;
   }
   const Tensor o = at::empty({B, inner}, x.options().requires_grad(false));
-  launch_decode(cp, news, caches, o.data_ptr(), t, rotary, overlap, ws.data_ptr(), part, stream);
+  launch_decode(cp, news, caches, o.data_ptr(), t, rotary, overlap, ws.data_ptr(), part, stream, use);
   return matmul_t(o, l.combine).view({B, 1, l.combine.size(0)});
 }
 
@@ -1023,21 +1049,35 @@ PyObject* py_first_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 PyObject* py_status_word(PyObject*, PyObject* device) {
-  return guarded([&] { return THPVariable_Wrap(status_word((int)arg_int(device))); });
+  return guarded([&] {
+    const int64_t index = arg_int(device);
+    Tensor t;
+    {
+      Unlocked u;
+      t = status_word((int)index);
+    }
+    return THPVariable_Wrap(t);
+  });
 }
 PyObject* py_status_devices(PyObject*, PyObject*) {
-  std::lock_guard<std::mutex> lock(state_mutex);
+  std::vector<int> devices;
+  {
+    Unlocked u;
+    std::lock_guard<std::mutex> lock(state_mutex);
+    for (const auto& kv : status_words) devices.push_back(kv.first);
+  }
   PyObject* list = PyList_New(0);
-  for (const auto& kv : status_words) {
-    PyObject* i = PyLong_FromLong(kv.first);
+  for (int d : devices) {
+    PyObject* i = PyLong_FromLong(d);
     PyList_Append(list, i);
     Py_DECREF(i);
   }
   return list;
 }
 PyObject* py_release_workspaces(PyObject*, PyObject*) {
-  std::map<std::pair<int, void*>, StreamState> old;
+  std::map<std::pair<int, void*>, std::shared_ptr<StreamState>> old;
   {
+    Unlocked u;
     std::lock_guard<std::mutex> lock(state_mutex);
     old.swap(stream_states);
   }
