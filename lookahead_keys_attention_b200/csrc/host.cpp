@@ -18,6 +18,7 @@
 #include <ATen/ATen.h>
 #include <ATen/autocast_mode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -78,9 +79,13 @@ void need(bool ok, const char* message) {
 // hand on through the scratch would be overwritten by a launch of another call in between.  A StreamUse is the stream's
 // turn: it holds the stream's lock from before the first launch that touches the scratch until after the last.  Nobody
 // waits for it (or for state_mutex) holding the interpreter lock, which a holder may need.
+//
+// What is captured into a CUDA graph gets scratch and words of its own (a fill of the words is a node of the graph): a
+// replay runs when it likes, beside eager work and other graphs that were captured on the same stream.
 struct StreamState {
   std::recursive_mutex mutex;
   Tensor scratch, words;
+  unsigned long long capture = 0;   // the capture that scratch and words belong to, 0 = none
 };
 std::mutex state_mutex;   // of the maps alone
 auto& stream_states = *new std::map<std::pair<int, void*>, std::shared_ptr<StreamState>>();
@@ -98,6 +103,14 @@ class StreamUse {
       state = e;
     }
     turn = std::unique_lock<std::recursive_mutex>(state->mutex);
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    if (cudaStreamGetCaptureInfo(s.stream(), &status, &capture) != cudaSuccess) (void)cudaGetLastError();   // (the launch will say why)
+    if (status != cudaStreamCaptureStatusActive) capture = 0;
+    if (capture != state->capture) {
+      state->scratch = state->words = Tensor();
+      state->capture = capture;
+    }
   }
   Tensor scratch(size_t bytes) {
     Tensor& t = state->scratch;
@@ -120,10 +133,24 @@ class StreamUse {
   std::unique_lock<std::recursive_mutex> turn;
 };
 
+// One word per device for all streams and graphs, so it is cleared outside of both: a fill on the caller's stream could
+// run after another stream's kernel has set a bit, and captured into a graph it would clear the word at each replay.
 Tensor status_word(int device) {
   std::lock_guard<std::mutex> lock(state_mutex);
   Tensor& t = status_words[device];
-  if (!t.defined()) t = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+  if (!t.defined()) {
+    const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+    const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);   // of another stream's capture
+    void* p = nullptr;
+    cudaStream_t side = nullptr;
+    C10_CUDA_CHECK(cudaMalloc(&p, sizeof(int32_t)));
+    C10_CUDA_CHECK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    C10_CUDA_CHECK(cudaMemsetAsync(p, 0, sizeof(int32_t), side));
+    C10_CUDA_CHECK(cudaStreamSynchronize(side));
+    C10_CUDA_CHECK(cudaStreamDestroy(side));
+    const c10::InferenceMode normal(false);   // check_status() clears it in any mode
+    t = at::from_blob(p, {1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));   // never given back
+  }
   return t;
 }
 
