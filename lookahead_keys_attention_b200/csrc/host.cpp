@@ -241,7 +241,7 @@ Problem make_problem(at::IntArrayRef bhnd, at::ScalarType dtype, int64_t long_se
 }
 
 // Rectangles of the (batch, head) grid that each need at most `limit` bytes of scratch: whole batch rows, or head
-// ranges of one row, so that per-pair buffers of a rectangle stay contiguous (ops.forward_chunks).
+// ranges of one row, so that per-pair buffers of a rectangle stay contiguous; as few as that takes, all about the same size.
 template <typename F>
 void for_chunks(int64_t B, int64_t H, int64_t per_pair, int64_t limit, F&& f) {
   const int64_t pairs = limit / std::max<int64_t>(per_pair, 1);
@@ -1063,6 +1063,20 @@ PyObject* py_decode_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// forward_chunks(B, H, bytes per pair, limit): the rectangles of a forward's launches as (b0, b1, h0, h1)
+PyObject* py_forward_chunks(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    arg_count(n, 4);
+    std::vector<std::array<int64_t, 4>> r;
+    for_chunks(arg_int(a[0]), arg_int(a[1]), arg_int(a[2]), arg_int(a[3]),
+               [&](int64_t b0, int64_t b1, int64_t h0, int64_t h1) { r.push_back({b0, b1, h0, h1}); });
+    PyObject* list = PyList_New((Py_ssize_t)r.size());
+    for (size_t i = 0; i < r.size(); ++i)
+      PyList_SET_ITEM(list, (Py_ssize_t)i, Py_BuildValue("(LLLL)", (long long)r[i][0], (long long)r[i][1], (long long)r[i][2], (long long)r[i][3]));
+    return list;
+  });
+}
+
 // first_rows(buffers, n): the buffers' [:, :, :n] views as a tuple
 PyObject* py_first_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
@@ -1136,6 +1150,7 @@ PyMethodDef methods[] = {{"bind", py_bind, METH_O, nullptr},
                          {"layer_forward", FAST(py_layer_forward), nullptr},
                          {"layer_decode", FAST(py_layer_decode), nullptr},
                          {"decode_packed", FAST(py_decode_packed), nullptr},
+                         {"forward_chunks", FAST(py_forward_chunks), nullptr},
                          {"first_rows", FAST(py_first_rows), nullptr},
                          {"status_word", py_status_word, METH_O, nullptr},
                          {"status_devices", py_status_devices, METH_NOARGS, nullptr},

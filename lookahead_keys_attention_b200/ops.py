@@ -58,23 +58,10 @@ MAX_WORKSPACE_BYTES = 16 << 30
 
 
 def forward_chunks(B: int, H: int, per_pair: int, limit: int | None = None):
-    """Rectangles (b0, b1, h0, h1) of the (batch, head) grid, each needing at most `limit` bytes of
-    scratch at `per_pair` bytes per pair.  A rectangle spans several batch rows only with all heads,
-    so that the per-pair fp32 buffers (lse, state) of a rectangle stay contiguous.  (csrc/host.cpp, for_chunks,
-    is the same rule where the launches are made.)"""
-    limit = MAX_WORKSPACE_BYTES if limit is None else limit
-    pairs = limit // max(per_pair, 1)
-    if pairs < 1:
-        raise RuntimeError(f"castle_attention: one (batch, head) pair needs {per_pair} bytes of forward scratch, "
-                           f"more than the {limit}-byte bound (sequence too long for this build)")
-    def even(total, most):   # cut `total` into the fewest pieces of at most `most`, all about the same size
-        n = -(-total // most)
-        size = -(-total // n)
-        return [(i, min(total, i + size)) for i in range(0, total, size)]
-
-    if pairs >= H:
-        return [(b0, b1, 0, H) for b0, b1 in even(B, min(B, pairs // H))]
-    return [(b, b + 1, h0, h1) for b in range(B) for h0, h1 in even(H, pairs)]
+    """Rectangles (b0, b1, h0, h1) of the (batch, head) grid that a forward is launched over, each needing at most
+    `limit` bytes of scratch at `per_pair` bytes per pair.  A rectangle spans several batch rows only with all heads,
+    so that the per-pair fp32 buffers (lse, state) of a rectangle stay contiguous.  (csrc/host.cpp, for_chunks.)"""
+    return _lib.host().forward_chunks(B, H, per_pair, MAX_WORKSPACE_BYTES if limit is None else limit)
 
 
 # From this sequence length on, bf16 callers are computed with fp16 operands.  The lookahead state W grows
