@@ -581,8 +581,13 @@ static int launch_decode_d(const DecodeParams& p, int BH, int D, bool ring, cuda
 
 using namespace castle;
 
+// The (batch, head) pairs are the grid's first dimension.
+static bool decode_pairs_ok(const castle_problem_t* p) {
+  return p->batch > 0 && p->heads > 0 && (int64_t)p->batch * p->heads <= 2147483647LL;
+}
+
 extern "C" size_t castle_decode_workspace_bytes(const castle_problem_t* p, int32_t cache_len) {
-  if (!p) return 0;
+  if (!p || !decode_pairs_ok(p)) return 0;
   int BH = p->batch * p->heads;
   int ns = decode_nsplit_fine(BH, cache_len, CASTLE_DECODE_MIN_CTAS), ns_ring = decode_nsplit_fine(BH, cache_len, kRingCtasPerSm);
   return (size_t)BH * (ns > ns_ring ? ns : ns_ring) * (2 + p->dim_head) * sizeof(float);
@@ -609,7 +614,7 @@ extern "C" int castle_decode_step_fused(const castle_problem_t* p, int32_t cache
                                         const castle_tensor_t* out, const castle_rotary_t* rotary, uint32_t* counters,
                                         int32_t overlap, void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
   if (!p) return reject("castle_decode_step: null problem");
-  if (p->batch <= 0 || p->heads <= 0) return reject("castle_decode_step: empty batch/heads");
+  if (!decode_pairs_ok(p)) return reject("castle_decode_step: empty batch/heads, or more than 2^31 pairs");
   if (cache_len < 0 || cache_len >= capacity)
     return reject("castle_decode_step: cache_len %d must be in [0, capacity %d)", cache_len, capacity);
   if (p->dtype != CASTLE_BF16 && p->dtype != CASTLE_F16 && p->dtype != CASTLE_F32)
@@ -686,7 +691,7 @@ extern "C" int castle_decode_step_static(const castle_problem_t* p, int32_t cach
                                          const castle_tensor_t* kc_cache, const castle_tensor_t* vc_cache,
                                          const castle_tensor_t* out, int32_t* status, void* stream) {
   if (!p) return reject("castle_decode_step_static: null problem");
-  if (p->batch <= 0 || p->heads <= 0) return reject("castle_decode_step_static: empty batch/heads");
+  if (!decode_pairs_ok(p)) return reject("castle_decode_step_static: empty batch/heads, or more than 2^31 pairs");
   if (cache_len < 0 || cache_len >= capacity)
     return reject("castle_decode_step_static: cache_len %d must be in [0, capacity %d)", cache_len, capacity);
   if (p->dtype != CASTLE_BF16 && p->dtype != CASTLE_F16 && p->dtype != CASTLE_F32)

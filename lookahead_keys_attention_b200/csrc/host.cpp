@@ -244,6 +244,7 @@ Problem make_problem(at::IntArrayRef bhnd, at::ScalarType dtype, int64_t long_se
 // ranges of one row, so that per-pair buffers of a rectangle stay contiguous; as few as that takes, all about the same size.
 template <typename F>
 void for_chunks(int64_t B, int64_t H, int64_t per_pair, int64_t limit, F&& f) {
+  need(B > 0 && H > 0, "castle_attention: empty problem");
   const int64_t pairs = limit / std::max<int64_t>(per_pair, 1);
   if (pairs < 1)
     throw std::runtime_error("castle_attention: one (batch, head) pair needs " + std::to_string(per_pair) +

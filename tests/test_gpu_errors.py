@@ -53,3 +53,16 @@ def test_out_of_memory_keeps_its_type():
             torch.cuda.set_per_process_memory_fraction(1.0)
         castle_attention_packed(x, 0.125)   # nothing is left half made
     check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("B,N", [(0, 40), (2, 0), (0, 1)])
+def test_empty_tensors_are_refused(dtype, B, N):
+    from lookahead_keys_attention_b200 import Castle, castle_attention, castle_attention_packed
+    x = torch.zeros(B, 2, N, 64, device="cuda", dtype=dtype)
+    with pytest.raises(RuntimeError):
+        castle_attention(x, x, x, x, x, x, 0.125)
+    with pytest.raises(RuntimeError):
+        castle_attention_packed(torch.zeros(B, N, 6, 2, 64, device="cuda", dtype=dtype), 0.125)
+    with pytest.raises(RuntimeError):
+        Castle(32, heads=2).cuda().to(dtype)(torch.zeros(B, N, 32, device="cuda", dtype=dtype))

@@ -198,3 +198,20 @@ def test_rotary_offset_and_norm():
     assert torch.allclose(full.norm(dim=-1), t.norm(dim=-1), atol=1e-5)
     assert torch.allclose(r.rotate(t[:, :, 4:7], offset=4), full[:, :, 4:7], atol=1e-6)
     assert torch.allclose(r.rotate(t[:, :, :1]), t[:, :, :1], atol=1e-6)  # position 0 is the identity
+
+
+def test_empty_and_oversized_problems_are_refused_on_the_host():
+    """Not by a division by zero, which would end the process."""
+    from lookahead_keys_attention_b200.ops import forward_chunks
+    for B, H in [(0, 8), (3, 0)]:
+        with pytest.raises(RuntimeError, match="empty"):
+            forward_chunks(B, H, 10, 1000)
+    L = _lib()
+    lib = L.load()
+    t = L.CastleTensor(16, 0, 0, 64)
+    args = [ctypes.byref(t)] * 11
+    for B, H in [(0, 8), (3, 0), (65536, 65536)]:
+        prob = L.CastleProblem(B, H, 1, 64, L.BF16, 0.125)
+        assert lib.castle_decode_workspace_bytes(ctypes.byref(prob), 100) == 0
+        assert lib.castle_decode_step(ctypes.byref(prob), 100, 200, *args, None, 0, None, None) < 0
+        assert lib.castle_decode_step_static(ctypes.byref(prob), 100, 200, *args, None, None) < 0
