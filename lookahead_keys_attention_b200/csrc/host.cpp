@@ -202,6 +202,18 @@ struct Rotary {
   castle_rotary_t desc(bool inverse) const {
     return {freqs.data_ptr(), dtype_code(freqs.scalar_type()), inverse ? 1 : 0, position0};
   }
+  // The kernels read dim_head / 2 values at the frequencies' address: a buffer that was left on the CPU or replaced is
+  // brought to where and how they expect it, as the element-wise form does, or refused.
+  void fit(const at::Device& dev, int64_t dim_head) {
+    if (!on()) return;
+    const int64_t count = freqs.numel();
+    if (count != 1 && (2 * count != dim_head || freqs.size(-1) != count))
+      throw std::runtime_error("castle: rotary frequencies must be (dim_head / 2) = " + std::to_string(dim_head / 2) + " values, or one");
+    const bool type_ok = dtype_code(freqs.scalar_type()) >= 0;
+    if (freqs.device() == dev && freqs.is_contiguous() && type_ok && 2 * count == dim_head) return;
+    at::NoGradGuard no_grad;
+    freqs = freqs.to(dev, type_ok ? freqs.scalar_type() : at::kFloat).reshape({count}).expand({dim_head / 2}).contiguous();
+  }
 };
 constexpr int kPackedOrder[6] = {3, 4, 5, 0, 1, 2};   // between the operator's order qc, kc, vc, qu, ku, vu and the packed one, both ways
 constexpr uint32_t kRotated = 0x1f;   // of qu, ku, vu, qc, kc, vc all but vc
@@ -530,11 +542,12 @@ Result attention_six(const Tensor* v /* qc, kc, vc, qu, ku, vu */, const Options
   return attention(p, std::move(in), o, std::vector<Tensor>(v, v + 6));
 }
 
-Result attention_packed(const Tensor& packed, const Options& o) {   // (B, N, 6, H, d), order qu, ku, vu, qc, kc, vc
+Result attention_packed(const Tensor& packed, Options o) {   // (B, N, 6, H, d), order qu, ku, vu, qc, kc, vc
   need(packed.is_cuda(), "castle_attention: expected CUDA tensors; this package has no CPU path");
   need(packed.dim() == 5 && packed.size(2) == 6, "castle_attention_packed: a (B, N, 6, H, d) tensor expected");
   const int64_t B = packed.size(0), N = packed.size(1), H = packed.size(3), d = packed.size(4);
   const Problem p = make_problem({B, H, N, d}, packed.scalar_type(), o.long_seq);
+  o.rotary.fit(packed.device(), d);
   Tensor t;
   {
     at::NoGradGuard no_grad;
@@ -573,8 +586,9 @@ void launch_decode(const castle_problem_t& cp, const castle_tensor_t* news, cons
 }
 
 Tensor decode_core(const castle_tensor_t* news, const Tensor* caches, int64_t B, int64_t H, int64_t d, at::ScalarType dtype,
-                   int64_t t, double scale, const Rotary& rotary, const at::Device& dev) {
+                   int64_t t, double scale, Rotary rotary, const at::Device& dev) {
   const c10::cuda::CUDAGuard guard(dev);
+  rotary.fit(dev, d);
   const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
   check_caches(caches, B, H, d, dtype);
   Tensor out = at::empty({B, H, 1, d}, caches[0].options());
@@ -705,6 +719,7 @@ Tensor layer_native(const Tensor& x, const Layer& l, Options o) {
   o.need_grad = need_x || need_qkv || need_norm;
   const int64_t B = x.size(0), N = x.size(1), dim = x.size(2), rows = B * N, inner = l.heads * l.dim_head;
   const Problem p = make_problem({B, l.heads, N, l.dim_head}, x.scalar_type(), o.long_seq);
+  o.rotary.fit(x.device(), l.dim_head);
   Tensor out, h, rstd, merged;
   Result r;
   {
@@ -789,9 +804,10 @@ bool own_projection(int dtype, int64_t rows, int64_t k, int64_t n, int64_t es) {
 
 // Norm, projection, step and output projection of one token, with what passes between them in the stream's scratch: on
 // the host the allocations would cost as much as the launches.
-Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_t t, double scale, const Rotary& rotary) {
+Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_t t, double scale, Rotary rotary) {
   const at::Device dev = x.device();
   const c10::cuda::CUDAGuard guard(dev);
+  rotary.fit(dev, l.dim_head);
   at::AutoDispatchBelowADInplaceOrView below;
   const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
   const auto dtype = x.scalar_type();
