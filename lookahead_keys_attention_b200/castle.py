@@ -156,12 +156,15 @@ class Castle(nn.Module):
             if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks:
                 return None
         wq, wc = qkv._parameters, combine._parameters
-        if wq["bias"] is not None or wc["bias"] is not None:
+        if wq.get("bias") is not None or wc.get("bias") is not None:
+            return None
+        weights = wq.get("weight"), wc.get("weight")   # a data-parallel replica holds them as plain attributes
+        if weights[0] is None or weights[1] is None:
             return None
         if type(norm) is nn.Identity:
-            return None, None, wq["weight"], wc["weight"], self.heads, self.dim_head
-        if type(norm) is nn.RMSNorm and norm._parameters["weight"] is not None and len(norm.normalized_shape) == 1:
-            return norm._parameters["weight"], norm.eps, wq["weight"], wc["weight"], self.heads, self.dim_head
+            return None, None, *weights, self.heads, self.dim_head
+        if type(norm) is nn.RMSNorm and norm._parameters.get("weight") is not None and len(norm.normalized_shape) == 1:
+            return norm._parameters["weight"], norm.eps, *weights, self.heads, self.dim_head
         return None
 
     def _project(self, x):

@@ -215,3 +215,21 @@ def test_empty_and_oversized_problems_are_refused_on_the_host():
         assert lib.castle_decode_workspace_bytes(ctypes.byref(prob), 100) == 0
         assert lib.castle_decode_step(ctypes.byref(prob), 100, 200, *args, None, 0, None, None) < 0
         assert lib.castle_decode_step_static(ctypes.byref(prob), 100, 200, *args, None, None) < 0
+
+
+def test_replica_without_parameters_is_called_through_its_submodules():
+    """torch.nn.parallel.replicate leaves a replica's weights as plain attributes."""
+    from lookahead_keys_attention_b200 import Castle
+    m = Castle(32, heads=2, dim_head=16, prenorm=True)
+    replica = m._replicate_for_data_parallel()
+    for name, child in m._modules.items():
+        copy = None if child is None else child._replicate_for_data_parallel()
+        replica._modules[name] = copy
+        for key, p in (child._parameters.items() if child is not None else ()):
+            if p is None:
+                copy._parameters[key] = None
+            else:
+                setattr(copy, key, p.detach().clone())
+    assert m._plain_layer() is not None and replica._plain_layer() is None
+    x = torch.randn(1, 5, 32)
+    assert torch.equal(replica._project(x), m._project(x))
