@@ -171,6 +171,29 @@ class Castle(nn.Module):
         """The packed projection (b, n, 6, heads, dim_head) with the submodules called as modules."""
         return self.to_all_qkv(self.norm(x)).view(x.shape[0], x.shape[1], 6, self.heads, self.dim_head)
 
+    def _merge(self, out):
+        return self.combine_heads(out.permute(0, 2, 1, 3).flatten(2))   # 'b h n d -> b n (h d)'
+
+    def _forward_rotated(self, x, cache, return_next_cache):
+        """With a rotary embedding of the caller's own (a subclass, or another object with `rotate(t, offset)`) in
+        the place of `_Rotary`: rotated by it, then the operators."""
+        seq_len = x.shape[1]
+        qu, ku, vu, qc, kc, vc = self._split(self.to_all_qkv(self.norm(x)))
+        t = cache[0].shape[-2] if cache is not None else 0
+        qc, kc, qu, ku, vu = (self.rotary_emb.rotate(v, t) for v in (qc, kc, qu, ku, vu))
+        if seq_len == 1:
+            with torch.no_grad():
+                state = self._buffers_for_step(cache, t, qu)
+                out = ops.castle_decode_step(qc, kc, vc, qu, ku, vu, *state.bufs, t, self.scale)
+            state.length = t + 1
+            return (self._merge(out), ModuleCache(state, t + 1)) if return_next_cache else self._merge(out)
+        assert cache is None, "must be inferencing single tokens if receiving cache"
+        if not return_next_cache:
+            return self._merge(ops.castle_attention(qc, kc, vc, qu, ku, vu, self.scale))
+        out, U = ops.castle_attention(qc, kc, vc, qu, ku, vu, self.scale, True)
+        state = self._buffers_for_step((U, qu, kc, vc), seq_len, qu)
+        return self._merge(out), ModuleCache(state, seq_len)
+
     def forward(self, x, cache: Cache | None = None, return_next_cache=None):
         host = _lib.host()
         seq_len = x.shape[1]
@@ -178,8 +201,11 @@ class Castle(nn.Module):
         if return_next_cache is None:
             return_next_cache = is_inference
         layer = self._plain_layer()
-        rotary = self.rotary_emb
-        freqs = None if rotary is None else rotary._buffers["freqs"]
+        rotary, freqs = self.rotary_emb, None
+        if rotary is not None:
+            if type(rotary) is not _Rotary or "rotate" in rotary.__dict__:
+                return self._forward_rotated(x, cache, return_next_cache)
+            freqs = rotary._buffers["freqs"]
 
         if is_inference:
             t = 0 if cache is None else cache._length if isinstance(cache, ModuleCache) else cache[0].shape[-2]
@@ -209,8 +235,7 @@ class Castle(nn.Module):
         if native:
             out = host.layer_forward(x, *layer, self.scale, freqs, views, *limits)
         else:
-            out = host.attention_packed(packed, self.scale, False, views, *limits, freqs, False)
-            out = self.combine_heads(out.permute(0, 2, 1, 3).reshape(*x.shape[:2], -1))   # 'b h n d -> b n (h d)'
+            out = self._merge(host.attention_packed(packed, self.scale, False, views, *limits, freqs, False))
         if not return_next_cache:
             return out
         state.length = seq_len

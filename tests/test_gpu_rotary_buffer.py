@@ -1,4 +1,5 @@
-"""GPU: the rotary frequencies wherever and however the module's buffer holds them."""
+"""GPU: the rotary frequencies wherever and however the module's buffer holds them, and rotary embeddings of the
+caller's own in the place of the module's."""
 import pytest
 import torch
 
@@ -43,3 +44,32 @@ def test_frequencies_of_another_shape_are_refused(freqs):
     for n in (1, 140):
         with torch.no_grad(), pytest.raises(RuntimeError, match="rotary frequencies"):
             m(torch.zeros(2, n, 96, device="cuda", dtype=torch.bfloat16))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_rotary_embedding_of_the_callers_own(dtype):
+    from lookahead_keys_attention_b200 import Castle
+    from lookahead_keys_attention_b200.castle import _Rotary
+    torch.manual_seed(0)
+    m = Castle(96, heads=2, dim_head=64, rotary_emb=True, prenorm=True).cuda().to(dtype)
+    x, g = (torch.randn(2, 140, 96, device="cuda").to(dtype) for _ in range(2))
+    want, want_grads = _run(m, x, g)
+
+    class Same(_Rotary):
+        def rotate(self, t, offset=0):
+            self.calls += 1
+            return super().rotate(t, offset)
+
+    own = Same(64).cuda().to(dtype)
+    own.calls = 0
+    m.rotary_emb = own
+    got, grads = _run(m, x, g)
+    assert own.calls == 10   # five tensors, prompt and step
+    tol = 2e-2 if dtype == torch.bfloat16 else 2e-3
+    for a, b in zip([*got, *grads], [*want, *want_grads]):
+        assert (a.float() - b.float()).norm() <= tol * b.float().norm()
+    m.rotary_emb.rotate = lambda t, offset=0: t      # and what it does is what counts
+    plain, _ = _run(m, x, g)
+    m.rotary_emb = None
+    for a, b in zip(plain, _run(m, x, g)[0]):
+        assert (a.float() - b.float()).norm() <= tol * b.float().norm()
