@@ -176,6 +176,11 @@ castle_tensor_t packed_desc(const Tensor& p, int i) {
   return {static_cast<char*>(p.data_ptr()) + i * p.stride(2) * p.element_size(), p.stride(0), p.stride(3), p.stride(1)};
 }
 
+// Contiguous at a 16-byte boundary (contiguous() leaves a view at an odd offset as it is).
+Tensor aligned_contiguous(const Tensor& t) {
+  return t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
+}
+
 // A packed (B, N, 6, H, d) tensor as the kernels take it: itself, or a copy.
 Tensor aligned_packed(const Tensor& t) {
   const int64_t es = t.element_size();
@@ -421,7 +426,7 @@ Tensor restored(const Tensor& t, at::IntArrayRef sizes, at::ScalarType dtype, co
 }
 Tensor restored_contiguous(const Tensor& t, at::IntArrayRef sizes, at::ScalarType dtype, const at::Device& dev) {
   restored(t, sizes, dtype, dev);
-  return t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
+  return aligned_contiguous(t);
 }
 
 // What the core's backward needs of its forward.  Unpacking may run a user's hooks (checkpointing runs the whole forward
@@ -728,7 +733,7 @@ Tensor layer_native(const Tensor& x, const Layer& l, Options o) {
     const auto stream = c10::cuda::getCurrentCUDAStream(x.device().index());
     h = x.contiguous().view({rows, dim});
     if (has_norm) {
-      const Tensor src = h;
+      const Tensor src = aligned_contiguous(h);
       h = at::empty({rows, dim}, x.options().requires_grad(false));
       if (o.need_grad) rstd = at::empty({rows}, x.options().dtype(at::kFloat).requires_grad(false));
       check(api.rmsnorm_fwd(dtype_code(p.dtype), rows, (int32_t)dim, src.data_ptr(), l.norm.data_ptr(), norm_eps(l), h.data_ptr(),
@@ -821,7 +826,7 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   char* packed = static_cast<char*>(ws.data_ptr()) + part;
   char* core = packed + 6 * row;
   Tensor keep;
-  const Tensor xs = x.stride(2) == 1 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * es % 16 == 0 ? x : x.contiguous();
+  const Tensor xs = x.stride(2) == 1 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * es % 16 == 0 ? x : aligned_contiguous(x);
   // The step and the last projection are launched ahead (see the C ABI's `overlap`).  The buffers they fetch early must be
   // in place before the first of the three launches: the words and the status word may launch a fill on first use.
   const bool overlap = own_projection(cp.dtype, B, dim, 6 * inner, es);
@@ -832,7 +837,7 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
                            l.norm.defined() ? l.norm.data_ptr() : nullptr, norm_eps(l), l.to_qkv.data_ptr(), packed, 0, stream.stream()),
           "castle_token_linear");
   } else {
-    Tensor h = xs.contiguous().view({B, dim});
+    Tensor h = aligned_contiguous(xs).view({B, dim});
     if (l.norm.defined()) {
       const Tensor src = h;
       h = at::empty({B, dim}, x.options().requires_grad(false));

@@ -71,3 +71,29 @@ def test_layer_backward_twice_and_inplace_change_raise():
         m.combine_heads.weight.mul_(2)
     with pytest.raises(RuntimeError, match="inplace"):
         out.sum().backward()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("prenorm", [False, True])
+@pytest.mark.parametrize("batch", [1, 3, 12])
+def test_input_at_an_odd_offset(dtype, prenorm, batch):
+    """A contiguous view that starts between 16-byte boundaries: prompt with gradients, and single tokens on each route."""
+    from lookahead_keys_attention_b200 import Castle
+    torch.manual_seed(batch)
+    m = Castle(96, heads=2, prenorm=prenorm).cuda().to(dtype)
+    g = torch.randn(batch, 40, 96, device="cuda").to(dtype)
+    flat = torch.randn(batch * 40 * 96 + 1, device="cuda").to(dtype)
+    token = torch.randn(batch * 96 + 1, device="cuda").to(dtype)
+
+    def go(x, t):
+        x = x.detach().requires_grad_()
+        out, cache = m(x, return_next_cache=True)
+        grads = torch.autograd.grad(out, [x, *m.parameters()], g)
+        with torch.no_grad():
+            step, _ = m(t, cache=cache)
+        return [out.detach(), step, *grads]
+
+    odd, even = (flat[1:].view(batch, 40, 96), token[1:].view(batch, 1, 96)), (flat[1:].clone().view(batch, 40, 96), token[1:].clone().view(batch, 1, 96))
+    assert odd[0].data_ptr() % 16 and odd[1].data_ptr() % 16 and odd[0].is_contiguous()
+    for a, b in zip(go(*odd), go(*even)):
+        assert (a.float() - b.float()).norm().item() <= 4e-3 * b.float().norm().item()
