@@ -112,7 +112,7 @@ int castle_convert_16bit(int32_t src_dtype, const void* src, void* dst, int64_t 
  * One pass over `count` (1 to 6) tensors of `p`'s shape, row width p->dim_head and type p->dtype: each row is
  * rotated (rotary may be NULL; bit i of rotary_mask = tensor i is rotated), stored as it is to copies[i] (NULL
  * array or null pointers: nowhere), multiplied by *mul (device pointer, may be NULL), converted to dst_dtype
- * (saturating where that is fp16 and the source is not) and stored to dst[i] (null pointer: nowhere) with rows
+ * (saturating where that is fp16 and the source is not; with a factor an infinity stays one) and stored to dst[i] (null pointer: nowhere) with rows
  * of dst_dim_head elements, cut or zero-padded.  Takes the place of the reference's rotary calls
  * (lookahead_keys_attention/lookahead_keys_attention.py:106-112), its `.half()` casts
  * (lookahead_keys_attention_triton.py:437-442, :523, :591-602) and the cache hand-off of callers whose type is
@@ -129,8 +129,8 @@ int castle_transform(const castle_problem_t* p, int32_t count, const castle_tens
                      int32_t dst_dtype, int32_t dst_dim_head, const castle_tensor_t* copies,
                      const castle_rotary_t* rotary, uint32_t rotary_mask, const float* mul, void* stream);
 
-/* The power of two that brings the largest |x| of `count` contiguous elements (a multiple of 8) to at most 64:
- * out[0] = it, out[1] = its reciprocal.  `state` = two words that are zero before the call; they are zero again
+/* The power of two that brings the largest finite |x| of `count` contiguous elements (a multiple of 8) to at most 64:
+ * out[0] = it (at most 2^24), out[1] = its reciprocal.  `state` = two words that are zero before the call; they are zero again
  * when its kernel has run, so calls on one stream can share them.
  */
 int castle_amax_scale(int32_t dtype, const void* x, int64_t count, uint32_t* state, float* out, void* stream);

@@ -68,30 +68,31 @@ __global__ void __launch_bounds__(kTransformThreads) castle_transform_kernel(con
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] *= mul;
       }
-      if (std::is_same<D, __half>::value && !std::is_same<S, __half>::value) {   // saturate instead of overflowing
+      // Saturate instead of overflowing.  With a factor the values are an upstream gradient's, which castle_amax_scale has
+      // brought into range: an infinity there is the caller's own and stays one, as loss scalers look for it.
+      if (std::is_same<D, __half>::value && !std::is_same<S, __half>::value) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = v[j] != v[j] ? v[j] : fminf(fmaxf(v[j], -65504.f), 65504.f);
+        for (int j = 0; j < 8; ++j) v[j] = v[j] != v[j] || (p.mul && fabsf(v[j]) == INFINITY) ? v[j] : fminf(fmaxf(v[j], -65504.f), 65504.f);
       }
       store8<D>(reinterpret_cast<D*>(d.ptr) + b * d.stride_b + h * d.stride_h + (int64_t)n * d.stride_n + c8, v);
     }
   }
 }
 
-// The largest |x| of a tensor and from it the power of two that brings a gradient to a fixed magnitude:
-// out[0] = s = 2^e, the largest power of two <= 64 / max (e within +-24), out[1] = 1 / s.  `state` is two zeroed
-// words (running maximum as bits of a non-negative float, blocks done) that the last block zeroes again.
+// The largest finite |x| of a tensor and from it the power of two that brings a gradient to a fixed magnitude:
+// out[0] = s = 2^e, the largest power of two <= 64 / max (e at most 24, so that zeros stay harmless), out[1] = 1 / s.
+// Infinities and NaN have no part in it: one of them leaves the other rows' gradients as they are without it.  `state` is
+// two zeroed words (running maximum as bits of a non-negative float, blocks done) that the last block zeroes again.
 template <typename S>
 __global__ void __launch_bounds__(256) castle_amax_scale_kernel(const S* __restrict__ x, int64_t n8, uint32_t* state, float* out) {
   float m = 0.f;
-  bool nan = false;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n8; i += (int64_t)gridDim.x * 256) {
     float v[8];
     load8<S>(x + i * 8, v);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { m = fmaxf(m, fabsf(v[j])); nan |= v[j] != v[j]; }
+    for (int j = 0; j < 8; ++j) m = fabsf(v[j]) < INFINITY ? fmaxf(m, fabsf(v[j])) : m;
   }
-  uint32_t bits = nan ? 0x7fffffffu : __float_as_uint(m);
-  bits = __reduce_max_sync(0xffffffffu, bits);
+  uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
   __shared__ uint32_t warp_bits[8];
   if ((threadIdx.x & 31) == 0) warp_bits[threadIdx.x >> 5] = bits;
   __syncthreads();
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(256) castle_amax_scale_kernel(const S* __restr
       state[1] = 0u;
       int e;
       frexpf(64.f / amax, &e);
-      e = min(max(e - 1, -24), 24);
+      e = min(e - 1, 24);
       out[0] = ldexpf(1.f, e);
       out[1] = ldexpf(1.f, -e);
     }

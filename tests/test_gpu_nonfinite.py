@@ -49,3 +49,37 @@ def test_exp2_of_the_score_passes():
     assert torch.equal(y[12:12 + whole.numel()], torch.exp2(whole.double()).float())
     ref = torch.exp2(x[12:].double())
     assert ((y[12:].double() - ref).abs() / ref).max().item() <= 1.7e-7
+
+
+@pytest.mark.parametrize("N,dtype,d", [(300, torch.float32, 64), (300, torch.float32, 128), (6200, torch.bfloat16, 64)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_a_bad_upstream_gradient_is_seen_and_stays_where_it_is(N, dtype, d, bad):
+    """Callers whose gradient is rescaled for fp16 operands: the (batch, head) pair of a bad element gets gradients that are
+    not finite (what loss scalers look for), and the other pairs the same as without it."""
+    from lookahead_keys_attention_b200 import castle_attention_packed
+    torch.manual_seed(N)
+    x = (torch.randn(2, N, 6, 2, d, device="cuda") * 3 ** -0.5).to(dtype).requires_grad_()
+    g = (torch.randn(2, 2, N, d, device="cuda") * 1e-3).to(dtype)
+    out = castle_attention_packed(x, d ** -0.5)
+    good = torch.autograd.grad(out, x, g, retain_graph=True)[0]
+    g[1, 1, N // 2, 3] = bad
+    grad = torch.autograd.grad(out, x, g)[0]
+    assert not grad[1, :, :, 1].isfinite().all()
+    for b, h in [(0, 0), (0, 1), (1, 0)]:
+        a, w = grad[b, :, :, h].float(), good[b, :, :, h].float()
+        assert (a - w).norm().item() <= 4e-3 * w.norm().item()   # sums in arrival order differ by a few ulps
+
+
+@pytest.mark.parametrize("top", [1e-20, 1e9, 3e13, 1e30])
+def test_the_gradients_magnitude_does_not_matter(top):
+    """A power of two of the upstream gradient is one of the gradients."""
+    from lookahead_keys_attention_b200 import castle_attention_packed
+    torch.manual_seed(0)
+    x = (torch.randn(1, 200, 6, 2, 64, device="cuda") * 3 ** -0.5).requires_grad_()
+    g = torch.randn(1, 2, 200, 64, device="cuda")
+    f = 2.0 ** torch.tensor(top).log2().round().item()
+    out = castle_attention_packed(x, 0.125)
+    a, b = (torch.autograd.grad(out, x, t, retain_graph=True)[0] for t in (g * f, g))
+    # below 2^-24 of the usual magnitude the factor stays 2^24 and fp16 loses what lies under its range
+    assert (a.double() / f - b.double()).norm().item() <= 4e-3 * b.double().norm().item() or top < 1e-9
+    assert a.isfinite().all()
