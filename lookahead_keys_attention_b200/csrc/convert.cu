@@ -1,12 +1,13 @@
-// Element-type conversions around the parallel kernels, for callers whose tensors the kernels do not take as
-// they are: bf16 tensors that are computed with fp16 operands (long sequences), in one pass each way.
+// Element-type conversion for hosts of the C ABI that hold contiguous tensors (this package's own passes go through
+// transform.cu): bf16 tensors that are computed with fp16 operands (long sequences), in one pass each way.
 // HBM-bound: 16 bytes in and 16 bytes out per thread and iteration, grid-stride.
 #include "common.cuh"
 #include "sm100.cuh"
 
 namespace castle {
 
-// bf16 -> fp16, saturating at +-65504 instead of overflowing to infinity; optional factor `*mul` (device scalar).
+// bf16 -> fp16, saturating at +-65504 instead of overflowing to infinity (NaN stays NaN); optional factor `*mul` (device scalar).
+__device__ __forceinline__ float saturate_f16(float x) { return x != x ? x : fminf(fmaxf(x, -65504.f), 65504.f); }
 __global__ void __launch_bounds__(256) castle_bf16_to_f16_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst,
                                                                  int64_t n8, const float* mul) {
   const float m = mul ? *mul : 1.f;
@@ -15,10 +16,8 @@ __global__ void __launch_bounds__(256) castle_bf16_to_f16_kernel(const uint4* __
     uint32_t* u = &v.x;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float2 f = Elem<__nv_bfloat16>::unpack2(u[j]);
-      f.x = fminf(fmaxf(f.x * m, -65504.f), 65504.f);
-      f.y = fminf(fmaxf(f.y * m, -65504.f), 65504.f);
-      u[j] = Elem<__half>::pack2(f.x, f.y);
+      const float2 f = Elem<__nv_bfloat16>::unpack2(u[j]);
+      u[j] = Elem<__half>::pack2(saturate_f16(f.x * m), saturate_f16(f.y * m));
     }
     dst[i] = v;
   }

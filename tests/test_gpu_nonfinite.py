@@ -83,3 +83,12 @@ def test_the_gradients_magnitude_does_not_matter(top):
     # below 2^-24 of the usual magnitude the factor stays 2^24 and fp16 loses what lies under its range
     assert (a.double() / f - b.double()).norm().item() <= 4e-3 * b.double().norm().item() or top < 1e-9
     assert a.isfinite().all()
+
+
+def test_conversion_keeps_nan():
+    from lookahead_keys_attention_b200 import _lib as L
+    x = torch.tensor([1.0, float("nan"), float("inf"), -float("inf"), 7e4, 0.0, -3.0, 5.0], device="cuda").bfloat16()
+    y = torch.empty_like(x, dtype=torch.float16)
+    L.check(L.load().castle_convert_16bit(L.BF16, x.data_ptr(), y.data_ptr(), x.numel(), None, None), "convert")
+    want = x.float().clamp(-65504, 65504).half()
+    assert y[1].isnan() and torch.equal(y[2:], want[2:]) and y[0] == 1
