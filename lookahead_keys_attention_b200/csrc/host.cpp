@@ -506,10 +506,16 @@ struct CastleBackward : public Node {
   }
 };
 
+// Whether forward-mode differentiation goes through the tensor, which the kernels would drop.
+bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
+
 // Forward with its gradient node; `vars` are the differentiable inputs (one packed, or six in operator order).
 Result attention(const Problem& p, Inputs in, Options o, const std::vector<Tensor>& vars) {
   bool any = false;
-  for (const auto& v : vars) any |= v.requires_grad();
+  for (const auto& v : vars) {
+    any |= v.requires_grad();
+    TORCH_CHECK_NOT_IMPLEMENTED(!has_tangent(v), "castle_attention: forward-mode differentiation is not implemented");
+  }
   o.need_grad = any && at::GradMode::is_enabled();
   const at::Device dev = vars[0].device();
   Result r;
@@ -629,14 +635,14 @@ struct Layer {
 };
 
 // Whether the layer can run natively around the core, too: plain CUDA tensors of one type, and nothing that changes what a
-// linear call means (autocast, a dispatch mode).
+// linear call means (autocast, a dispatch mode, forward-mode differentiation).
 bool plain_layer(const Tensor& x, const Layer& l) {
   auto plain = [&](const Tensor& t) {
     return t.is_cuda() && t.scalar_type() == x.scalar_type() && t.is_contiguous() && t.layout() == at::kStrided && t.device() == x.device() &&
-           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !t.unsafeGetTensorImpl()->is_python_dispatch();
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !t.unsafeGetTensorImpl()->is_python_dispatch() && !has_tangent(t);
   };
   const int64_t inner = l.heads * l.dim_head;
-  return x.dim() == 3 && x.is_cuda() && x.numel() > 0 && x.layout() == at::kStrided && !x.unsafeGetTensorImpl()->is_python_dispatch() &&
+  return x.dim() == 3 && x.is_cuda() && x.numel() > 0 && x.layout() == at::kStrided && !x.unsafeGetTensorImpl()->is_python_dispatch() && !has_tangent(x) &&
          dtype_code(x.scalar_type()) >= 0 && x.size(2) % 8 == 0 && plain(l.to_qkv) && plain(l.combine) &&
          (!l.norm.defined() || (plain(l.norm) && l.norm.dim() == 1 && l.norm.size(0) == x.size(2))) && l.to_qkv.dim() == 2 &&
          l.to_qkv.size(0) == 6 * inner && l.to_qkv.size(1) == x.size(2) && l.combine.dim() == 2 && l.combine.size(1) == inner &&

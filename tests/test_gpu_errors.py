@@ -66,3 +66,24 @@ def test_empty_tensors_are_refused(dtype, B, N):
         castle_attention_packed(torch.zeros(B, N, 6, 2, 64, device="cuda", dtype=dtype), 0.125)
     with pytest.raises(RuntimeError):
         Castle(32, heads=2).cuda().to(dtype)(torch.zeros(B, N, 32, device="cuda", dtype=dtype))
+
+
+@pytest.mark.parametrize("dual", ["x", "to_all_qkv", "norm"])
+def test_forward_mode_differentiation_is_refused(dual):
+    """Instead of dropping the tangent."""
+    import torch.autograd.forward_ad as fwAD
+    from lookahead_keys_attention_b200 import Castle, castle_attention_packed
+    m = Castle(32, heads=2, prenorm=True).cuda().requires_grad_(False)
+    x = torch.randn(2, 40, 32, device="cuda")
+    with fwAD.dual_level():
+        weights = {}
+        if dual == "x":
+            x = fwAD.make_dual(x, torch.ones_like(x))
+        else:
+            w = getattr(m, dual).weight.detach().clone()
+            weights = {dual + ".weight": fwAD.make_dual(w, torch.ones_like(w))}
+        with pytest.raises(NotImplementedError, match="forward-mode"):
+            torch.func.functional_call(m, weights, (x,))
+        p = torch.randn(1, 40, 6, 2, 64, device="cuda")
+        with pytest.raises(NotImplementedError, match="forward-mode"):
+            castle_attention_packed(fwAD.make_dual(p, p), 0.125)
