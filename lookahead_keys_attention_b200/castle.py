@@ -174,13 +174,14 @@ class Castle(nn.Module):
     def _merge(self, out):
         return self.combine_heads(out.permute(0, 2, 1, 3).flatten(2))   # 'b h n d -> b n (h d)'
 
-    def _forward_rotated(self, x, cache, return_next_cache):
-        """With a rotary embedding of the caller's own (a subclass, or another object with `rotate(t, offset)`) in
-        the place of `_Rotary`: rotated by it, then the operators."""
+    def _forward_operators(self, x, cache, return_next_cache):
+        """Submodules and operators called from here: under torch.jit.trace, which has to see them, and with a rotary
+        embedding of the caller's own (a subclass, or another object with `rotate(t, offset)`) in the place of `_Rotary`."""
         seq_len = x.shape[1]
         qu, ku, vu, qc, kc, vc = self._split(self.to_all_qkv(self.norm(x)))
         t = cache[0].shape[-2] if cache is not None else 0
-        qc, kc, qu, ku, vu = (self.rotary_emb.rotate(v, t) for v in (qc, kc, qu, ku, vu))
+        if self.rotary_emb is not None:
+            qc, kc, qu, ku, vu = (self.rotary_emb.rotate(v, t) for v in (qc, kc, qu, ku, vu))
         if seq_len == 1:
             with torch.no_grad():
                 state = self._buffers_for_step(cache, t, qu)
@@ -200,12 +201,12 @@ class Castle(nn.Module):
         is_inference = seq_len == 1
         if return_next_cache is None:
             return_next_cache = is_inference
-        layer = self._plain_layer()
         rotary, freqs = self.rotary_emb, None
         if rotary is not None:
-            if type(rotary) is not _Rotary or "rotate" in rotary.__dict__:
-                return self._forward_rotated(x, cache, return_next_cache)
-            freqs = rotary._buffers["freqs"]
+            freqs = rotary._buffers.get("freqs") if type(rotary) is _Rotary and "rotate" not in rotary.__dict__ else None
+        if (rotary is not None and freqs is None) or torch._C._is_tracing():
+            return self._forward_operators(x, cache, return_next_cache)
+        layer = self._plain_layer()
 
         if is_inference:
             t = 0 if cache is None else cache._length if isinstance(cache, ModuleCache) else cache[0].shape[-2]

@@ -76,6 +76,31 @@ def forward_chunks(B: int, H: int, per_pair: int, limit: int | None = None):
 LONG_SEQ_FP16 = 6144
 
 
+class _Traced(torch.autograd.Function):
+    """An operator while torch.jit.trace is recording: a Python autograd function becomes a node of the traced graph,
+    which calls it again when the graph runs; of the native operator the tracer would only see the allocations."""
+
+    @staticmethod
+    def forward(ctx, packed_op, scale, return_U, *inputs):
+        with torch.enable_grad():
+            leaves = [t.detach().requires_grad_(t.requires_grad) for t in inputs]
+            limits = (scale, return_U, None, MAX_WORKSPACE_BYTES, LONG_SEQ_FP16)
+            host = _lib.host()
+            result = host.attention_packed(*leaves, *limits, None, True) if packed_op else host.attention(*leaves, *limits)
+        out, *U = result if return_U else (result,)
+        ctx.graph = leaves, out
+        if return_U:
+            ctx.mark_non_differentiable(*U)
+        return (out.detach(), *U) if return_U else out.detach()
+
+    @staticmethod
+    def backward(ctx, grad, *_):
+        leaves, out = ctx.graph
+        wanted = [t for t in leaves if t.requires_grad]
+        grads = iter(torch.autograd.grad(out, wanted, grad, retain_graph=True))
+        return (None, None, None, *(next(grads) if t.requires_grad else None for t in leaves))
+
+
 def castle_attention_packed(packed, scale, return_U_for_cache=False, cache_out=None):
     """Parallel CASTLE attention on the packed projection output (B, N, 6, H, d), order
     qu,ku,vu,qc,kc,vc (the layout `to_all_qkv` produces).  Returns out (B, H, N, d) [, U].
@@ -83,6 +108,8 @@ def castle_attention_packed(packed, scale, return_U_for_cache=False, cache_out=N
     kernels write the cache rows themselves and the returned U is cache_out[0].
     Its gradient is the packed buffer the backward kernels write, so autograd has nothing to
     scatter or sum (six separate view-gradients cost ~10 extra passes)."""
+    if torch._C._is_tracing() and cache_out is None:
+        return _Traced.apply(True, float(scale), bool(return_U_for_cache), packed)
     return _lib.host().attention_packed(packed, scale, return_U_for_cache, cache_out, MAX_WORKSPACE_BYTES, LONG_SEQ_FP16,
                                         None, True)
 
@@ -90,6 +117,8 @@ def castle_attention_packed(packed, scale, return_U_for_cache=False, cache_out=N
 def castle_attention(qc, kc, vc, qu, ku, vu, scale, return_U_for_cache=False, cache_out=None):
     """Parallel CASTLE attention on (B, H, N, d) tensors (views are fine).
     Returns `out`, or `(out, U)` when `return_U_for_cache`; `cache_out` as in `castle_attention_packed`."""
+    if torch._C._is_tracing() and cache_out is None:
+        return _Traced.apply(False, float(scale), bool(return_U_for_cache), qc, kc, vc, qu, ku, vu)
     return _lib.host().attention(qc, kc, vc, qu, ku, vu, scale, return_U_for_cache, cache_out, MAX_WORKSPACE_BYTES,
                                  LONG_SEQ_FP16)
 
