@@ -201,19 +201,21 @@ class Castle(nn.Module):
         is_inference = seq_len == 1
         if return_next_cache is None:
             return_next_cache = is_inference
+        layer = self._plain_layer()
         rotary, freqs = self.rotary_emb, None
         if rotary is not None:
-            freqs = rotary._buffers.get("freqs") if type(rotary) is _Rotary and "rotate" not in rotary.__dict__ else None
-        if (rotary is not None and freqs is None) or torch._C._is_tracing():
-            return self._forward_operators(x, cache, return_next_cache)
-        layer = self._plain_layer()
+            if type(rotary) is not _Rotary or "rotate" in rotary.__dict__:
+                return self._forward_operators(x, cache, return_next_cache)
+            freqs = rotary._buffers["freqs"]
 
+        # The native calls return None where their torch functions have to be seen (a tracer, a torch function mode).
         if is_inference:
             t = 0 if cache is None else cache._length if isinstance(cache, ModuleCache) else cache[0].shape[-2]
             state = self._state_in_place(cache, t)
-            if layer is not None and state is not None:
-                out = host.layer_decode(x, *layer, self.scale, freqs, state.bufs, t)
-            else:
+            out = host.layer_decode(x, *layer, self.scale, freqs, state.bufs, t) if layer is not None and state is not None else None
+            if out is None:
+                if torch._C._is_tracing():
+                    return self._forward_operators(x, cache, return_next_cache)
                 packed = self._project(x)
                 if state is None:
                     state = self._buffers_for_step(cache, t, packed[:, :, 0].transpose(1, 2))
@@ -223,19 +225,25 @@ class Castle(nn.Module):
 
         assert cache is None, "must be inferencing single tokens if receiving cache"
         limits = (ops.MAX_WORKSPACE_BYTES, ops.LONG_SEQ_FP16)
-        native = layer is not None and not torch.is_autocast_enabled("cuda")   # under autocast only the projection knows the type
-        packed = None if native else self._project(x)
-        state = views = None
-        if return_next_cache:
+        out = state = views = None
+
+        def new_cache(like):
             # The cache lives in buffers with spare rows so that decode steps can append in place.  The forward's
             # kernels fill it themselves: from their operand tiles where those are the caller's values, otherwise
             # in the pass that makes the operands.
-            like = x if native else packed
             state = self._new_buffers(x.shape[0], self.heads, self.dim_head, seq_len, like.dtype, like.device)
-            views = state.views(seq_len)
-        if native:
+            return state, state.views(seq_len)
+
+        if layer is not None and not torch.is_autocast_enabled("cuda"):   # under autocast only the projection knows the type
+            if return_next_cache:
+                state, views = new_cache(x)
             out = host.layer_forward(x, *layer, self.scale, freqs, views, *limits)
-        else:
+        if out is None:
+            if torch._C._is_tracing():
+                return self._forward_operators(x, cache, return_next_cache)
+            packed = self._project(x)
+            if return_next_cache:
+                state, views = new_cache(packed)
             out = self._merge(host.attention_packed(packed, self.scale, False, views, *limits, freqs, False))
         if not return_next_cache:
             return out

@@ -15,7 +15,10 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+#include <torch/csrc/PyInterpreter.h>
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/autocast_mode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -1029,10 +1032,23 @@ Layer arg_layer(PyObject* const* a) {   // norm weight or None, eps or None, to_
   return l;
 }
 
-// layer_forward(x, <layer: 6>, scale, rotary freqs or None, caches or None, limit, long_seq)
+// Whether something records torch operations or may replace torch functions, so that the layer's have to be called from
+// Python: jit tracing, a tensor class of its own, or a torch function mode (but a default device).
+PyObject* device_context = nullptr;   // torch's class of the modes that set one
+bool watched(PyObject* const* a) {   // (x, <layer: 6>, ...)
+  if (torch::jit::tracer::isTracing()) return true;
+  for (int i : {0, 1, 3, 4})
+    if (a[i] != Py_None && !THPVariable_CheckExact(a[i])) return true;
+  for (int64_t i = 0; i < at::impl::PythonTorchFunctionTLS::stack_len(); ++i)
+    if (reinterpret_cast<PyObject*>(Py_TYPE(at::impl::PythonTorchFunctionTLS::get_stack_at(i)->ptr(getPyInterpreter()))) != device_context) return true;
+  return false;
+}
+
+// layer_forward(x, <layer: 6>, scale, rotary freqs or None, caches or None, limit, long_seq); None where it is watched()
 PyObject* py_layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return guarded([&] {
+  return guarded([&]() -> PyObject* {
     arg_count(n, 12);
+    if (watched(a)) Py_RETURN_NONE;
     const Tensor x = arg_tensor(a[0]);
     const Layer l = arg_layer(a + 1);
     Options o;
@@ -1050,10 +1066,11 @@ PyObject* py_layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
-// layer_decode(x, <layer: 6>, scale, rotary freqs or None, caches, cache_len)
+// layer_decode(x, <layer: 6>, scale, rotary freqs or None, caches, cache_len); None where it is watched()
 PyObject* py_layer_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  return guarded([&] {
+  return guarded([&]() -> PyObject* {
     arg_count(n, 11);
+    if (watched(a)) Py_RETURN_NONE;
     const Tensor x = arg_tensor(a[0]);
     const Layer l = arg_layer(a + 1);
     const double scale = arg_float(a[7]);
@@ -1166,6 +1183,11 @@ PyObject* py_bind(PyObject*, PyObject* d) {
     CASTLE_BIND(rmsnorm_fwd); CASTLE_BIND(rmsnorm_bwd_workspace_bytes); CASTLE_BIND(rmsnorm_bwd); CASTLE_BIND(bwd_workspace_bytes); CASTLE_BIND(bwd); CASTLE_BIND(transform); CASTLE_BIND(amax_scale);
     CASTLE_BIND(decode_workspace_bytes); CASTLE_BIND(decode_step_fused); CASTLE_BIND(token_linear_fits); CASTLE_BIND(token_linear);
 #undef CASTLE_BIND
+    PyObject* module = PyImport_ImportModule("torch.utils._device");
+    Py_XDECREF(device_context);
+    device_context = module ? PyObject_GetAttrString(module, "DeviceContext") : nullptr;
+    Py_XDECREF(module);
+    if (!device_context) return nullptr;
     Py_RETURN_NONE;
   });
 }

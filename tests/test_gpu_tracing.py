@@ -56,3 +56,46 @@ def test_jit_trace_of_the_operators(packed):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and not want[1].requires_grad
     g = torch.randn_like(got[0])
     assert _rel(torch.autograd.grad(got[0], b, g)[0], torch.autograd.grad(want[0], b, g)[0]) <= 4e-3
+
+
+class _Scaled(torch.Tensor):
+    """A weight that emulates another precision where it is used."""
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        plain = lambda t: t.as_subclass(torch.Tensor) * 2 if isinstance(t, cls) and func is torch.nn.functional.linear else t   # noqa: E731
+        return super().__torch_function__(func, types, tuple(plain(a) for a in args), kwargs)
+
+
+def test_torch_functions_are_called_where_they_may_be_replaced():
+    from torch.overrides import TorchFunctionMode
+    from lookahead_keys_attention_b200 import Castle
+
+    class DoubleLinear(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            y = func(*args, **(kwargs or {}))
+            return y * 2 if func is torch.nn.functional.linear else y
+
+    torch.manual_seed(0)
+    m = Castle(96, heads=2).cuda().bfloat16().requires_grad_(False)
+    x = torch.randn(2, 140, 96, device="cuda").bfloat16()
+    last = m.combine_heads.weight.clone()
+    with torch.no_grad():
+        plain, cache = m(x, return_next_cache=True)
+        step, _ = m(x[:, :1], cache=cache)
+        with torch.device("cuda"):                    # a default device replaces nothing
+            assert torch.equal(m(x), plain)
+        m.to_all_qkv.weight.mul_(2)
+        m.combine_heads.weight.mul_(2)
+        want, cache = m(x, return_next_cache=True)
+        want_step, _ = m(x[:, :1], cache=cache)
+        m.to_all_qkv.weight.mul_(0.5)
+        m.combine_heads.weight.mul_(0.5)
+        assert torch.equal(m.combine_heads.weight, last)
+        with DoubleLinear():
+            got, cache = m(x, return_next_cache=True)
+            got_step, _ = m(x[:, :1], cache=cache)
+        assert _rel(got, want) <= 1e-2 and _rel(got_step, want_step) <= 1e-2
+        for sub in (m.to_all_qkv, m.combine_heads):
+            sub._parameters["weight"] = sub.weight.detach().as_subclass(_Scaled)
+        assert _rel(m(x), want) <= 1e-2
