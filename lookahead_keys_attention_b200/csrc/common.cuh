@@ -80,6 +80,10 @@ inline encode_tiled_fn get_encode_fn() {
 // box (64, box_rows, 1, 1), 128-byte swizzle, out-of-range rows read as zero.
 inline int make_tmap_16bit(CUtensorMap* m, const castle_tensor_t* t, int dtype, int B, int H, int N, int D,
                            int box_rows, const char* name) {
+  // The map's dimensions are distinct places in memory: a repeated one (stride 0) has no map, and any other stride in
+  // its place would read past the tensor.
+  if ((N > 1 && t->stride_n == 0) || (H > 1 && t->stride_h == 0) || (B > 1 && t->stride_b == 0))
+    return reject("%s: a stride of 0 is not supported where there is more than one element", name);
   encode_tiled_fn fn = get_encode_fn();
   if (!fn) return reject("cuTensorMapEncodeTiled is not available from this driver");
   // The encoder is a driver call and needs a current context on the calling thread; a thread
@@ -93,9 +97,9 @@ inline int make_tmap_16bit(CUtensorMap* m, const castle_tensor_t* t, int dtype, 
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)N, (cuuint64_t)H, (cuuint64_t)B};
   // a size-1 dimension may carry any stride; give it a legal one
   cuuint64_t sn = (cuuint64_t)t->stride_n * 2, sh = (cuuint64_t)t->stride_h * 2, sb = (cuuint64_t)t->stride_b * 2;
-  if (N == 1 || sn == 0) sn = (cuuint64_t)D * 2;
-  if (H == 1 || sh == 0) sh = sn * (cuuint64_t)N;
-  if (B == 1 || sb == 0) sb = sh * (cuuint64_t)H;
+  if (N == 1) sn = (cuuint64_t)D * 2;
+  if (H == 1) sh = sn * (cuuint64_t)N;
+  if (B == 1) sb = sh * (cuuint64_t)H;
   cuuint64_t strides[3] = {sn, sh, sb};
   cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};

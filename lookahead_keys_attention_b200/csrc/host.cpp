@@ -166,11 +166,13 @@ castle_tensor_t desc(const Tensor& t) {   // (B, H, N, d), last dimension contig
   return {t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)};
 }
 
-// The ABI's alignment rules: 16-byte base and strides.
+// The ABI's rules: 16-byte base and strides, the last dimension contiguous, and no dimension that repeats one element's
+// row (stride 0, as expand() leaves it), which the kernels' tensor maps cannot express.
 bool aligned(const Tensor& t) {
-  const int64_t es = t.element_size();
-  return (t.stride(3) == 1 || t.size(3) == 1) && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && t.stride(0) * es % 16 == 0 &&
-         t.stride(1) * es % 16 == 0 && t.stride(2) * es % 16 == 0;
+  if ((t.stride(-1) != 1 && t.size(-1) != 1) || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0) return false;
+  for (int64_t i = 0; i + 1 < t.dim(); ++i)
+    if (t.stride(i) * t.element_size() % 16 != 0 || (t.stride(i) == 0 && t.size(i) > 1)) return false;
+  return true;
 }
 Tensor aligned_view(const Tensor& t) { return aligned(t) ? t : t.clone(at::MemoryFormat::Contiguous); }
 
@@ -182,14 +184,6 @@ castle_tensor_t packed_desc(const Tensor& p, int i) {
 // Contiguous at a 16-byte boundary (contiguous() leaves a view at an odd offset as it is).
 Tensor aligned_contiguous(const Tensor& t) {
   return t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
-}
-
-// A packed (B, N, 6, H, d) tensor as the kernels take it: itself, or a copy.
-Tensor aligned_packed(const Tensor& t) {
-  const int64_t es = t.element_size();
-  const bool ok = (t.stride(4) == 1 || t.size(4) == 1) && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && t.stride(0) * es % 16 == 0 &&
-                  t.stride(1) * es % 16 == 0 && t.stride(2) * es % 16 == 0 && t.stride(3) * es % 16 == 0;
-  return ok ? t : t.clone(at::MemoryFormat::Contiguous);
 }
 
 castle_tensor_t rect(castle_tensor_t t, int64_t es, int64_t b, int64_t h) {
@@ -474,7 +468,7 @@ struct SavedCore {
     castle_tensor_t in[6];
     std::vector<Tensor> keep;
     for (const auto& t : u.inputs) {
-      if (u.inputs.size() == 1) keep.push_back(aligned_packed(restored(t, {p.B, p.N, 6, p.H, p.dp}, p.cdtype, dev)));
+      if (u.inputs.size() == 1) keep.push_back(aligned_view(restored(t, {p.B, p.N, 6, p.H, p.dp}, p.cdtype, dev)));
       else keep.push_back(aligned_view(restored(t, bhnd, p.cdtype, dev)));
     }
     for (int i = 0; i < 6; ++i) in[i] = keep.size() == 1 ? packed_desc(keep[0], i) : desc(keep[i]);
@@ -565,7 +559,7 @@ Result attention_packed(const Tensor& packed, Options o) {   // (B, N, 6, H, d),
   Tensor t;
   {
     at::NoGradGuard no_grad;
-    t = aligned_packed(packed);
+    t = aligned_view(packed);
   }
   Inputs in;
   for (int i = 0; i < 6; ++i) in.t[i] = packed_desc(t, i);

@@ -237,3 +237,33 @@ def test_packed_operator_equals_six_view_operator():
     assert torch.allclose(a.grad.float(), b.grad.float(), atol=1e-2, rtol=1e-2)
     for i in (0, 4, 5):  # qu, kc, vc slots
         assert torch.equal(a.grad[:, :, i], b.grad[:, :, i])
+
+
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 64), (torch.float16, 128), (torch.float32, 64), (torch.bfloat16, 32)])
+@pytest.mark.parametrize("dim", [0, 1, 2])
+def test_expanded_inputs_and_gradients(dtype, d, dim):
+    """Tensors that repeat a batch row, a head (keys shared by the heads) or a position, and the upstream gradient that a
+    mean over one of them leaves: the same as their copies."""
+    from lookahead_keys_attention_b200 import castle_attention, castle_attention_packed
+    torch.manual_seed(d + dim)
+    B, H, N = 3, 2, 200
+
+    def rep(std):
+        shape = [B, H, N, d]
+        shape[dim] = 1
+        return (torch.randn(shape, device="cuda") * std).to(dtype).expand(B, H, N, d)
+
+    v = [(torch.randn(B, H, N, d, device="cuda") * 3 ** -0.5).to(dtype) for _ in range(4)] + [rep(3 ** -0.5), rep(3 ** -0.5)]
+    v = [v[0], v[4], v[1], v[2], v[5], v[3]]
+    g = rep(1.0)
+    x = [t.detach().requires_grad_() for t in v]
+    y = [t.detach().clone(memory_format=torch.contiguous_format).requires_grad_() for t in v]
+    a, b = castle_attention(*x, d ** -0.5), castle_attention(*y, d ** -0.5)
+    assert torch.equal(a, b)
+    for p, q in zip(torch.autograd.grad(a, x, g), torch.autograd.grad(b, y, g.contiguous())):
+        assert (p.float() - q.float()).norm().item() <= 4e-3 * q.float().norm().item()
+    shape = [B, N, 6, H, d]
+    shape[{0: 0, 1: 3, 2: 1}[dim]] = 1
+    p = (torch.randn(shape, device="cuda") * 3 ** -0.5).to(dtype).expand(B, N, 6, H, d)
+    with torch.no_grad():
+        assert torch.equal(castle_attention_packed(p, d ** -0.5), castle_attention_packed(p.clone(memory_format=torch.contiguous_format), d ** -0.5))

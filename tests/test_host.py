@@ -233,3 +233,19 @@ def test_replica_without_parameters_is_called_through_its_submodules():
     assert m._plain_layer() is not None and replica._plain_layer() is None
     x = torch.randn(1, 5, 32)
     assert torch.equal(replica._project(x), m._project(x))
+
+
+def test_repeated_dimensions_are_refused_by_the_abi():
+    """A tensor map has no stride of 0; the kernels would read past a tensor that repeats a head or a batch row."""
+    L = _lib()
+    lib = L.load()
+    good = ctypes.byref(L.CastleTensor(1 << 20, 2 * 128 * 64, 128 * 64, 64))
+    for B, H, N, bad in [(3, 2, 128, (0, 128 * 64, 64)), (1, 2, 128, (0, 0, 64)), (1, 1, 128, (0, 0, 0))]:
+        prob = L.CastleProblem(B, H, N, 64, L.BF16, 0.125)
+        t = ctypes.byref(L.CastleTensor(1 << 20, *bad))
+        size = lib.castle_fwd_workspace_bytes(ctypes.byref(prob))
+        rc = lib.castle_fwd(ctypes.byref(prob), t, *([good] * 6), 1 << 20, None, 0, None, 1 << 20, size, 1 << 20, None)
+        assert rc < 0 and "stride of 0" in L.last_error(), L.last_error()
+        size = lib.castle_bwd_workspace_bytes(ctypes.byref(prob))
+        rc = lib.castle_bwd(ctypes.byref(prob), t, *([good] * 7), 1 << 20, 1 << 20, *([good] * 6), 1 << 20, size, 1 << 20, None)
+        assert rc < 0 and "stride of 0" in L.last_error(), L.last_error()
