@@ -568,13 +568,14 @@ Result attention_packed(const Tensor& packed, Options o) {   // (B, N, 6, H, d),
 }
 
 // ------------------------------------------------------------------------------------------------ decode step
-void check_caches(const Tensor* caches, int64_t B, int64_t H, int64_t d, at::ScalarType dtype) {
+void check_caches(const Tensor* caches, int64_t B, int64_t H, int64_t d, at::ScalarType dtype, const at::Device& dev) {
   const int64_t cap = caches[0].size(2);
   for (int i = 0; i < 4; ++i) {
     const Tensor& c = caches[i];
     if (!(c.scalar_type() == dtype && c.dim() == 4 && c.size(0) == B && c.size(1) == H && c.size(2) == cap && c.size(3) == d &&
           c.stride(3) == 1))
       throw AssertError("castle_decode_step: the caches must be (B, H, capacity, d) buffers of the token's type");
+    need(c.device() == dev, "castle_decode_step: the caches must be on the token's device");
   }
 }
 
@@ -598,7 +599,7 @@ Tensor decode_core(const castle_tensor_t* news, const Tensor* caches, int64_t B,
   const c10::cuda::CUDAGuard guard(dev);
   rotary.fit(dev, d);
   const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
-  check_caches(caches, B, H, d, dtype);
+  check_caches(caches, B, H, d, dtype, dev);
   Tensor out = at::empty({B, H, 1, d}, caches[0].options());
   const castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
   StreamUse use(stream);
@@ -616,8 +617,8 @@ Tensor decode_step(const Tensor* news, const Tensor* caches, int64_t t, double s
   Tensor keep[6];
   castle_tensor_t nd[6];
   for (int i = 0; i < 6; ++i) {
-    need(news[i].scalar_type() == dtype && news[i].sizes() == news[0].sizes(),
-         "castle_decode_step: the new rows must have one shape and type");
+    need(news[i].scalar_type() == dtype && news[i].sizes() == news[0].sizes() && news[i].device() == news[0].device(),
+         "castle_decode_step: the new rows must have one shape, type and device");
     keep[i] = aligned_view(news[i]);
     nd[i] = desc(keep[i]);
   }
@@ -820,7 +821,7 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
   const auto dtype = x.scalar_type();
   const int64_t B = x.size(0), dim = x.size(2), H = l.heads, d = l.dim_head, inner = H * d, es = x.element_size();
-  check_caches(caches, B, H, d, dtype);
+  check_caches(caches, B, H, d, dtype, dev);
   const castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
   const int64_t row = (B * inner * es + 255) / 256 * 256;
   const size_t part = (api.decode_workspace_bytes(&cp, (int32_t)t) + 255) / 256 * 256;
@@ -922,13 +923,13 @@ void arg_count(Py_ssize_t n, Py_ssize_t want) {
 }
 
 // The operators' rule for caches: the kernels store their 16-bit operand tiles.
-void check_cache_out(const Options& o, at::IntArrayRef bhnd, at::ScalarType dtype) {
+void check_cache_out(const Options& o, at::IntArrayRef bhnd, at::ScalarType dtype, const at::Device& dev) {
   if (o.caches.empty()) return;
   const bool fills = (dtype == at::kHalf || (dtype == at::kBFloat16 && bhnd[2] < o.long_seq)) && (bhnd[3] == 64 || bhnd[3] == 128);
   need(o.return_U && fills, "castle_attention: cache_out needs return_U, a 16-bit dtype and dim_head 64 or 128");
   for (const auto& c : o.caches)
-    need(c.sizes() == bhnd && c.scalar_type() == dtype && c.stride(3) == 1,
-         "castle_attention: cache_out tensors must be (B, H, N, d) views in the input dtype");
+    need(c.sizes() == bhnd && c.scalar_type() == dtype && c.stride(3) == 1 && c.device() == dev,
+         "castle_attention: cache_out tensors must be (B, H, N, d) views in the input dtype, on the inputs' device");
 }
 
 // t[:, :, :rows] without the dispatcher (a token makes four of these; caches are no part of any graph).
@@ -967,7 +968,7 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     Result r;
     {
       Unlocked u;
-      if (v[0].dim() == 4) check_cache_out(o, v[0].sizes(), v[0].scalar_type());
+      if (v[0].dim() == 4) check_cache_out(o, v[0].sizes(), v[0].scalar_type(), v[0].device());
       r = attention_six(v, o);
     }
     return wrap_result(std::move(r), o.return_U);
@@ -992,7 +993,7 @@ PyObject* py_attention_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
     {
       Unlocked u;
       if (strict && packed.dim() == 5)
-        check_cache_out(o, {packed.size(0), packed.size(3), packed.size(1), packed.size(4)}, packed.scalar_type());
+        check_cache_out(o, {packed.size(0), packed.size(3), packed.size(1), packed.size(4)}, packed.scalar_type(), packed.device());
       r = attention_packed(packed, o);
     }
     return wrap_result(std::move(r), o.return_U);

@@ -87,3 +87,27 @@ def test_forward_mode_differentiation_is_refused(dual):
         p = torch.randn(1, 40, 6, 2, 64, device="cuda")
         with pytest.raises(NotImplementedError, match="forward-mode"):
             castle_attention_packed(fwAD.make_dual(p, p), 0.125)
+
+
+def test_tensors_of_another_device_are_refused():
+    from lookahead_keys_attention_b200 import Castle, cache_from_buffers, castle_attention, castle_attention_packed, castle_decode_step
+    z = lambda n, dev="cuda": torch.zeros(2, 2, n, 64, device=dev, dtype=torch.bfloat16)   # noqa: E731
+    new, caches = [z(1) for _ in range(6)], [z(40) for _ in range(4)]
+    for i in range(4):
+        with pytest.raises(RuntimeError, match="device"):
+            castle_decode_step(*new, *[z(40, "cpu") if j == i else c for j, c in enumerate(caches)], 30, 0.125)
+    for i in range(1, 6):
+        with pytest.raises(RuntimeError, match="device"):
+            castle_decode_step(*[z(1, "cpu") if j == i else t for j, t in enumerate(new)], *caches, 30, 0.125)
+    with pytest.raises(RuntimeError, match="device"):   # pinned host memory, too: the step's bulk copies do not read it
+        castle_decode_step(*new, *[z(40, "cpu").pin_memory() for _ in range(4)], 30, 0.125)
+    six = [z(40) for _ in range(6)]
+    out = [z(40)] * 3 + [z(40, "cpu")]
+    with pytest.raises(RuntimeError, match="device"):
+        castle_attention(*six, 0.125, True, out)
+    with pytest.raises(RuntimeError, match="device"):
+        castle_attention_packed(torch.zeros(2, 40, 6, 2, 64, device="cuda", dtype=torch.bfloat16), 0.125, True, out)
+    with torch.no_grad():
+        m, x = Castle(32, heads=2).cuda().bfloat16(), torch.zeros(2, 1, 32, device="cuda", dtype=torch.bfloat16)
+        with pytest.raises(RuntimeError, match="device"):
+            m(x, cache=cache_from_buffers(*[z(40, "cpu") for _ in range(4)], 30))
