@@ -147,24 +147,27 @@ class Castle(nn.Module):
 
     def _plain_layer(self):
         """What the native path takes of this layer: norm weight and eps, the two projection weights and the head
-        sizes; or None where a submodule was replaced, has a bias or has hooks, so that it must be called as a module."""
+        sizes; or None where a submodule was replaced, has a bias, hooks or a forward of its own (how offloading wraps
+        it), so that it must be called as a module."""
         mods = self._modules
         norm, qkv, combine = mods["norm"], mods["to_all_qkv"], mods["combine_heads"]
         if type(qkv) is not nn.Linear or type(combine) is not nn.Linear or _has_any_global_hook():
             return None
         for m in (norm, qkv, combine):
-            if m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks:
+            own = m.__dict__
+            if ("forward" in own or own["_forward_hooks"] or own["_forward_pre_hooks"] or own["_backward_hooks"]
+                    or own["_backward_pre_hooks"]):
                 return None
         wq, wc = qkv._parameters, combine._parameters
-        if wq.get("bias") is not None or wc.get("bias") is not None:
-            return None
-        weights = wq.get("weight"), wc.get("weight")   # a data-parallel replica holds them as plain attributes
-        if weights[0] is None or weights[1] is None:
-            return None
-        if type(norm) is nn.Identity:
-            return None, None, *weights, self.heads, self.dim_head
-        if type(norm) is nn.RMSNorm and norm._parameters.get("weight") is not None and len(norm.normalized_shape) == 1:
-            return norm._parameters["weight"], norm.eps, *weights, self.heads, self.dim_head
+        try:
+            if wq["bias"] is not None or wc["bias"] is not None:
+                return None
+            if type(norm) is nn.Identity:
+                return None, None, wq["weight"], wc["weight"], self.heads, self.dim_head
+            if type(norm) is nn.RMSNorm and norm._parameters["weight"] is not None and len(norm.normalized_shape) == 1:
+                return norm._parameters["weight"], norm.eps, wq["weight"], wc["weight"], self.heads, self.dim_head
+        except KeyError:   # a data-parallel replica holds its weights as plain attributes
+            pass
         return None
 
     def _project(self, x):

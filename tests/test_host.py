@@ -249,3 +249,17 @@ def test_repeated_dimensions_are_refused_by_the_abi():
         size = lib.castle_bwd_workspace_bytes(ctypes.byref(prob))
         rc = lib.castle_bwd(ctypes.byref(prob), t, *([good] * 7), 1 << 20, 1 << 20, *([good] * 6), 1 << 20, size, 1 << 20, None)
         assert rc < 0 and "stride of 0" in L.last_error(), L.last_error()
+
+
+def test_a_wrapped_submodule_is_called():
+    """Libraries that offload or quantise replace `forward` on the instance."""
+    from lookahead_keys_attention_b200 import Castle
+    for name in ("norm", "to_all_qkv", "combine_heads"):
+        m = Castle(32, heads=2, dim_head=16, prenorm=True)
+        sub = getattr(m, name)
+        assert m._plain_layer() is not None
+        inner = sub.forward
+        sub.forward = lambda *a: inner(*a)
+        assert m._plain_layer() is None
+        del sub.forward
+        assert m._plain_layer() is not None
