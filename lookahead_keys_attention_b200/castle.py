@@ -119,6 +119,12 @@ class Castle(nn.Module):
         cap = rows + max(self.cache_headroom, rows // 4)
         return _CacheBuffers([torch.empty(b, h, cap, d, dtype=dtype, device=device) for _ in range(4)], 0)
 
+    def _new_cache(self, like) -> _CacheBuffers:
+        """The cache of a prompt of `like`'s batch size, length and type lives in buffers with spare rows so that decode
+        steps can append in place.  The forward's kernels fill it themselves: from their operand tiles where those are
+        the caller's values, otherwise in the pass that makes the operands."""
+        return self._new_buffers(like.shape[0], self.heads, self.dim_head, like.shape[1], like.dtype, like.device)
+
     def _state_in_place(self, cache, t):
         """The capacity buffers behind `cache` if row t can be appended to them as they are, else None."""
         if not isinstance(cache, ModuleCache) or cache._length != t:
@@ -230,23 +236,18 @@ class Castle(nn.Module):
         limits = (ops.MAX_WORKSPACE_BYTES, ops.LONG_SEQ_FP16)
         out = state = views = None
 
-        def new_cache(like):
-            # The cache lives in buffers with spare rows so that decode steps can append in place.  The forward's
-            # kernels fill it themselves: from their operand tiles where those are the caller's values, otherwise
-            # in the pass that makes the operands.
-            state = self._new_buffers(x.shape[0], self.heads, self.dim_head, seq_len, like.dtype, like.device)
-            return state, state.views(seq_len)
-
         if layer is not None and not torch.is_autocast_enabled("cuda"):   # under autocast only the projection knows the type
             if return_next_cache:
-                state, views = new_cache(x)
+                state = self._new_cache(x)
+                views = state.views(seq_len)
             out = host.layer_forward(x, *layer, self.scale, freqs, views, *limits)
         if out is None:
             if torch._C._is_tracing():
                 return self._forward_operators(x, cache, return_next_cache)
             packed = self._project(x)
             if return_next_cache:
-                state, views = new_cache(packed)
+                state = self._new_cache(packed)
+                views = state.views(seq_len)
             out = self._merge(host.attention_packed(packed, self.scale, False, views, *limits, freqs, False))
         if not return_next_cache:
             return out

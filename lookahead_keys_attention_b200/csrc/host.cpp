@@ -504,7 +504,10 @@ struct CastleBackward : public Node {
 };
 
 // Whether forward-mode differentiation goes through the tensor, which the kernels would drop.
-bool has_tangent(const Tensor& t) { return t.defined() && t._fw_grad(/*level=*/0).defined(); }
+bool has_tangent(const Tensor& t) {
+  const torch::autograd::AutogradMeta* m = t.defined() ? torch::autograd::impl::get_autograd_meta(t) : nullptr;
+  return m && m->fw_grad_ && t._fw_grad(/*level=*/0).defined();
+}
 
 // Forward with its gradient node; `vars` are the differentiable inputs (one packed, or six in operator order).
 Result attention(const Problem& p, Inputs in, Options o, const std::vector<Tensor>& vars) {
