@@ -3,8 +3,11 @@
 arguments, state-dict keys (`to_all_qkv.weight`, `combine_heads.weight`,
 `norm.weight`), `forward(x, cache=None, return_next_cache=None)` conventions
 and `Cache` tuple.  The attention cores run as sm_100a kernels through the
-C-ABI library, rotary embedding included; the two projections and the optional
-RMSNorm stay torch ops, issued natively (csrc/host.cpp) together with the core.
+C-ABI library, rotary embedding included.  A plain layer is one native call
+(csrc/host.cpp): RMSNorm and the projections of a few tokens are kernels of this
+package, the other projections library products, and the gradient one autograd
+node.  Where a submodule was replaced, wrapped or hooked, or something records or
+replaces torch functions, the submodules are called as modules instead.
 
 Difference from the reference, by design: the decode step appends to
 pre-allocated cache buffers and rewrites the lookahead keys `U` IN PLACE

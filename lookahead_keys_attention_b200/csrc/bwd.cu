@@ -542,8 +542,9 @@ static int launch_bwd(const BwdParams& p, const CUtensorMap* maps, cudaStream_t 
 
 using namespace castle;
 
-// fp32 accumulators dqc, dvu, dku and delta; at dim_head 128 rounded up so that the tile scratch behind them
-// stays 1 KB aligned
+// fp32 accumulators dqc, dvu, dku and delta; at dim_head 128, where only the first is summed into (the other two are
+// reserved, so that the size a caller asks for does not depend on how the kernels share the work), rounded up so that
+// the tile scratch behind them stays 1 KB aligned
 static size_t bwd_acc_bytes(const castle_problem_t* p) {
   int64_t rows = (int64_t)p->batch * p->heads * p->seq_len;
   size_t b = (size_t)(rows * (3 * p->dim_head + 1) * sizeof(float));

@@ -807,8 +807,11 @@ Tensor decode_packed(const Tensor& packed, const Tensor* caches, int64_t t, doub
 }
 
 // Whether one projection of a token is the framework's own launch.  It is the faster one on the host (3 us against 8 for a
-// library call, with the norm in it); on the GPU the library wins where the weights are large for the rows (own / library:
-// 8 x 512 -> 3072 6.2 / 4 us, 8 x 1472 -> 8832 14.5 / 7, 2 x 2176 -> 13056 16.5 / 10, 1 x 2176 -> 13056 10.4 / 10).
+// library call, with the norm in it); on the GPU the library wins in 16 bits where the weights are large for the rows (own /
+// library in us, weights from memory: 8 x 512 -> 3072 4.2 / 4.0, 8 x 1024 -> 6144 6.1 / 5.2, 8 x 1408 -> 8448 9.3 / 6.6,
+// 2 x 1408 -> 8448 8.6 / 7.0, 2 x 2176 -> 13056 14.6 / 11.8, 1 x 2176 -> 13056 12.2 / 12.0).  In fp32, where every row count
+// takes the FMA kernel, the library is the slower one on both sides of the bound (3 x 512 -> 3072 5.9 / 7.0, 8 x 512 -> 3072
+// 7.2 / 14.7, 8 x 1024 -> 6144 12.8 / 27.2), but at one row (512 -> 3072 4.5 / 4.1).
 bool own_projection(int dtype, int64_t rows, int64_t k, int64_t n, int64_t es) {
   return rows <= 8 && k * n * es <= (rows == 1 ? 64 << 20 : rows == 2 ? 16 << 20 : 8 << 20) &&
          api.token_linear_fits(dtype, (int32_t)rows, (int32_t)k);

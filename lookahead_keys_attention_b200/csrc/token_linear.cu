@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kTokenThreads) castle_token_linear_kernel(cons
 
 // Three to eight rows of a 16-bit type: a matrix product with mma.sync, the weights as the 16 x 16 operand and the tokens as
 // its 8 columns, which keeps it a stream over the weights (with fp32 arithmetic, x from shared memory is read R times per
-// weight: 33 us for 8 x 2176 -> 13056, here 14.5).  A CTA stages the
+// weight: 33 us for 8 x 2176 -> 13056, here 14.7, weights from memory).  A CTA stages the
 // normalised x once and walks `groups` groups of 16 weight rows; its warps are KS slices of K times 8 / KS groups at a
 // time, so that narrow outputs fill the SMs too.  A lane's 16-byte load of a weight row holds eight adjacent k; both
 // operands use the same permutation of k inside a block of 32 (lane t of a quad: k = 8t .. 8t + 7), so the loads need no
