@@ -221,6 +221,24 @@ int castle_token_linear(int32_t dtype, int32_t rows, int32_t in_features, int32_
                         int64_t row_stride, const void* norm_weight, float eps, const void* weight, void* y, int32_t overlap,
                         void* stream);
 
+/* ---- a layer's whole cached single-token step ----------------------------------
+ * Norm, projection, cached step and output projection of one token
+ * (lookahead_keys_attention/lookahead_keys_attention.py:91-112, :166-207) as one launch: castle_token_linear(),
+ * castle_decode_step_fused() and castle_token_linear() with what passes between them on the chip.  p: batch, heads,
+ * dim_head, dtype and scale; x: batch rows of `dim` elements, row_stride apart; to_qkv: (6 * heads * dim_head, dim) in
+ * the order qu, ku, vu, qc, kc, vc; combine: (out_features, heads * dim_head); both contiguous; y: contiguous
+ * (batch, out_features).  The caches' rows must be adjacent in memory.  `counters`: 8 * batch words that are zero before
+ * the call and zero again when its kernel has run.  `overlap` != 0: the launch may become resident before the work ahead
+ * of it on the stream has ended (it reads nothing before that).  castle_token_layer_fits says whether a size is supported.
+ */
+int castle_token_layer_fits(const castle_problem_t* p, int32_t cache_len, int32_t dim, int32_t out_features);
+size_t castle_token_layer_workspace_bytes(const castle_problem_t* p, int32_t out_features);
+int castle_token_layer(const castle_problem_t* p, int32_t cache_len, int32_t capacity, int32_t dim, int32_t out_features,
+                       const void* x, int64_t row_stride, const void* norm_weight, float eps, const void* to_qkv,
+                       const void* combine, const castle_tensor_t* u_cache, const castle_tensor_t* qu_cache,
+                       const castle_tensor_t* kc_cache, const castle_tensor_t* vc_cache, const castle_rotary_t* rotary, void* y,
+                       uint32_t* counters, int32_t overlap, void* workspace, size_t workspace_bytes, int32_t* status, void* stream);
+
 /* ---- cached single-token step without caller scratch -----------------------
  * (no counterpart in the reference)  Same step and same arguments as
  * castle_decode_step(), minus the workspace: the split partials go to a fixed

@@ -62,6 +62,9 @@ struct Api {
   decltype(&castle_decode_step_fused) decode_step_fused;
   decltype(&castle_token_linear_fits) token_linear_fits;
   decltype(&castle_token_linear) token_linear;
+  decltype(&castle_token_layer_fits) token_layer_fits;
+  decltype(&castle_token_layer_workspace_bytes) token_layer_workspace_bytes;
+  decltype(&castle_token_layer) token_layer;
 } api{};
 
 void check(int rc, const char* what) {
@@ -817,6 +820,13 @@ bool own_projection(int dtype, int64_t rows, int64_t k, int64_t n, int64_t es) {
          api.token_linear_fits(dtype, (int32_t)rows, (int32_t)k);
 }
 
+// Whether the layer's whole token is one launch (csrc/token_layer.cu).
+bool whole_token_layer(const castle_problem_t& p, const Tensor* caches, int64_t t, int64_t dim, int64_t out_features, int64_t es) {
+  for (int i = 0; i < 4; ++i)
+    if (!aligned(caches[i]) || caches[i].stride(2) != p.dim_head) return false;
+  return api.token_layer_fits(&p, (int32_t)t, (int32_t)dim, (int32_t)out_features);
+}
+
 // Norm, projection, step and output projection of one token, with what passes between them in the stream's scratch: on
 // the host the allocations would cost as much as the launches.
 Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_t t, double scale, Rotary rotary) {
@@ -829,6 +839,22 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   const int64_t B = x.size(0), dim = x.size(2), H = l.heads, d = l.dim_head, inner = H * d, es = x.element_size();
   check_caches(caches, B, H, d, dtype, dev);
   const castle_problem_t cp{(int32_t)B, (int32_t)H, 1, (int32_t)d, dtype_code(dtype), (float)scale};
+  const Tensor xs = x.stride(2) == 1 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * es % 16 == 0 ? x : aligned_contiguous(x);
+  if (whole_token_layer(cp, caches, t, dim, l.combine.size(0), es)) {
+    const int64_t N = l.combine.size(0);
+    castle_tensor_t c[4];
+    for (int i = 0; i < 4; ++i) c[i] = desc(caches[i]);
+    castle_rotary_t rot{};
+    if (rotary.on()) rot = rotary.desc(false);
+    Tensor y = at::empty({B, 1, N}, x.options().requires_grad(false));
+    StreamUse use(stream);
+    const Tensor words = use.zero_words(8 * B), ws = use.scratch(api.token_layer_workspace_bytes(&cp, (int32_t)N)), status = status_word(dev.index());
+    check(api.token_layer(&cp, (int32_t)t, (int32_t)caches[0].size(2), (int32_t)dim, (int32_t)N, xs.data_ptr(), xs.stride(0),
+                          l.norm.defined() ? l.norm.data_ptr() : nullptr, norm_eps(l), l.to_qkv.data_ptr(), l.combine.data_ptr(), &c[0], &c[1],
+                          &c[2], &c[3], rotary.on() ? &rot : nullptr, y.data_ptr(), reinterpret_cast<uint32_t*>(words.data_ptr()) + kAmaxWords,
+                          1, ws.data_ptr(), ws.numel(), status.data_ptr<int32_t>(), stream.stream()), "castle_token_layer");
+    return y;
+  }
   const int64_t row = (B * inner * es + 255) / 256 * 256;
   const size_t part = (api.decode_workspace_bytes(&cp, (int32_t)t) + 255) / 256 * 256;
   StreamUse use(stream);
@@ -836,7 +862,6 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   char* packed = static_cast<char*>(ws.data_ptr()) + part;
   char* core = packed + 6 * row;
   Tensor keep;
-  const Tensor xs = x.stride(2) == 1 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 && x.stride(0) * es % 16 == 0 ? x : aligned_contiguous(x);
   // The step and the last projection are launched ahead (see the C ABI's `overlap`).  The buffers they fetch early must be
   // in place before the first of the three launches: the words and the status word may launch a fill on first use.
   const bool overlap = own_projection(cp.dtype, B, dim, 6 * inner, es);
@@ -1183,6 +1208,7 @@ PyObject* py_bind(PyObject*, PyObject* d) {
     CASTLE_BIND(last_error); CASTLE_BIND(fwd_workspace_bytes); CASTLE_BIND(fwd); CASTLE_BIND(fwd_prefill);
     CASTLE_BIND(rmsnorm_fwd); CASTLE_BIND(rmsnorm_bwd_workspace_bytes); CASTLE_BIND(rmsnorm_bwd); CASTLE_BIND(bwd_workspace_bytes); CASTLE_BIND(bwd); CASTLE_BIND(transform); CASTLE_BIND(amax_scale);
     CASTLE_BIND(decode_workspace_bytes); CASTLE_BIND(decode_step_fused); CASTLE_BIND(token_linear_fits); CASTLE_BIND(token_linear);
+    CASTLE_BIND(token_layer_fits); CASTLE_BIND(token_layer_workspace_bytes); CASTLE_BIND(token_layer);
 #undef CASTLE_BIND
     PyObject* module = PyImport_ImportModule("torch.utils._device");
     Py_XDECREF(device_context);
