@@ -208,6 +208,15 @@ int castle_decode_step_fused(const castle_problem_t* p, int32_t cache_len, int32
                              const castle_rotary_t* rotary, uint32_t* counters, int32_t overlap, void* workspace,
                              size_t workspace_bytes, int32_t* status, void* stream);
 
+/* ---- small matrix products ------------------------------------------------------
+ * The projections around the core for calls too short for a library product's cost on the host
+ * (lookahead_keys_attention/lookahead_keys_attention.py:67-80, :99-104, :207, and their gradients).  layout 0:
+ * c[m,n] = a[m,k] b[n,k]^T; 1: c[m,n] = a[m,k] b[k,n]; 2: c[m,n] = a[k,m]^T b[k,n].  Row-major, rows lda, ldb, ldc
+ * elements apart, 16-byte aligned; n, and k (m in layout 2), multiples of 16 bytes.  All of `dtype`, sums in fp32.
+ */
+int castle_linear(int32_t dtype, int32_t layout, int32_t m, int32_t n, int32_t k, const void* a, int64_t lda, const void* b,
+                  int64_t ldb, void* c, int64_t ldc, int32_t* status, void* stream);
+
 /* ---- a token's projections ----------------------------------------------------
  * y = norm(x) @ weight^T for 1 to 8 rows: the projections around the cached step
  * (lookahead_keys_attention/lookahead_keys_attention.py:67-80, :99-104, :207) as one launch each.  x: rows of

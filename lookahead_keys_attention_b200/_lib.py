@@ -14,7 +14,7 @@ from pathlib import Path
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libcastle_b200.so"
-SOURCES = ["api.cu", "decode.cu", "selftest.cu", "convert.cu", "transform.cu", "token_linear.cu", "token_layer.cu", "norm.cu", "fwd.cu", "bwd.cu", "bwd128.cu"]
+SOURCES = ["api.cu", "decode.cu", "selftest.cu", "convert.cu", "transform.cu", "token_linear.cu", "token_layer.cu", "linear.cu", "norm.cu", "fwd.cu", "bwd.cu", "bwd128.cu"]
 
 BF16, F16, F32 = 0, 1, 2
 
@@ -185,6 +185,7 @@ _SIGNATURES = {
     "castle_token_layer_workspace_bytes": (_sz, [_PR, _i32]),
     "castle_token_layer": (ctypes.c_int, [_PR] + [_i32] * 4 + [_vp, ctypes.c_int64, _vp, ctypes.c_float, _vp, _vp] + [_T] * 4 +
                            [P(CastleRotary), _vp, _vp, _i32, _vp, _sz, _vp, _vp]),
+    "castle_linear": (ctypes.c_int, [_i32] * 5 + [_vp, ctypes.c_int64] * 3 + [_vp, _vp]),
     "castle_decode_step_static": (ctypes.c_int, [_PR, _i32, _i32] + [_T] * 11 + [_vp, _vp]),
     "castle_set_kernel_events": (ctypes.c_int, [_i32, _vp, _vp]),
     "castle_selftest_mma_rate": (ctypes.c_int, [_i32, _i32, _i32, _vp, _vp, _vp]),

@@ -62,6 +62,7 @@ struct Api {
   decltype(&castle_decode_step_fused) decode_step_fused;
   decltype(&castle_token_linear_fits) token_linear_fits;
   decltype(&castle_token_linear) token_linear;
+  decltype(&castle_linear) linear;
   decltype(&castle_token_layer_fits) token_layer_fits;
   decltype(&castle_token_layer_workspace_bytes) token_layer_workspace_bytes;
   decltype(&castle_token_layer) token_layer;
@@ -655,8 +656,35 @@ bool plain_layer(const Tensor& x, const Layer& l) {
 
 float norm_eps(const Layer& l) { return (float)l.eps.value_or(std::numeric_limits<float>::epsilon()); }   // torch's default for every type
 
-// y = x @ w^T on two-dimensional x
-Tensor matmul_t(const Tensor& x, const Tensor& w) { return at::mm(x, w.t()); }
+// Whether a product of a call over `rows` positions is the framework's own launch (csrc/linear.cu).  A library product costs the
+// host 8 to 10 us, an own one 4, and such calls are bound by the host; on the GPU the library is 1 to 2 us faster in 16 bits
+// (us, own / library: 197 x 512 -> 3072 4.9 / 3.4, 512 x 512 -> 3072 9.1 / 4.3, 2048 x 512 -> 3072 14.7 / 8.3) and slower in
+// fp32 but where the tiles are many (512 x 128 -> 768 8.6 / 6.2, 512 x 768 -> 128 10.2 / 14.4, its weight's gradient 7.0 / 10.3,
+// 197 x 512 -> 3072 33.6 / 25.4).  From some 1024 positions on the GPU is the bound.  A graph's replay costs the host nothing.
+bool small_product(int64_t rows, int64_t m, int64_t n, int64_t k, at::ScalarType t) {
+  const bool f32 = t == at::kFloat;
+  if (rows > 1024 || 2 * m * n * k > (f32 ? 128000000LL : 1000000000LL)) return false;
+  return dtype_code(t) >= 0 && std::min(n, k) >= 64;
+}
+// layout 0: a @ b^T; 1: a @ b; 2: a^T @ b, for two-dimensional a and b
+Tensor product(int layout, const Tensor& a, const Tensor& b, int64_t rows) {
+  const int64_t k = layout == 2 ? a.size(0) : a.size(1), m = layout == 2 ? a.size(1) : a.size(0), n = layout == 0 ? b.size(0) : b.size(1);
+  const int64_t unit = 16 / a.element_size();
+  auto fits = [&](const Tensor& t) { return t.stride(1) == 1 && t.stride(0) >= t.size(1) && aligned(t); };
+  if (small_product(rows, m, n, k, a.scalar_type()) && b.scalar_type() == a.scalar_type() && n % unit == 0 && (layout == 2 ? m : k) % unit == 0 &&
+      fits(a) && fits(b)) {
+    const auto stream = c10::cuda::getCurrentCUDAStream(a.device().index());
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream.stream(), &capture) != cudaSuccess) (void)cudaGetLastError();
+    if (capture == cudaStreamCaptureStatusNone) {
+      const Tensor c = at::empty({m, n}, a.options().requires_grad(false)), status = status_word(a.device().index());
+      check(api.linear(dtype_code(a.scalar_type()), layout, (int32_t)m, (int32_t)n, (int32_t)k, a.data_ptr(), a.stride(0), b.data_ptr(), b.stride(0),
+                       c.data_ptr(), n, status.data_ptr<int32_t>(), stream.stream()), "castle_linear");
+      return c;
+    }
+  }
+  return layout == 0 ? at::mm(a, b.t()) : layout == 1 ? at::mm(a, b) : at::mm(a.t(), b);
+}
 
 // Gradient node of a whole layer.  Autograd over the single operations (norm, two linear layers, the views between them
 // and the core) cost 250 us of host time per training step where the kernels of a small one take 120.
@@ -701,13 +729,13 @@ struct LayerBackward : public Node {
     const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
     const Tensor g = grads[0].reshape({rows, grads[0].size(-1)});
     if (need_combine)
-      result[2] = at::mm(g.t(), separate_merged ? ms : restored(saved.out16, {p.B, p.H, p.N, p.dp}, p.cdtype, dev).permute({0, 2, 1, 3}).reshape({rows, inner}));
+      result[2] = product(2, g, separate_merged ? ms : restored(saved.out16, {p.B, p.H, p.N, p.dp}, p.cdtype, dev).permute({0, 2, 1, 3}).reshape({rows, inner}), rows);
     if (!need_core) return result;
-    const Tensor dcore = at::mm(g, wc).view({p.B, p.N, p.H, p.d}).permute({0, 2, 1, 3});
+    const Tensor dcore = product(1, g, wc, rows).view({p.B, p.N, p.H, p.d}).permute({0, 2, 1, 3});
     const Tensor dqkv = core.backward(saved, dcore).view({rows, 6 * inner});
-    if (need_qkv) result[1] = at::mm(dqkv.t(), separate_h ? hs : xs.reshape({rows, dim}));
+    if (need_qkv) result[1] = product(2, dqkv, separate_h ? hs : xs.reshape({rows, dim}), rows);
     if (!(need_x || need_norm)) return result;
-    Tensor dh = at::mm(dqkv, wq);
+    Tensor dh = product(1, dqkv, wq, rows);
     if (!has_norm) {
       result[0] = dh.view(x_sizes);
       return result;
@@ -749,13 +777,13 @@ Tensor layer_native(const Tensor& x, const Layer& l, Options o) {
       check(api.rmsnorm_fwd(dtype_code(p.dtype), rows, (int32_t)dim, src.data_ptr(), l.norm.data_ptr(), norm_eps(l), h.data_ptr(),
                             o.need_grad ? rstd.data_ptr<float>() : nullptr, stream.stream()), "castle_rmsnorm_fwd");
     }
-    const Tensor packed = matmul_t(h, l.to_qkv).view({B, N, 6, l.heads, l.dim_head});
+    const Tensor packed = product(0, h, l.to_qkv, rows).view({B, N, 6, l.heads, l.dim_head});
     Inputs in;
     for (int i = 0; i < 6; ++i) in.t[i] = packed_desc(packed, i);
     in.keep = {packed};
     r = run_forward(p, std::move(in), o, x.device());
     merged = r.out.permute({0, 2, 1, 3}).view({rows, inner});
-    out = matmul_t(merged, l.combine).view({B, N, l.combine.size(0)});
+    out = product(0, merged, l.combine, rows).view({B, N, l.combine.size(0)});
   }
   if (!(o.need_grad || need_combine)) return out;
   auto node = std::shared_ptr<LayerBackward>(new LayerBackward(), torch::autograd::deleteNode);
@@ -879,7 +907,7 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
       check(api.rmsnorm_fwd(cp.dtype, B, (int32_t)dim, src.data_ptr(), l.norm.data_ptr(), norm_eps(l), h.data_ptr(), nullptr, stream.stream()),
             "castle_rmsnorm_fwd");
     }
-    keep = matmul_t(h, l.to_qkv);
+    keep = at::mm(h, l.to_qkv.t());
     packed = static_cast<char*>(keep.data_ptr());
   }
   castle_tensor_t news[6];
@@ -893,7 +921,7 @@ Tensor token_layer(const Tensor& x, const Layer& l, const Tensor* caches, int64_
   }
   const Tensor o = at::empty({B, inner}, x.options().requires_grad(false));
   launch_decode(cp, news, caches, o.data_ptr(), t, rotary, overlap, ws.data_ptr(), part, stream, use);
-  return matmul_t(o, l.combine).view({B, 1, l.combine.size(0)});
+  return at::mm(o, l.combine.t()).view({B, 1, l.combine.size(0)});
 }
 
 Tensor layer_decode(const Tensor& x, const Layer& l, const Tensor* caches, int64_t t, double scale, const Rotary& rotary) {
@@ -1208,7 +1236,7 @@ PyObject* py_bind(PyObject*, PyObject* d) {
     CASTLE_BIND(last_error); CASTLE_BIND(fwd_workspace_bytes); CASTLE_BIND(fwd); CASTLE_BIND(fwd_prefill);
     CASTLE_BIND(rmsnorm_fwd); CASTLE_BIND(rmsnorm_bwd_workspace_bytes); CASTLE_BIND(rmsnorm_bwd); CASTLE_BIND(bwd_workspace_bytes); CASTLE_BIND(bwd); CASTLE_BIND(transform); CASTLE_BIND(amax_scale);
     CASTLE_BIND(decode_workspace_bytes); CASTLE_BIND(decode_step_fused); CASTLE_BIND(token_linear_fits); CASTLE_BIND(token_linear);
-    CASTLE_BIND(token_layer_fits); CASTLE_BIND(token_layer_workspace_bytes); CASTLE_BIND(token_layer);
+    CASTLE_BIND(linear); CASTLE_BIND(token_layer_fits); CASTLE_BIND(token_layer_workspace_bytes); CASTLE_BIND(token_layer);
 #undef CASTLE_BIND
     PyObject* module = PyImport_ImportModule("torch.utils._device");
     Py_XDECREF(device_context);
