@@ -54,8 +54,8 @@ class ModuleCache(Cache):
     (a plain tuple of the caller's tensors, slices, a re-wrapped copy) is treated as read-only
     input and copied into fresh buffers first, so the caller's memory is never written."""
 
-    def __new__(cls, state: _CacheBuffers, length: int):
-        self = tuple.__new__(cls, state.views(length))
+    def __new__(cls, state: _CacheBuffers, length: int, views=None):
+        self = tuple.__new__(cls, state.views(length) if views is None else views)
         self._state, self._length = state, int(length)
         return self
 
@@ -118,15 +118,15 @@ class Castle(nn.Module):
         # 'b n (qkv h d) -> qkv b h n d', order qu, ku, vu, qc, kc, vc (reference :77,104); views, no copies
         return qkvs.view(b, n, 6, self.heads, self.dim_head).permute(2, 0, 3, 1, 4).unbind(0)
 
-    def _new_buffers(self, b, h, d, rows, dtype, device) -> _CacheBuffers:
+    def _new_buffers(self, b, h, d, rows, like) -> _CacheBuffers:
         cap = rows + max(self.cache_headroom, rows // 4)
-        return _CacheBuffers([torch.empty(b, h, cap, d, dtype=dtype, device=device) for _ in range(4)], 0)
+        return _CacheBuffers(_lib.host().new_caches(like, b, h, cap, d), 0)
 
     def _new_cache(self, like) -> _CacheBuffers:
         """The cache of a prompt of `like`'s batch size, length and type lives in buffers with spare rows so that decode
         steps can append in place.  The forward's kernels fill it themselves: from their operand tiles where those are
         the caller's values, otherwise in the pass that makes the operands."""
-        return self._new_buffers(like.shape[0], self.heads, self.dim_head, like.shape[1], like.dtype, like.device)
+        return self._new_buffers(like.shape[0], self.heads, self.dim_head, like.shape[1], like)
 
     def _state_in_place(self, cache, t):
         """The capacity buffers behind `cache` if row t can be appended to them as they are, else None."""
@@ -146,7 +146,7 @@ class Castle(nn.Module):
             return state
         # a foreign cache, a full buffer, or functional semantics asked for: copy into fresh buffers
         b, h, _, d = like.shape
-        fresh = self._new_buffers(b, h, d, t + 1, like.dtype, like.device)
+        fresh = self._new_buffers(b, h, d, t + 1, like)
         if t > 0:
             with torch.no_grad():
                 for buf, src in zip(fresh.bufs, cache):
@@ -255,4 +255,4 @@ class Castle(nn.Module):
         if not return_next_cache:
             return out
         state.length = seq_len
-        return out, ModuleCache(state, seq_len)
+        return out, ModuleCache(state, seq_len, views)

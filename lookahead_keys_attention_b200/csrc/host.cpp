@@ -1188,6 +1188,27 @@ PyObject* py_first_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
   });
 }
 
+// new_caches(like, B, H, capacity, d): four buffers of like's type and device (one by one from Python they cost 8 us of a prompt)
+PyObject* py_new_caches(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    arg_count(n, 5);
+    const at::TensorOptions o = arg_tensor(a[0]).options().requires_grad(false).memory_format(c10::nullopt);
+    const std::array<int64_t, 4> sizes{arg_int(a[1]), arg_int(a[2]), arg_int(a[3]), arg_int(a[4])};
+    PyObject* list = PyList_New(4);
+    for (Py_ssize_t i = 0; list && i < 4; ++i) {
+      PyObject* t = nullptr;
+      try {
+        t = THPVariable_Wrap(at::empty(sizes, o));
+      } catch (...) {
+        Py_DECREF(list);
+        throw;
+      }
+      PyList_SET_ITEM(list, i, t);
+    }
+    return list;
+  });
+}
+
 PyObject* py_status_word(PyObject*, PyObject* device) {
   return guarded([&] {
     const int64_t index = arg_int(device);
@@ -1257,6 +1278,7 @@ PyMethodDef methods[] = {{"bind", py_bind, METH_O, nullptr},
                          {"decode_packed", FAST(py_decode_packed), nullptr},
                          {"forward_chunks", FAST(py_forward_chunks), nullptr},
                          {"first_rows", FAST(py_first_rows), nullptr},
+                         {"new_caches", FAST(py_new_caches), nullptr},
                          {"status_word", py_status_word, METH_O, nullptr},
                          {"status_devices", py_status_devices, METH_NOARGS, nullptr},
                          {"release_workspaces", py_release_workspaces, METH_NOARGS, nullptr},
