@@ -9,6 +9,7 @@
 // Rows are split over `nsplit` CTAs per (batch, head); each CTA keeps a running
 // (max, sum, weighted value sum) and writes one partial, which a small second
 // kernel merges.
+#include <algorithm>
 #include <mutex>
 #include "common.cuh"
 #include "decode_row.cuh"
@@ -464,10 +465,36 @@ static int decode_nsplit(int BH, int t, int ctas_per_sm = CASTLE_DECODE_MIN_CTAS
 
 constexpr int kRingCtasPerSm = 4;
 
+// The ring kernel's split, bf16 us per step as the rule above has it / as this one does (pairs x positions x dim_head):
+// 400 x 4000 x 64 205 / 174, 200 x 4000 x 64 109 / 97, 128 x 4000 x 64 71 / 65, 256 x 4000 x 64 128 / 116, 1024 x 8191 x 128
+// 1654 / 1593, 700 x 8191 x 128 1148 / 1091, 64 x 8191 x 128 121 / 118; single runs of one size differ by 2 %.  A grid of one
+// wave merges in the kernel and pays a CTA's start once, so it is taken where it fills its wave to 85 % and a CTA's share of
+// the caches is at most 1 MB, or 2 MB where the wave is full: longer walks of a single wave drift apart (256 x 8191 x 128 431 us
+// against 411, 592 x 1500 x 128 181 against 187).  Otherwise shares of at most 1 MB, as few as come within 5 % of the fullest
+// last wave: chasing the last percent with finer shares cost more in starts than it gained.
+static int decode_nsplit_ring(int BH, int t, int row_bytes) {
+  const int64_t slots = 148 * kRingCtasPerSm, most = 1 << 20;
+  const int one = (int)std::min<int64_t>(64, slots / BH);
+  const int64_t filled = (int64_t)BH * one * 100;
+  if (one >= 1 && t / one >= 128 && filled >= slots * 85 && (int64_t)t * row_bytes <= (filled >= slots * 97 ? 2 : 1) * most * one) return one;
+  const int max_ns = std::max(1, std::min(64, t / 128));
+  auto eff = [&](int ns) {
+    const int64_t total = (int64_t)BH * ns, waves = (total + slots - 1) / slots;
+    return (double)total / (double)(waves * slots);
+  };
+  const int least = (int)std::min<int64_t>(max_ns, ((int64_t)t * row_bytes + most - 1) / most);
+  double best = 0.0;
+  for (int ns = std::max(1, least); ns <= max_ns; ++ns) best = std::max(best, eff(ns));
+  for (int ns = std::max(1, least); ns <= max_ns; ++ns)
+    if (eff(ns) >= best - 0.05) return ns;
+  return 1;
+}
+
 // The same for steps that leave SMs idle at 128 rows per CTA (few pairs, short caches): there a CTA's serial walk over
 // its rows is the time, so the rows are cut as fine as two ring stages (32 rows) while the grid stays within one wave.
-static int decode_nsplit_fine(int BH, int t, int ctas_per_sm) {
-  const int best = decode_nsplit(BH, t, ctas_per_sm);
+// row_bytes: a position's bytes in the four caches.
+static int decode_nsplit_fine(int BH, int t, int ctas_per_sm, int row_bytes) {
+  const int best = ctas_per_sm == kRingCtasPerSm ? decode_nsplit_ring(BH, t, row_bytes) : decode_nsplit(BH, t, ctas_per_sm);
   const int64_t slots = 148 * ctas_per_sm;
   if ((int64_t)BH * best >= slots) return best;
   int ns = (t + 31) / 32;
@@ -530,7 +557,8 @@ static bool decode_pairs_ok(const castle_problem_t* p) {
 extern "C" size_t castle_decode_workspace_bytes(const castle_problem_t* p, int32_t cache_len) {
   if (!p || !decode_pairs_ok(p)) return 0;
   int BH = p->batch * p->heads;
-  int ns = decode_nsplit_fine(BH, cache_len, CASTLE_DECODE_MIN_CTAS), ns_ring = decode_nsplit_fine(BH, cache_len, kRingCtasPerSm);
+  const int row_bytes = 4 * p->dim_head * elem_size(p->dtype);
+  int ns = decode_nsplit_fine(BH, cache_len, CASTLE_DECODE_MIN_CTAS, row_bytes), ns_ring = decode_nsplit_fine(BH, cache_len, kRingCtasPerSm, row_bytes);
   return (size_t)BH * (ns > ns_ring ? ns : ns_ring) * (2 + p->dim_head) * sizeof(float);
 }
 
@@ -572,7 +600,7 @@ extern "C" int castle_decode_step_fused(const castle_problem_t* p, int32_t cache
   dp.H = p->heads; dp.t = cache_len; dp.scale = p->scale; dp.status = status;
   const castle_tensor_t* caches[4] = {u_cache, qu_cache, kc_cache, vc_cache};
   const bool ring = status != nullptr && decode_use_ring(p->dim_head, caches);
-  dp.nsplit = decode_nsplit_fine(BH, cache_len, ring ? kRingCtasPerSm : CASTLE_DECODE_MIN_CTAS);
+  dp.nsplit = decode_nsplit_fine(BH, cache_len, ring ? kRingCtasPerSm : CASTLE_DECODE_MIN_CTAS, 4 * p->dim_head * elem_size(p->dtype));
   dp.rows_per_split = (cache_len + dp.nsplit - 1) / dp.nsplit;
   if (dp.rows_per_split < 1) dp.rows_per_split = 1;
   dp.part = (float*)workspace;
