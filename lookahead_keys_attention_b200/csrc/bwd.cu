@@ -602,7 +602,7 @@ extern "C" int castle_bwd(const castle_problem_t* p, const castle_tensor_t* qc, 
   int64_t rows = (int64_t)p->batch * p->heads * p->seq_len;
   // dim_head 128: the tile hand-over scratch follows the accumulators
   bp.tiles = (uint8_t*)workspace + acc_bytes;
-  bp.ntiles = 0; bp.bh0 = 0; bp.chunk_pairs = 0;
+  bp.ntiles = 0; bp.bh0 = 0; bp.chunk_pairs = 0; bp.kv_split = 0;
   if (p->dim_head == 128) {
     size_t fit = (workspace_bytes - acc_bytes) / pair_bytes;
     bp.chunk_pairs = (int)(fit < (size_t)(p->batch * p->heads) ? fit : (size_t)(p->batch * p->heads));

@@ -17,6 +17,8 @@
 //
 // Tiles of a step (I,K): A, then dZ | dSu | Gb; 32 KB each, as they lie in shared memory (128-byte swizzle).  The scratch is
 // bounded (kTileScratchLimit): the (batch, head) pairs run in chunks, one launch of each kernel per chunk.
+#include <algorithm>
+
 #include "bwd_common.cuh"
 
 namespace castle {
@@ -103,7 +105,17 @@ __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K)
 // 3.6 k cycles.  So the loads that the next step starts with (Qu, Ku, Vu, Qc) are issued before the reduces, and what is
 // staged over are the tiles that it needs last: dO, and Vc, which is loaded again for that (step 21.7 k cycles with the
 // loads behind the reduces, 18.9 k so, 17.1 k with the next Z under the staging and 16.2 k with the copy of dSu behind the next Qu).
-template <typename T>
+// Few pairs: the grid is little more than a wave, whose length is the walk of key block 0, while the mean walk is about half as
+// long.  So long walks are cut in two parts of about equal cost, a CTA each (kv_split).  The second part first peels the state down
+// to where it begins, in steps of Z, gate and W alone, some 0.3 of a step each: with a cut after x of n steps both cost x = n / 1.7.
+// Each part leaves its fp32 sums of dkc and dvc, as they lie in shared memory, and a kernel of its own adds the two.
+__host__ __device__ inline int kv_cut(int walk) { return (int)((float)walk * (1.f / 1.7f) + 0.5f); }
+constexpr uint32_t kPartSum = 4 * kPanelB, kPart = 2 * kPartSum;   // 128 x 128 floats in four panels of 32 columns; dkc and dvc
+__device__ __forceinline__ uint8_t* kv_part(const BwdParams& p, int bh, int K, int part) {
+  return reinterpret_cast<uint8_t*>(p.acc_dvu) + ((int64_t)(bh * p.kv_split + K) * 2 + part) * kPart;
+}
+
+template <typename T, bool CUT>
 __global__ void __launch_bounds__(kB128Threads, 1)
 castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
                         const __grid_constant__ CUtensorMap m_vc, const __grid_constant__ CUtensorMap m_qu,
@@ -114,7 +126,11 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
   constexpr uint32_t ID_KK = make_idesc(128, 128, FMT, false, false, false), ID_KM = make_idesc(128, 128, FMT, false, true, false),
                      ID_KM_NEG = make_idesc(128, 128, FMT, false, true, true), ID_MM = make_idesc(128, 128, FMT, true, true, false);
   constexpr float kLog2e = 1.4426950408889634f;
-  const int K = blockIdx.y, k0 = K * kBlkB, steps = p.nblk - K;
+  // CUT: two CTAs per key block in the grid; of a key block that is not cut the second has nothing to do
+  const int K = CUT ? blockIdx.y >> 1 : blockIdx.y, part = CUT ? blockIdx.y & 1 : 0, k0 = K * kBlkB, walk = p.nblk - K;
+  const bool cut = CUT && K < p.kv_split;
+  if (part && !cut) return;
+  const int begin = part ? kv_cut(walk) : 0, end = cut && !part ? kv_cut(walk) : walk;   // steps with scores; state alone before them
   B128_BEGIN(7 * kSq, 11, 512)
   uint8_t *s0 = smem, *s1 = s0 + kSq, *s2 = s1 + kSq, *s3 = s2 + kSq, *s4 = s3 + kSq, *s5 = s4 + kSq, *s6 = s5 + kSq;
   const uint32_t a0 = smem_u32(s0), a1 = smem_u32(s1), a2 = smem_u32(s2), a3 = smem_u32(s3), a4 = smem_u32(s4), a5 = smem_u32(s5),
@@ -135,14 +151,14 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     mbar_expect_tx(bar_z, 2 * kSq);
     load_op(s0, m_qu, bar_z, k0, h, b);
     load_op(s1, m_ku, bar_z, il, h, b);
-    mbar_expect_tx(bar_in, 2 * kSq);
-    load_op(s3, m_qc, bar_in, il, h, b);
+    mbar_expect_tx(bar_in, begin == 0 ? 2 * kSq : kSq);
+    if (begin == 0) load_op(s3, m_qc, bar_in, il, h, b);
     load_op(s2, m_vu, bar_in, il, h, b);
     mbar_expect_tx(bar_do, 2 * kSq);
     mbar_expect_tx(bar_res, kSq);
     load_op(s4, m_kc, bar_res, k0, h, b);
   }
-  if (reducer && elect_one()) load_panel((p.nblk - 1) * kBlkB);
+  if (reducer && elect_one()) load_panel((p.nblk - 1 - begin) * kBlkB);
   __syncwarp();
   {  // W starts as the forward's final state
     const float* src = p.w_state + ((int64_t)bh * p.N + krow) * 128 + c0;
@@ -168,10 +184,11 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
   __syncwarp();
   uint32_t ph_mma = 0;
   const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
-  for (int n = 0; n < steps; ++n) {
-    const uint32_t ph = n & 1;
+  for (int n = 0; n < end; ++n) {
+    const int m = n - begin;                    // of the steps with scores
+    const uint32_t ph = n & 1, ph_m = m & 1;    // barriers that complete in every step; in steps with scores
     const int I = p.nblk - 1 - n, i0 = I * kBlkB, irow = i0 + row;
-    const bool diag = I == K, rvalid = irow < p.N, more = n + 1 < steps;
+    const bool diag = I == K, rvalid = irow < p.N, more = n + 1 < end;
     uint8_t* const tile = step_tiles(p, I, K);
     uint8_t *const sK = n & 1 ? s2 : s1, *const sV = n & 1 ? s1 : s2;
     const uint32_t aK = n & 1 ? a2 : a1, aV = n & 1 ? a1 : a2;
@@ -198,6 +215,31 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     }
     B128_SYNC()
     B128_MARK(0, n, 3);
+    if (CUT && m < 0) {
+      // ---- W -= A Vu alone; the next step's tiles land over both once they are consumed, Qu stays
+      if (warp == 0 && elect_one()) {
+        mbar_wait(bar_in, ph, abortp);
+        tc_fence_after();
+        gemm_km_t<8>(tmem + C_W, aK, aV, ID_KM_NEG, true);
+        mma_commit(bar_w);
+      }
+      if (loader && elect_one()) {
+        mbar_wait(bar_w, ph, abortp);
+        mbar_expect_tx(bar_z, kSq);
+        load_op(sV, m_ku, bar_z, i0 - kBlkB, h, b);
+        mbar_expect_tx(bar_in, m == -1 ? 2 * kSq : kSq);
+        if (m == -1) load_op(s3, m_qc, bar_in, i0 - kBlkB, h, b);
+        load_op(sK, m_vu, bar_in, i0 - kBlkB, h, b);
+      }
+      if (warp == 0 && elect_one()) {
+        mbar_wait(bar_z, ph ^ 1, abortp);
+        tc_fence_after();
+        gemm_kk_t<2>(tmem + C_S, a0, aV, ID_KK, false);
+        mma_commit(bar_mma);
+      }
+      __syncwarp();
+      continue;
+    }
     // ---- T = Qc Vu^T;  W -= A Vu
     if (warp == 0 && elect_one()) {
       mbar_wait(bar_in, ph, abortp);
@@ -209,7 +251,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     }
     if (storer && elect_one()) { bulk_s2g(tile + kTileA, sK, kSq); bulk_commit(); }
     __syncwarp();
-    mbar_wait(bar_t, ph, abortp);
+    mbar_wait(bar_t, ph_m, abortp);
     tc_fence_after();
     B128_MARK(0, n, 4);
     {  // T over Vu, Wb over Qu
@@ -232,7 +274,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       mma_commit(bar_mma);
     }
     __syncwarp();
-    if (reducer && n > 0 && elect_one()) {   // the reduce of the step before has had time to read its panel, and all wait for Su anyway
+    if (reducer && m > 0 && elect_one()) {   // the reduce of the step before has had time to read its panel, and all wait for Su anyway
       bulk_wait_read0();
       load_panel(i0);
     }
@@ -252,7 +294,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       __syncthreads();
       // ---- Sc/scale = Qc Kc^T, while silu' is formed
       if (warp == 0 && elect_one()) {
-        if (n == 0) mbar_wait(bar_res, 0, abortp);
+        if (m == 0) mbar_wait(bar_res, 0, abortp);
         tc_fence_after();
         gemm_kk_t<2>(tmem + C_S, a3, a4, ID_KK, false);
         mma_commit(bar_mma);
@@ -297,11 +339,11 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     B128_MARK(0, n, 8);
     // ---- dP = dO Vc^T;  dvc += P^T dO
     if (warp == 0 && elect_one()) {
-      mbar_wait(bar_do, ph, abortp);
+      mbar_wait(bar_do, ph_m, abortp);
       tc_fence_after();
       gemm_kk_t<2>(tmem + C_S, a6, a5, ID_KK, false);
       mma_commit(bar_mma);
-      gemm_mm_t<8>(tmem + C_DVC, aV, a6, ID_MM, n > 0);
+      gemm_mm_t<8>(tmem + C_DVC, aV, a6, ID_MM, m > 0);
       mma_commit(bar_dv);
     }
     __syncwarp();
@@ -321,7 +363,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         w[j] = -du.x; w[j + 1] = -du.y;
       }
       store_row32<T>(sK, kPanelB, row, c0, v);   // dS
-      mbar_wait(bar_dv, ph, abortp);
+      mbar_wait(bar_dv, ph_m, abortp);
       store_row32<T>(s6, kPanelB, row, c0, w);   // dSu, over dO
     }
     B128_SYNC()
@@ -333,7 +375,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       mma_commit(bar_x0);
       gemm_km_t<8>(tmem + C_S, aK, a4, ID_KM, !diag);
       mma_commit(bar_x);
-      gemm_mm_t<8>(tmem + C_DKC, aK, a3, ID_MM, n > 0);
+      gemm_mm_t<8>(tmem + C_DKC, aK, a3, ID_MM, m > 0);
       mma_commit(bar_k);
     }
     if (loader && elect_one()) {
@@ -342,14 +384,14 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       mbar_expect_tx(bar_in, 2 * kSq);
       mbar_expect_tx(bar_do, 2 * kSq);
       load_op(sV, m_ku, bar_z, i0 - kBlkB, h, b);   // over P
-      mbar_wait(bar_x0, ph, abortp);
+      mbar_wait(bar_x0, ph_m, abortp);
       load_op(s0, m_qu, bar_z, k0, h, b);
       }
       bulk_s2g(tile + kTileDsu, s6, kSq);   // behind what the next product waits for
       bulk_commit();
     }
     __syncwarp();
-    mbar_wait(bar_x, ph, abortp);
+    mbar_wait(bar_x, ph_m, abortp);
     tc_fence_after();
     B128_MARK(0, n, 11);
     float v[32];
@@ -368,7 +410,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     // before the reduces, which loads would queue behind
     if (loader && elect_one()) {
        if (more) {
-        mbar_wait(bar_k, ph, abortp);
+        mbar_wait(bar_k, ph_m, abortp);
         load_op(s3, m_qc, bar_in, i0 - kBlkB, h, b);
         load_op(sK, m_vu, bar_in, i0 - kBlkB, h, b);
       }
@@ -382,26 +424,65 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     group_sync(1 + cc);
     B128_MARK(0, n, 13);
     if (reducer && elect_one()) {
-      mbar_wait(bar_k, ph, abortp);
+      mbar_wait(bar_k, ph_m, abortp);
       tma_reduce_add_3d(&m_acc_dqc, panel, cc * 32, i0, bh);
       bulk_commit();
     }
   }
   if ((reducer || storer || loader) && elect_one()) bulk_wait0();
   __syncwarp();
-  mbar_wait(bar_k, (uint32_t)(steps - 1) & 1u, abortp);
+  mbar_wait(bar_k, (uint32_t)(end - begin - 1) & 1u, abortp);
   tc_fence_after();
   {
     float v[32], w[32];
     tmem_ld32(trow + C_DKC + c0, v);
     tmem_ld32(trow + C_DVC + c0, w);
     tmem_ld_wait();
-    if (krow < p.N) {
+    if (cut) {   // over Qu to Qc, which every product has read
+      uint8_t *pk = s0 + cc * kPanelB, *pv = s2 + cc * kPanelB;
+      store_row32_f32(pk, row, v);
+      store_row32_f32(pv, row, w);
+      fence_async_smem();
+      group_sync(1 + cc);
+      if (reducer && elect_one()) {
+        uint8_t* dst = kv_part(p, bh, K, part) + cc * kPanelB;
+        bulk_s2g(dst, pk, kPanelB);
+        bulk_s2g(dst + kPartSum, pv, kPanelB);
+        bulk_commit();
+        bulk_wait0();
+      }
+      __syncwarp();
+    } else if (krow < p.N) {
       store_grad32<T>(grad_row<T>(p.dkc, b, h, krow, c0), v, p.scale);
       store_grad32<T>(grad_row<T>(p.dvc, b, h, krow, c0), w, 1.f);
     }
   }
   B128_END(512)
+}
+
+// dkc and dvc of the key blocks that were walked in two parts: a block of 256 threads sums 16 rows of both.
+template <typename T>
+__global__ void __launch_bounds__(256) castle_bwd128_parts_kernel(const BwdParams p) {
+  const int bh = p.bh0 + blockIdx.x, K = blockIdx.y, b = bh / p.H, h = bh % p.H;
+  const int row = blockIdx.z * 16 + (threadIdx.x >> 4), c8 = threadIdx.x & 15, krow = K * kBlkB + row;
+  overlap_wait();
+  if (krow >= p.N) return;
+  const uint32_t at = (c8 >> 2) * kPanelB, chunk = (c8 & 3) * 2;   // eight columns: two 16-byte chunks of a panel's row
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const uint32_t off = t * kPartSum + at + swz_off(row, chunk + q);
+      const float4 x = *reinterpret_cast<const float4*>(kv_part(p, bh, K, 0) + off), y = *reinterpret_cast<const float4*>(kv_part(p, bh, K, 1) + off);
+      v[4 * q] = x.x + y.x; v[4 * q + 1] = x.y + y.y; v[4 * q + 2] = x.z + y.z; v[4 * q + 3] = x.w + y.w;
+    }
+    const float mul = t == 0 ? p.scale : 1.f;
+    uint4 o;
+    o.x = Elem<T>::pack2(v[0] * mul, v[1] * mul); o.y = Elem<T>::pack2(v[2] * mul, v[3] * mul);
+    o.z = Elem<T>::pack2(v[4] * mul, v[5] * mul); o.w = Elem<T>::pack2(v[6] * mul, v[7] * mul);
+    *reinterpret_cast<uint4*>(grad_row<T>(t == 0 ? p.dkc : p.dvc, b, h, krow, c8 * 8)) = o;
+  }
 }
 
 // ------------------------------------------------------------------------------------------------ reverse state
@@ -691,6 +772,7 @@ castle_bwd128_dqu_kernel(const BwdParams p, const __grid_constant__ CUtensorMap 
 }
 
 // ------------------------------------------------------------------------------------------------ launches
+constexpr int kKvSplitMin = 7;   // shorter walks are not cut
 constexpr int64_t kTileScratchLimit = (int64_t)8 << 30;
 size_t bwd128_pair_bytes(int nblk) { return (size_t)nblk * (nblk + 1) / 2 * kStepTiles; }
 int bwd128_chunk_pairs(int BH, int nblk) {
@@ -702,10 +784,10 @@ int bwd128_chunk_pairs(int BH, int nblk) {
 template <typename T>
 static int launch_bwd128_t(const BwdParams& p, const CUtensorMap* in, cudaStream_t st) {
   constexpr int D = 128;
-  const void* kernels[4] = {(const void*)castle_bwd128_kv_kernel<T>,
-                            (const void*)castle_bwd128_reverse_kernel<T>, (const void*)castle_bwd128_la_kernel<T>, (const void*)castle_bwd128_dqu_kernel<T>};
-  const size_t smem[4] = {kB128Smem, 6 * kSq + 256, kB128Smem, 6 * kSq + 256};
-  for (int i = 0; i < 4; ++i) {
+  const void* kernels[5] = {(const void*)castle_bwd128_kv_kernel<T, false>, (const void*)castle_bwd128_reverse_kernel<T>,
+                            (const void*)castle_bwd128_la_kernel<T>, (const void*)castle_bwd128_dqu_kernel<T>, (const void*)castle_bwd128_kv_kernel<T, true>};
+  const size_t smem[5] = {kB128Smem, 6 * kSq + 256, kB128Smem, 6 * kSq + 256, kB128Smem};
+  for (int i = 0; i < 5; ++i) {
     cudaError_t e = cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[i]);
     if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
   }
@@ -722,13 +804,21 @@ static int launch_bwd128_t(const BwdParams& p, const CUtensorMap* in, cudaStream
     q.bh0 = bh0;
     q.ntiles = (int64_t)p.nblk * (p.nblk + 1) / 2;
     const int pairs = BH - bh0 < chunk ? BH - bh0 : chunk;
-    const dim3 grid(pairs, p.nblk);
+    // Key blocks whose walks are cut: the longer half, where the steps per SM are less than half the longest walk.  us of the four
+    // kernels, uncut / cut: 4 pairs x 4096 positions 441 / 377 (0.45), 8 x 2048 237 / 220 (0.46), 2 x 900 122 / 112 (0.05),
+    // 12 x 1500 187 / 187 (0.53); above that the repeated state costs more than the balance gains: 16 x 1333 182 / 197 (0.65), 8 x
+    // 3000 355 / 370 (0.68).
+    const float load = (float)pairs * (float)(p.nblk + 1) * (0.5f / 148.f);
+    q.kv_split = p.nblk >= kKvSplitMin && load < 0.5f ? std::max(0, std::min(p.nblk + 1 - kKvSplitMin, p.N / (2 * kBlkB))) : 0;
+    const dim3 grid(pairs, p.nblk), kv_grid(pairs, q.kv_split ? 2 * p.nblk : p.nblk);
     // in[]: qc, kc, vc, qu, ku, vu, dout
     // each starts while the one before it ends
-    cudaError_t e = launch_kernel(castle_bwd128_kv_kernel<T>, grid, kB128Threads, smem[0], st, true, q, in[0], in[1], in[2], in[3], in[4], in[5], in[6], acc);
+    cudaError_t e = launch_kernel(q.kv_split ? castle_bwd128_kv_kernel<T, true> : castle_bwd128_kv_kernel<T, false>, kv_grid, kB128Threads, smem[0], st, true, q, in[0], in[1], in[2], in[3], in[4], in[5], in[6], acc);
     if (e == cudaSuccess && p.nblk > 1) e = launch_kernel(castle_bwd128_reverse_kernel<T>, dim3(pairs, p.nblk - 1), kB128Threads, smem[1], st, true, q, in[0]);
     if (e == cudaSuccess) e = launch_kernel(castle_bwd128_la_kernel<T>, grid, kB128Threads + 32, smem[2], st, true, q, in[0], in[3], in[5]);
     if (e == cudaSuccess) e = launch_kernel(castle_bwd128_dqu_kernel<T>, grid, 128, smem[3], st, true, q, in[4]);
+    if (e == cudaSuccess && q.kv_split)
+      e = launch_kernel(castle_bwd128_parts_kernel<T>, dim3(pairs, q.kv_split, kBlkB / 16), 256, 0, st, true, q);
     if (e != cudaSuccess) return cuda_fail(e, "castle_bwd launch");
   }
   ev_stop(CASTLE_KERNEL_BWD, st);

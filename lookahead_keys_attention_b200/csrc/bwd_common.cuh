@@ -22,6 +22,7 @@ struct BwdParams {
   int64_t ntiles;        // query-block x key-block pairs per (batch, head) pair
   int bh0;               // dim_head 128: first (batch, head) pair of this launch (the pairs run in chunks)
   int chunk_pairs;       // dim_head 128: pairs per chunk (what the caller's scratch holds)
+  int kv_split;          // dim_head 128: key blocks [0, kv_split) are walked in two parts; their sums use acc_dvu and acc_dku
   castle_tensor_t out, dout;
   castle_tensor_t dqc, dkc, dvc, dqu, dku, dvu;
   int32_t* status;
