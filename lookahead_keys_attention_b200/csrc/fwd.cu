@@ -18,6 +18,7 @@
 // partial (row max, row sum, P@Vc) and a second kernel merges the partials of a
 // query block.  After the last step W_K is exactly U[K], the lookahead keys the
 // decode cache stores, and (unrounded) the state the backward starts from.
+#include <algorithm>
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -64,10 +65,8 @@ __device__ inline int walk_cut(int walk, int nseg, int seg) {
 // Optional phase timing (debug builds only): thread 0 of CTA (0,0) stores clock64() at each phase
 // boundary of its first steps into the soft-max partial buffer's tail, which the host dumps.
 #ifdef CASTLE_PHASE_TIMING
-#define PHASE_MARK(i) do { if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && tstep < 8) p.timing[tstep * 16 + (i)] = clock64(); } while (0)
 #define PIPE_MARK(i) do { if ((tid & 31) == 0 && (tid == 0 || tid == 256) && blockIdx.x == 0 && blockIdx.y == 0 && I - I_begin < 16) p.timing[(I - I_begin) * 16 + (i)] = clock64(); } while (0)
 #else
-#define PHASE_MARK(i) do { } while (0)
 #define PIPE_MARK(i) do { } while (0)
 #endif
 
@@ -126,7 +125,34 @@ __device__ __forceinline__ void store_u32(void* base, int dtype, int64_t off, co
 
 // A masked T tile in global memory: [16 chunks of 8 columns][128 rows] x 16 bytes, so that a warp's access is contiguous.
 constexpr int64_t kTmTile = 16 * kBlk;   // in uint4
-constexpr int kTmBlocks = 4;             // from so many query blocks on the tiles are computed once, up front
+constexpr int kTmBlocks = 8;             // with fewer query blocks they never pay; from here on there is room for them (so that the scratch is linear in the pairs)
+
+// The forward's plan for a problem: parts per walk, whether the masked T tiles are computed once, up front, and the kernel.
+struct FwdPlan { int nseg; bool ahead, persistent; };
+static FwdPlan fwd_plan(int64_t pairs, int64_t nblk, int dim_head) {
+  FwdPlan f;
+  // Few pairs: the grid is one wave whose length is the walk of key block 0, while the mean walk is half as long or, with
+  // idle SMs, still less.  `load` = steps per SM over the longest walk.  us uncut / 2 / 3 parts: 4 pairs x 16 blocks at
+  // dim_head 128 74 / 60 / 52 (load 0.23), 4 x 12 44 / 37 / 34 (0.18), 8 x 12 44 / 37 / 40 (0.35), 4 x 32 100 / 78 / 88 (0.45), 16 x 11
+  // 43 / 46 / 52 (0.65), 8 x 32 103 / 138 / 166 (0.89).
+  const float load = (float)pairs * (float)(nblk + 1) * (0.5f / 148.f);
+  f.nseg = nblk < kSplitMin || load >= 0.6f ? 1 : load >= 0.3f ? 2 : 3;
+  // The tiles cost a launch of 8 us and 14 ns a tile (64 KB through memory); a step that reads one instead of computing it is
+  // 0.52 us shorter at dim_head 64 (a product less in the chain) and 0.37 at 128.  The steps that count are those of the busiest SM:
+  // their mean, or the longest walk (the first part has 0.65 and 0.54 of its steps).  us of a forward with / without the tiles,
+  // pairs x blocks: dim_head 64 512 x 4 228 / 211, 128 x 8 182 / 182, 64 x 10 147 / 144, 128 x 13 374 / 380, 64 x 17 306 / 321, 8 x 16
+  // 86 / 83, 16 x 17 109 / 106, 8 x 24 126 / 128, 4 x 32 116 / 115, 8 x 32 146 / 152; dim_head 128 256 x 4 213 / 195, 128 x 8 279 / 267,
+  // 8 x 11 81 / 73, 16 x 16 130 / 127, 64 x 16 416 / 413, 16 x 32 366 / 377.
+  const float longest = (float)nblk * (f.nseg == 1 ? 1.f : f.nseg == 2 ? 0.65f : 0.54f);
+  const float steps = std::max(longest, load * (float)nblk);
+  f.ahead = nblk >= kTmBlocks && steps * (dim_head == 64 ? 0.52f : 0.37f) > 8.f + 0.014f * (float)(pairs * nblk);
+  // A CTA that takes one walk after the other covers their starts and ends, but its steps are some 4 % longer (it looks up
+  // what comes next), so it is for short walks, and the longer they are the more of them there must be.  us of the kernel, walk after walk / a
+  // CTA per walk, pairs x blocks: 128 x 8 124 / 145, 48 x 12 103 / 110, 128 x 13 286 / 314, 128 x 17 460 / 485, 128 x 20 622 / 648, 64 x 24
+  // 442 / 447, 64 x 32 748 / 739; few: 32 x 8 45 / 47, 24 x 8 42 / 40, 40 x 12 102 / 104, 24 x 20 131 / 129, 20 x 24 158 / 148, 8 x 24 88 / 78.
+  f.persistent = dim_head == 64 && f.nseg == 1 && nblk <= 24 && (9.f * load >= (float)nblk || nblk < kSplitMin);
+  return f;
+}
 
 template <typename T, int D, bool TM>
 __global__ void __launch_bounds__(kFwdThreads, 1)
@@ -502,6 +528,409 @@ castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_
   if (tid == 0 && *abort_flag) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
 }
 
+// ---------------------------------------------------------------------------------------------
+// The pipeline above at dim_head 64, for CTAs that stay on their SM and walk one key block after the other: X goes on to the next
+// walk while Y is still on the last block of the one before, so that start and end of a walk, 7 to 9 us of a CTA that has but
+// one (tensor memory, first tiles, the fill of the pipeline, the last block), are covered.  A step is bound by its chain, as above.
+// B=16 N=1024 H=8 146 -> 124 us, B=8 N=2049 H=16 484 -> 460 us, B=64 N=512 H=8 182 -> 165 us against a CTA (or two per SM, below seven
+// blocks) for each walk.
+//
+// Tensor memory: W | R1 (Z) | R2 (Su) | R3 (Sc, issued by Y as soon as these columns are free again, then P as packed pairs and, in
+// its upper half, P @ Vc) | Tm.  Shared memory: Qu, Kc, Vc of the walk, the 16-bit copy of W, and two buffers each of Ku, Vu, Qc
+// and the gate, filled a step ahead.  n counts a CTA's steps, i its walks; a barrier's parity is its count's.
+struct Walk64 { int bh, K; };   // key block K of pair bh over query blocks [K, nblk)
+// The steps of a CTA, walk after walk.  The walks are ordered from the longest to the shortest (key blocks upwards, each over all
+// pairs) and dealt out to the CTAs back and forth, so that every CTA gets about as many steps.
+struct Steps64 {
+  Walk64 w;
+  int I, ahead, back;   // places from this walk to the next, and from that to the one behind
+  bool ok;
+  __device__ __forceinline__ Steps64(const FwdParams& p) {
+    const int pairs = p.B * p.H;
+    I = w.K = blockIdx.x / pairs;
+    w.bh = blockIdx.x % pairs;
+    ok = w.K < p.nblk;
+    ahead = 2 * (int)(gridDim.x - blockIdx.x) - 1;
+    back = 2 * blockIdx.x + 1;
+  }
+  __device__ __forceinline__ void advance(const FwdParams& p) {
+    if (++I < p.nblk) return;
+    const int t = ahead, pairs = p.B * p.H;
+    w.bh += ahead;
+    ahead = back;
+    back = t;
+    while (w.bh >= pairs && w.K < p.nblk) { w.bh -= pairs; ++w.K; }
+    ok = w.K < p.nblk;
+    I = w.K;
+  }
+  __device__ __forceinline__ bool first() const { return I == w.K; }
+};
+
+template <typename T, bool TM>
+__global__ void __launch_bounds__(kFwdThreads, 1)
+castle_fwd_pipe64_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
+                         const __grid_constant__ CUtensorMap m_vc, const __grid_constant__ CUtensorMap m_qu,
+                         const __grid_constant__ CUtensorMap m_ku, const __grid_constant__ CUtensorMap m_vu,
+                         const __grid_constant__ CUtensorMap m_quc, const __grid_constant__ CUtensorMap m_kcc,
+                         const __grid_constant__ CUtensorMap m_vcc) {
+  using L = FwdPipe<64>;
+  constexpr int D = 64;
+  constexpr uint32_t OPB = L::OPB;
+  constexpr uint32_t C_W = 0, C_R1 = D, C_R2 = D + 128, C_R3 = D + 256, C_O = C_R3 + 64, C_TM = C_R3 + 128;
+  constexpr int FMT = Elem<T>::fmt;
+  constexpr uint32_t ID_SQ = make_idesc(128, 128, FMT, false, false, false);
+  constexpr uint32_t ID_D = make_idesc(128, D, FMT, false, true, false);
+  constexpr float kLog2e = 1.4426950408889634f;
+
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t *sQu = smem, *sKc = sQu + OPB, *sVc = sKc + OPB, *sWb = sVc + OPB, *sStream = sWb + OPB;
+  auto sA = [&](uint32_t n) { return sStream + (n & 1) * 32768; };
+  auto sKu = [&](uint32_t n) { return sStream + 65536 + (n & 1) * OPB; };
+  auto sVu = [&](uint32_t n) { return sStream + 65536 + 2 * OPB + (n & 1) * OPB; };
+  auto sQc = [&](uint32_t n) { return sStream + 65536 + 4 * OPB + (n & 1) * OPB; };
+  float (*red_max)[kBlk] = reinterpret_cast<float (*)[kBlk]>(smem + L::kRed);
+  float (*red_sum)[kBlk] = red_max + 2;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
+  // loads: Qu, Kc, Vc of a walk; Vu and Qc of a step with Ku of the next (two, alternating); Ku of the first step
+  uint64_t *bar_qu = bars, *bar_kc = bars + 1, *bar_vc = bars + 2, *bar_in = bars + 3, *bar_ku0 = bars + 5;
+  uint64_t *bar_z = bars + 6, *bar_t = bars + 7, *bar_w = bars + 8, *bar_s = bars + 9, *bar_o = bars + 10;
+  uint64_t* bar_r = bars + 11;   // Y has Su in registers (one arrival per warp)
+  uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + 14);
+  int* abort_flag = reinterpret_cast<int*>(bars + 15);
+  volatile int* abortp = abort_flag;
+
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: uniform for the compiler, too
+  const int quarter = warp & 3, grp = (warp >> 2) & 1;   // TMEM lanes 32 * quarter.., columns 64 * grp.. of a score tile
+  const int row = quarter * 32 + lane, cbase = grp * 64;
+  Steps64 c(p);
+  if (!c.ok) return;
+
+  if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need 1024-byte alignment
+    if (tid == 0) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
+    return;
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 11; ++i) mbar_init(bars + i, bars + i == bar_s ? 2 : 1);   // the scores: Su by X, Sc by Y
+    mbar_init(bar_r, 8);
+    mbar_fence_init();
+    *abort_flag = 0;
+    tma_prefetch_desc(&m_qc); tma_prefetch_desc(&m_ku); tma_prefetch_desc(&m_vu);
+  }
+  if (warp == 0) { tmem_alloc(tmem_base_s, 512); tmem_relinquish(); }
+  overlap_wait();   // launched while the T tiles are being written
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_base_s;
+  const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
+  const uint32_t aQu = smem_u32(sQu), aKc = smem_u32(sKc), aVc = smem_u32(sVc), aWb = smem_u32(sWb);
+  const float half_scale = 0.5f * p.scale;
+
+  auto load = [&](uint8_t* dst, const CUtensorMap& map, uint64_t* bar, int block, int bh) {
+    tma_load_4d(dst, &map, bar, 0, block * kBlk, bh % p.H, bh / p.H);
+  };
+  // what step n reads, and Ku of the step behind it
+  auto load_step = [&](uint32_t n, const Steps64& s) {
+    Steps64 next = s;
+    next.advance(p);
+    uint64_t* bar = bar_in + (n & 1);
+    mbar_expect_tx(bar, OPB * (2 + next.ok));
+    if (next.ok) load(sKu(n + 1), m_ku, bar, next.I, next.w.bh);
+    load(sVu(n), m_vu, bar, s.I, s.w.bh);
+    load(sQc(n), m_qc, bar, s.I, s.w.bh);
+  };
+  // A walk's resident tile; in a prompt it is also what a decode cache holds for the key block, and is stored there as it is.  One
+  // lane does all of it for a tile, so that it knows when the store has read the tile that the next load overwrites.
+  auto load_resident = [&](uint8_t* dst, const CUtensorMap& map, uint64_t* bar, const Walk64& w) {
+    if (p.store_caches) bulk_wait_read0();
+    mbar_expect_tx(bar, OPB);
+    load(dst, map, bar, w.K, w.bh);
+  };
+  auto resident = [&](uint8_t* tile, const CUtensorMap& cache, uint64_t* bar, uint32_t i, const Walk64& w) {
+    mbar_wait_lazy_abort(bar, i & 1, abortp);
+    if (p.store_caches && !*abortp) {
+      tma_store_4d(&cache, tile, 0, w.K * kBlk, w.bh % p.H, w.bh / p.H);
+      bulk_commit();
+    }
+  };
+  // one polling lane per warp (see castle_fwd_pipe_kernel)
+  auto wait_warp = [&](uint64_t* bar, uint32_t parity) { if (elect_one()) mbar_wait_lazy_abort(bar, parity & 1, abortp); __syncwarp(); tc_fence_after(); };
+
+  if (warp < 8) {
+    // ============================================================ X: lookahead stage
+    uint32_t n = 0, i = 0;
+    if (warp == 0 && elect_one()) {
+      load_resident(sQu, m_qu, bar_qu, c.w);
+      mbar_expect_tx(bar_ku0, OPB);
+      load(sKu(0), m_ku, bar_ku0, c.w.K, c.w.bh);
+      load_step(0, c);
+      resident(sQu, m_quc, bar_qu, 0, c.w);
+      mbar_wait(bar_ku0, 0, abortp);
+      tc_fence_after();
+      gemm_kk_t<1>(tmem + C_R1, aQu, smem_u32(sKu(0)), ID_SQ, false);
+      mma_commit(bar_z);
+    }
+    Walk64 last{};
+#pragma unroll 1
+    while (c.ok) {
+      Steps64 next = c;
+      next.advance(p);
+      const bool diag = c.first(), more = next.ok;
+      const uint32_t aA = smem_u32(sA(n)), aVu = smem_u32(sVu(n)), aQc = smem_u32(sQc(n)), aKn = smem_u32(sKu(n + 1));
+
+      uint4 tq[8];   // this thread's 64 values of the masked T, on their way during the gate
+      if (TM) {
+        const uint4* src = p.tm + ((int64_t)c.w.bh * p.nblk + c.I) * kTmTile + (cbase / 8) * kBlk + row;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) tq[q] = __ldg(src + q * kBlk);
+      }
+      // ---- gate A = sigmoid(scale * Z), kept for j > k (rows k, columns j)
+      wait_warp(bar_z, n);
+      if (more && next.first() && warp == 0 && elect_one()) load_resident(sQu, m_qu, bar_qu, next.w);   // this Z was the last with the old one
+      __syncwarp();
+      {
+        float v[2][32];
+        tmem_ld32(trow + C_R1 + cbase, v[0]);
+        tmem_ld32(trow + C_R1 + cbase + 32, v[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float2 a = sigmoid2(make_float2(v[q][j], v[q][j + 1]), half_scale);
+            v[q][j] = a.x; v[q][j + 1] = a.y;
+          }
+          if (diag) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[q][j] = (cbase + q * 32 + j > row) ? v[q][j] : 0.f;
+          }
+          store_row32<T>(sA(n), kPanelBytes, row, cbase + q * 32, v[q]);
+        }
+      }
+      // Y has the scores of the step before, so its products are done: its buffers are filled for the next one
+      if (n > 0) wait_warp(bar_r, n - 1);
+      if (more && warp == 1 && elect_one()) load_step(n + 1, next);
+      __syncwarp();
+      if (diag && n > 0) {   // W is U of the walk before
+        if (p.u_out.ptr != nullptr || p.w_state != nullptr) {
+          const int c0 = grp * 32, krow = last.K * kBlk + row;
+          float v[32];
+          tmem_ld32(trow + C_W + c0, v);
+          tmem_ld_wait();
+          if (krow < p.N) {   // (the load is the whole warp's)
+            if (p.w_state != nullptr) store_u32(p.w_state, CASTLE_F32, ((int64_t)last.bh * p.N + krow) * D + c0, v);
+            if (p.u_out.ptr != nullptr)
+              store_u32(p.u_out.ptr, p.u_dtype, last.bh / p.H * p.u_out.stride_b + last.bh % p.H * p.u_out.stride_h + (int64_t)krow * p.u_out.stride_n + c0, v);
+          }
+        }
+      } else {   // the 16-bit copy of W (before this step's update)
+        const int c0 = grp * 32;
+        float v[32];
+        tmem_ld32(trow + C_W + c0, v);
+        tmem_ld_wait();
+        store_row32<T>(sWb, kPanelBytes, row, c0, v);
+      }
+      if (TM) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) tmem_st16(trow + C_TM + cbase / 2 + q * 16, reinterpret_cast<const uint32_t*>(tq + 4 * q));
+        tmem_st_wait();
+      }
+      fence_async_smem();
+      tc_fence_before();
+      // what the products below read is waited for here, by another warp than the issuing one
+      if (warp == 1 && elect_one()) mbar_wait_lazy_abort(bar_in + (n & 1), (n >> 1) & 1, abortp);
+      __syncwarp();
+      sync_x();
+      if (!TM) {
+        // ---- T[I,I] = Qc[I] @ Vu[I]^T over Z, masked (j <= i) into packed pairs
+        if (warp == 0 && elect_one()) {
+          tc_fence_after();
+          gemm_kk_t<1>(tmem + C_R1, aQc, aVu, ID_SQ, false);
+          mma_commit(bar_t);
+        }
+        wait_warp(bar_t, n);
+        float v[2][32];
+        tmem_ld32_lower(trow + C_R1 + cbase, row, cbase, v[0]);
+        tmem_ld32_lower(trow + C_R1 + cbase + 32, row, cbase + 32, v[1]);
+        tmem_st_packed32<T>(trow + C_TM + cbase / 2, v[0]);
+        tmem_st_packed32<T>(trow + C_TM + cbase / 2 + 16, v[1]);
+        tmem_st_wait();
+        tc_fence_before();
+        sync_x();
+      }
+
+      // ---- Z of the next step;  W_K += A @ Vu[I];  Su/scale = Qc[I] @ Wb^T + Tm @ A^T
+      if (warp == 0 && elect_one()) {
+        tc_fence_after();
+        if (more) {   // R1 has been read: Z first, the next gate waits for nothing else
+          if (next.first()) { resident(sQu, m_quc, bar_qu, i + 1, next.w); tc_fence_after(); }
+          gemm_kk_t<1>(tmem + C_R1, aQu, aKn, ID_SQ, false);
+          mma_commit(bar_z);
+        }
+        gemm_km_t<8>(tmem + C_W, aA, aVu, ID_D, !diag);
+        mma_commit(bar_w);
+        if (!diag) gemm_kk_t<1>(tmem + C_R2, aQc, aWb, ID_SQ, false);
+        gemm_tk_t<2>(tmem + C_R2, tmem + C_TM, aA, ID_SQ, !diag);
+        mma_commit(bar_s);
+        if (n == 0) {   // the first Sc (later ones are Y's)
+          mbar_wait(bar_kc, 0, abortp);
+          tc_fence_after();
+          gemm_kk_t<1>(tmem + C_R3, aQc, aKc, ID_SQ, false);
+          mma_commit(bar_s);
+        }
+      }
+      __syncwarp();
+      if (more && next.first()) ++i;
+      last = c.w;
+      ++n;
+      c = next;
+    }
+    // ---- the state of the last walk
+    if (p.u_out.ptr != nullptr || p.w_state != nullptr) {
+      wait_warp(bar_w, n - 1);
+      const int c0 = grp * 32, krow = last.K * kBlk + row;
+      float v[32];
+      tmem_ld32(trow + C_W + c0, v);
+      tmem_ld_wait();
+      if (krow < p.N) {
+        if (p.w_state != nullptr) store_u32(p.w_state, CASTLE_F32, ((int64_t)last.bh * p.N + krow) * D + c0, v);
+        if (p.u_out.ptr != nullptr)
+          store_u32(p.u_out.ptr, p.u_dtype, last.bh / p.H * p.u_out.stride_b + last.bh % p.H * p.u_out.stride_h + (int64_t)krow * p.u_out.stride_n + c0, v);
+      }
+    }
+    if (p.store_caches && warp == 0 && elect_one()) bulk_wait0();
+  } else {
+    // ============================================================ Y: soft-max stage
+    const float sl2 = p.scale * kLog2e;
+    uint32_t n = 0, i = 0;
+    // Kc by warp 8, which issues its product; Vc by warp 9
+    auto issue_sc = [&](uint32_t step) {   // Sc/scale = Qc[I] @ Kc[K]^T
+      tc_fence_after();
+      gemm_kk_t<1>(tmem + C_R3, smem_u32(sQc(step)), aKc, ID_SQ, false);
+      mma_commit(bar_s);
+    };
+    if (warp == 8 && elect_one()) {
+      load_resident(sKc, m_kc, bar_kc, c.w);
+      resident(sKc, m_kcc, bar_kc, 0, c.w);
+    }
+    if (warp == 9 && elect_one()) load_resident(sVc, m_vc, bar_vc, c.w);
+    __syncwarp();
+    bool first = true;   // block of a walk
+#pragma unroll 1
+    while (c.ok) {
+      Steps64 next = c;
+      next.advance(p);
+      const bool diag = c.first(), turn = next.ok && next.first();   // turn: the last block of a walk, and another one follows
+      const int irow = c.I * kBlk + row;
+      wait_warp(bar_s, n);
+      if (turn && warp == 8 && elect_one()) load_resident(sKc, m_kc, bar_kc, next.w);   // these scores were the last with the old one
+      __syncwarp();
+      // S/scale = Sc/scale - silu(Su)/scale (rows i, columns k); Su comes in pieces of 16 columns, one ahead of the arithmetic
+      float s[2][32];
+      {
+        float w[2][16];
+        tmem_ld16(trow + C_R2 + cbase, w[0]);
+        tmem_ld32(trow + C_R3 + cbase, s[0]);
+        tmem_ld32(trow + C_R3 + cbase + 32, s[1]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (q < 3) tmem_ld16(trow + C_R2 + cbase + 16 * (q + 1), w[(q + 1) & 1]);
+          float* sq = &s[q >> 1][(q & 1) * 16];
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {
+            const float2 u = make_float2(w[q & 1][j], w[q & 1][j + 1]);
+            const float2 x = fma2(u, neg_sigmoid2(u, half_scale), make_float2(sq[j], sq[j + 1]));
+            sq[j] = x.x; sq[j + 1] = x.y;
+          }
+          if (q < 3) tmem_ld_wait();
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_r);   // Su is in registers
+      if (diag) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+          for (int j = 0; j < 32; ++j) s[q][j] = (cbase + q * 32 + j <= row) ? s[q][j] : -INFINITY;
+      }
+      float mx = s[0][0];
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int j = 0; j < 32; ++j) mx = fmaxf(mx, s[q][j]);
+      red_max[grp][row] = mx;
+      sync_pair(7 + quarter);
+      tc_fence_after();
+      mx = fmaxf(mx, red_max[grp ^ 1][row]);   // column 0 is never masked, so the maximum is finite
+      const float mb = mx * sl2;
+      float2 lsum = splat(0.f);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 x = fma2(make_float2(s[q][j], s[q][j + 1]), splat(sl2), splat(-mb));
+          // exp(scale*v - max); masked entries give 0.  An eighth of them, where the special-function unit is the busiest (53 %), is
+          // computed on the FMA pipe: 752 -> 746 us at B=4 N=4096 H=16.
+          const float2 e = j % 16 == 0 ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));
+          s[q][j] = e.x;
+          s[q][j + 1] = e.y;
+          lsum = add2(lsum, make_float2(s[q][j], s[q][j + 1]));
+        }
+        tmem_st_packed32<T>(trow + C_R3 + cbase / 2 + q * 16, s[q]);   // P over Sc, which everybody has read
+      }
+      red_sum[grp][row] = lsum.x + lsum.y;
+      tmem_st_wait();
+      tc_fence_before();
+      if (first && warp == 9 && elect_one()) resident(sVc, m_vcc, bar_vc, i, c.w);
+      __syncwarp();
+      sync_y();
+      // ---- O_partial = P @ Vc[K]
+      if (warp == 8 && elect_one()) {
+        tc_fence_after();
+        gemm_tm_t<8>(tmem + C_O, tmem + C_R3, aVc, ID_D, false);
+        mma_commit(bar_o);
+      }
+      const int64_t tile = (int64_t)c.w.bh * tri(p.nblk) + tri(c.I) + c.w.K;
+      if (grp == 0 && irow < p.N)
+        reinterpret_cast<float2*>(p.part_ml)[tile * kBlk + row] = make_float2(mx * p.scale, red_sum[0][row] + red_sum[1][row]);
+      if (next.ok && warp == 9 && elect_one()) mbar_wait_lazy_abort(bar_in + ((n + 1) & 1), ((n + 1) >> 1) & 1, abortp);   // Qc for the next Sc
+      wait_warp(bar_o, n);
+      float o[32];
+      tmem_ld32(trow + C_O + grp * 32, o);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (turn && warp == 9 && elect_one()) load_resident(sVc, m_vc, bar_vc, next.w);
+      __syncwarp();
+      sync_y();
+      if (next.ok && warp == 8 && elect_one()) {   // over P and P @ Vc, which everybody has read
+        if (turn) resident(sKc, m_kcc, bar_kc, i + 1, next.w);
+        issue_sc(n + 1);
+      }
+      __syncwarp();
+      if (irow < p.N) {
+        uint4* dst = reinterpret_cast<uint4*>(p.part_o) + (tile * (D / 8) + grp * 4) * kBlk + row;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          dst[j * kBlk] = make_uint4(Elem<T>::pack2(o[8 * j], o[8 * j + 1]), Elem<T>::pack2(o[8 * j + 2], o[8 * j + 3]),
+                                     Elem<T>::pack2(o[8 * j + 4], o[8 * j + 5]), Elem<T>::pack2(o[8 * j + 6], o[8 * j + 7]));
+      }
+      if (turn) ++i;
+      first = turn;
+      ++n;
+      c = next;
+    }
+    if (p.store_caches && (warp == 8 || warp == 9) && elect_one()) bulk_wait0();
+    __syncwarp();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 512);
+  if (tid == 0 && *abort_flag) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
+}
+
 // The masked T tiles: one CTA of 128 threads (a row each) per query block.
 template <typename T, int D>
 __global__ void __launch_bounds__(128) castle_fwd_t_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc,
@@ -556,355 +985,6 @@ __global__ void __launch_bounds__(128) castle_fwd_t_kernel(const FwdParams p, co
   if (tid == 0 && abort_flag) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
 }
 
-// ---------------------------------------------------------------------------------------------
-// dim_head 64, many short walks (see launch_fwd): a leaner CTA (256 threads, 112 KB of shared memory, 256 TMEM columns) so
-// that TWO CTAs share an SM.  Each CTA's step is a serial chain of products and elementwise passes; with two resident
-// chains one CTA's start-up and waits are filled by the other's work.  To fit, only Qu[K] stays resident: Kc[K] and Vc[K]
-// are re-fetched by
-// TMA each step into slots that have just died (Kc over Vu[I] once Su is done, Vc over Qc[I] once Sc
-// is done); both fetches hide behind the elementwise pass that follows their issue.
-// The three products whose first operand is a tile the threads have just computed (gate A for the state
-// update, the masked T for the Su correction, P for P @ Vc) read it from TENSOR MEMORY, where the
-// threads put it as packed 16-bit pairs with tcgen05.st: that halves the shared-memory traffic of those
-// products (the port, not the tensor pipe, bounds a product with both operands in shared memory) and
-// saves the shared-memory copies of the masked T and of P.  The 64 packed columns alias accumulators
-// that are dead at that moment: gate and masked T over O, P over the first half of S.
-// Warp w owns TMEM lanes 32*(w%4).. and the column group w/4 of a 128-column accumulator: with G = 2
-// groups (256 threads) a thread works on 64 values of every 128x128 tile, with G = 4 (512 threads, 64
-// registers each) on 32 (measured slower, see below).
-constexpr uint32_t kFwd2Smem = 7 * kPanelBytes + 256;   // 112 KB of tiles + barriers
-#ifndef CASTLE_FWD_GROUPS
-#define CASTLE_FWD_GROUPS 2   // measured: 4 groups (512 threads, 63 registers) run the bench forward in 1.10 ms, 2 in 1.01 ms
-#endif
-constexpr int kFwd2Groups = CASTLE_FWD_GROUPS;
-
-// Tensor maps of the three decode caches a prefill launch stores into; the plain launch carries an empty struct
-// instead.  AUX = the kernel with the cache stores compiled in.
-template <bool AUX> struct CacheMaps {};
-template <> struct CacheMaps<true> { CUtensorMap qu, kc, vc; };
-
-template <typename T, int G, bool AUX>
-__global__ void __launch_bounds__(G * 128, 2)
-castle_fwd_kernel_d64(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
-                      const __grid_constant__ CUtensorMap m_vc, const __grid_constant__ CUtensorMap m_qu,
-                      const __grid_constant__ CUtensorMap m_ku, const __grid_constant__ CUtensorMap m_vu,
-                      const __grid_constant__ CacheMaps<AUX> m_cache) {
-  constexpr int D = 64;
-  constexpr int NCH = 4 / G;   // 32-column chunks of a 128-column tile per thread
-  constexpr uint32_t OPB = kPanelBytes;
-  constexpr uint32_t TM_COLS = 256;
-  constexpr uint32_t COL_W = 0, COL_S = 64, COL_O = 192;
-  constexpr int FMT = Elem<T>::fmt;
-  constexpr uint32_t ID_SQ = make_idesc(128, 128, FMT, false, false, false);
-  constexpr uint32_t ID_D = make_idesc(128, D, FMT, false, true, false);
-  constexpr float kLog2e = 1.4426950408889634f;
-
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* sQu = smem;                 // resident
-  uint8_t* sQV = sQu + OPB;            // Qc[I], then Vc[K]
-  uint8_t* sWb = sQV + OPB;
-  uint8_t* sKuA = sWb + OPB;           // Ku[I] -> gate A (32 KB; P lives in tensor memory)
-  uint8_t* sVuT = sKuA + 2 * OPB;      // Vu[I] -> Kc[K] in the first half (the masked T lives in tensor memory)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sVuT + 2 * OPB);
-  uint64_t *bar_qu = bars, *bar_qc = bars + 1, *bar_ku = bars + 2, *bar_vu = bars + 3, *bar_kc = bars + 4,
-           *bar_vc = bars + 5, *bar_mma = bars + 6;
-  uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(bars + 8);
-  int* abort_flag = reinterpret_cast<int*>(bars + 9);
-  // row max / row sum exchange between the two threads of a row: over the second half of the T slot,
-  // dead from the end of the Su product until the next step's masked T is written
-  float (*red_max)[kBlk] = reinterpret_cast<float (*)[kBlk]>(sVuT + OPB);
-  float (*red_sum)[kBlk] = reinterpret_cast<float (*)[kBlk]>(sVuT + OPB + G * kBlk * sizeof(float));
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int quarter = warp & 3, grp = warp >> 2;
-  const int cbase = grp * NCH * 32;
-  const int row = quarter * 32 + lane;
-  const int bh = blockIdx.x, K = blockIdx.y;
-  const int b = bh / p.H, h = bh % p.H;
-  const int k0 = K * kBlk;
-  const bool store_caches = AUX && p.store_caches;
-  const CUtensorMap *m_cache_qu = nullptr, *m_cache_kc = nullptr, *m_cache_vc = nullptr;
-  if constexpr (AUX) { m_cache_qu = &m_cache.qu; m_cache_kc = &m_cache.kc; m_cache_vc = &m_cache.vc; }
-  if ((smem_u32(smem) & 1023u) != 0) {  // the swizzled tiles need 1024-byte alignment
-    if (tid == 0) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
-    return;
-  }
-  if (tid == 0) {
-    for (int i = 0; i < 7; ++i) mbar_init(bars + i, 1);
-    mbar_fence_init();
-    *abort_flag = 0;
-    tma_prefetch_desc(&m_qc); tma_prefetch_desc(&m_ku); tma_prefetch_desc(&m_vu);
-    tma_prefetch_desc(&m_kc); tma_prefetch_desc(&m_vc);
-  }
-  if (warp == 0) { tmem_alloc(tmem_base_s, TM_COLS); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_base_s;
-  const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-  volatile int* abortp = abort_flag;
-
-  if (tid == 0) {
-    mbar_expect_tx(bar_qu, OPB);
-    tma_load_4d(sQu, &m_qu, bar_qu, 0, k0, h, b);
-    mbar_expect_tx(bar_qc, OPB);
-    tma_load_4d(sQV, &m_qc, bar_qc, 0, k0, h, b);
-    mbar_expect_tx(bar_ku, OPB);
-    tma_load_4d(sKuA, &m_ku, bar_ku, 0, k0, h, b);
-    mbar_expect_tx(bar_vu, OPB);
-    tma_load_4d(sVuT, &m_vu, bar_vu, 0, k0, h, b);
-    mbar_wait(bar_qu, 0, abortp);
-    // Prefill hand-off: Qu[K] is the block's rows of the decode cache; Kc[K] and Vc[K] follow in the
-    // first step, each when its fetch has landed (see there).
-    if (store_caches && !*abortp) tma_store_4d(m_cache_qu, sQu, 0, k0, h, b);
-  }
-
-  uint32_t ph_ld = 0, ph_mma = 0;   // the load barriers flip once per step
-  const uint32_t aQu = smem_u32(sQu), aQV = smem_u32(sQV), aWb = smem_u32(sWb), aKuA = smem_u32(sKuA),
-                 aVuT = smem_u32(sVuT);
-  const int krow = k0 + row;
-  const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
-
-#define F2_MMA_WAIT()                              \
-  mbar_wait_lazy_abort(bar_mma, ph_mma, abortp);   \
-  ph_mma ^= 1;                          \
-  tc_fence_after();
-#define F2_SYNC()      \
-  fence_async_smem();  \
-  tc_fence_before();   \
-  __syncthreads();
-
-  for (int I = K; I < p.nblk; ++I) {
-    const int i0 = I * kBlk;
-    const bool diag = (I == K), last = (I == p.nblk - 1);
-#ifdef CASTLE_PHASE_TIMING
-    const int tstep = I - K;
-#endif
-    PHASE_MARK(0);
-
-    // ---- Z[K,I] = Qu[K] @ Ku[I]^T
-    if (tid == 0) {
-      mbar_wait(bar_ku, ph_ld, abortp);
-      tc_fence_after();
-      gemm_kk_t<1>(tmem + COL_S, aQu, aKuA, ID_SQ, false);
-      mma_commit(bar_mma);
-    }
-    F2_MMA_WAIT();
-    PHASE_MARK(1);
-#pragma unroll
-    for (int c = 0; c < NCH; ++c) {  // gate A = sigmoid(scale * Z), kept for j > k; over Ku[I]
-      const int c0 = cbase + c * 32;
-      float v[32];
-      tmem_ld32(trow + COL_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), half_scale);
-        v[j] = a.x; v[j + 1] = a.y;
-      }
-      if (diag) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
-      }
-      store_row32<T>(sKuA, kPanelBytes, row, c0, v);   // operand of the Su correction (read along rows)
-      tmem_st_packed32<T>(trow + COL_O + c0 / 2, v);             // first operand of the state update
-    }
-    tmem_st_wait();
-    F2_SYNC();
-    PHASE_MARK(2);
-
-    // ---- W_K += A @ Vu[I]   and   T[I,I] = Qc[I] @ Vu[I]^T
-    if (tid == 0) {
-      mbar_wait(bar_vu, ph_ld, abortp);
-      mbar_wait(bar_qc, ph_ld, abortp);
-      tc_fence_after();
-      gemm_tm_t<8>(tmem + COL_W, tmem + COL_O, aVuT, ID_D, !diag);
-      gemm_kk_t<1>(tmem + COL_S, aQV, aVuT, ID_SQ, false);
-      mma_commit(bar_mma);
-    }
-    F2_MMA_WAIT();
-    PHASE_MARK(3);
-#pragma unroll
-    for (int c = 0; c < NCH; ++c) {  // masked T (j <= i), unscaled; over Vu[I]
-      const int c0 = cbase + c * 32;
-      float v[32];
-      tmem_ld32_lower(trow + COL_S + c0, row, c0, v);
-      tmem_st_packed32<T>(trow + COL_O + c0 / 2, v);   // over the gate's packed copy, which the update has consumed
-    }
-    tmem_st_wait();
-    tc_fence_before();
-    __syncthreads();
-    PHASE_MARK(4);
-
-    // ---- Su/scale = Qc[I] @ Wb^T + Tm @ A^T
-    if (tid == 0) {
-      tc_fence_after();
-      if (!diag) gemm_kk_t<1>(tmem + COL_S, aQV, aWb, ID_SQ, false);
-      gemm_tk_t<2>(tmem + COL_S, tmem + COL_O, aKuA, ID_SQ, !diag);
-      mma_commit(bar_mma);
-    }
-    F2_MMA_WAIT();
-    PHASE_MARK(5);
-    if (tid == 0) {  // Vu[I] is long consumed: fetch Kc[K] into its slot
-      mbar_expect_tx(bar_kc, OPB);
-      tma_load_4d(sVuT, &m_kc, bar_kc, 0, k0, h, b);
-    }
-#pragma unroll
-    for (int c = 0; c < NCH; ++c) {  // penalty -silu(Su)/scale back into the accumulator
-      const int c0 = cbase + c * 32;
-      float v[32];
-      tmem_ld32(trow + COL_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 u = make_float2(v[j], v[j + 1]);
-        const float2 x = mul2(u, neg_sigmoid2(u, half_scale));
-        v[j] = x.x; v[j + 1] = x.y;
-      }
-      tmem_st32(trow + COL_S + c0, v);
-    }
-    if (grp < 2) {  // refresh the 16-bit copy of W (now including block I)
-      float v[32];
-      tmem_ld32(trow + COL_W + grp * 32, v);
-      tmem_ld_wait();
-      store_row32<T>(sWb, kPanelBytes, row, grp * 32, v);
-    }
-    tmem_st_wait();
-    F2_SYNC();
-    PHASE_MARK(6);
-
-    // ---- S/scale = penalty + Qc[I] @ Kc[K]^T
-    if (tid == 0) {
-      mbar_wait(bar_kc, ph_ld, abortp);
-      tc_fence_after();
-      gemm_kk_t<1>(tmem + COL_S, aQV, aVuT, ID_SQ, true);
-      mma_commit(bar_mma);
-      if (diag && store_caches && !*abortp) tma_store_4d(m_cache_kc, sVuT, 0, k0, h, b);
-    }
-    F2_MMA_WAIT();
-    PHASE_MARK(7);
-    if (tid == 0) {  // Qc[I] and Kc[K] are consumed: fetch Vc[K] over Qc, and the next Vu over Kc
-      mbar_expect_tx(bar_vc, OPB);
-      tma_load_4d(sQV, &m_vc, bar_vc, 0, k0, h, b);
-    }
-    const int irow = i0 + row;
-    float mrow;
-    float2 lsum = splat(0.f);
-    {
-      float v[NCH][32];
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) tmem_ld32(trow + COL_S + cbase + c * 32, v[c]);
-      tmem_ld_wait();
-      if (diag) {
-#pragma unroll
-        for (int c = 0; c < NCH; ++c)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) v[c][j] = (cbase + c * 32 + j <= row) ? v[c][j] : -INFINITY;
-      }
-      float mx = v[0][0];
-#pragma unroll
-      for (int c = 0; c < NCH; ++c)
-#pragma unroll
-        for (int j = 0; j < 32; ++j) mx = fmaxf(mx, v[c][j]);
-      red_max[grp][row] = mx;
-      __syncthreads();
-#pragma unroll
-      for (int g = 0; g < G; ++g) mx = fmaxf(mx, red_max[g][row]);
-      mrow = mx * p.scale;
-      const float mb = mx * sl2;
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          const float2 x = fma2(make_float2(v[c][j], v[c][j + 1]), splat(sl2), splat(-mb));
-          v[c][j] = ex2_approx(x.x);
-          v[c][j + 1] = ex2_approx(x.y);
-          lsum = add2(lsum, make_float2(v[c][j], v[c][j + 1]));
-        }
-      }
-      red_sum[grp][row] = lsum.x + lsum.y;
-      // P as packed pairs over the first 64 columns of S: every thread of the row has its values in
-      // registers since the barrier above, so the accumulator may be overwritten
-#pragma unroll
-      for (int c = 0; c < NCH; ++c) tmem_st_packed32<T>(trow + COL_S + (cbase + c * 32) / 2, v[c]);
-    }
-    tmem_st_wait();
-    tc_fence_before();
-    __syncthreads();
-    PHASE_MARK(8);
-
-    // ---- O_partial = P @ Vc[K]
-    if (tid == 0) {
-      mbar_wait(bar_vc, ph_ld, abortp);
-      tc_fence_after();
-      gemm_tm_t<8>(tmem + COL_O, tmem + COL_S, aQV, ID_D, false);
-      mma_commit(bar_mma);
-      if (diag && store_caches) {
-        if (!*abortp) tma_store_4d(m_cache_vc, sQV, 0, k0, h, b);
-        bulk_commit();
-      }
-    }
-    const int64_t tile = (int64_t)bh * tri(p.nblk) + tri(I) + K;
-    if (grp == 0 && irow < p.N) {
-      float2* ml = reinterpret_cast<float2*>(p.part_ml) + tile * kBlk + row;
-      float l = red_sum[0][row];
-#pragma unroll
-      for (int g = 1; g < G; ++g) l += red_sum[g][row];
-      *ml = make_float2(mrow, l);
-    }
-    fence_async_smem();  // the exchange buffer is read here and written by TMA (next Vu) below
-    F2_MMA_WAIT();
-    PHASE_MARK(9);
-    if (tid == 0 && !last) {  // every slot of this step is dead: fetch the next step's Qc, Ku, Vu
-      const int in0 = i0 + kBlk;
-      if (diag && store_caches) bulk_wait_read0();   // the cache stores have read the Kc and Vc slots
-      mbar_expect_tx(bar_qc, OPB);
-      tma_load_4d(sQV, &m_qc, bar_qc, 0, in0, h, b);
-      mbar_expect_tx(bar_ku, OPB);
-      tma_load_4d(sKuA, &m_ku, bar_ku, 0, in0, h, b);
-      mbar_expect_tx(bar_vu, OPB);
-      tma_load_4d(sVuT, &m_vu, bar_vu, 0, in0, h, b);
-    }
-    if (grp < 2) {
-      uint4* dst = reinterpret_cast<uint4*>(p.part_o) + (tile * (D / 8) + grp * 4) * kBlk + row;
-      float v[32];
-      tmem_ld32(trow + COL_O + grp * 32, v);
-      tmem_ld_wait();
-      if (irow < p.N) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          dst[j * kBlk] = make_uint4(Elem<T>::pack2(v[8 * j], v[8 * j + 1]), Elem<T>::pack2(v[8 * j + 2], v[8 * j + 3]),
-                              Elem<T>::pack2(v[8 * j + 4], v[8 * j + 5]), Elem<T>::pack2(v[8 * j + 6], v[8 * j + 7]));
-      }
-    }
-    ph_ld ^= 1;
-    tc_fence_before();
-    __syncthreads();
-    PHASE_MARK(10);
-  }
-#undef F2_MMA_WAIT
-#undef F2_SYNC
-
-  // ---- W_K is now U[K]
-  if (grp < 2 && (p.u_out.ptr != nullptr || p.w_state != nullptr)) {
-    tc_fence_after();
-    const int c0 = grp * 32;
-    float v[32];
-    tmem_ld32(trow + COL_W + c0, v);
-    tmem_ld_wait();
-    if (krow < p.N) {
-      if (p.w_state != nullptr) store_u32(p.w_state, CASTLE_F32, ((int64_t)bh * p.N + krow) * D + c0, v);
-      if (p.u_out.ptr != nullptr)
-        store_u32(p.u_out.ptr, p.u_dtype, b * p.u_out.stride_b + h * p.u_out.stride_h + (int64_t)krow * p.u_out.stride_n + c0, v);
-    }
-  }
-  if (store_caches && tid == 0) bulk_wait0();
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, TM_COLS);
-  if (tid == 0 && *abort_flag) atomicOr(p.status, CASTLE_STATUS_WAIT_TIMEOUT);
-}
-
 // Merge the per-key-block partials of one query block: out = sum_K e^{m_K - m} O_K / sum_K e^{m_K - m} l_K.
 // One CTA per query block and 32 rows; a warp owns a chunk of eight columns of them (a lane a row), so that its loads
 // are contiguous.
@@ -944,48 +1024,28 @@ __global__ void __launch_bounds__(32 * D / 8) castle_fwd_merge_kernel(const FwdP
   if (c8 == 0) p.lse[(int64_t)bh * p.N + i] = m + __logf(l);
 }
 
-template <typename T>
-static int launch_fwd_short(const FwdParams& p, const CUtensorMap* maps, cudaStream_t st) {
-  constexpr int G = kFwd2Groups;
-  dim3 grid(p.B * p.H, p.nblk);
-  if (p.store_caches) {
-    cudaError_t e = cudaFuncSetAttribute(castle_fwd_kernel_d64<T, G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
-    if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
-    CacheMaps<true> cm;
-    cm.qu = maps[6]; cm.kc = maps[7]; cm.vc = maps[8];
-    castle_fwd_kernel_d64<T, G, true><<<grid, G * 128, kFwd2Smem, st>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], cm);
-  } else {
-    cudaError_t e = cudaFuncSetAttribute(castle_fwd_kernel_d64<T, G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFwd2Smem);
-    if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
-    castle_fwd_kernel_d64<T, G, false><<<grid, G * 128, kFwd2Smem, st>>>(p, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5],
-                                                                        CacheMaps<false>{});
-  }
-  return 0;
-}
-
 template <typename T, int D>
 static int launch_fwd_pipe(const FwdParams& p, const CUtensorMap* maps, cudaStream_t st) {
-  // Few pairs: the grid is one wave whose length is the walk of key block 0, while the mean walk is half as long or, with
-  // idle SMs, still less.  `load` = steps per SM over the longest walk.  us uncut / 2 / 3 parts: 4 pairs x 16 blocks at
-  // dim_head 128 74 / 60 / 52 (load 0.23), 4 x 12 44 / 37 / 34 (0.18), 8 x 12 44 / 37 / 40 (0.35), 4 x 32 100 / 78 / 88 (0.45), 16 x 11
-  // 43 / 46 / 52 (0.65), 8 x 32 103 / 138 / 166 (0.89).
-  const float load = (float)(p.B * p.H) * (float)(p.nblk + 1) * (0.5f / 148.f);
-  const int nseg = p.nblk < kSplitMin || load >= 0.6f ? 1 : load >= 0.3f ? 2 : 3;
-  auto kernel = p.tm ? castle_fwd_pipe_kernel<T, D, true> : castle_fwd_pipe_kernel<T, D, false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FwdPipe<D>::kSmem);   // per device, so on every call (cheap)
-  if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
-  e = launch_kernel(kernel, dim3(p.B * p.H, p.nblk, nseg), kFwdThreads, FwdPipe<D>::kSmem, st, p.tm != nullptr, p, maps[0], maps[1], maps[2],
-                    maps[3], maps[4], maps[5], maps[6], maps[7], maps[8]);
+  const FwdPlan plan = fwd_plan((int64_t)p.B * p.H, p.nblk, D);
+  cudaError_t e;
+  if (plan.persistent) {
+    auto kernel = p.tm ? castle_fwd_pipe64_kernel<T, true> : castle_fwd_pipe64_kernel<T, false>;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FwdPipe<64>::kSmem);   // per device, so on every call (cheap)
+    if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
+    e = launch_kernel(kernel, dim3((unsigned)std::min<int64_t>(148, (int64_t)p.B * p.H * p.nblk)), kFwdThreads, FwdPipe<64>::kSmem, st, p.tm != nullptr, p,
+                      maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], maps[8]);
+  } else {
+    auto kernel = p.tm ? castle_fwd_pipe_kernel<T, D, true> : castle_fwd_pipe_kernel<T, D, false>;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FwdPipe<D>::kSmem);
+    if (e != cudaSuccess) return cuda_fail(e, "castle_fwd attribute");
+    e = launch_kernel(kernel, dim3(p.B * p.H, p.nblk, plan.nseg), kFwdThreads, FwdPipe<D>::kSmem, st, p.tm != nullptr, p, maps[0], maps[1], maps[2],
+                      maps[3], maps[4], maps[5], maps[6], maps[7], maps[8]);
+  }
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_fwd launch");
 }
 
 template <typename T, int D>
-static int launch_fwd(FwdParams p, const CUtensorMap* maps, cudaStream_t st) {
-  // One CTA per SM leaves a CTA's start-up (some 10 us: tensor memory, first tiles, the fill of the pipeline) uncovered, so
-  // where the walks are short and the grid is more than a wave, dim_head 64 takes the kernel with two CTAs per SM.  us, short /
-  // pipeline: 512 pairs x 1 block 28 / 38, 256 x 4 92 / 100, 128 x 5 71 / 74, 128 x 8 143 / 139.
-  const bool brief = D == 64 && p.nblk <= 6 && (int64_t)p.B * p.H * p.nblk > 2 * 148;
-  if (brief) p.tm = nullptr;
+static int launch_fwd(const FwdParams& p, const CUtensorMap* maps, cudaStream_t st) {
   if (p.tm) {
     constexpr size_t smem = 2 * (D / 64) * kPanelBytes;
     cudaError_t e = cudaFuncSetAttribute(castle_fwd_t_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -993,10 +1053,7 @@ static int launch_fwd(FwdParams p, const CUtensorMap* maps, cudaStream_t st) {
     castle_fwd_t_kernel<T, D><<<dim3(p.B * p.H, p.nblk), 128, smem, st>>>(p, maps[0], maps[5]);
   }
   ev_start(CASTLE_KERNEL_FWD, st);
-  int rc;
-  if constexpr (D == 64) rc = brief ? launch_fwd_short<T>(p, maps, st) : launch_fwd_pipe<T, D>(p, maps, st);
-  else rc = launch_fwd_pipe<T, D>(p, maps, st);
-  if (rc) return rc;
+  if (const int rc = launch_fwd_pipe<T, D>(p, maps, st)) return rc;
   ev_stop(CASTLE_KERNEL_FWD, st);
   cudaError_t e = launch_kernel(castle_fwd_merge_kernel<T, D>, dim3(p.nblk * (kBlk / 32), p.B * p.H), 32 * D / 8, 0, st, true, p);
   if (e == cudaSuccess) e = cudaGetLastError();
@@ -1063,7 +1120,7 @@ static int fwd_impl(const char* who, const castle_problem_t* p, const castle_ten
   fp.u_dtype = u_dtype;
   fp.out = *out; fp.status = status;
   fp.store_caches = caches ? 1 : 0;
-  fp.tm = fp.nblk >= kTmBlocks ? (uint4*)((uint8_t*)workspace + tiles * kBlk * (2 * sizeof(float) + p->dim_head * 2)) : nullptr;
+  fp.tm = fwd_plan((int64_t)p->batch * p->heads, fp.nblk, p->dim_head).ahead ? (uint4*)((uint8_t*)workspace + tiles * kBlk * (2 * sizeof(float) + p->dim_head * 2)) : nullptr;
 #ifdef CASTLE_PHASE_TIMING
   fp.timing = (long long*)((char*)workspace + need);  // the caller leaves 1 KB beyond the partials
 #endif

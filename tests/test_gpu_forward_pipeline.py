@@ -1,5 +1,5 @@
 """GPU: the forward's dispatch - masked T tiles computed up front or inside the walk, walks whole or cut in two or three
-parts, the two-CTA kernel for many short walks - against the oracle, output and lookahead keys."""
+parts, many short walks - against the oracle, output and lookahead keys."""
 import pytest
 import torch
 
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
     (1, 1, 1024, 64), (1, 1, 1023, 128), (1, 2, 1500, 64), (1, 2, 2049, 128),  # three parts
     (1, 12, 1100, 64), (1, 9, 1281, 128),                                      # two parts
     (3, 7, 1030, 64), (3, 7, 1030, 128),                                       # whole walks, more than one wave
-    (38, 4, 257, 64), (30, 3, 641, 64), (100, 3, 1, 64)])                      # the two-CTA kernel
+    (38, 4, 257, 64), (30, 3, 641, 64), (100, 3, 1, 64)])                      # many short walks
 def test_forward_dispatch(B, H, N, d):
     from lookahead_keys_attention_b200 import castle_attention_packed, check_status
     torch.manual_seed(N + d)
