@@ -125,7 +125,7 @@ __device__ __forceinline__ void store_u32(void* base, int dtype, int64_t off, co
 
 // A masked T tile in global memory: [16 chunks of 8 columns][128 rows] x 16 bytes, so that a warp's access is contiguous.
 constexpr int64_t kTmTile = 16 * kBlk;   // in uint4
-constexpr int kTmBlocks = 8;             // with fewer query blocks they never pay; from here on there is room for them (so that the scratch is linear in the pairs)
+constexpr int kTmBlocks = 8;             // with fewer query blocks they do not pay (64 x 16 heads x 6 blocks 709 / 697 us); from here on there is room for them (so that the scratch is linear in the pairs)
 
 // The forward's plan for a problem: parts per walk, whether the masked T tiles are computed once, up front, and the kernel.
 struct FwdPlan { int nseg; bool ahead, persistent; };
@@ -137,15 +137,16 @@ static FwdPlan fwd_plan(int64_t pairs, int64_t nblk, int dim_head) {
   // 43 / 46 / 52 (0.65), 8 x 32 103 / 138 / 166 (0.89).
   const float load = (float)pairs * (float)(nblk + 1) * (0.5f / 148.f);
   f.nseg = nblk < kSplitMin || load >= 0.6f ? 1 : load >= 0.3f ? 2 : 3;
-  // The tiles cost a launch of 8 us and 14 ns a tile (64 KB through memory); a step that reads one instead of computing it is
-  // 0.52 us shorter at dim_head 64 (a product less in the chain) and 0.37 at 128.  The steps that count are those of the busiest SM:
-  // their mean, or the longest walk (the first part has 0.65 and 0.54 of its steps).  us of a forward with / without the tiles,
-  // pairs x blocks: dim_head 64 512 x 4 228 / 211, 128 x 8 182 / 182, 64 x 10 147 / 144, 128 x 13 374 / 380, 64 x 17 306 / 321, 8 x 16
-  // 86 / 83, 16 x 17 109 / 106, 8 x 24 126 / 128, 4 x 32 116 / 115, 8 x 32 146 / 152; dim_head 128 256 x 4 213 / 195, 128 x 8 279 / 267,
-  // 8 x 11 81 / 73, 16 x 16 130 / 127, 64 x 16 416 / 413, 16 x 32 366 / 377.
-  const float longest = (float)nblk * (f.nseg == 1 ? 1.f : f.nseg == 2 ? 0.65f : 0.54f);
+  // The tiles cost 4 us of their kernel's latency and 7.5 ns (dim_head 64) or 12.5 ns a tile through memory; a step that reads one
+  // instead of computing it is 0.43 and 0.36 us shorter (a product less in the chain).  The steps that count are those of the
+  // busiest SM: their mean, or the longest walk, of whose parts some have few steps with scores.  us of a forward with /
+  // without the tiles, pairs x blocks: dim_head 64 128 x 8 155.0 / 157.8, 64 x 10 119.7 / 121.9, 128 x 11 261.7 / 269.6, 64 x 17 278 / 297, 16 x 17
+  // 77.4 / 78.9, 8 x 24 88.6 / 96.7, 4 x 32 87.3 / 91.8, 48 x 8 70.0 / 69.2, 4 x 12 39.4 / 35.8, 2 x 24 63.7 / 61.8, 1 x 32 77.9 / 76.1; dim_head 128
+  // 16 x 22 186 / 191, 64 x 24 772 / 797, 64 x 16 388.6 / 388.4, 16 x 16 106.9 / 106.5, 128 x 8 253.8 / 246.0, 64 x 11 209.7 / 207.4, 16 x 11 69.6 / 68.5.
+  const float longest = (float)nblk * (f.nseg == 1 ? 1.f : f.nseg == 2 ? 0.7f : 0.25f);
   const float steps = std::max(longest, load * (float)nblk);
-  f.ahead = nblk >= kTmBlocks && steps * (dim_head == 64 ? 0.52f : 0.37f) > 8.f + 0.014f * (float)(pairs * nblk);
+  const bool narrow = dim_head == 64;
+  f.ahead = nblk >= kTmBlocks && steps * (narrow ? 0.43f : 0.36f) > 4.f + (narrow ? 0.0075f : 0.0125f) * (float)(pairs * nblk);
   // A CTA that takes one walk after the other covers their starts and ends, but its steps are some 4 % longer (it looks up
   // what comes next), so it is for short walks, and the longer they are the more of them there must be.  us of the kernel, walk after walk / a
   // CTA per walk, pairs x blocks: 128 x 8 124 / 145, 48 x 12 103 / 110, 128 x 13 286 / 314, 128 x 17 460 / 485, 128 x 20 622 / 648, 64 x 24
