@@ -671,8 +671,9 @@ Tensor product(int layout, const Tensor& a, const Tensor& b, int64_t rows) {
   const int64_t k = layout == 2 ? a.size(0) : a.size(1), m = layout == 2 ? a.size(1) : a.size(0), n = layout == 0 ? b.size(0) : b.size(1);
   const int64_t unit = 16 / a.element_size();
   auto fits = [&](const Tensor& t) { return t.stride(1) == 1 && t.stride(0) >= t.size(1) && aligned(t); };
-  if (small_product(rows, m, n, k, a.scalar_type()) && b.scalar_type() == a.scalar_type() && n % unit == 0 && (layout == 2 ? m : k) % unit == 0 &&
-      fits(a) && fits(b)) {
+  // what does not match (in k, type or device) is the library's to refuse
+  const bool match = b.scalar_type() == a.scalar_type() && b.device() == a.device() && b.size(layout == 0 ? 1 : 0) == k;
+  if (match && small_product(rows, m, n, k, a.scalar_type()) && n % unit == 0 && (layout == 2 ? m : k) % unit == 0 && fits(a) && fits(b)) {
     const auto stream = c10::cuda::getCurrentCUDAStream(a.device().index());
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream.stream(), &capture) != cudaSuccess) (void)cudaGetLastError();
@@ -719,9 +720,11 @@ struct LayerBackward : public Node {
     SavedCore::Unpacked saved;   // (unpacking raises on a second backward)
     if (need_core) saved = core.unpack(shared_from_this());
     else if (need_out) saved.out16 = core.out16.unpack();
-    const Tensor wc = need_core ? combine.unpack() : Tensor(), wq = need_x || need_norm ? to_qkv.unpack() : Tensor(),
-                 xs = (need_qkv && !separate_h) || (has_norm && (need_x || need_norm)) ? x.unpack() : Tensor(),
-                 hs = need_qkv && separate_h ? h.unpack() : Tensor(), ms = need_combine && separate_merged ? merged.unpack() : Tensor(),
+    const Tensor wc = need_core ? restored(combine.unpack(), {grads[0].size(-1), inner}, dtype, dev) : Tensor(),
+                 wq = need_x || need_norm ? restored(to_qkv.unpack(), {6 * inner, dim}, dtype, dev) : Tensor(),
+                 xs = (need_qkv && !separate_h) || (has_norm && (need_x || need_norm)) ? restored(x.unpack(), x_sizes, dtype, dev) : Tensor(),
+                 hs = need_qkv && separate_h ? restored(h.unpack(), {rows, dim}, dtype, dev) : Tensor(),
+                 ms = need_combine && separate_merged ? restored(merged.unpack(), {rows, inner}, dtype, dev) : Tensor(),
                  ws_norm = has_norm && (need_x || need_norm) ? norm.unpack() : Tensor(),
                  rs_norm = has_norm && (need_x || need_norm) ? rstd.unpack() : Tensor();
     at::AutoDispatchBelowADInplaceOrView below;
@@ -740,7 +743,7 @@ struct LayerBackward : public Node {
       result[0] = dh.view(x_sizes);
       return result;
     }
-    const Tensor xc = restored_contiguous(xs, x_sizes, dtype, dev), wn = restored_contiguous(ws_norm, {dim}, dtype, dev),
+    const Tensor xc = aligned_contiguous(xs), wn = restored_contiguous(ws_norm, {dim}, dtype, dev),
                  rs = restored_contiguous(rs_norm, {rows}, at::kFloat, dev);
     if (need_x) result[0] = at::empty(x_sizes, dh.options());
     if (need_norm) result[3] = at::empty({dim}, dh.options());

@@ -105,6 +105,28 @@ def test_hooks_that_change_a_tensor_are_refused():
         torch.autograd.grad(out, wanted, g)
 
 
+@pytest.mark.parametrize("change", ["device", "rows", "type"])
+@pytest.mark.parametrize("prenorm,sizes", [(True, (DIM, 64 * H)), (True, (6 * 64 * H, DIM)), (True, (B, N, DIM)), (True, (B * N, DIM)),
+                                           (True, (B * N, 64 * H)), (False, (B, N, DIM))])
+def test_hooks_that_change_one_tensor_of_the_layer_are_refused(prenorm, sizes, change):
+    """The weights, the input, the projection's input and the merged heads, one at a time, in a call whose products are the
+    framework's own launches: they get addresses and would read host memory or past the end."""
+    m, wanted, g = _layer(torch.float32, prenorm, False, 64)
+    changed = []
+
+    def unpack(t):
+        if tuple(t.shape) != sizes:
+            return t
+        changed.append(t)
+        return {"device": t.cpu, "rows": lambda: t[..., :-1, :], "type": t.half}[change]()
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        out = m(wanted[0])
+    with pytest.raises(RuntimeError, match="saved tensor came back"):
+        torch.autograd.grad(out, wanted, g)
+    assert len(changed) == 1
+
+
 def test_only_what_a_gradient_needs_is_guarded_against_changes():
     """As with the single operations: a frozen projection's input may change after the forward."""
     m, wanted, g = _layer(torch.bfloat16, False, False, 64)
