@@ -19,6 +19,7 @@
 #include <torch/csrc/PyInterpreter.h>
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/autocast_mode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -670,7 +671,8 @@ bool small_product(int64_t rows, int64_t m, int64_t n, int64_t k, at::ScalarType
 Tensor product(int layout, const Tensor& a, const Tensor& b, int64_t rows) {
   const int64_t k = layout == 2 ? a.size(0) : a.size(1), m = layout == 2 ? a.size(1) : a.size(0), n = layout == 0 ? b.size(0) : b.size(1);
   const int64_t unit = 16 / a.element_size();
-  auto fits = [&](const Tensor& t) { return t.stride(1) == 1 && t.stride(0) >= t.size(1) && aligned(t); };
+  // a tensor without memory of its own (a batched gradient's wrapper) and a dispatch mode that counts or replaces the products: the library's path
+  auto fits = [&](const Tensor& t) { return !at::isTensorSubclassLike(t) && t.stride(1) == 1 && t.stride(0) >= t.size(1) && aligned(t); };
   // what does not match (in k, type or device) is the library's to refuse
   const bool match = b.scalar_type() == a.scalar_type() && b.device() == a.device() && b.size(layout == 0 ? 1 : 0) == k;
   if (match && small_product(rows, m, n, k, a.scalar_type()) && n % unit == 0 && (layout == 2 ? m : k) % unit == 0 && fits(a) && fits(b)) {

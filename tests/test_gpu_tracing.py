@@ -99,3 +99,43 @@ def test_torch_functions_are_called_where_they_may_be_replaced():
         for sub in (m.to_all_qkv, m.combine_heads):
             sub._parameters["weight"] = sub.weight.detach().as_subclass(_Scaled)
         assert _rel(m(x), want) <= 1e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n", [140, 600])   # 280 positions: products of the framework's own; 1200: the library's
+def test_batched_gradients_of_the_output_projection(dtype, n):
+    from lookahead_keys_attention_b200 import Castle
+    torch.manual_seed(n)
+    m = Castle(96, heads=2).cuda().to(dtype)
+    x = torch.randn(2, n, 96, device="cuda").to(dtype)
+    g = torch.randn(3, 2, n, 96, device="cuda").to(dtype)
+    for frozen in (True, False):
+        m.to_all_qkv.requires_grad_(not frozen)
+        out, w = m(x), m.combine_heads.weight
+        got, = torch.autograd.grad(out, w, g, is_grads_batched=True, retain_graph=True)
+        # sums in another order: a 16-bit result may be rounded the other way (2^-8 of a value), an fp32 one differs by sqrt(k) 2^-24
+        for a, b in zip(got, g):
+            assert _rel(a, torch.autograd.grad(out, w, b, retain_graph=True)[0]) <= (4e-3 if dtype == torch.bfloat16 else 1e-5)
+
+
+def test_dispatch_modes_see_the_products_of_the_gradient():
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from lookahead_keys_attention_b200 import Castle
+    seen = []
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    torch.manual_seed(0)
+    m = Castle(96, heads=2).cuda()
+    x, g = (torch.randn(2, 140, 96, device="cuda") for _ in range(2))
+    wanted = [x.requires_grad_(), *m.parameters()]
+    out = m(x)
+    plain = torch.autograd.grad(out, wanted, g, retain_graph=True)
+    with Watch():
+        got = torch.autograd.grad(out, wanted, g)
+    assert seen.count(torch.ops.aten.mm.default) == 4   # both weights, the merged heads, the input
+    for a, b in zip(got, plain):   # the core's gradient is rounded to its 16-bit operands' type: by at most 2^-10 of a value another way
+        assert _rel(a, b) <= 2e-3
