@@ -467,6 +467,8 @@ struct SavedCore {
   }
   Tensor backward(const Unpacked& u, const Tensor& grad) const {
     const at::Device dev = grad.device();
+    const std::array<int64_t, 4> grad_sizes{p.B, p.H, p.N, p.d};
+    need(grad.sizes() == at::IntArrayRef(grad_sizes) && grad.scalar_type() == p.dtype, "castle_attention: the gradient's shape or type is not the output's");
     const std::vector<int64_t> bhnd{p.B, p.H, p.N, p.dp};
     Options now = o;
     if (o.rotary.on()) now.rotary.freqs = restored_contiguous(u.freqs, o.rotary.freqs.sizes(), o.rotary.freqs.scalar_type(), dev);
@@ -730,6 +732,8 @@ struct LayerBackward : public Node {
                  ws_norm = has_norm && (need_x || need_norm) ? norm.unpack() : Tensor(),
                  rs_norm = has_norm && (need_x || need_norm) ? rstd.unpack() : Tensor();
     at::AutoDispatchBelowADInplaceOrView below;
+    // A backward called under autocast: the products keep the layer's type, in which the kernels behind them read their results.
+    const c10::impl::ExcludeDispatchKeyGuard no_autocast(c10::autocast_dispatch_keyset);
     const c10::cuda::CUDAGuard guard(dev);
     const auto stream = c10::cuda::getCurrentCUDAStream(dev.index());
     const Tensor g = grads[0].reshape({rows, grads[0].size(-1)});

@@ -97,3 +97,21 @@ def test_input_at_an_odd_offset(dtype, prenorm, batch):
     assert odd[0].data_ptr() % 16 and odd[1].data_ptr() % 16 and odd[0].is_contiguous()
     for a, b in zip(go(*odd), go(*even)):
         assert (a.float() - b.float()).norm().item() <= 4e-3 * b.float().norm().item()
+
+
+@pytest.mark.parametrize("n", [140, 600])   # products of the framework's own, and the library's, which autocast would change
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("prenorm", [False, True])
+def test_backward_under_autocast(dtype, prenorm, n):
+    from lookahead_keys_attention_b200 import Castle
+    torch.manual_seed(n)
+    m = Castle(96, heads=2, prenorm=prenorm).cuda().to(dtype)
+    x, g = (torch.randn(2, n, 96, device="cuda").to(dtype) for _ in range(2))
+    wanted = [x.requires_grad_(), *m.parameters()]
+    out = m(x)
+    plain = torch.autograd.grad(out, wanted, g, retain_graph=True)
+    for other in (torch.float16, torch.bfloat16):
+        with torch.autocast("cuda", dtype=other):
+            got = torch.autograd.grad(out, wanted, g, retain_graph=True)
+        for a, b in zip(got, plain):   # the same launches; dqc, dku and dvu are added in arrival order
+            assert a.dtype == b.dtype and (a.float() - b.float()).norm().item() <= 4e-3 * b.float().norm().item()
