@@ -172,8 +172,10 @@ castle_tensor_t desc(const Tensor& t) {   // (B, H, N, d), last dimension contig
 }
 
 // The ABI's rules: 16-byte base and strides, the last dimension contiguous, and no dimension that repeats one element's
-// row (stride 0, as expand() leaves it), which the kernels' tensor maps cannot express.
+// row (stride 0, as expand() leaves it), which the kernels' tensor maps cannot express.  And the memory holds the tensor's values,
+// which a lazy negation's (an imaginary part of a conjugate) does not; a copy has them.
 bool aligned(const Tensor& t) {
+  if (t.is_neg()) return false;
   if ((t.stride(-1) != 1 && t.size(-1) != 1) || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0) return false;
   for (int64_t i = 0; i + 1 < t.dim(); ++i)
     if (t.stride(i) * t.element_size() % 16 != 0 || (t.stride(i) == 0 && t.size(i) > 1)) return false;
@@ -188,7 +190,7 @@ castle_tensor_t packed_desc(const Tensor& p, int i) {
 
 // Contiguous at a 16-byte boundary (contiguous() leaves a view at an odd offset as it is).
 Tensor aligned_contiguous(const Tensor& t) {
-  return t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
+  return !t.is_neg() && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone(at::MemoryFormat::Contiguous);
 }
 
 castle_tensor_t rect(castle_tensor_t t, int64_t es, int64_t b, int64_t h) {
@@ -647,10 +649,10 @@ struct Layer {
 bool plain_layer(const Tensor& x, const Layer& l) {
   auto plain = [&](const Tensor& t) {
     return t.is_cuda() && t.scalar_type() == x.scalar_type() && t.is_contiguous() && t.layout() == at::kStrided && t.device() == x.device() &&
-           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !t.unsafeGetTensorImpl()->is_python_dispatch() && !has_tangent(t);
+           reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !t.is_neg() && !t.unsafeGetTensorImpl()->is_python_dispatch() && !has_tangent(t);
   };
   const int64_t inner = l.heads * l.dim_head;
-  return x.dim() == 3 && x.is_cuda() && x.numel() > 0 && x.layout() == at::kStrided && !x.unsafeGetTensorImpl()->is_python_dispatch() && !has_tangent(x) &&
+  return x.dim() == 3 && x.is_cuda() && x.numel() > 0 && x.layout() == at::kStrided && !x.is_neg() && !x.unsafeGetTensorImpl()->is_python_dispatch() && !has_tangent(x) &&
          dtype_code(x.scalar_type()) >= 0 && x.size(2) % 8 == 0 && plain(l.to_qkv) && plain(l.combine) &&
          (!l.norm.defined() || (plain(l.norm) && l.norm.dim() == 1 && l.norm.size(0) == x.size(2))) && l.to_qkv.dim() == 2 &&
          l.to_qkv.size(0) == 6 * inner && l.to_qkv.size(1) == x.size(2) && l.combine.dim() == 2 && l.combine.size(1) == inner &&

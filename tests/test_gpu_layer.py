@@ -115,3 +115,29 @@ def test_backward_under_autocast(dtype, prenorm, n):
             got = torch.autograd.grad(out, wanted, g, retain_graph=True)
         for a, b in zip(got, plain):   # the same launches; dqc, dku and dvu are added in arrival order
             assert a.dtype == b.dtype and (a.float() - b.float()).norm().item() <= 4e-3 * b.float().norm().item()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_lazily_negated_tensors(dtype):
+    """Their memory holds the values without the sign (as the imaginary part of a conjugate does)."""
+    from lookahead_keys_attention_b200 import Castle, castle_attention, castle_decode_step
+    torch.manual_seed(0)
+    lazy = torch._neg_view
+    m = Castle(96, heads=2, prenorm=True).cuda().to(dtype)
+    six = [(torch.randn(2, 2, 140, 64, device="cuda") * 3 ** -0.5).to(dtype) for _ in range(6)]
+    x, g = (torch.randn(2, 140, 96, device="cuda").to(dtype) for _ in range(2))
+    gs, rows = torch.randn(2, 2, 140, 64, device="cuda").to(dtype), [torch.randn(2, 2, 1, 64, device="cuda").to(dtype) for _ in range(6)]
+
+    def go(neg):
+        a = neg(x.clone()).requires_grad_()
+        out, cache = m(a, return_next_cache=True)
+        grads = torch.autograd.grad(out, [a, *m.parameters()], neg(g))
+        with torch.no_grad():
+            step, _ = m(neg(x[:, :1].clone()), cache=cache)
+        ts = [neg(t.clone()).requires_grad_() for t in six]
+        y = castle_attention(*ts, 0.125)
+        return [out.detach(), step, *grads, y.detach(), *torch.autograd.grad(y, ts, neg(gs)),
+                castle_decode_step(*[neg(r) for r in rows], *[torch.ones(2, 2, 9, 64, device="cuda", dtype=dtype) for _ in range(4)], 8, 0.125)]
+
+    for a, b in zip(go(lazy), go(torch.neg)):   # single operations around the lazily negated input: 16-bit roundings that fall the other way
+        assert (a.float() - b.float()).norm().item() <= 2e-2 * b.float().norm().item()
