@@ -1,4 +1,4 @@
-// What the cached-step kernels (decode.cu, token_layer.cu) share: 16-byte vectors of a row as floats, the sums over the
+// What the cached-step kernels (decode.cu, token_layer.cu, token_linear.cu) share: 16-byte vectors of a row as floats, the sums over the
 // lanes of a row, the rotation of the new rows.
 #pragma once
 #include "rotary.cuh"

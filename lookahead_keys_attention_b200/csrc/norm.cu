@@ -111,7 +111,6 @@ __global__ void __launch_bounds__(kNormThreads) castle_rmsnorm_dw_kernel(const T
 // row on its way meanwhile, and keeps its share of the weight's gradient in registers.  us of both gradients, before (a
 // pass for each) -> now: 16384 x 512 bf16 23.0 -> 12.6, fp32 37.2 -> 17.9 (the bytes take 7.7 and 15.4 from memory), 50000 x 512 bf16 54 -> 35, 200 x 512
 // bf16 12.4 -> 8.2.
-template <typename T> struct Raw8 { uint4 q[sizeof(T) / 2]; };
 template <typename T, int C>
 __global__ void __launch_bounds__(kNormThreads, 2) castle_rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                                                                              const float* __restrict__ rstd, T* __restrict__ dx,

@@ -6,31 +6,13 @@
 // launch.  A warp owns WR rows of w and streams them with 16-byte loads; x sits in shared memory as fp32; all sums are
 // fp32.  At 1 x 512 -> 3072 -> 512 bf16 the kernels take 2.8 and 2.3 us where the library calls took 2.7 + 3.8 and 3.0.
 #include "common.cuh"
+#include "decode_row.cuh"
 #include "vec.cuh"
 
 namespace castle {
 
 constexpr int kTokenThreads = 128;
 constexpr int kTokenSmem = 96 * 1024;   // x as fp32
-
-template <typename T> struct Wide;      // 16 bytes of T
-template <> struct Wide<float> {
-  static constexpr int N = 4;
-  static __device__ __forceinline__ void unpack(uint4 q, float* v) {
-    v[0] = __uint_as_float(q.x); v[1] = __uint_as_float(q.y); v[2] = __uint_as_float(q.z); v[3] = __uint_as_float(q.w);
-  }
-  static __device__ __forceinline__ float round(float x) { return x; }
-  static __device__ __forceinline__ float cast(float x) { return x; }
-};
-template <typename T> struct Wide {
-  static constexpr int N = 8;
-  static __device__ __forceinline__ void unpack(uint4 q, float* v) {
-    const float2 a = Elem<T>::unpack2(q.x), b = Elem<T>::unpack2(q.y), c = Elem<T>::unpack2(q.z), d = Elem<T>::unpack2(q.w);
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
-  }
-  static __device__ __forceinline__ float round(float x) { return Elem<T>::to_f(Elem<T>::from_f(x)); }
-  static __device__ __forceinline__ T cast(float x) { return Elem<T>::from_f(x); }
-};
 
 struct TokenLinearParams {
   const void *x, *norm, *w;
@@ -44,7 +26,7 @@ struct TokenLinearParams {
 // R = rows of x (padded up to 1, 2, 4 or 8), WR = rows of w per warp.
 template <typename T, int R, int WR>
 __global__ void __launch_bounds__(kTokenThreads) castle_token_linear_kernel(const TokenLinearParams p) {
-  constexpr int V = Wide<T>::N, NW = kTokenThreads / 32;
+  constexpr int V = Vec<T>::N, NW = kTokenThreads / 32;
   extern __shared__ __align__(16) float xs[];   // [R][K]
   __shared__ float part[NW][R];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -69,7 +51,7 @@ __global__ void __launch_bounds__(kTokenThreads) castle_token_linear_kernel(cons
     const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.x) + (int64_t)min(r, p.rows - 1) * p.ldx);
     for (int c = threadIdx.x; c < chunks; c += kTokenThreads) {
       float v[V];
-      Wide<T>::unpack(src[c], v);
+      Vec<T>::unpack(src[c], v);
 #pragma unroll
       for (int j = 0; j < V; ++j) { ss[r] = fmaf(v[j], v[j], ss[r]); xs[r * p.K + c * V + j] = v[j]; }
     }
@@ -91,11 +73,11 @@ __global__ void __launch_bounds__(kTokenThreads) castle_token_linear_kernel(cons
       const float inv = rsqrtf(s / (float)p.K + p.eps);
       for (int c = threadIdx.x; c < chunks; c += kTokenThreads) {   // the thread's own elements
         float g[V];
-        Wide<T>::unpack(nw[c], g);
+        Vec<T>::unpack(nw[c], g);
 #pragma unroll
         for (int j = 0; j < V; ++j) {
           float& e = xs[r * p.K + c * V + j];
-          e = Wide<T>::round(e * inv * g[j]);   // the norm's result has the type of x
+          e = round_to<T>(e * inv * g[j]);   // the norm's result has the type of x
         }
       }
     }
@@ -109,7 +91,7 @@ __global__ void __launch_bounds__(kTokenThreads) castle_token_linear_kernel(cons
   for (int c = lane; c < chunks; c += 32) {
     float wv[WR][V];
 #pragma unroll
-    for (int i = 0; i < WR; ++i) Wide<T>::unpack(q[i], wv[i]);
+    for (int i = 0; i < WR; ++i) Vec<T>::unpack(q[i], wv[i]);
     if (c + 32 < chunks) {
 #pragma unroll
       for (int i = 0; i < WR; ++i) q[i] = wrow[i][c + 32];
@@ -135,8 +117,11 @@ __global__ void __launch_bounds__(kTokenThreads) castle_token_linear_kernel(cons
     for (int r = 0; r < R; ++r) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc[i][r] += __shfl_xor_sync(0xffffffffu, acc[i][r], o);
-      if (lane == i * R + r && n0 + i < p.N && r < p.rows)
-        reinterpret_cast<T*>(p.y)[(int64_t)r * p.N + n0 + i] = Wide<T>::cast(acc[i][r]);
+      if (lane == i * R + r && n0 + i < p.N && r < p.rows) {
+        T* y = reinterpret_cast<T*>(p.y) + (int64_t)r * p.N + n0 + i;
+        if constexpr (sizeof(T) == 4) *y = acc[i][r];
+        else *y = Elem<T>::from_f(acc[i][r]);
+      }
     }
 }
 

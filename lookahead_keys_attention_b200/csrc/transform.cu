@@ -27,9 +27,6 @@ struct TransformParams {
 constexpr int kTransformThreads = 256, kTransformLines = 4;
 constexpr int kTransformTable = 2048;   // cos/sin pairs a block keeps in shared memory
 
-// Eight elements as they lie
-template <typename T> struct alignas(16) Raw8 { uint4 q[sizeof(T) / 2]; };
-
 // x / d by a multiplication with inv = ceil(2^32 / d), exact for x * d < 2^32; inv = 0: a plain division (d of 1, or beyond 2^15)
 __host__ inline uint32_t inverse_of(int d) { return d > 1 && d <= 1 << 15 ? (uint32_t)((((uint64_t)1 << 32) + d - 1) / d) : 0; }
 __device__ __forceinline__ int quotient(int x, int d, uint32_t inv) { return inv ? (int)__umulhi((uint32_t)x, inv) : x / d; }

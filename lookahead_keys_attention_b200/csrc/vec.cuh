@@ -4,6 +4,8 @@
 
 namespace castle {
 
+template <typename T> struct Raw8 { uint4 q[sizeof(T) / 2]; };   // as they lie
+
 template <typename T> __device__ __forceinline__ void load8(const T* p, float* v) {
   uint4 q = *reinterpret_cast<const uint4*>(p);
   const uint32_t* u = &q.x;
