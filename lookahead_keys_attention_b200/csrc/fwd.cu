@@ -155,6 +155,134 @@ static FwdPlan fwd_plan(int64_t pairs, int64_t nblk, int dim_head) {
   return f;
 }
 
+// ---------------------------------------------------------------------------------------------
+// The arithmetic of a step, as both kernels below run it.  A thread has 64 values of a 128 x 128 tile, columns cbase.. of one row;
+// tensor-memory addresses have the lanes of its warp.
+
+// Gate A = sigmoid(scale * Z), kept for j > k (rows k, columns j), into its swizzled tile
+template <typename T>
+__device__ __forceinline__ void gate_pass(uint32_t z, uint8_t* tile, int row, int cbase, float half_scale, bool diag) {
+  float v[2][32];
+  tmem_ld32(z + cbase, v[0]);
+  tmem_ld32(z + cbase + 32, v[1]);
+  tmem_ld_wait();
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const float2 a = sigmoid2(make_float2(v[c][j], v[c][j + 1]), half_scale);
+      v[c][j] = a.x; v[c][j + 1] = a.y;
+    }
+    if (diag) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[c][j] = (cbase + c * 32 + j > row) ? v[c][j] : 0.f;
+    }
+    store_row32<T>(tile, kPanelBytes, row, cbase + c * 32, v[c]);
+  }
+}
+
+// The 16-bit copy of W; a group has half of the columns
+template <typename T, int D>
+__device__ __forceinline__ void state_copy(uint32_t w, uint8_t* tile, int row, int grp) {
+#pragma unroll
+  for (int c = 0; c < D / 64; ++c) {
+    const int c0 = (grp * (D / 64) + c) * 32;
+    float v[32];
+    tmem_ld32(w + c0, v);
+    tmem_ld_wait();
+    store_row32<T>(tile, kPanelBytes, row, c0, v);
+  }
+}
+
+// The final state of a walk, U[K], into the caller's tensors (either may be null)
+template <int D>
+__device__ __forceinline__ void state_out(const FwdParams& p, uint32_t w, int bh, int K, int row, int grp) {
+  const int krow = K * kBlk + row;
+#pragma unroll 1
+  for (int c = 0; c < D / 64; ++c) {
+    const int c0 = (grp * (D / 64) + c) * 32;
+    float v[32];
+    tmem_ld32(w + c0, v);
+    tmem_ld_wait();
+    if (krow < p.N) {   // (the load is the whole warp's)
+      if (p.w_state != nullptr) store_u32(p.w_state, CASTLE_F32, ((int64_t)bh * p.N + krow) * D + c0, v);
+      if (p.u_out.ptr != nullptr)
+        store_u32(p.u_out.ptr, p.u_dtype, bh / p.H * p.u_out.stride_b + bh % p.H * p.u_out.stride_h + (int64_t)krow * p.u_out.stride_n + c0, v);
+    }
+  }
+}
+
+// S/scale = Sc/scale - silu(Su)/scale (rows i, columns k); Su comes in pieces of 16 columns, one ahead of the arithmetic
+__device__ __forceinline__ void score_pass(uint32_t su, uint32_t sc, float half_scale, float (&s)[2][32]) {
+  float w[2][16];
+  tmem_ld16(su, w[0]);
+  tmem_ld32(sc, s[0]);
+  tmem_ld32(sc + 32, s[1]);
+  tmem_ld_wait();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (q < 3) tmem_ld16(su + 16 * (q + 1), w[(q + 1) & 1]);
+    float* sq = &s[q >> 1][(q & 1) * 16];
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      const float2 u = make_float2(w[q & 1][j], w[q & 1][j + 1]);
+      const float2 x = fma2(u, neg_sigmoid2(u, half_scale), make_float2(sq[j], sq[j + 1]));
+      sq[j] = x.x; sq[j + 1] = x.y;
+    }
+    if (q < 3) tmem_ld_wait();
+  }
+}
+
+// Causal mask of a diagonal block and the largest of the 64
+__device__ __forceinline__ float masked_max(float (&s)[2][32], int row, int cbase, bool diag) {
+  if (diag) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int j = 0; j < 32; ++j) s[c][j] = (cbase + c * 32 + j <= row) ? s[c][j] : -INFINITY;
+  }
+  float mx = s[0][0];
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int j = 0; j < 32; ++j) mx = fmaxf(mx, s[c][j]);
+  return mx;
+}
+
+// P = exp(scale * v - max) as packed pairs into tensor memory (masked entries give 0) and its sum.  An eighth of the exponentials at
+// dim_head 64, where the special-function unit is the busiest (53 %), is computed on the FMA pipe: 752 -> 746 us at B=4 N=4096
+// H=16; no gain at 128.
+template <typename T, int D>
+__device__ __forceinline__ float exp_pass(float (&s)[2][32], float sl2, float mb, uint32_t dst) {
+  float2 lsum = splat(0.f);
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const float2 x = fma2(make_float2(s[c][j], s[c][j + 1]), splat(sl2), splat(-mb));
+      const float2 e = D == 64 && j % 16 == 0 ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));
+      s[c][j] = e.x;
+      s[c][j + 1] = e.y;
+      lsum = add2(lsum, make_float2(s[c][j], s[c][j + 1]));
+    }
+    tmem_st_packed32<T>(dst + c * 16, s[c]);
+  }
+  return lsum.x + lsum.y;
+}
+
+// A group's columns of the un-normalised P @ Vc of one tile
+template <typename T, int D>
+__device__ __forceinline__ void store_partial(const FwdParams& p, int64_t tile, int row, int grp, const float (&o)[D / 64][32]) {
+#pragma unroll
+  for (int c = 0; c < D / 64; ++c) {
+    uint4* dst = reinterpret_cast<uint4*>(p.part_o) + (tile * (D / 8) + (grp * (D / 64) + c) * 4) * kBlk + row;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      dst[j * kBlk] = make_uint4(Elem<T>::pack2(o[c][8 * j], o[c][8 * j + 1]), Elem<T>::pack2(o[c][8 * j + 2], o[c][8 * j + 3]),
+                                 Elem<T>::pack2(o[c][8 * j + 4], o[c][8 * j + 5]), Elem<T>::pack2(o[c][8 * j + 6], o[c][8 * j + 7]));
+  }
+}
+
 template <typename T, int D, bool TM>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
@@ -283,25 +411,7 @@ castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_
       // ---- gate A = sigmoid(scale * Z), kept for j > k (rows k, columns j)
       wait_warp(bar_z, ph);
       PIPE_MARK(0);
-      {
-        float v[2][32];
-        tmem_ld32(trow + C_R1 + cbase, v[0]);
-        tmem_ld32(trow + C_R1 + cbase + 32, v[1]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float2 a = sigmoid2(make_float2(v[c][j], v[c][j + 1]), half_scale);
-            v[c][j] = a.x; v[c][j + 1] = a.y;
-          }
-          if (diag) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[c][j] = (cbase + c * 32 + j > row) ? v[c][j] : 0.f;
-          }
-          store_row32<T>(sA(n), kPanelBytes, row, cbase + c * 32, v[c]);
-        }
-      }
+      gate_pass<T>(trow + C_R1, sA(n), row, cbase, half_scale, diag);
       PIPE_MARK(1);
       if (B2) {
         // Y has the scores of the step before, so its products are done: its buffers are filled for the next one
@@ -309,16 +419,7 @@ castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_
         if (more && warp == 1 && elect_one()) load_step(n + 1);
         __syncwarp();
       }
-      if (!pre) {   // the 16-bit copy of W (before this step's update)
-#pragma unroll
-        for (int c = 0; c < NP; ++c) {
-          const int c0 = (grp * NP + c) * 32;
-          float v[32];
-          tmem_ld32(trow + C_W + c0, v);
-          tmem_ld_wait();
-          store_row32<T>(sWb, kPanelBytes, row, c0, v);
-        }
-      }
+      if (!pre) state_copy<T, D>(trow + C_W, sWb, row, grp);   // before this step's update
       if (TM && !pre) {
         if (!B2) { tc_fence_before(); sync_pair(3 + quarter); tc_fence_after(); }   // the masked T goes over Z
 #pragma unroll
@@ -392,18 +493,7 @@ castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_
     // ---- W_K is now U[K] (in the CTA that walked to the last query block)
     if (I_end == p.nblk && (p.u_out.ptr != nullptr || p.w_state != nullptr)) {
       wait_warp(bar_w, (uint32_t)(I_end - 1 - K) & 1u);
-#pragma unroll 1
-      for (int c = 0; c < NP; ++c) {
-        const int c0 = (grp * NP + c) * 32;
-        float v[32];
-        tmem_ld32(trow + C_W + c0, v);
-        tmem_ld_wait();
-        if (k0 + row < p.N) {   // (the load is the whole warp's)
-          if (p.w_state != nullptr) store_u32(p.w_state, CASTLE_F32, ((int64_t)bh * p.N + k0 + row) * D + c0, v);
-          if (p.u_out.ptr != nullptr)
-            store_u32(p.u_out.ptr, p.u_dtype, b * p.u_out.stride_b + h * p.u_out.stride_h + (int64_t)(k0 + row) * p.u_out.stride_n + c0, v);
-        }
-      }
+      state_out<D>(p, trow + C_W, bh, K, row, grp);
     }
     if (p.store_caches && warp == 0 && elect_one()) bulk_wait0();
   } else {
@@ -425,65 +515,21 @@ castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_
       const int irow = I * kBlk + row;
       wait_warp(bar_s, ph_m);
       PIPE_MARK(8);
-      // S/scale = Sc/scale - silu(Su)/scale (rows i, columns k); Su comes in pieces of 16 columns, one ahead of the arithmetic
       float s[2][32];
-      {
-        float w[2][16];
-        tmem_ld16(trow + C_R2 + cbase, w[0]);
-        tmem_ld32(trow + C_R3 + cbase, s[0]);
-        tmem_ld32(trow + C_R3 + cbase + 32, s[1]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (q < 3) tmem_ld16(trow + C_R2 + cbase + 16 * (q + 1), w[(q + 1) & 1]);
-          float* sq = &s[q >> 1][(q & 1) * 16];
-#pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            const float2 u = make_float2(w[q & 1][j], w[q & 1][j + 1]);
-            const float2 x = fma2(u, neg_sigmoid2(u, half_scale), make_float2(sq[j], sq[j + 1]));
-            sq[j] = x.x; sq[j + 1] = x.y;
-          }
-          if (q < 3) tmem_ld_wait();
-        }
-      }
+      score_pass(trow + C_R2 + cbase, trow + C_R3 + cbase, half_scale, s);
       tc_fence_before();
       if (B2) {   // Su is in registers; at dim_head 128 its columns take P @ Vc first
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_r);
       }
-      if (diag) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) s[c][j] = (cbase + c * 32 + j <= row) ? s[c][j] : -INFINITY;
-      }
-      float mx = s[0][0];
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int j = 0; j < 32; ++j) mx = fmaxf(mx, s[c][j]);
+      float mx = masked_max(s, row, cbase, diag);
       red_max[grp][row] = mx;
       PIPE_MARK(9);
       sync_pair(7 + quarter);
       tc_fence_after();
       mx = fmaxf(mx, red_max[grp ^ 1][row]);   // column 0 is never masked, so the maximum is finite
       const float mb = mx * sl2;
-      float2 lsum = splat(0.f);
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          const float2 x = fma2(make_float2(s[c][j], s[c][j + 1]), splat(sl2), splat(-mb));
-          // exp(scale*v - max); masked entries give 0.  An eighth of them at dim_head 64, where the special-function unit is
-          // the busiest (53 %), is computed on the FMA pipe: 752 -> 746 us at B=4 N=4096 H=16; no gain at 128.
-          const float2 e = D == 64 && j % 16 == 0 ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));
-          s[c][j] = e.x;
-          s[c][j + 1] = e.y;
-          lsum = add2(lsum, make_float2(s[c][j], s[c][j + 1]));
-        }
-        tmem_st_packed32<T>(trow + C_R3 + cbase / 2 + c * 16, s[c]);   // P over Sc, which everybody has read
-      }
-      red_sum[grp][row] = lsum.x + lsum.y;
+      red_sum[grp][row] = exp_pass<T, D>(s, sl2, mb, trow + C_R3 + cbase / 2);   // P over Sc, which everybody has read
       tmem_st_wait();
       tc_fence_before();
       sync_y();
@@ -511,16 +557,7 @@ castle_fwd_pipe_kernel(const FwdParams p, const __grid_constant__ CUtensorMap m_
       else if (lane == 0) mbar_arrive(bar_r);
       PIPE_MARK(12);
       if (B2) issue_sc(I + 1);   // over P and P @ Vc, which everybody has read
-      if (irow < p.N) {
-#pragma unroll
-        for (int c = 0; c < NP; ++c) {
-          uint4* dst = reinterpret_cast<uint4*>(p.part_o) + (tile * (D / 8) + (grp * NP + c) * 4) * kBlk + row;
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            dst[j * kBlk] = make_uint4(Elem<T>::pack2(o[c][8 * j], o[c][8 * j + 1]), Elem<T>::pack2(o[c][8 * j + 2], o[c][8 * j + 3]),
-                                       Elem<T>::pack2(o[c][8 * j + 4], o[c][8 * j + 5]), Elem<T>::pack2(o[c][8 * j + 6], o[c][8 * j + 7]));
-        }
-      }
+      if (irow < p.N) store_partial<T, D>(p, tile, row, grp, o);
     }
   }
   tc_fence_before();
@@ -689,47 +726,15 @@ castle_fwd_pipe64_kernel(const FwdParams p, const __grid_constant__ CUtensorMap 
       wait_warp(bar_z, n);
       if (more && next.first() && warp == 0 && elect_one()) load_resident(sQu, m_qu, bar_qu, next.w);   // this Z was the last with the old one
       __syncwarp();
-      {
-        float v[2][32];
-        tmem_ld32(trow + C_R1 + cbase, v[0]);
-        tmem_ld32(trow + C_R1 + cbase + 32, v[1]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float2 a = sigmoid2(make_float2(v[q][j], v[q][j + 1]), half_scale);
-            v[q][j] = a.x; v[q][j + 1] = a.y;
-          }
-          if (diag) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[q][j] = (cbase + q * 32 + j > row) ? v[q][j] : 0.f;
-          }
-          store_row32<T>(sA(n), kPanelBytes, row, cbase + q * 32, v[q]);
-        }
-      }
+      gate_pass<T>(trow + C_R1, sA(n), row, cbase, half_scale, diag);
       // Y has the scores of the step before, so its products are done: its buffers are filled for the next one
       if (n > 0) wait_warp(bar_r, n - 1);
       if (more && warp == 1 && elect_one()) load_step(n + 1, next);
       __syncwarp();
       if (diag && n > 0) {   // W is U of the walk before
-        if (p.u_out.ptr != nullptr || p.w_state != nullptr) {
-          const int c0 = grp * 32, krow = last.K * kBlk + row;
-          float v[32];
-          tmem_ld32(trow + C_W + c0, v);
-          tmem_ld_wait();
-          if (krow < p.N) {   // (the load is the whole warp's)
-            if (p.w_state != nullptr) store_u32(p.w_state, CASTLE_F32, ((int64_t)last.bh * p.N + krow) * D + c0, v);
-            if (p.u_out.ptr != nullptr)
-              store_u32(p.u_out.ptr, p.u_dtype, last.bh / p.H * p.u_out.stride_b + last.bh % p.H * p.u_out.stride_h + (int64_t)krow * p.u_out.stride_n + c0, v);
-          }
-        }
-      } else {   // the 16-bit copy of W (before this step's update)
-        const int c0 = grp * 32;
-        float v[32];
-        tmem_ld32(trow + C_W + c0, v);
-        tmem_ld_wait();
-        store_row32<T>(sWb, kPanelBytes, row, c0, v);
+        if (p.u_out.ptr != nullptr || p.w_state != nullptr) state_out<D>(p, trow + C_W, last.bh, last.K, row, grp);
+      } else {
+        state_copy<T, D>(trow + C_W, sWb, row, grp);   // before this step's update
       }
       if (TM) {
 #pragma unroll
@@ -789,15 +794,7 @@ castle_fwd_pipe64_kernel(const FwdParams p, const __grid_constant__ CUtensorMap 
     // ---- the state of the last walk
     if (p.u_out.ptr != nullptr || p.w_state != nullptr) {
       wait_warp(bar_w, n - 1);
-      const int c0 = grp * 32, krow = last.K * kBlk + row;
-      float v[32];
-      tmem_ld32(trow + C_W + c0, v);
-      tmem_ld_wait();
-      if (krow < p.N) {
-        if (p.w_state != nullptr) store_u32(p.w_state, CASTLE_F32, ((int64_t)last.bh * p.N + krow) * D + c0, v);
-        if (p.u_out.ptr != nullptr)
-          store_u32(p.u_out.ptr, p.u_dtype, last.bh / p.H * p.u_out.stride_b + last.bh % p.H * p.u_out.stride_h + (int64_t)krow * p.u_out.stride_n + c0, v);
-      }
+      state_out<D>(p, trow + C_W, last.bh, last.K, row, grp);
     }
     if (p.store_caches && warp == 0 && elect_one()) bulk_wait0();
   } else {
@@ -826,62 +823,18 @@ castle_fwd_pipe64_kernel(const FwdParams p, const __grid_constant__ CUtensorMap 
       wait_warp(bar_s, n);
       if (turn && warp == 8 && elect_one()) load_resident(sKc, m_kc, bar_kc, next.w);   // these scores were the last with the old one
       __syncwarp();
-      // S/scale = Sc/scale - silu(Su)/scale (rows i, columns k); Su comes in pieces of 16 columns, one ahead of the arithmetic
       float s[2][32];
-      {
-        float w[2][16];
-        tmem_ld16(trow + C_R2 + cbase, w[0]);
-        tmem_ld32(trow + C_R3 + cbase, s[0]);
-        tmem_ld32(trow + C_R3 + cbase + 32, s[1]);
-        tmem_ld_wait();
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (q < 3) tmem_ld16(trow + C_R2 + cbase + 16 * (q + 1), w[(q + 1) & 1]);
-          float* sq = &s[q >> 1][(q & 1) * 16];
-#pragma unroll
-          for (int j = 0; j < 16; j += 2) {
-            const float2 u = make_float2(w[q & 1][j], w[q & 1][j + 1]);
-            const float2 x = fma2(u, neg_sigmoid2(u, half_scale), make_float2(sq[j], sq[j + 1]));
-            sq[j] = x.x; sq[j + 1] = x.y;
-          }
-          if (q < 3) tmem_ld_wait();
-        }
-      }
+      score_pass(trow + C_R2 + cbase, trow + C_R3 + cbase, half_scale, s);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_r);   // Su is in registers
-      if (diag) {
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-#pragma unroll
-          for (int j = 0; j < 32; ++j) s[q][j] = (cbase + q * 32 + j <= row) ? s[q][j] : -INFINITY;
-      }
-      float mx = s[0][0];
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-#pragma unroll
-        for (int j = 0; j < 32; ++j) mx = fmaxf(mx, s[q][j]);
+      float mx = masked_max(s, row, cbase, diag);
       red_max[grp][row] = mx;
       sync_pair(7 + quarter);
       tc_fence_after();
       mx = fmaxf(mx, red_max[grp ^ 1][row]);   // column 0 is never masked, so the maximum is finite
       const float mb = mx * sl2;
-      float2 lsum = splat(0.f);
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          const float2 x = fma2(make_float2(s[q][j], s[q][j + 1]), splat(sl2), splat(-mb));
-          // exp(scale*v - max); masked entries give 0.  An eighth of them, where the special-function unit is the busiest (53 %), is
-          // computed on the FMA pipe: 752 -> 746 us at B=4 N=4096 H=16.
-          const float2 e = j % 16 == 0 ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));
-          s[q][j] = e.x;
-          s[q][j + 1] = e.y;
-          lsum = add2(lsum, make_float2(s[q][j], s[q][j + 1]));
-        }
-        tmem_st_packed32<T>(trow + C_R3 + cbase / 2 + q * 16, s[q]);   // P over Sc, which everybody has read
-      }
-      red_sum[grp][row] = lsum.x + lsum.y;
+      red_sum[grp][row] = exp_pass<T, D>(s, sl2, mb, trow + C_R3 + cbase / 2);   // P over Sc, which everybody has read
       tmem_st_wait();
       tc_fence_before();
       if (first && warp == 9 && elect_one()) resident(sVc, m_vcc, bar_vc, i, c.w);
@@ -898,8 +851,8 @@ castle_fwd_pipe64_kernel(const FwdParams p, const __grid_constant__ CUtensorMap 
         reinterpret_cast<float2*>(p.part_ml)[tile * kBlk + row] = make_float2(mx * p.scale, red_sum[0][row] + red_sum[1][row]);
       if (next.ok && warp == 9 && elect_one()) mbar_wait_lazy_abort(bar_in + ((n + 1) & 1), ((n + 1) >> 1) & 1, abortp);   // Qc for the next Sc
       wait_warp(bar_o, n);
-      float o[32];
-      tmem_ld32(trow + C_O + grp * 32, o);
+      float o[1][32];
+      tmem_ld32(trow + C_O + grp * 32, o[0]);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
@@ -911,13 +864,7 @@ castle_fwd_pipe64_kernel(const FwdParams p, const __grid_constant__ CUtensorMap 
         issue_sc(n + 1);
       }
       __syncwarp();
-      if (irow < p.N) {
-        uint4* dst = reinterpret_cast<uint4*>(p.part_o) + (tile * (D / 8) + grp * 4) * kBlk + row;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          dst[j * kBlk] = make_uint4(Elem<T>::pack2(o[8 * j], o[8 * j + 1]), Elem<T>::pack2(o[8 * j + 2], o[8 * j + 3]),
-                                     Elem<T>::pack2(o[8 * j + 4], o[8 * j + 5]), Elem<T>::pack2(o[8 * j + 6], o[8 * j + 7]));
-      }
+      if (irow < p.N) store_partial<T, D>(p, tile, row, grp, o);
       if (turn) ++i;
       first = turn;
       ++n;
