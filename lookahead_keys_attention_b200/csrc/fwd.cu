@@ -77,9 +77,9 @@ __device__ inline int walk_cut(int walk, int nseg, int seg) {
 // and Sc into P, issues P @ Vc and stores the partial.  One CTA per SM; a group has 256 threads, each with 64 values
 // of a 128x128 tile.
 //
-// The masked T[I,I] = tril(Qc[I] @ Vu[I]^T) is the same for every key block, so from four query blocks on a small kernel
-// computes the tiles once (castle_fwd_t_kernel) and X's threads carry theirs from global memory to tensor memory; that
-// takes a product, an elementwise pass and two hand-offs out of X's chain.  Below that (TM = false) X forms T itself.
+// The masked T[I,I] = tril(Qc[I] @ Vu[I]^T) is the same for every key block, so where that pays (fwd_plan, from kTmBlocks query
+// blocks on) a small kernel computes the tiles once (castle_fwd_t_kernel) and X's threads carry theirs from global memory to tensor
+// memory; that takes a product, an elementwise pass and two hand-offs out of X's chain.  Elsewhere (TM = false) X forms T itself.
 //
 // Tensor memory: W | R1 | R2 | R3 (| Tm), D + 3 * 128 (+ 64) columns.
 //   R1  Z; at dim_head 128 then the masked T as packed pairs (first operand of the Su correction)
@@ -151,7 +151,16 @@ static FwdPlan fwd_plan(int64_t pairs, int64_t nblk, int dim_head) {
   // what comes next), so it is for short walks, and the longer they are the more of them there must be.  us of the kernel, walk after walk / a
   // CTA per walk, pairs x blocks: 128 x 8 124 / 145, 48 x 12 103 / 110, 128 x 13 286 / 314, 128 x 17 460 / 485, 128 x 20 622 / 648, 64 x 24
   // 442 / 447, 64 x 32 748 / 739; few: 32 x 8 45 / 47, 24 x 8 42 / 40, 40 x 12 102 / 104, 24 x 20 131 / 129, 20 x 24 158 / 148, 8 x 24 88 / 78.
-  f.persistent = dim_head == 64 && f.nseg == 1 && nblk <= 24 && (9.f * load >= (float)nblk || nblk < kSplitMin);
+  // Below eight blocks a CTA per walk is the better one while no SM's second walk outlasts the longest one: in one wave, or if the
+  // second walk, which starts behind a first of nblk - 148 / pairs steps and is as short, ends in time (start and end of a walk count
+  // 2.4 steps): 2 (nblk - 148 / pairs + 2.4) <= nblk + 2.4.  us of a forward, walk after walk / a CTA per walk: 37 x 1 11.3 / 10.9, 148 x 1
+  // 13.2 / 12.7, 163 x 1 17.1 / 20.2, 71 x 2 16.4 / 16.0, 83 x 2 17.6 / 20.9, 42 x 3 20.2 / 19.6, 51 x 3 20.7 / 21.2, 41 x 4 24.2 / 23.1, 48 x 4 24.8 /
+  // 25.4, 34 x 5 28.0 / 26.5, 45 x 5 30.0 / 32.1, 30 x 6 32.1 / 30.3, 39 x 6 33.9 / 35.7, 26 x 7 36.2 / 34.1, 34 x 7 38.5 / 39.7.
+  // Not here: two CTAs an SM, a walk each, in half the tensor memory.  Some sizes would be 3 to 5 % faster than walk after walk (500 x 1
+  // 27.2 / 28.6, 256 x 2 35.8 / 37.0, 256 x 3 62.6 / 65.5), the others of more than a wave are up to 20 % slower (2048 x 1 95.0 / 92.1, 500 x 3
+  // 117 / 108, 256 x 7 270 / 224): not worth a third kernel.
+  const bool few = pairs * nblk <= 148 || (float)pairs * ((float)nblk + 2.4f) <= 296.f;
+  f.persistent = dim_head == 64 && f.nseg == 1 && nblk <= 24 && (nblk < kSplitMin ? !few : 9.f * load >= (float)nblk);
   return f;
 }
 

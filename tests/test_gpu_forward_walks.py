@@ -8,8 +8,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11)])
 # pairs x blocks: 148 and 149 walks, two and three turns of the CTAs, one block each, masked last blocks, T tiles inside and up front, the
-# longest walks of the rule
-@pytest.mark.parametrize("B,H,N", [(2, 37, 256), (1, 149, 77), (1, 297, 128), (3, 99, 300), (5, 30, 1000), (7, 19, 1153), (3, 45, 1665), (2, 40, 3072)])
+# longest walks of the rule; first, for each number of blocks below eight, the last problem with a CTA per walk and the first without
+@pytest.mark.parametrize("B,H,N", [(1, 148, 77), (3, 25, 250), (6, 9, 384), (5, 11, 380), (2, 23, 511), (1, 47, 512), (4, 10, 640), (1, 41, 639), (5, 7, 768), (4, 9, 760), (1, 31, 896), (4, 8, 890),
+                                   (2, 37, 256), (1, 149, 77), (1, 297, 128), (3, 99, 300), (5, 30, 1000), (7, 19, 1153), (3, 45, 1665), (2, 40, 3072)])
 def test_walk_after_walk_matches_single_walks(dtype, tol, B, H, N):
     from lookahead_keys_attention_b200 import castle_attention, check_status
     torch.manual_seed(N)
