@@ -1,9 +1,12 @@
 """GPU: a layer's cached token as one launch (csrc/token_layer.cu) against the submodules and the step's own kernel, at the
-edges of what it takes: CTAs of a cluster without rows, two rows per lane group, the last size that fits and the next one."""
+edges of what it takes: CTAs of a cluster without rows, two rows per lane group, the last size that fits and the next one; and
+against the oracle in fp64."""
 import ctypes
 
 import pytest
 import torch
+
+from oracle import castle_oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +65,47 @@ def test_nan_and_infinity_reach_the_output():
         with torch.no_grad():
             y, _ = m(x, cache=cache_from_buffers(*bufs, 65))
         assert not bool(y.isfinite().all())
+
+
+def _exact(m, x, caches, t):
+    """The token in fp64 on the CPU, from the layer's weights and the caches as they are stored."""
+    w = {k: v.double().cpu() for k, v in m.state_dict().items()}
+    h = x.double().cpu()
+    if "norm.weight" in w:
+        h = torch.nn.functional.rms_norm(h, h.shape[-1:], w["norm.weight"], torch.finfo(torch.float32).eps)
+    qu, ku, vu, qc, kc, vc = O.split_heads(h @ w["to_all_qkv.weight"].t(), m.heads)
+    if m.rotary_emb is not None:
+        ang = t * m.rotary_emb.freqs.double().cpu()
+
+        def rotate(v):
+            a, b = v[..., 0::2], v[..., 1::2]
+            return torch.stack((a * ang.cos() - b * ang.sin(), a * ang.sin() + b * ang.cos()), -1).flatten(-2)
+        qu, ku, vu, qc, kc = map(rotate, (qu, ku, vu, qc, kc))
+    out, cache = O.castle_decode_step(qc, kc, vc, qu, ku, vu, O.Cache(*(c.double().cpu() for c in caches)), m.scale)
+    return out.permute(0, 2, 1, 3).flatten(2) @ w["combine_heads.weight"].t(), cache
+
+
+@pytest.mark.parametrize("dtype", [BF16, F16, F32])
+@pytest.mark.parametrize("B,H,d,t,dim,norm,rotary", [(1, 1, 32, 0, 8, False, False), (1, 8, 64, 300, 512, True, True), (2, 8, 64, 128, 512, False, False),
+                                                      (3, 5, 32, 33, 480, True, True), (1, 3, 128, 250, 896, True, False)])
+def test_one_launch_against_fp64(dtype, B, H, d, t, dim, norm, rotary):
+    from lookahead_keys_attention_b200 import Castle, cache_from_buffers, check_status
+    assert _fits(dtype, B, H, d, t, dim, dim) == 1
+    torch.manual_seed(dim + t)
+    m = Castle(dim, heads=H, dim_head=d, prenorm=norm, rotary_emb=rotary)
+    if norm:
+        torch.nn.init.uniform_(m.norm.weight, 0.5, 1.5)
+    m.to("cuda", dtype)
+    x = torch.randn(B, 1, dim, device="cuda").to(dtype)
+    bufs = [torch.randn(B, H, t + 4, d, device="cuda").to(dtype) for _ in range(4)]
+    want, caches = _exact(m, x, [b[:, :, :t] for b in bufs], t)
+    with torch.no_grad():
+        y, new = m(x, cache=cache_from_buffers(*bufs, t))
+    # Roundings to the type between x and the result, at most half a unit (u) each: the norm, the new rows, U, the head outputs and
+    # the result, and u of a score moves a probability by no more than the row does; the rotation has four of its own (its cosines and
+    # sines, two products, their sum), its angle another 2^-24 t.  fp32: the sums' order and exp, some ten units.
+    u = {BF16: 2.0 ** -9, F16: 2.0 ** -12, F32: 4 * 2.0 ** -24}[dtype]
+    tol = (6 + 4 * rotary) * u + rotary * t * 2.0 ** -24
+    for a, b in zip((y, *new), (want, *caches)):
+        assert a.shape == b.shape and (a.double().cpu() - b).norm() <= tol * b.norm()
+    check_status()
