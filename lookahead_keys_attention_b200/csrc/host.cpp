@@ -665,7 +665,9 @@ float norm_eps(const Layer& l) { return (float)l.eps.value_or(std::numeric_limit
 // host 8 to 10 us, an own one 4, and such calls are bound by the host; on the GPU the library is 1 to 2 us faster in 16 bits
 // (us, own / library: 197 x 512 -> 3072 4.9 / 3.4, 512 x 512 -> 3072 9.1 / 4.3, 2048 x 512 -> 3072 14.7 / 8.3) and slower in
 // fp32 but where the tiles are many (512 x 128 -> 768 8.6 / 6.2, 512 x 768 -> 128 10.2 / 14.4, its weight's gradient 7.0 / 10.3,
-// 197 x 512 -> 3072 33.6 / 25.4).  From some 1024 positions on the GPU is the bound.  A graph's replay costs the host nothing.
+// 197 x 512 -> 3072 33.6 / 25.4).  From some 1024 positions on the GPU is the bound.  A graph's replay costs the host nothing, so a
+// capture takes the library's products; the two add in different orders, so a replay and an eager call differ by fp32 rounding of the
+// sums (and a 16-bit result now and then by its last place).  A loop whose host runs ahead of the GPU pays the 1 to 2 us.
 bool small_product(int64_t rows, int64_t m, int64_t n, int64_t k, at::ScalarType t) {
   const bool f32 = t == at::kFloat;
   if (rows > 1024 || 2 * m * n * k > (f32 ? 128000000LL : 1000000000LL)) return false;

@@ -108,9 +108,9 @@ __global__ void __launch_bounds__(kNormThreads) castle_rmsnorm_dw_kernel(const T
 }
 
 // Both gradients in one pass over dy and x: a warp takes every eighth row of its CTA's range, whole (C x 256 columns), the next
-// row on its way meanwhile, and keeps its share of the weight's gradient in registers.  us of both gradients, before (a
-// pass for each) -> now: 16384 x 512 bf16 23.0 -> 12.6, fp32 37.2 -> 17.9 (the bytes take 7.7 and 15.4 from memory), 50000 x 512 bf16 54 -> 35, 200 x 512
-// bf16 12.4 -> 8.2.
+// row on its way meanwhile, and keeps its share of the weight's gradient in registers.  us of both gradients with the sum of the
+// partials, replayed from a graph, a pass for each / so: 16384 x 512 bf16 15.6 / 10.2, fp32 30.9 / 16.6 (the bytes take 7.7 and 15.4 from
+// memory), 50000 x 512 bf16 48.9 / 33.8, 200 x 512 bf16 5.7 / 4.7, 512 x 128 fp32 5.5 / 4.3.
 template <typename T, int C>
 __global__ void __launch_bounds__(kNormThreads, 2) castle_rmsnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ w,
                                                                              const float* __restrict__ rstd, T* __restrict__ dx,

@@ -58,10 +58,11 @@ __device__ __forceinline__ uint32_t mbar_wait(uint64_t* bar, uint32_t parity, vo
   return poll_limit;
 }
 
-// The same wait with the abort flag looked at on every 64th poll only.  With two CTAs per SM (the dim_head-64
-// forward) the flag reads of one CTA's waiting threads share the shared-memory port with the other CTA's
-// products and passes: 0.971 against 0.978 ms on the bench workload, same GPU.  (With one CTA per SM, in the backward,
-// the same change measured slower: there the flag read paces the polls.)
+// The same wait with the abort flag looked at on every 64th poll only: the flag reads of one group's polling lanes share the
+// shared-memory port with the other group's products and passes.  us of a forward, so / with the flag read at every poll:
+// 8 x 16 x 2049 x 64 562 / 577, 16 x 8 x 1024 x 64 150 / 152, 1 x 8 x 8190 x 128 701 / 708, 4 x 16 x 4096 x 64 925 / 924.  (The waits of
+// the dim_head-128 backward's loading warps: no difference.  In the dim_head-64 backward, where whole groups poll, it was slower: there
+// the flag read paces the polls.)
 __device__ __forceinline__ void mbar_wait_lazy_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t i = 0; i < kWaitPollLimit; ++i) {
     if (mbar_try_wait(bar, parity)) return;

@@ -9,11 +9,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("B,H,N,d", [
-    (2, 3, 384, 64), (2, 3, 385, 64), (2, 3, 384, 128), (2, 3, 512, 128),      # three and four query blocks: T inside / up front
+    (2, 3, 384, 64), (2, 3, 385, 64), (2, 3, 384, 128), (2, 3, 512, 128),      # three and four query blocks, T inside
     (1, 1, 1024, 64), (1, 1, 1023, 128), (1, 2, 1500, 64), (1, 2, 2049, 128),  # three parts
     (1, 12, 1100, 64), (1, 9, 1281, 128),                                      # two parts
     (3, 7, 1030, 64), (3, 7, 1030, 128),                                       # whole walks, more than one wave
-    (38, 4, 257, 64), (30, 3, 641, 64), (100, 3, 1, 64)])                      # many short walks
+    (38, 4, 257, 64), (30, 3, 641, 64), (100, 3, 1, 64),                       # many short walks
+    (12, 4, 1500, 64), (28, 1, 2000, 64), (16, 1, 2750, 128)])                 # T up front: walk after walk, a CTA per walk
 def test_forward_dispatch(B, H, N, d):
     from lookahead_keys_attention_b200 import castle_attention_packed, check_status
     torch.manual_seed(N + d)
