@@ -18,39 +18,42 @@
 //
 // Shared memory (224 KB) is time-shared: the 128x128 16-bit operands the
 // threads produce (gate A, masked T, P, dS, dSu, dZ, dT) rotate through four
-// 32 KB slots, two of which overlay input tiles that are dead by then
-// (slot 3 over Vc|dO holds dS then dT, slot 4 over Ku|spare holds P then dSu).
+// 32 KB slots, two of which overlay input tiles that are dead by then.
+//
+// What bounds a step: some 1.5 MB through shared memory (11.7 k cycles at 128 bytes a cycle) and a chain of nine products
+// with a pass behind each.  So sixteen warps do the passes and nothing else, one warp issues every product and one moves the
+// tiles: a thread that issues products waits as long as the tensor unit's queue is full, and its warp then came late to the
+// pass that everybody waited for.  A pass reports twice, on named barriers where only the issuing warp waits: when the accumulator
+// columns are in registers (the next product into them starts under the arithmetic) and when its results are in shared memory.
+// Step 19.1 k -> 15.5 k cycles; the kernel at B=4 N=4096 H=16 2390 -> 1936 us, B=16 H=8 N=1024 387 -> 332, 15 pairs of 777 78.2 -> 63.3.
 #include "bwd_common.cuh"
 
 namespace castle {
 
-constexpr int kBwdThreads = 512;
-constexpr int kPrefetchTid = 384;
+constexpr int kBwdWorkers = 512;               // warps 0-15: the passes
+constexpr int kBwdThreads = kBwdWorkers + 128; // warp 16 issues the products, warp 17 moves tiles; two more fill up the warpgroup
+// Registers a thread: the launch's 640 x 96 are shared out anew, 512 x 112 + 128 x 32 = 61440.
+constexpr int kBwdLaunchRegs = 96, kBwdWorkerRegs = 112, kBwdHelperRegs = 32;
+static_assert(kBwdWorkers * kBwdWorkerRegs + 128 * kBwdHelperRegs <= kBwdThreads * kBwdLaunchRegs, "setmaxnreg would wait forever");
 
 // Optional phase timing (debug builds only): thread 0 of CTA (0,0) stores clock64() at each phase
 // boundary of its first steps behind the fp32 workspace, which the host dumps.
 #ifdef CASTLE_PHASE_TIMING
-#define BPHASE_MARK(i) do { if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && tstep < 8) p.timing[tstep * 32 + (i)] = clock64(); } while (0)
+#define BPHASE_MARK(i) do { if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && n < 8) p.timing[n * 32 + (i)] = clock64(); } while (0)
 #else
 #define BPHASE_MARK(i) do { } while (0)
 #endif
 
-// 512 threads: warp w works on TMEM lanes 32*(w%4).. and on the 32-column chunk w/4 of a
-// 128-column accumulator, so thread (row, chunk) owns 32 values of every 128x128 tile.
-// One 128 x 64 fp32 accumulator tile from tensor memory into two swizzled 128 x 32 staging panels.
-__device__ __forceinline__ void stage_f32_tile(uint32_t taddr, uint8_t* panel0, uint8_t* panel1, uint32_t row) {
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    float v[32];
-    tmem_ld32(taddr + c * 32, v);
-    tmem_ld_wait();
-    store_row32_f32(c == 0 ? panel0 : panel1, row, v);
-  }
-}
 // Timing experiments only (never in the shipped library): drop the reduces to see what they cost.
 #ifdef CASTLE_TIMING_SKIP_REDUCE
 #define tma_reduce_add_3d(...) do { } while (0)
 #endif
+
+// Named barriers on which the passes' warps arrive and go on, and one helper warp waits.
+enum BwdEvent { kEvRead = 1, kEvStored = 2, kEvStoredT = 3, kEvStoredZ = 4, kEvDqc = 5, kEvDku = 6, kEvDvu = 7 };
+constexpr int kWorkers = 8, kEpilogue = 9;   // and those of the passes among themselves: all 512, and 9 to 11 a chunk group each
+__device__ __forceinline__ void ev_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads + 32) : "memory"); }
+__device__ __forceinline__ void ev_wait(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads + 32) : "memory"); }
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kBwdThreads, 1)
@@ -79,33 +82,35 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   uint8_t* sKc = sQu + OPB;            // resident
   uint8_t* sQc = sKc + OPB;            // per step
   uint8_t* sVu = sQc + OPB;            // per step
-  uint8_t* sVD = sVu + OPB;            // [Vc | dO] per step, later slot 3: dS -> dSu -> dT
+  uint8_t* sVD = sVu + OPB;            // [Vc | dO] per step, later slot 3: dS -> dT -> staging of dvu
   uint8_t* sVc = sVD;
   uint8_t* sdO = sVD + OPB;
-  uint8_t* sKP = sVD + SQB;            // [Ku | spare], later slot 4: P, then Ku again in the first half
-  uint8_t* sWb = sKP + SQB;
+  uint8_t* sKP = sVD + SQB;            // [Ku | spare], later slot 4: P -> dSu, then the next Ku in the first half
+  uint8_t* sWb = sKP + SQB;            // copy of W, then Ku again
   uint8_t* sGb = sWb + OPB;
   uint8_t* sA = sGb + OPB;             // slot 1: gate A
-  uint8_t* sT = sA + SQB;              // slot 2: masked T, later dZ
-  __shared__ uint64_t bar_res, bar_load, bar_vd, bar_ku, bar_mma, bar_x1, bar_x2, bar_kn, bar_w, bar_dv, bar_g;
+  uint8_t* sT = sA + SQB;              // slot 2: masked T -> dZ -> staging of dku
+  // Each of these completes once per step.
+  __shared__ uint64_t bar_res, bar_load, bar_vd, bar_ku, bar_kn;   // tiles
+  __shared__ uint64_t bar_z, bar_t, bar_w, bar_su, bar_sc, bar_dp, bar_dv, bar_da, bar_dt, bar_g, bar_x, bar_l;   // products
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
+  __shared__ float zero_s;
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const int quarter = warp & 3, cc = warp >> 2;
-  const int row = quarter * 32 + lane;
-  const int c0 = cc * 32;
   const int bh = blockIdx.x, K = blockIdx.y;
   const int b = bh / p.H, h = bh % p.H;
-  const int k0 = K * kBlkB;
+  const int k0 = K * kBlkB, walk = p.nblk - K;
 
   if (tid == 0) {
     if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
-    mbar_init(&bar_res, 1); mbar_init(&bar_load, 1); mbar_init(&bar_vd, 1); mbar_init(&bar_ku, 1); mbar_init(&bar_mma, 1);
-    mbar_init(&bar_x1, 1); mbar_init(&bar_x2, 1); mbar_init(&bar_kn, 1);
-    mbar_init(&bar_w, 1); mbar_init(&bar_dv, 1); mbar_init(&bar_g, 1);
+    uint64_t* const bars[17] = {&bar_res, &bar_load, &bar_vd, &bar_ku, &bar_kn, &bar_z, &bar_t, &bar_w,
+                                &bar_su, &bar_sc, &bar_dp, &bar_dv, &bar_da, &bar_dt, &bar_g, &bar_x, &bar_l};
+#pragma unroll
+    for (int i = 0; i < 17; ++i) mbar_init(bars[i], bars[i] == &bar_t || bars[i] == &bar_w ? 2 : 1);   // these two: the product, and the slot written next is free
     mbar_fence_init();
     abort_flag = 0;
+    zero_s = 0.f;
   }
   if (warp == 0) { tmem_alloc(&tmem_base_s, 512); tmem_relinquish(); }
   overlap_wait();   // launched while delta is being written
@@ -113,414 +118,437 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;
-  const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
   volatile int* abortp = &abort_flag;
 
-  if (tid == 0) {
-    mbar_expect_tx(&bar_res, 2 * OPB);
-    tma_load_4d(sQu, &m_qu, &bar_res, 0, k0, h, b);
-    tma_load_4d(sKc, &m_kc, &bar_res, 0, k0, h, b);
-    // first step's Qc, Vu, Ku; later steps prefetch theirs at the end of the step before
-    mbar_expect_tx(&bar_kn, OPB);
-    tma_load_4d(sKP, &m_ku, &bar_kn, 0, (p.nblk - 1) * kBlkB, h, b);
-    mbar_expect_tx(&bar_load, 2 * OPB);
-    tma_load_4d(sQc, &m_qc, &bar_load, 0, (p.nblk - 1) * kBlkB, h, b);
-    tma_load_4d(sVu, &m_vu, &bar_load, 0, (p.nblk - 1) * kBlkB, h, b);
-  }
-  // W_K starts as the forward's final state, brought in whole lines (rows of 64 floats over the threads, through the gate's slot):
-  // a row per lane, here and where the gradients are stored, took 2 us of a key block each; 1036 pairs of one block 150.5 ->
-  // 142.3 us, B=16 H=8 N=1024 402 -> 392 us
-#pragma unroll
-  for (int i = 0; i < kBlkB * (D / 4) / kBwdThreads; ++i) {
-    const int e = i * kBwdThreads + tid, r = e / (D / 4), c = e % (D / 4);
-    const float4 q = (k0 + r < p.N) ? *reinterpret_cast<const float4*>(p.w_state + ((int64_t)bh * p.N + k0 + r) * D + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-    *reinterpret_cast<float4*>(sA + (c >> 3) * kPanelB + swz_off(r, c & 7)) = q;
-  }
-  __syncthreads();
-  if (c0 < D) {
-    float v[32];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float4 q = *reinterpret_cast<const float4*>(sA + cc * kPanelB + swz_off(row, j));
-      v[4 * j] = q.x; v[4 * j + 1] = q.y; v[4 * j + 2] = q.z; v[4 * j + 3] = q.w;
-    }
-    tmem_st32(trow + C_W + c0, v);
-    tmem_st_wait();
-  }
-  mbar_wait(&bar_res, 0, abortp);
-  tc_fence_before();
-  __syncthreads();
-
-  uint32_t ph_load = 0, ph_vd = 0, ph_ku = 0, ph_mma = 0, ph_x = 0;
-  const uint32_t aQu = smem_u32(sQu), aKc = smem_u32(sKc), aQc = smem_u32(sQc), aVu = smem_u32(sVu),
-                 aVc = smem_u32(sVc), adO = smem_u32(sdO), aKP = smem_u32(sKP), aVD = smem_u32(sVD),
-                 aWb = smem_u32(sWb), aGb = smem_u32(sGb), aA = smem_u32(sA), aT = smem_u32(sT);
-  const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
-
-// (the issuing thread's warp converges before it polls)
-#define MMA_WAIT()                       \
-  __syncwarp();                          \
-  mbar_wait(&bar_mma, ph_mma, abortp);   \
-  ph_mma ^= 1;                           \
-  tc_fence_after();
-#define SMEM_TO_MMA_SYNC() \
-  fence_async_smem();      \
-  tc_fence_before();       \
-  __syncthreads();
-
-  auto issue_z = [&](uint32_t phase) {
-    mbar_wait(&bar_kn, phase, abortp);
-    tc_fence_after();
-    uint32_t base = smem_u32(smem);
-    asm volatile("" : "+r"(base));   // the descriptors are made here, not kept in registers over the step
-    gemm_kk_t<1>(tmem + C_S, base + (uint32_t)(sQu - smem), base + (uint32_t)(sKP - smem), ID_SQ_KK, false);
-    mma_commit(&bar_mma);
-  };
-  if (tid == 0) issue_z(0);
-  for (int I = p.nblk - 1; I >= K; --I) {
-    const int i0 = I * kBlkB, irow = i0 + row;
-    const bool diag = (I == K), first = (I == p.nblk - 1);
-    const bool rvalid = irow < p.N;
-#ifdef CASTLE_PHASE_TIMING
-    const int tstep = p.nblk - 1 - I;
-#endif
-    BPHASE_MARK(0);
-
-    // ---- M1: Z = Qu[K] @ Ku[I]^T was issued at the end of the step before
-    BPHASE_MARK(1);
-    MMA_WAIT();
-    BPHASE_MARK(2);
-    {  // gate A (rows k, columns j), zero unless j > k
-      float v[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), half_scale);
-        v[j] = a.x; v[j + 1] = a.y;
-      }
-      if (diag) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
-      }
-      store_row32<T>(sA, kPanelB, row, c0, v);
-    }
-    SMEM_TO_MMA_SYNC();
-    BPHASE_MARK(3);
-
-    // ---- M2: T = Qc[I] @ Vu[I]^T;  peel W_K -= A @ Vu[I], a commit each: T is masked while the state is peeled
-    if (tid == 0) {
-      mbar_wait(&bar_load, ph_load, abortp);   // Qc[I], Vu[I]
-      BPHASE_MARK(21);
-      tc_fence_after();
-      gemm_kk_t<1>(tmem + C_S, aQc, aVu, ID_SQ_KK, false);
-      mma_commit(&bar_mma);
-      gemm_km_t<8>(tmem + C_W, aA, aVu, ID_D_KM_NEG, true);
-      mma_commit(&bar_w);
-    }
-    // The reduces of the step before must have finished reading their staging tiles before these are
-    // written again.  A reduce takes a few thousand cycles to drain, so each issuing lane waits for its
-    // own as late as the first overwrite allows: here for dqc and dku (Wb and slot 2 are written by the
-    // pass below), after the next products are issued for dvu (Vc|dO is re-loaded there).
-    if ((cc == 1 || cc == 2) && quarter == 0 && lane == 0) bulk_wait_read0();
-    MMA_WAIT();
-    BPHASE_MARK(22);
-    __syncthreads();
-    BPHASE_MARK(4);
-    {  // masked T (rows i, columns j <= i), unscaled
-      float v[32];
-      tmem_ld32_lower(trow + C_S + c0, row, c0, v);
-      store_row32<T>(sT, kPanelB, row, c0, v);
-    }
-    mbar_wait(&bar_w, ph_x, abortp);
-    tc_fence_after();
-    if (c0 < D) {  // 16-bit copy of the peeled state
-      float v[32];
-      tmem_ld32(trow + C_W + c0, v);
-      tmem_ld_wait();
-      store_row32<T>(sWb, kPanelB, row, c0, v);
-    }
-    SMEM_TO_MMA_SYNC();
-    BPHASE_MARK(5);
-
-    // ---- M3: Su/scale = Qc[I] @ Wb^T + Tm @ A^T
-    if (tid == 0) {
-      tc_fence_after();
-      if (!diag) gemm_kk_t<1>(tmem + C_S, aQc, aWb, ID_SQ_KK, false);
-      gemm_kk_t<2>(tmem + C_S, aT, aA, ID_SQ_KK, !diag);
-      mma_commit(&bar_mma);
-      mbar_expect_tx(&bar_vd, 2 * OPB);   // needed at the fifth phase; each into the panel that its issuer's dvu reduce of the
-      bulk_wait_read0();                  // step before has read
-      tma_load_4d(sVc, &m_vc, &bar_vd, 0, k0, h, b);
-    }
-    if (tid == kPrefetchTid) {
-      bulk_wait_read0();
-      tma_load_4d(sdO, &m_do, &bar_vd, 0, i0, h, b);
-    }
-    // loaded here, not at the top of the step, where the wait for Z is short (2552 -> 2467 us)
-    const float lse_i = rvalid ? p.lse[(int64_t)bh * p.N + irow] : 0.f, delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
-    MMA_WAIT();
-    BPHASE_MARK(6);
-    uint32_t dpk[16];  // silu'(Su), later dSu, two 16-bit values per register
-    uint32_t ppk[16];  // P
-    {
-      float v[32], w[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncthreads();
-      BPHASE_MARK(7);
-      // ---- M4: Sc/scale = Qc[I] @ Kc[K]^T, while silu' is formed
-      if (tid == 0) {
+  if (warp >= kBwdWorkers / 32) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kBwdHelperRegs));
+    if (warp == 16) {
+      // ---- the products, in the order that the passes need them; what a pass does not wait for goes behind its commit
+      // operand addresses are made where they are used: kept in registers over the step they would be spilled
+      auto at = [&](const uint8_t* tile) {
+        uint32_t base = smem_u32(smem);
+        asm volatile("" : "+r"(base));
+        return base + (uint32_t)(tile - smem);
+      };
+      auto next = [&](int id) {
+        __syncwarp();
+        ev_wait(id, kBwdWorkers);
         tc_fence_after();
-        gemm_kk_t<1>(tmem + C_S, aQc, aKc, ID_SQ_KK, false);
-        mma_commit(&bar_mma);
+      };
+      auto issue_z = [&](uint32_t ph) {
+        mbar_wait(&bar_kn, ph, abortp);
+        tc_fence_after();
+        gemm_kk_t<1>(tmem + C_S, at(sQu), at(sKP), ID_SQ_KK, false);
+        mma_commit(&bar_z);
+      };
+      if (elect_one()) {
+        mbar_wait(&bar_res, 0, abortp);
+        issue_z(0);
       }
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 u = make_float2(v[j], v[j + 1]);
-        const float2 g = sigmoid2(u, half_scale);
-        // silu'(su) = g + silu(su) (1 - g)
-        const float2 q = mul2(mul2(u, g), splat(-1.f));   // -silu(su) / scale
-        v[j] = q.x; v[j + 1] = q.y;
-        const float2 d = fma2(mul2(q, splat(-p.scale)), fma2(g, splat(-1.f), splat(1.f)), g);
-        dpk[j / 2] = Elem<T>::pack2(d.x, d.y);
+#pragma unroll 1
+      for (int n = 0; n < walk; ++n) {
+        const uint32_t ph = n & 1;
+        const bool first = n == 0, diag = n == walk - 1;
+        next(kEvRead);     // Z
+        if (elect_one()) {
+          mbar_wait(&bar_load, ph, abortp);
+          tc_fence_after();
+          gemm_kk_t<1>(tmem + C_S, at(sQc), at(sVu), ID_SQ_KK, false);          // T = Qc[I] Vu[I]^T, while the gate is formed
+          mma_commit(&bar_t);
+        }
+        next(kEvStored);   // A
+        if (elect_one()) {
+          if (!diag) gemm_km_t<8>(tmem + C_W, at(sA), at(sVu), ID_D_KM_NEG, true);   // W_K -= A Vu[I], while T is masked; zero at the diagonal block, where nothing reads it
+          mma_commit(&bar_w);
+        }
+        next(kEvStoredT);  // masked T
+        if (elect_one()) gemm_kk_t<2>(tmem + C_S, at(sT), at(sA), ID_SQ_KK, false);    // Su/scale = T A^T + Qc[I] Wb^T, while W is copied
+        next(kEvStored);   // copy of W
+        if (elect_one()) {
+          if (!diag) gemm_kk_t<1>(tmem + C_S, at(sQc), at(sWb), ID_SQ_KK, true);
+          mma_commit(&bar_su);
+        }
+        next(kEvRead);     // Su
+        if (elect_one()) {
+          gemm_kk_t<1>(tmem + C_S, at(sQc), at(sKc), ID_SQ_KK, false);          // Sc/scale = Qc[I] Kc[K]^T, while silu' is formed
+          mma_commit(&bar_sc);
+        }
+        next(kEvRead);     // Sc
+        if (elect_one()) {
+          mbar_wait(&bar_vd, ph, abortp);
+          tc_fence_after();
+          gemm_kk_t<1>(tmem + C_S, at(sdO), at(sVc), ID_SQ_KK, false);          // dP = dO[I] Vc[K]^T, while P is formed
+          mma_commit(&bar_dp);
+        }
+        next(kEvStored);   // P
+        if (elect_one()) {
+          gemm_mm_t<8>(tmem + C_DVC, at(sKP), at(sdO), ID_D_MM, !first);        // dvc += P^T dO[I], while dS is formed
+          mma_commit(&bar_dv);
+        }
+        next(kEvRead);     // dP
+        if (!first && elect_one()) gemm_kk_t<1>(tmem + C_S, at(sGb), at(sVu), ID_SQ_KK, false);   // dA/scale = Gb Vu[I]^T + dSu^T T
+        next(kEvStored);   // dS, dSu
+        if (elect_one()) {
+          gemm_mm_t<8>(tmem + C_S, at(sKP), at(sT), ID_SQ_MM, !first);
+          mma_commit(&bar_da);
+          gemm_mm_t<8>(tmem + C_DKC, at(sVD), at(sQc), ID_D_MM, !first);        // dkc += dS^T Qc[I]
+          gemm_km_t<8>(tmem + C_X, at(sVD), at(sKc), ID_D_KM, false);           // X = dS Kc[K] + dSu Wb + dT Vu[I]
+        }
+        next(kEvRead);     // dA
+        if (elect_one()) {
+          gemm_km_t<8>(tmem + C_S, at(sKP), at(sA), ID_SQ_KM, false);           // dT = dSu A, while dZ is formed
+          mma_commit(&bar_dt);
+          if (!diag) {
+            gemm_km_t<8>(tmem + C_X, at(sKP), at(sWb), ID_D_KM, true);
+            gemm_mm_t<8>(tmem + C_G, at(sKP), at(sQc), ID_D_MM, !first);        // G += dSu^T Qc[I]
+          }
+          mma_commit(&bar_g);
+        }
+        next(kEvStoredZ);  // dZ
+        next(kEvRead);     // dT
+        if (elect_one()) gemm_mm_t<8>(tmem + C_X3, at(sT), at(sQu), ID_D_MM, false);   // X3 = dZ^T Qu[K]
+        next(kEvStored);   // masked dT
+        if (elect_one()) {
+          gemm_mm_t<8>(tmem + C_X2, at(sVD), at(sQc), ID_D_MM, false);          // X2 = dT^T Qc[I] + A^T Gb
+          gemm_km_t<8>(tmem + C_X, at(sVD), at(sVu), ID_D_KM, true);
+          mbar_wait(&bar_ku, ph, abortp);
+          tc_fence_after();
+          gemm_km_t<8>(tmem + C_DQU, at(sT), at(sWb), ID_D_KM, !first);         // dqu += dZ Ku[I]
+          mma_commit(&bar_x);
+          if (!first) gemm_mm_t<8>(tmem + C_X2, at(sA), at(sGb), ID_D_MM, true);
+          mma_commit(&bar_l);
+        }
+        next(kEvRead);     // X2, X3
+        if (!diag && elect_one()) issue_z(ph ^ 1);
       }
-      MMA_WAIT();
-      BPHASE_MARK(8);
-      // P = exp(S - lse) (rows i, columns k); into slot 4 over Ku
-      tmem_ld32(trow + C_S + c0, w);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(sl2), splat(-lse_i * kLog2e));
-        const float2 e = j % 16 == 0 ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));   // an eighth off the busiest unit: 2421 -> 2410 us
-        v[j] = e.x; v[j + 1] = e.y;
-      }
-      if (diag) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
-      }
-      if (!rvalid) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0.f;
-      }
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) ppk[j / 2] = Elem<T>::pack2(v[j], v[j + 1]);
-      store_row32<T>(sKP, kPanelB, row, c0, v);
-    }
-    SMEM_TO_MMA_SYNC();
-    BPHASE_MARK(9);
-
-    // ---- M5: dP = dO[I] @ Vc[K]^T;  dvc += P^T @ dO[I], which runs while dS is formed
-    if (tid == 0) {
-      tc_fence_after();
-      mbar_wait(&bar_vd, ph_vd, abortp);
-      gemm_kk_t<1>(tmem + C_S, adO, aVc, ID_SQ_KK, false);
-      mma_commit(&bar_mma);
-      gemm_mm_t<8>(tmem + C_DVC, aKP, adO, ID_D_MM, !first);
-      mma_commit(&bar_dv);
-    }
-    MMA_WAIT();
-    BPHASE_MARK(10);
-    ph_vd ^= 1;
-    {  // dS = P * (dP - delta) -> slot 3 (over Vc|dO); dSu = -dS * silu'(Su) -> slot 4 (over P)
-      float v[32], w[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 ds = mul2(Elem<T>::unpack2(ppk[j / 2]), add2(make_float2(v[j], v[j + 1]), splat(-delta_i)));
-        const float2 du = mul2(ds, Elem<T>::unpack2(dpk[j / 2]));
-        v[j] = ds.x; v[j + 1] = ds.y;
-        w[j] = -du.x; w[j + 1] = -du.y;
-      }
-      mbar_wait(&bar_dv, ph_x, abortp);   // dO and P have been read
-      store_row32<T>(sVD, kPanelB, row, c0, v);
-      store_row32<T>(sKP, kPanelB, row, c0, w);
-    }
-    SMEM_TO_MMA_SYNC();
-    BPHASE_MARK(11);
-
-    // ---- M6: dkc += dS^T @ Qc[I];  X = dS @ Kc[K] + dSu @ Wb;  dA/scale = Gb @ Vu[I]^T + dSu^T @ Tm
-    if (tid == 0) {
-      tc_fence_after();
-      // dA first and committed alone: the pass that turns it into dZ only needs dA, so it overlaps the
-      // products issued after the commit (dkc, X), which the next phase's commit covers
-      if (!first) gemm_kk_t<1>(tmem + C_S, aGb, aVu, ID_SQ_KK, false);
-      gemm_mm_t<8>(tmem + C_S, aKP, aT, ID_SQ_MM, !first);
-      mma_commit(&bar_mma);
-      gemm_mm_t<8>(tmem + C_DKC, aVD, aQc, ID_D_MM, !first);
-      gemm_km_t<8>(tmem + C_X, aVD, aKc, ID_D_KM, false);
-      if (!diag) gemm_km_t<8>(tmem + C_X, aKP, aWb, ID_D_KM, true);
-    }
-    MMA_WAIT();
-    BPHASE_MARK(12);
-    {  // dZ = dA * A * (1 - A) -> slot 2 (over Tm)
-      float v[32], a[32];
-      tmem_ld32(trow + C_S + c0, v);
-      load_row32<T>(sA, kPanelB, row, c0, a);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 g = make_float2(a[j], a[j + 1]);
-        const float2 x = mul2(mul2(make_float2(v[j], v[j + 1]), splat(p.scale)), fma2(mul2(g, splat(-1.f)), g, g));   // a (1 - a) = a - a a
-        v[j] = x.x; v[j + 1] = x.y;
-      }
-      store_row32<T>(sT, kPanelB, row, c0, v);
-    }
-    SMEM_TO_MMA_SYNC();
-    BPHASE_MARK(13);
-
-    // ---- M8: G += dSu^T @ Qc[I];  dT = dSu @ A
-    if (tid == 0) {
-      tc_fence_after();
-      // dT first and committed alone: masking it overlaps the G update, which the next phase's first
-      // commit covers (dSu stays in slot 4 until then)
-      gemm_km_t<8>(tmem + C_S, aKP, aA, ID_SQ_KM, false);
-      mma_commit(&bar_mma);
-      gemm_mm_t<8>(tmem + C_G, aKP, aQc, ID_D_MM, !first);
-      mma_commit(&bar_g);
-    }
-    MMA_WAIT();
-    BPHASE_MARK(14);
-    if (tid == 0) {  // Ku[I] comes back for the dqu product, into Wb's slot (its last reader is covered by the commit above)
-      mbar_expect_tx(&bar_ku, OPB);
-      tma_load_4d(sWb, &m_ku, &bar_ku, 0, i0, h, b);
-    }
-    {  // masked dT (rows i, columns j <= i) -> slot 3 (over dS)
-      float v[32];
-      tmem_ld32_lower(trow + C_S + c0, row, c0, v);
-      store_row32<T>(sVD, kPanelB, row, c0, v);
-    }
-    SMEM_TO_MMA_SYNC();
-    BPHASE_MARK(15);
-
-    // ---- M9: dqu += dZ @ Ku[I];  X2 = dT^T @ Qc[I] + A^T @ Gb;  X += dT @ Vu[I];  X3 = dZ^T @ Qu[K]
-    // Three commits.  The first covers every product that reads a per-step input tile, so the next
-    // step's Qc, Vu, Ku are fetched right behind it, ahead of the reduces in the TMA queue (a reduce
-    // takes thousands of cycles to drain and loads issued behind one wait for it).  After each commit the
-    // query-block gradient it completes is staged as fp32 panels in an operand slot that is dead by then
-    // and handed to a TMA reduce (whole lines at L2 instead of scattered atomics): chunk group 1 takes
-    // dqc (into Wb + the spare half of slot 4), group 2 dku (into slot 2, which held dZ), groups 0 and 3 a panel each of dvu
-    // (into Vc|dO, which held dT and is re-loaded last in the next step); group 3 also fetches the next tiles and refreshes the
-    // 16-bit copy of G.  Z of the next step is issued as soon as dvu has been read from its columns and runs under that
-    // staging; Ku is fetched first, behind the G update (2582 -> 2551 us at B=4 N=4096 H=16 bf16; 2589 -> 2485 at B=1 N=16384 H=4).
-    if (tid == 0) {
-      tc_fence_after();
-      gemm_mm_t<8>(tmem + C_X2, aVD, aQc, ID_D_MM, false);
-      gemm_km_t<8>(tmem + C_X, aVD, aVu, ID_D_KM, true);
-      mbar_wait(&bar_ku, ph_ku, abortp);
-      gemm_km_t<8>(tmem + C_DQU, aT, aWb, ID_D_KM, !first);
-      mma_commit(&bar_x1);
-      gemm_mm_t<8>(tmem + C_X3, aT, aQu, ID_D_MM, false);
-      mma_commit(&bar_x2);
-      if (!first) gemm_mm_t<8>(tmem + C_X2, aA, aGb, ID_D_MM, true);
-      mma_commit(&bar_mma);
-    }
-    ph_ku ^= 1;
-    if (cc == 1) {
-      mbar_wait(&bar_x1, ph_x, abortp);
-      tc_fence_after();
-      stage_f32_tile(trow + C_X, sWb, sKP + kPanelB, row);
-      fence_async_smem();
-      group_sync(1);
-      if (quarter == 0 && lane == 0) {
-        tma_reduce_add_3d(&m_acc_dqc, sWb, 0, i0, bh);
-        tma_reduce_add_3d(&m_acc_dqc, sKP + kPanelB, 32, i0, bh);
-        bulk_commit();
-      }
-    } else if (cc == 2) {
-      mbar_wait(&bar_x2, ph_x, abortp);
-      tc_fence_after();
-      stage_f32_tile(trow + C_X3, sT, sT + kPanelB, row);
-      fence_async_smem();
-      group_sync(2);
-      if (quarter == 0 && lane == 0) {
-        tma_reduce_add_3d(&m_acc_dku, sT, 0, i0, bh);
-        tma_reduce_add_3d(&m_acc_dku, sT + kPanelB, 32, i0, bh);
-        bulk_commit();
-      }
-    } else if (cc == 3) {
-      const int in0 = i0 - kBlkB;
-      if (tid == kPrefetchTid && I > K) {   // Ku first: the next Z waits for it, and its slot (dSu) is free as soon as G is done
-        mbar_wait(&bar_g, ph_x, abortp);
+      __syncwarp();
+    } else if (warp == 17) {
+      // ---- the tiles.  The TMA unit works its queue off in order and a reduce takes thousands of cycles, so loads go ahead of them.
+      if (elect_one()) {
+        const int il = (p.nblk - 1) * kBlkB;
+        mbar_expect_tx(&bar_res, 2 * OPB);
+        tma_load_4d(sQu, &m_qu, &bar_res, 0, k0, h, b);
         mbar_expect_tx(&bar_kn, OPB);
-        tma_load_4d(sKP, &m_ku, &bar_kn, 0, in0, h, b);
-      }
-      mbar_wait(&bar_x1, ph_x, abortp);   // Qc[I], Vu[I], Ku[I] are consumed
-      if (tid == kPrefetchTid && I > K) {
+        tma_load_4d(sKP, &m_ku, &bar_kn, 0, il, h, b);
+        tma_load_4d(sKc, &m_kc, &bar_res, 0, k0, h, b);
         mbar_expect_tx(&bar_load, 2 * OPB);
-        tma_load_4d(sQc, &m_qc, &bar_load, 0, in0, h, b);
-        tma_load_4d(sVu, &m_vu, &bar_load, 0, in0, h, b);
+        tma_load_4d(sQc, &m_qc, &bar_load, 0, il, h, b);
+        tma_load_4d(sVu, &m_vu, &bar_load, 0, il, h, b);
+        mbar_arrive(&bar_t);
+        mbar_arrive(&bar_w);
+        mbar_expect_tx(&bar_vd, 2 * OPB);
+        tma_load_4d(sVc, &m_vc, &bar_vd, 0, k0, h, b);
+        tma_load_4d(sdO, &m_do, &bar_vd, 0, il, h, b);
       }
+#pragma unroll 1
+      for (int n = 0; n < walk; ++n) {
+        const uint32_t ph = n & 1;
+        const bool more = n + 1 < walk;
+        const int i0 = (p.nblk - 1 - n) * kBlkB, in0 = i0 - kBlkB;
+        __syncwarp();
+        if (elect_one()) {
+          mbar_wait(&bar_g, ph, abortp);         // copy of W and dSu have been read
+          mbar_expect_tx(&bar_ku, OPB);
+          tma_load_4d(sWb, &m_ku, &bar_ku, 0, i0, h, b);
+          if (more) {
+            mbar_expect_tx(&bar_kn, OPB);
+            tma_load_4d(sKP, &m_ku, &bar_kn, 0, in0, h, b);
+          }
+          mbar_wait(&bar_x, ph, abortp);         // Qc[I], Vu[I], Ku[I] as well
+          if (more) {
+            mbar_expect_tx(&bar_load, 2 * OPB);
+            tma_load_4d(sQc, &m_qc, &bar_load, 0, in0, h, b);
+            tma_load_4d(sVu, &m_vu, &bar_load, 0, in0, h, b);
+          }
+        }
+        __syncwarp();
+        ev_wait(kEvDku, 128);                    // its slot is needed first
+        if (elect_one()) {
+          tma_reduce_add_3d(&m_acc_dku, sT, 0, i0, bh);
+          tma_reduce_add_3d(&m_acc_dku, sT + kPanelB, 32, i0, bh);
+          bulk_commit();
+        }
+        __syncwarp();
+        ev_wait(kEvDqc, 128);
+        if (elect_one()) {
+          tma_reduce_add_3d(&m_acc_dqc, sWb, 0, i0, bh);
+          tma_reduce_add_3d(&m_acc_dqc, sKP + kPanelB, 32, i0, bh);
+          bulk_commit();
+        }
+        __syncwarp();
+        ev_wait(kEvDvu, 256);
+        if (elect_one()) {
+          tma_reduce_add_3d(&m_acc_dvu, sVD, 0, i0, bh);
+          tma_reduce_add_3d(&m_acc_dvu, sVD + kPanelB, 32, i0, bh);
+          bulk_commit();
+          bulk_wait_read2();
+          if (more) mbar_arrive(&bar_t);         // T may go over the staging of dku
+          bulk_wait_read1();
+          if (more) mbar_arrive(&bar_w);         // and the copy of W and P over that of dqc
+          bulk_wait_read0();
+          if (more) {
+            mbar_expect_tx(&bar_vd, 2 * OPB);
+            tma_load_4d(sVc, &m_vc, &bar_vd, 0, k0, h, b);
+            tma_load_4d(sdO, &m_do, &bar_vd, 0, in0, h, b);
+          }
+        }
+      }
+      __syncwarp();
+      if (elect_one()) bulk_wait0();
+      __syncwarp();
     }
-    ph_x ^= 1;
-    ph_load ^= 1;
-    BPHASE_MARK(16);
-    MMA_WAIT();
-    BPHASE_MARK(17);
-    // The products' last columns are read, then the next step's Z is issued over them and runs while dvu is staged and G copied.
-    float v[32];
-    if (cc == 0 || cc == 3) {   // a panel of dvu each
-      tmem_ld32(trow + C_X2 + (cc == 3 ? 32 : 0), v);
-      tmem_ld_wait();
-    }
-    tc_fence_before();
-    __syncthreads();
-    BPHASE_MARK(18);
-    if (tid == 0 && I > K) issue_z(ph_load);
-    if (cc == 0 || cc == 3) {
-      uint8_t* panel = cc == 3 ? sVD + kPanelB : sVD;
-      store_row32_f32(panel, row, v);
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kBwdWorkerRegs));
+    const int quarter = warp & 3, cc = warp >> 2;
+    const int row = quarter * 32 + lane;
+    const int c0 = cc * 32;
+    const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
+    const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
+    auto wait = [&](uint64_t* bar, uint32_t ph) {
+      mbar_wait(bar, ph, abortp);
+      tc_fence_after();
+    };
+    // This thread's part of the scratch columns is in registers.  Returns 0, read from shared memory behind the arrival: the compiler
+    // moves an arrival behind arithmetic that does not depend on it, and the next product then starts a pass late, so a constant
+    // of the pass has this added to it (2044 -> 1964 us at B=4 N=4096 H=16).
+    auto read = [&]() {
+      tc_fence_before();
+      ev_arrive(kEvRead, kBwdWorkers);
+      float zero;
+      asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(zero) : "r"(smem_u32(&zero_s)) : "memory");
+      return zero;
+    };
+    auto stored = [&](int id) {
       fence_async_smem();
-      group_sync(3 + cc);
-      if (quarter == 0 && lane == 0) {
-        tma_reduce_add_3d(&m_acc_dvu, panel, cc == 3 ? 32 : 0, i0, bh);
-        bulk_commit();
-      }
+      tc_fence_before();
+      ev_arrive(id, kBwdWorkers);
+    };
+    // W_K starts as the forward's final state, brought in whole lines (rows of 64 floats over the threads, through the gate's slot):
+    // a row per lane, here and where the gradients are stored, took 2 us of a key block each; 1036 pairs of one block 150.5 ->
+    // 142.3 us, B=16 H=8 N=1024 402 -> 392 us
+#pragma unroll
+    for (int i = 0; i < kBlkB * (D / 4) / kBwdWorkers; ++i) {
+      const int e = i * kBwdWorkers + tid, r = e / (D / 4), c = e % (D / 4);
+      const float4 q = (k0 + r < p.N) ? *reinterpret_cast<const float4*>(p.w_state + ((int64_t)bh * p.N + k0 + r) * D + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(sA + (c >> 3) * kPanelB + swz_off(r, c & 7)) = q;
     }
-    if (cc == 3 && !diag) {  // 16-bit copy of G including block I, for the next (lower) block; ordered by the next step's barriers
+    asm volatile("bar.sync %0, %1;" ::"n"(kWorkers), "n"(kBwdWorkers) : "memory");
+    if (c0 < D) {
+      float v[32];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 q = *reinterpret_cast<const float4*>(sA + cc * kPanelB + swz_off(row, j));
+        v[4 * j] = q.x; v[4 * j + 1] = q.y; v[4 * j + 2] = q.z; v[4 * j + 3] = q.w;
+      }
+      tmem_st32(trow + C_W + c0, v);
+      tmem_st_wait();
+    }
+    asm volatile("bar.sync %0, %1;" ::"n"(kWorkers), "n"(kBwdWorkers) : "memory");
+
+#pragma unroll 1
+    for (int n = 0; n < walk; ++n) {
+      const uint32_t ph = n & 1;
+      const int I = p.nblk - 1 - n, irow = I * kBlkB + row;
+      const bool diag = I == K, rvalid = irow < p.N;
+      BPHASE_MARK(0);
+      wait(&bar_z, ph);
+      BPHASE_MARK(1);
+      {  // gate A (rows k, columns j), zero unless j > k
+        float v[32];
+        tmem_ld32(trow + C_S + c0, v);
+        tmem_ld_wait();
+        const float hs = half_scale + read();
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), hs);
+          v[j] = a.x; v[j + 1] = a.y;
+        }
+        if (diag) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
+        }
+        store_row32<T>(sA, kPanelB, row, c0, v);
+      }
+      stored(kEvStored);
+      BPHASE_MARK(2);
+      wait(&bar_t, ph);
+      BPHASE_MARK(3);
+      {  // masked T (rows i, columns j <= i), unscaled
+        float v[32];
+        tmem_ld32_lower(trow + C_S + c0, row, c0, v);
+        store_row32<T>(sT, kPanelB, row, c0, v);
+      }
+      stored(kEvStoredT);
+      wait(&bar_w, ph);
+      BPHASE_MARK(4);
+      if (c0 < D) {  // 16-bit copy of the peeled state
+        float v[32];
+        tmem_ld32(trow + C_W + c0, v);
+        tmem_ld_wait();
+        store_row32<T>(sWb, kPanelB, row, c0, v);
+      }
+      stored(kEvStored);
+      BPHASE_MARK(5);
+      // loaded here, not at the top of the step, where the wait for Z is short
+      const float lse_i = rvalid ? p.lse[(int64_t)bh * p.N + irow] : 0.f, delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
+      wait(&bar_su, ph);
+      BPHASE_MARK(6);
+      uint32_t dpk[16];  // silu'(Su), two 16-bit values per register
+      uint32_t ppk[16];  // P
+      {
+        float v[32], w[32];
+        tmem_ld32(trow + C_S + c0, v);
+        tmem_ld_wait();
+        const float hs = half_scale + read();
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 u = make_float2(v[j], v[j + 1]);
+          const float2 g = sigmoid2(u, hs);
+          // silu'(su) = g + silu(su) (1 - g)
+          const float2 q = mul2(mul2(u, g), splat(-1.f));   // -silu(su) / scale
+          v[j] = q.x; v[j + 1] = q.y;
+          const float2 d = fma2(mul2(q, splat(-p.scale)), fma2(g, splat(-1.f), splat(1.f)), g);
+          dpk[j / 2] = Elem<T>::pack2(d.x, d.y);
+        }
+        BPHASE_MARK(7);
+        wait(&bar_sc, ph);
+        BPHASE_MARK(8);
+        // P = exp(S - lse) (rows i, columns k); into slot 4 over Ku
+        tmem_ld32(trow + C_S + c0, w);
+        tmem_ld_wait();
+        const float s2 = sl2 + read();
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(s2), splat(-lse_i * kLog2e));
+          const float2 e = j % 16 == 0 ? exp2_fma2(x) : make_float2(ex2_approx(x.x), ex2_approx(x.y));   // an eighth off the busiest unit
+          v[j] = e.x; v[j + 1] = e.y;
+        }
+        if (diag) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+        }
+        if (!rvalid) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) ppk[j / 2] = Elem<T>::pack2(v[j], v[j + 1]);
+        store_row32<T>(sKP, kPanelB, row, c0, v);
+      }
+      stored(kEvStored);
+      BPHASE_MARK(9);
+      wait(&bar_dp, ph);
+      BPHASE_MARK(10);
+      {  // dS = P * (dP - delta) -> slot 3 (over Vc|dO); dSu = -dS * silu'(Su) -> slot 4 (over P)
+        float v[32], w[32];
+        tmem_ld32(trow + C_S + c0, v);
+        tmem_ld_wait();
+        const float dl = delta_i + read();
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 ds = mul2(Elem<T>::unpack2(ppk[j / 2]), add2(make_float2(v[j], v[j + 1]), splat(-dl)));
+          const float2 du = mul2(ds, Elem<T>::unpack2(dpk[j / 2]));
+          v[j] = ds.x; v[j + 1] = ds.y;
+          w[j] = -du.x; w[j + 1] = -du.y;
+        }
+        mbar_wait(&bar_dv, ph, abortp);   // dO and P have been read
+        store_row32<T>(sVD, kPanelB, row, c0, v);
+        store_row32<T>(sKP, kPanelB, row, c0, w);
+      }
+      stored(kEvStored);
+      BPHASE_MARK(11);
+      wait(&bar_da, ph);
+      BPHASE_MARK(12);
+      {  // dZ = dA * A * (1 - A) -> slot 2 (over T)
+        float v[32], a[32];
+        tmem_ld32(trow + C_S + c0, v);
+        tmem_ld_wait();
+        const float sc = p.scale + read();
+        load_row32<T>(sA, kPanelB, row, c0, a);
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 g = make_float2(a[j], a[j + 1]);
+          const float2 x = mul2(mul2(make_float2(v[j], v[j + 1]), splat(sc)), fma2(mul2(g, splat(-1.f)), g, g));   // a (1 - a) = a - a a
+          v[j] = x.x; v[j + 1] = x.y;
+        }
+        store_row32<T>(sT, kPanelB, row, c0, v);
+      }
+      stored(kEvStoredZ);   // an event of its own: the wait below does not cover it
+      BPHASE_MARK(13);
+      wait(&bar_dt, ph);
+      BPHASE_MARK(14);
+      {  // masked dT (rows i, columns j <= i) -> slot 3 (over dS)
+        float v[32];
+        tmem_ld32_lower(trow + C_S + c0, row, c0, v);
+        read();
+        store_row32<T>(sVD, kPanelB, row, c0, v);
+      }
+      stored(kEvStored);
+      BPHASE_MARK(15);
+      // The query block's gradients are staged as fp32 panels in operand slots that are dead by then and handed to TMA reduces
+      // (whole lines at L2 instead of scattered atomics): chunk group 1 takes dqc (into the copy of W's slot and the spare half of
+      // slot 4), group 2 dku (into slot 2), groups 0 and 3 a panel each of dvu (into slot 3).  Groups 1 and 2 also make the
+      // 16-bit copy of G, including block I, for the next (lower) block; the next step's events order it.
+      const int part = cc >> 1;
+      if (cc == 1 || cc == 2) {
+        wait(&bar_x, ph);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          float v[32];
+          tmem_ld32(trow + (cc == 1 ? C_X : C_X3) + c * 32, v);
+          tmem_ld_wait();
+          if (c == 1) read();
+          store_row32_f32(cc == 2 ? sT + c * kPanelB : c == 0 ? sWb : sKP + kPanelB, row, v);
+        }
+        fence_async_smem();
+        ev_arrive(cc == 1 ? kEvDqc : kEvDku, 128);
+        wait(&bar_l, ph);
+        if (!diag) {
+          float v[32];
+          tmem_ld32(trow + C_G + part * 32, v);
+          tmem_ld_wait();
+          store_row32<T>(sGb, kPanelB, row, part * 32, v);
+        }
+      } else {
+        wait(&bar_l, ph);
+        BPHASE_MARK(16);
+        float v[32];
+        tmem_ld32(trow + C_X2 + part * 32, v);
+        tmem_ld_wait();
+        read();
+        store_row32_f32(sVD + part * kPanelB, row, v);
+        fence_async_smem();
+        ev_arrive(kEvDvu, 256);
+      }
+      BPHASE_MARK(17);
+    }
+
+    // ---- key-block gradients: dkc (x scale), dvc, dqu (x scale); one chunk group each, through the gate's slot and the copy of
+    // G, so that eight lanes store a row in whole lines
+    if (cc < 3) {
+      const uint32_t col = (cc == 0) ? C_DKC : (cc == 1 ? C_DVC : C_DQU);
+      const castle_tensor_t& dt = (cc == 0) ? p.dkc : (cc == 1 ? p.dvc : p.dqu);
+      const float mul = (cc == 1) ? 1.f : p.scale;
+      uint8_t* panel = cc == 0 ? sA : (cc == 1 ? sA + kPanelB : sGb);
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
-        tmem_ld32(trow + C_G + c * 32, v);
+        float v[32];
+        tmem_ld32(trow + col + c * 32, v);
         tmem_ld_wait();
-        store_row32<T>(sGb, kPanelB, row, c * 32, v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] *= mul;
+        store_row32<T>(panel, kPanelB, row, c * 32, v);
+      }
+      group_sync(kEpilogue + cc);
+      T* dst = reinterpret_cast<T*>(dt.ptr) + b * dt.stride_b + h * dt.stride_h + (lane & 7) * 8;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = (quarter * 8 + j) * 4 + (lane >> 3);
+        if (k0 + r < p.N)
+          *reinterpret_cast<uint4*>(dst + (int64_t)(k0 + r) * dt.stride_n) = *reinterpret_cast<const uint4*>(panel + swz_off(r, lane & 7));
       }
     }
-    BPHASE_MARK(19);
-    BPHASE_MARK(20);
   }
-#undef MMA_WAIT
-#undef SMEM_TO_MMA_SYNC
-
-  // ---- key-block gradients: dkc (x scale), dvc, dqu (x scale); one chunk group each, through the gate's slot and the copy of
-  // G, so that eight lanes store a row in whole lines
-  if (cc < 3) {
-    tc_fence_after();
-    const uint32_t col = (cc == 0) ? C_DKC : (cc == 1 ? C_DVC : C_DQU);
-    const castle_tensor_t& dt = (cc == 0) ? p.dkc : (cc == 1 ? p.dvc : p.dqu);
-    const float mul = (cc == 1) ? 1.f : p.scale;
-    uint8_t* panel = cc == 0 ? sA : (cc == 1 ? sA + kPanelB : sGb);
-#pragma unroll 1
-    for (int c = 0; c < D / 32; ++c) {
-      float v[32];
-      tmem_ld32(trow + col + c * 32, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] *= mul;
-      store_row32<T>(panel, kPanelB, row, c * 32, v);
-    }
-    group_sync(7 + cc);
-    T* dst = reinterpret_cast<T*>(dt.ptr) + b * dt.stride_b + h * dt.stride_h + (lane & 7) * 8;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int r = (quarter * 8 + j) * 4 + (lane >> 3);
-      if (k0 + r < p.N)
-        *reinterpret_cast<uint4*>(dst + (int64_t)(k0 + r) * dt.stride_n) = *reinterpret_cast<const uint4*>(panel + swz_off(r, lane & 7));
-    }
-  }
-  if (quarter == 0 && lane == 0) bulk_wait0();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);
@@ -534,6 +562,11 @@ static int launch_bwd(const BwdParams& p, const CUtensorMap* maps, cudaStream_t 
     cudaError_t e = cudaFuncSetAttribute(castle_bwd_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
   }
+  static const int launch_regs = [] {   // what the kernel was compiled to start with
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, castle_bwd_kernel<T, D>) == cudaSuccess ? a.numRegs : -1;
+  }();
+  if (launch_regs != kBwdLaunchRegs) return reject("castle_bwd: compiled with %d registers a thread instead of %d", launch_regs, kBwdLaunchRegs);
   const int64_t rows = (int64_t)p.B * p.H * p.N;
   constexpr int RPB = 256 / (D / 8);
   castle_bwd_delta_kernel<T, D, 3><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
