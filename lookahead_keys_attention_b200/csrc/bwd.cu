@@ -30,12 +30,6 @@
 
 namespace castle {
 
-constexpr int kBwdWorkers = 512;               // warps 0-15: the passes
-constexpr int kBwdThreads = kBwdWorkers + 128; // warp 16 issues the products, warp 17 moves tiles; two more fill up the warpgroup
-// Registers a thread: the launch's 640 x 96 are shared out anew, 512 x 112 + 128 x 32 = 61440.
-constexpr int kBwdLaunchRegs = 96, kBwdWorkerRegs = 112, kBwdHelperRegs = 32;
-static_assert(kBwdWorkers * kBwdWorkerRegs + 128 * kBwdHelperRegs <= kBwdThreads * kBwdLaunchRegs, "setmaxnreg would wait forever");
-
 // Optional phase timing (debug builds only): thread 0 of CTA (0,0) stores clock64() at each phase
 // boundary of its first steps behind the fp32 workspace, which the host dumps.
 #ifdef CASTLE_PHASE_TIMING
@@ -49,14 +43,12 @@ static_assert(kBwdWorkers * kBwdWorkerRegs + 128 * kBwdHelperRegs <= kBwdThreads
 #define tma_reduce_add_3d(...) do { } while (0)
 #endif
 
-// Named barriers on which the passes' warps arrive and go on, and one helper warp waits.
+// named barriers (ev_arrive)
 enum BwdEvent { kEvRead = 1, kEvStored = 2, kEvStoredT = 3, kEvStoredZ = 4, kEvDqc = 5, kEvDku = 6, kEvDvu = 7 };
 constexpr int kWorkers = 8, kEpilogue = 9;   // and those of the passes among themselves: all 512, and 9 to 11 a chunk group each
-__device__ __forceinline__ void ev_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads + 32) : "memory"); }
-__device__ __forceinline__ void ev_wait(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads + 32) : "memory"); }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(kBwdThreads, 1)
+__global__ void __launch_bounds__(kSplitThreads, 1)
 castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
                   const __grid_constant__ CUtensorMap m_vc, const __grid_constant__ CUtensorMap m_qu,
                   const __grid_constant__ CUtensorMap m_ku, const __grid_constant__ CUtensorMap m_vu,
@@ -120,8 +112,8 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   const uint32_t tmem = tmem_base_s;
   volatile int* abortp = &abort_flag;
 
-  if (warp >= kBwdWorkers / 32) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kBwdHelperRegs));
+  if (warp >= kSplitWorkers / 32) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSplitHelperRegs));
     if (warp == 16) {
       // ---- the products, in the order that the passes need them; what a pass does not wait for goes behind its commit
       // operand addresses are made where they are used: kept in registers over the step they would be spilled
@@ -132,7 +124,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       };
       auto next = [&](int id) {
         __syncwarp();
-        ev_wait(id, kBwdWorkers);
+        ev_wait(id, kSplitWorkers);
         tc_fence_after();
       };
       auto issue_z = [&](uint32_t ph) {
@@ -298,7 +290,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       __syncwarp();
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kBwdWorkerRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSplitWorkerRegs));
     const int quarter = warp & 3, cc = warp >> 2;
     const int row = quarter * 32 + lane;
     const int c0 = cc * 32;
@@ -308,31 +300,22 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       mbar_wait(bar, ph, abortp);
       tc_fence_after();
     };
-    // This thread's part of the scratch columns is in registers.  Returns 0, read from shared memory behind the arrival: the compiler
-    // moves an arrival behind arithmetic that does not depend on it, and the next product then starts a pass late, so a constant
-    // of the pass has this added to it (2044 -> 1964 us at B=4 N=4096 H=16).
-    auto read = [&]() {
-      tc_fence_before();
-      ev_arrive(kEvRead, kBwdWorkers);
-      float zero;
-      asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(zero) : "r"(smem_u32(&zero_s)) : "memory");
-      return zero;
-    };
+    auto read = [&]() { return ev_arrive_read(kEvRead, kSplitWorkers, &zero_s); };
     auto stored = [&](int id) {
       fence_async_smem();
       tc_fence_before();
-      ev_arrive(id, kBwdWorkers);
+      ev_arrive(id, kSplitWorkers);
     };
     // W_K starts as the forward's final state, brought in whole lines (rows of 64 floats over the threads, through the gate's slot):
     // a row per lane, here and where the gradients are stored, took 2 us of a key block each; 1036 pairs of one block 150.5 ->
     // 142.3 us, B=16 H=8 N=1024 402 -> 392 us
 #pragma unroll
-    for (int i = 0; i < kBlkB * (D / 4) / kBwdWorkers; ++i) {
-      const int e = i * kBwdWorkers + tid, r = e / (D / 4), c = e % (D / 4);
+    for (int i = 0; i < kBlkB * (D / 4) / kSplitWorkers; ++i) {
+      const int e = i * kSplitWorkers + tid, r = e / (D / 4), c = e % (D / 4);
       const float4 q = (k0 + r < p.N) ? *reinterpret_cast<const float4*>(p.w_state + ((int64_t)bh * p.N + k0 + r) * D + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
       *reinterpret_cast<float4*>(sA + (c >> 3) * kPanelB + swz_off(r, c & 7)) = q;
     }
-    asm volatile("bar.sync %0, %1;" ::"n"(kWorkers), "n"(kBwdWorkers) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"n"(kWorkers), "n"(kSplitWorkers) : "memory");
     if (c0 < D) {
       float v[32];
 #pragma unroll
@@ -343,7 +326,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       tmem_st32(trow + C_W + c0, v);
       tmem_st_wait();
     }
-    asm volatile("bar.sync %0, %1;" ::"n"(kWorkers), "n"(kBwdWorkers) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"n"(kWorkers), "n"(kSplitWorkers) : "memory");
 
 #pragma unroll 1
     for (int n = 0; n < walk; ++n) {
@@ -562,17 +545,14 @@ static int launch_bwd(const BwdParams& p, const CUtensorMap* maps, cudaStream_t 
     cudaError_t e = cudaFuncSetAttribute(castle_bwd_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
   }
-  static const int launch_regs = [] {   // what the kernel was compiled to start with
-    cudaFuncAttributes a;
-    return cudaFuncGetAttributes(&a, castle_bwd_kernel<T, D>) == cudaSuccess ? a.numRegs : -1;
-  }();
-  if (launch_regs != kBwdLaunchRegs) return reject("castle_bwd: compiled with %d registers a thread instead of %d", launch_regs, kBwdLaunchRegs);
+  static const int regs_rc = check_launch_regs(castle_bwd_kernel<T, D>, "castle_bwd");
+  if (regs_rc) return regs_rc;
   const int64_t rows = (int64_t)p.B * p.H * p.N;
   constexpr int RPB = 256 / (D / 8);
   castle_bwd_delta_kernel<T, D, 3><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);
   dim3 grid(p.B * p.H, p.nblk);
   ev_start(CASTLE_KERNEL_BWD, st);
-  cudaError_t e = launch_kernel(castle_bwd_kernel<T, D>, grid, kBwdThreads, smem, st, true, p, maps[0], maps[1], maps[2], maps[3], maps[4],
+  cudaError_t e = launch_kernel(castle_bwd_kernel<T, D>, grid, kSplitThreads, smem, st, true, p, maps[0], maps[1], maps[2], maps[3], maps[4],
                                 maps[5], maps[6], maps[7], maps[8], maps[9]);
   ev_stop(CASTLE_KERNEL_BWD, st);
   if (e == cudaSuccess) e = launch_kernel(castle_bwd_finish_kernel<T, D, 3>, dim3((unsigned)((rows + RPB - 1) / RPB)), 256, 0, st, true, p);

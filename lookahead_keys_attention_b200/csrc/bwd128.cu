@@ -10,10 +10,9 @@
 // Every gradient but dqc is owned by a CTA that keeps it in tensor memory.  A TMA reduce moves some 18 bytes per cycle and SM,
 // so a lookahead kernel that owned a key block and reduced dku[I] and dvu[I] (128 KB a step, with dT masked and multiplied in
 // every step) took 18.5 k cycles a step, 12.1 k without the reduces; reverse + la + dqu take 3.1 + 7.3 + 1.9 k, and kv, which
-// no longer forms dT, went from 20.8 to 16.2 k.  Measured on B=1 H=8 N=8190 bf16: 2365 -> 1708 us for the kernels, B=2 H=8 N=1333:
-// 249 -> 182 us.  What bounds them: kv its chain of six products with a pass behind each; la and reverse the tiles, which
-// come at 20 to 30 bytes per cycle and SM with one step's worth of shared memory to prefetch into; dqu HBM.  (Handing W on
-// as well, from a kernel of its own, so that kv starts at Su: 4.4 + 17 k cycles.)
+// no longer forms dT, 4.6 k less.  Measured on B=1 H=8 N=8190 bf16: 2365 -> 1708 us for the kernels, B=2 H=8 N=1333:
+// 249 -> 182 us.  What bounds them: kv its chain of products and passes and shared memory; la and reverse the tiles, which
+// come at 20 to 30 bytes per cycle and SM with one step's worth of shared memory to prefetch into; dqu HBM.  
 //
 // Tiles of a step (I,K): A, then dZ | dSu | Gb; 32 KB each, as they lie in shared memory (128-byte swizzle).  The scratch is
 // bounded (kTileScratchLimit): the (batch, head) pairs run in chunks, one launch of each kernel per chunk.
@@ -53,8 +52,9 @@ __device__ __forceinline__ void load_op(uint8_t* dst, const CUtensorMap& m, uint
 __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K) {   // of this CTA's pair
   return p.tiles + ((int64_t)blockIdx.x * p.ntiles + (int64_t)I * (I + 1) / 2 + K) * kStepTiles;
 }
-// What every kernel starts with: shared memory behind the operands, barriers, tensor memory.  NBAR barriers (of one arrival).
-#define B128_BEGIN(OPERANDS, NBAR, COLS)                                                      \
+// What every kernel starts with: shared memory behind the operands, barriers, tensor memory.  NBAR barriers of one arrival, but
+// two at barrier PAIR (-1: none).
+#define B128_BEGIN(OPERANDS, NBAR, PAIR, COLS)                                                      \
   extern __shared__ __align__(1024) uint8_t smem[];                                            \
   uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + (OPERANDS));                       \
   uint32_t* const tmem_base_s = reinterpret_cast<uint32_t*>(bars + (NBAR));                    \
@@ -63,7 +63,7 @@ __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K)
   const int bh = p.bh0 + blockIdx.x, b = bh / p.H, h = bh % p.H;                               \
   if (tid == 0) {                                                                              \
     if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);                  \
-    for (int i = 0; i < (NBAR); ++i) mbar_init(bars + i, 1);                                   \
+    for (int i = 0; i < (NBAR); ++i) mbar_init(bars + i, i == (PAIR) ? 2 : 1);                 \
     mbar_fence_init();                                                                         \
     *abortp = 0;                                                                               \
   }                                                                                            \
@@ -95,16 +95,20 @@ __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K)
   __syncthreads();
 
 // ------------------------------------------------------------------------------------------------ scores, dkc, dvc, dqc
-// One chain per step, six products with a pass behind each:
-//   Z | gate A;  T, W -= A Vu | T masked, Wb;  Su | silu';  Sc (while silu' is formed) | P;  dP, dvc | dS, dSu;  dqc, dkc | staging
+// One chain per step, products and passes in turn:
+//   Z | gate A (T under it);  W -= A Vu | T masked, Wb (T A^T under it);  Su | silu' (Sc under it) | P (dP under it);  dvc | dS, dSu;
+//   dqc, dkc | staging (the next Z under it)
+// Sixteen warps do the passes, one issues the products, one moves the tiles (ev_arrive).  While warp 0 issued the products and also
+// worked in the passes, it waited as long as the tensor unit's queue was full and the others waited for it: step 15.2 k -> 12.9 k
+// cycles, the kernel at B=1 H=8 N=8190 995 -> 884 us, B=2 H=8 N=1333 104 -> 95, B=8 H=16 N=512 141 -> 133.  What bounds it now: 10.7 k
+// cycles of a step's 1.4 MB through shared memory, and the wait for Qc and Vu, whose slots the last product of a step frees.
 // Tensor memory: W | dkc | dvc | scratch.  Shared memory, seven tiles:
 //   s0 Qu, then Wb | s1 Ku, A, dS | s2 Vu, T, P | s3 Qc | s4 Kc | s5 Vc, staging | s6 dO, dSu, staging
 // with the roles of s1 and s2 exchanged in every other step: P dies first, so that the next Ku lands over it and the next Z runs
 // while dqc is staged.
 // TMA works its queue off in order, and a reduce moves some 18 bytes a cycle: a load queued behind the 64 KB of dqc waits
 // 3.6 k cycles.  So the loads that the next step starts with (Qu, Ku, Vu, Qc) are issued before the reduces, and what is
-// staged over are the tiles that it needs last: dO, and Vc, which is loaded again for that (step 21.7 k cycles with the
-// loads behind the reduces, 18.9 k so, 17.1 k with the next Z under the staging and 16.2 k with the copy of dSu behind the next Qu).
+// staged over are the tiles that it needs last: dO, and Vc, which is loaded again for that.
 // Few pairs: the grid is little more than a wave, whose length is the walk of key block 0, while the mean walk is about half as
 // long.  So long walks are cut in two parts of about equal cost, a CTA each (kv_split).  The second part first peels the state down
 // to where it begins, in steps of Z, gate and W alone, some 0.3 of a step each: with a cut after x of n steps both cost x = n / 1.7.
@@ -115,8 +119,12 @@ __device__ __forceinline__ uint8_t* kv_part(const BwdParams& p, int bh, int K, i
   return reinterpret_cast<uint8_t*>(p.acc_dvu) + ((int64_t)(bh * p.kv_split + K) * 2 + part) * kPart;
 }
 
+enum KvBar { kKvRes, kKvZin /* Qu, Ku */, kKvIn /* Qc, Vu */, kKvDo /* Vc, dO */, kKvZ, kKvT, kKvW, kKvSu, kKvSc, kKvDp, kKvDv, kKvX0, kKvX, kKvK,
+             kKvCopied /* dSu */, kKvBars };
+enum KvEvent { kKvRead = 1, kKvStored = 2, kKvStoredT = 3, kKvStaged = 4, kKvGroups = 5 };
+
 template <typename T, bool CUT>
-__global__ void __launch_bounds__(kB128Threads, 1)
+__global__ void __launch_bounds__(kSplitThreads, 1)
 castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, const __grid_constant__ CUtensorMap m_kc,
                         const __grid_constant__ CUtensorMap m_vc, const __grid_constant__ CUtensorMap m_qu,
                         const __grid_constant__ CUtensorMap m_ku, const __grid_constant__ CUtensorMap m_vu,
@@ -131,320 +139,340 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
   const bool cut = CUT && K < p.kv_split;
   if (part && !cut) return;
   const int begin = part ? kv_cut(walk) : 0, end = cut && !part ? kv_cut(walk) : walk;   // steps with scores; state alone before them
-  B128_BEGIN(7 * kSq, 11, 512)
-  uint8_t *s0 = smem, *s1 = s0 + kSq, *s2 = s1 + kSq, *s3 = s2 + kSq, *s4 = s3 + kSq, *s5 = s4 + kSq, *s6 = s5 + kSq;
-  const uint32_t a0 = smem_u32(s0), a1 = smem_u32(s1), a2 = smem_u32(s2), a3 = smem_u32(s3), a4 = smem_u32(s4), a5 = smem_u32(s5),
-                 a6 = smem_u32(s6);
-  uint64_t *bar_res = bars, *bar_z = bars + 1 /* Qu, Ku */, *bar_in = bars + 2 /* Qc, Vu */, *bar_do = bars + 3,
-           *bar_mma = bars + 4 /* Z, Su, Sc, dP: one after another */, *bar_t = bars + 5, *bar_w = bars + 6, *bar_dv = bars + 7,
-           *bar_x0 = bars + 8, *bar_x = bars + 9, *bar_k = bars + 10;
-  const int row = (warp & 3) * 32 + lane, cc = warp >> 2, c0 = cc * 32, krow = k0 + row;
-  // Lanes with a duty besides the products (warp 0's): the panel of dqc that chunk group cc stages and that panel's
-  // refill with Vc or dO; the copies of A and dSu; the other loads.
-  const bool reducer = (warp & 3) == 1, storer = warp == 8, loader = warp == 10;
-  auto load_panel = [&](int i0) {
-    if (cc < 2) tma_load_4d(s5 + cc * kPanelB, &m_vc, bar_do, cc * 64, k0, h, b);
-    else tma_load_4d(s5 + cc * kPanelB, &m_do, bar_do, (cc - 2) * 64, i0, h, b);
-  };
-  if (loader && elect_one()) {
-    const int il = (p.nblk - 1) * kBlkB;
-    mbar_expect_tx(bar_z, 2 * kSq);
-    load_op(s0, m_qu, bar_z, k0, h, b);
-    load_op(s1, m_ku, bar_z, il, h, b);
-    mbar_expect_tx(bar_in, begin == 0 ? 2 * kSq : kSq);
-    if (begin == 0) load_op(s3, m_qc, bar_in, il, h, b);
-    load_op(s2, m_vu, bar_in, il, h, b);
-    mbar_expect_tx(bar_do, 2 * kSq);
-    mbar_expect_tx(bar_res, kSq);
-    load_op(s4, m_kc, bar_res, k0, h, b);
-  }
-  if (reducer && elect_one()) load_panel((p.nblk - 1 - begin) * kBlkB);
-  __syncwarp();
-  {  // W starts as the forward's final state
-    const float* src = p.w_state + ((int64_t)bh * p.N + krow) * 128 + c0;
-    float v[32];
-#pragma unroll
-    for (int j = 0; j < 32; j += 4) {
-      const float4 q = (krow < p.N) ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w;
-    }
-    tmem_st32(trow + C_W + c0, v);
-    tmem_st_wait();
-  }
-  tc_fence_before();
+  B128_BEGIN(7 * kSq, kKvBars, kKvDp, 512)
+  // the slot of Ku, A, dS and that of Vu, T, P change places from step to step
+  auto slot_k = [](int n) { return (n & 1 ? 2u : 1u) * kSq; };
+  auto slot_v = [](int n) { return (n & 1 ? 1u : 2u) * kSq; };
+  constexpr uint32_t S0 = 0, S3 = 3 * kSq, S4 = 4 * kSq, S5 = 5 * kSq, S6 = 6 * kSq;
+  float* const zero_s = reinterpret_cast<float*>(bars + kKvBars + 1);
+  if (tid == 0) *zero_s = 0.f;
   __syncthreads();
 
-  // Z = Qu Ku^T of the first step; a later one's is issued in the step before
-  if (warp == 0 && elect_one()) {
-    mbar_wait(bar_z, 0, abortp);
-    tc_fence_after();
-    gemm_kk_t<2>(tmem + C_S, a0, a1, ID_KK, false);
-    mma_commit(bar_mma);
-  }
-  __syncwarp();
-  uint32_t ph_mma = 0;
-  const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
-  for (int n = 0; n < end; ++n) {
-    const int m = n - begin;                    // of the steps with scores
-    const uint32_t ph = n & 1, ph_m = m & 1;    // barriers that complete in every step; in steps with scores
-    const int I = p.nblk - 1 - n, i0 = I * kBlkB, irow = i0 + row;
-    const bool diag = I == K, rvalid = irow < p.N, more = n + 1 < end;
-    uint8_t* const tile = step_tiles(p, I, K);
-    uint8_t *const sK = n & 1 ? s2 : s1, *const sV = n & 1 ? s1 : s2;
-    const uint32_t aK = n & 1 ? a2 : a1, aV = n & 1 ? a1 : a2;
-    B128_MARK(0, n, 0);
-    B128_MARK(0, n, 1);
-    mbar_wait(bar_mma, ph_mma, abortp);
-    ph_mma ^= 1;
-    tc_fence_after();
-    B128_MARK(0, n, 2);
-    {
+  if (warp >= kSplitWorkers / 32) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSplitHelperRegs));
+    if (warp == kSplitWorkers / 32) {
+      // ---- the products, in the order that the passes need them
+      auto at = [&](uint32_t off) {   // made where it is used: kept in registers over the step the addresses would be spilled
+        uint32_t base = smem_u32(smem);
+        asm volatile("" : "+r"(base));
+        return base + off;
+      };
+      auto next = [&](int id) {
+        __syncwarp();
+        ev_wait(id, kSplitWorkers);
+        tc_fence_after();
+      };
+      auto issue_z = [&](int n) {     // Z = Qu[K] Ku[I]^T
+        mbar_wait(bars + kKvZin, n & 1, abortp);
+        tc_fence_after();
+        gemm_kk_t<2>(tmem + C_S, at(S0), at(slot_k(n)), ID_KK, false);
+        mma_commit(bars + kKvZ);
+      };
+      if (elect_one()) issue_z(0);
+#pragma unroll 1
+      for (int n = 0; n < end; ++n) {
+        const int m = n - begin;
+        const uint32_t ph = n & 1, ph_m = m & 1, sK = slot_k(n), sV = slot_v(n);
+        const bool diag = n == walk - 1, more = n + 1 < end;
+        if (CUT && m < 0) {
+          next(kKvStored);
+          if (elect_one()) {
+            mbar_wait(bars + kKvIn, ph, abortp);
+            tc_fence_after();
+            gemm_km_t<8>(tmem + C_W, at(sK), at(sV), ID_KM_NEG, true);   // W -= A Vu alone
+            mma_commit(bars + kKvW);
+            issue_z(n + 1);
+          }
+          continue;
+        }
+        next(kKvRead);     // Z
+        if (elect_one()) {
+          mbar_wait(bars + kKvIn, ph, abortp);
+          tc_fence_after();
+          gemm_kk_t<2>(tmem + C_S, at(S3), at(sV), ID_KK, false);        // T = Qc Vu^T, while the gate is formed
+          mma_commit(bars + kKvT);
+        }
+        next(kKvStored);   // A
+        if (elect_one()) {
+          if (!diag) gemm_km_t<8>(tmem + C_W, at(sK), at(sV), ID_KM_NEG, true);   // W -= A Vu; at the diagonal block nothing reads it
+          mma_commit(bars + kKvW);
+        }
+        next(kKvStoredT);  // masked T
+        if (elect_one()) gemm_kk_t<2>(tmem + C_S, at(sV), at(sK), ID_KK, false);  // Su/scale = T A^T + Qc Wb^T, while W is copied
+        next(kKvStored);   // copy of W
+        if (elect_one()) {
+          if (!diag) gemm_kk_t<2>(tmem + C_S, at(S3), at(S0), ID_KK, true);
+          mma_commit(bars + kKvSu);
+        }
+        next(kKvRead);     // Su
+        if (elect_one()) {
+          if (m == 0) mbar_wait(bars + kKvRes, 0, abortp);
+          tc_fence_after();
+          gemm_kk_t<2>(tmem + C_S, at(S3), at(S4), ID_KK, false);        // Sc/scale = Qc Kc^T, while silu' is formed
+          mma_commit(bars + kKvSc);
+        }
+        next(kKvRead);     // Sc
+        if (elect_one()) {
+          mbar_wait(bars + kKvDo, ph_m, abortp);
+          tc_fence_after();
+          gemm_kk_t<2>(tmem + C_S, at(S6), at(S5), ID_KK, false);        // dP = dO Vc^T, while P is formed
+          mma_commit(bars + kKvDp);
+        }
+        next(kKvStored);   // P
+        if (elect_one()) {
+          gemm_mm_t<8>(tmem + C_DVC, at(sV), at(S6), ID_MM, m > 0);      // dvc += P^T dO, while dS is formed
+          mma_commit(bars + kKvDv);
+        }
+        next(kKvStored);   // dS, dSu
+        if (elect_one()) {
+          if (!diag) gemm_km_t<8>(tmem + C_S, at(S6), at(S0), ID_KM, false);   // dqc = dSu Wb + dS Kc
+          mma_commit(bars + kKvX0);
+          gemm_km_t<8>(tmem + C_S, at(sK), at(S4), ID_KM, !diag);
+          mma_commit(bars + kKvX);
+          gemm_mm_t<8>(tmem + C_DKC, at(sK), at(S3), ID_MM, m > 0);      // dkc += dS^T Qc
+          mma_commit(bars + kKvK);
+        }
+        next(kKvRead);     // dqc
+        if (more && elect_one()) issue_z(n + 1);
+      }
+      __syncwarp();
+    } else if (warp == kSplitWorkers / 32 + 1) {
+      // ---- the tiles
+      if (elect_one()) {
+        const int il = (p.nblk - 1) * kBlkB;
+        mbar_expect_tx(bars + kKvZin, 2 * kSq);
+        load_op(smem + S0, m_qu, bars + kKvZin, k0, h, b);
+        load_op(smem + slot_k(0), m_ku, bars + kKvZin, il, h, b);
+        mbar_expect_tx(bars + kKvIn, begin == 0 ? 2 * kSq : kSq);
+        if (begin == 0) load_op(smem + S3, m_qc, bars + kKvIn, il, h, b);
+        load_op(smem + slot_v(0), m_vu, bars + kKvIn, il, h, b);
+        mbar_expect_tx(bars + kKvRes, kSq);
+        load_op(smem + S4, m_kc, bars + kKvRes, k0, h, b);
+        mbar_expect_tx(bars + kKvDo, 2 * kSq);
+        load_op(smem + S5, m_vc, bars + kKvDo, k0, h, b);
+        load_op(smem + S6, m_do, bars + kKvDo, il - begin * kBlkB, h, b);
+      }
+#pragma unroll 1
+      for (int n = 0; n < end; ++n) {
+        const int m = n - begin, i0 = (p.nblk - 1 - n) * kBlkB, in0 = i0 - kBlkB;
+        const uint32_t ph = n & 1, ph_m = m & 1;
+        const bool more = n + 1 < end;
+        uint8_t *const tile = step_tiles(p, p.nblk - 1 - n, K), *const sK = smem + slot_k(n), *const sV = smem + slot_v(n);
+        __syncwarp();
+        if (CUT && m < 0) {   // the next step's tiles land over both once they are consumed, Qu stays
+          if (elect_one()) {
+            mbar_wait(bars + kKvW, ph, abortp);
+            mbar_expect_tx(bars + kKvZin, kSq);
+            load_op(sV, m_ku, bars + kKvZin, in0, h, b);
+            mbar_expect_tx(bars + kKvIn, m == -1 ? 2 * kSq : kSq);
+            if (m == -1) load_op(smem + S3, m_qc, bars + kKvIn, in0, h, b);
+            load_op(sK, m_vu, bars + kKvIn, in0, h, b);
+          }
+          continue;
+        }
+        if (elect_one()) {
+          mbar_wait(bars + kKvW, ph, abortp);       // the gate is there
+          bulk_s2g(tile + kTileA, sK, kSq);
+          bulk_commit();
+          if (m > 0) {
+            bulk_wait_read1();                      // the reduces of the step before have read their panels
+            mbar_expect_tx(bars + kKvDo, 2 * kSq);
+            load_op(smem + S5, m_vc, bars + kKvDo, k0, h, b);
+            load_op(smem + S6, m_do, bars + kKvDo, i0, h, b);
+          }
+          bulk_wait_read0();
+          mbar_arrive(bars + kKvDp);                // dS may go over the gate
+          mbar_wait(bars + kKvDv, ph_m, abortp);
+          if (more) {
+            mbar_expect_tx(bars + kKvZin, 2 * kSq);
+            mbar_expect_tx(bars + kKvIn, 2 * kSq);
+            load_op(sV, m_ku, bars + kKvZin, in0, h, b);   // over P
+          }
+          mbar_wait(bars + kKvX0, ph_m, abortp);
+          if (more) load_op(smem + S0, m_qu, bars + kKvZin, k0, h, b);
+          bulk_s2g(tile + kTileDsu, smem + S6, kSq);       // behind what the next product waits for
+          bulk_commit();
+          mbar_wait(bars + kKvK, ph_m, abortp);
+          if (more) {                               // before the reduces, which loads would queue behind
+            load_op(smem + S3, m_qc, bars + kKvIn, in0, h, b);
+            load_op(sK, m_vu, bars + kKvIn, in0, h, b);
+          }
+          bulk_wait_read0();
+          mbar_arrive(bars + kKvCopied);            // dqc may be staged over dSu
+        }
+        __syncwarp();
+        ev_wait(kKvStaged, kSplitWorkers);
+        if (elect_one()) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tma_reduce_add_3d(&m_acc_dqc, smem + S5 + c * kPanelB, c * 32, i0, bh);
+          bulk_commit();
+        }
+      }
+      __syncwarp();
+      if (elect_one()) bulk_wait0();
+      __syncwarp();
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSplitWorkerRegs));
+    const int row = (warp & 3) * 32 + lane, cc = warp >> 2, c0 = cc * 32, krow = k0 + row;
+    const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
+    auto wait = [&](int bar, uint32_t ph) {
+      mbar_wait(bars + bar, ph, abortp);
+      tc_fence_after();
+    };
+    auto read = [&]() { return ev_arrive_read(kKvRead, kSplitWorkers, zero_s); };
+    auto stored = [&](int id) {
+      fence_async_smem();
+      tc_fence_before();
+      ev_arrive(id, kSplitWorkers);
+    };
+    {  // W starts as the forward's final state
+      const float* src = p.w_state + ((int64_t)bh * p.N + krow) * 128 + c0;
+      float v[32];
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) {
+        const float4 q = (krow < p.N) ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w;
+      }
+      tmem_st32(trow + C_W + c0, v);
+      tmem_st_wait();
+    }
+#pragma unroll 1
+    for (int n = 0; n < end; ++n) {
+      const int m = n - begin;                    // of the steps with scores
+      const uint32_t ph = n & 1, ph_m = m & 1;    // barriers that complete in every step; in steps with scores
+      const int I = p.nblk - 1 - n, irow = I * kBlkB + row;
+      const bool diag = I == K, rvalid = irow < p.N;
+      uint8_t *const sK = smem + slot_k(n), *const sV = smem + slot_v(n);
+      B128_MARK(0, n, 0);
+      wait(kKvZ, ph);
+      B128_MARK(0, n, 1);
+      {
+        float v[32];
+        tmem_ld32(trow + C_S + c0, v);
+        tmem_ld_wait();
+        float hs = half_scale;
+        if (!CUT || m >= 0) hs += read();
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), hs);
+          v[j] = a.x; v[j + 1] = a.y;
+        }
+        if (diag) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
+        }
+        store_row32<T>(sK, kPanelB, row, c0, v);
+      }
+      stored(kKvStored);
+      if (CUT && m < 0) continue;
+      B128_MARK(0, n, 2);
+      wait(kKvT, ph_m);
+      {  // T over Vu, which the state has then read
+        float v[32];
+        tmem_ld32_lower(trow + C_S + c0, row, c0, v);
+        wait(kKvW, ph);
+        B128_MARK(0, n, 3);
+        store_row32<T>(sV, kPanelB, row, c0, v);
+      }
+      stored(kKvStoredT);
+      if (!diag) {   // Wb over Qu
+        float v[32];
+        tmem_ld32(trow + C_W + c0, v);
+        tmem_ld_wait();
+        store_row32<T>(smem + S0, kPanelB, row, c0, v);
+      }
+      stored(kKvStored);
+      B128_MARK(0, n, 4);
+      // loaded here, not at the top of the step, where the wait for Z is short
+      const float lse_i = rvalid ? p.lse[(int64_t)bh * p.N + irow] : 0.f, delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
+      wait(kKvSu, ph_m);
+      B128_MARK(0, n, 5);
+      uint32_t dpk[16], ppk[16];
+      {
+        float v[32], w[32];
+        tmem_ld32(trow + C_S + c0, v);
+        tmem_ld_wait();
+        const float hs = half_scale + read();
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 u = make_float2(v[j], v[j + 1]);
+          const float2 g = sigmoid2(u, hs);
+          // silu'(su) = g + silu(su) (1 - g)
+          const float2 q = mul2(mul2(u, g), splat(-1.f));   // -silu(su) / scale
+          v[j] = q.x; v[j + 1] = q.y;
+          const float2 d = fma2(mul2(q, splat(-p.scale)), fma2(g, splat(-1.f), splat(1.f)), g);
+          dpk[j / 2] = Elem<T>::pack2(d.x, d.y);
+        }
+        B128_MARK(0, n, 6);
+        wait(kKvSc, ph_m);
+        B128_MARK(0, n, 7);
+        tmem_ld32(trow + C_S + c0, w);
+        tmem_ld_wait();
+        const float s2 = sl2 + read();
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(s2), splat(-lse_i * kLog2e));
+          v[j] = ex2_approx(x.x); v[j + 1] = ex2_approx(x.y);
+        }
+        if (diag) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
+        }
+        if (!rvalid) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) ppk[j / 2] = Elem<T>::pack2(v[j], v[j + 1]);
+        store_row32<T>(sV, kPanelB, row, c0, v);   // P, over T
+      }
+      stored(kKvStored);
+      B128_MARK(0, n, 8);
+      wait(kKvDp, ph_m);
+      B128_MARK(0, n, 9);
+      {
+        float v[32], w[32];
+        tmem_ld32(trow + C_S + c0, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float2 ds = mul2(Elem<T>::unpack2(ppk[j / 2]), add2(make_float2(v[j], v[j + 1]), splat(-delta_i)));
+          const float2 du = mul2(ds, Elem<T>::unpack2(dpk[j / 2]));
+          v[j] = ds.x; v[j + 1] = ds.y;
+          w[j] = -du.x; w[j + 1] = -du.y;
+        }
+        store_row32<T>(sK, kPanelB, row, c0, v);   // dS
+        mbar_wait(bars + kKvDv, ph_m, abortp);
+        store_row32<T>(smem + S6, kPanelB, row, c0, w);   // dSu, over dO
+      }
+      stored(kKvStored);
+      B128_MARK(0, n, 10);
+      wait(kKvX, ph_m);
+      B128_MARK(0, n, 11);
+      // ---- dqc staged over Vc and dSu
       float v[32];
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), half_scale);
-        v[j] = a.x; v[j + 1] = a.y;
-      }
-      if (diag) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = (c0 + j > row) ? v[j] : 0.f;
-      }
-      store_row32<T>(sK, kPanelB, row, c0, v);
+      read();
+      if (cc >= 2) mbar_wait(bars + kKvCopied, ph_m, abortp);
+      store_row32_f32(smem + S5 + cc * kPanelB, row, v);
+      fence_async_smem();
+      ev_arrive(kKvStaged, kSplitWorkers);
+      B128_MARK(0, n, 12);
     }
-    B128_SYNC()
-    B128_MARK(0, n, 3);
-    if (CUT && m < 0) {
-      // ---- W -= A Vu alone; the next step's tiles land over both once they are consumed, Qu stays
-      if (warp == 0 && elect_one()) {
-        mbar_wait(bar_in, ph, abortp);
-        tc_fence_after();
-        gemm_km_t<8>(tmem + C_W, aK, aV, ID_KM_NEG, true);
-        mma_commit(bar_w);
-      }
-      if (loader && elect_one()) {
-        mbar_wait(bar_w, ph, abortp);
-        mbar_expect_tx(bar_z, kSq);
-        load_op(sV, m_ku, bar_z, i0 - kBlkB, h, b);
-        mbar_expect_tx(bar_in, m == -1 ? 2 * kSq : kSq);
-        if (m == -1) load_op(s3, m_qc, bar_in, i0 - kBlkB, h, b);
-        load_op(sK, m_vu, bar_in, i0 - kBlkB, h, b);
-      }
-      if (warp == 0 && elect_one()) {
-        mbar_wait(bar_z, ph ^ 1, abortp);
-        tc_fence_after();
-        gemm_kk_t<2>(tmem + C_S, a0, aV, ID_KK, false);
-        mma_commit(bar_mma);
-      }
-      __syncwarp();
-      continue;
-    }
-    // ---- T = Qc Vu^T;  W -= A Vu
-    if (warp == 0 && elect_one()) {
-      mbar_wait(bar_in, ph, abortp);
-      tc_fence_after();
-      gemm_kk_t<2>(tmem + C_S, a3, aV, ID_KK, false);
-      mma_commit(bar_t);
-      gemm_km_t<8>(tmem + C_W, aK, aV, ID_KM_NEG, true);
-      mma_commit(bar_w);
-    }
-    if (storer && elect_one()) { bulk_s2g(tile + kTileA, sK, kSq); bulk_commit(); }
-    __syncwarp();
-    mbar_wait(bar_t, ph_m, abortp);
-    tc_fence_after();
-    B128_MARK(0, n, 4);
-    {  // T over Vu, Wb over Qu
-      float v[32], w[32];
-      tmem_ld32_lower(trow + C_S + c0, row, c0, v);
-      mbar_wait(bar_w, ph, abortp);
-      tc_fence_after();
-      tmem_ld32(trow + C_W + c0, w);
-      store_row32<T>(sV, kPanelB, row, c0, v);
-      tmem_ld_wait();
-      store_row32<T>(s0, kPanelB, row, c0, w);
-    }
-    B128_SYNC()
-    B128_MARK(0, n, 5);
-    // ---- Su/scale = Qc Wb^T + T A^T
-    if (warp == 0 && elect_one()) {
-      tc_fence_after();
-      if (!diag) gemm_kk_t<2>(tmem + C_S, a3, a0, ID_KK, false);
-      gemm_kk_t<2>(tmem + C_S, aV, aK, ID_KK, !diag);
-      mma_commit(bar_mma);
-    }
-    __syncwarp();
-    if (reducer && m > 0 && elect_one()) {   // the reduce of the step before has had time to read its panel, and all wait for Su anyway
-      bulk_wait_read0();
-      load_panel(i0);
-    }
-    __syncwarp();
-    // loaded here, not at the top of the step, where the wait for Z is short (1777 -> 1746 us at N=8190 H=8)
-    const float lse_i = rvalid ? p.lse[(int64_t)bh * p.N + irow] : 0.f, delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
-    mbar_wait(bar_mma, ph_mma, abortp);
-    ph_mma ^= 1;
-    tc_fence_after();
-    B128_MARK(0, n, 6);
-    uint32_t dpk[16], ppk[16];
-    {
-      float v[32], w[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncthreads();
-      // ---- Sc/scale = Qc Kc^T, while silu' is formed
-      if (warp == 0 && elect_one()) {
-        if (m == 0) mbar_wait(bar_res, 0, abortp);
-        tc_fence_after();
-        gemm_kk_t<2>(tmem + C_S, a3, a4, ID_KK, false);
-        mma_commit(bar_mma);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 u = make_float2(v[j], v[j + 1]);
-        const float2 g = sigmoid2(u, half_scale);
-        // silu'(su) = g + silu(su) (1 - g)
-        const float2 q = mul2(mul2(u, g), splat(-1.f));   // -silu(su) / scale
-        v[j] = q.x; v[j + 1] = q.y;
-        const float2 d = fma2(mul2(q, splat(-p.scale)), fma2(g, splat(-1.f), splat(1.f)), g);
-        dpk[j / 2] = Elem<T>::pack2(d.x, d.y);
-      }
-      B128_MARK(0, n, 7);
-      mbar_wait(bar_mma, ph_mma, abortp);
-      ph_mma ^= 1;
-      tc_fence_after();
-      tmem_ld32(trow + C_S + c0, w);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(sl2), splat(-lse_i * kLog2e));
-        v[j] = ex2_approx(x.x); v[j + 1] = ex2_approx(x.y);
-      }
-      if (diag) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = (c0 + j <= row) ? v[j] : 0.f;
-      }
-      if (!rvalid) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0.f;
-      }
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) ppk[j / 2] = Elem<T>::pack2(v[j], v[j + 1]);
-      store_row32<T>(sV, kPanelB, row, c0, v);   // P, over T
-    }
-    if (storer && elect_one()) bulk_wait_read0();   // A has been read: dS goes there
-    __syncwarp();
-    B128_SYNC()
-    B128_MARK(0, n, 8);
-    // ---- dP = dO Vc^T;  dvc += P^T dO
-    if (warp == 0 && elect_one()) {
-      mbar_wait(bar_do, ph_m, abortp);
-      tc_fence_after();
-      gemm_kk_t<2>(tmem + C_S, a6, a5, ID_KK, false);
-      mma_commit(bar_mma);
-      gemm_mm_t<8>(tmem + C_DVC, aV, a6, ID_MM, m > 0);
-      mma_commit(bar_dv);
-    }
-    __syncwarp();
-    mbar_wait(bar_mma, ph_mma, abortp);
-    ph_mma ^= 1;
-    tc_fence_after();
-    B128_MARK(0, n, 9);
-    {
-      float v[32], w[32];
-      tmem_ld32(trow + C_S + c0, v);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float2 ds = mul2(Elem<T>::unpack2(ppk[j / 2]), add2(make_float2(v[j], v[j + 1]), splat(-delta_i)));
-        const float2 du = mul2(ds, Elem<T>::unpack2(dpk[j / 2]));
-        v[j] = ds.x; v[j + 1] = ds.y;
-        w[j] = -du.x; w[j + 1] = -du.y;
-      }
-      store_row32<T>(sK, kPanelB, row, c0, v);   // dS
-      mbar_wait(bar_dv, ph_m, abortp);
-      store_row32<T>(s6, kPanelB, row, c0, w);   // dSu, over dO
-    }
-    B128_SYNC()
-    B128_MARK(0, n, 10);
-    // ---- dqc = dSu Wb + dS Kc;  dkc += dS^T Qc
-    if (warp == 0 && elect_one()) {
-      tc_fence_after();
-      if (!diag) gemm_km_t<8>(tmem + C_S, a6, a0, ID_KM, false);
-      mma_commit(bar_x0);
-      gemm_km_t<8>(tmem + C_S, aK, a4, ID_KM, !diag);
-      mma_commit(bar_x);
-      gemm_mm_t<8>(tmem + C_DKC, aK, a3, ID_MM, m > 0);
-      mma_commit(bar_k);
-    }
-    if (loader && elect_one()) {
-      if (more) {
-      mbar_expect_tx(bar_z, 2 * kSq);
-      mbar_expect_tx(bar_in, 2 * kSq);
-      mbar_expect_tx(bar_do, 2 * kSq);
-      load_op(sV, m_ku, bar_z, i0 - kBlkB, h, b);   // over P
-      mbar_wait(bar_x0, ph_m, abortp);
-      load_op(s0, m_qu, bar_z, k0, h, b);
-      }
-      bulk_s2g(tile + kTileDsu, s6, kSq);   // behind what the next product waits for
-      bulk_commit();
-    }
-    __syncwarp();
-    mbar_wait(bar_x, ph_m, abortp);
-    tc_fence_after();
-    B128_MARK(0, n, 11);
-    float v[32];
-    tmem_ld32(trow + C_S + c0, v);
-    tmem_ld_wait();
-    tc_fence_before();
-    __syncthreads();
-    B128_MARK(0, n, 12);
-    // ---- the next step's Z, while dqc is staged
-    if (warp == 0 && more && elect_one()) {
-      mbar_wait(bar_z, ph ^ 1, abortp);
-      tc_fence_after();
-      gemm_kk_t<2>(tmem + C_S, a0, aV, ID_KK, false);
-      mma_commit(bar_mma);
-    }
-    // before the reduces, which loads would queue behind
-    if (loader && elect_one()) {
-       if (more) {
-        mbar_wait(bar_k, ph_m, abortp);
-        load_op(s3, m_qc, bar_in, i0 - kBlkB, h, b);
-        load_op(sK, m_vu, bar_in, i0 - kBlkB, h, b);
-      }
-      bulk_wait_read0();   // dSu has been read
-    }
-    __syncwarp();
-    if (cc >= 2) asm volatile("bar.sync 5, 256;" ::: "memory");   // the two groups that stage over dSu
-    uint8_t* panel = s5 + cc * kPanelB;
-    store_row32_f32(panel, row, v);
-    fence_async_smem();
-    group_sync(1 + cc);
-    B128_MARK(0, n, 13);
-    if (reducer && elect_one()) {
-      mbar_wait(bar_k, ph_m, abortp);
-      tma_reduce_add_3d(&m_acc_dqc, panel, cc * 32, i0, bh);
-      bulk_commit();
-    }
-  }
-  if ((reducer || storer || loader) && elect_one()) bulk_wait0();
-  __syncwarp();
-  mbar_wait(bar_k, (uint32_t)(end - begin - 1) & 1u, abortp);
-  tc_fence_after();
-  {
+    wait(kKvK, (uint32_t)(end - begin - 1) & 1u);
     float v[32], w[32];
     tmem_ld32(trow + C_DKC + c0, v);
     tmem_ld32(trow + C_DVC + c0, w);
     tmem_ld_wait();
     if (cut) {   // over Qu to Qc, which every product has read
-      uint8_t *pk = s0 + cc * kPanelB, *pv = s2 + cc * kPanelB;
+      uint8_t *pk = smem + S0 + cc * kPanelB, *pv = smem + 2 * kSq + cc * kPanelB;
       store_row32_f32(pk, row, v);
       store_row32_f32(pv, row, w);
       fence_async_smem();
-      group_sync(1 + cc);
-      if (reducer && elect_one()) {
+      group_sync(kKvGroups + cc);
+      if ((warp & 3) == 1 && elect_one()) {
         uint8_t* dst = kv_part(p, bh, K, part) + cc * kPanelB;
         bulk_s2g(dst, pk, kPanelB);
         bulk_s2g(dst + kPartSum, pv, kPanelB);
@@ -492,7 +520,7 @@ __global__ void __launch_bounds__(kB128Threads, 1)
 castle_bwd128_reverse_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc) {
   constexpr uint32_t ID_MM = make_idesc(128, 128, Elem<T>::fmt, true, true, false);
   const int K = blockIdx.y, steps = p.nblk - 1 - K;
-  B128_BEGIN(6 * kSq, 4, 128)
+  B128_BEGIN(6 * kSq, 4, -1, 128)
   uint64_t *bar_in = bars, *bar_g = bars + 2;   // two each
   const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;
   const bool loader = warp == 4, storer = warp == 8;
@@ -561,7 +589,7 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
                      ID_MM = make_idesc(128, 128, FMT, true, true, false);
   const int I = p.nblk - 1 - blockIdx.y, i0 = I * kBlkB;   // the longest walks first
   const bool last = I == p.nblk - 1;                       // no G there yet
-  B128_BEGIN(7 * kSq, 10, 512)
+  B128_BEGIN(7 * kSq, 10, -1, 512)
   uint8_t *sVu = smem, *sT = smem + kSq, *sA = smem + 2 * kSq, *sS = smem + 3 * kSq, *sG = smem + 4 * kSq, *sQu = smem + 5 * kSq,
           *sZ = smem + 6 * kSq;
   uint64_t *bar_res = bars, *bar_in = bars + 1, *bar_qu = bars + 2, *bar_da = bars + 3, *bar_v = bars + 4, *bar_k = bars + 5, *bar_t = bars + 6,
@@ -733,7 +761,7 @@ __global__ void __launch_bounds__(128)
 castle_bwd128_dqu_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_ku) {
   constexpr uint32_t ID_KM = make_idesc(128, 128, Elem<T>::fmt, false, true, false);
   const int K = blockIdx.y, k0 = K * kBlkB, steps = p.nblk - K;
-  B128_BEGIN(6 * kSq, 7, 128)
+  B128_BEGIN(6 * kSq, 7, -1, 128)
   uint64_t *bar_in = bars, *bar_done = bars + 3, *bar_end = bars + 6;   // three, three, one
   if (warp == 0 && elect_one()) {
     auto load = [&](int n) {
@@ -786,6 +814,9 @@ static int launch_bwd128_t(const BwdParams& p, const CUtensorMap* in, cudaStream
   constexpr int D = 128;
   const void* kernels[5] = {(const void*)castle_bwd128_kv_kernel<T, false>, (const void*)castle_bwd128_reverse_kernel<T>,
                             (const void*)castle_bwd128_la_kernel<T>, (const void*)castle_bwd128_dqu_kernel<T>, (const void*)castle_bwd128_kv_kernel<T, true>};
+  static const int regs_rc[2] = {check_launch_regs(castle_bwd128_kv_kernel<T, false>, "castle_bwd"), check_launch_regs(castle_bwd128_kv_kernel<T, true>, "castle_bwd")};
+  for (int rc : regs_rc)
+    if (rc) return rc;
   const size_t smem[5] = {kB128Smem, 6 * kSq + 256, kB128Smem, 6 * kSq + 256, kB128Smem};
   for (int i = 0; i < 5; ++i) {
     cudaError_t e = cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[i]);
@@ -813,7 +844,7 @@ static int launch_bwd128_t(const BwdParams& p, const CUtensorMap* in, cudaStream
     const dim3 grid(pairs, p.nblk), kv_grid(pairs, q.kv_split ? 2 * p.nblk : p.nblk);
     // in[]: qc, kc, vc, qu, ku, vu, dout
     // each starts while the one before it ends
-    cudaError_t e = launch_kernel(q.kv_split ? castle_bwd128_kv_kernel<T, true> : castle_bwd128_kv_kernel<T, false>, kv_grid, kB128Threads, smem[0], st, true, q, in[0], in[1], in[2], in[3], in[4], in[5], in[6], acc);
+    cudaError_t e = launch_kernel(q.kv_split ? castle_bwd128_kv_kernel<T, true> : castle_bwd128_kv_kernel<T, false>, kv_grid, kSplitThreads, smem[0], st, true, q, in[0], in[1], in[2], in[3], in[4], in[5], in[6], acc);
     if (e == cudaSuccess && p.nblk > 1) e = launch_kernel(castle_bwd128_reverse_kernel<T>, dim3(pairs, p.nblk - 1), kB128Threads, smem[1], st, true, q, in[0]);
     if (e == cudaSuccess) e = launch_kernel(castle_bwd128_la_kernel<T>, grid, kB128Threads + 32, smem[2], st, true, q, in[0], in[3], in[5]);
     if (e == cudaSuccess) e = launch_kernel(castle_bwd128_dqu_kernel<T>, grid, 128, smem[3], st, true, q, in[4]);

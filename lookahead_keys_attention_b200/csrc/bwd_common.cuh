@@ -31,6 +31,35 @@ struct BwdParams {
 #endif
 };
 
+// The kernels whose passes, products and tiles are the work of different warps (castle_bwd_kernel, castle_bwd128_kv_kernel): warps
+// 0-15 do the passes, warp 16 issues the products, warp 17 moves tiles, two more fill up the warpgroup.  The launch's registers
+// are shared out anew, 640 x 96 = 61440 as 512 x 112 + 128 x 32.
+constexpr int kSplitWorkers = 512, kSplitThreads = kSplitWorkers + 128;
+constexpr int kSplitLaunchRegs = 96, kSplitWorkerRegs = 112, kSplitHelperRegs = 32;
+static_assert(kSplitWorkers * kSplitWorkerRegs + 128 * kSplitHelperRegs <= kSplitThreads * kSplitLaunchRegs, "setmaxnreg would wait forever");
+
+// Named barriers on which the passes' `threads` arrive and go on, and one warp besides waits.
+__device__ __forceinline__ void ev_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads + 32) : "memory"); }
+__device__ __forceinline__ void ev_wait(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads + 32) : "memory"); }
+// The arrival when a thread's accumulator columns are in registers.  Returns 0, read from shared memory behind it: the compiler
+// moves an arrival behind arithmetic that does not depend on it, and the next product then starts a pass late, so a constant of
+// the pass has this added to it (dim_head 64, B=4 N=4096 H=16: 2044 -> 1936 us).
+__device__ __forceinline__ float ev_arrive_read(int id, int threads, const float* zero_s) {
+  tc_fence_before();
+  ev_arrive(id, threads);
+  float zero;
+  asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(zero) : "r"(smem_u32(zero_s)) : "memory");
+  return zero;
+}
+// 0 if `kernel` was compiled to start with the registers that the sharing above counts on
+template <typename Kernel>
+int check_launch_regs(Kernel kernel, const char* name) {
+  cudaFuncAttributes a;
+  const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+  if (e != cudaSuccess) return cuda_fail(e, name);
+  return a.numRegs == kSplitLaunchRegs ? 0 : reject("%s: compiled with %d registers a thread instead of %d", name, a.numRegs, kSplitLaunchRegs);
+}
+
 // delta[b,h,i] = sum_d out * dout  (lookahead_keys_attention_triton.py:175-214 in the reference); clears the first NACC of the
 // fp32 accumulators on the way (a memset of its own is a launch more).
 template <typename T, int D, int NACC>
