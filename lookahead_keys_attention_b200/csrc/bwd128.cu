@@ -12,7 +12,7 @@
 // every step) took 18.5 k cycles a step, 12.1 k without the reduces; reverse + la + dqu take 3.1 + 7.3 + 1.9 k, and kv, which
 // no longer forms dT, 4.6 k less.  Measured on B=1 H=8 N=8190 bf16: 2365 -> 1708 us for the kernels, B=2 H=8 N=1333:
 // 249 -> 182 us.  What bounds them: kv its chain of products and passes and shared memory; la and reverse the tiles, which
-// come at 20 to 30 bytes per cycle and SM with one step's worth of shared memory to prefetch into; dqu HBM.  
+// come at 20 to 30 bytes per cycle and SM with one step's worth of shared memory to prefetch into; dqu HBM.
 //
 // Tiles of a step (I,K): A, then dZ | dSu | Gb; 32 KB each, as they lie in shared memory (128-byte swizzle).  The scratch is
 // bounded (kTileScratchLimit): the (batch, head) pairs run in chunks, one launch of each kernel per chunk.
@@ -100,7 +100,7 @@ __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K)
 //   dqc, dkc | staging (the next Z under it)
 // Sixteen warps do the passes, one issues the products, one moves the tiles (ev_arrive).  While warp 0 issued the products and also
 // worked in the passes, it waited as long as the tensor unit's queue was full and the others waited for it: step 15.2 k -> 12.9 k
-// cycles, the kernel at B=1 H=8 N=8190 995 -> 884 us, B=2 H=8 N=1333 104 -> 95, B=8 H=16 N=512 141 -> 133.  What bounds it now: 10.7 k
+// cycles, the kernel at B=1 H=8 N=8190 995 -> 884 us, B=2 H=8 N=1333 104 -> 92, B=8 H=16 N=512 141 -> 133.  What bounds it now: 10.7 k
 // cycles of a step's 1.4 MB through shared memory, and the wait for Qc and Vu, whose slots the last product of a step frees.
 // Tensor memory: W | dkc | dvc | scratch.  Shared memory, seven tiles:
 //   s0 Qu, then Wb | s1 Ku, A, dS | s2 Vu, T, P | s3 Qc | s4 Kc | s5 Vc, staging | s6 dO, dSu, staging
@@ -317,7 +317,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
     const int row = (warp & 3) * 32 + lane, cc = warp >> 2, c0 = cc * 32, krow = k0 + row;
     const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
     auto wait = [&](int bar, uint32_t ph) {
-      mbar_wait(bars + bar, ph, abortp);
+      mbar_wait_lazy_abort(bars + bar, ph, abortp);   // B=2 H=8 N=1333: 95.2 -> 92.3 us (one polling lane a warp: 100.7); no difference at dim_head 64
       tc_fence_after();
     };
     auto read = [&]() { return ev_arrive_read(kKvRead, kSplitWorkers, zero_s); };
