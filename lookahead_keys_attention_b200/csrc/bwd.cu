@@ -26,6 +26,8 @@
 // pass that everybody waited for.  A pass reports twice, on named barriers where only the issuing warp waits: when the accumulator
 // columns are in registers (the next product into them starts under the arithmetic) and when its results are in shared memory.
 // Step 19.1 k -> 15.5 k cycles; the kernel at B=4 N=4096 H=16 2390 -> 1936 us, B=16 H=8 N=1024 387 -> 332, 15 pairs of 777 78.2 -> 63.3.
+// The first tiles and the state are asked for before the CTA's first barrier, and a CTA leaves when its last reduces have been
+// read, not done: 1024 pairs of one block 115.2 -> 112.3 us, 4 pairs of two 23.7 -> 22.3.
 #include "bwd_common.cuh"
 
 namespace castle {
@@ -94,7 +96,9 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   const int b = bh / p.H, h = bh % p.H;
   const int k0 = K * kBlkB, walk = p.nblk - K;
 
-  if (tid == 0) {
+  // The first tiles are on their way before the barrier below; nothing in flight writes what they read (only the sums and delta are
+  // being written by the kernel before this one).
+  if (warp == 17 && elect_one()) {
     if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
     uint64_t* const bars[17] = {&bar_res, &bar_load, &bar_vd, &bar_ku, &bar_kn, &bar_z, &bar_t, &bar_w,
                                 &bar_su, &bar_sc, &bar_dp, &bar_dv, &bar_da, &bar_dt, &bar_g, &bar_x, &bar_l};
@@ -103,6 +107,30 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     mbar_fence_init();
     abort_flag = 0;
     zero_s = 0.f;
+    const int il = (p.nblk - 1) * kBlkB;
+    mbar_expect_tx(&bar_res, 2 * OPB);
+    tma_load_4d(sQu, &m_qu, &bar_res, 0, k0, h, b);
+    mbar_expect_tx(&bar_kn, OPB);
+    tma_load_4d(sKP, &m_ku, &bar_kn, 0, il, h, b);
+    tma_load_4d(sKc, &m_kc, &bar_res, 0, k0, h, b);
+    mbar_expect_tx(&bar_load, 2 * OPB);
+    tma_load_4d(sQc, &m_qc, &bar_load, 0, il, h, b);
+    tma_load_4d(sVu, &m_vu, &bar_load, 0, il, h, b);
+    mbar_arrive(&bar_t);
+    mbar_arrive(&bar_w);
+    mbar_expect_tx(&bar_vd, 2 * OPB);
+    tma_load_4d(sVc, &m_vc, &bar_vd, 0, k0, h, b);
+    tma_load_4d(sdO, &m_do, &bar_vd, 0, il, h, b);
+  }
+  __syncwarp();
+  constexpr int kWLoads = kBlkB * (D / 4) / kSplitWorkers;
+  float4 w0[kWLoads];   // of the forward's final state
+  if (warp < kSplitWorkers / 32) {
+#pragma unroll
+    for (int i = 0; i < kWLoads; ++i) {
+      const int e = i * kSplitWorkers + tid, r = e / (D / 4), c = e % (D / 4);
+      w0[i] = (k0 + r < p.N) ? *reinterpret_cast<const float4*>(p.w_state + ((int64_t)bh * p.N + k0 + r) * D + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
   if (warp == 0) { tmem_alloc(&tmem_base_s, 512); tmem_relinquish(); }
   overlap_wait();   // launched while delta is being written
@@ -216,22 +244,6 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       __syncwarp();
     } else if (warp == 17) {
       // ---- the tiles.  The TMA unit works its queue off in order and a reduce takes thousands of cycles, so loads go ahead of them.
-      if (elect_one()) {
-        const int il = (p.nblk - 1) * kBlkB;
-        mbar_expect_tx(&bar_res, 2 * OPB);
-        tma_load_4d(sQu, &m_qu, &bar_res, 0, k0, h, b);
-        mbar_expect_tx(&bar_kn, OPB);
-        tma_load_4d(sKP, &m_ku, &bar_kn, 0, il, h, b);
-        tma_load_4d(sKc, &m_kc, &bar_res, 0, k0, h, b);
-        mbar_expect_tx(&bar_load, 2 * OPB);
-        tma_load_4d(sQc, &m_qc, &bar_load, 0, il, h, b);
-        tma_load_4d(sVu, &m_vu, &bar_load, 0, il, h, b);
-        mbar_arrive(&bar_t);
-        mbar_arrive(&bar_w);
-        mbar_expect_tx(&bar_vd, 2 * OPB);
-        tma_load_4d(sVc, &m_vc, &bar_vd, 0, k0, h, b);
-        tma_load_4d(sdO, &m_do, &bar_vd, 0, il, h, b);
-      }
 #pragma unroll 1
       for (int n = 0; n < walk; ++n) {
         const uint32_t ph = n & 1;
@@ -286,7 +298,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         }
       }
       __syncwarp();
-      if (elect_one()) bulk_wait0();
+      if (elect_one()) bulk_wait_read0();   // the sums themselves are complete when the kernel is
       __syncwarp();
     }
   } else {
@@ -297,7 +309,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
     const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
     auto wait = [&](uint64_t* bar, uint32_t ph) {
-      mbar_wait(bar, ph, abortp);
+      mbar_wait_lazy_abort(bar, ph, abortp);   // (one polling lane a warp: 1970 -> 2126 us at B=4 N=4096 H=16)
       tc_fence_after();
     };
     auto read = [&]() { return ev_arrive_read(kEvRead, kSplitWorkers, &zero_s); };
@@ -310,10 +322,9 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     // a row per lane, here and where the gradients are stored, took 2 us of a key block each; 1036 pairs of one block 150.5 ->
     // 142.3 us, B=16 H=8 N=1024 402 -> 392 us
 #pragma unroll
-    for (int i = 0; i < kBlkB * (D / 4) / kSplitWorkers; ++i) {
+    for (int i = 0; i < kWLoads; ++i) {
       const int e = i * kSplitWorkers + tid, r = e / (D / 4), c = e % (D / 4);
-      const float4 q = (k0 + r < p.N) ? *reinterpret_cast<const float4*>(p.w_state + ((int64_t)bh * p.N + k0 + r) * D + c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(sA + (c >> 3) * kPanelB + swz_off(r, c & 7)) = q;
+      *reinterpret_cast<float4*>(sA + (c >> 3) * kPanelB + swz_off(r, c & 7)) = w0[i];
     }
     asm volatile("bar.sync %0, %1;" ::"n"(kWorkers), "n"(kSplitWorkers) : "memory");
     if (c0 < D) {

@@ -52,9 +52,8 @@ __device__ __forceinline__ void load_op(uint8_t* dst, const CUtensorMap& m, uint
 __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K) {   // of this CTA's pair
   return p.tiles + ((int64_t)blockIdx.x * p.ntiles + (int64_t)I * (I + 1) / 2 + K) * kStepTiles;
 }
-// What every kernel starts with: shared memory behind the operands, barriers, tensor memory.  NBAR barriers of one arrival, but
-// two at barrier PAIR (-1: none).
-#define B128_BEGIN(OPERANDS, NBAR, PAIR, COLS)                                                      \
+// What every kernel starts with: shared memory behind the operands, barriers, tensor memory.  NBAR barriers of one arrival.
+#define B128_BEGIN(OPERANDS, NBAR, COLS)                                                      \
   extern __shared__ __align__(1024) uint8_t smem[];                                            \
   uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + (OPERANDS));                       \
   uint32_t* const tmem_base_s = reinterpret_cast<uint32_t*>(bars + (NBAR));                    \
@@ -63,7 +62,7 @@ __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K)
   const int bh = p.bh0 + blockIdx.x, b = bh / p.H, h = bh % p.H;                               \
   if (tid == 0) {                                                                              \
     if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);                  \
-    for (int i = 0; i < (NBAR); ++i) mbar_init(bars + i, i == (PAIR) ? 2 : 1);                 \
+    for (int i = 0; i < (NBAR); ++i) mbar_init(bars + i, 1);                                   \
     mbar_fence_init();                                                                         \
     *abortp = 0;                                                                               \
   }                                                                                            \
@@ -139,14 +138,55 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
   const bool cut = CUT && K < p.kv_split;
   if (part && !cut) return;
   const int begin = part ? kv_cut(walk) : 0, end = cut && !part ? kv_cut(walk) : walk;   // steps with scores; state alone before them
-  B128_BEGIN(7 * kSq, kKvBars, kKvDp, 512)
   // the slot of Ku, A, dS and that of Vu, T, P change places from step to step
   auto slot_k = [](int n) { return (n & 1 ? 2u : 1u) * kSq; };
   auto slot_v = [](int n) { return (n & 1 ? 1u : 2u) * kSq; };
   constexpr uint32_t S0 = 0, S3 = 3 * kSq, S4 = 4 * kSq, S5 = 5 * kSq, S6 = 6 * kSq;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + 7 * kSq);
+  uint32_t* const tmem_base_s = reinterpret_cast<uint32_t*>(bars + kKvBars);
+  volatile int* const abortp = reinterpret_cast<int*>(bars + kKvBars) + 1;
   float* const zero_s = reinterpret_cast<float*>(bars + kKvBars + 1);
-  if (tid == 0) *zero_s = 0.f;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int bh = p.bh0 + blockIdx.x, b = bh / p.H, h = bh % p.H;
+  // The first tiles and the state are asked for before the barrier below; nothing in flight writes what they read (only tiles, sums
+  // and gradients are being written by the kernels before this one).
+  if (warp == kSplitWorkers / 32 + 1 && elect_one()) {
+    if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
+    for (int i = 0; i < kKvBars; ++i) mbar_init(bars + i, i == kKvDp ? 2 : 1);   // dP: the product, and the copy of the gate that dS goes over
+    mbar_fence_init();
+    *abortp = 0;
+    *zero_s = 0.f;
+    const int il = (p.nblk - 1) * kBlkB;
+    mbar_expect_tx(bars + kKvZin, 2 * kSq);
+    load_op(smem + S0, m_qu, bars + kKvZin, k0, h, b);
+    load_op(smem + slot_k(0), m_ku, bars + kKvZin, il, h, b);
+    mbar_expect_tx(bars + kKvIn, begin == 0 ? 2 * kSq : kSq);
+    if (begin == 0) load_op(smem + S3, m_qc, bars + kKvIn, il, h, b);
+    load_op(smem + slot_v(0), m_vu, bars + kKvIn, il, h, b);
+    mbar_expect_tx(bars + kKvRes, kSq);
+    load_op(smem + S4, m_kc, bars + kKvRes, k0, h, b);
+    mbar_expect_tx(bars + kKvDo, 2 * kSq);
+    load_op(smem + S5, m_vc, bars + kKvDo, k0, h, b);
+    load_op(smem + S6, m_do, bars + kKvDo, il - begin * kBlkB, h, b);
+  }
+  __syncwarp();
+  float w0[32];   // of the forward's final state
+  if (warp < kSplitWorkers / 32) {
+    const int krow = k0 + (warp & 3) * 32 + lane;
+    const float* src = p.w_state + ((int64_t)bh * p.N + krow) * 128 + (warp >> 2) * 32;
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+      const float4 q = (krow < p.N) ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+      w0[j] = q.x; w0[j + 1] = q.y; w0[j + 2] = q.z; w0[j + 3] = q.w;
+    }
+  }
+  if (warp == 0) { tmem_alloc(tmem_base_s, 512); tmem_relinquish(); }
+  overlap_wait();
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_base_s, trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
 
   if (warp >= kSplitWorkers / 32) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSplitHelperRegs));
@@ -238,20 +278,6 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       __syncwarp();
     } else if (warp == kSplitWorkers / 32 + 1) {
       // ---- the tiles
-      if (elect_one()) {
-        const int il = (p.nblk - 1) * kBlkB;
-        mbar_expect_tx(bars + kKvZin, 2 * kSq);
-        load_op(smem + S0, m_qu, bars + kKvZin, k0, h, b);
-        load_op(smem + slot_k(0), m_ku, bars + kKvZin, il, h, b);
-        mbar_expect_tx(bars + kKvIn, begin == 0 ? 2 * kSq : kSq);
-        if (begin == 0) load_op(smem + S3, m_qc, bars + kKvIn, il, h, b);
-        load_op(smem + slot_v(0), m_vu, bars + kKvIn, il, h, b);
-        mbar_expect_tx(bars + kKvRes, kSq);
-        load_op(smem + S4, m_kc, bars + kKvRes, k0, h, b);
-        mbar_expect_tx(bars + kKvDo, 2 * kSq);
-        load_op(smem + S5, m_vc, bars + kKvDo, k0, h, b);
-        load_op(smem + S6, m_do, bars + kKvDo, il - begin * kBlkB, h, b);
-      }
 #pragma unroll 1
       for (int n = 0; n < end; ++n) {
         const int m = n - begin, i0 = (p.nblk - 1 - n) * kBlkB, in0 = i0 - kBlkB;
@@ -309,7 +335,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         }
       }
       __syncwarp();
-      if (elect_one()) bulk_wait0();
+      if (elect_one()) bulk_wait_read0();   // the sums themselves are complete when the kernel is
       __syncwarp();
     }
   } else {
@@ -326,17 +352,8 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       tc_fence_before();
       ev_arrive(id, kSplitWorkers);
     };
-    {  // W starts as the forward's final state
-      const float* src = p.w_state + ((int64_t)bh * p.N + krow) * 128 + c0;
-      float v[32];
-#pragma unroll
-      for (int j = 0; j < 32; j += 4) {
-        const float4 q = (krow < p.N) ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-        v[j] = q.x; v[j + 1] = q.y; v[j + 2] = q.z; v[j + 3] = q.w;
-      }
-      tmem_st32(trow + C_W + c0, v);
-      tmem_st_wait();
-    }
+    tmem_st32(trow + C_W + c0, w0);
+    tmem_st_wait();
 #pragma unroll 1
     for (int n = 0; n < end; ++n) {
       const int m = n - begin;                    // of the steps with scores
@@ -477,7 +494,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         bulk_s2g(dst, pk, kPanelB);
         bulk_s2g(dst + kPartSum, pv, kPanelB);
         bulk_commit();
-        bulk_wait0();
+        bulk_wait_read0();
       }
       __syncwarp();
     } else if (krow < p.N) {
@@ -520,7 +537,7 @@ __global__ void __launch_bounds__(kB128Threads, 1)
 castle_bwd128_reverse_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc) {
   constexpr uint32_t ID_MM = make_idesc(128, 128, Elem<T>::fmt, true, true, false);
   const int K = blockIdx.y, steps = p.nblk - 1 - K;
-  B128_BEGIN(6 * kSq, 4, -1, 128)
+  B128_BEGIN(6 * kSq, 4, 128)
   uint64_t *bar_in = bars, *bar_g = bars + 2;   // two each
   const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * 32;
   const bool loader = warp == 4, storer = warp == 8;
@@ -589,7 +606,7 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
                      ID_MM = make_idesc(128, 128, FMT, true, true, false);
   const int I = p.nblk - 1 - blockIdx.y, i0 = I * kBlkB;   // the longest walks first
   const bool last = I == p.nblk - 1;                       // no G there yet
-  B128_BEGIN(7 * kSq, 10, -1, 512)
+  B128_BEGIN(7 * kSq, 10, 512)
   uint8_t *sVu = smem, *sT = smem + kSq, *sA = smem + 2 * kSq, *sS = smem + 3 * kSq, *sG = smem + 4 * kSq, *sQu = smem + 5 * kSq,
           *sZ = smem + 6 * kSq;
   uint64_t *bar_res = bars, *bar_in = bars + 1, *bar_qu = bars + 2, *bar_da = bars + 3, *bar_v = bars + 4, *bar_k = bars + 5, *bar_t = bars + 6,
@@ -761,7 +778,7 @@ __global__ void __launch_bounds__(128)
 castle_bwd128_dqu_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_ku) {
   constexpr uint32_t ID_KM = make_idesc(128, 128, Elem<T>::fmt, false, true, false);
   const int K = blockIdx.y, k0 = K * kBlkB, steps = p.nblk - K;
-  B128_BEGIN(6 * kSq, 7, -1, 128)
+  B128_BEGIN(6 * kSq, 7, 128)
   uint64_t *bar_in = bars, *bar_done = bars + 3, *bar_end = bars + 6;   // three, three, one
   if (warp == 0 && elect_one()) {
     auto load = [&](int n) {
