@@ -556,8 +556,8 @@ static int launch_bwd(const BwdParams& p, const CUtensorMap* maps, cudaStream_t 
     cudaError_t e = cudaFuncSetAttribute(castle_bwd_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
   }
-  static const int regs_rc = check_launch_regs(castle_bwd_kernel<T, D>, "castle_bwd");
-  if (regs_rc) return regs_rc;
+  static std::atomic<bool> regs_known{false};
+  if (const int rc = check_launch_regs(castle_bwd_kernel<T, D>, regs_known)) return rc;
   const int64_t rows = (int64_t)p.B * p.H * p.N;
   constexpr int RPB = 256 / (D / 8);
   castle_bwd_delta_kernel<T, D, 3><<<(unsigned)((rows + RPB - 1) / RPB), 256, 0, st>>>(p);

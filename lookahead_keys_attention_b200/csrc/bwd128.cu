@@ -831,16 +831,17 @@ static int launch_bwd128_t(const BwdParams& p, const CUtensorMap* in, cudaStream
   constexpr int D = 128;
   const void* kernels[5] = {(const void*)castle_bwd128_kv_kernel<T, false>, (const void*)castle_bwd128_reverse_kernel<T>,
                             (const void*)castle_bwd128_la_kernel<T>, (const void*)castle_bwd128_dqu_kernel<T>, (const void*)castle_bwd128_kv_kernel<T, true>};
-  static const int regs_rc[2] = {check_launch_regs(castle_bwd128_kv_kernel<T, false>, "castle_bwd"), check_launch_regs(castle_bwd128_kv_kernel<T, true>, "castle_bwd")};
-  for (int rc : regs_rc)
-    if (rc) return rc;
+  static std::atomic<bool> regs_known[2] = {{false}, {false}};
+  int rc = check_launch_regs(castle_bwd128_kv_kernel<T, false>, regs_known[0]);
+  if (!rc) rc = check_launch_regs(castle_bwd128_kv_kernel<T, true>, regs_known[1]);
+  if (rc) return rc;
   const size_t smem[5] = {kB128Smem, 6 * kSq + 256, kB128Smem, 6 * kSq + 256, kB128Smem};
   for (int i = 0; i < 5; ++i) {
     cudaError_t e = cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[i]);
     if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
   }
   CUtensorMap acc;
-  int rc = make_tmap_f32_rows(&acc, p.acc_dqc, p.B * p.H, p.N, D, "gradient workspace");
+  rc = make_tmap_f32_rows(&acc, p.acc_dqc, p.B * p.H, p.N, D, "gradient workspace");
   if (rc) return rc;
   const int64_t rows = (int64_t)p.B * p.H * p.N;
   constexpr int RPB = 256 / (D / 8);

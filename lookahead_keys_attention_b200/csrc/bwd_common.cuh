@@ -1,6 +1,7 @@
 // Shared by the backward kernels (dim_head 64 in bwd.cu, dim_head 128 in bwd128.cu): launch
 // parameters, the delta pre-pass and the kernel that turns fp32 accumulators into gradients.
 #pragma once
+#include <atomic>
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -51,13 +52,16 @@ __device__ __forceinline__ float ev_arrive_read(int id, int threads, const float
   asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(zero) : "r"(smem_u32(zero_s)) : "memory");
   return zero;
 }
-// 0 if `kernel` was compiled to start with the registers that the sharing above counts on
+// 0 if `kernel` was compiled to start with the registers that the sharing above counts on; asked once per kernel (`known`)
 template <typename Kernel>
-int check_launch_regs(Kernel kernel, const char* name) {
+int check_launch_regs(Kernel kernel, std::atomic<bool>& known) {
+  if (known.load(std::memory_order_relaxed)) return 0;
   cudaFuncAttributes a;
   const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
-  if (e != cudaSuccess) return cuda_fail(e, name);
-  return a.numRegs == kSplitLaunchRegs ? 0 : reject("%s: compiled with %d registers a thread instead of %d", name, a.numRegs, kSplitLaunchRegs);
+  if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
+  if (a.numRegs != kSplitLaunchRegs) return reject("castle_bwd: compiled with %d registers a thread instead of %d", a.numRegs, kSplitLaunchRegs);
+  known.store(true, std::memory_order_relaxed);
+  return 0;
 }
 
 // delta[b,h,i] = sum_d out * dout  (lookahead_keys_attention_triton.py:175-214 in the reference); clears the first NACC of the
