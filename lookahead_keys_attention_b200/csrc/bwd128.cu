@@ -853,10 +853,10 @@ static int launch_bwd128_t(const BwdParams& p, const CUtensorMap* in, cudaStream
     q.bh0 = bh0;
     q.ntiles = (int64_t)p.nblk * (p.nblk + 1) / 2;
     const int pairs = BH - bh0 < chunk ? BH - bh0 : chunk;
-    // Key blocks whose walks are cut: the longer half, where the steps per SM are less than half the longest walk.  us of the four
-    // kernels, uncut / cut: 4 pairs x 4096 positions 441 / 377 (0.45), 8 x 2048 237 / 220 (0.46), 2 x 900 122 / 112 (0.05),
-    // 12 x 1500 187 / 187 (0.53); above that the repeated state costs more than the balance gains: 16 x 1333 182 / 197 (0.65), 8 x
-    // 3000 355 / 370 (0.68).
+    // Key blocks whose walks are cut: the longer half, where the steps per SM are less than half the longest walk.  us of forward and
+    // backward, uncut / cut: 4 pairs x 4096 positions 535 / 480 (0.45), 8 x 2048 301 / 287 (0.46), 10 x 1024 163 / 157 (0.30),
+    // 12 x 1500 247 / 248 (0.53); above that the repeated state costs more than the balance gains: 16 x 1333 248 / 263 (0.65), 8 x
+    // 3000 469 / 480 (0.68).
     const float load = (float)pairs * (float)(p.nblk + 1) * (0.5f / 148.f);
     q.kv_split = p.nblk >= kKvSplitMin && load < 0.5f ? std::max(0, std::min(p.nblk + 1 - kKvSplitMin, p.N / (2 * kBlkB))) : 0;
     const dim3 grid(pairs, p.nblk), kv_grid(pairs, q.kv_split ? 2 * p.nblk : p.nblk);
