@@ -52,6 +52,12 @@ int castle_selftest_mma_rate(int32_t form, int32_t n, int32_t reps, long long* c
  * polls[0] receives the number of polls the first wait made, polls[1] the second (device int32[2]). */
 int castle_selftest_wait_timeout(int32_t poll_limit, int32_t* polls, int32_t* status, void* stream);
 
+/* The same for warps with one job each (no counterpart in the reference): four warps arrive on two events a round, `rounds`
+ * (1 .. 1024) times, one warp takes them and answers the first, after it has waited for a tile.  form 0: neither the tile nor an answer
+ * ever comes; 1: both come; 2: the tile does not come, the answers do.  Waits give up after `poll_limit` polls, every event is taken
+ * all the same and the kernel ends.  result[0] receives whether the tile came, result[1] the events taken (device int32[2]). */
+int castle_selftest_event_timeout(int32_t poll_limit, int32_t rounds, int32_t form, int32_t* result, int32_t* status, void* stream);
+
 /* y[i] = 2^x[i] for `count` (even, at most 2^26) values as the score passes at dim_head 64 compute a part of their
  * exponentials, without the special-function unit (no counterpart in the reference). */
 int castle_selftest_exp2(const float* x, float* y, int32_t count, void* stream);

@@ -191,6 +191,7 @@ _SIGNATURES = {
     "castle_selftest_mma_rate": (ctypes.c_int, [_i32, _i32, _i32, _vp, _vp, _vp]),
     "castle_selftest_mma": (ctypes.c_int, [_i32, _vp, _vp, _vp, _vp, _vp]),
     "castle_selftest_wait_timeout": (ctypes.c_int, [_i32, _vp, _vp, _vp]),
+    "castle_selftest_event_timeout": (ctypes.c_int, [_i32, _i32, _i32, _vp, _vp, _vp]),
     "castle_selftest_exp2": (ctypes.c_int, [_vp, _vp, _i32, _vp]),
 }
 

@@ -45,9 +45,12 @@ namespace castle {
 #define tma_reduce_add_3d(...) do { } while (0)
 #endif
 
-// named barriers (ev_arrive)
-enum BwdEvent { kEvRead = 1, kEvStored = 2, kEvStoredT = 3, kEvStoredZ = 4, kEvDqc = 5, kEvDku = 6, kEvDvu = 7 };
-constexpr int kWorkers = 8, kEpilogue = 9;   // and those of the passes among themselves: all 512, and 9 to 11 a chunk group each
+// The events of a step that the issuing warp takes (ev_arrive), in their order; they take turns on four named barriers.
+enum BwdEvent { kEvReadZ, kEvGate, kEvT, kEvCopyW, kEvReadSu, kEvReadSc, kEvP, kEvReadDp, kEvDs, kEvReadDa, kEvDz, kEvReadDt, kEvDt, kEvReadX, kEvCount };
+__device__ constexpr int bwd_event(int k) { return 1 + k % 4; }
+// Those that the moving warp takes, and after each other step by step.
+enum BwdStaged { kEvDqc = 5, kEvDku = 6, kEvDvu = 7 };   // and 8 to 10 in odd steps
+constexpr int kWorkers = 11, kEpilogue = 12;             // of the passes among themselves: all 512, and 12 to 14 a chunk group each
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kSplitThreads, 1)
@@ -87,6 +90,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   // Each of these completes once per step.
   __shared__ uint64_t bar_res, bar_load, bar_vd, bar_ku, bar_kn;   // tiles
   __shared__ uint64_t bar_z, bar_t, bar_w, bar_su, bar_sc, bar_dp, bar_dv, bar_da, bar_dt, bar_g, bar_x, bar_l;   // products
+  __shared__ uint64_t bar_end;                                     // once: no product is in flight
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   __shared__ float zero_s;
@@ -100,10 +104,10 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   // being written by the kernel before this one).
   if (warp == 17 && elect_one()) {
     if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
-    uint64_t* const bars[17] = {&bar_res, &bar_load, &bar_vd, &bar_ku, &bar_kn, &bar_z, &bar_t, &bar_w,
-                                &bar_su, &bar_sc, &bar_dp, &bar_dv, &bar_da, &bar_dt, &bar_g, &bar_x, &bar_l};
+    uint64_t* const bars[18] = {&bar_res, &bar_load, &bar_vd, &bar_ku, &bar_kn, &bar_z, &bar_t, &bar_w, &bar_su,
+                                &bar_sc, &bar_dp, &bar_dv, &bar_da, &bar_dt, &bar_g, &bar_x, &bar_l, &bar_end};
 #pragma unroll
-    for (int i = 0; i < 17; ++i) mbar_init(bars[i], bars[i] == &bar_t || bars[i] == &bar_w ? 2 : 1);   // these two: the product, and the slot written next is free
+    for (int i = 0; i < 18; ++i) mbar_init(bars[i], bars[i] == &bar_t || bars[i] == &bar_w ? 2 : 1);   // these two: the product, and the slot written next is free
     mbar_fence_init();
     abort_flag = 0;
     zero_s = 0.f;
@@ -150,9 +154,9 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         asm volatile("" : "+r"(base));
         return base + (uint32_t)(tile - smem);
       };
-      auto next = [&](int id) {
+      auto next = [&](int k) {
         __syncwarp();
-        ev_wait(id, kSplitWorkers);
+        ev_wait(bwd_event(k), kSplitWorkers);
         tc_fence_after();
       };
       auto issue_z = [&](uint32_t ph) {
@@ -169,52 +173,52 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       for (int n = 0; n < walk; ++n) {
         const uint32_t ph = n & 1;
         const bool first = n == 0, diag = n == walk - 1;
-        next(kEvRead);     // Z
+        next(kEvReadZ);
         if (elect_one()) {
           mbar_wait(&bar_load, ph, abortp);
           tc_fence_after();
           gemm_kk_t<1>(tmem + C_S, at(sQc), at(sVu), ID_SQ_KK, false);          // T = Qc[I] Vu[I]^T, while the gate is formed
           mma_commit(&bar_t);
         }
-        next(kEvStored);   // A
+        next(kEvGate);
         if (elect_one()) {
           if (!diag) gemm_km_t<8>(tmem + C_W, at(sA), at(sVu), ID_D_KM_NEG, true);   // W_K -= A Vu[I], while T is masked; zero at the diagonal block, where nothing reads it
           mma_commit(&bar_w);
         }
-        next(kEvStoredT);  // masked T
+        next(kEvT);        // masked
         if (elect_one()) gemm_kk_t<2>(tmem + C_S, at(sT), at(sA), ID_SQ_KK, false);    // Su/scale = T A^T + Qc[I] Wb^T, while W is copied
-        next(kEvStored);   // copy of W
+        next(kEvCopyW);
         if (elect_one()) {
           if (!diag) gemm_kk_t<1>(tmem + C_S, at(sQc), at(sWb), ID_SQ_KK, true);
           mma_commit(&bar_su);
         }
-        next(kEvRead);     // Su
+        next(kEvReadSu);
         if (elect_one()) {
           gemm_kk_t<1>(tmem + C_S, at(sQc), at(sKc), ID_SQ_KK, false);          // Sc/scale = Qc[I] Kc[K]^T, while silu' is formed
           mma_commit(&bar_sc);
         }
-        next(kEvRead);     // Sc
+        next(kEvReadSc);
         if (elect_one()) {
           mbar_wait(&bar_vd, ph, abortp);
           tc_fence_after();
           gemm_kk_t<1>(tmem + C_S, at(sdO), at(sVc), ID_SQ_KK, false);          // dP = dO[I] Vc[K]^T, while P is formed
           mma_commit(&bar_dp);
         }
-        next(kEvStored);   // P
+        next(kEvP);
         if (elect_one()) {
           gemm_mm_t<8>(tmem + C_DVC, at(sKP), at(sdO), ID_D_MM, !first);        // dvc += P^T dO[I], while dS is formed
           mma_commit(&bar_dv);
         }
-        next(kEvRead);     // dP
+        next(kEvReadDp);
         if (!first && elect_one()) gemm_kk_t<1>(tmem + C_S, at(sGb), at(sVu), ID_SQ_KK, false);   // dA/scale = Gb Vu[I]^T + dSu^T T
-        next(kEvStored);   // dS, dSu
+        next(kEvDs);       // and dSu
         if (elect_one()) {
           gemm_mm_t<8>(tmem + C_S, at(sKP), at(sT), ID_SQ_MM, !first);
           mma_commit(&bar_da);
           gemm_mm_t<8>(tmem + C_DKC, at(sVD), at(sQc), ID_D_MM, !first);        // dkc += dS^T Qc[I]
           gemm_km_t<8>(tmem + C_X, at(sVD), at(sKc), ID_D_KM, false);           // X = dS Kc[K] + dSu Wb + dT Vu[I]
         }
-        next(kEvRead);     // dA
+        next(kEvReadDa);
         if (elect_one()) {
           gemm_km_t<8>(tmem + C_S, at(sKP), at(sA), ID_SQ_KM, false);           // dT = dSu A, while dZ is formed
           mma_commit(&bar_dt);
@@ -224,10 +228,10 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
           }
           mma_commit(&bar_g);
         }
-        next(kEvStoredZ);  // dZ
-        next(kEvRead);     // dT
+        next(kEvDz);
+        next(kEvReadDt);
         if (elect_one()) gemm_mm_t<8>(tmem + C_X3, at(sT), at(sQu), ID_D_MM, false);   // X3 = dZ^T Qu[K]
-        next(kEvStored);   // masked dT
+        next(kEvDt);       // masked
         if (elect_one()) {
           gemm_mm_t<8>(tmem + C_X2, at(sVD), at(sQc), ID_D_MM, false);          // X2 = dT^T Qc[I] + A^T Gb
           gemm_km_t<8>(tmem + C_X, at(sVD), at(sVu), ID_D_KM, true);
@@ -238,49 +242,56 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
           if (!first) gemm_mm_t<8>(tmem + C_X2, at(sA), at(sGb), ID_D_MM, true);
           mma_commit(&bar_l);
         }
-        next(kEvRead);     // X2, X3
+        next(kEvReadX);
         if (!diag && elect_one()) issue_z(ph ^ 1);
+      }
+      __syncwarp();
+      if (elect_one()) {
+        mma_commit(&bar_end);
+        mbar_drain(&bar_end, 0);
       }
       __syncwarp();
     } else if (warp == 17) {
       // ---- the tiles.  The TMA unit works its queue off in order and a reduce takes thousands of cycles, so loads go ahead of them.
+      int n = 0;
+      bool half = false;   // a wait that did not end well ended the walk, the second of its step
 #pragma unroll 1
-      for (int n = 0; n < walk; ++n) {
+      for (; n < walk; ++n) {
         const uint32_t ph = n & 1;
         const bool more = n + 1 < walk;
-        const int i0 = (p.nblk - 1 - n) * kBlkB, in0 = i0 - kBlkB;
-        __syncwarp();
+        const int i0 = (p.nblk - 1 - n) * kBlkB, in0 = i0 - kBlkB, odd = 3 * (n & 1);
+        if (mbar_wait_failed(&bar_g, ph, abortp)) break;                  // copy of W and dSu have been read
         if (elect_one()) {
-          mbar_wait(&bar_g, ph, abortp);         // copy of W and dSu have been read
           mbar_expect_tx(&bar_ku, OPB);
           tma_load_4d(sWb, &m_ku, &bar_ku, 0, i0, h, b);
           if (more) {
             mbar_expect_tx(&bar_kn, OPB);
             tma_load_4d(sKP, &m_ku, &bar_kn, 0, in0, h, b);
           }
-          mbar_wait(&bar_x, ph, abortp);         // Qc[I], Vu[I], Ku[I] as well
-          if (more) {
-            mbar_expect_tx(&bar_load, 2 * OPB);
-            tma_load_4d(sQc, &m_qc, &bar_load, 0, in0, h, b);
-            tma_load_4d(sVu, &m_vu, &bar_load, 0, in0, h, b);
-          }
         }
         __syncwarp();
-        ev_wait(kEvDku, 128);                    // its slot is needed first
+        if (mbar_wait_failed(&bar_x, ph, abortp)) { half = true; break; } // Qc[I], Vu[I], Ku[I] as well
+        if (more && elect_one()) {
+          mbar_expect_tx(&bar_load, 2 * OPB);
+          tma_load_4d(sQc, &m_qc, &bar_load, 0, in0, h, b);
+          tma_load_4d(sVu, &m_vu, &bar_load, 0, in0, h, b);
+        }
+        __syncwarp();
+        ev_wait(kEvDku + odd, 128);              // its slot is needed first
         if (elect_one()) {
           tma_reduce_add_3d(&m_acc_dku, sT, 0, i0, bh);
           tma_reduce_add_3d(&m_acc_dku, sT + kPanelB, 32, i0, bh);
           bulk_commit();
         }
         __syncwarp();
-        ev_wait(kEvDqc, 128);
+        ev_wait(kEvDqc + odd, 128);
         if (elect_one()) {
           tma_reduce_add_3d(&m_acc_dqc, sWb, 0, i0, bh);
           tma_reduce_add_3d(&m_acc_dqc, sKP + kPanelB, 32, i0, bh);
           bulk_commit();
         }
         __syncwarp();
-        ev_wait(kEvDvu, 256);
+        ev_wait(kEvDvu + odd, 256);
         if (elect_one()) {
           tma_reduce_add_3d(&m_acc_dvu, sVD, 0, i0, bh);
           tma_reduce_add_3d(&m_acc_dvu, sVD + kPanelB, 32, i0, bh);
@@ -296,10 +307,26 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
             tma_load_4d(sdO, &m_do, &bar_vd, 0, in0, h, b);
           }
         }
+        __syncwarp();
+      }
+      if (elect_one()) {
+        if (*abortp) {   // tiles that were asked for and that nobody may have waited for must not land after the CTA has left
+          const int last = n < walk ? n : walk - 1;
+          mbar_drain(&bar_res, 0);
+          mbar_drain(&bar_load, last & 1);
+          mbar_drain(&bar_vd, last & 1);
+          mbar_drain(&bar_ku, (n == walk || half ? last : last - 1) & 1);
+          mbar_drain(&bar_kn, (half && last + 1 < walk ? last + 1 : last) & 1);
+        }
+        bulk_wait_read0();   // the sums themselves are complete when the kernel is
       }
       __syncwarp();
-      if (elect_one()) bulk_wait_read0();   // the sums themselves are complete when the kernel is
-      __syncwarp();
+      for (; n < walk; ++n) {   // nothing is asked for any more, for a barrier's last phase may still be open
+        const int odd = 3 * (n & 1);
+        ev_wait(kEvDku + odd, 128);
+        ev_wait(kEvDqc + odd, 128);
+        ev_wait(kEvDvu + odd, 256);
+      }
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSplitWorkerRegs));
@@ -308,16 +335,21 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     const int c0 = cc * 32;
     const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
     const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
+    bool failed;
     auto wait = [&](uint64_t* bar, uint32_t ph) {
-      mbar_wait_lazy_abort(bar, ph, abortp);   // (one polling lane a warp: 1970 -> 2126 us at B=4 N=4096 H=16)
+      failed = mbar_wait_failed(bar, ph, abortp);   // (one polling lane a warp: 1970 -> 2126 us at B=4 N=4096 H=16)
       tc_fence_after();
     };
-    auto read = [&]() { return ev_arrive_read(kEvRead, kSplitWorkers, &zero_s); };
-    auto stored = [&](int id) {
+    // a wait that did not end well ends the walk; `arrived`: the events of this step that the warp has arrived on before
+#define BWD_CHECK(ARRIVED) if (failed) { arrived = ARRIVED; goto stopped; }
+    auto read = [&](int k) { return ev_arrive_read(bwd_event(k), kSplitWorkers, &zero_s); };
+    auto stored = [&](int k) {
       fence_async_smem();
       tc_fence_before();
-      ev_arrive(id, kSplitWorkers);
+      ev_arrive(bwd_event(k), kSplitWorkers);
     };
+    int n = 0;
+    uint32_t arrived = 0;
     // W_K starts as the forward's final state, brought in whole lines (rows of 64 floats over the threads, through the gate's slot):
     // a row per lane, here and where the gradients are stored, took 2 us of a key block each; 1036 pairs of one block 150.5 ->
     // 142.3 us, B=16 H=8 N=1024 402 -> 392 us
@@ -340,7 +372,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
     asm volatile("bar.sync %0, %1;" ::"n"(kWorkers), "n"(kSplitWorkers) : "memory");
 
 #pragma unroll 1
-    for (int n = 0; n < walk; ++n) {
+    for (; n < walk; ++n) {
       const uint32_t ph = n & 1;
       const int I = p.nblk - 1 - n, irow = I * kBlkB + row;
       const bool diag = I == K, rvalid = irow < p.N;
@@ -351,7 +383,8 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         float v[32];
         tmem_ld32(trow + C_S + c0, v);
         tmem_ld_wait();
-        const float hs = half_scale + read();
+        BWD_CHECK(kEvReadZ)
+        const float hs = half_scale + read(kEvReadZ);
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), hs);
@@ -363,17 +396,19 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         }
         store_row32<T>(sA, kPanelB, row, c0, v);
       }
-      stored(kEvStored);
+      stored(kEvGate);
       BPHASE_MARK(2);
       wait(&bar_t, ph);
       BPHASE_MARK(3);
       {  // masked T (rows i, columns j <= i), unscaled
         float v[32];
         tmem_ld32_lower(trow + C_S + c0, row, c0, v);
+        BWD_CHECK(kEvT)
         store_row32<T>(sT, kPanelB, row, c0, v);
       }
-      stored(kEvStoredT);
+      stored(kEvT);
       wait(&bar_w, ph);
+      BWD_CHECK(kEvCopyW)
       BPHASE_MARK(4);
       if (c0 < D) {  // 16-bit copy of the peeled state
         float v[32];
@@ -381,7 +416,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         tmem_ld_wait();
         store_row32<T>(sWb, kPanelB, row, c0, v);
       }
-      stored(kEvStored);
+      stored(kEvCopyW);
       BPHASE_MARK(5);
       // loaded here, not at the top of the step, where the wait for Z is short
       const float lse_i = rvalid ? p.lse[(int64_t)bh * p.N + irow] : 0.f, delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
@@ -393,7 +428,8 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         float v[32], w[32];
         tmem_ld32(trow + C_S + c0, v);
         tmem_ld_wait();
-        const float hs = half_scale + read();
+        BWD_CHECK(kEvReadSu)
+        const float hs = half_scale + read(kEvReadSu);
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float2 u = make_float2(v[j], v[j + 1]);
@@ -410,7 +446,8 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         // P = exp(S - lse) (rows i, columns k); into slot 4 over Ku
         tmem_ld32(trow + C_S + c0, w);
         tmem_ld_wait();
-        const float s2 = sl2 + read();
+        BWD_CHECK(kEvReadSc)
+        const float s2 = sl2 + read(kEvReadSc);
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(s2), splat(-lse_i * kLog2e));
@@ -429,7 +466,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         for (int j = 0; j < 32; j += 2) ppk[j / 2] = Elem<T>::pack2(v[j], v[j + 1]);
         store_row32<T>(sKP, kPanelB, row, c0, v);
       }
-      stored(kEvStored);
+      stored(kEvP);
       BPHASE_MARK(9);
       wait(&bar_dp, ph);
       BPHASE_MARK(10);
@@ -437,7 +474,8 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         float v[32], w[32];
         tmem_ld32(trow + C_S + c0, v);
         tmem_ld_wait();
-        const float dl = delta_i + read();
+        BWD_CHECK(kEvReadDp)
+        const float dl = delta_i + read(kEvReadDp);
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float2 ds = mul2(Elem<T>::unpack2(ppk[j / 2]), add2(make_float2(v[j], v[j + 1]), splat(-dl)));
@@ -445,11 +483,12 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
           v[j] = ds.x; v[j + 1] = ds.y;
           w[j] = -du.x; w[j + 1] = -du.y;
         }
-        mbar_wait(&bar_dv, ph, abortp);   // dO and P have been read
+        wait(&bar_dv, ph);   // dO and P have been read
+        BWD_CHECK(kEvDs)
         store_row32<T>(sVD, kPanelB, row, c0, v);
         store_row32<T>(sKP, kPanelB, row, c0, w);
       }
-      stored(kEvStored);
+      stored(kEvDs);
       BPHASE_MARK(11);
       wait(&bar_da, ph);
       BPHASE_MARK(12);
@@ -457,7 +496,8 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         float v[32], a[32];
         tmem_ld32(trow + C_S + c0, v);
         tmem_ld_wait();
-        const float sc = p.scale + read();
+        BWD_CHECK(kEvReadDa)
+        const float sc = p.scale + read(kEvReadDa);
         load_row32<T>(sA, kPanelB, row, c0, a);
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
@@ -467,36 +507,39 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         }
         store_row32<T>(sT, kPanelB, row, c0, v);
       }
-      stored(kEvStoredZ);   // an event of its own: the wait below does not cover it
+      stored(kEvDz);   // an event of its own: the wait below does not cover it
       BPHASE_MARK(13);
       wait(&bar_dt, ph);
       BPHASE_MARK(14);
       {  // masked dT (rows i, columns j <= i) -> slot 3 (over dS)
         float v[32];
         tmem_ld32_lower(trow + C_S + c0, row, c0, v);
-        read();
+        BWD_CHECK(kEvReadDt)
+        read(kEvReadDt);
         store_row32<T>(sVD, kPanelB, row, c0, v);
       }
-      stored(kEvStored);
+      stored(kEvDt);
       BPHASE_MARK(15);
       // The query block's gradients are staged as fp32 panels in operand slots that are dead by then and handed to TMA reduces
       // (whole lines at L2 instead of scattered atomics): chunk group 1 takes dqc (into the copy of W's slot and the spare half of
       // slot 4), group 2 dku (into slot 2), groups 0 and 3 a panel each of dvu (into slot 3).  Groups 1 and 2 also make the
       // 16-bit copy of G, including block I, for the next (lower) block; the next step's events order it.
-      const int part = cc >> 1;
+      const int part = cc >> 1, staged = (cc == 1 ? kEvDqc : cc == 2 ? kEvDku : kEvDvu) + 3 * (n & 1);
       if (cc == 1 || cc == 2) {
         wait(&bar_x, ph);
+        BWD_CHECK(kEvReadX)
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           float v[32];
           tmem_ld32(trow + (cc == 1 ? C_X : C_X3) + c * 32, v);
           tmem_ld_wait();
-          if (c == 1) read();
+          if (c == 1) read(kEvReadX);
           store_row32_f32(cc == 2 ? sT + c * kPanelB : c == 0 ? sWb : sKP + kPanelB, row, v);
         }
         fence_async_smem();
-        ev_arrive(cc == 1 ? kEvDqc : kEvDku, 128);
+        ev_arrive(staged, 128);
         wait(&bar_l, ph);
+        BWD_CHECK(kEvCount + 1)
         if (!diag) {
           float v[32];
           tmem_ld32(trow + C_G + part * 32, v);
@@ -509,12 +552,20 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
         float v[32];
         tmem_ld32(trow + C_X2 + part * 32, v);
         tmem_ld_wait();
-        read();
+        BWD_CHECK(kEvReadX)
+        read(kEvReadX);
         store_row32_f32(sVD + part * kPanelB, row, v);
         fence_async_smem();
-        ev_arrive(kEvDvu, 256);
+        ev_arrive(staged, 256);
       }
       BPHASE_MARK(17);
+    }
+#undef BWD_CHECK
+  stopped:
+    for (; n < walk; ++n, arrived = 0) {   // what is left of the events
+#pragma unroll 1
+      for (; arrived < kEvCount; ++arrived) ev_wait(bwd_event((int)arrived), kSplitWorkers);
+      if (arrived == kEvCount) ev_wait((cc == 1 ? kEvDqc : cc == 2 ? kEvDku : kEvDvu) + 3 * (n & 1), cc == 1 || cc == 2 ? 128 : 256);
     }
 
     // ---- key-block gradients: dkc (x scale), dvc, dqu (x scale); one chunk group each, through the gate's slot and the copy of

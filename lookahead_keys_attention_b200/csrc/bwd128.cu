@@ -88,11 +88,6 @@ __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K)
 #define B128_MARK(base, n, i) do { } while (0)
 #endif
 
-#define B128_SYNC()    \
-  fence_async_smem();   \
-  tc_fence_before();    \
-  __syncthreads();
-
 // ------------------------------------------------------------------------------------------------ scores, dkc, dvc, dqc
 // One chain per step, products and passes in turn:
 //   Z | gate A (T under it);  W -= A Vu | T masked, Wb (T A^T under it);  Su | silu' (Sc under it) | P (dP under it);  dvc | dS, dSu;
@@ -119,8 +114,14 @@ __device__ __forceinline__ uint8_t* kv_part(const BwdParams& p, int bh, int K, i
 }
 
 enum KvBar { kKvRes, kKvZin /* Qu, Ku */, kKvIn /* Qc, Vu */, kKvDo /* Vc, dO */, kKvZ, kKvT, kKvW, kKvSu, kKvSc, kKvDp, kKvDv, kKvX0, kKvX, kKvK,
-             kKvCopied /* dSu */, kKvBars };
-enum KvEvent { kKvRead = 1, kKvStored = 2, kKvStoredT = 3, kKvStaged = 4, kKvGroups = 5 };
+             kKvCopied /* dSu */, kKvEnd /* no product is in flight */, kKvBars };
+static_assert(7 * kSq + kKvBars * 8 + 12 <= kB128Smem, "barriers, the address of tensor memory, the abort flag and a zero");
+// The events of a step with scores that the issuing warp takes (ev_arrive), in their order; they take turns on five named barriers.
+enum KvEvent { kKvReadZ, kKvGate, kKvMaskedT, kKvCopyW, kKvReadSu, kKvReadSc, kKvP, kKvDs, kKvReadX, kKvEvents };
+__device__ constexpr int kv_event(int k) { return 1 + k % 5; }
+__device__ constexpr int kv_gate_alone(int n) { return 6 + (n & 1); }   // that of a step without scores
+__device__ constexpr int kv_staged(int m) { return 8 + (m & 1); }       // that which the moving warp takes
+constexpr int kKvGroups = 10;                                           // the chunk groups among themselves: 10 to 13
 
 template <typename T, bool CUT>
 __global__ void __launch_bounds__(kSplitThreads, 1)
@@ -197,11 +198,12 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         asm volatile("" : "+r"(base));
         return base + off;
       };
-      auto next = [&](int id) {
+      auto next_on = [&](int id) {
         __syncwarp();
         ev_wait(id, kSplitWorkers);
         tc_fence_after();
       };
+      auto next = [&](int k) { next_on(kv_event(k)); };
       auto issue_z = [&](int n) {     // Z = Qu[K] Ku[I]^T
         mbar_wait(bars + kKvZin, n & 1, abortp);
         tc_fence_after();
@@ -215,7 +217,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         const uint32_t ph = n & 1, ph_m = m & 1, sK = slot_k(n), sV = slot_v(n);
         const bool diag = n == walk - 1, more = n + 1 < end;
         if (CUT && m < 0) {
-          next(kKvStored);
+          next_on(kv_gate_alone(n));
           if (elect_one()) {
             mbar_wait(bars + kKvIn, ph, abortp);
             tc_fence_after();
@@ -225,45 +227,45 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
           }
           continue;
         }
-        next(kKvRead);     // Z
+        next(kKvReadZ);
         if (elect_one()) {
           mbar_wait(bars + kKvIn, ph, abortp);
           tc_fence_after();
           gemm_kk_t<2>(tmem + C_S, at(S3), at(sV), ID_KK, false);        // T = Qc Vu^T, while the gate is formed
           mma_commit(bars + kKvT);
         }
-        next(kKvStored);   // A
+        next(kKvGate);
         if (elect_one()) {
           if (!diag) gemm_km_t<8>(tmem + C_W, at(sK), at(sV), ID_KM_NEG, true);   // W -= A Vu; at the diagonal block nothing reads it
           mma_commit(bars + kKvW);
         }
-        next(kKvStoredT);  // masked T
+        next(kKvMaskedT);
         if (elect_one()) gemm_kk_t<2>(tmem + C_S, at(sV), at(sK), ID_KK, false);  // Su/scale = T A^T + Qc Wb^T, while W is copied
-        next(kKvStored);   // copy of W
+        next(kKvCopyW);
         if (elect_one()) {
           if (!diag) gemm_kk_t<2>(tmem + C_S, at(S3), at(S0), ID_KK, true);
           mma_commit(bars + kKvSu);
         }
-        next(kKvRead);     // Su
+        next(kKvReadSu);
         if (elect_one()) {
           if (m == 0) mbar_wait(bars + kKvRes, 0, abortp);
           tc_fence_after();
           gemm_kk_t<2>(tmem + C_S, at(S3), at(S4), ID_KK, false);        // Sc/scale = Qc Kc^T, while silu' is formed
           mma_commit(bars + kKvSc);
         }
-        next(kKvRead);     // Sc
+        next(kKvReadSc);
         if (elect_one()) {
           mbar_wait(bars + kKvDo, ph_m, abortp);
           tc_fence_after();
           gemm_kk_t<2>(tmem + C_S, at(S6), at(S5), ID_KK, false);        // dP = dO Vc^T, while P is formed
           mma_commit(bars + kKvDp);
         }
-        next(kKvStored);   // P
+        next(kKvP);
         if (elect_one()) {
           gemm_mm_t<8>(tmem + C_DVC, at(sV), at(S6), ID_MM, m > 0);      // dvc += P^T dO, while dS is formed
           mma_commit(bars + kKvDv);
         }
-        next(kKvStored);   // dS, dSu
+        next(kKvDs);       // and dSu
         if (elect_one()) {
           if (!diag) gemm_km_t<8>(tmem + C_S, at(S6), at(S0), ID_KM, false);   // dqc = dSu Wb + dS Kc
           mma_commit(bars + kKvX0);
@@ -272,32 +274,38 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
           gemm_mm_t<8>(tmem + C_DKC, at(sK), at(S3), ID_MM, m > 0);      // dkc += dS^T Qc
           mma_commit(bars + kKvK);
         }
-        next(kKvRead);     // dqc
+        next(kKvReadX);    // dqc
         if (more && elect_one()) issue_z(n + 1);
+      }
+      __syncwarp();
+      if (elect_one()) {
+        mma_commit(bars + kKvEnd);
+        mbar_drain(bars + kKvEnd, 0);
       }
       __syncwarp();
     } else if (warp == kSplitWorkers / 32 + 1) {
       // ---- the tiles
+      auto failed = [&](int bar, uint32_t parity) { return mbar_wait_failed(bars + bar, parity, abortp); };
+      int n = 0, done = 0;   // a wait that did not end well ended the walk, after so many of its step
 #pragma unroll 1
-      for (int n = 0; n < end; ++n) {
+      for (; n < end; ++n, done = 0) {
         const int m = n - begin, i0 = (p.nblk - 1 - n) * kBlkB, in0 = i0 - kBlkB;
         const uint32_t ph = n & 1, ph_m = m & 1;
         const bool more = n + 1 < end;
         uint8_t *const tile = step_tiles(p, p.nblk - 1 - n, K), *const sK = smem + slot_k(n), *const sV = smem + slot_v(n);
-        __syncwarp();
-        if (CUT && m < 0) {   // the next step's tiles land over both once they are consumed, Qu stays
+        if (failed(kKvW, ph)) break;   // the gate is there
+        if (CUT && m < 0) {         // the next step's tiles land over both, which are consumed, Qu stays
           if (elect_one()) {
-            mbar_wait(bars + kKvW, ph, abortp);
             mbar_expect_tx(bars + kKvZin, kSq);
             load_op(sV, m_ku, bars + kKvZin, in0, h, b);
             mbar_expect_tx(bars + kKvIn, m == -1 ? 2 * kSq : kSq);
             if (m == -1) load_op(smem + S3, m_qc, bars + kKvIn, in0, h, b);
             load_op(sK, m_vu, bars + kKvIn, in0, h, b);
           }
+          __syncwarp();
           continue;
         }
         if (elect_one()) {
-          mbar_wait(bars + kKvW, ph, abortp);       // the gate is there
           bulk_s2g(tile + kTileA, sK, kSq);
           bulk_commit();
           if (m > 0) {
@@ -308,17 +316,26 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
           }
           bulk_wait_read0();
           mbar_arrive(bars + kKvDp);                // dS may go over the gate
-          mbar_wait(bars + kKvDv, ph_m, abortp);
-          if (more) {
-            mbar_expect_tx(bars + kKvZin, 2 * kSq);
-            mbar_expect_tx(bars + kKvIn, 2 * kSq);
-            load_op(sV, m_ku, bars + kKvZin, in0, h, b);   // over P
-          }
-          mbar_wait(bars + kKvX0, ph_m, abortp);
+        }
+        __syncwarp();
+        done = 1;
+        if (failed(kKvDv, ph_m)) break;
+        if (more && elect_one()) {
+          mbar_expect_tx(bars + kKvZin, 2 * kSq);
+          mbar_expect_tx(bars + kKvIn, 2 * kSq);
+          load_op(sV, m_ku, bars + kKvZin, in0, h, b);   // over P
+        }
+        __syncwarp();
+        done = 2;
+        if (failed(kKvX0, ph_m)) break;
+        if (elect_one()) {
           if (more) load_op(smem + S0, m_qu, bars + kKvZin, k0, h, b);
           bulk_s2g(tile + kTileDsu, smem + S6, kSq);       // behind what the next product waits for
           bulk_commit();
-          mbar_wait(bars + kKvK, ph_m, abortp);
+        }
+        __syncwarp();
+        if (failed(kKvK, ph_m)) break;
+        if (elect_one()) {
           if (more) {                               // before the reduces, which loads would queue behind
             load_op(smem + S3, m_qc, bars + kKvIn, in0, h, b);
             load_op(sK, m_vu, bars + kKvIn, in0, h, b);
@@ -327,35 +344,53 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
           mbar_arrive(bars + kKvCopied);            // dqc may be staged over dSu
         }
         __syncwarp();
-        ev_wait(kKvStaged, kSplitWorkers);
+        ev_wait(kv_staged(m), kSplitWorkers);
         if (elect_one()) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) tma_reduce_add_3d(&m_acc_dqc, smem + S5 + c * kPanelB, c * 32, i0, bh);
           bulk_commit();
         }
+        __syncwarp();
+      }
+      if (elect_one()) {
+        if (*abortp) {   // tiles that were asked for and that nobody may have waited for must not land after the CTA has left
+          const int last = n < end ? n : end - 1, next = done == 2 && last + 1 < end ? last + 1 : last;
+          const int last_do = last - begin - (n < end && done == 0 ? 1 : 0);
+          mbar_drain(bars + kKvRes, 0);
+          mbar_drain(bars + kKvZin, next & 1);   // (these two run into their limit where they were asked for in part)
+          mbar_drain(bars + kKvIn, next & 1);
+          mbar_drain(bars + kKvDo, last_do > 0 ? last_do & 1 : 0);
+        }
+        bulk_wait_read0();   // the sums themselves are complete when the kernel is
       }
       __syncwarp();
-      if (elect_one()) bulk_wait_read0();   // the sums themselves are complete when the kernel is
-      __syncwarp();
+      for (; n < end; ++n)   // nothing is asked for any more, for a barrier's last phase may still be open
+        if (n >= begin) ev_wait(kv_staged(n - begin), kSplitWorkers);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSplitWorkerRegs));
     const int row = (warp & 3) * 32 + lane, cc = warp >> 2, c0 = cc * 32, krow = k0 + row;
     const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
+    bool failed;
     auto wait = [&](int bar, uint32_t ph) {
-      mbar_wait_lazy_abort(bars + bar, ph, abortp);   // B=2 H=8 N=1333: 95.2 -> 92.3 us (one polling lane a warp: 100.7); no difference at dim_head 64
+      failed = mbar_wait_failed(bars + bar, ph, abortp);   // the flag on every 64th poll: B=2 H=8 N=1333 95.2 -> 92.3 us (one polling lane a warp: 100.7)
       tc_fence_after();
     };
-    auto read = [&]() { return ev_arrive_read(kKvRead, kSplitWorkers, zero_s); };
-    auto stored = [&](int id) {
+    // a wait that did not end well ends the walk; `arrived`: the events of this step that the warp has arrived on before
+#define KV_CHECK(ARRIVED) if (failed) { arrived = ARRIVED; goto stopped; }
+    auto read = [&](int k) { return ev_arrive_read(kv_event(k), kSplitWorkers, zero_s); };
+    auto stored_on = [&](int id) {
       fence_async_smem();
       tc_fence_before();
       ev_arrive(id, kSplitWorkers);
     };
+    auto stored = [&](int k) { stored_on(kv_event(k)); };
+    int n = 0;
+    uint32_t arrived = 0;
     tmem_st32(trow + C_W + c0, w0);
     tmem_st_wait();
 #pragma unroll 1
-    for (int n = 0; n < end; ++n) {
+    for (; n < end; ++n) {
       const int m = n - begin;                    // of the steps with scores
       const uint32_t ph = n & 1, ph_m = m & 1;    // barriers that complete in every step; in steps with scores
       const int I = p.nblk - 1 - n, irow = I * kBlkB + row;
@@ -368,8 +403,9 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         float v[32];
         tmem_ld32(trow + C_S + c0, v);
         tmem_ld_wait();
+        KV_CHECK(kKvReadZ)
         float hs = half_scale;
-        if (!CUT || m >= 0) hs += read();
+        if (!CUT || m >= 0) hs += read(kKvReadZ);
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float2 a = sigmoid2(make_float2(v[j], v[j + 1]), hs);
@@ -381,25 +417,30 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         }
         store_row32<T>(sK, kPanelB, row, c0, v);
       }
-      stored(kKvStored);
-      if (CUT && m < 0) continue;
+      if (CUT && m < 0) {
+        stored_on(kv_gate_alone(n));
+        continue;
+      }
+      stored(kKvGate);
       B128_MARK(0, n, 2);
       wait(kKvT, ph_m);
       {  // T over Vu, which the state has then read
         float v[32];
         tmem_ld32_lower(trow + C_S + c0, row, c0, v);
+        KV_CHECK(kKvMaskedT)
         wait(kKvW, ph);
         B128_MARK(0, n, 3);
         store_row32<T>(sV, kPanelB, row, c0, v);
+        KV_CHECK(kKvMaskedT)
       }
-      stored(kKvStoredT);
+      stored(kKvMaskedT);
       if (!diag) {   // Wb over Qu
         float v[32];
         tmem_ld32(trow + C_W + c0, v);
         tmem_ld_wait();
         store_row32<T>(smem + S0, kPanelB, row, c0, v);
       }
-      stored(kKvStored);
+      stored(kKvCopyW);
       B128_MARK(0, n, 4);
       // loaded here, not at the top of the step, where the wait for Z is short
       const float lse_i = rvalid ? p.lse[(int64_t)bh * p.N + irow] : 0.f, delta_i = rvalid ? p.delta[(int64_t)bh * p.N + irow] : 0.f;
@@ -410,7 +451,8 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         float v[32], w[32];
         tmem_ld32(trow + C_S + c0, v);
         tmem_ld_wait();
-        const float hs = half_scale + read();
+        KV_CHECK(kKvReadSu)
+        const float hs = half_scale + read(kKvReadSu);
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float2 u = make_float2(v[j], v[j + 1]);
@@ -426,7 +468,8 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         B128_MARK(0, n, 7);
         tmem_ld32(trow + C_S + c0, w);
         tmem_ld_wait();
-        const float s2 = sl2 + read();
+        KV_CHECK(kKvReadSc)
+        const float s2 = sl2 + read(kKvReadSc);
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float2 x = fma2(add2(make_float2(w[j], w[j + 1]), make_float2(v[j], v[j + 1])), splat(s2), splat(-lse_i * kLog2e));
@@ -444,7 +487,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         for (int j = 0; j < 32; j += 2) ppk[j / 2] = Elem<T>::pack2(v[j], v[j + 1]);
         store_row32<T>(sV, kPanelB, row, c0, v);   // P, over T
       }
-      stored(kKvStored);
+      stored(kKvP);
       B128_MARK(0, n, 8);
       wait(kKvDp, ph_m);
       B128_MARK(0, n, 9);
@@ -452,6 +495,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         float v[32], w[32];
         tmem_ld32(trow + C_S + c0, v);
         tmem_ld_wait();
+        KV_CHECK(kKvDs)
 #pragma unroll
         for (int j = 0; j < 32; j += 2) {
           const float2 ds = mul2(Elem<T>::unpack2(ppk[j / 2]), add2(make_float2(v[j], v[j + 1]), splat(-delta_i)));
@@ -460,10 +504,11 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
           w[j] = -du.x; w[j + 1] = -du.y;
         }
         store_row32<T>(sK, kPanelB, row, c0, v);   // dS
-        mbar_wait(bars + kKvDv, ph_m, abortp);
+        wait(kKvDv, ph_m);
         store_row32<T>(smem + S6, kPanelB, row, c0, w);   // dSu, over dO
+        KV_CHECK(kKvDs)
       }
-      stored(kKvStored);
+      stored(kKvDs);
       B128_MARK(0, n, 10);
       wait(kKvX, ph_m);
       B128_MARK(0, n, 11);
@@ -471,12 +516,27 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
       float v[32];
       tmem_ld32(trow + C_S + c0, v);
       tmem_ld_wait();
-      read();
-      if (cc >= 2) mbar_wait(bars + kKvCopied, ph_m, abortp);
+      KV_CHECK(kKvReadX)
+      read(kKvReadX);
+      if (cc >= 2) {
+        wait(kKvCopied, ph_m);
+        KV_CHECK(kKvEvents)
+      }
       store_row32_f32(smem + S5 + cc * kPanelB, row, v);
       fence_async_smem();
-      ev_arrive(kKvStaged, kSplitWorkers);
+      ev_arrive(kv_staged(m), kSplitWorkers);
       B128_MARK(0, n, 12);
+    }
+#undef KV_CHECK
+  stopped:
+    for (; n < end; ++n, arrived = 0) {   // what is left of the events
+      if (CUT && n < begin) {
+        ev_wait(kv_gate_alone(n), kSplitWorkers);
+        continue;
+      }
+#pragma unroll 1
+      for (; arrived < kKvEvents; ++arrived) ev_wait(kv_event((int)arrived), kSplitWorkers);
+      ev_wait(kv_staged(n - begin), kSplitWorkers);
     }
     wait(kKvK, (uint32_t)(end - begin - 1) & 1u);
     float v[32], w[32];

@@ -4,6 +4,7 @@
 // a preset accumulator and a negated operand), plus the two forms whose first operand sits in tensor
 // memory as packed 16-bit pairs.
 #include "common.cuh"
+#include "bwd_common.cuh"
 #include "sm100.cuh"
 
 namespace castle {
@@ -225,6 +226,69 @@ extern "C" int castle_selftest_wait_timeout(int32_t poll_limit, int32_t* polls, 
   castle_wait_timeout_kernel<<<1, 128, 0, (cudaStream_t)stream>>>((uint32_t)poll_limit, polls, status);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : cuda_fail(e, "castle_selftest_wait_timeout launch");
+}
+
+// The same for warps with one job each (ev_arrive), in the roles of the backward's kernels: warp 4 waits for a tile, then takes two
+// events a round from warps 0 to 3 and answers the first of them; they wait for the answer in between.  form 0: neither the tile nor an
+// answer ever comes; 1: both come; 2: the tile does not come, the answers do.
+namespace castle {
+__global__ void __launch_bounds__(160) castle_event_timeout_kernel(uint32_t poll_limit, int32_t rounds, int32_t form, int32_t* result, int32_t* status) {
+  __shared__ uint64_t tile, answer;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  auto event = [](int e) { return 1 + (e & 3); };   // in turn on four barriers: the first after a wait that ran out is not one of the two before it
+  if (tid == 0) {
+    mbar_init(&tile, 1); mbar_init(&answer, 1);
+    mbar_fence_init();
+    abort_flag = 0;
+  }
+  if (warp == 0) { tmem_alloc(&tmem_base_s, 32); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base_s;
+  if (warp == 4) {
+    if (elect_one()) {
+      if (form == 1) mbar_arrive(&tile);
+      result[0] = mbar_wait_ok(&tile, 0, &abort_flag, poll_limit);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int r = 0; r < rounds; ++r) {
+      ev_wait(event(2 * r), 128);
+      if (form != 0 && elect_one()) mbar_arrive(&answer);
+      __syncwarp();
+      ev_wait(event(2 * r + 1), 128);
+    }
+    if (elect_one()) result[1] = 2 * rounds;
+    __syncwarp();
+  } else {
+    int r = 0;
+    uint32_t arrived = 0;
+#pragma unroll 1
+    for (; r < rounds; ++r) {
+      ev_arrive(event(2 * r), 128);
+      if (mbar_wait_failed(&answer, r & 1, &abort_flag, poll_limit)) { arrived = 1; break; }
+      ev_arrive(event(2 * r + 1), 128);
+    }
+    for (; r < rounds; ++r, arrived = 0)
+      for (; arrived < 2; ++arrived) ev_wait(event(2 * r + (int)arrived), 128);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 32);
+  if (tid == 0 && abort_flag) atomicOr(status, CASTLE_STATUS_WAIT_TIMEOUT);
+}
+}  // namespace castle
+
+extern "C" int castle_selftest_event_timeout(int32_t poll_limit, int32_t rounds, int32_t form, int32_t* result, int32_t* status, void* stream) {
+  if (poll_limit < 1 || poll_limit > 65536 || rounds < 1 || rounds > 1024 || form < 0 || form > 2)
+    return reject("castle_selftest_event_timeout: poll_limit must be 1..65536, rounds 1..1024, form 0..2");
+  if (!result || !status) return reject("castle_selftest_event_timeout: null pointer");
+  castle_event_timeout_kernel<<<1, 160, 0, (cudaStream_t)stream>>>((uint32_t)poll_limit, rounds, form, result, status);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : cuda_fail(e, "castle_selftest_event_timeout launch");
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -71,6 +71,27 @@ __device__ __forceinline__ void mbar_wait_lazy_abort(uint64_t* bar, uint32_t par
   *abort_flag = 1;
 }
 
+// The same, for threads that must not go on without what they wait for: whether the phase completed.  LAZY: the flag on every 64th poll.
+template <bool LAZY = false>
+__device__ __forceinline__ bool mbar_wait_ok(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t poll_limit = kWaitPollLimit) {
+  for (uint32_t i = 0; i < poll_limit; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((!LAZY || (i & 63u) == 63u) && *abort_flag) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+// By a whole warp: whether it ended without the phase, the same answer in every lane.  (The vote takes some 35 cycles: the answer is best
+// looked at behind the load from tensor memory that follows.)
+__device__ __forceinline__ bool mbar_wait_failed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t poll_limit = kWaitPollLimit) {
+  const bool over = mbar_wait_ok<true>(bar, parity, abort_flag, poll_limit);
+  return __any_sync(0xffffffffu, !over);
+}
+// For copies and products that are still in flight when a CTA leaves, whatever the abort flag says; bounded as well.
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  for (uint32_t i = 0; i < (1u << 16) && !mbar_try_wait(bar, parity); ++i) { }
+}
+
 // Barrier over the 128 threads (four warps) of one chunk group; ids 1..15 (0 is __syncthreads).
 __device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
