@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import re
 import shutil
 import subprocess
 from pathlib import Path
@@ -115,6 +116,14 @@ def _locked(fn):
             fcntl.flock(lock, fcntl.LOCK_UN)
 
 
+def wrong_registers(text: str):
+    """What ptxas -v says (`text`) against the registers that the kernels which share their launch's registers out anew count on
+    (`check_launch_regs` refuses such a kernel at its launch): a message per kernel that was compiled with another number."""
+    wanted = int(re.search(r"kSplitLaunchRegs = (\d+)", (CSRC / "bwd_common.cuh").read_text()).group(1))
+    used = re.findall(r"Compiling entry function '(\w*castle_(?:bwd_kernel|bwd128_kv_kernel)\w*)'(?:(?!Compiling entry).)*?Used (\d+) registers", text, re.S)
+    return [f"{kernel} was compiled with {n} registers a thread instead of {wanted}" for kernel, n in used if int(n) != wanted]
+
+
 def _compile(jobs, verbose: bool = False):
     """Run the compilers of `jobs` (target, stamp, digest, command for an output path) side by side; readers see
     each old file or the complete new one, never half of it."""
@@ -125,11 +134,12 @@ def _compile(jobs, verbose: bool = False):
     failed = []
     for target, stamp, digest, tmp, proc in running:
         text = proc.communicate()[0]
-        if proc.returncode == 0:
+        wrong = wrong_registers(text)
+        if proc.returncode == 0 and not wrong:
             os.replace(tmp, target)
             stamp.write_text(digest + "\n")
         else:
-            failed.append(f"building {target.name} failed:\n{text}")
+            failed.append(f"building {target.name} failed:\n" + ("\n".join(wrong) if proc.returncode == 0 else text))
             if tmp.exists():
                 tmp.unlink()
         if verbose:
@@ -140,7 +150,7 @@ def _compile(jobs, verbose: bool = False):
 
 def _build_unlocked(force: bool = False, verbose: bool = False):
     def nvcc(out):
-        return [_nvcc()] + NVCC_FLAGS + ["-t", "0", "-Xptxas", "-v" if verbose else "-warn-spills", "-o", str(out)] + \
+        return [_nvcc()] + NVCC_FLAGS + ["-t", "0", "-Xptxas", "-v", "-o", str(out)] + \
                [str(s) for s in _sources()]
     jobs = []
     if force or needs_build():
