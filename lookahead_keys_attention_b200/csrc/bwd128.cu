@@ -361,7 +361,7 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
           mbar_drain(bars + kKvIn, next & 1);
           mbar_drain(bars + kKvDo, last_do > 0 ? last_do & 1 : 0);
         }
-        bulk_wait_read0();   // the sums themselves are complete when the kernel is
+        bulk_wait_read0();   // tiles and sums are complete when the kernel is
       }
       __syncwarp();
       for (; n < end; ++n)   // nothing is asked for any more, for a barrier's last phase may still be open
@@ -642,7 +642,7 @@ castle_bwd128_reverse_kernel(const BwdParams p, const __grid_constant__ CUtensor
     }
     __syncwarp();
   }
-  if (storer && elect_one()) bulk_wait0();
+  if (storer && elect_one()) bulk_wait_read0();
   __syncwarp();
   B128_END(128)
 }
@@ -711,7 +711,6 @@ castle_bwd128_la_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         bulk_wait_read0();
         mbar_arrive(bar_zf);
       }
-      bulk_wait0();
     }
     __syncwarp();
   } else {

@@ -155,6 +155,10 @@ __device__ __forceinline__ void bulk_g2s(void* sdst, const void* gsrc, uint32_t 
                "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// What a CTA owes its bulk stores and reduces before it leaves: that their sources in shared memory have been read (bulk_wait_read0).  The
+// writes themselves are memory operations of the grid like any other: complete and visible to a kernel that starts after the grid, and
+// behind overlap_wait() to one that started before its end (griddepcontrol.wait holds until all prerequisite grids have
+// completed and their memory operations are visible).  bulk_wait0 waits for the writes, which only the CTA itself could need.
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
