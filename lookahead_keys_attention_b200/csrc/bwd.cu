@@ -33,11 +33,14 @@
 namespace castle {
 
 // Optional phase timing (debug builds only): thread 0 of CTA (0,0) stores clock64() at each phase
-// boundary of its first steps behind the fp32 workspace, which the host dumps.
+// boundary of its first steps behind the fp32 workspace, which the host dumps; behind 8 x 32 of these the warp that issues
+// the products does, when what an event let it issue is on its way.
 #ifdef CASTLE_PHASE_TIMING
+#define BISSUE_MARK(k) do { if (lane == 0 && blockIdx.x == 0 && blockIdx.y == 0 && n < 8) p.timing[256 + n * 32 + (k)] = clock64(); } while (0)
 #define BPHASE_MARK(i) do { if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && n < 8) p.timing[n * 32 + (i)] = clock64(); } while (0)
 #else
 #define BPHASE_MARK(i) do { } while (0)
+#define BISSUE_MARK(k) do { } while (0)
 #endif
 
 // Timing experiments only (never in the shipped library): drop the reduces to see what they cost.
@@ -180,23 +183,28 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
           gemm_kk_t<1>(tmem + C_S, at(sQc), at(sVu), ID_SQ_KK, false);          // T = Qc[I] Vu[I]^T, while the gate is formed
           mma_commit(&bar_t);
         }
+        BISSUE_MARK(kEvReadZ);
         next(kEvGate);
         if (elect_one()) {
           if (!diag) gemm_km_t<8>(tmem + C_W, at(sA), at(sVu), ID_D_KM_NEG, true);   // W_K -= A Vu[I], while T is masked; zero at the diagonal block, where nothing reads it
           mma_commit(&bar_w);
         }
+        BISSUE_MARK(kEvGate);
         next(kEvT);        // masked
         if (elect_one()) gemm_kk_t<2>(tmem + C_S, at(sT), at(sA), ID_SQ_KK, false);    // Su/scale = T A^T + Qc[I] Wb^T, while W is copied
+        BISSUE_MARK(kEvT);
         next(kEvCopyW);
         if (elect_one()) {
           if (!diag) gemm_kk_t<1>(tmem + C_S, at(sQc), at(sWb), ID_SQ_KK, true);
           mma_commit(&bar_su);
         }
+        BISSUE_MARK(kEvCopyW);
         next(kEvReadSu);
         if (elect_one()) {
           gemm_kk_t<1>(tmem + C_S, at(sQc), at(sKc), ID_SQ_KK, false);          // Sc/scale = Qc[I] Kc[K]^T, while silu' is formed
           mma_commit(&bar_sc);
         }
+        BISSUE_MARK(kEvReadSu);
         next(kEvReadSc);
         if (elect_one()) {
           mbar_wait(&bar_vd, ph, abortp);
@@ -204,13 +212,16 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
           gemm_kk_t<1>(tmem + C_S, at(sdO), at(sVc), ID_SQ_KK, false);          // dP = dO[I] Vc[K]^T, while P is formed
           mma_commit(&bar_dp);
         }
+        BISSUE_MARK(kEvReadSc);
         next(kEvP);
         if (elect_one()) {
           gemm_mm_t<8>(tmem + C_DVC, at(sKP), at(sdO), ID_D_MM, !first);        // dvc += P^T dO[I], while dS is formed
           mma_commit(&bar_dv);
         }
+        BISSUE_MARK(kEvP);
         next(kEvReadDp);
         if (!first && elect_one()) gemm_kk_t<1>(tmem + C_S, at(sGb), at(sVu), ID_SQ_KK, false);   // dA/scale = Gb Vu[I]^T + dSu^T T
+        BISSUE_MARK(kEvReadDp);
         next(kEvDs);       // and dSu
         if (elect_one()) {
           gemm_mm_t<8>(tmem + C_S, at(sKP), at(sT), ID_SQ_MM, !first);
@@ -218,6 +229,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
           gemm_mm_t<8>(tmem + C_DKC, at(sVD), at(sQc), ID_D_MM, !first);        // dkc += dS^T Qc[I]
           gemm_km_t<8>(tmem + C_X, at(sVD), at(sKc), ID_D_KM, false);           // X = dS Kc[K] + dSu Wb + dT Vu[I]
         }
+        BISSUE_MARK(kEvDs);
         next(kEvReadDa);
         if (elect_one()) {
           gemm_km_t<8>(tmem + C_S, at(sKP), at(sA), ID_SQ_KM, false);           // dT = dSu A, while dZ is formed
@@ -228,9 +240,11 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
           }
           mma_commit(&bar_g);
         }
+        BISSUE_MARK(kEvReadDa);
         next(kEvDz);
         next(kEvReadDt);
         if (elect_one()) gemm_mm_t<8>(tmem + C_X3, at(sT), at(sQu), ID_D_MM, false);   // X3 = dZ^T Qu[K]
+        BISSUE_MARK(kEvReadDt);
         next(kEvDt);       // masked
         if (elect_one()) {
           gemm_mm_t<8>(tmem + C_X2, at(sVD), at(sQc), ID_D_MM, false);          // X2 = dT^T Qc[I] + A^T Gb
@@ -242,8 +256,10 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
           if (!first) gemm_mm_t<8>(tmem + C_X2, at(sA), at(sGb), ID_D_MM, true);
           mma_commit(&bar_l);
         }
+        BISSUE_MARK(kEvDt);
         next(kEvReadX);
         if (!diag && elect_one()) issue_z(ph ^ 1);
+        BISSUE_MARK(kEvReadX);
       }
       __syncwarp();
       if (elect_one()) {
