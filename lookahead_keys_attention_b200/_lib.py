@@ -117,10 +117,10 @@ def _locked(fn):
 
 
 def wrong_registers(text: str):
-    """What ptxas -v says (`text`) against the registers that the kernels which share their launch's registers out anew count on
-    (`check_launch_regs` refuses such a kernel at its launch): a message per kernel that was compiled with another number."""
+    """What ptxas -v says (`text`) against the registers that the kernel which shares its launch's registers out anew counts on
+    (`check_launch_regs` refuses it at its launch): a message per instance that was compiled with another number."""
     wanted = int(re.search(r"kSplitLaunchRegs = (\d+)", (CSRC / "bwd_common.cuh").read_text()).group(1))
-    used = re.findall(r"Compiling entry function '(\w*castle_(?:bwd_kernel|bwd128_kv_kernel)\w*)'(?:(?!Compiling entry).)*?Used (\d+) registers", text, re.S)
+    used = re.findall(r"Compiling entry function '(\w*castle_bwd_kernel\w*)'(?:(?!Compiling entry).)*?Used (\d+) registers", text, re.S)
     return [f"{kernel} was compiled with {n} registers a thread instead of {wanted}" for kernel, n in used if int(n) != wanted]
 
 

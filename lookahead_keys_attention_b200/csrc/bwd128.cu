@@ -96,6 +96,9 @@ __device__ __forceinline__ uint8_t* step_tiles(const BwdParams& p, int I, int K)
 // worked in the passes, it waited as long as the tensor unit's queue was full and the others waited for it: step 15.2 k -> 12.9 k
 // cycles, the kernel at B=1 H=8 N=8190 995 -> 884 us, B=2 H=8 N=1333 104 -> 92, B=8 H=16 N=512 141 -> 133.  What bounds it now: 10.7 k
 // cycles of a step's 1.4 MB through shared memory, and the wait for Qc and Vu, whose slots the last product of a step frees.
+// Every warp keeps the 96 registers of the launch, which is enough.  Shared out as 112 and 32 (castle_bwd_kernel) the issuing and the moving
+// warp spilled: us of the four kernels, so / kept, 16 pairs of 1333 positions 176.2 / 174.1, 8 of 8190 1637 / 1631, 128 of 512 270.4 / 268.3,
+// cut walks of 4 x 4096 and 8 x 2048 360.5 / 356.4 and 214 / 211; as 104 and 64 in between.
 // Tensor memory: W | dkc | dvc | scratch.  Shared memory, seven tiles:
 //   s0 Qu, then Wb | s1 Ku, A, dS | s2 Vu, T, P | s3 Qc | s4 Kc | s5 Vc, staging | s6 dO, dSu, staging
 // with the roles of s1 and s2 exchanged in every other step: P dies first, so that the next Ku lands over it and the next Z runs
@@ -190,7 +193,6 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
   const uint32_t tmem = *tmem_base_s, trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
 
   if (warp >= kSplitWorkers / 32) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSplitHelperRegs));
     if (warp == kSplitWorkers / 32) {
       // ---- the products, in the order that the passes need them
       auto at = [&](uint32_t off) {   // made where it is used: kept in registers over the step the addresses would be spilled
@@ -368,7 +370,6 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
         if (n >= begin) ev_wait(kv_staged(n - begin), kSplitWorkers);
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSplitWorkerRegs));
     const int row = (warp & 3) * 32 + lane, cc = warp >> 2, c0 = cc * 32, krow = k0 + row;
     const float sl2 = p.scale * kLog2e, half_scale = 0.5f * p.scale;
     bool failed;
@@ -890,17 +891,13 @@ static int launch_bwd128_t(const BwdParams& p, const CUtensorMap* in, cudaStream
   constexpr int D = 128;
   const void* kernels[5] = {(const void*)castle_bwd128_kv_kernel<T, false>, (const void*)castle_bwd128_reverse_kernel<T>,
                             (const void*)castle_bwd128_la_kernel<T>, (const void*)castle_bwd128_dqu_kernel<T>, (const void*)castle_bwd128_kv_kernel<T, true>};
-  static std::atomic<bool> regs_known[2] = {{false}, {false}};
-  int rc = check_launch_regs(castle_bwd128_kv_kernel<T, false>, regs_known[0]);
-  if (!rc) rc = check_launch_regs(castle_bwd128_kv_kernel<T, true>, regs_known[1]);
-  if (rc) return rc;
   const size_t smem[5] = {kB128Smem, 6 * kSq + 256, kB128Smem, 6 * kSq + 256, kB128Smem};
   for (int i = 0; i < 5; ++i) {
     cudaError_t e = cudaFuncSetAttribute(kernels[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[i]);
     if (e != cudaSuccess) return cuda_fail(e, "castle_bwd attribute");
   }
   CUtensorMap acc;
-  rc = make_tmap_f32_rows(&acc, p.acc_dqc, p.B * p.H, p.N, D, "gradient workspace");
+  int rc = make_tmap_f32_rows(&acc, p.acc_dqc, p.B * p.H, p.N, D, "gradient workspace");
   if (rc) return rc;
   const int64_t rows = (int64_t)p.B * p.H * p.N;
   constexpr int RPB = 256 / (D / 8);

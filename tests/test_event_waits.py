@@ -31,7 +31,7 @@ class Kernel:
         modulus = int(re.search(function + r"\(int k\) \{ return 1 \+ k % (\d+); \}", text).group(1))
         self.barrier = lambda k: 1 + k % modulus
         kernel = text[text.index(start):]
-        helpers, passes = kernel.index("setmaxnreg.dec"), kernel.index("setmaxnreg.inc")
+        helpers, passes = kernel.index("if (warp >= kSplitWorkers / 32) {"), kernel.index("bool failed;")
         mover = kernel.index("(warp == 17)" if name == "bwd64" else "(warp == kSplitWorkers / 32 + 1)", helpers)
         issuer = kernel[helpers:mover]
         issuer = issuer[issuer.index("#pragma unroll 1"):]
