@@ -26,15 +26,15 @@
 // pass that everybody waited for.  A pass reports twice, on named barriers where only the issuing warp waits: when the accumulator
 // columns are in registers (the next product into them starts under the arithmetic) and when its results are in shared memory.
 // Step 19.1 k -> 15.5 k cycles; the kernel at B=4 N=4096 H=16 2390 -> 1936 us, B=16 H=8 N=1024 387 -> 332, 15 pairs of 777 78.2 -> 63.3.
-// The first tiles and the state are asked for before the CTA's first barrier, and a CTA leaves when its last reduces have been
-// read, not done: 1024 pairs of one block 115.2 -> 112.3 us, 4 pairs of two 23.7 -> 22.3.
+// The first tiles and the state are asked for before the CTA's first barrier: whole backward of 1024 pairs of one block 169.2 ->
+// 167.5 us, B=16 H=8 N=1024 370 -> 367.5.  That a CTA leaves when its last reduces have been read, not done, makes no difference to either.
 #include "bwd_common.cuh"
 
 namespace castle {
 
 // Optional phase timing (debug builds only): thread 0 of CTA (0,0) stores clock64() at each phase
 // boundary of its first steps behind the fp32 workspace, which the host dumps; behind 8 x 32 of these the warp that issues
-// the products does, when what an event let it issue is on its way.
+// the products does, when what an event let it issue is on its way (none for kEvDz, which lets it issue nothing).
 #ifdef CASTLE_PHASE_TIMING
 #define BISSUE_MARK(k) do { if (lane == 0 && blockIdx.x == 0 && blockIdx.y == 0 && n < 8) p.timing[256 + n * 32 + (k)] = clock64(); } while (0)
 #define BPHASE_MARK(i) do { if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0 && n < 8) p.timing[n * 32 + (i)] = clock64(); } while (0)

@@ -153,8 +153,8 @@ castle_bwd128_kv_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m
   float* const zero_s = reinterpret_cast<float*>(bars + kKvBars + 1);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int bh = p.bh0 + blockIdx.x, b = bh / p.H, h = bh % p.H;
-  // The first tiles and the state are asked for before the barrier below; nothing in flight writes what they read (only tiles, sums
-  // and gradients are being written by the kernels before this one).
+  // What B128_BEGIN does, from the moving warp, which can then ask for the first tiles ahead of the barrier below, as the passes do for
+  // the state; nothing in flight writes what they read (only tiles, sums and gradients are being written by the kernels before this one).
   if (warp == kSplitWorkers / 32 + 1 && elect_one()) {
     if (smem_u32(smem) & 1023u) atomicOr(p.status, CASTLE_STATUS_BAD_LAUNCH);
     for (int i = 0; i < kKvBars; ++i) mbar_init(bars + i, i == kKvDp ? 2 : 1);   // dP: the product, and the copy of the gate that dS goes over

@@ -54,7 +54,7 @@ __device__ __forceinline__ void ev_arrive(int id, int threads) { asm volatile("b
 __device__ __forceinline__ void ev_wait(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads + 32) : "memory"); }
 // The arrival when a thread's accumulator columns are in registers.  Returns 0, read from shared memory behind it: the compiler
 // moves an arrival behind arithmetic that does not depend on it, and the next product then starts a pass late, so a constant of
-// the pass has this added to it (dim_head 64, B=4 N=4096 H=16: 2044 -> 1936 us).
+// the pass has this added to it (dim_head 64, B=4 N=4096 H=16: 2120 -> 1960 us; dim_head 128, 8 pairs of 8190: 1770 -> 1635).
 __device__ __forceinline__ float ev_arrive_read(int id, int threads, const float* zero_s) {
   tc_fence_before();
   ev_arrive(id, threads);

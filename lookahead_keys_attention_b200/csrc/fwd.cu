@@ -1079,7 +1079,7 @@ static int fwd_impl(const char* who, const castle_problem_t* p, const castle_ten
   fp.store_caches = caches ? 1 : 0;
   fp.tm = fwd_plan((int64_t)p->batch * p->heads, fp.nblk, p->dim_head).ahead ? (uint4*)((uint8_t*)workspace + tiles * kBlk * (2 * sizeof(float) + p->dim_head * 2)) : nullptr;
 #ifdef CASTLE_PHASE_TIMING
-  fp.timing = (long long*)((char*)workspace + need);  // the caller leaves 1 KB beyond the partials
+  fp.timing = (long long*)((char*)workspace + need);  // the caller leaves 2 KB beyond the partials
 #endif
 
   CUtensorMap maps[9];

@@ -3,10 +3,13 @@
 // allocation, tcgen05.mma with shared-memory operand descriptors, and
 // tcgen05.ld/st between TMEM and registers.
 //
-// Every wait is bounded.  A wait that runs out of polls raises a CTA-wide
-// abort flag in shared memory; from then on every wait in that CTA returns at
-// once, the kernel falls through its (bounded) loops, frees its TMEM and
-// records an error code in the status word the host reads back.
+// Every wait on an mbarrier is bounded.  A wait that runs out of polls raises a
+// CTA-wide abort flag in shared memory; from then on every such wait in that
+// CTA returns at once, the kernel falls through its (bounded) loops, frees its
+// TMEM and records an error code in the status word the host reads back.
+// A wait at a named barrier sees no flag: every warp makes each of its arrivals
+// there also after an abort (ev_arrive in bwd_common.cuh says how, for the
+// kernels whose warps do not all wait where they arrive).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -61,8 +64,7 @@ __device__ __forceinline__ uint32_t mbar_wait(uint64_t* bar, uint32_t parity, vo
 // The same wait with the abort flag looked at on every 64th poll only: the flag reads of one group's polling lanes share the
 // shared-memory port with the other group's products and passes.  us of a forward, so / with the flag read at every poll:
 // 8 x 16 x 2049 x 64 562 / 577, 16 x 8 x 1024 x 64 150 / 152, 1 x 8 x 8190 x 128 701 / 708, 4 x 16 x 4096 x 64 925 / 924.  (The waits of
-// the dim_head-128 backward's loading warps: no difference.  In the dim_head-64 backward, where whole groups poll, it was slower: there
-// the flag read paces the polls.)
+// la's loading warp in the dim_head-128 backward: no difference.)
 __device__ __forceinline__ void mbar_wait_lazy_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t i = 0; i < kWaitPollLimit; ++i) {
     if (mbar_try_wait(bar, parity)) return;
@@ -82,7 +84,8 @@ __device__ __forceinline__ bool mbar_wait_ok(uint64_t* bar, uint32_t parity, vol
   return false;
 }
 // By a whole warp: whether it ended without the phase, the same answer in every lane.  (The vote takes some 35 cycles: the answer is best
-// looked at behind the load from tensor memory that follows.)
+// looked at behind the load from tensor memory that follows.)  us of the backward's kernels, so / with the flag read at every poll: dim_head
+// 64, 1024 pairs of one block 132 / 136, 4 x 16 x 4096 1938 / 1932; dim_head 128, 16 pairs of 1333 174 / 180, 8 of 8190 1628 / 1658.
 __device__ __forceinline__ bool mbar_wait_failed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t poll_limit = kWaitPollLimit) {
   const bool over = mbar_wait_ok<true>(bar, parity, abort_flag, poll_limit);
   return __any_sync(0xffffffffu, !over);
