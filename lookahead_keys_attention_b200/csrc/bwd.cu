@@ -148,7 +148,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
   volatile int* abortp = &abort_flag;
 
   if (warp >= kSplitWorkers / 32) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSplitHelperRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SplitRegs<T>::others));
     if (warp == 16) {
       // ---- the products, in the order that the passes need them; what a pass does not wait for goes behind its commit
       // operand addresses are made where they are used: kept in registers over the step they would be spilled
@@ -345,7 +345,7 @@ castle_bwd_kernel(const BwdParams p, const __grid_constant__ CUtensorMap m_qc, c
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSplitWorkerRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SplitRegs<T>::passes));
     const int quarter = warp & 3, cc = warp >> 2;
     const int row = quarter * 32 + lane;
     const int c0 = cc * 32;

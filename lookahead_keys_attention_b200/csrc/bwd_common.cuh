@@ -34,10 +34,16 @@ struct BwdParams {
 
 // The kernels whose passes, products and tiles are the work of different warps (castle_bwd_kernel, castle_bwd128_kv_kernel): warps
 // 0-15 do the passes, warp 16 issues the products, warp 17 moves tiles, two more fill up the warpgroup.  castle_bwd_kernel shares the
-// launch's registers out anew, 640 x 96 = 61440 as 512 x 112 + 128 x 32 (B=4 N=4096 H=16: 1941 us; 104 and 64 1951, left alone 1976).
+// launch's registers out anew, 640 x 96 = 61440 (SplitRegs).
 constexpr int kSplitWorkers = 512, kSplitThreads = kSplitWorkers + 128;
-constexpr int kSplitLaunchRegs = 96, kSplitWorkerRegs = 112, kSplitHelperRegs = 32;
-static_assert(kSplitWorkers * kSplitWorkerRegs + 128 * kSplitHelperRegs <= kSplitThreads * kSplitLaunchRegs, "setmaxnreg would wait forever");
+constexpr int kSplitLaunchRegs = 96;
+// Each type's share of the passes and of the other warps, as measured: no share makes any instance spill, but the compiler orders the passes
+// otherwise under each.  us of a backward, 112 and 32 / 104 and 64 / 96 everywhere: bfloat16 64 pairs of 4096 positions 2012 / 2019 / 2045,
+// 8 of 3000 210.8 / 210.9 / 214.3; float16 2064 / 2025 / 2074, 216.8 / 209.8 / 218.2, 15 of 777 72.4 / 70.5 / 72.6.
+template <typename T> struct SplitRegs { static constexpr int passes = 112, others = 32; };
+template <> struct SplitRegs<__half> { static constexpr int passes = 104, others = 64; };
+template <typename T> constexpr bool split_regs_fit() { return kSplitWorkers * SplitRegs<T>::passes + 128 * SplitRegs<T>::others <= kSplitThreads * kSplitLaunchRegs; }
+static_assert(split_regs_fit<__half>() && split_regs_fit<__nv_bfloat16>(), "setmaxnreg would wait forever");
 
 // Events: named barriers on which the passes' `threads` arrive and go on, and one warp besides waits.  Such a barrier counts arrivals,
 // whoever makes them, and sees no abort flag: a warp that arrived again before its last arrival there was taken would upset the count and
